@@ -1,5 +1,5 @@
-// Absorbed multi-head latent attention (MLA) over the token-granular latent KV pool — decode and
-// ragged extend in one kernel.  DeepSeek-V2-Lite, BASELINE configs[3].
+// Absorbed multi-head latent attention (MLA) over the token-granular latent KV pool on tcgen05 — decode and ragged
+// extend in one kernel.
 //
 // Reference: DeepseekV2AttentionMLA.forward_absorb (python/sglang/srt/models/deepseek_v2.py:633-706)
 // over MLATokenToKVPool rows [kv_a_normed(kv_lora) || k_pe_roped(rope)] (mem_cache/memory_pool.py:
@@ -10,23 +10,51 @@
 // prefill batches without a cached prefix; the absorbed form used here for every batch is the same
 // function of the same inputs (oracle/deepseek_oracle.py checks both against each other).
 //
-// One CTA = one query token x one group of 16 heads x one KV split.  Both products run on the
-// tensor cores through warp-level mma.sync m16n8k16 (M = the 16 heads): this is the first MLA
-// kernel of the repo; the tcgen05 swap-AB form of attn_decode.cu with N = 16 real heads is the
-// planned successor.  Per 32-token chunk:
-//   K rows (= V rows) -> smem by 16-byte cp.async through req_to_token, double buffered;
-//   S[16 x 32]  = Q[16 x DL] K^T      k-steps split over the 8 warps, partials reduced in smem;
-//   online softmax, one warp per pair of heads, exp2 domain;
-//   O[16 x DV] += P[16 x 32] V        warp w owns output columns [64 w, 64 w + 64).
+// Swap-AB formulation: an item is TQ query tokens x 16 heads = N columns (decode: 1 x 16, extend: 4 x 16),
+//     S^T[64 kv x N]  = K_tile[64 x 576] * Q^T           (36 MMAs, M = 64)
+//     O^T[512 x N]   += V_tile^T[512 x 64 kv] * P^T       (4 blocks of 128 value columns x 4 MMAs, M = 128)
+// so a latent row enters an SM once per N columns, serves both products from the same shared memory, and the fp32
+// output of a whole item (4 N columns of TMEM) stays on chip.  N = 64 is what fits: 72 KB of Q, two 72 KB K/V tiles
+// and 8 KB of P are the 227 KB of an SM, 256 columns of O^T and two S^T in two halves the 512 of its TMEM.
+//
+// Work split.  The tiles of all items, one after another, are one list that the CTAs (one per SM) cut into equal
+// contiguous ranges; lengths are read on the device, so nothing is planned on the host.  A CTA that starts or ends
+// inside an item leaves a partial (max, sum, O^T) in the workspace and a second small kernel merges the parts of each
+// such item; with many items per CTA the cuts are moved to item starts instead (`snap`) and nothing is merged.
+//
+// warps 0-3: softmax, O rescale, epilogue     warps 4-5: loaders     warp 6: MMA issuer + TMEM allocator.
+// The K/V ring is made of slots of 16 KB (one pair of a tile's 64-column blocks, what one PV block reads) and of 8 KB
+// (its rope block, free after S), each given back by itself: 2.75 tiles at N = 16, 2 at N = 64.  A tile's copies meet on
+// one barrier.  Full tiles of 64 consecutive slots come by TMA (four boxes of 64 rows x 2 blocks and one of 64 x 1),
+// anything else by 16-byte cp.async through req_to_token.  The
+// softmax is the lazily rescaled one of attn_decode.cu: scores are read from TMEM in the 16x256b fragment layout (all
+// 32 lanes of a warp busy although M = 64 fills 16 lanes per warp), P goes back as stmatrix-transposed K-major rows.
+//
+// Decode streams each latent row once: 64 requests of 1088 keys (83 MB) take 28 us, about 3000 clk per 72 KB tile and SM
+// (6.8 TB/s in the steady state) after 9000 clk until the first tile has landed; one CTA per token, head group and split
+// with warp-level MMAs took 54 us.  MMAs (M = 64: 23 clk at N = 16, 31 at N = 64) are hidden as long as the issuer's code
+// stays a short loop.
+//
+// Every mbarrier wait is bounded: a wait that runs out marks the CTA dead, all later waits fall through, the kernel
+// finishes without waiting and counts itself in g_mla_wait_expired.
+#include <cuda.h>
+
 #include "common.cuh"
 #include "ptx.cuh"
+#include "tmap.cuh"
 
 namespace spd {
 
-constexpr int kMlaThreads = 256;
-constexpr int kMlaChunk = 32;
-constexpr int kMlaHeads = 16;
-constexpr int kMlaMaxSplits = 8;
+constexpr int kMlaThreads = 224;
+constexpr int kMlaTile = 64;     // kv tokens per tile
+constexpr int kMlaHeads = 16;    // heads per item
+constexpr int kMlaDL = 576, kMlaDV = 512;
+constexpr int kMlaBlk = kMlaTile * 128;       // one [64 rows x 64 columns] swizzle block of a tile
+constexpr int kMlaMisc = 2048;
+constexpr float kMlaRescale = 8.0f;           // log2 units a score may exceed the reference max before it is raised
+constexpr int kMlaWaitTries = 1 << 22;
+
+__device__ unsigned int g_mla_wait_expired;
 
 struct MlaParams {
   void* out;             // [items, H, DV]
@@ -37,264 +65,769 @@ struct MlaParams {
   const int64_t* seq_lens;          // decode (extend: nullptr)
   const int32_t* prefix_lens;       // extend
   const int32_t* extend_start_loc;  // extend
-  int batch, H, splits;
+  int batch, total, H, hgs;         // total: query tokens (extend); hgs: groups of 16 heads
   int64_t q_stride, out_stride, rtt_stride;
   float scale_log2;
-  float* o_part;   // [item][H][splits][DV]
-  float* ml_part;  // [item][H][splits][2]
+  int min_tiles;   // fewest tiles a CTA takes
+  int snap;        // 1: CTA ranges start at item starts, nothing is split
+  int cols;        // columns of a partial: TQ x min(H, 16)
+  float* o_part;   // [2 * grid][cols][DV]
+  float* ml_part;  // [2 * grid][cols][2]
+  int* info;       // [grid][8]: see mla_merge_kernel
 };
 
-template <typename T>
-__device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1);
-template <>
-__device__ __forceinline__ void mma_16816<__nv_bfloat16>(float (&d)[4], const uint32_t (&a)[4], uint32_t b0,
-                                                         uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-template <>
-__device__ __forceinline__ void mma_16816<__half>(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+template <bool kExtend>
+struct MlaShape {
+  static constexpr int TQ = kExtend ? 4 : 1;
+  static constexpr int N = TQ * kMlaHeads;
+  static constexpr int kQBytes = 9 * N * 128;
+  static constexpr int kPBytes = N * 128;
+  static constexpr int kPairs = kExtend ? 8 : 11;  // ring slots of 16 KB: one pair of 64-column blocks of a tile
+  static constexpr int kRopes = kExtend ? 2 : 3;   // ring slots of 8 KB: a tile's rope block
+  static constexpr int kRing = kPairs * 2 * kMlaBlk + kRopes * kMlaBlk;
+  static constexpr int kBars = kPairs + kRopes + 4 + 9;
+  static constexpr int kSmem = kQBytes + kRing + kPBytes + kMlaMisc + 1024;
+  static constexpr int kOCols = 4 * N;             // TMEM columns of O^T, then two S^T of two halves
+  static constexpr int kTmem = 8 * N;
+};
+static_assert(MlaShape<true>::kSmem <= 232448 && MlaShape<false>::kSmem <= 232448 && MlaShape<true>::kTmem <= 512,
+              "does not fit an SM");
+static_assert(MlaShape<true>::kBars * 8 + 40 + 256 + 5 * 4 * 64 <= kMlaMisc &&
+                  MlaShape<false>::kBars * 8 + 40 + 256 + 5 * 4 * 16 <= kMlaMisc,
+              "misc area");
+
+// a place in a ring and the parity of its current round
+template <int n>
+struct MlaSlot {
+  int i = 0;
+  uint32_t round = 0;
+  __device__ __forceinline__ void next() {
+    if (++i == n) {
+      i = 0;
+      round ^= 1;
+    }
+  }
+};
+
+__device__ __forceinline__ void mla_wait(uint64_t* bar, uint32_t parity, volatile int* dead) {
+  for (int i = 0; i < kMlaWaitTries; ++i) {
+    if (mbar_try_wait(bar, parity)) return;
+    if (*dead) return;
+  }
+  *dead = 1;
 }
 
-// DL, DV: latent row width and value width (elements).  Row stride in smem = DL + 8 elements:
-// (DL + 8) / 2 = 292 words = 4 (mod 32), so the 8 rows x 4 words an MMA fragment load touches fall
-// into 32 distinct banks.
-template <typename T, int DL, int DV, bool kExtend>
-__global__ void __launch_bounds__(kMlaThreads)
-attn_mla_kernel(const MlaParams p) {
-  constexpr int LD = DL + 8;
-  constexpr int KSTEPS = DL / 16;
-  constexpr int VEC_PER_ROW = DL / 8;
-  extern __shared__ __align__(16) uint8_t mla_smem[];
-  T* sQ = reinterpret_cast<T*>(mla_smem);                       // [16][LD]
-  T* sK = sQ + kMlaHeads * LD;                                  // [2][32][LD]
-  float* sS = reinterpret_cast<float*>(sK + 2 * kMlaChunk * LD);  // [8][16][32] partial scores
-  T* sP = reinterpret_cast<T*>(sS + 8 * kMlaHeads * kMlaChunk);   // [16][40]
-  float* s_m = reinterpret_cast<float*>(sP + kMlaHeads * 40);     // [16]
-  float* s_l = s_m + 16;
-  float* s_alpha = s_l + 16;
+// an item: one token (decode) or group of four tokens (extend) of a request, times 16 heads
+struct MlaItem {
+  int hg, r, j;                       // head group, request, token group
+  int row0, ntok, p0, vis, load_end;  // first query row, tokens, position of the first, visible keys, loadable keys
+  int ntiles, next_r;                 // next_r: 1 when the request has no further group
+};
 
-  griddep_wait();
-  const int item = blockIdx.z, hg = blockIdx.y, split = blockIdx.x;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int g = lane >> 2, tq = lane & 3;
-  const int h0 = hg * kMlaHeads;
-  const int nh = min(kMlaHeads, p.H - h0);
-  int req, L;
+__device__ __forceinline__ void mla_request(const MlaParams& p, int r, int& start, int& ext, int& prefix) {
+  start = p.extend_start_loc[r];
+  ext = (r + 1 < p.batch ? p.extend_start_loc[r + 1] : p.total) - start;
+  prefix = p.prefix_lens[r];
+}
+
+template <bool kExtend>
+__device__ __forceinline__ void mla_set_item(const MlaParams& p, MlaItem& it) {
   if constexpr (kExtend) {
-    int lo = 0, hi = p.batch - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (p.extend_start_loc[mid] <= item) lo = mid; else hi = mid - 1;
-    }
-    req = lo;
-    L = p.prefix_lens[req] + (item - p.extend_start_loc[req]) + 1;
+    constexpr int TQ = MlaShape<true>::TQ;
+    int start, ext, prefix;
+    mla_request(p, it.r, start, ext, prefix);
+    const int i0 = it.j * TQ;
+    it.ntok = min(TQ, ext - i0);
+    it.row0 = start + i0;
+    it.p0 = prefix + i0;
+    it.vis = it.p0 + it.ntok;
+    it.load_end = prefix + ext;
+    it.next_r = i0 + TQ >= ext;
   } else {
-    req = item;
-    L = static_cast<int>(p.seq_lens[req]);
+    const int L = static_cast<int>(p.seq_lens[it.r]);
+    it.ntok = 1;
+    it.row0 = it.r;
+    it.p0 = L - 1;
+    it.vis = it.load_end = L;
+    it.next_r = 1;
   }
-  const int32_t* rtt = p.req_to_token + p.req_pool_indices[req] * p.rtt_stride;
-  int per = (L + p.splits - 1) / p.splits;
-  per = (per + kMlaChunk - 1) / kMlaChunk * kMlaChunk;
-  const int t0 = split * per;
-  const int t1 = min(L, t0 + per);
-  const int n_chunks = t1 > t0 ? (t1 - t0 + kMlaChunk - 1) / kMlaChunk : 0;
+  it.ntiles = max(1, (it.vis + kMlaTile - 1) / kMlaTile);
+}
 
-  // Q rows of this head group (rows >= nh are zero)
-  {
-    const T* qb = reinterpret_cast<const T*>(p.q) + item * p.q_stride + static_cast<int64_t>(h0) * DL;
-    for (int v = tid; v < kMlaHeads * VEC_PER_ROW; v += kMlaThreads) {
-      const int r = v / VEC_PER_ROW, c = v - r * VEC_PER_ROW;
-      uint4 val = make_uint4(0, 0, 0, 0);
-      if (r < nh) val = *reinterpret_cast<const uint4*>(qb + r * DL + c * 8);
-      *reinterpret_cast<uint4*>(sQ + r * LD + c * 8) = val;
-    }
-    if (tid < 16) { s_m[tid] = -INFINITY; s_l[tid] = 0.f; }
+// tiles of the first n token groups of 4 with `prefix` cached tokens, all of them full:
+// sum over k = 1..n of ceil((prefix + 4 k) / 64) = sum of floor((k + u) / 16), u = floor((prefix + 63) / 4)
+__device__ __forceinline__ int mla_floor16_sum(int x) {  // sum of floor(i / 16), i = 0..x
+  const int q = x >> 4;
+  return 8 * q * (q - 1) + q * ((x & 15) + 1);
+}
+__device__ __forceinline__ int mla_group_tiles(int prefix, int n) {
+  const int u = (prefix + 63) >> 2;
+  return mla_floor16_sum(n + u) - mla_floor16_sum(u);
+}
+template <bool kExtend>
+__device__ __forceinline__ int mla_request_tiles(const MlaParams& p, int r) {
+  if constexpr (kExtend) {
+    int start, ext, prefix;
+    mla_request(p, r, start, ext, prefix);
+    if (ext <= 0) return 0;
+    return mla_group_tiles(prefix, ext / 4) + (ext % 4 ? (prefix + ext + kMlaTile - 1) / kMlaTile : 0);
+  } else {
+    return max(1, (static_cast<int>(p.seq_lens[r]) + kMlaTile - 1) / kMlaTile);
   }
-  const T* pool = reinterpret_cast<const T*>(p.kv_pool);
-  auto load_chunk = [&](int ci) {
-    T* dst = sK + (ci & 1) * kMlaChunk * LD;
-    const int base = t0 + ci * kMlaChunk;
-    for (int v = tid; v < kMlaChunk * VEC_PER_ROW; v += kMlaThreads) {
-      const int r = v / VEC_PER_ROW, c = v - r * VEC_PER_ROW;
-      const bool valid = base + r < t1;
-      const int64_t slot = valid ? rtt[base + r] : 0;
-      cp_async16(smem_u32(dst + r * LD + c * 8), pool + slot * DL + c * 8, valid);
-    }
-    cp_async_commit();
-  };
+}
 
-  float o_acc[8][4];
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) o_acc[i][j] = 0.f;
+template <bool kExtend>
+__device__ __forceinline__ void mla_next_item(const MlaParams& p, MlaItem& it) {
+  if (!it.next_r) {
+    ++it.j;
+  } else {
+    it.j = 0;
+    do {
+      if (++it.r == p.batch) {
+        it.r = 0;
+        if (++it.hg == p.hgs) return;  // past the end: the caller has no tiles left
+      }
+      if constexpr (kExtend) {
+        int start, ext, prefix;
+        mla_request(p, it.r, start, ext, prefix);
+        if (ext > 0) break;
+      } else {
+        break;
+      }
+    } while (true);
+  }
+  mla_set_item<kExtend>(p, it);
+}
 
-  if (n_chunks > 0) load_chunk(0);
-  for (int ci = 0; ci < n_chunks; ++ci) {
-    if (ci + 1 < n_chunks) {
-      load_chunk(ci + 1);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
+// walks the CTA's tiles: every role keeps its own copy
+template <bool kExtend>
+struct MlaCursor {
+  MlaItem it;
+  int tile, left, seg;  // left: tiles of the CTA's range that remain; seg: items left behind so far
+  bool valid;
+  __device__ __forceinline__ void init(const MlaParams& p, const int* start, int count) {
+    it.hg = start[0];
+    it.r = start[1];
+    it.j = start[2];
+    tile = start[3];
+    left = count;
+    seg = 0;
+    valid = left > 0;
+    if (!valid) return;
+    mla_set_item<kExtend>(p, it);
+    if (p.snap && tile > 0) {  // the item belongs to the CTA before
+      left -= it.ntiles - tile;
+      tile = 0;
+      valid = left > 0;
+      if (valid) mla_next_item<kExtend>(p, it);
     }
-    __syncthreads();
-    const T* kb = sK + (ci & 1) * kMlaChunk * LD;
-    const int n_valid = min(kMlaChunk, t1 - (t0 + ci * kMlaChunk));
-    // ---- S partials: this warp's k-steps ----
-    float s_acc[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) s_acc[i][j] = 0.f;
-    for (int ks = warp; ks < KSTEPS; ks += 8) {
-      const int k0 = ks * 16;
-      uint32_t a[4];
-      a[0] = *reinterpret_cast<const uint32_t*>(sQ + g * LD + k0 + 2 * tq);
-      a[1] = *reinterpret_cast<const uint32_t*>(sQ + (g + 8) * LD + k0 + 2 * tq);
-      a[2] = *reinterpret_cast<const uint32_t*>(sQ + g * LD + k0 + 8 + 2 * tq);
-      a[3] = *reinterpret_cast<const uint32_t*>(sQ + (g + 8) * LD + k0 + 8 + 2 * tq);
-#pragma unroll
-      for (int nt = 0; nt < 4; ++nt) {
-        const T* kr = kb + (nt * 8 + g) * LD + k0 + 2 * tq;
-        const uint32_t b0 = *reinterpret_cast<const uint32_t*>(kr);
-        const uint32_t b1 = *reinterpret_cast<const uint32_t*>(kr + 8);
-        mma_16816<T>(s_acc[nt], a, b0, b1);
+  }
+  // whether this tile is the last of its item here
+  __device__ __forceinline__ bool ends(const MlaParams& p) const {
+    return tile + 1 == it.ntiles || (!p.snap && left == 1);
+  }
+  __device__ __forceinline__ void next(const MlaParams& p) {
+    const bool e = ends(p);
+    --left;
+    if (!e) {
+      ++tile;
+      return;
+    }
+    ++seg;
+    tile = 0;
+    valid = left > 0;
+    if (valid) mla_next_item<kExtend>(p, it);
+  }
+};
+
+// [rows x 64 columns] 16-bit swizzle block: 16-byte chunk `c` (0..7) of row `row`
+__device__ __forceinline__ uint32_t mla_off(int row, int c) { return row * 128 + ((c ^ (row & 7)) << 4); }
+
+__device__ __forceinline__ bool mla_bar_or(bool pred) {  // barrier + OR over the 128 softmax threads
+  uint32_t out;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 q, %1, 0;\n\t"
+      "barrier.cta.red.or.pred p, 1, 128, q;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(out)
+      : "r"(static_cast<uint32_t>(pred))
+      : "memory");
+  return out != 0;
+}
+__device__ __forceinline__ void mla_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+__device__ __forceinline__ bool mla_loader_and(bool pred) {  // barrier + AND over the 64 loader threads
+  uint32_t out;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 q, %1, 0;\n\t"
+      "barrier.cta.red.and.pred p, 2, 64, q;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(out)
+      : "r"(static_cast<uint32_t>(pred))
+      : "memory");
+  return out != 0;
+}
+
+// 16 lanes x N columns of fp32 accumulators as mma fragments: value 4 g + e of lane l is row (l >> 2) + 8 (e >> 1),
+// column 8 g + 2 (l & 3) + (e & 1)
+__device__ __forceinline__ void mla_ld_frag(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
+}
+__device__ __forceinline__ void mla_ld_frag(uint32_t taddr, uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x8.b32 "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]),
+        "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
+        "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr)
+      : "memory");
+}
+// four 8 x 8 fragments stored transposed: lane i's address is row (i & 7) of matrix i >> 3
+__device__ __forceinline__ void mla_stsm_x4_t(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b),
+               "r"(c), "r"(d)
+               : "memory");
+}
+
+template <typename T, bool kExtend>
+__global__ void __launch_bounds__(kMlaThreads, 1)
+attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant__ CUtensorMap tmR, const MlaParams p) {
+  using S = MlaShape<kExtend>;
+  constexpr int N = S::N, TQ = S::TQ;
+  extern __shared__ uint8_t mla_smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(mla_smem_raw) + 1023) &
+                                             ~static_cast<uintptr_t>(1023));
+  uint8_t* sK = smem;                          // kPairs x 16 KB
+  uint8_t* sR = sK + S::kPairs * 2 * kMlaBlk;  // kRopes x 8 KB
+  uint8_t* sQ = sK + S::kRing;                 // 9 blocks of [N x 64]
+  uint8_t* sP = sQ + S::kQBytes;               // [N x 64]
+  uint64_t* t_full = reinterpret_cast<uint64_t*>(sP + S::kPBytes);  // [4]: tile t & 3 has landed
+  uint64_t* k_empty = t_full + 4;                                   // [kPairs]
+  uint64_t* r_empty = k_empty + S::kPairs;                          // [kRopes]
+  uint64_t* s_full = r_empty + S::kRopes;                           // [2]
+  uint64_t* s_empty = s_full + 2;                                   // [2]
+  uint64_t* p_full = s_empty + 2;
+  uint64_t* p_empty = p_full + 1;
+  uint64_t* o_empty = p_full + 2;
+  uint64_t* q_full = p_full + 3;
+  uint64_t* q_empty = p_full + 4;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(p_full + 5);
+  volatile int* dead = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  int* s_start = reinterpret_cast<int*>(tmem_slot + 2);  // hg, r, j, tile
+  volatile int* s_gath = s_start + 4;                    // [4]: whether tile t & 3 was gathered
+  int* s_slot = s_start + 8;                             // [64] slots of a gathered tile
+  float* red = reinterpret_cast<float*>(s_slot + 64);    // [4][N]
+  float* s_col = red + 4 * N;                            // [N]: rescale factors, then 1 / sum
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (warp == 6) {
+    if (lane == 0) {
+      for (int i = 0; i < 4; ++i) mbar_init(&t_full[i], 65);
+      for (int i = 0; i < S::kPairs; ++i) mbar_init(&k_empty[i], 1);
+      for (int i = 0; i < S::kRopes; ++i) mbar_init(&r_empty[i], 1);
+      for (int i = 0; i < 2; ++i) {
+        mbar_init(&s_full[i], 1);
+        mbar_init(&s_empty[i], 4);
       }
+      mbar_init(p_full, 128);
+      mbar_init(p_empty, 1);
+      mbar_init(o_empty, 4);
+      mbar_init(q_full, 64);
+      mbar_init(q_empty, 1);
+      *dead = 0;
+      fence_barrier_init();
     }
-    {
-      float* my = sS + warp * (kMlaHeads * kMlaChunk);
+    __syncwarp();
+    tmem_alloc(tmem_slot, S::kTmem);
+    tmem_relinquish();
+  }
+  griddep_wait();
+
+  // ---- this CTA's range of the tile list ----
+  int* scan = reinterpret_cast<int*>(sK);
+  const int per_thread = (p.batch + kMlaThreads - 1) / kMlaThreads;
+  const int r0 = tid * per_thread, r1 = min(p.batch, r0 + per_thread);
+  int sum = 0;
+  for (int r = r0; r < r1; ++r) sum += mla_request_tiles<kExtend>(p, r);
+  int incl = sum;
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt) {
-        const int col = nt * 8 + 2 * tq;
-        my[g * kMlaChunk + col] = s_acc[nt][0];
-        my[g * kMlaChunk + col + 1] = s_acc[nt][1];
-        my[(g + 8) * kMlaChunk + col] = s_acc[nt][2];
-        my[(g + 8) * kMlaChunk + col + 1] = s_acc[nt][3];
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  if (lane == 31) scan[warp] = incl;
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  int before = 0, all = 0;
+#pragma unroll
+  for (int w = 0; w < kMlaThreads / 32; ++w) {
+    if (w < warp) before += scan[w];
+    all += scan[w];
+  }
+  const int total = all * p.hgs;
+  const int grid = static_cast<int>(gridDim.x), cta = static_cast<int>(blockIdx.x);
+  const int per = max(p.min_tiles, (total + grid - 1) / grid);
+  const int t_begin = min(total, per * cta), t_count = min(total, t_begin + per) - t_begin;
+  if (t_count > 0) {
+    const int hg = t_begin / all;
+    int rem = t_begin - hg * all - (before + incl - sum);
+    if (rem >= 0 && rem < sum) {  // exactly one thread: the one whose requests the range starts in
+      int r = r0;
+      for (;; ++r) {
+        const int w = mla_request_tiles<kExtend>(p, r);
+        if (rem < w) break;
+        rem -= w;
       }
-    }
-    __syncthreads();
-    // ---- reduce the 8 partials + online softmax: warp w owns heads w and w + 8, lane = token ----
-#pragma unroll
-    for (int hh = 0; hh < 2; ++hh) {
-      const int h = warp + hh * 8;
-      float s = 0.f;
-#pragma unroll
-      for (int w8 = 0; w8 < 8; ++w8) s += sS[w8 * (kMlaHeads * kMlaChunk) + h * kMlaChunk + lane];
-      s = lane < n_valid ? s * p.scale_log2 : -INFINITY;
-      const float m_old = s_m[h];
-      const float m_new = fmaxf(m_old, warp_max(s));
-      const float pj = exp2f(s - m_new);
-      const T pt = from_f32<T>(pj);
-      const float ps = warp_sum(to_f32<T>(pt));  // sum what the tensor core multiplies
-      const float alpha = (m_old == -INFINITY) ? 0.f : exp2f(m_old - m_new);
-      sP[h * 40 + lane] = pt;
-      __syncwarp();
-      if (lane == 0) { s_m[h] = m_new; s_l[h] = s_l[h] * alpha + ps; s_alpha[h] = alpha; }
-    }
-    __syncthreads();
-    // ---- O += P V : this warp's 64 output columns ----
-    {
-      const float al0 = s_alpha[g], al1 = s_alpha[g + 8];
-#pragma unroll
-      for (int nt = 0; nt < 8; ++nt) {
-        o_acc[nt][0] *= al0; o_acc[nt][1] *= al0; o_acc[nt][2] *= al1; o_acc[nt][3] *= al1;
-      }
-#pragma unroll
-      for (int kk = 0; kk < 2; ++kk) {
-        uint32_t a[4];
-        a[0] = *reinterpret_cast<const uint32_t*>(sP + g * 40 + kk * 16 + 2 * tq);
-        a[1] = *reinterpret_cast<const uint32_t*>(sP + (g + 8) * 40 + kk * 16 + 2 * tq);
-        a[2] = *reinterpret_cast<const uint32_t*>(sP + g * 40 + kk * 16 + 8 + 2 * tq);
-        a[3] = *reinterpret_cast<const uint32_t*>(sP + (g + 8) * 40 + kk * 16 + 8 + 2 * tq);
-        const unsigned short* vb = reinterpret_cast<const unsigned short*>(kb);
-#pragma unroll
-        for (int nt = 0; nt < 8; ++nt) {
-          const int d = warp * 64 + nt * 8 + g;
-          const int r0 = kk * 16 + 2 * tq;
-          const uint32_t b0 = static_cast<uint32_t>(vb[r0 * LD + d]) |
-                              (static_cast<uint32_t>(vb[(r0 + 1) * LD + d]) << 16);
-          const uint32_t b1 = static_cast<uint32_t>(vb[(r0 + 8) * LD + d]) |
-                              (static_cast<uint32_t>(vb[(r0 + 9) * LD + d]) << 16);
-          mma_16816<T>(o_acc[nt], a, b0, b1);
+      int j = 0;
+      if constexpr (kExtend) {
+        int start, ext, prefix;
+        mla_request(p, r, start, ext, prefix);
+        int lo = 0, hi = (ext - 1) / TQ;  // last group that starts at or before tile `rem`
+        while (lo < hi) {
+          const int mid = (lo + hi + 1) >> 1;
+          if (mla_group_tiles(prefix, mid) <= rem) lo = mid; else hi = mid - 1;
         }
+        j = lo;
+        rem -= mla_group_tiles(prefix, j);
+      }
+      s_start[0] = hg;
+      s_start[1] = r;
+      s_start[2] = j;
+      s_start[3] = rem;
+    }
+  }
+  fence_proxy_async_smem();  // the scan's generic writes to the tile area, before copies land there
+  __syncthreads();
+  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_O = tmem_base, tmem_S = tmem_base + S::kOCols;
+  MlaCursor<kExtend> c;
+  c.init(p, s_start, t_count);
+
+  if (warp == 6) {
+    // ===================== MMA issuer =====================
+    // One copy of each step in one loop: straight-line code of 52 MMAs would stream through the instruction cache
+    // (it ran at 190 clk per MMA).
+    if (elect_one()) {
+      constexpr uint32_t idesc_s = umma_idesc<T>(64, N, 0, 0);   // A = K (K-major), B = Q (K-major)
+      constexpr uint32_t idesc_o = umma_idesc<T>(128, N, 1, 0);  // A = V^T (MN-major), B = P^T (K-major)
+      // descriptors in halves: the upper one is a constant, the lower one moves by 16-byte units
+      const uint64_t dk = umma_desc_sw128(smem_u32(sK), 16, 1024), dr = umma_desc_sw128(smem_u32(sR), 16, 1024);
+      const uint32_t hi = static_cast<uint32_t>(dk >> 32), k_lo = static_cast<uint32_t>(dk), r_lo = static_cast<uint32_t>(dr);
+      const uint32_t v_lo = static_cast<uint32_t>(umma_desc_sw128(smem_u32(sK), kMlaBlk, 1024));
+      const uint32_t q_lo = static_cast<uint32_t>(umma_desc_sw128(smem_u32(sQ), 16, 1024));
+      const uint32_t p_lo = static_cast<uint32_t>(umma_desc_sw128(smem_u32(sP), 16, 1024));
+      int ts = 0, tp = 0;             // tiles whose S / PV has been issued
+      uint32_t firsts = 0, segs = 0;  // bit (tile & 1): first tile of its item here; parity of its item's number
+      bool cross = true;              // the next S belongs to another item than the last
+      MlaSlot<S::kPairs> ks, kp;      // next pair of the S stream / of the PV stream
+      MlaSlot<S::kRopes> rs;
+      while (c.valid || tp < ts) {
+        // S of the next tile goes before PV of this one if its rows have landed — and not across items, where its Q may
+        // still be on the way: PV frees ring slots, so it never waits behind a copy
+        if (c.valid && (ts == tp || (ts == tp + 1 && !cross && mbar_test(&t_full[ts & 3], (ts >> 2) & 1)))) {
+          const int b = ts & 1;
+          if (cross) mla_wait(q_full, c.seg & 1, dead);
+          firsts = (firsts & ~(1u << b)) | (cross ? 1u << b : 0u);
+          segs = (segs & ~(1u << b)) | ((c.seg & 1) << b);
+          mla_wait(&s_empty[b], ((ts >> 1) & 1) ^ 1, dead);
+          const uint32_t d = tmem_S + b * 2 * N;
+          mla_wait(&t_full[ts & 3], (ts >> 2) & 1, dead);
+          if (cross || s_gath[ts & 3]) fence_proxy_async_smem();  // Q, and gathered tiles, come by cp.async
+          tc_fence_after_sync();
+          // two accumulators in turn; the softmax adds them
+          uint32_t qa = q_lo;
+#pragma unroll 1
+          for (int i = 0; i < 4; ++i) {
+            const uint32_t ka = k_lo + ks.i * (2 * kMlaBlk >> 4);
+            ks.next();
+#pragma unroll
+            for (int kk = 0; kk < 8; ++kk)
+              umma_ss_lo(d + (kk & 1) * N, ka + (kk >> 2) * (kMlaBlk >> 4) + (kk & 3) * 2,
+                         qa + (kk >> 2) * (N * 128 >> 4) + (kk & 3) * 2, hi, idesc_s, (i > 0 || kk > 1) ? 1u : 0u);
+            qa += 2 * (N * 128 >> 4);
+          }
+          const uint32_t ra = r_lo + rs.i * (kMlaBlk >> 4);
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk) umma_ss_lo(d + (kk & 1) * N, ra + kk * 2, qa + kk * 2, hi, idesc_s, 1u);
+          umma_commit(&r_empty[rs.i]);
+          rs.next();
+          umma_commit(&s_full[b]);
+          cross = c.ends(p);
+          if (cross) umma_commit(q_empty);
+          ++ts;
+          c.next(p);
+          continue;
+        }
+        const int b = tp & 1;
+        mla_wait(p_full, tp & 1, dead);
+        const bool first = (firsts >> b) & 1;
+        if (first) mla_wait(o_empty, ((segs >> b) & 1) ^ 1, dead);
+        tc_fence_after_sync();  // (P's writers have fenced; the rows were fenced for S)
+#pragma unroll 1
+        for (int i = 0; i < 4; i += 2) {  // two blocks of 128 value columns in turn
+          const int slot0 = kp.i;
+          kp.next();
+          const int slot1 = kp.i;
+          kp.next();
+          const uint32_t v0 = v_lo + slot0 * (2 * kMlaBlk >> 4), v1 = v_lo + slot1 * (2 * kMlaBlk >> 4);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const uint32_t acc = (!first || k > 0) ? 1u : 0u;
+            umma_ss_lo(tmem_O + i * N, v0 + k * 128, p_lo + k * 2, hi, idesc_o, acc);
+            umma_ss_lo(tmem_O + (i + 1) * N, v1 + k * 128, p_lo + k * 2, hi, idesc_o, acc);
+          }
+          umma_commit(&k_empty[slot0]);
+          umma_commit(&k_empty[slot1]);
+        }
+        umma_commit(p_empty);
+        ++tp;
       }
     }
-    __syncthreads();  // sS / sP / this K buffer are rewritten by the next iterations
-  }
-
-  // ---- epilogue ----
-#pragma unroll
-  for (int half = 0; half < 2; ++half) {
-    const int hr = g + half * 8;
-    if (hr < nh) {
-      const int h = h0 + hr;
-      const float l = s_l[hr];
-      if (p.splits == 1) {
-        T* dst = reinterpret_cast<T*>(p.out) + item * p.out_stride + static_cast<int64_t>(h) * DV;
-        const float inv = l > 0.f ? 1.f / l : 0.f;
-#pragma unroll
-        for (int nt = 0; nt < 8; ++nt) {
-          const int d = warp * 64 + nt * 8 + 2 * tq;
-          *reinterpret_cast<uint32_t*>(dst + d) = pack2<T>(o_acc[nt][half * 2] * inv, o_acc[nt][half * 2 + 1] * inv);
+  } else if (warp >= 4) {
+    // ===================== loaders =====================
+    const int lt = tid - 128;  // 0..63: also the row of a tile this thread looks up
+    const T* pool = reinterpret_cast<const T*>(p.kv_pool);
+    if (lt == 0) {
+      tma_prefetch_desc(&tmKV);
+      tma_prefetch_desc(&tmR);
+    }
+    int t = 0, gather_age = 4;  // gather_age: tiles since one was gathered
+    auto lookup = [&](const MlaCursor<kExtend>& cc, int& base) {
+      const int32_t* page = p.req_to_token + p.req_pool_indices[cc.it.r] * p.rtt_stride;
+      const int pos = cc.tile * kMlaTile;
+      base = pos + kMlaTile <= cc.it.load_end ? __ldg(page + pos) : -1;  // a full tile: candidate TMA row
+      return pos + lt < cc.it.load_end ? __ldg(page + pos + lt) : -1;
+    };
+    MlaSlot<S::kPairs> ks;
+    MlaSlot<S::kRopes> rs;
+    int base = -1, slot = -1;
+    if (c.valid) slot = lookup(c, base);
+    bool first = true;
+    while (c.valid) {
+      const MlaItem it = c.it;
+      const int seg = c.seg;
+      const bool load_q = first;
+      first = c.ends(p);
+      c.next(p);
+      int nbase = -1, nslot = -1;
+      if (c.valid) nslot = lookup(c, nbase);  // the next tile's page-table entries, off the critical path
+      const bool contig = mla_loader_and(base >= 0 && slot == base + lt);
+      if (lt == 0) s_gath[t & 3] = !contig;  // published by this thread's extra arrival below
+      gather_age = contig ? gather_age + 1 : 0;
+      if (!contig) {
+        s_slot[lt] = slot;  // (both warps have passed the barrier above: the previous tile's rows have been read)
+        mla_loader_and(true);
+      }
+      uint64_t* full = &t_full[t & 3];
+      if (contig) {
+        if (lt == 0) {
+          if (gather_age < 4) fence_proxy_async_smem();  // the slots may last have been written by the gather path
+          mbar_expect_tx(full, 9 * kMlaBlk);
+#pragma unroll 1
+          for (int st = 0; st < 4; ++st) {
+            mla_wait(&k_empty[ks.i], ks.round ^ 1, dead);
+            tma_load_3d(sK + ks.i * 2 * kMlaBlk, &tmKV, full, 0, base, 2 * st, kEvictNormal);
+            ks.next();
+          }
+          mla_wait(&r_empty[rs.i], rs.round ^ 1, dead);
+          tma_load_2d(sR + rs.i * kMlaBlk, &tmR, full, kMlaDV, base, kEvictNormal);
+          rs.next();
+          mbar_arrive_n(full, 64);
+        } else {
+          for (int st = 0; st < 4; ++st) ks.next();
+          rs.next();
         }
       } else {
-        const int64_t idx = (static_cast<int64_t>(item) * p.H + h) * p.splits + split;
-        float* dst = p.o_part + idx * DV;
-#pragma unroll
-        for (int nt = 0; nt < 8; ++nt) {
-          const int d = warp * 64 + nt * 8 + 2 * tq;
-          dst[d] = o_acc[nt][half * 2];
-          dst[d + 1] = o_acc[nt][half * 2 + 1];
+#pragma unroll 1
+        for (int st = 0; st < 5; ++st) {
+          uint8_t* dst = st < 4 ? sK + ks.i * 2 * kMlaBlk : sR + rs.i * kMlaBlk;
+          mla_wait(st < 4 ? &k_empty[ks.i] : &r_empty[rs.i], (st < 4 ? ks.round : rs.round) ^ 1, dead);
+          const int shift = st < 4 ? 4 : 3;  // log2 of the 16-byte chunks of a row in a pair / in the rope block
+#pragma unroll 4
+          for (int i = lt; i < kMlaTile << shift; i += 64) {
+            const int row = i >> shift, ch = i - (row << shift);
+            const int s = s_slot[row];
+            cp_async16(smem_u32(dst + (ch >> 3) * kMlaBlk + mla_off(row, ch & 7)),
+                       pool + static_cast<int64_t>(s < 0 ? 0 : s) * kMlaDL + st * 128 + ch * 8, s >= 0);
+          }
+          if (st < 4) ks.next(); else rs.next();
         }
-        if (warp == 0 && tq == 0) { p.ml_part[idx * 2] = s_m[hr]; p.ml_part[idx * 2 + 1] = l; }
+        cp_async_mbar_arrive_noinc(full);
+        if (lt == 0) mbar_arrive(full);
+      }
+      if (load_q) {
+        // the item's N query rows (token, head), zero where there is none; the tile above is already on its way
+        mla_wait(q_empty, (seg & 1) ^ 1, dead);
+        const T* qb = reinterpret_cast<const T*>(p.q);
+        const int h0 = it.hg * kMlaHeads, nh = min(kMlaHeads, p.H - h0);
+#pragma unroll 4
+        for (int i = lt; i < N * 72; i += 64) {
+          const int col = i / 72, ch = i - col * 72;
+          const int tok = col >> 4, h = col & 15;
+          const bool ok = tok < it.ntok && h < nh;
+          cp_async16(smem_u32(sQ + (ch >> 3) * (N * 128) + mla_off(col, ch & 7)),
+                     qb + (ok ? (it.row0 + tok) * p.q_stride + static_cast<int64_t>(h0 + h) * kMlaDL + ch * 8 : 0), ok);
+        }
+        cp_async_mbar_arrive_noinc(q_full);
+      }
+      ++t;
+      base = nbase;
+      slot = nslot;
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+  } else {
+    // ===================== softmax / correction / epilogue =====================
+    const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
+    constexpr int C = N / 4;  // columns of this thread: 8 (i >> 1) + 2 (lane & 3) + (i & 1)
+    const int col0 = 2 * (lane & 3);
+    if (tid == 0 && !p.snap) {
+      // what the merge kernel needs of an item that began in an earlier CTA and ends here
+      int* info = p.info + cta * 8;
+      const bool tail = t_count > 0 && c.tile > 0 && c.it.ntiles - c.tile <= t_count;
+      info[0] = tail;
+      if (tail) {
+        info[1] = (t_begin - c.tile) / per;  // CTA of the item's first tile
+        info[2] = c.it.row0;
+        info[3] = c.it.ntok;
+        info[4] = c.it.hg * kMlaHeads;
       }
     }
+    int t = 0;
+    while (c.valid) {
+      const MlaItem it = c.it;
+      const int tile0 = c.tile;
+      int tile_last = tile0;
+      float m_ref[C], l_thr[C];
+#pragma unroll
+      for (int i = 0; i < C; ++i) { m_ref[i] = -INFINITY; l_thr[i] = 0.f; }
+      bool end = false;
+      while (!end) {
+        end = c.ends(p);
+        tile_last = c.tile;
+        const int kv0 = c.tile * kMlaTile;
+        const bool first = c.tile == tile0;
+        c.next(p);
+        const int sb = t & 1;
+        mla_wait(&s_full[sb], (t >> 1) & 1, dead);
+        tc_fence_after_sync();
+        uint32_t r[N / 2], r2[N / 2];
+        mla_ld_frag(tmem_S + lane_base + sb * 2 * N, r);
+        mla_ld_frag(tmem_S + lane_base + sb * 2 * N + N, r2);
+        tmem_ld_wait();
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&s_empty[sb]);
+        float s[N / 2];
+        const int pos = kv0 + warp * 16 + (lane >> 2);
+        const bool all_seen = kv0 + kMlaTile - 1 <= it.p0;  // every column sees the whole tile
+#pragma unroll
+        for (int i = 0; i < N / 2; ++i) {
+          const float v = (__uint_as_float(r[i]) + __uint_as_float(r2[i])) * p.scale_log2;
+          s[i] = all_seen || pos + 8 * ((i >> 1) & 1) <= it.p0 + (i >> 3) ? v : -INFINITY;  // i >> 3: the column's token
+        }
+        bool exceed = false;
+#pragma unroll
+        for (int i = 0; i < N / 2; ++i) exceed |= s[i] > m_ref[(i >> 2) * 2 + (i & 1)] + kMlaRescale;
+        if (mla_bar_or(exceed)) {
+          // first tile of an item, rarely later: true tile max per column, raise m_ref, rescale O^T
+#pragma unroll
+          for (int i = 0; i < C; ++i) {
+            float m = fmaxf(s[(i >> 1) * 4 + (i & 1)], s[(i >> 1) * 4 + 2 + (i & 1)]);
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 4));
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 16));
+            if (lane < 4) red[warp * N + (i >> 1) * 8 + col0 + (i & 1)] = m;
+          }
+          mla_bar();
+#pragma unroll
+          for (int i = 0; i < C; ++i) {
+            const int col = (i >> 1) * 8 + col0 + (i & 1);
+            const float mt = fmaxf(fmaxf(red[col], red[N + col]), fmaxf(red[2 * N + col], red[3 * N + col]));
+            const float m_new = fmaxf(m_ref[i], mt);
+            // (a column that has seen no key yet has nothing to scale; -inf - -inf stays out)
+            const float alpha = m_ref[i] == -INFINITY ? 0.f : fast_exp2(m_ref[i] - m_new);
+            l_thr[i] *= alpha;
+            m_ref[i] = m_new;
+            if (tid < 4) s_col[col] = alpha;
+          }
+          mla_bar();
+          if (!first) {
+            mla_wait(p_empty, (t & 1) ^ 1, dead);  // PV of the previous tile has finished: O^T is stable
+            tc_fence_after_sync();
+#pragma unroll 1
+            for (int cc = 0; cc < 4 * N; cc += 16) {
+              uint32_t o[16];
+              tmem_ld_32x32b_x16(tmem_O + lane_base + cc, o);
+              tmem_ld_wait();
+#pragma unroll
+              for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * s_col[(cc & (N - 1)) + e]);
+              tmem_st_32x32b_x16(tmem_O + lane_base + cc, o);
+            }
+            tmem_st_wait();
+            tc_fence_before_sync();
+          }
+          mla_bar();  // red / s_col may be written again
+        }
+        // P^T -> shared memory (B operand, K-major: row = column of the item, 64 kv); sums of what is multiplied
+        uint32_t pk[N / 4];
+#pragma unroll
+        for (int g = 0; g < N / 8; ++g)
+#pragma unroll
+          for (int x = 0; x < 2; ++x) {
+            const float m0 = m_ref[2 * g] == -INFINITY ? 0.f : m_ref[2 * g];
+            const float m1 = m_ref[2 * g + 1] == -INFINITY ? 0.f : m_ref[2 * g + 1];
+            pk[2 * g + x] = pack2<T>(fast_exp2(s[4 * g + 2 * x] - m0), fast_exp2(s[4 * g + 2 * x + 1] - m1));
+            const float2 v = unpack2<T>(pk[2 * g + x]);
+            l_thr[2 * g] += v.x;
+            l_thr[2 * g + 1] += v.y;
+          }
+        mla_wait(p_empty, (t & 1) ^ 1, dead);
+#pragma unroll
+        for (int g = 0; g < N / 8; g += 2) {
+          // matrices: (columns 8 g.., kv 0-7), (8 g.., kv 8-15), (8 (g + 1).., kv 0-7), (8 (g + 1).., kv 8-15)
+          const int row = 8 * (g + (lane >> 4)) + (lane & 7);
+          mla_stsm_x4_t(smem_u32(sP + mla_off(row, warp * 2 + ((lane >> 3) & 1))), pk[2 * g], pk[2 * g + 1], pk[2 * g + 2],
+                        pk[2 * g + 3]);
+        }
+        fence_proxy_async_smem();
+        mbar_arrive(p_full);
+        ++t;
+      }
+      // ---- epilogue: column sums over the kv rows of all tiles, then O^T / sum (or the partial as it is) ----
+      const bool whole = tile0 == 0 && tile_last + 1 == it.ntiles;
+      const int h0 = it.hg * kMlaHeads, nh = min(kMlaHeads, p.H - h0), nhm = min(kMlaHeads, p.H);
+      const int64_t part0 = static_cast<int64_t>(2 * cta + (tile0 > 0 ? 0 : 1)) * p.cols;
+#pragma unroll
+      for (int i = 0; i < C; ++i) {
+        float l = l_thr[i];
+        l += __shfl_xor_sync(0xffffffffu, l, 4);
+        l += __shfl_xor_sync(0xffffffffu, l, 8);
+        l += __shfl_xor_sync(0xffffffffu, l, 16);
+        if (lane < 4) red[warp * N + (i >> 1) * 8 + col0 + (i & 1)] = l;
+      }
+      mla_bar();
+      if (tid < 4) {
+#pragma unroll
+        for (int i = 0; i < C; ++i) {
+          const int col = (i >> 1) * 8 + col0 + (i & 1);
+          const float l = (red[col] + red[N + col]) + (red[2 * N + col] + red[3 * N + col]);
+          s_col[col] = l > 0.f ? 1.f / l : 0.f;
+          const int tok = col >> 4, h = col & 15;
+          if (!whole && tok < it.ntok && h < nh) {
+            float* ml = p.ml_part + (part0 + tok * nhm + h) * 2;
+            ml[0] = m_ref[i];
+            ml[1] = l;
+          }
+        }
+      }
+      mla_bar();
+      mla_wait(p_empty, (t - 1) & 1, dead);  // the last PV of the item has finished
+      tc_fence_after_sync();
+      T* out = reinterpret_cast<T*>(p.out) + it.row0 * p.out_stride + static_cast<int64_t>(h0) * kMlaDV + warp * 32;
+#pragma unroll 1
+      for (int blk = 0; blk < 4; ++blk) {
+#pragma unroll 1
+        for (int cc = 0; cc < N; cc += 16) {
+          uint32_t o[16];
+          tmem_ld_32x32b_x16(tmem_O + lane_base + blk * N + cc, o);
+          tmem_ld_wait();
+          const int tok = cc >> 4;
+          if (whole) {
+            // neighbouring lanes swap halves of two columns: 4-byte stores, 64 bytes of a row per half warp
+#pragma unroll
+            for (int e = 0; e < 16; e += 2) {
+              const float v0 = __uint_as_float(o[e]) * s_col[cc + e], v1 = __uint_as_float(o[e + 1]) * s_col[cc + e + 1];
+              const float got = __shfl_xor_sync(0xffffffffu, (lane & 1) ? v0 : v1, 1);
+              const int h = e + (lane & 1);
+              const uint32_t w = (lane & 1) ? pack2<T>(got, v1) : pack2<T>(v0, got);
+              if (tok < it.ntok && h < nh)
+                *reinterpret_cast<uint32_t*>(out + tok * p.out_stride + h * kMlaDV + blk * 128 + (lane & ~1)) = w;
+            }
+          } else if (tok < it.ntok) {
+#pragma unroll
+            for (int e = 0; e < 16; ++e)
+              if (e < nh) p.o_part[(part0 + tok * nhm + e) * kMlaDV + blk * 128 + warp * 32 + lane] = __uint_as_float(o[e]);
+          }
+        }
+      }
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(o_empty);
+      mla_bar();  // red / s_col belong to the next item
+    }
   }
+
   griddep_launch_dependents();
-}
-
-template <typename T, int DV>
-__global__ void __launch_bounds__(256)
-mla_merge_kernel(T* __restrict__ out, const float* __restrict__ o_part, const float* __restrict__ ml_part, int H,
-                 int splits, int64_t out_stride) {
-  griddep_wait();
-  const int item = blockIdx.y, h = blockIdx.x;
-  const int64_t base = (static_cast<int64_t>(item) * H + h) * splits;
-  float M = -INFINITY;
-  for (int s = 0; s < splits; ++s)
-    if (ml_part[(base + s) * 2 + 1] > 0.f) M = fmaxf(M, ml_part[(base + s) * 2]);
-  for (int t = threadIdx.x; t < DV; t += 256) {
-    float num = 0.f, den = 0.f;
-    for (int s = 0; s < splits; ++s) {
-      const float m = ml_part[(base + s) * 2], l = ml_part[(base + s) * 2 + 1];
-      if (l > 0.f) {
-        const float w = exp2f(m - M);
-        num += w * o_part[(base + s) * DV + t];
-        den += w * l;
-      }
-    }
-    out[item * out_stride + static_cast<int64_t>(h) * DV + t] = from_f32<T>(den > 0.f ? num / den : 0.f);
+  tc_fence_before_sync();
+  __syncthreads();
+  if (warp == 6) tmem_dealloc(tmem_base, S::kTmem);
+  if (*dead) {  // a wait ran out: let copies in flight land before the shared memory is given back
+    for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+    if (tid == 0) atomicAdd(&g_mla_wait_expired, 1u);
   }
 }
 
-template <int DL>
-constexpr int mla_smem_bytes() {
-  return (kMlaHeads + 2 * kMlaChunk) * (DL + 8) * 2 + 8 * kMlaHeads * kMlaChunk * 4 + kMlaHeads * 40 * 2 + 48 * 4;
+// Merges the parts of the items that span several CTAs.  Block (c, 4 columns) serves the item that ends in CTA c after
+// beginning in CTA info[1] < c: that CTA left its part in slot 2 info[1] + 1, the following ones up to c in slot 2 i.
+// info: {any, first CTA, first query row, tokens, first head}.
+template <typename T>
+__global__ void __launch_bounds__(512)
+mla_merge_kernel(const MlaParams p) {
+  griddep_wait();
+  const int c = blockIdx.x, nhm = min(kMlaHeads, p.H);
+  const int* info = p.info + c * 8;
+  if (!info[0]) return;
+  const int col = blockIdx.y * 4 + (threadIdx.x >> 7), x = threadIdx.x & 127;
+  const int tok = col / nhm, h = col % nhm;
+  if (tok >= info[3] || info[4] + h >= p.H) return;
+  const int c0 = info[1];
+  auto at = [&](int i) { return static_cast<int64_t>(i == c0 ? 2 * i + 1 : 2 * i) * p.cols + col; };
+  float M = -INFINITY;
+  for (int i = c0; i <= c; ++i) M = fmaxf(M, p.ml_part[at(i) * 2]);  // (-inf where a part saw no key)
+  float4 num = make_float4(0.f, 0.f, 0.f, 0.f);
+  float den = 0.f;
+#pragma unroll 4
+  for (int i = c0; i <= c; ++i) {
+    const float2 ml = *reinterpret_cast<const float2*>(p.ml_part + at(i) * 2);
+    const float4 o = *reinterpret_cast<const float4*>(p.o_part + at(i) * kMlaDV + x * 4);
+    const float w = ml.y > 0.f ? fast_exp2(ml.x - M) : 0.f;
+    num.x = fmaf(w, o.x, num.x);
+    num.y = fmaf(w, o.y, num.y);
+    num.z = fmaf(w, o.z, num.z);
+    num.w = fmaf(w, o.w, num.w);
+    den = fmaf(w, ml.y, den);
+  }
+  const float inv = den > 0.f ? 1.f / den : 0.f;
+  T* dst = reinterpret_cast<T*>(p.out) + (static_cast<int64_t>(info[2]) + tok) * p.out_stride +
+           static_cast<int64_t>(info[4] + h) * kMlaDV + x * 4;
+  *reinterpret_cast<uint2*>(dst) = make_uint2(pack2<T>(num.x * inv, num.y * inv), pack2<T>(num.z * inv, num.w * inv));
 }
 
-static int mla_splits(int64_t items, int head_groups, int sms) {
-  const int64_t ctas = items * head_groups;
-  int s = static_cast<int>((2ll * sms + ctas - 1) / ctas);
-  if (s < 1) s = 1;
-  if (s > kMlaMaxSplits) s = kMlaMaxSplits;
-  return s;
+template <typename T, bool kExtend>
+static int mla_launch(const MlaParams& p, int grid, cudaStream_t st) {
+  CUtensorMap tm, tr;
+  // the C-ABI does not carry the pool's slot count: rows are slot ids read from req_to_token, so the maximum is declared
+  if (int rc = make_tmap_blocks_sw128(&tm, p.kv_pool, 1ull << 31, 9, kMlaDL, kMlaTile, 2)) return rc;
+  if (int rc = get_tmap(&tr, p.kv_pool, 1ull << 31, kMlaDL, kMlaDL, kMlaTile)) return rc;
+  auto kern = attn_mla_kernel<T, kExtend>;
+  static bool configured = false;
+  if (!configured) {
+    SPD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MlaShape<kExtend>::kSmem));
+    configured = true;
+  }
+  SPD_CUDA(launch(kern, dim3(grid), dim3(kMlaThreads), MlaShape<kExtend>::kSmem, st, pdl_enabled(), tm, tr, p));
+  if (!p.snap) SPD_CUDA(launch(mla_merge_kernel<T>, dim3(grid, (p.cols + 3) / 4), dim3(512), 0, st, pdl_enabled(), p));
+  return 0;
 }
 
 }  // namespace spd
@@ -304,9 +837,10 @@ using namespace spd;
 extern "C" {
 
 int64_t spd_attn_mla_workspace_bytes(int num_heads, int kv_lora_rank) {
-  // splits are only used while items x head groups < 2 x SMs: at most 2 x SMs items
+  // two partials per CTA of up to 4 tokens x min(heads, 16) rows, and 32 bytes per CTA; 8 rows per head of two per SM
+  // cover that for any number of heads
   const int64_t items = 2ll * device_sm_count_cached();
-  return items * num_heads * kMlaMaxSplits * (kv_lora_rank + 2) * 4 + 256;
+  return items * num_heads * 8 * (kv_lora_rank + 2) * 4 + 256;
 }
 
 int spd_attn_mla(void* out, const void* q, const void* kv_pool, const int32_t* req_to_token,
@@ -319,7 +853,7 @@ int spd_attn_mla(void* out, const void* q, const void* kv_pool, const int32_t* r
   const bool extend = seq_lens == nullptr;
   SPD_REQUIRE(!extend || (prefix_lens && extend_start_loc), SPD_E_BADARG,
               "spd_attn_mla: give seq_lens (decode) or prefix_lens + extend_start_loc (extend)");
-  SPD_REQUIRE(kv_lora_rank == 512 && rope_dim == 64, SPD_E_SHAPE,
+  SPD_REQUIRE(kv_lora_rank == kMlaDV && rope_dim == kMlaDL - kMlaDV, SPD_E_SHAPE,
               "spd_attn_mla: built for kv_lora_rank 512 + rope 64 (got %d + %d)", kv_lora_rank, rope_dim);
   SPD_REQUIRE(num_heads > 0 && batch >= 0 && total_tokens >= 0, SPD_E_BADARG, "spd_attn_mla: bad sizes");
   SPD_REQUIRE(q_stride % 8 == 0 && out_stride % 8 == 0 && aligned16(out) && aligned16(q) && aligned16(kv_pool),
@@ -327,9 +861,9 @@ int spd_attn_mla(void* out, const void* q, const void* kv_pool, const int32_t* r
   const int64_t items = extend ? total_tokens : batch;
   if (items == 0) return 0;
   SPD_REQUIRE(items < 65536, SPD_E_SHAPE, "spd_attn_mla: more than 65535 query tokens in one call");
-  constexpr int DL = 576, DV = 512;
-  const int sms = sm_budget > 0 ? sm_budget : device_sm_count_cached();
-  const int hgs = (num_heads + kMlaHeads - 1) / kMlaHeads;
+  const int device_sms = device_sm_count_cached();
+  const int sms = sm_budget > 0 ? sm_budget : device_sms;
+  const int grid = sms < device_sms ? sms : device_sms;
   MlaParams p{};
   p.out = out;
   p.q = q;
@@ -340,45 +874,35 @@ int spd_attn_mla(void* out, const void* q, const void* kv_pool, const int32_t* r
   p.prefix_lens = prefix_lens;
   p.extend_start_loc = extend_start_loc;
   p.batch = static_cast<int>(batch);
+  p.total = static_cast<int>(total_tokens);
   p.H = num_heads;
+  p.hgs = (num_heads + kMlaHeads - 1) / kMlaHeads;
   p.q_stride = q_stride;
   p.out_stride = out_stride;
   p.rtt_stride = req_to_token_stride;
   p.scale_log2 = sm_scale * 1.4426950408889634f;
-  p.splits = mla_splits(items, hgs, sms);
-  if (p.splits > 1) {
-    const int64_t need = items * num_heads * p.splits * (DV + 2) * 4;
-    SPD_REQUIRE(workspace && workspace_bytes >= need, SPD_E_WORKSPACE,
-                "spd_attn_mla: workspace too small (%lld < %lld)", (long long)workspace_bytes, (long long)need);
+  p.min_tiles = 2;
+  const int tq = extend ? MlaShape<true>::TQ : MlaShape<false>::TQ;
+  p.cols = tq * (num_heads < kMlaHeads ? num_heads : kMlaHeads);
+  const int64_t rows = 2ll * grid * p.cols, need = rows * (kMlaDV + 2) * 4 + grid * 32ll;
+  const int64_t groups = (items + tq - 1) / tq * p.hgs;
+  // what a call has to bring: room for the partials of a fixed split by query tokens, or nothing where those alone fill
+  // the SMs twice; a workspace of just that size still serves calls cut at item starts
+  const int64_t ctas = items * p.hgs;
+  int64_t splits = (2ll * sms + ctas - 1) / ctas;
+  splits = splits < 8 ? splits : 8;
+  const int64_t least = splits > 1 ? items * num_heads * splits * (kMlaDV + 2) * 4 : 0;
+  SPD_REQUIRE(least == 0 || (workspace && workspace_bytes >= least), SPD_E_WORKSPACE,
+              "spd_attn_mla: workspace too small (%lld < %lld)", (long long)workspace_bytes, (long long)least);
+  p.snap = workspace == nullptr || workspace_bytes < need || groups >= 16ll * grid;
+  if (!p.snap) {
     p.o_part = reinterpret_cast<float*>(workspace);
-    p.ml_part = p.o_part + items * num_heads * p.splits * DV;
+    p.ml_part = p.o_part + rows * kMlaDV;
+    p.info = reinterpret_cast<int*>(p.ml_part + rows * 2);
   }
-  const dim3 grid(p.splits, hgs, static_cast<unsigned>(items));
-  constexpr int smem = mla_smem_bytes<DL>();
   cudaStream_t st = as_stream(stream);
   SPD_DISPATCH_DTYPE(dtype, {
-    if (extend) {
-      auto kern = attn_mla_kernel<T, DL, DV, true>;
-      static bool configured = false;
-      if (!configured) {
-        SPD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        configured = true;
-      }
-      SPD_CUDA(launch(kern, grid, dim3(kMlaThreads), smem, st, pdl_enabled(), p));
-    } else {
-      auto kern = attn_mla_kernel<T, DL, DV, false>;
-      static bool configured = false;
-      if (!configured) {
-        SPD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        configured = true;
-      }
-      SPD_CUDA(launch(kern, grid, dim3(kMlaThreads), smem, st, pdl_enabled(), p));
-    }
-    if (p.splits > 1) {
-      SPD_CUDA(launch(mla_merge_kernel<T, DV>, dim3(num_heads, static_cast<unsigned>(items)), dim3(256), 0, st,
-                      pdl_enabled(), reinterpret_cast<T*>(out), (const float*)p.o_part, (const float*)p.ml_part,
-                      num_heads, p.splits, out_stride));
-    }
+    return extend ? mla_launch<T, true>(p, grid, st) : mla_launch<T, false>(p, grid, st);
   });
   return 0;
 }

@@ -76,6 +76,28 @@ int make_tmap_2d_sw128(CUtensorMap* out, const void* base, uint64_t rows, uint64
   return 0;
 }
 
+int make_tmap_blocks_sw128(CUtensorMap* out, const void* base, uint64_t rows, uint64_t blocks, uint64_t row_stride_elems,
+                           uint32_t box_rows, uint32_t box_blocks) {
+  using Fn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                          const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
+                          CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
+                          CUtensorMapFloatOOBfill);
+  static Fn fn = driver_fn<Fn>("cuTensorMapEncodeTiled");
+  if (!fn) return set_error(SPD_E_DRIVER, "cuTensorMapEncodeTiled not available from the driver");
+  cuuint64_t gdim[3] = {64, rows, blocks};
+  cuuint64_t gstride[2] = {row_stride_elems * 2, 128};
+  cuuint32_t box[3] = {64, box_rows, box_blocks};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), gdim, gstride,
+                  box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS)
+    return set_error(SPD_E_DRIVER, "cuTensorMapEncodeTiled failed (%d): base=%p rows=%llu blocks=%llu stride=%llu box=%ux%u",
+                     (int)r, base, (unsigned long long)rows, (unsigned long long)blocks,
+                     (unsigned long long)row_stride_elems, box_rows, box_blocks);
+  return 0;
+}
+
 }  // namespace spd
 
 using namespace spd;

@@ -11,6 +11,11 @@ namespace spd {
 int make_tmap_2d_sw128(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols,
                        uint64_t row_stride_elems, uint32_t box_rows, uint32_t box_cols);
 
+// The same rows as [blocks][rows][64 columns]: one box of box_rows x box_blocks lands as box_blocks consecutive
+// swizzle blocks of [box_rows x 128 bytes], with one copy instruction instead of one per block.
+int make_tmap_blocks_sw128(CUtensorMap* out, const void* base, uint64_t rows, uint64_t blocks, uint64_t row_stride_elems,
+                           uint32_t box_rows, uint32_t box_blocks);
+
 // Cached variant (implemented in gemm.cu): descriptors are pure functions of (pointer, shape,
 // box), so steady-state launches do no driver work.  box_cols is fixed at 64 (one swizzle atom).
 int get_tmap(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t stride,

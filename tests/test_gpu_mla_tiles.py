@@ -1,0 +1,115 @@
+"""attn_mla on its tile and split edges: consecutive slots (one copy per pair of column blocks) beside scattered ones and
+both in one request, lengths around the 64-key tile, requests cut over several SMs or sharing one, head counts that fill
+no group of 16, a workspace of the least size a call has to bring, a batch large enough to be cut at request starts."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+R, DR = 512, 64
+
+
+def _pool(lens, dtype, layout, g):
+    """Latent rows and a page table: "runs" of 128 consecutive slots (the pool's allocator), "scattered", or runs with a
+    stray slot in every third tile."""
+    room = sum(-(-n // 128) * 128 for n in lens) + 200
+    pool = (torch.randn(room, R + DR, generator=g) * 0.5).to(dtype)
+    rtt = torch.zeros(len(lens), max(max(lens), 1) + 8, dtype=torch.int32)
+    if layout == "scattered":
+        perm, at = torch.randperm(room - 1, generator=g) + 1, 0
+        for b, n in enumerate(lens):
+            rtt[b, :n] = perm[at:at + n].int()
+            at += n
+        return pool, rtt
+    order = torch.randperm(sum(-(-n // 128) for n in lens), generator=g).tolist()
+    for b, n in enumerate(lens):
+        for i in range(0, n, 128):
+            k = min(128, n - i)
+            rtt[b, i:i + k] = torch.arange(k, dtype=torch.int32) + 1 + 128 * order.pop()
+        if layout == "stray":
+            for i in range(70, n, 192):
+                rtt[b, i] = room - 1 - (i % 50)
+    return pool, rtt
+
+
+def _reference(q, pool, rtt, pre, ext, scale):
+    out, at = [], 0
+    for b, (p, e) in enumerate(zip(pre, ext)):
+        rows = pool[rtt[b, :p + e].long()].double()
+        sc = torch.einsum("qhl,kl->hqk", q[at:at + e].double(), rows) * scale
+        sc = sc + torch.full((e, p + e), float("-inf"), dtype=torch.float64).triu(p + 1)
+        out.append(torch.einsum("hqk,kr->qhr", sc.softmax(-1), rows[:, :R]))
+        at += e
+    return torch.cat(out)
+
+
+# probabilities and outputs are rounded to 16 bits (2^-9 / 2^-12 relative); values are N(0, 0.25) averaged over the keys, so
+# the largest of them is that of a request of one key, |v| <= 2.5: half an ulp of the output plus the same for P
+TOL = {torch.float16: 2e-3, torch.bfloat16: 1.6e-2}
+
+
+def _run(pre, ext, H, dtype, layout, decode, ws_bytes=None, sms=0):
+    from semi_pd_b200 import ops
+    g = torch.Generator().manual_seed(sum(ext) + 7 * sum(pre) + H)
+    lens = [p + e for p, e in zip(pre, ext)]
+    pool, rtt = _pool(lens, dtype, layout, g)
+    q = (torch.randn(sum(ext), H, R + DR, generator=g) * 0.5).to(dtype)
+    scale = 192 ** -0.5
+    want = _reference(q, pool, rtt, pre, ext, scale)
+    need = ops.lib.spd_attn_mla_workspace_bytes(H, R) if ws_bytes is None else ws_bytes
+    ws = torch.full((need,), 255, dtype=torch.uint8, device=DEV)  # (not zeroed: NaN patterns)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
+    if decode:
+        more = dict(seq_lens=torch.tensor(lens, dtype=torch.int64, device=DEV))
+    else:
+        starts = [sum(ext[:i]) for i in range(len(ext))]
+        more = dict(prefix_lens=i32(pre), extend_start_loc=i32(starts))
+    ops.set_sm_budget(sms)
+    try:
+        out = ops.attn_mla(q.to(DEV).view(q.shape[0], -1), pool.to(DEV), rtt.to(DEV), torch.arange(len(ext), device=DEV), H,
+                           R, DR, scale, ws, **more)
+    finally:
+        ops.set_sm_budget(0)
+    err = (out.cpu().double().view(want.shape) - want).abs().max().item()
+    assert err < TOL[dtype], err
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("layout", ["runs", "scattered", "stray"])
+@pytest.mark.parametrize("lens", [[63], [64], [65], [128, 129, 1, 191, 640], [5000], [2000] * 3 + [3] * 40])
+def test_decode_tiles(dtype, layout, lens):
+    _run([n - 1 for n in lens], [1] * len(lens), 16, dtype, layout, True)
+
+
+@pytest.mark.parametrize("H", [1, 5, 20, 48])
+@pytest.mark.parametrize("decode", [True, False])
+def test_head_counts(H, decode):
+    ext = [1, 1, 1] if decode else [9, 1, 70]
+    _run([300, 64, 700], ext, H, torch.bfloat16, "runs", decode)
+
+
+@pytest.mark.parametrize("layout", ["runs", "scattered", "stray"])
+@pytest.mark.parametrize("pre,ext", [([0], [3]), ([0], [64]), ([61], [7]), ([0, 130, 5], [1, 65, 4]), ([2000], [2]),
+                                     ([0, 640], [700, 259])])
+def test_extend_tiles(layout, pre, ext):
+    _run(pre, ext, 16, torch.bfloat16, layout, False)
+
+
+def test_empty_requests_in_an_extend_batch():
+    _run([0, 40, 0, 10, 3], [0, 9, 0, 70, 0], 16, torch.float16, "runs", False)
+
+
+def test_small_partition_and_request_starts():
+    # 40 requests on 2 SMs: 20 per SM, cut at request starts; on 8 SMs the ranges cut requests
+    for sms in (2, 8):
+        _run([50 + 9 * i for i in range(40)], [1] * 40, 16, torch.bfloat16, "runs", True, sms=sms)
+
+
+@pytest.mark.parametrize("decode", [True, False])
+def test_least_workspace(decode):
+    # items x heads x splits x 514 floats is what a call has to bring; nothing is split over SMs then
+    H, ext = 16, [1, 1] if decode else [5, 2]
+    least = sum(ext) * H * 8 * 514 * 4
+    _run([200, 100], ext, H, torch.bfloat16, "runs", decode, ws_bytes=least)
+    with pytest.raises(RuntimeError):
+        _run([200, 100], ext, H, torch.bfloat16, "runs", decode, ws_bytes=least - 4)
