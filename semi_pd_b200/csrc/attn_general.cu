@@ -569,12 +569,25 @@ pool_key_blocks_kernel(T* __restrict__ k_pool, T* __restrict__ v_pool, const int
   }
 }
 
+// Whether a portion of at most `ext` new tokens takes the tcgen05 prefill kernel (tiles of 128 queries x 128 keys) rather
+// than the mma.sync one (64 x 64): a query tile has to meet several whole key tiles.  16 / 4 heads, 4 requests of 200
+// tokens after 1500, window 1024: 52 us (mma.sync) / 28 us; of 500, window 128: 25 / 31 us, of 1500, window 128: 66 / 55 us;
+// one of 40 tokens, no prefix: 6.0 / 7.0 us.  The prefixes are on the device, so they do not enter the rule.
+inline bool window_tc_wins(int64_t ext, int window) { return window <= 0 || window >= 512 ? ext >= 192 : ext >= 1024; }
+
 int attn_general_mma_try(void* out, const void* q, const void* k_pool, const void* v_pool, const int32_t* req_to_token,
                          const int64_t* req_pool_indices, const int32_t* prefix_lens, const int32_t* extend_lens,
                          const int32_t* extend_start_loc, int64_t batch, int64_t max_extend_len, int H, int G, int dk,
                          int dv, int64_t q_stride, int64_t out_stride, int64_t r2t_stride, float sm_scale, int window,
                          const float* sinks, const float* slopes, float qtemp_coef, int qtemp_every, float softcap,
                          int Gv, int64_t v_slot, KeyBlocks kb, DistanceBias db, int dtype, cudaStream_t stream);
+
+int attn_prefill_window_try(void* out, const void* q, const void* k_pool, const void* v_pool, const int32_t* req_to_token,
+                            const int64_t* req_pool_indices, const int32_t* prefix_lens, const int32_t* extend_lens,
+                            const int32_t* extend_start_loc, int64_t batch, int64_t total_tokens, int64_t max_extend_len,
+                            int H, int G, int64_t q_stride, int64_t out_stride, int64_t r2t_stride, float sm_scale,
+                            int window, const float* sinks, float qtemp_coef, int qtemp_every, int dtype,
+                            cudaStream_t stream);
 
 int attn_general_mma_decode_try(void* out, const void* q, const void* k_pool, const void* v_pool,
                                 const int32_t* req_to_token, const int64_t* req_pool_indices, const int64_t* seq_lens,
@@ -736,6 +749,16 @@ int spd_attn_general_keys(void* out, const void* q, const void* k_pool, const vo
                       Gv, v_slot, kb, db));
     });
     return 0;
+  }
+  // 16-bit prefill at head size 128 on tcgen05, for the options that kernel has
+  if (window_tc_wins(max_extend_len, window) && dtype != SPD_F32 && head_dim == 128 && v_dim == 128 && slopes == nullptr &&
+      db.table == nullptr && !(softcap > 0.f) && kb.size == 0 && kb.keep == 0 && Gv == num_kv_heads &&
+      v_slot == (int64_t)num_kv_heads * 128) {
+    const int rc = attn_prefill_window_try(out, q, k_pool, v_pool, req_to_token, req_pool_indices, prefix_lens, extend_lens,
+                                           extend_start_loc, batch, total_tokens, max_extend_len, num_q_heads, num_kv_heads,
+                                           q_stride, out_stride, req_to_token_stride, sm_scale, window, sinks, qtemp_coef,
+                                           qtemp_every, dtype, as_stream(stream));
+    if (rc != 1) return rc;
   }
   if (max_extend_len > 0) {  // 16-bit prefill on the tensor cores where the head sizes are instantiated
     const int rc = attn_general_mma_try(out, q, k_pool, v_pool, req_to_token, req_pool_indices, prefix_lens, extend_lens,

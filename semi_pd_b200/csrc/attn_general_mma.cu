@@ -5,8 +5,8 @@
 // on warp-level mma.sync.m16n8k16 (fp32 accumulators), and the online softmax — scale, temperature,
 // bias, window mask, sink — is fp32 in the exp2 domain.  Only the keys a tile can see are visited:
 // [first row - window + 1, last row], preceded by the pooled blocks or kept first tokens it can see.  The CUDA-core kernel of attn_general.cu keeps decode, float32
-// models and head sizes outside the instantiated set.  (mma.sync, not tcgen05: the first tensor-core
-// kernel of this mechanism.)
+// models and head sizes outside the instantiated set.  Portions of some length at head size 128 without a distance bias,
+// score cap, blocks or kept tokens take the tcgen05 kernel of attn_prefill.cu (window_tc_wins in attn_general.cu).
 #include "common.cuh"
 #include "ptx.cuh"
 #include "key_blocks.cuh"

@@ -82,6 +82,11 @@ struct PrefillParams {
   // heads_x, GQA group) as multiply-high + shift: four dependent integer divisions sat on every
   // item boundary of every role
   uint32_t per_x_m, per_x_s, heads_x_m, heads_x_s, group_m, group_s;
+  // kWin only: keys a query sees up to and with itself; a logit per head in the softmax denominator (nullptr: none); query
+  // temperature 1 + coef ln(floor((pos + 1) / every) + 1) (every 0: none)
+  int window, qtemp_every;
+  const float* sinks;
+  float qtemp_coef;
   long long* trace;  // debug timeline of CTA 0 (scripts/debug_attn_prefill_timeline.py); kTrace builds only
   int trace_cap;
 };
@@ -100,7 +105,8 @@ __device__ __forceinline__ void pf_trace(const PrefillParams& p, int region, uin
 }
 
 struct PfItem {
-  int req, pre, hk, n;         // n = KV tiles of the item (max over the two query tiles)
+  int req, pre, hk, n;         // n = end of the item's KV tiles (max over the two query tiles), j0 = the first of them
+  int j0;
   int head[2], m0[2], rows[2], nt[2], q_row0[2];
   int kv_len;
 };
@@ -133,6 +139,7 @@ __device__ __forceinline__ PfRaw pf_raw(const PrefillParams& p, int idx) {
   return r;
 }
 
+template <bool kWin>
 __device__ __forceinline__ PfItem pf_item(const PrefillParams& p, int idx, const PfRaw& raw) {
   PfItem it;
   const int per_x = p.heads_x * p.batch;
@@ -165,6 +172,9 @@ __device__ __forceinline__ PfItem pf_item(const PrefillParams& p, int idx, const
     if (rows > 0) it.kv_len = max(it.kv_len, kv);
   }
   it.n = max(it.nt[0], it.nt[1]);
+  // first key that the first row sees (the later tile of an item, if any, sees no earlier one)
+  it.j0 = 0;
+  if constexpr (kWin) it.j0 = max(0, it.pre + it.m0[0] - p.window + 1) / kPfN;
   return it;
 }
 
@@ -214,9 +224,15 @@ __device__ __forceinline__ uint64_t fadd2(uint64_t a, uint64_t b) {
 }
 
 // 32 columns of one tile row: p = exp2(s*scale - m_off), packed to 16 bits into pk[0..16)
-template <typename T, bool kMask>
+// key `kv` of a masked unit is visible: kv <= limit, and with a window (span = its size - 1) limit - kv <= span
+template <bool kWin>
+__device__ __forceinline__ bool pf_visible(int kv, int limit, int span) {
+  if constexpr (kWin) return static_cast<uint32_t>(limit - kv) <= static_cast<uint32_t>(span);
+  return kv <= limit;
+}
+template <typename T, bool kMask, bool kWin>
 __device__ __forceinline__ void softmax_chunk(const uint32_t* r, int c, uint32_t* pk, uint64_t scale2,
-                                              uint64_t neg_m2, int kv0, int limit, uint64_t& ps) {
+                                              uint64_t neg_m2, int kv0, int limit, int span, uint64_t& ps) {
 #pragma unroll
   for (int i = 0; i < 32; i += 2) {
     float x0, x1;
@@ -224,8 +240,8 @@ __device__ __forceinline__ void softmax_chunk(const uint32_t* r, int c, uint32_t
     float p0 = fast_exp2(x0);
     float p1 = fast_exp2(x1);
     if constexpr (kMask) {
-      p0 = (kv0 + c + i) <= limit ? p0 : 0.f;
-      p1 = (kv0 + c + i + 1) <= limit ? p1 : 0.f;
+      p0 = pf_visible<kWin>(kv0 + c + i, limit, span) ? p0 : 0.f;
+      p1 = pf_visible<kWin>(kv0 + c + i + 1, limit, span) ? p1 : 0.f;
     }
     ps = fadd2(ps, pack_f32x2(p0, p1));
     pk[i >> 1] = pack2<T>(p0, p1);
@@ -237,9 +253,9 @@ __device__ __forceinline__ void softmax_chunk(const uint32_t* r, int c, uint32_t
 // loads are in flight while the previous 32 columns are exponentiated.  kMask is a template
 // parameter so that the unmasked units run the lean loop: FFMA + MUFU.EX2 + FADD + half an F2FP
 // per element.
-template <typename T, bool kMask, int kU>
+template <typename T, bool kMask, int kU, bool kWin>
 __device__ __forceinline__ float softmax_row_pass(uint32_t ts, uint32_t* pk, float scale_log2, float m_off,
-                                                  int kv0, int limit) {
+                                                  int kv0, int limit, int span) {
   const uint64_t scale2 = pack_f32x2(scale_log2, scale_log2);
   const uint64_t neg_m2 = pack_f32x2(-m_off, -m_off);
   uint64_t ps = pack_f32x2(0.f, 0.f);
@@ -247,14 +263,14 @@ __device__ __forceinline__ float softmax_row_pass(uint32_t ts, uint32_t* pk, flo
   tmem_ld_32x32b_x32(ts, ra);
   tmem_ld_32x32b_x32(ts + 32, rb);
   tmem_ld_wait();
-  softmax_chunk<T, kMask>(ra, 0, pk, scale2, neg_m2, kv0, limit, ps);
+  softmax_chunk<T, kMask, kWin>(ra, 0, pk, scale2, neg_m2, kv0, limit, span, ps);
   if constexpr (kU == 128) tmem_ld_32x32b_x32(ts + 64, ra);  // in flight under the next chunk
-  softmax_chunk<T, kMask>(rb, 32, pk + 16, scale2, neg_m2, kv0, limit, ps);
+  softmax_chunk<T, kMask, kWin>(rb, 32, pk + 16, scale2, neg_m2, kv0, limit, span, ps);
   if constexpr (kU == 128) {
     tmem_ld_32x32b_x32(ts + 96, rb);
     tmem_ld_wait();
-    softmax_chunk<T, kMask>(ra, 64, pk + 32, scale2, neg_m2, kv0, limit, ps);
-    softmax_chunk<T, kMask>(rb, 96, pk + 48, scale2, neg_m2, kv0, limit, ps);
+    softmax_chunk<T, kMask, kWin>(ra, 64, pk + 32, scale2, neg_m2, kv0, limit, span, ps);
+    softmax_chunk<T, kMask, kWin>(rb, 96, pk + 48, scale2, neg_m2, kv0, limit, span, ps);
   }
   float ps0, ps1;
   unpack_f32x2(ps, ps0, ps1);
@@ -262,21 +278,21 @@ __device__ __forceinline__ float softmax_row_pass(uint32_t ts, uint32_t* pk, flo
 }
 
 // max of the visible raw scores of one row of an S unit (TMEM)
-template <bool kMask>
-__device__ __forceinline__ void rowmax_chunk(const uint32_t* r, int c, int kv0, int limit, float& m0, float& m1) {
+template <bool kMask, bool kWin>
+__device__ __forceinline__ void rowmax_chunk(const uint32_t* r, int c, int kv0, int limit, int span, float& m0, float& m1) {
 #pragma unroll
   for (int i = 0; i < 32; i += 2) {
     float a = __uint_as_float(r[i]), b = __uint_as_float(r[i + 1]);
     if constexpr (kMask) {
-      a = (kv0 + c + i) <= limit ? a : -INFINITY;
-      b = (kv0 + c + i + 1) <= limit ? b : -INFINITY;
+      a = pf_visible<kWin>(kv0 + c + i, limit, span) ? a : -INFINITY;
+      b = pf_visible<kWin>(kv0 + c + i + 1, limit, span) ? b : -INFINITY;
     }
     m0 = fmaxf(m0, a);
     m1 = fmaxf(m1, b);
   }
 }
-template <bool kMask, int kU>
-__device__ __forceinline__ float softmax_row_max(uint32_t ts, int kv0, int limit) {
+template <bool kMask, int kU, bool kWin>
+__device__ __forceinline__ float softmax_row_max(uint32_t ts, int kv0, int limit, int span) {
   float m0 = -INFINITY, m1 = -INFINITY;
 #pragma unroll
   for (int c = 0; c < kU; c += 64) {
@@ -284,8 +300,8 @@ __device__ __forceinline__ float softmax_row_max(uint32_t ts, int kv0, int limit
     tmem_ld_32x32b_x32(ts + c, ra);
     tmem_ld_32x32b_x32(ts + c + 32, rb);
     tmem_ld_wait();
-    rowmax_chunk<kMask>(ra, c, kv0, limit, m0, m1);
-    rowmax_chunk<kMask>(rb, c + 32, kv0, limit, m0, m1);
+    rowmax_chunk<kMask, kWin>(ra, c, kv0, limit, span, m0, m1);
+    rowmax_chunk<kMask, kWin>(rb, c + 32, kv0, limit, span, m0, m1);
   }
   return fmaxf(m0, m1);
 }
@@ -294,7 +310,11 @@ __device__ __forceinline__ float softmax_row_max(uint32_t ts, int kv0, int limit
 // unit per K/V tile — S = Q K^T goes out as ONE N = 128 group (8 instead of 16 SS-form MMAs per
 // tile, the form whose fixed cost per instruction dominates at N = 64) and the two warpgroups
 // alternate on the tensor core tile by tile.
-template <typename T, int kU, bool kTrace>
+// kWin: a sliding window (KV tiles before the item's first visible key are skipped), sinks and a query temperature — the
+// general attention of the hybrid families at head size 128 (see spd::attn_prefill_window_try).
+// 4 requests of 2048 new tokens, 16 / 4 heads, window 1024: 320 us on warp-level MMAs with 64 x 64 tiles, 114 us here
+// (60 GFLOP visible; a query tile of 128 meets nine key tiles, two of them masked).
+template <typename T, int kU, bool kTrace, bool kWin>
 __global__ void __launch_bounds__(kPfThreads, 1)
 attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
@@ -362,7 +382,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       int idx = pf_rank(0, cta, ncta);
       PfRaw raw = pf_raw(p, idx);
       for (int k = 0; idx < p.total_items; ++k) {
-        const PfItem it = pf_item(p, idx, raw);
+        const PfItem it = pf_item<kWin>(p, idx, raw);
         idx = pf_rank(k + 1, cta, ncta);
         raw = pf_raw(p, idx);
         if (it.n == 0) continue;
@@ -391,7 +411,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       int idx = pf_rank(0, cta, ncta);
       PfRaw raw = pf_raw(p, idx);
       for (int kk = 0; idx < p.total_items; ++kk) {
-        const PfItem it = pf_item(p, idx, raw);
+        const PfItem it = pf_item<kWin>(p, idx, raw);
         idx = pf_rank(kk + 1, cta, ncta);
         raw = pf_raw(p, idx);
         if (it.n == 0) continue;
@@ -411,7 +431,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         // alternating TS- and SS-form MMAs costs more than either stream alone (8 x 42 + 8 x 75
         // by the probe), the alternation benefit exists for SS next to SS only.)
         auto issue_s = [&](int w, int j, int h) {
-          const uint32_t pos = 2 * (t_base + j);
+          const uint32_t pos = 2 * (t_base + j - it.j0);
           mbar_wait(&kv_full[pos % kPfSlots], (pos / kPfSlots) & 1);
           tc_fence_after_sync();
           const uint32_t q_addr = smem_u32(sQ + w * kTileBytes);
@@ -427,7 +447,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         // after every unit of S(j) of both warpgroups has been issued: release K_j, and Q after
         // the item's last S
         auto s_tile_issued = [&](int j) {
-          umma_commit(&kv_empty[(2 * (t_base + j)) % kPfSlots]);
+          umma_commit(&kv_empty[(2 * (t_base + j - it.j0)) % kPfSlots]);
           if (j == it.n - 1) umma_commit(q_empty);
         };
         // the epilogue of the previous item reads O, not S — and its last PVs (reading P in the S
@@ -436,10 +456,10 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         for (int h = 0; h < kNU; ++h)
 #pragma unroll
           for (int w = 0; w < 2; ++w)
-            if (it.nt[w] > 0) issue_s(w, 0, h);
-        s_tile_issued(0);
-        for (int j = 0; j < it.n; ++j) {
-          const uint32_t vpos = 2 * (t_base + j) + 1;
+            if (it.nt[w] > 0) issue_s(w, it.j0, h);
+        s_tile_issued(it.j0);
+        for (int j = it.j0; j < it.n; ++j) {
+          const uint32_t vpos = 2 * (t_base + j - it.j0) + 1;
 #pragma unroll
           for (int h = 0; h < kNU; ++h) {
 #pragma unroll
@@ -449,7 +469,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
               mbar_wait(&p_full[w * 2 + h], (pq[w] / kNU) & 1);
               pf_trace<kTrace>(p, 2, tn, 0x200 + w * 2 + h);  // P ready
               mbar_wait(&kv_full[vpos % kPfSlots], (vpos / kPfSlots) & 1);
-              if (j == 0 && h == 0) mbar_wait(&o_free[w], (eq[w] & 1) ^ 1);  // previous item's O has been read
+              if (j == it.j0 && h == 0) mbar_wait(&o_free[w], (eq[w] & 1) ^ 1);  // previous item's O has been read
               tc_fence_after_sync();
               const uint32_t v_addr = smem_u32(sKV + (vpos % kPfSlots) * kTileBytes) + h * (kU * 128);
 #pragma unroll
@@ -458,7 +478,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                 // blocks of 64 d, LBO = 16 KB; kv rows 128 B apart, 8-row groups SBO = 1 KB)
                 umma_ts(tmem_O + w * kPfD, tmem_S + w * kPfN + h * kU + k * 8,
                         umma_desc_sw128(v_addr + k * 2048, 16384, 1024), idesc_pv,
-                        (j > 0 || h > 0 || k > 0) ? 1u : 0u);
+                        (j > it.j0 || h > 0 || k > 0) ? 1u : 0u);
               }
               umma_commit(&pv_done[w * 2 + h]);
               ++pq[w];
@@ -472,7 +492,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 #pragma unroll
         for (int w = 0; w < 2; ++w)
           if (it.nt[w] > 0) ++eq[w];
-        t_base += it.n;
+        t_base += it.n - it.j0;
         ++itn;
       }
     }
@@ -488,13 +508,13 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     int idx = pf_rank(0, cta, ncta);
     PfRaw raw = pf_raw(p, idx);
     for (int k = 0; idx < p.total_items; ++k) {
-      const PfItem it = pf_item(p, idx, raw);
+      const PfItem it = pf_item<kWin>(p, idx, raw);
       idx = pf_rank(k + 1, cta, ncta);
       raw = pf_raw(p, idx);
       if (it.n == 0) continue;
       const int32_t* rtt = p.req_to_token + p.req_pool_indices[it.req] * p.rtt_stride;
       const int64_t col = static_cast<int64_t>(it.hk) * kPfD + chunk * 8;
-      for (int j = 0; j < it.n; ++j, ++t) {
+      for (int j = it.j0; j < it.n; ++j, ++t) {
         // page-table lookups first, all in flight together (the cp.async asm is a compiler
         // barrier; interleaving the lookups with it would serialise the dependent load latencies)
         int slot[64];
@@ -648,7 +668,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     int idx = pf_rank(0, cta, ncta);
     PfRaw raw = pf_raw(p, idx);
     for (int k = 0; idx < p.total_items; ++k) {
-      const PfItem it = pf_item(p, idx, raw);
+      const PfItem it = pf_item<kWin>(p, idx, raw);
       idx = pf_rank(k + 1, cta, ncta);
       raw = pf_raw(p, idx);
       const int nt = w == 0 ? it.nt[0] : it.nt[1];
@@ -658,36 +678,47 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       const int head = w == 0 ? it.head[0] : it.head[1];
       const int q_row0 = w == 0 ? it.q_row0[0] : it.q_row0[1];
       const int limit = it.pre + m0 + row;  // last visible key of this row (causal)
+      float scale = p.scale_log2;
+      int span = 0;
+      if constexpr (kWin) {
+        span = p.window - 1;
+        if (p.qtemp_every > 0)
+          scale *= 1.f + p.qtemp_coef * logf(static_cast<float>((limit + 1) / p.qtemp_every + 1));
+      }
       float m_used = -INFINITY;  // max currently folded into O and l (raw score units)
       float l = 0.f;
-      for (int jh = 0; jh < kNU * nt; ++jh, ++u) {
+      for (int jh = 0; jh < kNU * (nt - it.j0); ++jh, ++u) {
         const int h = jh % kNU;
-        const int kv0 = (jh / kNU) * kPfN + h * kU;
-        const bool need_mask = (kv0 + kU - 1) > (it.pre + m0);
+        const int kv0 = (it.j0 + jh / kNU) * kPfN + h * kU;
+        // a row that does not see the whole unit: the first one past its end, or the last one with its window past its start
+        const bool need_mask = (kv0 + kU - 1) > (it.pre + m0) || (kWin && kv0 < it.pre + m0 + kPfM - p.window);
         const uint32_t tsh = ts + h * kU;
         if (tracer) pf_trace<kTrace>(p, w, tn, 0x100 + h);  // waiting for S
         mbar_wait(&s_full[w * 2 + h], (u / kNU) & 1);
         tc_fence_after_sync();
         if (tracer) pf_trace<kTrace>(p, w, tn, 0x200 + h);  // S ready
-        if (jh == 0) {
-          // first unit of the item: establish the reference max with a max-only pre-pass
-          m_used = need_mask ? softmax_row_max<true, kU>(tsh, kv0, limit) : softmax_row_max<false, kU>(tsh, kv0, limit);
+        if (jh == 0 || (kWin && __any_sync(0xffffffffu, m_used == -INFINITY))) {
+          // first unit of the item — with a window, also as long as some row has seen no key — establish the reference
+          // max with a max-only pre-pass
+          const float mx = need_mask ? softmax_row_max<true, kU, kWin>(tsh, kv0, limit, span)
+                                     : softmax_row_max<false, kU, kWin>(tsh, kv0, limit, span);
+          if (m_used == -INFINITY) m_used = mx;
         }
-        float m_off = (m_used == -INFINITY) ? 0.f : m_used * p.scale_log2;
+        float m_off = (m_used == -INFINITY) ? 0.f : m_used * scale;
         uint32_t pk[kU / 2];
-        float psum = need_mask ? softmax_row_pass<T, true, kU>(tsh, pk, p.scale_log2, m_off, kv0, limit)
-                               : softmax_row_pass<T, false, kU>(tsh, pk, p.scale_log2, m_off, kv0, limit);
+        float psum = need_mask ? softmax_row_pass<T, true, kU, kWin>(tsh, pk, scale, m_off, kv0, limit, span)
+                               : softmax_row_pass<T, false, kU, kWin>(tsh, pk, scale, m_off, kv0, limit, span);
         // raise the reference max only when some row may have outgrown it by > 2^8 (an element
         // above 2^8 implies a row sum above 2^8; warp-uniform decision: tcgen05.ld/st are
         // warp-collective); S is still intact (P is stored below), so the unit is simply redone
         if (__any_sync(0xffffffffu, psum > kRescaleTrigger)) {
-          const float mx = need_mask ? softmax_row_max<true, kU>(tsh, kv0, limit)
-                                     : softmax_row_max<false, kU>(tsh, kv0, limit);
+          const float mx = need_mask ? softmax_row_max<true, kU, kWin>(tsh, kv0, limit, span)
+                                     : softmax_row_max<false, kU, kWin>(tsh, kv0, limit, span);
           const float m_new = fmaxf(m_used, mx);
-          const float alpha = (m_used == -INFINITY) ? 0.f : fast_exp2((m_used - m_new) * p.scale_log2);
+          const float alpha = (m_used == -INFINITY) ? 0.f : fast_exp2((m_used - m_new) * scale);
           l *= alpha;
           m_used = m_new;
-          m_off = (m_used == -INFINITY) ? 0.f : m_used * p.scale_log2;
+          m_off = (m_used == -INFINITY) ? 0.f : m_used * scale;
           if (jh > 0) {
             // O must be quiescent: S of this unit was issued after PV of unit u-kNU (so units
             // <= u-kNU are complete), but PV of the units in between (the other half) may still
@@ -706,8 +737,8 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
               tmem_st_32x32b_x32(to + c, r);
             }
           }
-          psum = need_mask ? softmax_row_pass<T, true, kU>(tsh, pk, p.scale_log2, m_off, kv0, limit)
-                           : softmax_row_pass<T, false, kU>(tsh, pk, p.scale_log2, m_off, kv0, limit);
+          psum = need_mask ? softmax_row_pass<T, true, kU, kWin>(tsh, pk, scale, m_off, kv0, limit, span)
+                           : softmax_row_pass<T, false, kU, kWin>(tsh, pk, scale, m_off, kv0, limit, span);
         }
         l += psum;
         // P over the first kU/2 columns of this S unit (every column of it is in registers by now)
@@ -720,6 +751,9 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         if (tracer) pf_trace<kTrace>(p, w, tn, 0x300 + h);  // P published
       }
       if (tracer) pf_trace<kTrace>(p, w, tn, 0x400);  // item done
+      if constexpr (kWin) {
+        if (p.sinks != nullptr) l += fast_exp2(p.sinks[head] * 1.4426950408889634f - m_used * scale);
+      }
       e_l = l;
       e_rows = rows_valid;
       e_head = head;
@@ -734,6 +768,91 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 10) tmem_dealloc(tmem_base, 512);
+}
+
+static int pf_setup(PrefillParams& p, CUtensorMap& tq, CUtensorMap& tk, CUtensorMap& tv, CUtensorMap& to, void* out,
+                    const void* q, const void* k_pool, const void* v_pool, const int32_t* req_to_token,
+                    const int64_t* req_pool_indices, const int32_t* prefix_lens, const int32_t* extend_lens,
+                    const int32_t* extend_start_loc, int64_t batch, int64_t total_tokens, int64_t max_extend_len,
+                    int num_q_heads, int num_kv_heads, int64_t q_stride, int64_t out_stride, int64_t req_to_token_stride,
+                    float sm_scale) {
+  p.out = out;
+  p.k_pool = k_pool;
+  p.v_pool = v_pool;
+  p.req_to_token = req_to_token;
+  p.req_pool_indices = req_pool_indices;
+  p.prefix_lens = prefix_lens;
+  p.extend_lens = extend_lens;
+  p.extend_start_loc = extend_start_loc;
+  p.Hq = num_q_heads;
+  p.Hk = num_kv_heads;
+  p.out_stride = out_stride;
+  p.rtt_stride = req_to_token_stride;
+  p.scale_log2 = sm_scale * 1.4426950408889634f;
+  const int q_tiles = static_cast<int>((max_extend_len + kPfM - 1) / kPfM);
+  p.pair_heads = ((num_q_heads / num_kv_heads) % 2 == 0) ? 1 : 0;
+  p.tiles_x = p.pair_heads ? q_tiles : (q_tiles + 1) / 2;
+  p.heads_x = p.pair_heads ? num_q_heads / 2 : num_q_heads;
+  p.batch = static_cast<int>(batch);
+  const int64_t total = static_cast<int64_t>(p.tiles_x) * p.heads_x * batch;
+  SPD_REQUIRE(total < (1ll << 30), SPD_E_SHAPE, "prefill attention: too many work items");
+  p.total_items = static_cast<int>(total);
+  fastdiv_magic(static_cast<uint32_t>(p.heads_x) * static_cast<uint32_t>(p.batch), p.per_x_m, p.per_x_s);
+  fastdiv_magic(static_cast<uint32_t>(p.heads_x), p.heads_x_m, p.heads_x_s);
+  fastdiv_magic(static_cast<uint32_t>(num_q_heads / num_kv_heads), p.group_m, p.group_s);
+  if (int rc = get_tmap(&tq, q, static_cast<uint64_t>(total_tokens),
+                     static_cast<uint64_t>(num_q_heads) * kPfD, static_cast<uint64_t>(q_stride), kPfM))
+    return rc;
+  // the output as a TMA-store target: same geometry as Q (rows beyond total_tokens are clipped)
+  if (int rc = get_tmap(&to, out, static_cast<uint64_t>(total_tokens),
+                     static_cast<uint64_t>(num_q_heads) * kPfD, static_cast<uint64_t>(out_stride), kPfM))
+    return rc;
+  // K/V pools as [slots, Hk*D] tensors, box 128 rows x 64 columns (the row extent only bounds the
+  // coordinates; they are slot ids taken from req_to_token)
+  static const bool tma_on = []() { const char* e = getenv("SPD_ATTN_TMA"); return !(e && e[0] == '0'); }();
+  p.use_tma = tma_on ? 1 : 0;
+  const uint64_t row_elems = static_cast<uint64_t>(num_kv_heads) * kPfD;
+  if (int rc = get_tmap(&tk, k_pool, 1ull << 31, row_elems, row_elems, kPfN)) return rc;
+  if (int rc = get_tmap(&tv, v_pool, 1ull << 31, row_elems, row_elems, kPfN)) return rc;
+  return 0;
+}
+
+// Ragged extend of the general attention at head size 128 with a window, sinks and a query temperature (no distance bias,
+// score cap, pooled blocks or kept first tokens).  → 0 launched, 1 not applicable, else an error.
+int attn_prefill_window_try(void* out, const void* q, const void* k_pool, const void* v_pool, const int32_t* req_to_token,
+                            const int64_t* req_pool_indices, const int32_t* prefix_lens, const int32_t* extend_lens,
+                            const int32_t* extend_start_loc, int64_t batch, int64_t total_tokens, int64_t max_extend_len,
+                            int H, int G, int64_t q_stride, int64_t out_stride, int64_t r2t_stride, float sm_scale,
+                            int window, const float* sinks, float qtemp_coef, int qtemp_every, int dtype,
+                            cudaStream_t stream) {
+  // a reference max of raw scores serves the scaled ones only where the scale is not negative
+  if (!(sm_scale >= 0.f) || !(qtemp_every <= 0 || qtemp_coef >= 0.f)) return 1;
+  if (q_stride % 8 != 0 || out_stride % 8 != 0 || !aligned16(out) || !aligned16(q) || !aligned16(k_pool) || !aligned16(v_pool))
+    return 1;
+  const int64_t items = (max_extend_len + kPfM - 1) / kPfM * H * batch;
+  if (total_tokens <= 0 || items >= (1ll << 30) || total_tokens >= (1ll << 31)) return 1;
+  PrefillParams p{};
+  CUtensorMap tq, tk, tv, to;
+  if (int rc = pf_setup(p, tq, tk, tv, to, out, q, k_pool, v_pool, req_to_token, req_pool_indices, prefix_lens, extend_lens,
+                        extend_start_loc, batch, total_tokens, max_extend_len, H, G, q_stride, out_stride, r2t_stride,
+                        sm_scale))
+    return rc;
+  p.window = window > 0 && window < (1 << 30) ? window : 1 << 30;
+  p.sinks = sinks;
+  p.qtemp_coef = qtemp_coef;
+  p.qtemp_every = qtemp_every > 0 ? qtemp_every : 0;
+  const int sms = device_sm_count_cached();
+  const int grid = p.total_items < sms ? p.total_items : sms;
+  SPD_DISPATCH_DTYPE(dtype, {
+    auto kern = attn_prefill_kernel<T, 64, false, true>;
+    static bool configured = false;
+    if (!configured) {
+      SPD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmem));
+      configured = true;
+    }
+    SPD_CUDA(launch(kern, dim3(grid), dim3(kPfThreads), kPfSmem, stream, pdl_enabled(), tq, tk, tv, to, p));
+  });
+  return 0;
 }
 
 int check_attn_args(const char* fn, const void* out, const void* q, const void* k_pool,
@@ -773,52 +892,18 @@ extern "C" int spd_attn_prefill_ragged(void* out, const void* q, const void* k_p
               "spd_attn_prefill_ragged: head_dim must be 128 on the tcgen05 path (got %d)", head_dim);
   if (batch == 0 || total_tokens == 0 || max_extend_len == 0) return 0;
   PrefillParams p{};
-  p.out = out;
-  p.k_pool = k_pool;
-  p.v_pool = v_pool;
-  p.req_to_token = req_to_token;
-  p.req_pool_indices = req_pool_indices;
-  p.prefix_lens = prefix_lens;
-  p.extend_lens = extend_lens;
-  p.extend_start_loc = extend_start_loc;
-  p.Hq = num_q_heads;
-  p.Hk = num_kv_heads;
-  p.out_stride = out_stride;
-  p.rtt_stride = req_to_token_stride;
-  p.scale_log2 = sm_scale * 1.4426950408889634f;
-  const int q_tiles = static_cast<int>((max_extend_len + kPfM - 1) / kPfM);
-  p.pair_heads = ((num_q_heads / num_kv_heads) % 2 == 0) ? 1 : 0;
-  p.tiles_x = p.pair_heads ? q_tiles : (q_tiles + 1) / 2;
-  p.heads_x = p.pair_heads ? num_q_heads / 2 : num_q_heads;
-  p.batch = static_cast<int>(batch);
-  const int64_t total = static_cast<int64_t>(p.tiles_x) * p.heads_x * batch;
-  SPD_REQUIRE(total < (1ll << 30), SPD_E_SHAPE, "spd_attn_prefill_ragged: too many work items");
-  p.total_items = static_cast<int>(total);
-  fastdiv_magic(static_cast<uint32_t>(p.heads_x) * static_cast<uint32_t>(p.batch), p.per_x_m, p.per_x_s);
-  fastdiv_magic(static_cast<uint32_t>(p.heads_x), p.heads_x_m, p.heads_x_s);
-  fastdiv_magic(static_cast<uint32_t>(num_q_heads / num_kv_heads), p.group_m, p.group_s);
   CUtensorMap tq, tk, tv, to;
-  if ((rc = get_tmap(&tq, q, static_cast<uint64_t>(total_tokens),
-                     static_cast<uint64_t>(num_q_heads) * head_dim, static_cast<uint64_t>(q_stride), kPfM)))
+  if ((rc = pf_setup(p, tq, tk, tv, to, out, q, k_pool, v_pool, req_to_token, req_pool_indices, prefix_lens, extend_lens,
+                     extend_start_loc, batch, total_tokens, max_extend_len, num_q_heads, num_kv_heads, q_stride, out_stride,
+                     req_to_token_stride, sm_scale)))
     return rc;
-  // the output as a TMA-store target: same geometry as Q (rows beyond total_tokens are clipped)
-  if ((rc = get_tmap(&to, out, static_cast<uint64_t>(total_tokens),
-                     static_cast<uint64_t>(num_q_heads) * head_dim, static_cast<uint64_t>(out_stride), kPfM)))
-    return rc;
-  // K/V pools as [slots, Hk*D] tensors, box 128 rows x 64 columns (the row extent only bounds the
-  // coordinates; they are slot ids taken from req_to_token)
-  static const bool tma_on = []() { const char* e = getenv("SPD_ATTN_TMA"); return !(e && e[0] == '0'); }();
-  p.use_tma = tma_on ? 1 : 0;
-  const uint64_t row_elems = static_cast<uint64_t>(num_kv_heads) * head_dim;
-  if ((rc = get_tmap(&tk, k_pool, 1ull << 31, row_elems, row_elems, kPfN))) return rc;
-  if ((rc = get_tmap(&tv, v_pool, 1ull << 31, row_elems, row_elems, kPfN))) return rc;
   const int sms = sm_budget > 0 ? sm_budget : device_sm_count_cached();
   const int grid = p.total_items < sms ? p.total_items : sms;
   // SPD_ATTN_PF_UNIT = 64 | 128: width of a softmax / MMA unit (see the kernel's kU)
   static const int unit = []() { const char* e = getenv("SPD_ATTN_PF_UNIT"); return (e && atoi(e) == 128) ? 128 : 64; }();
 #define SPD_PF_LAUNCH(U, TR)                                                                           \
   do {                                                                                                 \
-    auto kern = attn_prefill_kernel<T, U, TR>;                                                         \
+    auto kern = attn_prefill_kernel<T, U, TR, false>;                                                       \
     static bool configured = false;                                                                    \
     if (!configured) {                                                                                 \
       SPD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmem));      \
