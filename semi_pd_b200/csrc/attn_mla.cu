@@ -52,7 +52,6 @@ constexpr int kMlaDL = 576, kMlaDV = 512;
 constexpr int kMlaBlk = kMlaTile * 128;       // one [64 rows x 64 columns] swizzle block of a tile
 constexpr int kMlaMisc = 2048;
 constexpr float kMlaRescale = 8.0f;           // log2 units a score may exceed the reference max before it is raised
-constexpr int kMlaWaitTries = 1 << 22;
 
 __device__ unsigned int g_mla_wait_expired;
 
@@ -108,14 +107,6 @@ struct MlaSlot {
     }
   }
 };
-
-__device__ __forceinline__ void mla_wait(uint64_t* bar, uint32_t parity, volatile int* dead) {
-  for (int i = 0; i < kMlaWaitTries; ++i) {
-    if (mbar_try_wait(bar, parity)) return;
-    if (*dead) return;
-  }
-  *dead = 1;
-}
 
 // an item: one token (decode) or group of four tokens (extend) of a request, times 16 heads
 struct MlaItem {
@@ -435,12 +426,12 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
         // still be on the way: PV frees ring slots, so it never waits behind a copy
         if (c.valid && (ts == tp || (ts == tp + 1 && !cross && mbar_test(&t_full[ts & 3], (ts >> 2) & 1)))) {
           const int b = ts & 1;
-          if (cross) mla_wait(q_full, c.seg & 1, dead);
+          if (cross) mbar_wait_bounded(q_full, c.seg & 1, dead);
           firsts = (firsts & ~(1u << b)) | (cross ? 1u << b : 0u);
           segs = (segs & ~(1u << b)) | ((c.seg & 1) << b);
-          mla_wait(&s_empty[b], ((ts >> 1) & 1) ^ 1, dead);
+          mbar_wait_bounded(&s_empty[b], ((ts >> 1) & 1) ^ 1, dead);
           const uint32_t d = tmem_S + b * 2 * N;
-          mla_wait(&t_full[ts & 3], (ts >> 2) & 1, dead);
+          mbar_wait_bounded(&t_full[ts & 3], (ts >> 2) & 1, dead);
           if (cross || s_gath[ts & 3]) fence_proxy_async_smem();  // Q, and gathered tiles, come by cp.async
           tc_fence_after_sync();
           // two accumulators in turn; the softmax adds them
@@ -468,9 +459,9 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
           continue;
         }
         const int b = tp & 1;
-        mla_wait(p_full, tp & 1, dead);
+        mbar_wait_bounded(p_full, tp & 1, dead);
         const bool first = (firsts >> b) & 1;
-        if (first) mla_wait(o_empty, ((segs >> b) & 1) ^ 1, dead);
+        if (first) mbar_wait_bounded(o_empty, ((segs >> b) & 1) ^ 1, dead);
         tc_fence_after_sync();  // (P's writers have fenced; the rows were fenced for S)
 #pragma unroll 1
         for (int i = 0; i < 4; i += 2) {  // two blocks of 128 value columns in turn
@@ -534,11 +525,11 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
           mbar_expect_tx(full, 9 * kMlaBlk);
 #pragma unroll 1
           for (int st = 0; st < 4; ++st) {
-            mla_wait(&k_empty[ks.i], ks.round ^ 1, dead);
+            mbar_wait_bounded(&k_empty[ks.i], ks.round ^ 1, dead);
             tma_load_3d(sK + ks.i * 2 * kMlaBlk, &tmKV, full, 0, base, 2 * st, kEvictNormal);
             ks.next();
           }
-          mla_wait(&r_empty[rs.i], rs.round ^ 1, dead);
+          mbar_wait_bounded(&r_empty[rs.i], rs.round ^ 1, dead);
           tma_load_2d(sR + rs.i * kMlaBlk, &tmR, full, kMlaDV, base, kEvictNormal);
           rs.next();
           mbar_arrive_n(full, 64);
@@ -550,7 +541,7 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
 #pragma unroll 1
         for (int st = 0; st < 5; ++st) {
           uint8_t* dst = st < 4 ? sK + ks.i * 2 * kMlaBlk : sR + rs.i * kMlaBlk;
-          mla_wait(st < 4 ? &k_empty[ks.i] : &r_empty[rs.i], (st < 4 ? ks.round : rs.round) ^ 1, dead);
+          mbar_wait_bounded(st < 4 ? &k_empty[ks.i] : &r_empty[rs.i], (st < 4 ? ks.round : rs.round) ^ 1, dead);
           const int shift = st < 4 ? 4 : 3;  // log2 of the 16-byte chunks of a row in a pair / in the rope block
 #pragma unroll 4
           for (int i = lt; i < kMlaTile << shift; i += 64) {
@@ -566,7 +557,7 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
       }
       if (load_q) {
         // the item's N query rows (token, head), zero where there is none; the tile above is already on its way
-        mla_wait(q_empty, (seg & 1) ^ 1, dead);
+        mbar_wait_bounded(q_empty, (seg & 1) ^ 1, dead);
         const T* qb = reinterpret_cast<const T*>(p.q);
         const int h0 = it.hg * kMlaHeads, nh = min(kMlaHeads, p.H - h0);
 #pragma unroll 4
@@ -618,7 +609,7 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
         const bool first = c.tile == tile0;
         c.next(p);
         const int sb = t & 1;
-        mla_wait(&s_full[sb], (t >> 1) & 1, dead);
+        mbar_wait_bounded(&s_full[sb], (t >> 1) & 1, dead);
         tc_fence_after_sync();
         uint32_t r[N / 2], r2[N / 2];
         mla_ld_frag(tmem_S + lane_base + sb * 2 * N, r);
@@ -662,7 +653,7 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
           }
           mla_bar();
           if (!first) {
-            mla_wait(p_empty, (t & 1) ^ 1, dead);  // PV of the previous tile has finished: O^T is stable
+            mbar_wait_bounded(p_empty, (t & 1) ^ 1, dead);  // PV of the previous tile has finished: O^T is stable
             tc_fence_after_sync();
 #pragma unroll 1
             for (int cc = 0; cc < 4 * N; cc += 16) {
@@ -691,7 +682,7 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
             l_thr[2 * g] += v.x;
             l_thr[2 * g + 1] += v.y;
           }
-        mla_wait(p_empty, (t & 1) ^ 1, dead);
+        mbar_wait_bounded(p_empty, (t & 1) ^ 1, dead);
 #pragma unroll
         for (int g = 0; g < N / 8; g += 2) {
           // matrices: (columns 8 g.., kv 0-7), (8 g.., kv 8-15), (8 (g + 1).., kv 0-7), (8 (g + 1).., kv 8-15)
@@ -731,7 +722,7 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
         }
       }
       mla_bar();
-      mla_wait(p_empty, (t - 1) & 1, dead);  // the last PV of the item has finished
+      mbar_wait_bounded(p_empty, (t - 1) & 1, dead);  // the last PV of the item has finished
       tc_fence_after_sync();
       T* out = reinterpret_cast<T*>(p.out) + it.row0 * p.out_stride + static_cast<int64_t>(h0) * kMlaDV + warp * 32;
 #pragma unroll 1
