@@ -432,6 +432,15 @@ int spd_retention(float* o, const void* q, const void* k, const void* v, float* 
                   int64_t batch, int num_heads, int head_dim, int v_dim, int64_t q_stride, int64_t k_stride,
                   int64_t v_stride, const float* decay, const float* cos_sin, int rot_dims,
                   int64_t max_positions, float k_scale, int in_act, int dtype, spd_stream_t stream);
+/* Ragged extend of spd_retention for a caller that knows the batch's new tokens: portions of some length run in chunks on
+ * the tensor cores where sizes and types allow it (16-bit, head_dim 128, v_dim a multiple of 64, rot_dims a multiple of
+ * 16, no in_act), everything else as spd_retention. */
+int spd_retention_extend(float* o, const void* q, const void* k, const void* v, float* state,
+                         const int64_t* req_pool_indices, const int32_t* prefix_lens, const int32_t* extend_lens,
+                         const int32_t* extend_start_loc, int64_t batch, int64_t total_tokens, int num_heads, int head_dim,
+                         int v_dim, int64_t q_stride, int64_t k_stride, int64_t v_stride, const float* decay,
+                         const float* cos_sin, int rot_dims, int64_t max_positions, float k_scale, int in_act, int dtype,
+                         spd_stream_t stream);
 
 /* spd_residual_rmsnorm with a second weight: out2 = the same normed row times (weight_offset + w2)
  * (out2 and w2 both NULL or both given) */

@@ -211,7 +211,8 @@ int retention_chunked_try(float* o, const void* q, const void* k, const void* v,
                           const int64_t* req_pool_indices, const int32_t* prefix_lens, const int32_t* extend_lens,
                           const int32_t* extend_start_loc, int64_t batch, int H, int dk, int dv, int64_t q_stride,
                           int64_t k_stride, int64_t v_stride, const float* decay, const float* cos_sin, int rot,
-                          int64_t max_positions, float k_scale, int in_act, int dtype, cudaStream_t stream);
+                          int64_t max_positions, float k_scale, int in_act, int dtype, int64_t total_tokens,
+                          cudaStream_t stream);
 
 template <typename T, int W, int ROWS, bool ASYNC, int TOK>
 int retention_launch(dim3 grid, size_t smem, cudaStream_t stream, float* o, const void* q, const void* k, const void* v,
@@ -254,12 +255,6 @@ int spd_retention(float* o, const void* q, const void* k, const void* v, float* 
               SPD_E_BADARG, "spd_retention: bad rotation (rot_dims %d)", rot_dims);
   SPD_REQUIRE(in_act == 0 || in_act == 1, SPD_E_BADARG, "spd_retention: in_act is 0 (none) or 1 (SiLU)");
   if (batch == 0) return 0;
-  if (seq_lens == nullptr) {
-    const int rc = retention_chunked_try(o, q, k, v, state, req_pool_indices, prefix_lens, extend_lens, extend_start_loc,
-                                         batch, num_heads, head_dim, v_dim, q_stride, k_stride, v_stride, decay, cos_sin,
-                                         rot_dims, max_positions, k_scale, in_act, dtype, as_stream(stream));
-    if (rc != 1) return rc;
-  }
   const dim3 grid((unsigned)batch, (unsigned)num_heads, (unsigned)((v_dim + kRetCols - 1) / kRetCols));
   // warps x rows per thread covering head_dim: 8 rows per thread up to 128, 16 above
   const int warps = head_dim <= 32 ? 4 : head_dim <= 64 ? 8 : 16;
@@ -292,6 +287,26 @@ int spd_retention(float* o, const void* q, const void* k, const void* v, float* 
 #undef SPD_RET_SHAPE
 #undef SPD_RET_ARGS
   return 0;
+}
+
+int spd_retention_extend(float* o, const void* q, const void* k, const void* v, float* state,
+                         const int64_t* req_pool_indices, const int32_t* prefix_lens, const int32_t* extend_lens,
+                         const int32_t* extend_start_loc, int64_t batch, int64_t total_tokens, int num_heads, int head_dim,
+                         int v_dim, int64_t q_stride, int64_t k_stride, int64_t v_stride, const float* decay,
+                         const float* cos_sin, int rot_dims, int64_t max_positions, float k_scale, int in_act, int dtype,
+                         spd_stream_t stream) {
+  const bool checked = o && q && k && v && state && req_pool_indices && decay && prefix_lens && extend_lens &&
+                       extend_start_loc && num_heads > 0 && head_dim > 0 && v_dim > 0 && rot_dims >= 0 &&
+                       rot_dims <= head_dim && (rot_dims == 0 || (cos_sin && max_positions > 0)) && batch > 0;
+  if (checked) {  // (what is not is reported by the call below)
+    const int rc = retention_chunked_try(o, q, k, v, state, req_pool_indices, prefix_lens, extend_lens, extend_start_loc,
+                                         batch, num_heads, head_dim, v_dim, q_stride, k_stride, v_stride, decay, cos_sin,
+                                         rot_dims, max_positions, k_scale, in_act, dtype, total_tokens, as_stream(stream));
+    if (rc != 1) return rc;
+  }
+  return spd_retention(o, q, k, v, state, req_pool_indices, nullptr, nullptr, prefix_lens, extend_lens, extend_start_loc,
+                       batch, num_heads, head_dim, v_dim, q_stride, k_stride, v_stride, decay, cos_sin, rot_dims,
+                       max_positions, k_scale, in_act, dtype, stream);
 }
 
 }  // extern "C"

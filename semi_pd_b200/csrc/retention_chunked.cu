@@ -11,13 +11,15 @@
 // has one part: v (two parts for fp16 values), and the channels of bf16 q and k that are not rotated.  Against 64 bits
 // the outputs' relative error is no larger than the recurrence's (tests).
 //
-// Per chunk (256 threads, one CTA per SM):
+// Per chunk (512 threads, one CTA per SM):
 //   split q, k, v' = c d^(n-1-j) v into shared memory (128-byte swizzle); fetch the next chunk's raw rows (cp.async)
 //   MMA  A~ = Q K^T [64 x 64], O1 = Q S [64 x 64], U = K^T V' [128 x 64]
 //   A~ -> decay, mask, split -> shared memory (over Q);   MMA  O2 = A V [64 x 64]
-//   S (fp32, 32 values per thread in registers) = d^n S + U -> split -> shared memory;   o = d^(i+1) O1 + O2
+//   S (fp32, 16 values per thread in registers) = d^n S + U -> split -> shared memory;   o = d^(i+1) O1 + O2
 // K is stored once: rows of tokens serve Q K^T as K-major and K^T V' as MN-major operand.  Rows past the portion are
-// zeros.  What bounds it: the chain of a chunk (split 1500 clk, MMAs 3500, decay and split of A, read-out).
+// zeros.  What bounds it: the chain of a chunk (split 2800 clk, Q K^T and
+// Q S 3600, A 800, A V and the rest 3000), one after another in a CTA that fills an SM.  4 requests, 8192 tokens, 16 heads
+// of 128 x 128: 875 us token by token, 256 us here (41 chunks of 6 us for the longest request).
 //
 // The sums of a portion are cut every 64 tokens from its start, so results depend in their last bits on how a prompt is
 // cut into portions (the token-by-token kernel's do not).
@@ -29,7 +31,7 @@ namespace spd {
 constexpr int kRcTok = 64;       // tokens per chunk
 constexpr int kRcDk = 128;       // key channels
 constexpr int kRcDv = 64;        // value columns per CTA
-constexpr int kRcThreads = 256;
+constexpr int kRcThreads = 512;
 constexpr int kRcQ = 2 * kRcTok * 128;   // one part of q or k: two [64 x 128 B] swizzle blocks
 constexpr int kRcS = kRcDk * 128;        // one part of S: [128 x 128 B]
 constexpr int kRcV = kRcTok * 128;       // one part of v, v', A: [64 x 128 B]
@@ -83,19 +85,23 @@ __device__ __forceinline__ void rc_load8(const T* p, float (&x)[8]) {
   }
 }
 
-// 16 lanes x 32 columns as mma fragments: value 4 g + e is row (lane >> 2) + 8 (e >> 1), column 8 g + 2 (lane & 3) + (e & 1)
-__device__ __forceinline__ void rc_ld_frag(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
+// 16 lanes x 16 columns as mma fragments: value 4 g + e is row (lane >> 2) + 8 (e >> 1), column 8 g + 2 (lane & 3) + (e & 1)
+__device__ __forceinline__ void rc_ld_frag(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
+}
+
+// one warp polls, the others wait at a barrier
+__device__ __forceinline__ void rc_wait(uint64_t* bar, uint32_t parity, int warp, volatile int* dead) {
+  if (warp == 0) mbar_wait_bounded(bar, parity, dead);
+  asm volatile("bar.sync 1, %0;" ::"n"(kRcThreads) : "memory");
 }
 
 // parts (a, b) of the six products, smallest first
-__device__ __forceinline__ int rc_pa(int i) { return (0x001102 >> (4 * i)) & 15; }  // 2 0 1 1 0 0
-__device__ __forceinline__ int rc_pb(int i) { return (0x010120 >> (4 * i)) & 15; }  // 0 2 1 0 1 0
+__host__ __device__ constexpr int rc_pa(int i) { return (0x001102 >> (4 * i)) & 15; }  // 2 0 1 1 0 0
+__host__ __device__ constexpr int rc_pb(int i) { return (0x010120 >> (4 * i)) & 15; }  // 0 2 1 0 1 0
 
 template <typename T, int VS>  // VS: bf16 parts of a value as it is stored (1: bf16, 2: fp16)
 __global__ void __launch_bounds__(kRcThreads, 1)
@@ -160,19 +166,19 @@ retention_chunked_kernel(const RetChunkParams p) {
   };
   fetch(0);
 
-  // this thread's piece of the state: channel sr, value columns sc .. sc + 31
-  const int sr = (warp & 3) * 32 + lane, sc = (warp >> 2) * 32;
+  // this thread's piece of the state: channel sr, value columns sc .. sc + 15
+  const int sr = (warp & 3) * 32 + lane, sc = (warp >> 2) * 16;
   float* st = p.state + (p.req_pool_indices[r] * p.H + h) * static_cast<int64_t>(kRcDk) * p.dv +
               static_cast<int64_t>(sr) * p.dv + col0 + sc;
-  float S[32];
+  float S[16];
 #pragma unroll
-  for (int i = 0; i < 32; i += 4) {
+  for (int i = 0; i < 16; i += 4) {
     const float4 x = pos0 > 0 ? *reinterpret_cast<const float4*>(st + i) : make_float4(0.f, 0.f, 0.f, 0.f);
     S[i] = x.x; S[i + 1] = x.y; S[i + 2] = x.z; S[i + 3] = x.w;
   }
   auto put_state = [&]() {
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
+    for (int c = 0; c < 2; ++c) {
       float x[8];
 #pragma unroll
       for (int e = 0; e < 8; ++e) x[e] = S[8 * c + e];
@@ -183,88 +189,84 @@ retention_chunked_kernel(const RetChunkParams p) {
   const int half = p.rot >> 1;
   const int rot_steps = sizeof(T) == 2 && VS == 1 ? p.rot / 16 : kRcDk / 16;  // k-steps whose q, k need three parts
   const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
-  const int ar = (warp & 3) * 16 + (lane >> 2), ac = (warp >> 2) * 32 + 2 * (lane & 3);  // fragment row (+ 8), column
+  const int ar = (warp & 3) * 16 + (lane >> 2), ac = (warp >> 2) * 16 + 2 * (lane & 3);  // fragment row (+ 8), column
 
+  // this thread's part of a chunk's preparation: token ut; value columns 8 u ..; key channels d0 .. d0 + 7 and d1 .. d1 + 7,
+  // the two halves of a rotation where they are rotated, neighbours elsewhere
+  const int ut = tid >> 3, u = tid & 7;
+  const int d0 = u * 16 < p.rot ? u * 8 : u * 16, d1 = u * 16 < p.rot ? d0 + half : d0 + 8;
+  float cs[8], sn[8];
+  auto angles = [&](int t0) {  // cos / sin of this thread's token and channels, loaded a chunk ahead
+    if (d0 >= p.rot) return;
+    int64_t pos = pos0 + t0 + ut;
+    pos = pos < p.max_positions ? pos : p.max_positions - 1;
+    const float4* cp = reinterpret_cast<const float4*>(p.cos_sin + pos * p.rot + d0);
+    const float4* sp = reinterpret_cast<const float4*>(p.cos_sin + pos * p.rot + half + d0);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const float4 a = __ldg(cp + e), b = __ldg(sp + e);
+      cs[4 * e] = a.x; cs[4 * e + 1] = a.y; cs[4 * e + 2] = a.z; cs[4 * e + 3] = a.w;
+      sn[4 * e] = b.x; sn[4 * e + 1] = b.y; sn[4 * e + 2] = b.z; sn[4 * e + 3] = b.w;
+    }
+  };
+  angles(0);
   int nt = 0;
   for (int t0 = 0, it = 0; t0 < n; t0 += nt, ++it) {
     const uint32_t par = it & 1;
     cp_async_wait<0>();
     bool odd = false;  // an infinite or NaN value among those this thread has fetched
-    for (int i = tid; i < kRcTok * 8; i += kRcThreads) {
-      float x[8];
-      rc_load8<T>(rv + (i >> 3) * kRcDv + (i & 7) * 8, x);
+    float v8[8];
+    {
+      rc_load8<T>(rv + ut * kRcDv + u * 8, v8);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) odd |= !(fabsf(x[e]) <= 3.4028235e38f);
+      for (int e = 0; e < 8; ++e) odd |= !(fabsf(v8[e]) <= 3.4028235e38f);
     }
     tc_fence_before_sync();
     // raw rows visible; the previous chunk's operands and accumulators have been read.  With such a value the zeros of the
     // masked A would spoil the tokens before it: its chunk is taken one token at a time.
     nt = __syncthreads_or(odd) ? 1 : min(kRcTok, n - t0);
-    // ---- q, k: rotate, split ----
-    for (int i = tid; i < kRcTok * 16; i += kRcThreads) {
-      const int t = i >> 4, ch = i & 15, d = ch * 8;
-      float x[8], y[8];
-      if (t >= nt) {
+    {
+      // ---- q, k: rotate, split: 16 channels of a token and of each ----
+      const bool live = ut < nt;
 #pragma unroll
-        for (int e = 0; e < 8; ++e) x[e] = y[e] = 0.f;
-        const uint32_t off = (ch >> 3) * kRcV + rc_off(t, ch & 7);
-        rc_split8(x, sQ + off, kRcQ);
-        rc_split8(y, sK + off, kRcQ);
-        continue;
-      }
-      rc_load8<T>(rq + t * kRcDk + d, x);
-      rc_load8<T>(rk + t * kRcDk + d, y);
-      if (d < p.rot) {
-        const bool low = d < half;
-        const int od = low ? d + half : d - half, ci = low ? d : d - half;
-        float ox[8], oy[8], c[8], s[8];
-        rc_load8<T>(rq + t * kRcDk + od, ox);
-        rc_load8<T>(rk + t * kRcDk + od, oy);
-        int64_t pos = pos0 + t0 + t;
-        pos = pos < p.max_positions ? pos : p.max_positions - 1;
-        const float4* cp = reinterpret_cast<const float4*>(p.cos_sin + pos * p.rot + ci);
-        const float4* sp = reinterpret_cast<const float4*>(p.cos_sin + pos * p.rot + half + ci);
+      for (int w = 0; w < 2; ++w) {
+        const T* raw = (w ? rk : rq) + ut * kRcDk;
+        float x[8], y[8];
+        rc_load8<T>(raw + d0, x);
+        rc_load8<T>(raw + d1, y);
+        if (d0 < p.rot) {
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const float4 a = __ldg(cp + e), b = __ldg(sp + e);
-          c[4 * e] = a.x; c[4 * e + 1] = a.y; c[4 * e + 2] = a.z; c[4 * e + 3] = a.w;
-          s[4 * e] = b.x; s[4 * e + 1] = b.y; s[4 * e + 2] = b.z; s[4 * e + 3] = b.w;
+          for (int e = 0; e < 8; ++e) {
+            const float a = x[e], b = y[e];
+            x[e] = a * cs[e] - b * sn[e];
+            y[e] = b * cs[e] + a * sn[e];
+          }
         }
+        if (!live) {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const float sn = low ? -s[e] : s[e];
-          x[e] = x[e] * c[e] + ox[e] * sn;
-          y[e] = y[e] * c[e] + oy[e] * sn;
+          for (int e = 0; e < 8; ++e) x[e] = y[e] = 0.f;
         }
+        uint8_t* dst = w ? sK : sQ;
+        rc_split8(x, dst + (d0 >> 6) * kRcV + rc_off(ut, (d0 >> 3) & 7), kRcQ);
+        rc_split8(y, dst + (d1 >> 6) * kRcV + rc_off(ut, (d1 >> 3) & 7), kRcQ);
       }
-      const uint32_t off = (ch >> 3) * kRcV + rc_off(t, ch & 7);
-      rc_split8(x, sQ + off, kRcQ);
-      rc_split8(y, sK + off, kRcQ);
-    }
-    // ---- v, v' ----
-    for (int i = tid; i < kRcTok * 8; i += kRcThreads) {
-      const int t = i >> 3, ch = i & 7;
-      float x[8];
-      rc_load8<T>(rv + t * kRcDv + ch * 8, x);
-      if (t >= nt) {
+      // ---- v, v' ----
+      {
+        if (!live) {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) x[e] = 0.f;
-      }
-      const uint32_t off = rc_off(t, ch);
-      if constexpr (VS == 1) {
-        *reinterpret_cast<uint4*>(sV + off) =
-            t < nt ? *reinterpret_cast<const uint4*>(rv + t * kRcDv + ch * 8) : make_uint4(0u, 0u, 0u, 0u);
-      } else {
+          for (int e = 0; e < 8; ++e) v8[e] = 0.f;
+        }
+        const uint32_t off = rc_off(ut, u);
         uint32_t hh[4], mm[4], ll;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) rc_split2(x[2 * e], x[2 * e + 1], hh[e], mm[e], ll);
+        for (int e = 0; e < 4; ++e) rc_split2(v8[2 * e], v8[2 * e + 1], hh[e], mm[e], ll);
         *reinterpret_cast<uint4*>(sV + off) = make_uint4(hh[0], hh[1], hh[2], hh[3]);
-        *reinterpret_cast<uint4*>(sV + kRcV + off) = make_uint4(mm[0], mm[1], mm[2], mm[3]);
-      }
-      const float f = pw[max(nt - 1 - t, 0)] * p.k_scale;
+        if constexpr (VS == 2) *reinterpret_cast<uint4*>(sV + kRcV + off) = make_uint4(mm[0], mm[1], mm[2], mm[3]);
+        const float f = pw[max(nt - 1 - ut, 0)] * p.k_scale;
 #pragma unroll
-      for (int e = 0; e < 8; ++e) x[e] *= f;
-      rc_split8(x, sW + off, kRcV);
+        for (int e = 0; e < 8; ++e) v8[e] *= f;
+        rc_split8(v8, sW + off, kRcV);
+      }
     }
     fence_proxy_async_smem();
     __syncthreads();
@@ -276,37 +278,35 @@ retention_chunked_kernel(const RetChunkParams p) {
     const uint32_t hi = static_cast<uint32_t>(dq >> 32), q_lo = static_cast<uint32_t>(dq);
     if (warp == 0 && elect_one()) {
       constexpr uint32_t id_qk = umma_idesc<__nv_bfloat16>(64, 64, 0, 0);
-      constexpr uint32_t id_qs = umma_idesc<__nv_bfloat16>(64, 64, 0, 1);
       constexpr uint32_t id_kv = umma_idesc<__nv_bfloat16>(128, 64, 1, 1);
+      constexpr uint32_t id_qs = umma_idesc<__nv_bfloat16>(64, 64, 0, 1);
       const uint32_t k_lo = static_cast<uint32_t>(umma_desc_sw128(smem_u32(sK), 16, 1024));
       const uint32_t s_lo = static_cast<uint32_t>(umma_desc_sw128(smem_u32(sS), 16, 1024));
+      // everything but the number of rotated steps is known at compile time: an addition or two per MMA
+      uint32_t acc = 0;
+#pragma unroll
+      for (int pr = 0; pr < 6; ++pr)
+#pragma unroll
+        for (int s = 0; s < kRcDk / 16; ++s)
+          if (pr == 5 || s < rot_steps) {
+            const uint32_t at = (s >> 2) * (kRcV >> 4) + (s & 3) * 2;
+            umma_ss_lo(tA, q_lo + rc_pa(pr) * (kRcQ >> 4) + at, k_lo + rc_pb(pr) * (kRcQ >> 4) + at, hi, id_qk, acc);
+            acc = 1;
+          }
+      acc = 0;
+#pragma unroll
+      for (int pr = 0; pr < 6; ++pr)
+#pragma unroll
+        for (int s = 0; s < kRcDk / 16; ++s)
+          if (rc_pa(pr) == 0 || s < rot_steps) {
+            umma_ss_lo(tO1, q_lo + rc_pa(pr) * (kRcQ >> 4) + (s >> 2) * (kRcV >> 4) + (s & 3) * 2,
+                       s_lo + rc_pb(pr) * (kRcS >> 4) + s * 128, hi, id_qs, acc);
+            acc = 1;
+          }
+      umma_commit(&bars[0]);
       const uint32_t km_lo = static_cast<uint32_t>(umma_desc_sw128(smem_u32(sK), kRcV, 1024));
       const uint32_t w_lo = static_cast<uint32_t>(umma_desc_sw128(smem_u32(sW), 16, 1024));
-      uint32_t acc = 0;
-#pragma unroll 1
-      for (int pr = 0; pr < 6; ++pr) {
-        const uint32_t a = q_lo + rc_pa(pr) * (kRcQ >> 4), b = k_lo + rc_pb(pr) * (kRcQ >> 4);
-        const int steps = pr == 5 ? kRcDk / 16 : rot_steps;
-#pragma unroll 1
-        for (int s = 0; s < steps; ++s) {
-          const uint32_t at = (s >> 2) * (kRcV >> 4) + (s & 3) * 2;
-          umma_ss_lo(tA, a + at, b + at, hi, id_qk, acc);
-          acc = 1;
-        }
-      }
-      acc = 0;
-#pragma unroll 1
-      for (int pr = 0; pr < 6; ++pr) {
-        const uint32_t a = q_lo + rc_pa(pr) * (kRcQ >> 4), b = s_lo + rc_pb(pr) * (kRcS >> 4);
-        const int steps = rc_pa(pr) == 0 ? kRcDk / 16 : rot_steps;
-#pragma unroll 1
-        for (int s = 0; s < steps; ++s) {
-          umma_ss_lo(tO1, a + (s >> 2) * (kRcV >> 4) + (s & 3) * 2, b + s * 128, hi, id_qs, acc);
-          acc = 1;
-        }
-      }
-      umma_commit(&bars[0]);
-#pragma unroll 1
+#pragma unroll
       for (int pr = 0; pr < 6; ++pr) {
         const uint32_t a = km_lo + rc_pa(pr) * (kRcQ >> 4), b = w_lo + rc_pb(pr) * (kRcV >> 4);
 #pragma unroll
@@ -315,16 +315,19 @@ retention_chunked_kernel(const RetChunkParams p) {
       umma_commit(&bars[1]);
     }
     __syncwarp();
-    if (t0 + nt < n) fetch(t0 + nt);
+    if (t0 + nt < n) {
+      fetch(t0 + nt);
+      angles(t0 + nt);
+    }
     // ---- A: decay, mask, split (over Q, which the MMAs have read) ----
-    mbar_wait_bounded(&bars[0], par, dead);
+    mbar_wait_bounded(&bars[0], par, dead);  // (by every warp: warp 0 is still handing in U's MMAs)
     tc_fence_after_sync();
     {
-      uint32_t a[16];
-      rc_ld_frag(tA + lane_base + (warp >> 2) * 32, a);
+      uint32_t a[8];
+      rc_ld_frag(tA + lane_base + (warp >> 2) * 16, a);
       tmem_ld_wait();
 #pragma unroll
-      for (int g = 0; g < 4; ++g)
+      for (int g = 0; g < 2; ++g)
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
           const int i = ar + 8 * x, j = ac + 8 * g;
@@ -346,7 +349,7 @@ retention_chunked_kernel(const RetChunkParams p) {
       constexpr uint32_t id_av = umma_idesc<__nv_bfloat16>(64, 64, 0, 1);
       const uint32_t v_lo = static_cast<uint32_t>(umma_desc_sw128(smem_u32(sV), 16, 1024));
       uint32_t acc = 0;
-#pragma unroll 1
+#pragma unroll
       for (int pr = 0; pr < 6; ++pr) {
         if (rc_pb(pr) >= VS) continue;
         const uint32_t a = q_lo + rc_pa(pr) * (kRcV >> 4), b = v_lo + rc_pb(pr) * (kRcV >> 4);
@@ -360,24 +363,24 @@ retention_chunked_kernel(const RetChunkParams p) {
     }
     __syncwarp();
     // ---- state ----
-    mbar_wait_bounded(&bars[1], par, dead);
+    rc_wait(&bars[1], par, warp, dead);
     tc_fence_after_sync();
     {
-      uint32_t u[32];
-      tmem_ld_32x32b_x32(tU + lane_base + sc, u);
+      uint32_t x[16];
+      tmem_ld_32x32b_x16(tU + lane_base + sc, x);
       tmem_ld_wait();
       const float dn = pw[nt];
 #pragma unroll
-      for (int i = 0; i < 32; ++i) S[i] = fmaf(dn, S[i], __uint_as_float(u[i]));
+      for (int i = 0; i < 16; ++i) S[i] = fmaf(dn, S[i], __uint_as_float(x[i]));
     }
     if (t0 + nt < n) put_state();
     // ---- outputs ----
-    mbar_wait_bounded(&bars[2], par, dead);
+    rc_wait(&bars[2], par, warp, dead);
     tc_fence_after_sync();
     {
-      uint32_t a[16], b[16];
-      rc_ld_frag(tO1 + lane_base + (warp >> 2) * 32, a);
-      rc_ld_frag(tO2 + lane_base + (warp >> 2) * 32, b);
+      uint32_t a[8], b[8];
+      rc_ld_frag(tO1 + lane_base + (warp >> 2) * 16, a);
+      rc_ld_frag(tO2 + lane_base + (warp >> 2) * 16, b);
       tmem_ld_wait();
       float* og = p.o + ((row0 + t0) * p.H + h) * static_cast<int64_t>(p.dv) + col0;
 #pragma unroll
@@ -387,7 +390,7 @@ retention_chunked_kernel(const RetChunkParams p) {
           const float f = pw[i + 1];
           float* dst = og + static_cast<int64_t>(i) * p.H * p.dv + ac;
 #pragma unroll
-          for (int g = 0; g < 4; ++g)
+          for (int g = 0; g < 2; ++g)
             *reinterpret_cast<float2*>(dst + 8 * g) =
                 make_float2(fmaf(f, __uint_as_float(a[4 * g + 2 * x]), __uint_as_float(b[4 * g + 2 * x])),
                             fmaf(f, __uint_as_float(a[4 * g + 2 * x + 1]), __uint_as_float(b[4 * g + 2 * x + 1])));
@@ -396,7 +399,7 @@ retention_chunked_kernel(const RetChunkParams p) {
     }
   }
 #pragma unroll
-  for (int i = 0; i < 32; i += 4) *reinterpret_cast<float4*>(st + i) = make_float4(S[i], S[i + 1], S[i + 2], S[i + 3]);
+  for (int i = 0; i < 16; i += 4) *reinterpret_cast<float4*>(st + i) = make_float4(S[i], S[i + 1], S[i + 2], S[i + 3]);
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 0) tmem_dealloc(*tmem_slot, 256);
@@ -423,7 +426,11 @@ int retention_chunked_try(float* o, const void* q, const void* k, const void* v,
                           const int64_t* req_pool_indices, const int32_t* prefix_lens, const int32_t* extend_lens,
                           const int32_t* extend_start_loc, int64_t batch, int H, int dk, int dv, int64_t q_stride,
                           int64_t k_stride, int64_t v_stride, const float* decay, const float* cos_sin, int rot,
-                          int64_t max_positions, float k_scale, int in_act, int dtype, cudaStream_t stream) {
+                          int64_t max_positions, float k_scale, int in_act, int dtype, int64_t total_tokens,
+                          cudaStream_t stream) {
+  // A chunk costs what some tens of tokens cost one by one, and its CTA takes a whole SM: 4 requests of 16 tokens 12.1 us
+  // (token by token) / 11.8, of 64 tokens 32.9 / 16; 16 requests of 16 tokens 30 / 41 us, of 40 tokens 63 / 41.
+  if (total_tokens <= 40 * batch) return 1;
   // 16-bit rows without an activation (their parts are what the split was counted for), 128 channels, whole 64-column
   // slices, a rotation in whole 16-byte pieces, 16-byte rows
   if (dtype == SPD_F32 || in_act != 0 || dk != kRcDk || dv % kRcDv != 0 || rot % 16 != 0) return 1;

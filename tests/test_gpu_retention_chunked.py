@@ -62,7 +62,8 @@ def _rel(a, b):
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("rot", [0, 16, 64, 128])
-@pytest.mark.parametrize("pre,ext", [([0], [1]), ([0, 5], [63, 64]), ([9, 0, 0], [65, 0, 130]), ([200], [300])])
+@pytest.mark.parametrize("pre,ext", [([0], [1]), ([7, 0, 30], [130, 1, 24]), ([0, 5], [63, 64]), ([9, 0, 0], [65, 0, 130]),
+                                     ([200], [300])])
 def test_portions(dtype, rot, pre, ext):
     H, dv = 3, 128
     a = _case(pre, ext, H, dv, rot, dtype, [0.97, 0.999, 0.875])
@@ -104,7 +105,7 @@ def test_strided_rows_and_a_cut_prompt():
     parts = (qkv[:, : H * DK], qkv[:, H * DK: 2 * H * DK], qkv[:, 2 * H * DK:])
     whole, ws = _run(*parts, state, table, decay, [0], [n], H, dv, 64, DK ** -0.5)
     got, st, at = [], state, 0
-    for m in (100, 1, n - 101):
+    for m in (100, 1, n - 101):  # (the single token goes through the token-by-token kernel)
         o, s = _run(*(x[at:at + m].contiguous() for x in parts), st.float(), table, decay, [at], [m], H, dv, 64, DK ** -0.5)
         got.append(o)
         st, at = s, at + m
