@@ -30,10 +30,12 @@
 // softmax is the lazily rescaled one of attn_decode.cu: scores are read from TMEM in the 16x256b fragment layout (all
 // 32 lanes of a warp busy although M = 64 fills 16 lanes per warp), P goes back as stmatrix-transposed K-major rows.
 //
-// Decode streams each latent row once: 64 requests of 1088 keys (83 MB) take 28 us, about 3000 clk per 72 KB tile and SM
+// Decode streams each latent row once: 64 requests of 1088 keys (83 MB) take 26 us, about 3000 clk per 72 KB tile and SM
 // (6.8 TB/s in the steady state) after 9000 clk until the first tile has landed; one CTA per token, head group and split
 // with warp-level MMAs took 54 us.  MMAs (M = 64: 23 clk at N = 16, 31 at N = 64) are hidden as long as the issuer's code
-// stays a short loop.
+// stays a short loop.  Extend, 4096 new tokens in 4 requests (two with 515 cached): 1496 -> 394 us; bounded by the ring of
+// two tiles (a tile's copies start when the PV before last has finished: 4400 clk a tile against 2000 of MMAs) and by
+// beginning and ending items, which therefore count in the split (without that, SMs with short items took 870 us).
 //
 // Every mbarrier wait is bounded: a wait that runs out marks the CTA dead, all later waits fall through, the kernel
 // finishes without waiting and counts itself in g_mla_wait_expired.
@@ -79,6 +81,7 @@ template <bool kExtend>
 struct MlaShape {
   static constexpr int TQ = kExtend ? 4 : 1;
   static constexpr int N = TQ * kMlaHeads;
+  static constexpr int E = kExtend ? 2 : 1;  // what beginning and ending an item costs, in tiles: it counts in the work split
   static constexpr int kQBytes = 9 * N * 128;
   static constexpr int kPBytes = N * 128;
   static constexpr int kPairs = kExtend ? 8 : 11;  // ring slots of 16 KB: one pair of 64-column blocks of a tile
@@ -155,15 +158,17 @@ __device__ __forceinline__ int mla_group_tiles(int prefix, int n) {
   const int u = (prefix + 63) >> 2;
   return mla_floor16_sum(n + u) - mla_floor16_sum(u);
 }
+// units of a request in the work list: the tiles of its items, and E for each item (in front of its tiles)
 template <bool kExtend>
 __device__ __forceinline__ int mla_request_tiles(const MlaParams& p, int r) {
   if constexpr (kExtend) {
     int start, ext, prefix;
     mla_request(p, r, start, ext, prefix);
     if (ext <= 0) return 0;
-    return mla_group_tiles(prefix, ext / 4) + (ext % 4 ? (prefix + ext + kMlaTile - 1) / kMlaTile : 0);
+    return mla_group_tiles(prefix, ext / 4) + (ext % 4 ? (prefix + ext + kMlaTile - 1) / kMlaTile : 0) +
+           (ext + 3) / 4 * MlaShape<true>::E;
   } else {
-    return max(1, (static_cast<int>(p.seq_lens[r]) + kMlaTile - 1) / kMlaTile);
+    return max(1, (static_cast<int>(p.seq_lens[r]) + kMlaTile - 1) / kMlaTile) + MlaShape<false>::E;
   }
 }
 
@@ -193,24 +198,32 @@ __device__ __forceinline__ void mla_next_item(const MlaParams& p, MlaItem& it) {
 // walks the CTA's tiles: every role keeps its own copy
 template <bool kExtend>
 struct MlaCursor {
+  static constexpr int E = MlaShape<kExtend>::E;
   MlaItem it;
-  int tile, left, seg;  // left: tiles of the CTA's range that remain; seg: items left behind so far
+  int tile, left, seg;  // left: units of the CTA's range that remain, from this tile on; seg: items left behind so far
   bool valid;
   __device__ __forceinline__ void init(const MlaParams& p, const int* start, int count) {
     it.hg = start[0];
     it.r = start[1];
     it.j = start[2];
-    tile = start[3];
+    const int at = start[3];  // units of the item before the range
     left = count;
-    seg = 0;
+    seg = tile = 0;
     valid = left > 0;
     if (!valid) return;
     mla_set_item<kExtend>(p, it);
-    if (p.snap && tile > 0) {  // the item belongs to the CTA before
-      left -= it.ntiles - tile;
-      tile = 0;
+    if (p.snap) {  // an item belongs to the CTA whose range holds its first unit
+      if (at > 0) {
+        left -= it.ntiles + E - at;
+        valid = left > 0;
+        if (valid) mla_next_item<kExtend>(p, it);
+      }
+      left -= E;
+    } else if (at <= E) {
+      left -= E - at;
       valid = left > 0;
-      if (valid) mla_next_item<kExtend>(p, it);
+    } else {
+      tile = at - E;
     }
   }
   // whether this tile is the last of its item here
@@ -226,7 +239,8 @@ struct MlaCursor {
     }
     ++seg;
     tile = 0;
-    valid = left > 0;
+    valid = p.snap ? left > 0 : left > E;
+    left -= E;
     if (valid) mla_next_item<kExtend>(p, it);
   }
 };
@@ -312,7 +326,7 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
   uint64_t* q_empty = p_full + 4;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(p_full + 5);
   volatile int* dead = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  int* s_start = reinterpret_cast<int*>(tmem_slot + 2);  // hg, r, j, tile
+  int* s_start = reinterpret_cast<int*>(tmem_slot + 2);  // hg, r, j, units of the item before the range
   volatile int* s_gath = s_start + 4;                    // [4]: whether tile t & 3 was gathered
   int* s_slot = s_start + 8;                             // [64] slots of a gathered tile
   float* red = reinterpret_cast<float*>(s_slot + 64);    // [4][N]
@@ -382,13 +396,13 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
       if constexpr (kExtend) {
         int start, ext, prefix;
         mla_request(p, r, start, ext, prefix);
-        int lo = 0, hi = (ext - 1) / TQ;  // last group that starts at or before tile `rem`
+        int lo = 0, hi = (ext - 1) / TQ;  // last group that starts at or before unit `rem`
         while (lo < hi) {
           const int mid = (lo + hi + 1) >> 1;
-          if (mla_group_tiles(prefix, mid) <= rem) lo = mid; else hi = mid - 1;
+          if (mla_group_tiles(prefix, mid) + mid * S::E <= rem) lo = mid; else hi = mid - 1;
         }
         j = lo;
-        rem -= mla_group_tiles(prefix, j);
+        rem -= mla_group_tiles(prefix, j) + j * S::E;
       }
       s_start[0] = hg;
       s_start[1] = r;
@@ -587,7 +601,7 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
       const bool tail = t_count > 0 && c.tile > 0 && c.it.ntiles - c.tile <= t_count;
       info[0] = tail;
       if (tail) {
-        info[1] = (t_begin - c.tile) / per;  // CTA of the item's first tile
+        info[1] = (t_begin - c.tile) / per;  // CTA of the item's first tile (tiles are consecutive units)
         info[2] = c.it.row0;
         info[3] = c.it.ntok;
         info[4] = c.it.hg * kMlaHeads;
@@ -725,29 +739,48 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
       mbar_wait_bounded(p_empty, (t - 1) & 1, dead);  // the last PV of the item has finished
       tc_fence_after_sync();
       T* out = reinterpret_cast<T*>(p.out) + it.row0 * p.out_stride + static_cast<int64_t>(h0) * kMlaDV + warp * 32;
+      if (whole) {
+        // neighbouring lanes swap halves of two columns: 4-byte stores, 64 bytes of a row per half warp
+        const bool odd = lane & 1;
+        T* dst = out + (lane & ~1) + (odd ? kMlaDV : 0);
 #pragma unroll 1
-      for (int blk = 0; blk < 4; ++blk) {
-#pragma unroll 1
-        for (int cc = 0; cc < N; cc += 16) {
-          uint32_t o[16];
-          tmem_ld_32x32b_x16(tmem_O + lane_base + blk * N + cc, o);
-          tmem_ld_wait();
-          const int tok = cc >> 4;
-          if (whole) {
-            // neighbouring lanes swap halves of two columns: 4-byte stores, 64 bytes of a row per half warp
+        for (int blk = 0; blk < 4; ++blk, dst += 128) {
+          uint32_t o[N];
 #pragma unroll
-            for (int e = 0; e < 16; e += 2) {
-              const float v0 = __uint_as_float(o[e]) * s_col[cc + e], v1 = __uint_as_float(o[e + 1]) * s_col[cc + e + 1];
-              const float got = __shfl_xor_sync(0xffffffffu, (lane & 1) ? v0 : v1, 1);
-              const int h = e + (lane & 1);
-              const uint32_t w = (lane & 1) ? pack2<T>(got, v1) : pack2<T>(v0, got);
-              if (tok < it.ntok && h < nh)
-                *reinterpret_cast<uint32_t*>(out + tok * p.out_stride + h * kMlaDV + blk * 128 + (lane & ~1)) = w;
+          for (int cc = 0; cc < N; cc += 16) tmem_ld_32x32b_x16(tmem_O + lane_base + blk * N + cc, o + cc);
+          tmem_ld_wait();
+#pragma unroll
+          for (int cc = 0; cc < N; cc += 16) {
+            if ((cc >> 4) >= it.ntok) break;
+            T* row = dst + (cc >> 4) * p.out_stride;
+#pragma unroll
+            for (int e = 0; e < 16; e += 4) {
+              const float4 f = *reinterpret_cast<const float4*>(s_col + cc + e);
+              const float a0 = __uint_as_float(o[cc + e]) * f.x, a1 = __uint_as_float(o[cc + e + 1]) * f.y;
+              const float b0 = __uint_as_float(o[cc + e + 2]) * f.z, b1 = __uint_as_float(o[cc + e + 3]) * f.w;
+              const float ga = __shfl_xor_sync(0xffffffffu, odd ? a0 : a1, 1);
+              const float gb = __shfl_xor_sync(0xffffffffu, odd ? b0 : b1, 1);
+              if (e + odd < nh) *reinterpret_cast<uint32_t*>(row + e * kMlaDV) = odd ? pack2<T>(ga, a1) : pack2<T>(a0, ga);
+              if (e + 2 + odd < nh)
+                *reinterpret_cast<uint32_t*>(row + (e + 2) * kMlaDV) = odd ? pack2<T>(gb, b1) : pack2<T>(b0, gb);
             }
-          } else if (tok < it.ntok) {
+          }
+        }
+      } else {
+        float* dst = p.o_part + part0 * kMlaDV + warp * 32 + lane;
+#pragma unroll 1
+        for (int blk = 0; blk < 4; ++blk, dst += 128) {
+          uint32_t o[N];
+#pragma unroll
+          for (int cc = 0; cc < N; cc += 16) tmem_ld_32x32b_x16(tmem_O + lane_base + blk * N + cc, o + cc);
+          tmem_ld_wait();
+#pragma unroll
+          for (int cc = 0; cc < N; cc += 16) {
+            if ((cc >> 4) >= it.ntok) break;
+            float* row = dst + static_cast<int64_t>((cc >> 4) * nhm) * kMlaDV;
 #pragma unroll
             for (int e = 0; e < 16; ++e)
-              if (e < nh) p.o_part[(part0 + tok * nhm + e) * kMlaDV + blk * 128 + warp * 32 + lane] = __uint_as_float(o[e]);
+              if (e < nh) row[e * kMlaDV] = __uint_as_float(o[cc + e]);
           }
         }
       }
