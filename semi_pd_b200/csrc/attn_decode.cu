@@ -11,11 +11,13 @@
 // the tensor core; the 16-wide N makes the MMAs ~60 cycles per 64 KB tile — the kernel's only
 // real cost is the stream itself.
 //
-// grid = #SMs (or the partition's SM budget); each CTA walks work items (request, kv head,
-// kv split) with a static stride and keeps its TMEM, barriers and the 3-stage K/V ring alive
-// across items, so the gather of the next item overlaps the epilogue of the current one.
-// Splits (only used when request x kv-head pairs do not fill the SMs) are merged by the
-// last-arriving CTA of a pair — no host plan, no second launch, CUDA-graph safe.
+// grid = #SMs (or the partition's SM budget).  Work items (request, kv head) are dealt to the CTAs with a static stride, or,
+// where that would leave SMs idle, cut: their 128-token tiles, one after another and with one more unit per item for its
+// epilogue, are one list that the CTAs share in equal contiguous ranges.  Lengths are read on the device.  A CTA keeps its TMEM, barriers and the 3-stage K/V ring alive across items, so the gather of the
+// next item overlaps the epilogue of the current one.  The parts of an item that was cut are merged by the last-arriving
+// of its CTAs — no host plan, no second launch, CUDA-graph safe.  (A fixed number of splits per
+// item, for the SMs to be covered, took two rounds for the 160 splits of 5 requests x 8 heads: 7000 tokens each 52 us, 36
+// as ranges; one request of 1000 tokens 19.3 / 13.9 us.)
 //
 // Softmax without per-tile reductions: every thread owns one kv token of the tile (a TMEM lane of
 // S^T).  All threads exponentiate against a shared REFERENCE max m_ref that is only raised when
@@ -57,8 +59,9 @@ constexpr int kDcLenCache = 1024;         // seq_lens cached in smem
 constexpr int kDcQBufs = 4;  // Q staging buffers: item i uses i % 4 (see the loader)
 constexpr int kDcMisc = 1024 + kDcLenCache * 4;
 constexpr int kDcSmem = kDcStages * 2 * kDcTileBytes + (kDcQBufs + 2) * kDcQBytes + 1024 + kDcMisc;
-constexpr int kDcMaxSplits = 32;
 constexpr int kDcMaxGroup = 8;
+constexpr int kDcItemUnits = 1;   // what an item's epilogue costs, in tiles: it counts in the work split
+constexpr int kDcMinUnits = 2;    // a share shorter than two tiles costs more in merge traffic than it saves in streaming
 constexpr float kDcRescale = 8.0f;  // log2 units a score may exceed m_ref before it is raised
 
 struct DecodeParams {
@@ -69,65 +72,84 @@ struct DecodeParams {
   const int32_t* req_to_token;
   const int64_t* req_pool_indices;
   const int64_t* seq_lens;
-  int batch, Hq, Hk, splits;
+  int batch, Hq, Hk;
+  float idle;      // share of the SMs' time that whole items leave unused, per unit (0: none may be cut, or nothing is gained)
   int64_t q_stride, out_stride, rtt_stride;
   float scale_log2;
-  float* o_part;   // [b][Hq][splits][D]
-  float* ml_part;  // [b][Hq][splits][2]
+  float* o_part;   // [2 * grid][G][D]: a CTA's part of an item begun earlier, then of one that goes on
+  float* ml_part;  // [2 * grid][G][2]
   int* counters;   // [b][Hk]
   int use_tma;     // 0: always gather (SPD_ATTN_TMA=0)
 };
 
-struct DcItem {
-  int b, hk, split, t0, t1, n_tiles, n_ne;  // n_ne: non-empty splits of this (request, kv head)
-};
-
-__device__ __forceinline__ DcItem dc_item(const DecodeParams& p, const int* s_len, int w) {
-  DcItem it;
-  it.split = w % p.splits;
-  const int r = w / p.splits;
-  it.hk = r % p.Hk;
-  it.b = r / p.Hk;
-  const int L = it.b < kDcLenCache ? s_len[it.b] : static_cast<int>(p.seq_lens[it.b]);
-  int per = (L + p.splits - 1) / p.splits;
-  per = (per + kDcTile - 1) / kDcTile * kDcTile;
-  // a split shorter than two tiles costs more in merge traffic than it saves in streaming time:
-  // short sequences therefore use fewer (non-empty) splits than the launch provides
-  if (p.splits > 1) per = max(per, 2 * kDcTile);
-  it.n_ne = (L + per - 1) / per;
-  it.t0 = it.split * per;
-  it.t1 = min(L, it.t0 + per);
-  it.n_tiles = it.t1 > it.t0 ? (it.t1 - it.t0 + kDcTile - 1) / kDcTile : 0;
-  return it;
+__device__ __forceinline__ int dc_len(const DecodeParams& p, const int* s_len, int b) {
+  return b < kDcLenCache ? s_len[b] : static_cast<int>(p.seq_lens[b]);
 }
+__device__ __forceinline__ int dc_tiles(int L) { return max(1, (L + kDcTile - 1) / kDcTile); }
 
-// walks the CTA's global tile sequence: (item, tile within item).  `iter` counts NON-EMPTY items
-// only: it selects the Q / O double buffers, and consecutive non-empty items must alternate.
+// walks the CTA's tiles; every role keeps its own copy.  `iter` counts the items left behind: it selects the Q / O
+// double buffers.
 struct DcCursor {
-  int w, iter, j;
-  DcItem item;
-  bool valid;
-  __device__ __forceinline__ void init(const DecodeParams& p, const int* s_len, int total) {
-    w = blockIdx.x;
-    iter = 0;
-    j = 0;
-    settle(p, s_len, total);
+  int b, hk, L, n;             // the item, its length and tiles
+  int tile, tile0, left, iter;  // tile0: this CTA's first tile of the item; left: units of the range from this tile on
+  bool valid, whole;            // whole: items dealt with a static stride instead of a range
+  __device__ __forceinline__ void set(const DecodeParams& p, const int* s_len) {
+    L = dc_len(p, s_len, b);
+    n = dc_tiles(L);
   }
-  __device__ __forceinline__ void settle(const DecodeParams& p, const int* s_len, int total) {
-    valid = false;
-    while (w < total) {
-      item = dc_item(p, s_len, w);
-      if (item.n_tiles > 0) { valid = true; return; }
-      w += gridDim.x;  // empty items carry no tiles (the softmax warps still publish them)
-    }
+  __device__ __forceinline__ void init_whole(const DecodeParams& p, const int* s_len) {
+    whole = true;
+    left = 0;
+    iter = tile = tile0 = 0;
+    b = static_cast<int>(blockIdx.x) / p.Hk;
+    hk = static_cast<int>(blockIdx.x) - b * p.Hk;
+    valid = b < p.batch;
+    if (valid) set(p, s_len);
   }
-  __device__ __forceinline__ void next(const DecodeParams& p, const int* s_len, int total) {
-    if (++j >= item.n_tiles) {
-      j = 0;
-      w += gridDim.x;
-      ++iter;
-      settle(p, s_len, total);
+  __device__ __forceinline__ void init_range(const DecodeParams& p, const int* s_len, const int* start, int count) {
+    whole = false;
+    b = start[0];
+    hk = start[1];
+    const int at = start[2];  // units of the item before the range
+    left = count;
+    iter = tile = 0;
+    valid = left > 0;
+    if (valid) {
+      set(p, s_len);
+      if (at <= kDcItemUnits) {
+        left -= kDcItemUnits - at;
+        valid = left > 0;
+      } else {
+        tile = at - kDcItemUnits;
+      }
     }
+    tile0 = tile;
+  }
+  // whether this tile is the last of its item here
+  __device__ __forceinline__ bool ends() const { return tile + 1 == n || (!whole && left == 1); }
+  __device__ __forceinline__ void next(const DecodeParams& p, const int* s_len) {
+    const bool e = ends();
+    --left;
+    if (!e) {
+      ++tile;
+      return;
+    }
+    ++iter;
+    tile = tile0 = 0;
+    if (whole) {
+      const int w = b * p.Hk + hk + static_cast<int>(gridDim.x);
+      b = w / p.Hk;
+      hk = w - b * p.Hk;
+      valid = b < p.batch;
+    } else {
+      valid = left > kDcItemUnits;
+      left -= kDcItemUnits;
+      if (++hk == p.Hk) {
+        hk = 0;
+        ++b;
+      }
+    }
+    if (valid) set(p, s_len);
   }
 };
 
@@ -205,11 +227,11 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
   int* flag_slot = reinterpret_cast<int*>(tmem_slot + 1);
   float* red = reinterpret_cast<float*>(misc + 256);   // [4 warps][8 heads] scratch (+ 8 totals)
   int* s_len = reinterpret_cast<int*>(misc + 1024);    // seq_lens[0 .. kDcLenCache)
+  int* s_scan = reinterpret_cast<int*>(misc + 512);    // [9] warps' units; then the range's start: request, kv head, units before
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int G = p.Hq / p.Hk;
-  const int total = p.batch * p.Hk * p.splits;
 
   if (warp == 8) {
     if (lane == 0) {
@@ -245,11 +267,62 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
   // moment the previous GEMM's CTA leaves it and stream its weights under this kernel.
   griddep_launch_dependents();
   griddep_wait();
-  for (int i = threadIdx.x; i < min(p.batch, kDcLenCache); i += kDcThreads)
-    s_len[i] = static_cast<int>(p.seq_lens[i]);
+  // this CTA's range of the work list: thread t counts the units of requests [b0, b1)
+  const int per_thread = (p.batch + kDcThreads - 1) / kDcThreads;
+  const int b0 = threadIdx.x * per_thread, b1 = min(p.batch, b0 + per_thread);
+  int sum = 0;
+  for (int b = b0; b < b1; ++b) {
+    const int L = static_cast<int>(p.seq_lens[b]);
+    if (b < kDcLenCache) s_len[b] = L;
+    sum += (dc_tiles(L) + kDcItemUnits) * p.Hk;
+  }
+  const int warp_units = __reduce_add_sync(0xffffffffu, sum);
+  if (lane == 0) s_scan[warp] = warp_units;
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  const int cta = static_cast<int>(blockIdx.x);
+  int total = 0;
+#pragma unroll
+  for (int w = 0; w < kDcThreads / 32; ++w) total += s_scan[w];
+  // Whole items leave SMs idle for what the last round of the stride lacks.  A cut costs two partial epilogues and a merge
+  // per CTA, about five tiles' time in all: it pays where that idle time is longer (or where there are fewer items than
+  // SMs).  20 requests x 8 heads on 148 SMs: 400 tokens 12.6 us whole / 15.5 cut, 1000 21.4 / 21.5, 3000 67 / 45.
+  const bool whole = p.idle * static_cast<float>(total) < 5.f;
+  int per = 1, u_begin = 0, u_end = 0;
+  if (!whole) {
+    int incl = sum, before = 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+#pragma unroll
+    for (int w = 0; w < kDcThreads / 32; ++w)
+      if (w < warp) before += s_scan[w];
+    per = max(kDcMinUnits, (total + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x));
+    u_begin = min(total, per * cta);
+    u_end = min(total, u_begin + per);
+    int rem = u_begin - (before + incl - sum);
+    if (u_begin < u_end && rem >= 0 && rem < sum) {  // exactly one thread: the range starts in its requests
+      int b = b0;
+      for (;; ++b) {
+        const int w = (dc_tiles(dc_len(p, s_len, b)) + kDcItemUnits) * p.Hk;
+        if (rem < w) break;
+        rem -= w;
+      }
+      const int w = dc_tiles(dc_len(p, s_len, b)) + kDcItemUnits;
+      s_scan[16] = b;
+      s_scan[17] = rem / w;
+      s_scan[18] = rem % w;
+    }
+    __syncthreads();
+  }
+  DcCursor c;
+  if (whole)
+    c.init_whole(p, s_len);
+  else
+    c.init_range(p, s_len, s_scan + 16, u_end - u_begin);
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tmem_S = tmem_base;        // 2 x 16 columns
   const uint32_t tmem_O = tmem_base + 32;   // 2 x 16 columns
@@ -259,9 +332,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     if (elect_one()) {
       constexpr uint32_t idesc_s = umma_idesc<T>(128, kDcN, 0, 0);  // A = K (K-major), B = Q (K-major)
       constexpr uint32_t idesc_o = umma_idesc<T>(128, kDcN, 1, 0);  // A = V (MN-major), B = P^T (K-major)
-      DcCursor cs, cp;  // cs runs one tile ahead of cp
-      cs.init(p, s_len, total);
-      cp.init(p, s_len, total);
+      DcCursor cs = c, cp = c;  // cs runs one tile ahead of cp
       int ts = 0;  // global tile counter of the S stream
       auto issue_s = [&]() {
         const int st = ts % kDcStages, sb = ts & 1;
@@ -281,7 +352,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
         umma_commit(&k_empty[st]);  // K_t: consumed once these MMAs have read it
         umma_commit(&s_full[sb]);
         ++ts;
-        cs.next(p, s_len, total);
+        cs.next(p, s_len);
       };
       if (cs.valid) issue_s();
       int tp = 0;  // global tile counter of the PV stream
@@ -292,7 +363,8 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
         mbar_wait(&p_full[pb], (tp >> 1) & 1);
         mbar_wait(&v_full[st], (tp / kDcStages) & 1);
         fence_proxy_async_smem();
-        if (cp.j == 0) {
+        const bool first = cp.tile == cp.tile0;
+        if (first) {
           mbar_wait(&o_empty[ob], (o_uses[ob] & 1) ^ 1);
           ++o_uses[ob];
         }
@@ -303,13 +375,13 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
         for (int k = 0; k < kDcTile / 16; ++k) {
           umma_ss(tmem_O + ob * kDcN, umma_desc_sw128(v_addr + k * 2048, 16384, 1024),
                   umma_desc_sw128(p_addr + (k >> 2) * 2048 + (k & 3) * 32, 16, 1024), idesc_o,
-                  (cp.j > 0 || k > 0) ? 1u : 0u);
+                  (!first || k > 0) ? 1u : 0u);
         }
         umma_commit(&v_empty[st]);
         umma_commit(&p_empty[pb]);
         umma_commit(o_done);
         ++tp;
-        cp.next(p, s_len, total);
+        cp.next(p, s_len);
       }
     }
   } else if (warp >= 4) {
@@ -326,23 +398,20 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     uint64_t* full = is_v ? v_full : k_full;
     uint64_t* empty = is_v ? v_empty : k_empty;
     const int64_t row_elems = static_cast<int64_t>(p.Hk) * kDcD;
-    DcCursor c;
-    c.init(p, s_len, total);
     int t = 0;
     // Page-table lookups run ONE TILE AHEAD of the gather (32 slots per thread), so the dependent
     // chain req_pool_indices -> req_to_token -> pool row is off the issue path.
     // `base` = slot of the tile's first row when the tile is FULL (else -1): the candidate TMA row.
     auto lookup = [&](const DcCursor& cc, int* sl, int& base) {
-      const DcItem& it = cc.item;
-      const int32_t* rtt0 = p.req_to_token + p.req_pool_indices[it.b] * p.rtt_stride;
-      const int tile0 = it.t0 + cc.j * kDcTile;
+      const int32_t* rtt0 = p.req_to_token + p.req_pool_indices[cc.b] * p.rtt_stride;
+      const int tile0 = cc.tile * kDcTile;
       const int tokb = tile0 + rsub;
 #pragma unroll
       for (int i = 0; i < 32; ++i) {
         const int tok = tokb + i * 4;
-        sl[i] = tok < it.t1 ? __ldg(rtt0 + tok) : -1;
+        sl[i] = tok < cc.L ? __ldg(rtt0 + tok) : -1;
       }
-      base = (p.use_tma && tile0 + kDcTile <= it.t1) ? __ldg(rtt0 + tile0) : -1;
+      base = (p.use_tma && tile0 + kDcTile <= cc.L) ? __ldg(rtt0 + tile0) : -1;
     };
     const CUtensorMap* tmap = is_v ? &tmV : &tmK;
     if (lt == 0) tma_prefetch_desc(tmap);
@@ -350,8 +419,9 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     if (c.valid) lookup(c, slot, base);
     while (c.valid) {
       const int st = t % kDcStages;
-      const int b = c.item.b, hk = c.item.hk, cj = c.j, citer = c.iter;
-      c.next(p, s_len, total);
+      const int b = c.b, hk = c.hk, citer = c.iter;
+      const bool load_q = c.tile == c.tile0;
+      c.next(p, s_len);
       int nslot[32], nbase = -1;
       if (c.valid) lookup(c, nslot, nbase);
       // Are the tile's 128 page-table entries consecutive slots?  Each thread checks its 32 rows
@@ -361,7 +431,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
       for (int i = 0; i < 32; ++i) contig &= (slot[i] == base + i * 4 + rsub);
       if (p.use_tma) contig = loader_bar_and(contig, is_v);
       mbar_wait(&empty[st], ((t / kDcStages) & 1) ^ 1);
-      if (!is_v && cj == 0) {
+      if (!is_v && load_q) {
         // stage the G query rows of this (request, kv head) as the K-major B operand, in the same
         // cp.async group as the K tile.  Buffer citer % 4 was last read by the S MMAs of item
         // citer - 4, whose tiles are all older than tile t-3 — complete once k_empty[st] fired.
@@ -408,15 +478,18 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     // ===================== softmax / correction / epilogue =====================
     const int tid = threadIdx.x;  // TMEM lane: kv token within tile (S^T) or head-dim index (O^T)
     const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
-    int t = 0;     // global tile counter
-    int iter = 0;  // non-empty items seen so far (same convention as DcCursor::iter)
-    for (int w = blockIdx.x; w < total; w += gridDim.x) {
-      const DcItem it = dc_item(p, s_len, w);
+    int t = 0;  // global tile counter
+    while (c.valid) {
+      const int ib = c.b, ihk = c.hk, L = c.L, n = c.n, tile0 = c.tile0, ob = c.iter & 1;
+      const int unit0 = u_end - c.left - c.tile;  // unit of the item's tile 0
       float m_ref[kDcMaxGroup], l_thr[kDcMaxGroup];
 #pragma unroll
-      for (int g = 0; g < kDcMaxGroup; ++g) { m_ref[g] = -INFINITY; l_thr[g] = 0.f; }
-      const int ob = iter & 1;
-      for (int j = 0; j < it.n_tiles; ++j, ++t) {
+      for (int g = 0; g < kDcMaxGroup; ++g) { m_ref[g] = L > 0 ? -INFINITY : 0.f; l_thr[g] = 0.f; }
+      int tile = tile0;
+      for (bool end = false; !end; ++t) {
+        end = c.ends();
+        tile = c.tile;
+        c.next(p, s_len);
         const int sb = t & 1;
         mbar_wait(&s_full[sb], (t >> 1) & 1);
         tc_fence_after_sync();
@@ -426,7 +499,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(&s_empty[sb]);
-        const bool valid = (it.t0 + j * kDcTile + tid) < it.t1;
+        const bool valid = tile * kDcTile + tid < L;
         float s[kDcMaxGroup];
         bool exceed = false;
 #pragma unroll
@@ -452,7 +525,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
             l_thr[g] *= alpha[g];
             m_ref[g] = m_new;
           }
-          if (j > 0) {
+          if (tile > tile0) {
             // O^T stable once PV_{t-1} is complete.  That completion is observed on p_empty (committed
             // with every PV): this thread waited for the PREVIOUS phase of that barrier at tile t-1,
             // so the parity wait cannot alias — a per-PV barrier that is only waited on now and then
@@ -496,7 +569,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
 #pragma unroll
       for (int g = 0; g < kDcMaxGroup; ++g)
         l_tot[g] = (red[g] + red[8 + g]) + (red[16 + g] + red[24 + g]);
-      if (it.n_tiles > 0) {
+      {
         mbar_wait(&p_empty[(t - 1) & 1], ((t - 1) >> 1) & 1);  // last PV of the item complete
         tc_fence_after_sync();
         uint32_t r[16];
@@ -507,62 +580,56 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
         if (lane == 0) mbar_arrive(&o_empty[ob]);
 #pragma unroll
         for (int g = 0; g < kDcMaxGroup; ++g) o[g] = __uint_as_float(r[g]);
-        ++iter;
-      } else {
-#pragma unroll
-        for (int g = 0; g < kDcMaxGroup; ++g) o[g] = 0.f;
       }
-      if (p.splits == 1) {
-        T* dst = reinterpret_cast<T*>(p.out) + it.b * p.out_stride +
-                 static_cast<int64_t>(it.hk) * G * kDcD + tid;
+      if (tile0 == 0 && tile + 1 == n) {
+        T* dst = reinterpret_cast<T*>(p.out) + ib * p.out_stride + static_cast<int64_t>(ihk) * G * kDcD + tid;
 #pragma unroll
         for (int g = 0; g < kDcMaxGroup; ++g)
           if (g < G) dst[g * kDcD] = from_f32<T>(l_tot[g] > 0.f ? o[g] / l_tot[g] : 0.f);
         softmax_bar();  // `red` is rewritten by the next item
       } else {
+        const int64_t part = static_cast<int64_t>(2 * cta + (tile0 > 0 ? 0 : 1)) * G;
 #pragma unroll
         for (int g = 0; g < kDcMaxGroup; ++g)
-          if (g < G && it.n_tiles > 0) {
-            const int64_t idx = (static_cast<int64_t>(it.b) * p.Hq + it.hk * G + g) * p.splits + it.split;
-            p.o_part[idx * kDcD + tid] = o[g];
-            if (tid == 0) { p.ml_part[idx * 2] = m_ref[g]; p.ml_part[idx * 2 + 1] = l_tot[g]; }
+          if (g < G) {
+            p.o_part[(part + g) * kDcD + tid] = o[g];
+            if (tid == 0) { p.ml_part[(part + g) * 2] = m_ref[g]; p.ml_part[(part + g) * 2 + 1] = l_tot[g]; }
           }
+        const int c0 = unit0 / per, c1 = (unit0 + n - 1) / per;  // the CTAs that share the item
         __threadfence();
         softmax_bar();
-        if (tid == 0) *flag_slot = atomicAdd(&p.counters[it.b * p.Hk + it.hk], 1);
+        if (tid == 0) *flag_slot = atomicAdd(&p.counters[ib * p.Hk + ihk], 1);
         softmax_bar();
-        if (*flag_slot == p.splits - 1) {
-          // last split of this (request, kv head): merge the non-empty partials in split order,
-          // all heads of the group at once so the loads of one split are independent
+        if (*flag_slot == c1 - c0) {
+          // last of them: merge the parts in order, all heads of the group at once so the loads of one part are
+          // independent
           __threadfence();
-          const int64_t base0 = (static_cast<int64_t>(it.b) * p.Hq + it.hk * G) * p.splits;
+          auto at = [&](int i) { return static_cast<int64_t>(i == c0 ? 2 * i + 1 : 2 * i) * G; };
           float M[kDcMaxGroup], num[kDcMaxGroup], den[kDcMaxGroup];
 #pragma unroll
           for (int g = 0; g < kDcMaxGroup; ++g) { M[g] = -INFINITY; num[g] = 0.f; den[g] = 0.f; }
 #pragma unroll 2
-          for (int s2 = 0; s2 < it.n_ne; ++s2)
+          for (int i = c0; i <= c1; ++i)
 #pragma unroll
             for (int g = 0; g < kDcMaxGroup; ++g)
-              if (g < G) M[g] = fmaxf(M[g], __ldcg(&p.ml_part[(base0 + g * p.splits + s2) * 2]));
+              if (g < G) M[g] = fmaxf(M[g], __ldcg(&p.ml_part[(at(i) + g) * 2]));
 #pragma unroll 2
-          for (int s2 = 0; s2 < it.n_ne; ++s2) {
+          for (int i = c0; i <= c1; ++i) {
 #pragma unroll
             for (int g = 0; g < kDcMaxGroup; ++g)
               if (g < G) {
-                const int64_t idx = base0 + g * p.splits + s2;
-                const float2 ml = __ldcg(reinterpret_cast<const float2*>(&p.ml_part[idx * 2]));
-                const float ov = __ldcg(&p.o_part[idx * kDcD + tid]);
+                const float2 ml = __ldcg(reinterpret_cast<const float2*>(&p.ml_part[(at(i) + g) * 2]));
+                const float ov = __ldcg(&p.o_part[(at(i) + g) * kDcD + tid]);
                 const float wgt = ml.y > 0.f ? fast_exp2(ml.x - M[g]) : 0.f;
                 num[g] += wgt * ov;
                 den[g] += wgt * ml.y;
               }
           }
-          T* dst = reinterpret_cast<T*>(p.out) + it.b * p.out_stride +
-                   static_cast<int64_t>(it.hk) * G * kDcD + tid;
+          T* dst = reinterpret_cast<T*>(p.out) + ib * p.out_stride + static_cast<int64_t>(ihk) * G * kDcD + tid;
 #pragma unroll
           for (int g = 0; g < kDcMaxGroup; ++g)
             if (g < G) dst[g * kDcD] = from_f32<T>(den[g] > 0.f ? num[g] / den[g] : 0.f);
-          if (tid == 0) p.counters[it.b * p.Hk + it.hk] = 0;  // re-arm for the next launch
+          if (tid == 0) p.counters[ib * p.Hk + ihk] = 0;  // re-arm for the next launch
         }
         softmax_bar();  // flag_slot / red are reused by the next item
       }
@@ -613,24 +680,28 @@ extern "C" int spd_attn_decode_paged(void* out, const void* q, const void* k_poo
   p.out_stride = out_stride;
   p.rtt_stride = req_to_token_stride;
   p.scale_log2 = sm_scale * 1.4426950408889634f;
-  // KV splits only when the (request, kv head) pairs cannot fill the SMs; the choice depends on
-  // the launch shape alone (lengths are device-side) — nothing to plan on the host per step.
   const int64_t pairs = batch * num_kv_heads;
-  int splits = 1;
-  if (pairs < sms) {
-    splits = static_cast<int>((sms + pairs - 1) / pairs);
-    if (splits > kDcMaxSplits) splits = kDcMaxSplits;
-  }
-  p.splits = splits;
-  if (splits > 1) {
+  SPD_REQUIRE(pairs < (1ll << 24), SPD_E_SHAPE, "spd_attn_decode_paged: batch x kv heads exceeds 2^24");
+  if (pairs < sms)
     SPD_REQUIRE(workspace && workspace_bytes >= spd_attn_decode_workspace_bytes(batch, num_q_heads, head_dim),
                 SPD_E_WORKSPACE, "spd_attn_decode_paged: workspace too small (%lld bytes)",
                 (long long)workspace_bytes);
-    SPD_REQUIRE(pairs <= 16384, SPD_E_SHAPE, "spd_attn_decode_paged: batch x kv heads exceeds 16384");
+  // Items may be cut where a workspace is there: two parts per CTA (with pairs < sms it holds those of 16 CTAs per pair at
+  // least).  Whether they are, the kernel decides by the lengths.
+  const int64_t cta_bytes = 2ll * (num_q_heads / num_kv_heads) * (head_dim + 2) * 4;
+  const int64_t room = workspace ? (workspace_bytes - 65536) / cta_bytes : 0;
+  const int64_t most = sms < device_sm_count_cached() ? sms : device_sm_count_cached();
+  const bool whole = pairs > 16384 || (pairs >= sms ? room < most : room < 1);
+  const int grid = static_cast<int>(whole ? (pairs < most ? pairs : most) : (room < most ? room : most));
+  if (!whole) {
+    // items per CTA in whole rounds, less what they come to on average, as a share of all items; of two rounds the second
+    // runs on few SMs that have the memory to themselves, so the bound is nine tiles there
+    p.idle = pairs < grid ? INFINITY : static_cast<float>((pairs + grid - 1) / grid) / pairs - 1.f / grid;
+    if (pairs < 2ll * grid) p.idle *= 5.f / 9.f;
     // layout (attn_simt.cu: spd_attn_decode_workspace_bytes): counters at a fixed offset first
     p.counters = reinterpret_cast<int*>(workspace);
     p.o_part = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(workspace) + 65536);
-    p.ml_part = p.o_part + batch * num_q_heads * kDcMaxSplits * head_dim;
+    p.ml_part = p.o_part + 2ll * grid * (num_q_heads / num_kv_heads) * head_dim;
   }
   // tensor maps over the pools: [slots, Hk*D] 16-bit, box 128 rows x 64 columns.  The C-ABI does
   // not carry the pool's slot count; the row extent only bounds the coordinates the kernel may
@@ -641,8 +712,6 @@ extern "C" int spd_attn_decode_paged(void* out, const void* q, const void* k_poo
   const uint64_t row_elems = static_cast<uint64_t>(num_kv_heads) * head_dim;
   if ((rc = get_tmap(&tk, k_pool, 1ull << 31, row_elems, row_elems, kDcTile))) return rc;
   if ((rc = get_tmap(&tv, v_pool, 1ull << 31, row_elems, row_elems, kDcTile))) return rc;
-  const int64_t total = pairs * splits;
-  const int grid = static_cast<int>(total < sms ? total : sms);
   SPD_DISPATCH_DTYPE(dtype, {
     auto kern = attn_decode_kernel<T>;
     static bool configured = false;
