@@ -316,9 +316,18 @@ int gemm_pair_try(void* C, const void* A, const void* W, int64_t M, int64_t N, i
                   cudaStream_t stream) {
   static const int enabled = getenv("SPD_GEMM_2CTA") ? atoi(getenv("SPD_GEMM_2CTA")) : 1;
   if (!enabled || M <= 256 || sms < 2) return 1;
-  // a 256-row pair tile must not pad M more than the 128-row tiles would, unless M is large
+  // A wave of 256 x 256 pair tiles takes about 0.9 of the time of a wave of 128 x 256 single tiles, so the pair serves also
+  // where its taller tiles pad M more, unless that costs it another wave — or the call is so short (under 48 k-blocks in
+  // all waves) that the pair's longer start and end decide.  4096 x 14336 weights: M = 300 87 -> 70 us, 600 87 -> 72,
+  // 1300 167 -> 156; 3648 x 2048, M = 600: 15.7 us single, 17.9 pair, 1300: 35 single, 28 pair.
   const int64_t rows_pair = (M + 255) / 256 * 256, rows_single = (M + 127) / 128 * 128;
-  if (rows_pair != rows_single && M < 2048) return 1;
+  if (rows_pair != rows_single && M < 2048) {
+    const int n_tile = epilogue == SPD_EPI_SILU_MUL ? kPgBN / 2 : kPgBN;
+    const int64_t cols = (N + n_tile - 1) / n_tile, kblocks = (K + kPgBK - 1) / kPgBK;
+    const int64_t waves_pair = (rows_pair / 256 * cols + sms / 2 - 1) / (sms / 2);
+    const int64_t waves_single = (rows_single / 128 * cols + sms - 1) / sms;
+    if (waves_pair * 9 >= waves_single * 10 || waves_single * kblocks < 48) return 1;
+  }
   PairGemmParams p{};
   p.C = C;
   p.ldc = ldc;
