@@ -803,6 +803,14 @@ int spd_gemm_grouped(void* C, const void* A, const void* W, int64_t M, int64_t N
                 SPD_E_BADARG, "spd_gemm_grouped: bad w_group_col_stride");
     p.x_tile_group = tile_group;
     p.y_rows = N;
+    // Tile order: all y tiles of a row tile before the next row tile, as far as their weights (40 MB) stay in L2.  The SMs
+    // then work on some row tiles of a few neighbouring experts, whose weights and rows are read once; row tiles innermost
+    // re-read the whole activation for every y tile (4096 tokens, 64 experts, top 6: gate / up 357 -> 258 us, down 218 -> 150
+    // together with its 128 x 256 tiles).
+    auto panel_of = [&](int bn, int64_t y_tiles) -> int {
+      const int64_t q = (40ll << 20) / (static_cast<int64_t>(bn) * K * 2);
+      return static_cast<int>(q < 1 ? 1 : q < y_tiles ? q : y_tiles);
+    };
     if ((rc = get_tmap(&tx, A, M, K, lda, kBM))) return rc;
     if (epilogue == SPD_EPI_SILU_MUL) {
       constexpr int BN = 256;
@@ -810,6 +818,7 @@ int spd_gemm_grouped(void* C, const void* A, const void* W, int64_t M, int64_t N
       p.y_group_rows = 2 * N;
       p.y_rows_w = N;
       p.y_tiles = static_cast<int>((N + BN / 2 - 1) / (BN / 2));
+      p.panel = panel_of(BN, p.y_tiles);
       const int total = p.x_tiles * p.y_tiles;
       const int grid = total < sms ? total : sms;
       if ((rc = get_tmap(&ty, W, static_cast<uint64_t>(num_groups) * 2 * N, K, ldw, BN / 2))) return rc;
@@ -817,9 +826,10 @@ int spd_gemm_grouped(void* C, const void* A, const void* W, int64_t M, int64_t N
     }
     // 128 x 256 tiles where they pad N no more than 128 x 128 ones by an eighth and still fill the SMs
     const int64_t pad256 = (N + 255) / 256 * 256, pad128 = (N + 127) / 128 * 128;
-    const bool use256 = w_group_col_stride == 0 && pad256 - pad128 <= N / 8 && p.x_tiles * (pad256 / 256) >= sms;
+    const bool use256 = pad256 - pad128 <= N / 8 && p.x_tiles * (pad256 / 256) >= sms;
     const int BN = use256 ? 256 : 128;
     p.y_tiles = static_cast<int>((N + BN - 1) / BN);
+    p.panel = panel_of(BN, p.y_tiles);
     const int total = p.x_tiles * p.y_tiles;
     const int grid = total < sms ? total : sms;
     if (w_group_col_stride > 0) {
