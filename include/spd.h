@@ -335,6 +335,15 @@ int spd_moe_dense_act(void* act, const void* gate_up, const int32_t* topk_ids, c
  * w_kc), out [tokens, H, kv_lora_rank].  replaces DeepseekV2AttentionMLA.forward_absorb's attention
  * call (S/models/deepseek_v2.py:684-700 → S/layers/attention/triton_ops/decode_attention.py:235-470,
  * extend_attention.py:291-410). */
+/* Between the fused projection qa [tokens, heads * (nope + rope) || kv_lora || rope] and spd_attn_mla: RMS norm of the
+ * latent and rotation (interleaved pairs, cos_sin [positions, rope] fp32 = cos || sin) of its rope part -> row loc[t] of
+ * kv_pool; rotation of every head's rope part -> q_lat [tokens, heads, kv_lora + rope] behind the kv_lora columns, which
+ * the caller fills.  replaces the q_pe / k_pe half of forward_absorb (models/deepseek_v2.py:633-684) and
+ * MLATokenToKVPool.set_kv_buffer (mem_cache/memory_pool.py:435-452) */
+int spd_mla_rotary_store(void* q_lat, const void* qa, void* kv_pool, const void* norm_weight, const float* cos_sin_cache,
+                         const int64_t* positions, const int64_t* loc, int64_t tokens, int num_heads, int nope_dim,
+                         int kv_lora_rank, int rope_dim, int64_t qa_stride, int64_t q_lat_stride, float eps, int dtype,
+                         spd_stream_t stream);
 int64_t spd_attn_mla_workspace_bytes(int num_heads, int kv_lora_rank);
 int spd_attn_mla(void* out, const void* q, const void* kv_pool, const int32_t* req_to_token,
                  const int64_t* req_pool_indices, const int64_t* seq_lens, const int32_t* prefix_lens,

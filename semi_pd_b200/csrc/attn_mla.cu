@@ -837,6 +837,59 @@ mla_merge_kernel(const MlaParams p) {
   *reinterpret_cast<uint2*>(dst) = make_uint2(pack2<T>(num.x * inv, num.y * inv), pack2<T>(num.z * inv, num.w * inv));
 }
 
+// What stands between the fused q / latent projection and the attention, one CTA per token: the latent row (RMS norm of
+// its 512 columns, rotation of its 64) goes to its cache slot, the rotated part of every query head to its place behind
+// the absorbed part.  Replaces four launches (norm in place, rotation in place, cache write, a strided copy of the rotated
+// queries: 8.2 + 7.9 + 5.5 + 12.5 us at 4096 tokens); it moves 13 KB a token, what bounds it is latency at small batches.
+template <typename T>
+__global__ void __launch_bounds__(256)
+mla_rotary_store_kernel(T* __restrict__ q_lat, const T* __restrict__ qa, T* __restrict__ pool, const T* __restrict__ w,
+                        const float* __restrict__ cos_sin, const int64_t* __restrict__ positions,
+                        const int64_t* __restrict__ loc, int H, int nope, int64_t qa_stride, int64_t q_lat_stride,
+                        float eps) {
+  constexpr int kRot = kMlaDL - kMlaDV;
+  __shared__ float part[2];
+  griddep_launch_dependents();
+  griddep_wait();
+  const int64_t t = blockIdx.x;
+  const int tid = threadIdx.x, q_size = H * (nope + kRot);
+  const T* row = qa + t * qa_stride;
+  T* dst = pool + loc[t] * kMlaDL;
+  if (tid < 64) {  // the norm: eight columns per thread of two warps
+    const Vec16<T> x = ldv(row + q_size + tid * 8), wv = ldv(w + tid * 8);
+    float f[8], ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      f[i] = to_f32<T>(x.e()[i]);
+      ss += f[i] * f[i];
+    }
+    ss = warp_sum(ss);
+    if ((tid & 31) == 0) part[tid >> 5] = ss;
+    asm volatile("bar.sync 1, 64;" ::: "memory");
+    const float inv = rsqrtf((part[0] + part[1]) / static_cast<float>(kMlaDV) + eps);
+    Vec16<T> o;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) o.e()[i] = from_f32<T>(f[i] * inv * to_f32<T>(wv.e()[i]));
+    stv(dst + tid * 8, o);
+    return;
+  }
+  const float* cs = cos_sin + positions[t] * kRot;  // cos of the 32 pairs, then sin
+  for (int i = tid - 64; i < (H + 1) * (kRot / 8); i += 192) {
+    const int h = i >> 3, c = i & 7;  // four (even, odd) pairs of head h, or of the latent's own rotated part
+    const Vec16<T> x = ldv(h < H ? row + h * (nope + kRot) + nope + c * 8 : row + q_size + kMlaDV + c * 8);
+    const float4 cv = *reinterpret_cast<const float4*>(cs + c * 4), sv = *reinterpret_cast<const float4*>(cs + kRot / 2 + c * 4);
+    const float co[4] = {cv.x, cv.y, cv.z, cv.w}, si[4] = {sv.x, sv.y, sv.z, sv.w};
+    Vec16<T> o;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float a = to_f32<T>(x.e()[2 * j]), b = to_f32<T>(x.e()[2 * j + 1]);
+      o.e()[2 * j] = from_f32<T>(a * co[j] - b * si[j]);
+      o.e()[2 * j + 1] = from_f32<T>(b * co[j] + a * si[j]);
+    }
+    stv(h < H ? q_lat + t * q_lat_stride + h * kMlaDL + kMlaDV + c * 8 : dst + kMlaDV + c * 8, o);
+  }
+}
+
 template <typename T, bool kExtend>
 static int mla_launch(const MlaParams& p, int grid, cudaStream_t st) {
   CUtensorMap tm, tr;
@@ -859,6 +912,27 @@ static int mla_launch(const MlaParams& p, int grid, cudaStream_t st) {
 using namespace spd;
 
 extern "C" {
+
+int spd_mla_rotary_store(void* q_lat, const void* qa, void* kv_pool, const void* norm_weight, const float* cos_sin_cache,
+                         const int64_t* positions, const int64_t* loc, int64_t tokens, int num_heads, int nope_dim,
+                         int kv_lora_rank, int rope_dim, int64_t qa_stride, int64_t q_lat_stride, float eps, int dtype,
+                         spd_stream_t stream) {
+  SPD_REQUIRE(q_lat && qa && kv_pool && norm_weight && cos_sin_cache && positions && loc, SPD_E_BADARG,
+              "spd_mla_rotary_store: null pointer");
+  SPD_REQUIRE(kv_lora_rank == kMlaDV && rope_dim == kMlaDL - kMlaDV, SPD_E_SHAPE,
+              "spd_mla_rotary_store: built for kv_lora_rank 512 + rope 64 (got %d + %d)", kv_lora_rank, rope_dim);
+  SPD_REQUIRE(tokens >= 0 && tokens < (1ll << 31) && num_heads > 0 && nope_dim >= 0, SPD_E_BADARG, "spd_mla_rotary_store: bad sizes");
+  SPD_REQUIRE(nope_dim % 8 == 0 && qa_stride % 8 == 0 && q_lat_stride % 8 == 0 && aligned16(q_lat) && aligned16(qa) &&
+                  aligned16(kv_pool) && aligned16(norm_weight) && aligned16(cos_sin_cache),
+              SPD_E_ALIGN, "spd_mla_rotary_store: strides must be multiples of 8 and pointers 16-B aligned");
+  if (tokens == 0) return 0;
+  SPD_DISPATCH_DTYPE(dtype, {
+    SPD_CUDA(launch(mla_rotary_store_kernel<T>, dim3((unsigned)tokens), dim3(256), 0, as_stream(stream), pdl_enabled(),
+                    (T*)q_lat, (const T*)qa, (T*)kv_pool, (const T*)norm_weight, cos_sin_cache, positions, loc, num_heads,
+                    nope_dim, qa_stride, q_lat_stride, eps));
+  });
+  return 0;
+}
 
 int64_t spd_attn_mla_workspace_bytes(int num_heads, int kv_lora_rank) {
   // two partials per CTA of up to 4 tokens x min(heads, 16) rows, and 32 bytes per CTA; 8 rows per head of two per SM

@@ -24,7 +24,6 @@ from typing import Dict, Iterable, Optional, Tuple
 import torch
 
 from . import ops
-from ._lib import check, lib
 from .attention_backend import RadixAttention
 from .distributed import get_tensor_model_parallel_world_size
 from .forward_batch_info import ForwardBatch, LogitsProcessorOutput
@@ -195,23 +194,15 @@ class DeepseekV2AttentionMLA:
         H, DL, R = self.num_heads, self.latent_dim, self.kv_lora_rank
         qa = ops.linear(hidden_states, self.q_kv_a_proj.weight)          # [T, H*192 + 576]
         q = qa[:, : self.q_size]
-        latent = qa[:, self.q_size:]
-        # latent row in place: RMSNorm on the kv_lora part, interleaved RoPE on the rope part (and
-        # on every head's q_pe) — then it IS the pool row
-        ops.rmsnorm(latent[:, :R], self.kv_a_layernorm.weight, self.kv_a_layernorm.variance_epsilon,
-                    out=latent[:, :R])
-        esz = qa.element_size()
-        check(lib.spd_rope_inplace(qa.data_ptr() + self.qk_nope_head_dim * esz,
-                                   qa.data_ptr() + (self.q_size + R) * esz, self.cos_sin_cache.data_ptr(),
-                                   positions.data_ptr(), T, H, 1, self.qk_head_dim, self.qk_rope_head_dim,
-                                   qa.stride(0), qa.stride(0), 1, ops._dt(qa), ops._stream()), "spd_rope_inplace")
+        # latent row (RMSNorm on the kv_lora part, interleaved RoPE on the rope part) into its pool slot, and every head's
+        # rotated q_pe behind its absorbed query [q_nope W_kc || q_pe]
         pool = forward_batch.token_to_kv_pool
-        pool.set_kv_buffer(self.attn_mqa, forward_batch.out_cache_loc, latent)
-        # absorbed query: [q_nope W_kc || q_pe] per head
         q_lat = torch.empty((T, H * DL), device=qa.device, dtype=qa.dtype)
+        ops.mla_rotary_store(qa, q_lat, pool.get_key_buffer(self.layer_id), positions, forward_batch.out_cache_loc,
+                             self.kv_a_layernorm.weight, self.cos_sin_cache, H, self.qk_nope_head_dim, R,
+                             self.qk_rope_head_dim, self.kv_a_layernorm.variance_epsilon)
         ops.linear_block_diag(q, self.w_kc_t, H, self.qk_nope_head_dim, R, self.qk_head_dim, out=q_lat,
                               out_group_stride=DL)
-        q_lat.view(T, H, DL)[:, :, R:].copy_(q.view(T, H, self.qk_head_dim)[:, :, self.qk_nope_head_dim:])
         o_lat = forward_batch.attn_backend.forward_mla(q_lat, self.attn_mqa, forward_batch)   # [T, H * R]
         attn_out = ops.linear_block_diag(o_lat, self.w_vc, H, R, self.v_head_dim, R)          # [T, H * v]
         return ops.linear(attn_out, self.o_proj.weight)

@@ -434,6 +434,24 @@ def kv_write_single(rows: torch.Tensor, pool: torch.Tensor, loc: torch.Tensor) -
                            r2.stride(0), 0, _dt(rows), _stream()), "spd_kv_write")
 
 
+def mla_rotary_store(qa: torch.Tensor, q_lat: torch.Tensor, kv_pool: torch.Tensor, positions: torch.Tensor,
+                     loc: torch.Tensor, norm_weight: torch.Tensor, cos_sin_cache: torch.Tensor, num_heads: int,
+                     nope_dim: int, kv_lora_rank: int, rope_dim: int, eps: float) -> None:
+    """qa [T, H (nope + rope) + kv_lora + rope], the fused projection: kv_pool[loc[t]] = normed latent || rotated rope part;
+    q_lat [T, H (kv_lora + rope)] gets every head's rotated rope part (its kv_lora columns are the caller's)."""
+    _cuda(qa, q_lat, kv_pool, positions, loc, norm_weight, cos_sin_cache)
+    if cos_sin_cache.dtype != torch.float32 or positions.dtype != torch.int64:
+        raise RuntimeError("mla_rotary_store: cos_sin_cache is float32, positions are int64")
+    if not (qa.dtype == q_lat.dtype == kv_pool.dtype == norm_weight.dtype):
+        raise RuntimeError("mla_rotary_store: qa, q_lat, the pool and the norm weight share a dtype")
+    if loc.dtype != torch.int64:
+        loc = loc.long()
+    check(lib.spd_mla_rotary_store(q_lat.data_ptr(), qa.data_ptr(), kv_pool.data_ptr(), norm_weight.data_ptr(),
+                                   cos_sin_cache.data_ptr(), positions.data_ptr(), loc.data_ptr(), qa.shape[0], num_heads,
+                                   nope_dim, kv_lora_rank, rope_dim, qa.stride(0), q_lat.stride(0), float(eps), _dt(qa),
+                                   _stream()), "spd_mla_rotary_store")
+
+
 def attn_mla(q: torch.Tensor, kv_pool: torch.Tensor, req_to_token, req_pool_indices, num_heads: int,
              kv_lora_rank: int, rope_dim: int, sm_scale: float, workspace: torch.Tensor, seq_lens=None,
              prefix_lens=None, extend_start_loc=None, out: Optional[torch.Tensor] = None) -> torch.Tensor:

@@ -113,3 +113,38 @@ def test_least_workspace(decode):
     _run([200, 100], ext, H, torch.bfloat16, "runs", decode, ws_bytes=least)
     with pytest.raises(RuntimeError):
         _run([200, 100], ext, H, torch.bfloat16, "runs", decode, ws_bytes=least - 4)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("T,H", [(1, 16), (3, 1), (130, 5), (7, 32)])
+def test_rotary_store(dtype, T, H):
+    from semi_pd_b200 import ops
+    g = torch.Generator().manual_seed(T + H)
+    nope = 128
+    qa = torch.randn(T, H * (nope + DR) + R + DR + 8, generator=g).to(dtype)[:, : H * (nope + DR) + R + DR]
+    w = (1 + 0.1 * torch.randn(R, generator=g)).to(dtype)
+    ang = torch.rand(500, DR // 2, generator=g) * 6
+    table = torch.cat((ang.cos(), ang.sin()), 1)
+    pos, loc = torch.randint(0, 500, (T,), generator=g), torch.randperm(T + 20, generator=g)[:T]
+    q_lat = torch.zeros(T, H * (R + DR), dtype=dtype, device=DEV)
+    pool = torch.zeros(T + 20, 1, R + DR, dtype=dtype, device=DEV)
+    whole = torch.empty(T, qa.shape[1] + 8, dtype=dtype, device=DEV)
+    d_qa = whole[:, : qa.shape[1]]
+    d_qa.copy_(qa)
+    ops.mla_rotary_store(d_qa, q_lat, pool, pos.to(DEV), loc.to(DEV), w.to(DEV), table.to(DEV), H, nope, R, DR, 1e-6)
+    c, s = table[pos].double()[:, None, : DR // 2], table[pos].double()[:, None, DR // 2:]
+
+    def rot(x):  # interleaved pairs
+        a, b = x.double()[..., 0::2], x.double()[..., 1::2]
+        return torch.stack((a * c - b * s, b * c + a * s), -1).flatten(-2)
+
+    x = qa[:, H * (nope + DR): H * (nope + DR) + R].double()
+    want = torch.zeros(T + 20, R + DR, dtype=torch.float64)
+    want[loc, :R] = x / (x.square().mean(-1, keepdim=True) + 1e-6).sqrt() * w.double()
+    want[loc, R:] = rot(qa[:, None, H * (nope + DR) + R:])[:, 0]
+    q_want = torch.zeros(T, H, R + DR, dtype=torch.float64)
+    q_want[..., R:] = rot(qa[:, : H * (nope + DR)].view(T, H, nope + DR)[..., nope:])
+    # one rounding to 16 bits of fp32 results of at most about 8
+    tol = 2 ** -11 * 8 + 1e-5 if dtype == torch.float16 else 2 ** -8 * 8 + 1e-5
+    assert (pool.cpu().double()[:, 0] - want).abs().max().item() < tol
+    assert (q_lat.cpu().double().view(T, H, -1) - q_want).abs().max().item() < tol
