@@ -27,15 +27,16 @@
 // (its rope block, free after S), each given back by itself: 2.75 tiles at N = 16, 2 at N = 64.  A tile's copies meet on
 // one barrier.  Full tiles of 64 consecutive slots come by TMA (four boxes of 64 rows x 2 blocks and one of 64 x 1),
 // anything else by 16-byte cp.async through req_to_token.  The
-// softmax is the lazily rescaled one of attn_decode.cu: scores are read from TMEM in the 16x256b fragment layout (all
+// softmax keeps the true running max per column (see there): scores are read from TMEM in the 16x256b fragment layout (all
 // 32 lanes of a warp busy although M = 64 fills 16 lanes per warp), P goes back as stmatrix-transposed K-major rows.
 //
-// Decode streams each latent row once: 64 requests of 1088 keys (83 MB) take 26 us, about 3000 clk per 72 KB tile and SM
-// (6.8 TB/s in the steady state) after 9000 clk until the first tile has landed; one CTA per token, head group and split
-// with warp-level MMAs took 54 us.  MMAs (M = 64: 23 clk at N = 16, 31 at N = 64) are hidden as long as the issuer's code
-// stays a short loop.  Extend, 4096 new tokens in 4 requests (two with 515 cached): 1496 -> 394 us; bounded by the ring of
-// two tiles (a tile's copies start when the PV before last has finished: 4400 clk a tile against 2000 of MMAs) and by
-// beginning and ending items, which therefore count in the split (without that, SMs with short items took 870 us).
+// Decode streams each latent row once, 64 requests of 1088 keys (83 MB) in 34 us with the merge launch; one CTA per token,
+// head group and split with warp-level MMAs took 62 us.  About 9000 clk pass until the first tile has landed, then 3000 clk
+// per 72 KB tile and SM.  MMAs (M = 64: 23 clk at N = 16, 31 at N = 64) are hidden as long as the issuer's code stays a
+// short loop.  Extend, 4096 new tokens in 4 requests (two with 515 cached), whole layer: 1645 -> 600 us; bounded by the
+// ring of two tiles (a tile's copies start when the PV before last has finished), by the rescale of O^T whenever a tile
+// raises one of 64 columns, and by beginning and ending items, which therefore count in the split (without that, SMs with
+// short items took twice as long).
 //
 // Every mbarrier wait is bounded: a wait that runs out marks the CTA dead, all later waits fall through, the kernel
 // finishes without waiting and counts itself in g_mla_wait_expired.
@@ -53,7 +54,6 @@ constexpr int kMlaHeads = 16;    // heads per item
 constexpr int kMlaDL = 576, kMlaDV = 512;
 constexpr int kMlaBlk = kMlaTile * 128;       // one [64 rows x 64 columns] swizzle block of a tile
 constexpr int kMlaMisc = 2048;
-constexpr float kMlaRescale = 8.0f;           // log2 units a score may exceed the reference max before it is raised
 
 __device__ unsigned int g_mla_wait_expired;
 
@@ -642,9 +642,12 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
         }
         bool exceed = false;
 #pragma unroll
-        for (int i = 0; i < N / 2; ++i) exceed |= s[i] > m_ref[(i >> 2) * 2 + (i & 1)] + kMlaRescale;
+        for (int i = 0; i < N / 2; ++i) exceed |= s[i] > m_ref[(i >> 2) * 2 + (i & 1)];
         if (mla_bar_or(exceed)) {
-          // first tile of an item, rarely later: true tile max per column, raise m_ref, rescale O^T
+          // The true running max per column, so that a column's largest P is exactly 1: a reference that lags by up to 2^8
+          // saves most of these rescales but rounds that P too (decode: 32.4 instead of 33.8 us and extend 548
+          // instead of 600, but 6 - 14 % more rms error of a decode against 64-bit results; what is left is about 2.5 %, perhaps the
+          // max being taken per 64 keys where the warp-level kernel took it per 32).
 #pragma unroll
           for (int i = 0; i < C; ++i) {
             float m = fmaxf(s[(i >> 1) * 4 + (i & 1)], s[(i >> 1) * 4 + 2 + (i & 1)]);

@@ -312,7 +312,7 @@ __device__ __forceinline__ float softmax_row_max(uint32_t ts, int kv0, int limit
 // alternate on the tensor core tile by tile.
 // kWin: a sliding window (KV tiles before the item's first visible key are skipped), sinks and a query temperature — the
 // general attention of the hybrid families at head size 128 (see spd::attn_prefill_window_try).
-// 4 requests of 2048 new tokens, 16 / 4 heads, window 1024: 320 us on warp-level MMAs with 64 x 64 tiles, 114 us here
+// 4 requests of 2048 new tokens, 16 / 4 heads, window 1024: 320 us on warp-level MMAs with 64 x 64 tiles, 140 us here
 // (60 GFLOP visible; a query tile of 128 meets nine key tiles, two of them masked).
 template <typename T, int kU, bool kTrace, bool kWin>
 __global__ void __launch_bounds__(kPfThreads, 1)
@@ -665,6 +665,24 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       }
       if (tracer) pf_trace<kTrace>(p, w, tn, 0x600);  // O stored
     };
+    const auto rescale_o = [&](float alpha, uint32_t unit) {
+      // O must be quiescent: S of this unit was issued after PV of unit u-kNU (so units
+      // <= u-kNU are complete), but PV of the units in between (the other half) may still
+      // be running.  pv_done is per unit-of-tile so that this wait cannot alias: on that
+      // barrier at most the one phase we wait for is outstanding (a parity wait only tells
+      // the current phase from the one before it).
+      mbar_wait(&pv_done[w * 2 + ((unit - 1) % kNU)], ((unit - 1) / kNU) & 1);
+      tc_fence_after_sync();
+#pragma unroll 1
+      for (int c = 0; c < kPfD; c += 32) {
+        uint32_t r[32];
+        tmem_ld_32x32b_x32(to + c, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * alpha);
+        tmem_st_32x32b_x32(to + c, r);
+      }
+    };
     int idx = pf_rank(0, cta, ncta);
     PfRaw raw = pf_raw(p, idx);
     for (int k = 0; idx < p.total_items; ++k) {
@@ -697,12 +715,23 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         mbar_wait(&s_full[w * 2 + h], (u / kNU) & 1);
         tc_fence_after_sync();
         if (tracer) pf_trace<kTrace>(p, w, tn, 0x200 + h);  // S ready
-        if (jh == 0 || (kWin && __any_sync(0xffffffffu, m_used == -INFINITY))) {
-          // first unit of the item — with a window, also as long as some row has seen no key — establish the reference
-          // max with a max-only pre-pass
+        if constexpr (kWin) {
+          // The true running max, raised at every unit: the largest P of a row is then exactly 1, as in the warp-level kernel
+          // that serves the other calls.  (A reference that lags, as below, rounds that P too: 113 us instead of 140, but
+          // 9 - 15 % more rms error against 64-bit results.)
           const float mx = need_mask ? softmax_row_max<true, kU, kWin>(tsh, kv0, limit, span)
                                      : softmax_row_max<false, kU, kWin>(tsh, kv0, limit, span);
-          if (m_used == -INFINITY) m_used = mx;
+          if (__any_sync(0xffffffffu, mx > m_used)) {
+            const float m_new = fmaxf(m_used, mx);
+            const float alpha = (m_used == -INFINITY) ? 0.f : fast_exp2((m_used - m_new) * scale);
+            l *= alpha;
+            m_used = m_new;
+            if (jh > 0) rescale_o(alpha, u);
+          }
+        } else if (jh == 0) {
+          // first unit of the item: establish the reference max with a max-only pre-pass
+          m_used = need_mask ? softmax_row_max<true, kU, kWin>(tsh, kv0, limit, span)
+                             : softmax_row_max<false, kU, kWin>(tsh, kv0, limit, span);
         }
         float m_off = (m_used == -INFINITY) ? 0.f : m_used * scale;
         uint32_t pk[kU / 2];
@@ -711,7 +740,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         // raise the reference max only when some row may have outgrown it by > 2^8 (an element
         // above 2^8 implies a row sum above 2^8; warp-uniform decision: tcgen05.ld/st are
         // warp-collective); S is still intact (P is stored below), so the unit is simply redone
-        if (__any_sync(0xffffffffu, psum > kRescaleTrigger)) {
+        if (!kWin && __any_sync(0xffffffffu, psum > kRescaleTrigger)) {
           const float mx = need_mask ? softmax_row_max<true, kU, kWin>(tsh, kv0, limit, span)
                                      : softmax_row_max<false, kU, kWin>(tsh, kv0, limit, span);
           const float m_new = fmaxf(m_used, mx);
@@ -719,24 +748,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           l *= alpha;
           m_used = m_new;
           m_off = (m_used == -INFINITY) ? 0.f : m_used * scale;
-          if (jh > 0) {
-            // O must be quiescent: S of this unit was issued after PV of unit u-kNU (so units
-            // <= u-kNU are complete), but PV of the units in between (the other half) may still
-            // be running.  pv_done is per unit-of-tile so that this wait cannot alias: on that
-            // barrier at most the one phase we wait for is outstanding (a parity wait only tells
-            // the current phase from the one before it).
-            mbar_wait(&pv_done[w * 2 + ((u - 1) % kNU)], ((u - 1) / kNU) & 1);
-            tc_fence_after_sync();
-#pragma unroll 1
-            for (int c = 0; c < kPfD; c += 32) {
-              uint32_t r[32];
-              tmem_ld_32x32b_x32(to + c, r);
-              tmem_ld_wait();
-#pragma unroll
-              for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * alpha);
-              tmem_st_32x32b_x32(to + c, r);
-            }
-          }
+          if (jh > 0) rescale_o(alpha, u);
           psum = need_mask ? softmax_row_pass<T, true, kU, kWin>(tsh, pk, scale, m_off, kv0, limit, span)
                            : softmax_row_pass<T, false, kU, kWin>(tsh, pk, scale, m_off, kv0, limit, span);
         }
