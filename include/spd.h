@@ -201,7 +201,8 @@ int spd_attn_prefill_ragged(void* out, const void* q, const void* k_pool, const 
                             int sm_budget, spd_stream_t stream);
 /* Batched paged-decode attention: one query row per request over its seq_lens[b] cached rows
  * (including the token just written).  Split-KV with an in-kernel merge; workspace from
- * spd_attn_decode_workspace_bytes().  replaces FlashInferAttnBackend.forward_decode
+ * spd_attn_decode_workspace_bytes(), zeroed once before its first use (it is used at any batch size; each call leaves its
+ * counters at zero), one per stream.  replaces FlashInferAttnBackend.forward_decode
  * (flashinfer_backend.py:454-488); semantics torch_native_backend.py:111-179. */
 int64_t spd_attn_decode_workspace_bytes(int64_t max_batch, int num_q_heads, int head_dim);
 int spd_attn_decode_paged(void* out, const void* q, const void* k_pool, const void* v_pool,

@@ -569,11 +569,16 @@ pool_key_blocks_kernel(T* __restrict__ k_pool, T* __restrict__ v_pool, const int
   }
 }
 
-// Whether a portion of at most `ext` new tokens takes the tcgen05 prefill kernel (tiles of 128 queries x 128 keys) rather
-// than the mma.sync one (64 x 64): a query tile has to meet several whole key tiles.  16 / 4 heads, 4 requests of 200
-// tokens after 1500, window 1024: 52 us (mma.sync) / 28 us; of 500, window 128: 25 / 31 us, of 1500, window 128: 66 / 55 us;
-// one of 40 tokens, no prefix: 6.0 / 7.0 us.  The prefixes are on the device, so they do not enter the rule.
-inline bool window_tc_wins(int64_t ext, int window) { return window <= 0 || window >= 512 ? ext >= 192 : ext >= 1024; }
+// Whether portions of at most `ext` new tokens take the tcgen05 prefill kernel (tiles of 128 queries x 128 keys) rather
+// than the mma.sync one (64 x 64): a query tile has to meet several whole key tiles, and a request alone, whose few tiles
+// leave SMs idle either way, has to be longer.  16 / 4 heads, mma.sync / tcgen05: 4 requests of 192 tokens, window 1024
+// 17.0 / 12.4 us, after 1500 tokens, window 512 29.4 / 23.7; of 1024, window 128 46.6 / 33.9.  One request of 192, window
+// 1024 9.8 / 10.2, of 500 after 1500, window 512 22.0 / 23.5, of 1024 29.4 / 23.3; window 128: of 1024 13.6 / 15.1, of 1500
+// 21.9 / 17.1.  The prefixes are on the device, so they do not enter the rule.
+inline bool window_tc_wins(int64_t batch, int64_t ext, int window) {
+  if (window <= 0 || window >= 512) return ext >= (batch > 1 ? 192 : 1024);
+  return ext >= (batch > 1 ? 1024 : 1500);
+}
 
 int attn_general_mma_try(void* out, const void* q, const void* k_pool, const void* v_pool, const int32_t* req_to_token,
                          const int64_t* req_pool_indices, const int32_t* prefix_lens, const int32_t* extend_lens,
@@ -751,7 +756,7 @@ int spd_attn_general_keys(void* out, const void* q, const void* k_pool, const vo
     return 0;
   }
   // 16-bit prefill at head size 128 on tcgen05, for the options that kernel has
-  if (window_tc_wins(max_extend_len, window) && dtype != SPD_F32 && head_dim == 128 && v_dim == 128 && slopes == nullptr &&
+  if (window_tc_wins(batch, max_extend_len, window) && dtype != SPD_F32 && head_dim == 128 && v_dim == 128 && slopes == nullptr &&
       db.table == nullptr && !(softcap > 0.f) && kb.size == 0 && kb.keep == 0 && Gv == num_kv_heads &&
       v_slot == (int64_t)num_kv_heads * 128) {
     const int rc = attn_prefill_window_try(out, q, k_pool, v_pool, req_to_token, req_pool_indices, prefix_lens, extend_lens,

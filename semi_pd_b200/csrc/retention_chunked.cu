@@ -429,7 +429,7 @@ int retention_chunked_try(float* o, const void* q, const void* k, const void* v,
                           int64_t max_positions, float k_scale, int in_act, int dtype, int64_t total_tokens,
                           cudaStream_t stream) {
   // A chunk costs what some tens of tokens cost one by one, and its CTA takes a whole SM: 4 requests of 16 tokens 12.1 us
-  // (token by token) / 11.8, of 64 tokens 32.9 / 16; 16 requests of 16 tokens 30 / 41 us, of 40 tokens 63 / 41.
+  // (token by token) / 11.8, of 64 tokens 32.9 / 17.6; 16 requests of 16 tokens 30 / 41 us, of 40 tokens 63 / 41.
   if (total_tokens <= 40 * batch) return 1;
   // 16-bit rows without an activation (their parts are what the split was counted for), 128 channels, whole 64-column
   // slices, a rotation in whole 16-byte pieces, 16-byte rows

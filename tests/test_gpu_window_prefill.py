@@ -75,8 +75,8 @@ def test_scattered_slots_and_no_options(window):
 @pytest.mark.parametrize("shift", [-60.0, 60.0])
 def test_scores_far_from_zero(shift):
     # every score is moved by +-60: rows that see nothing in their item's first units must not start from zero
-    _run([700], [260], 4, 2, 512, torch.bfloat16, shift=shift, scale=1.0 / 8)
-    _run([0], [1100], 4, 2, 70, torch.bfloat16, shift=shift, scale=1.0 / 8)
+    _run([700, 0], [260, 9], 4, 2, 512, torch.bfloat16, shift=shift, scale=1.0 / 8)
+    _run([0, 4], [1100, 9], 4, 2, 70, torch.bfloat16, shift=shift, scale=1.0 / 8)
 
 
 def test_large_sinks_and_empty_requests():
@@ -85,5 +85,10 @@ def test_large_sinks_and_empty_requests():
 
 def test_negative_scale_and_temperature_keep_their_results():
     # a reference maximum of raw scores does not serve negative factors: these stay on the other kernel
-    _run([10], [250], 2, 1, 512, torch.float16, scale=-D ** -0.5)
-    _run([10], [250], 2, 1, 512, torch.float16, qtemp=(-0.1, 64))
+    _run([10, 0], [250, 9], 2, 1, 512, torch.float16, scale=-D ** -0.5)
+    _run([10, 0], [250, 9], 2, 1, 512, torch.float16, qtemp=(-0.1, 64))
+
+
+@pytest.mark.parametrize("ext,window", [(1023, 512), (1024, 512), (1499, 128), (1500, 128)])
+def test_a_request_alone(ext, window):
+    _run([77], [ext], 4, 2, window, torch.bfloat16, sinks=1.0)
