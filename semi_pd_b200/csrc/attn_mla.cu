@@ -742,6 +742,7 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
       mbar_wait_bounded(p_empty, (t - 1) & 1, dead);  // the last PV of the item has finished
       tc_fence_after_sync();
       T* out = reinterpret_cast<T*>(p.out) + it.row0 * p.out_stride + static_cast<int64_t>(h0) * kMlaDV + warp * 32;
+      float z[2] = {0.f, 0.f};  // kExtend: NaN when an output is infinite or NaN
       if (whole) {
         // neighbouring lanes swap halves of two columns: 4-byte stores, 64 bytes of a row per half warp
         const bool odd = lane & 1;
@@ -755,6 +756,10 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
 #pragma unroll
           for (int cc = 0; cc < N; cc += 16) {
             if ((cc >> 4) >= it.ntok) break;
+            if constexpr (kExtend) {
+#pragma unroll
+              for (int e = 0; e < 16; ++e) z[e & 1] = fmaf(__uint_as_float(o[cc + e]), 0.f, z[e & 1]);
+            }
             T* row = dst + (cc >> 4) * p.out_stride;
 #pragma unroll
             for (int e = 0; e < 16; e += 4) {
@@ -780,6 +785,10 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
 #pragma unroll
           for (int cc = 0; cc < N; cc += 16) {
             if ((cc >> 4) >= it.ntok) break;
+            if constexpr (kExtend) {
+#pragma unroll
+              for (int e = 0; e < 16; ++e) z[e & 1] = fmaf(__uint_as_float(o[cc + e]), 0.f, z[e & 1]);
+            }
             float* row = dst + static_cast<int64_t>((cc >> 4) * nhm) * kMlaDV;
 #pragma unroll
             for (int e = 0; e < 16; ++e)
@@ -790,6 +799,73 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(o_empty);
+      if constexpr (kExtend) {
+        // The tiles hold rows that some or all of the item's tokens may not see.  Their P is 0, but 0 times an infinite or
+        // NaN value is NaN: an output that is not finite is computed again from the visible keys, where such a row was there.  (Looking at every output and the
+        // barrier: 605 -> 610 us for a layer of 4096 new tokens.)
+        if (mla_bar_or(isnan(z[0] + z[1]))) {
+          if (tid < 4) {
+#pragma unroll
+            for (int i = 0; i < C; ++i) red[(i >> 1) * 8 + col0 + (i & 1)] = m_ref[i];
+          }
+          const int32_t* page = p.req_to_token + p.req_pool_indices[it.r] * p.rtt_stride;
+          const T* pool = reinterpret_cast<const T*>(p.kv_pool);
+          const int end_key = min(it.load_end, (tile_last + 1) * kMlaTile);
+          const int hid0 = max(it.p0 + 1, tile0 * kMlaTile);  // from here on some token does not see the rows
+          bool odd_v = false;
+#pragma unroll 1
+          for (int i = tid; i < (end_key - hid0) * (kMlaDV / 8); i += 128) {
+            const Vec16<T> x = ldv(pool + static_cast<int64_t>(page[hid0 + i / (kMlaDV / 8)]) * kMlaDL + i % (kMlaDV / 8) * 8);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) odd_v |= !(fabsf(to_f32<T>(x.e()[e])) <= 3.4028235e38f);
+          }
+          if (mla_bar_or(odd_v)) {
+            float* pk_s = red + 2 * N;  // probabilities of 128 keys
+            const T* qb = reinterpret_cast<const T*>(p.q) + it.row0 * p.q_stride + static_cast<int64_t>(h0) * kMlaDL;
+#pragma unroll 1
+            for (int col = 0; col < it.ntok * kMlaHeads; ++col) {
+              const int tok = col >> 4, h = col & 15;
+              if (h >= nh) continue;
+              const T* qr = qb + tok * p.q_stride + h * kMlaDL;
+              const int seen = min(end_key, it.p0 + tok + 1);
+              const float m = red[col];
+              float acc[4] = {0.f, 0.f, 0.f, 0.f};  // value columns 4 tid ..
+#pragma unroll 1
+              for (int k0 = tile0 * kMlaTile; k0 < seen; k0 += 128) {
+                float dot = 0.f;
+                if (k0 + tid < seen) {
+                  const T* kr = pool + static_cast<int64_t>(page[k0 + tid]) * kMlaDL;
+#pragma unroll 1
+                  for (int d = 0; d < kMlaDL; d += 8) {
+                    const Vec16<T> a = ldv(qr + d), b = ldv(kr + d);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) dot = fmaf(to_f32<T>(a.e()[e]), to_f32<T>(b.e()[e]), dot);
+                  }
+                }
+                pk_s[tid] = to_f32<T>(from_f32<T>(fast_exp2(dot * p.scale_log2 - m)));
+                mla_bar();
+#pragma unroll 1
+                for (int i = 0; i < min(128, seen - k0); ++i) {
+                  const T* vr = pool + static_cast<int64_t>(page[k0 + i]) * kMlaDL + tid * 4;
+#pragma unroll
+                  for (int e = 0; e < 4; ++e) acc[e] = fmaf(pk_s[i], to_f32<T>(vr[e]), acc[e]);
+                }
+                mla_bar();
+              }
+              if (whole) {
+                T* row = reinterpret_cast<T*>(p.out) + (it.row0 + tok) * p.out_stride +
+                         static_cast<int64_t>(h0 + h) * kMlaDV + tid * 4;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) row[e] = from_f32<T>(acc[e] * s_col[col]);
+              } else {
+                float* row = p.o_part + (part0 + tok * nhm + h) * kMlaDV + tid * 4;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) row[e] = acc[e];
+              }
+            }
+          }
+        }
+      }
       mla_bar();  // red / s_col belong to the next item
     }
   }

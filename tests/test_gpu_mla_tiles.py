@@ -48,7 +48,7 @@ def _reference(q, pool, rtt, pre, ext, scale):
 TOL = {torch.float16: 2e-3, torch.bfloat16: 1.6e-2}
 
 
-def _run(pre, ext, H, dtype, layout, decode, ws_bytes=None, sms=0):
+def _run(pre, ext, H, dtype, layout, decode, ws_bytes=None, sms=0, odd=()):
     from semi_pd_b200 import ops
     g = torch.Generator().manual_seed(sum(ext) + 7 * sum(pre) + H)
     lens = [p + e for p, e in zip(pre, ext)]
@@ -56,6 +56,11 @@ def _run(pre, ext, H, dtype, layout, decode, ws_bytes=None, sms=0):
     q = (torch.randn(sum(ext), H, R + DR, generator=g) * 0.5).to(dtype)
     scale = 192 ** -0.5
     want = _reference(q, pool, rtt, pre, ext, scale)
+    blind = torch.ones(len(q), dtype=torch.bool)  # query rows that see none of the infinite or NaN values put in below
+    for b, pos, channel, value in odd:
+        pool[rtt[b, pos].long(), channel] = value
+        at = sum(ext[:b])
+        blind[at + max(0, pos - pre[b]): at + ext[b]] = False
     need = ops.lib.spd_attn_mla_workspace_bytes(H, R) if ws_bytes is None else ws_bytes
     ws = torch.full((need,), 255, dtype=torch.uint8, device=DEV)  # (not zeroed: NaN patterns)
     i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
@@ -70,8 +75,12 @@ def _run(pre, ext, H, dtype, layout, decode, ws_bytes=None, sms=0):
                            R, DR, scale, ws, **more)
     finally:
         ops.set_sm_budget(0)
-    err = (out.cpu().double().view(want.shape) - want).abs().max().item()
+    out = out.cpu().double().view(want.shape)
+    err = (out - want)[blind].abs().max().item()
     assert err < TOL[dtype], err
+    for b, pos, channel, value in odd:
+        at = sum(ext[:b])
+        assert not out[at + max(0, pos - pre[b]): at + ext[b], :, channel].isfinite().any()
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
@@ -93,6 +102,20 @@ def test_head_counts(H, decode):
                                      ([0, 640], [700, 259])])
 def test_extend_tiles(layout, pre, ext):
     _run(pre, ext, 16, torch.bfloat16, layout, False)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("layout", ["runs", "scattered"])
+@pytest.mark.parametrize("pre,ext,odd", [
+    ([0], [64], [(0, 63, 5, float("nan"))]),                       # the last row of a full tile
+    ([100], [130], [(0, 150, 511, float("inf")), (0, 229, 0, float("-inf"))]),
+    ([0, 500], [70, 66], [(0, 2, 17, float("inf")), (1, 502, 3, float("nan"))]),   # inside a group of four tokens
+    ([1500], [6], [(0, 1504, 100, float("nan"))]),                 # items cut over several SMs
+    ([0, 3], [700, 300], [(0, 640, 1, float("inf")), (1, 200, 2, float("nan"))]),  # whole items
+])
+def test_values_that_are_not_finite_reach_no_earlier_token(dtype, layout, pre, ext, odd):
+    _run(pre, ext, 16, dtype, layout, False, odd=odd)
+    _run(pre, ext, 5, dtype, layout, False, odd=odd, sms=2)
 
 
 def test_empty_requests_in_an_extend_batch():
