@@ -85,6 +85,8 @@ struct PrefillParams {
   // kWin only: keys a query sees up to and with itself; a logit per head in the softmax denominator (nullptr: none); query
   // temperature 1 + coef ln(floor((pos + 1) / every) + 1) (every 0: none)
   int window, qtemp_every;
+  const void* q;
+  int64_t q_stride;
   const float* sinks;
   float qtemp_coef;
   long long* trace;  // debug timeline of CTA 0 (scripts/debug_attn_prefill_timeline.py); kTrace builds only
@@ -304,6 +306,44 @@ __device__ __forceinline__ float softmax_row_max(uint32_t ts, int kv0, int limit
     rowmax_chunk<kMask, kWin>(rb, c + 32, kv0, limit, span, m0, m1);
   }
   return fmaxf(m0, m1);
+}
+
+// Output of one query row by a warp, from the keys the row sees alone; before the division by the sum, columns
+// c + 2 lane and c + 2 lane + 1.  (kWin, for rows whose output is not finite: the tiles hold keys that the row does not
+// see, and their P of 0 times an infinite or NaN value is NaN.  Looking for them in the epilogue: 140.6 -> 143.4 us for
+// 4 requests of 2048 new tokens, 16 / 4 heads, window 1024.)
+template <typename T>
+__device__ __noinline__ float2 pf_row_alone(const T* q, const T* k_pool, const T* v_pool, const int32_t* page,
+                                            int64_t row_elems, int kv0, int kv1, int c, float scale, float m_off) {
+  const int lane = threadIdx.x & 31;
+  float2 acc = make_float2(0.f, 0.f);
+#pragma unroll 1
+  for (int j0 = kv0; j0 < kv1; j0 += 32) {
+    const int j = j0 + lane;
+    int64_t at = 0;
+    float prob = 0.f;
+    if (j < kv1) {
+      at = page[j] * row_elems;
+      float dot = 0.f;
+#pragma unroll 1
+      for (int d = 0; d < kPfD; d += 8) {
+        const Vec16<T> a = ldv(q + d), b = ldv(k_pool + at + d);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) dot = fmaf(to_f32<T>(a.e()[e]), to_f32<T>(b.e()[e]), dot);
+      }
+      prob = to_f32<T>(from_f32<T>(fast_exp2(fmaf(dot, scale, -m_off))));
+    }
+    const int n = min(32, kv1 - j0);
+#pragma unroll 1
+    for (int i = 0; i < n; ++i) {
+      const float pi = __shfl_sync(0xffffffffu, prob, i);
+      const T* v = v_pool + __shfl_sync(0xffffffffu, at, i) + c + 2 * lane;
+      acc.x = fmaf(pi, to_f32<T>(v[0]), acc.x);
+      acc.y = fmaf(pi, to_f32<T>(v[1]), acc.y);
+    }
+    if (__all_sync(0xffffffffu, isnan(acc.x) && isnan(acc.y))) break;  // nothing changes that any more
+  }
+  return acc;
 }
 
 // kU: columns of one softmax / MMA unit.  64: the half-tile pipeline described above.  128: one
@@ -605,6 +645,35 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     float e_l = 0.f;  // state of the item being written out
     int e_rows = 0, e_head = 0, e_q_row0 = 0;
     uint32_t e_u = 0;
+    int e_req = 0, e_hk = 0, e_limit = 0;  // kWin
+    float e_scale = 0.f, e_m_off = 0.f;
+    // kWin: the warp's rows whose columns c .. c + 63 have a value that is not finite (z is NaN), again; into the staging
+    // block or (nullptr) to global memory
+    auto rows_alone = [&](float z, int c, float inv_l, uint8_t* stage) {
+      uint32_t todo = __ballot_sync(0xffffffffu, isnan(z));
+      if (todo == 0) return;
+      __syncwarp();
+      const int64_t col = static_cast<int64_t>(e_hk) * kPfD;
+#pragma unroll 1
+      for (; todo != 0; todo &= todo - 1) {
+        const int src = __ffs(todo) - 1, r = (row & ~31) + src;
+        const int lim = __shfl_sync(0xffffffffu, e_limit, src);
+        const float2 f = pf_row_alone<T>(
+            reinterpret_cast<const T*>(p.q) + static_cast<int64_t>(e_q_row0 + r) * p.q_stride +
+                static_cast<int64_t>(e_head) * kPfD,
+            reinterpret_cast<const T*>(p.k_pool) + col, reinterpret_cast<const T*>(p.v_pool) + col,
+            p.req_to_token + p.req_pool_indices[e_req] * p.rtt_stride, static_cast<int64_t>(p.Hk) * kPfD,
+            max(0, lim - p.window + 1), lim + 1, c, __shfl_sync(0xffffffffu, e_scale, src),
+            __shfl_sync(0xffffffffu, e_m_off, src));
+        const float inv = __shfl_sync(0xffffffffu, inv_l, src);
+        const uint32_t pair = pack2<T>(f.x * inv, f.y * inv);
+        if (stage != nullptr)
+          *reinterpret_cast<uint32_t*>(stage + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4) = pair;
+        else
+          *reinterpret_cast<uint32_t*>(reinterpret_cast<T*>(p.out) + static_cast<int64_t>(e_q_row0 + r) * p.out_stride +
+                                       static_cast<int64_t>(e_head) * kPfD + c + 2 * lane) = pair;
+      }
+    };
     auto epilogue = [&]() {
       // last unit = half b of the last tile; S of that unit complete => PV(b) of the tile before is
       // complete, so only this one phase of pv_done[w][b] can be outstanding; PV(b) complete => PV(a)
@@ -633,6 +702,14 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           __syncwarp();
           if (lane == 0) mbar_arrive(&o_free[w]);
         }
+        float z0 = 0.f, z1 = 0.f;  // kWin: NaN when a value of these columns is infinite or NaN
+        if constexpr (kWin) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            z0 = fmaf(__uint_as_float(a[i]), 0.f, z0);
+            z1 = fmaf(__uint_as_float(b[i]), 0.f, z1);
+          }
+        }
         uint4 v[8];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -652,15 +729,19 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 #pragma unroll
           for (int i = 0; i < 8; ++i)  // [128 rows x 128 B], 128-byte swizzle: chunk ^ (row % 8)
             *reinterpret_cast<uint4*>(stage + row * 128 + ((i ^ (row & 7)) << 4)) = v[i];
+          if constexpr (kWin) rows_alone(z0 + z1, c, inv_l, stage);
           fence_proxy_async_smem();
           asm volatile("bar.sync %0, 128;" ::"r"(2 + w) : "memory");
           if (row == 0) {
             tma_store_2d(&tmO, stage, e_head * kPfD + c, e_q_row0);
             bulk_commit_group();
           }
-        } else if (row < e_rows) {
+        } else {
+          if (row < e_rows) {
 #pragma unroll
-          for (int i = 0; i < 8; ++i) *reinterpret_cast<uint4*>(dst + c + 8 * i) = v[i];
+            for (int i = 0; i < 8; ++i) *reinterpret_cast<uint4*>(dst + c + 8 * i) = v[i];
+          }
+          if constexpr (kWin) rows_alone(row < e_rows ? z0 + z1 : 0.f, c, inv_l, nullptr);
         }
       }
       if (tracer) pf_trace<kTrace>(p, w, tn, 0x600);  // O stored
@@ -771,6 +852,13 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       e_head = head;
       e_q_row0 = q_row0;
       e_u = u;
+      if constexpr (kWin) {
+        e_req = it.req;
+        e_hk = it.hk;
+        e_limit = limit;
+        e_scale = scale;
+        e_m_off = m_used == -INFINITY ? 0.f : m_used * scale;
+      }
       epilogue();
     }
   }
@@ -849,6 +937,8 @@ int attn_prefill_window_try(void* out, const void* q, const void* k_pool, const 
                         extend_start_loc, batch, total_tokens, max_extend_len, H, G, q_stride, out_stride, r2t_stride,
                         sm_scale))
     return rc;
+  p.q = q;
+  p.q_stride = q_stride;
   p.window = window > 0 && window < (1 << 30) ? window : 1 << 30;
   p.sinks = sinks;
   p.qtemp_coef = qtemp_coef;

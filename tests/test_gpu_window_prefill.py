@@ -9,7 +9,8 @@ DEV = "cuda"
 D = 128
 
 
-def _run(pre, ext, H, G, window, dtype, sinks=None, qtemp=(0.0, 0), scattered=False, shift=0.0, scale=D ** -0.5):
+def _run(pre, ext, H, G, window, dtype, sinks=None, qtemp=(0.0, 0), scattered=False, shift=0.0, scale=D ** -0.5,
+         odd=()):
     from semi_pd_b200 import ops
     g = torch.Generator().manual_seed(sum(ext) + 31 * H + window)
     lens = [p + e for p, e in zip(pre, ext)]
@@ -43,6 +44,12 @@ def _run(pre, ext, H, G, window, dtype, sinks=None, qtemp=(0.0, 0), scattered=Fa
         want.append(torch.einsum("hqk,khd->qhd", torch.softmax(s, -1)[..., : p + e], vv))
         o += e
     want = torch.cat(want).flatten(1)
+    blind = torch.ones(want.shape, dtype=torch.bool)  # outputs that meet none of the infinite or NaN values put in below
+    for b, pos, head, channel, value in odd:
+        v[rtt[b, pos].long(), head, channel] = value
+        at, first = sum(ext[:b]), max(0, pos - pre[b])
+        last = min(ext[b], pos - pre[b] + window) if window > 0 else ext[b]
+        blind.view(-1, H, D)[at + first: at + max(first, last), head * (H // G): (head + 1) * (H // G), channel] = False
     i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
     out = ops.attn_general(q.flatten(1).to(DEV), k.to(DEV), v.to(DEV), rtt.to(DEV), torch.arange(len(ext), device=DEV), H, G,
                            D, D, scale, window=window, sinks=None if sk is None else sk.to(DEV), qtemp_coef=qtemp[0],
@@ -50,8 +57,10 @@ def _run(pre, ext, H, G, window, dtype, sinks=None, qtemp=(0.0, 0), scattered=Fa
                            extend_start_loc=i32([sum(ext[:b]) for b in range(len(ext))]), max_extend_len=max(ext))
     # P and the output are rounded to 16 bits: relative 2^-9 (2^-12) each of values up to |v| ~ 5
     tol = 3e-2 if dtype == torch.bfloat16 else 4e-3
-    err = (out.cpu().double() - want).abs().max().item()
+    out = out.cpu().double()
+    err = (out - want)[blind].abs().max().item()
     assert err < tol, err
+    assert not out[~blind].isfinite().any()
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
@@ -81,6 +90,16 @@ def test_scores_far_from_zero(shift):
 
 def test_large_sinks_and_empty_requests():
     _run([100, 50, 0], [256, 0, 200], 4, 2, 512, torch.bfloat16, sinks=150.0)
+
+
+@pytest.mark.parametrize("H,G,window", [(4, 2, 512), (3, 3, 130), (4, 2, -1), (2, 1, 1)])
+@pytest.mark.parametrize("scattered", [False, True])
+def test_values_that_are_not_finite_reach_only_the_rows_that_see_them(H, G, window, scattered):
+    # a later token of the same tile, a token that the window has left within it and before it, cached ones
+    nan, inf = float("nan"), float("inf")
+    odd = [(0, 700, 0, 5, nan), (0, 1024, 0, 100, inf), (1, 333, G - 1, 64, -inf), (1, 1600, G - 1, 0, nan)]
+    for dtype in (torch.bfloat16, torch.float16):
+        _run([0, 600], [1030, 1100], H, G, window, dtype, sinks=1.0, qtemp=(0.3, 128), scattered=scattered, odd=odd)
 
 
 def test_negative_scale_and_temperature_keep_their_results():
