@@ -201,9 +201,12 @@ int spd_attn_prefill_ragged(void* out, const void* q, const void* k_pool, const 
                             int sm_budget, spd_stream_t stream);
 /* Batched paged-decode attention: one query row per request over its seq_lens[b] cached rows
  * (including the token just written).  Split-KV with an in-kernel merge; workspace from
- * spd_attn_decode_workspace_bytes(), zeroed once before its first use (it is used at any batch size; each call leaves its
- * counters at zero), one per stream.  replaces FlashInferAttnBackend.forward_decode
- * (flashinfer_backend.py:454-488); semantics torch_native_backend.py:111-179. */
+ * spd_attn_decode_workspace_bytes(), zeroed once before its first use (each call leaves its counters at zero), one per
+ * stream.  A call with batch * num_kv_heads >= the SMs it may occupy does not touch it (it may be NULL).
+ * replaces FlashInferAttnBackend.forward_decode (flashinfer_backend.py:454-488); semantics
+ * torch_native_backend.py:111-179.
+ * spd_attn_decode_paged_own: the workspace is zeroed and belongs to this stream's calls of every batch size, so that
+ * requests are also cut where they are many but of unequal work (NULL or too small for that: they are not). */
 int64_t spd_attn_decode_workspace_bytes(int64_t max_batch, int num_q_heads, int head_dim);
 int spd_attn_decode_paged(void* out, const void* q, const void* k_pool, const void* v_pool,
                           const int32_t* req_to_token, const int64_t* req_pool_indices,
@@ -211,6 +214,12 @@ int spd_attn_decode_paged(void* out, const void* q, const void* k_pool, const vo
                           int num_kv_heads, int head_dim, int64_t q_stride, int64_t out_stride,
                           int64_t req_to_token_stride, float sm_scale, int dtype, void* workspace,
                           int64_t workspace_bytes, int sm_budget, spd_stream_t stream);
+int spd_attn_decode_paged_own(void* out, const void* q, const void* k_pool, const void* v_pool,
+                              const int32_t* req_to_token, const int64_t* req_pool_indices,
+                              const int64_t* seq_lens, int64_t batch, int num_q_heads,
+                              int num_kv_heads, int head_dim, int64_t q_stride, int64_t out_stride,
+                              int64_t req_to_token_stride, float sm_scale, int dtype, void* workspace,
+                              int64_t workspace_bytes, int sm_budget, spd_stream_t stream);
 /* Plain SIMT implementations of the two calls above (no tensor cores).  Bring-up / on-device
  * cross-check only; the product path never calls them. */
 int spd_attn_prefill_simt(void* out, const void* q, const void* k_pool, const void* v_pool,

@@ -69,6 +69,10 @@ SIGNATURES = {
         _i,
         [_p, _p, _p, _p, _p, _p, _p, _i64, _i, _i, _i, _i64, _i64, _i64, _f, _i, _p, _i64, _i, _p],
     ),
+    "spd_attn_decode_paged_own": (
+        _i,
+        [_p, _p, _p, _p, _p, _p, _p, _i64, _i, _i, _i, _i64, _i64, _i64, _f, _i, _p, _i64, _i, _p],
+    ),
     "spd_comm_create": (_i, [_i, _i, _i64, C.POINTER(_p), _p]),
     "spd_comm_connect": (_i, [_p, _p]),
     "spd_comm_max_bytes": (_i64, [_p]),

@@ -136,13 +136,13 @@ class SpdAttnBackend(AttentionBackend):
         # cross-checks and serves the head_dim-64 plumbing model (OPT-125m)
         self.impl = os.environ.get("SPD_ATTN_IMPL", "tc" if self.head_dim == 128 else "simt")
         self.max_extend_len = 0
-        # Split-KV scratch of the decode kernel.  Captured CUDA graphs bake its address in, so it
-        # is allocated exactly ONCE here and never replaced: the kernel only splits when
-        # batch x kv_heads is below the SM count, i.e. for at most ceil(SMs / kv_heads) requests,
-        # which bounds the scratch whatever batch size an eager step later runs with.
+        # Scratch of the decode kernel: 64 KB of arrival counters, zeroed here and left at zero by every call, and two
+        # parts of requests per CTA, whatever the batch size (sized for the largest batch that must bring one).  It
+        # belongs to this worker's stream alone.  Captured CUDA graphs bake its address in, so it is allocated exactly
+        # ONCE here and never replaced.
         if self.is_mla:
-            # absorbed MLA: one latent "kv head"; the split-KV scratch of spd_attn_mla (bounded by
-            # 2 x SMs query tokens, see csrc/attn_mla.cu) — allocated once, like the one below
+            # absorbed MLA: one latent "kv head"; the scratch of spd_attn_mla (two parts of items per CTA) —
+            # allocated once, like the one below
             cfg = model_runner.model_config
             need = ops.lib.spd_attn_mla_workspace_bytes(self.num_q_heads, cfg.kv_lora_rank)
             self.mla_workspace = torch.zeros((need,), dtype=torch.uint8, device=self.device)
@@ -329,7 +329,7 @@ class SpdAttnBackend(AttentionBackend):
             q, k_buf, v_buf, forward_batch.req_to_token_pool.req_to_token,
             forward_batch.req_pool_indices, forward_batch.seq_lens, layer.tp_q_head_num,
             layer.tp_k_head_num, layer.head_dim, layer.scaling, impl=self.impl,
-            workspace=self.decode_workspace)
+            workspace=self.decode_workspace, own_workspace=True)
 
     def forward_mla(self, q_lat, layer: RadixAttention, forward_batch: ForwardBatch):
         """Absorbed MLA attention over the latent pool (DeepseekV2AttentionMLA.forward_absorb's

@@ -649,14 +649,13 @@ int check_attn_args(const char* fn, const void* out, const void* q, const void* 
 
 using namespace spd;
 
-extern "C" int spd_attn_decode_paged(void* out, const void* q, const void* k_pool,
-                                     const void* v_pool, const int32_t* req_to_token,
-                                     const int64_t* req_pool_indices, const int64_t* seq_lens,
-                                     int64_t batch, int num_q_heads, int num_kv_heads, int head_dim,
-                                     int64_t q_stride, int64_t out_stride,
-                                     int64_t req_to_token_stride, float sm_scale, int dtype,
-                                     void* workspace, int64_t workspace_bytes, int sm_budget,
-                                     spd_stream_t stream) {
+// own_workspace: the workspace is zeroed and this stream's alone at every batch size (spd_attn_decode_paged_own), so items
+// may also be cut where their number fills the SMs; otherwise such a call leaves it untouched.
+static int attn_decode(void* out, const void* q, const void* k_pool, const void* v_pool, const int32_t* req_to_token,
+                       const int64_t* req_pool_indices, const int64_t* seq_lens, int64_t batch, int num_q_heads,
+                       int num_kv_heads, int head_dim, int64_t q_stride, int64_t out_stride, int64_t req_to_token_stride,
+                       float sm_scale, int dtype, void* workspace, int64_t workspace_bytes, bool own_workspace,
+                       int sm_budget, spd_stream_t stream) {
   int rc = check_attn_args("spd_attn_decode_paged", out, q, k_pool, v_pool, req_to_token,
                            req_pool_indices, num_q_heads, num_kv_heads, head_dim, q_stride, out_stride);
   if (rc) return rc;
@@ -686,6 +685,8 @@ extern "C" int spd_attn_decode_paged(void* out, const void* q, const void* k_poo
     SPD_REQUIRE(workspace && workspace_bytes >= spd_attn_decode_workspace_bytes(batch, num_q_heads, head_dim),
                 SPD_E_WORKSPACE, "spd_attn_decode_paged: workspace too small (%lld bytes)",
                 (long long)workspace_bytes);
+  else if (!own_workspace)
+    workspace = nullptr;
   // Items may be cut where a workspace is there: two parts per CTA (with pairs < sms it holds those of 16 CTAs per pair at
   // least).  Whether they are, the kernel decides by the lengths.
   const int64_t cta_bytes = 2ll * (num_q_heads / num_kv_heads) * (head_dim + 2) * 4;
@@ -722,4 +723,25 @@ extern "C" int spd_attn_decode_paged(void* out, const void* q, const void* k_poo
     SPD_CUDA(launch(kern, dim3(grid), dim3(kDcThreads), kDcSmem, as_stream(stream), pdl_enabled(), tk, tv, p));
   });
   return 0;
+}
+
+extern "C" int spd_attn_decode_paged(void* out, const void* q, const void* k_pool, const void* v_pool,
+                                     const int32_t* req_to_token, const int64_t* req_pool_indices, const int64_t* seq_lens,
+                                     int64_t batch, int num_q_heads, int num_kv_heads, int head_dim, int64_t q_stride,
+                                     int64_t out_stride, int64_t req_to_token_stride, float sm_scale, int dtype,
+                                     void* workspace, int64_t workspace_bytes, int sm_budget, spd_stream_t stream) {
+  return attn_decode(out, q, k_pool, v_pool, req_to_token, req_pool_indices, seq_lens, batch, num_q_heads, num_kv_heads,
+                     head_dim, q_stride, out_stride, req_to_token_stride, sm_scale, dtype, workspace, workspace_bytes, false,
+                     sm_budget, stream);
+}
+
+extern "C" int spd_attn_decode_paged_own(void* out, const void* q, const void* k_pool, const void* v_pool,
+                                         const int32_t* req_to_token, const int64_t* req_pool_indices,
+                                         const int64_t* seq_lens, int64_t batch, int num_q_heads, int num_kv_heads,
+                                         int head_dim, int64_t q_stride, int64_t out_stride, int64_t req_to_token_stride,
+                                         float sm_scale, int dtype, void* workspace, int64_t workspace_bytes, int sm_budget,
+                                         spd_stream_t stream) {
+  return attn_decode(out, q, k_pool, v_pool, req_to_token, req_pool_indices, seq_lens, batch, num_q_heads, num_kv_heads,
+                     head_dim, q_stride, out_stride, req_to_token_stride, sm_scale, dtype, workspace, workspace_bytes, true,
+                     sm_budget, stream);
 }

@@ -489,8 +489,13 @@ def _attn_workspace(device, batch: int, hq: int, d: int) -> torch.Tensor:
 
 
 def attn_decode(q, k_pool, v_pool, req_to_token, req_pool_indices, seq_lens, num_q_heads,
-                num_kv_heads, head_dim, sm_scale, out=None, impl: str = "tc", workspace=None):
+                num_kv_heads, head_dim, sm_scale, out=None, impl: str = "tc", workspace=None,
+                own_workspace: bool = False):
+    """own_workspace: `workspace` was zeroed once, is never replaced and serves one stream at a time at every batch size;
+    without that promise a batch that fills the SMs leaves it untouched (and cuts no request)."""
     _cuda(q, k_pool, v_pool, req_to_token, req_pool_indices, seq_lens)
+    if own_workspace and workspace is None:
+        raise RuntimeError("attn_decode: own_workspace needs a workspace")
     B = q.shape[0]
     q2 = q.view(B, -1)
     if out is None:
@@ -499,12 +504,11 @@ def attn_decode(q, k_pool, v_pool, req_to_token, req_pool_indices, seq_lens, num
         raise RuntimeError("attn_decode: req_pool_indices and seq_lens must be int64")
     ws = workspace if workspace is not None else _attn_workspace(q.device, B, num_q_heads, head_dim)
     if impl == "tc":
-        check(lib.spd_attn_decode_paged(out.data_ptr(), q2.data_ptr(), k_pool.data_ptr(),
-                                        v_pool.data_ptr(), req_to_token.data_ptr(),
-                                        req_pool_indices.data_ptr(), seq_lens.data_ptr(), B,
-                                        num_q_heads, num_kv_heads, head_dim, q2.stride(0),
-                                        out.stride(0), req_to_token.stride(0), float(sm_scale),
-                                        _dt(q), ws.data_ptr(), ws.numel(), get_sm_budget(), _stream()),
+        call = lib.spd_attn_decode_paged_own if own_workspace else lib.spd_attn_decode_paged
+        check(call(out.data_ptr(), q2.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), req_to_token.data_ptr(),
+                   req_pool_indices.data_ptr(), seq_lens.data_ptr(), B, num_q_heads, num_kv_heads, head_dim,
+                   q2.stride(0), out.stride(0), req_to_token.stride(0), float(sm_scale), _dt(q), ws.data_ptr(),
+                   ws.numel(), get_sm_budget(), _stream()),
               "spd_attn_decode_paged")
     elif impl == "simt":
         check(lib.spd_attn_decode_simt(out.data_ptr(), q2.data_ptr(), k_pool.data_ptr(),
