@@ -285,10 +285,12 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
   int total = 0;
 #pragma unroll
   for (int w = 0; w < kDcThreads / 32; ++w) total += s_scan[w];
-  // Whole items leave SMs idle for what the last round of the stride lacks.  A cut costs two partial epilogues and a merge
-  // per CTA, about five tiles' time in all: it pays where that idle time is longer (or where there are fewer items than
-  // SMs).  20 requests x 8 heads on 148 SMs: 400 tokens 12.6 us whole / 15.5 cut, 1000 21.4 / 21.5, 3000 67 / 45.
-  const bool whole = p.idle * static_cast<float>(total) < 5.f;
+  // Whole items leave SMs idle for what the last round of the stride lacks, and the SMs that are not have the memory to
+  // themselves; a cut costs two partial epilogues and a merge per CTA.  It pays where the idle time is longer than about
+  // 18 tiles' (or where there are fewer items than SMs).  8 kv heads on 148 SMs, pages and workspace not in L2, idle tiles:
+  // us whole / cut: 64 requests x 1088 tokens 5.8: 64.5 / 66; 56 x 1088 10.3: 56.3 / 58.2; 19 x 2000 16.6: 39.8 / 43.9;
+  // 56 x 2000 16.6: 86.9 / 92; 26 x 4000 19.4: 102 / 89; 40 x 4000 27.4: 143 / 126; 19 x 4000 31.8: 92 / 70.
+  const bool whole = p.idle * static_cast<float>(total) < 18.f;
   int per = 1, u_begin = 0, u_end = 0;
   if (!whole) {
     int incl = sum, before = 0;
@@ -695,10 +697,8 @@ static int attn_decode(void* out, const void* q, const void* k_pool, const void*
   const bool whole = pairs > 16384 || (pairs >= sms ? room < most : room < 1);
   const int grid = static_cast<int>(whole ? (pairs < most ? pairs : most) : (room < most ? room : most));
   if (!whole) {
-    // items per CTA in whole rounds, less what they come to on average, as a share of all items; of two rounds the second
-    // runs on few SMs that have the memory to themselves, so the bound is nine tiles there
+    // items per CTA in whole rounds, less what they come to on average, as a share of all items
     p.idle = pairs < grid ? INFINITY : static_cast<float>((pairs + grid - 1) / grid) / pairs - 1.f / grid;
-    if (pairs < 2ll * grid) p.idle *= 5.f / 9.f;
     // layout (attn_simt.cu: spd_attn_decode_workspace_bytes): counters at a fixed offset first
     p.counters = reinterpret_cast<int*>(workspace);
     p.o_part = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(workspace) + 65536);
