@@ -19,7 +19,8 @@
 // K is stored once: rows of tokens serve Q K^T as K-major and K^T V' as MN-major operand.  Rows past the portion are
 // zeros.  What bounds it: the chain of a chunk (split 2800 clk, Q K^T and
 // Q S 3600, A 800, A V and the rest 3000), one after another in a CTA that fills an SM.  4 requests, 8192 tokens, 16 heads
-// of 128 x 128: 875 us token by token, 256 us here (41 chunks of 6 us for the longest request).
+// of 128 x 128: 875 us token by token, 265 us here (41 chunks of 6.4 us for the longest request; 256 without the watch for
+// values that cannot be split, see rc_watch).
 //
 // The sums of a portion are cut every 64 tokens from its start, so results depend in their last bits on how a prompt is
 // cut into portions (the token-by-token kernel's do not).
@@ -64,14 +65,18 @@ __device__ __forceinline__ void rc_split2(float x0, float x1, uint32_t& h, uint3
   f = unpack2<__nv_bfloat16>(m);
   l = pack2<__nv_bfloat16>(x0 - f.x, x1 - f.y);
 }
-// eight numbers -> one 16-byte chunk per part at dst, dst + part, dst + 2 part
-__device__ __forceinline__ void rc_split8(const float (&x)[8], uint8_t* dst, int part) {
+// eight numbers -> one 16-byte chunk per part at dst, dst + part, dst + 2 part; the upper parts
+struct RcUpper {
+  uint32_t h[4];
+};
+__device__ __forceinline__ RcUpper rc_split8(const float (&x)[8], uint8_t* dst, int part) {
   uint32_t h[4], m[4], l[4];
 #pragma unroll
   for (int e = 0; e < 4; ++e) rc_split2(x[2 * e], x[2 * e + 1], h[e], m[e], l[e]);
   *reinterpret_cast<uint4*>(dst) = make_uint4(h[0], h[1], h[2], h[3]);
   *reinterpret_cast<uint4*>(dst + part) = make_uint4(m[0], m[1], m[2], m[3]);
   *reinterpret_cast<uint4*>(dst + 2 * part) = make_uint4(l[0], l[1], l[2], l[3]);
+  return {{h[0], h[1], h[2], h[3]}};
 }
 template <typename T>
 __device__ __forceinline__ void rc_load8(const T* p, float (&x)[8]) {
@@ -83,6 +88,16 @@ __device__ __forceinline__ void rc_load8(const T* p, float (&x)[8]) {
     x[2 * e] = f.x;
     x[2 * e + 1] = f.y;
   }
+}
+
+// Keeps watch over numbers that have no three parts (an infinity or NaN: inf - inf), and over ones so large that A might
+// overflow where the token-by-token sums do not: z + 2^96 h in bf16 is not finite any more once an |h| was 2^32 or more
+// (from 2^26 on where many were), and stays so.  One instruction per two numbers.
+__device__ __forceinline__ void rc_watch(uint32_t h, uint32_t& z) {
+  asm("fma.rn.bf16x2 %0, %1, %2, %0;" : "+r"(z) : "r"(h), "r"(0x6f806f80u));
+}
+__device__ __forceinline__ bool rc_spoilt(uint32_t z) {
+  return (z & 0x7f80u) == 0x7f80u || (z & 0x7f800000u) == 0x7f800000u;
 }
 
 // 16 lanes x 16 columns as mma fragments: value 4 g + e is row (lane >> 2) + 8 (e >> 1), column 8 g + 2 (lane & 3) + (e & 1)
@@ -99,13 +114,73 @@ __device__ __forceinline__ void rc_wait(uint64_t* bar, uint32_t parity, int warp
   asm volatile("bar.sync 1, %0;" ::"n"(kRcThreads) : "memory");
 }
 
+// Tokens t0 .. n - 1 of a portion one after another on the CUDA cores, as retention.cu takes them.  f: 96 KB for [64][128]
+// rotated q, rotated and scaled k, [64][64] v and [2][4][64] partial sums; state: this thread's 16 values.  Behind the
+// chunks' loop and not inside it: there the call (never made) took 40 us of 256.
+template <typename T>
+__device__ __forceinline__ void rc_token_by_token(const RetChunkParams* p, int t0, int n, int64_t pos0, int64_t row0, float* f,
+                                               float* state, float dec) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, half = p->rot >> 1, h = blockIdx.y;
+  const int sr = (warp & 3) * 32 + lane, sc = (warp >> 2) * 16, col0 = blockIdx.z * kRcDv;
+  float *fq = f, *fk = fq + kRcTok * kRcDk, *fv = fk + kRcTok * kRcDk, *part = fv + kRcTok * kRcDv;
+  float S[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) S[i] = state[i];
+#pragma unroll 1
+  for (; t0 < n; t0 += kRcTok) {
+    const int nt = min(kRcTok, n - t0);
+    __syncthreads();  // what stood in `f` has been read
+#pragma unroll 1
+    for (int i = tid; i < nt * kRcDk; i += kRcThreads) {
+      const int t = i / kRcDk, d = i % kRcDk;
+      const int64_t row = row0 + t0 + t;
+      const T* qr = reinterpret_cast<const T*>(p->q) + row * p->q_stride + h * kRcDk;
+      const T* kr = reinterpret_cast<const T*>(p->k) + row * p->k_stride + h * kRcDk;
+      float q = to_f32<T>(qr[d]), k = to_f32<T>(kr[d]);
+      if (d < p->rot) {
+        int64_t pos = pos0 + t0 + t;
+        pos = pos < p->max_positions ? pos : p->max_positions - 1;
+        const int j = d < half ? d : d - half, other = d < half ? d + half : d - half;
+        const float c = p->cos_sin[pos * p->rot + j], s = p->cos_sin[pos * p->rot + half + j];
+        const float q2 = to_f32<T>(qr[other]), k2 = to_f32<T>(kr[other]);
+        q = d < half ? q * c - q2 * s : q * c + q2 * s;
+        k = d < half ? k * c - k2 * s : k * c + k2 * s;
+      }
+      fq[i] = q;
+      fk[i] = k * p->k_scale;
+    }
+#pragma unroll 1
+    for (int i = tid; i < nt * kRcDv; i += kRcThreads)
+      fv[i] = to_f32<T>(reinterpret_cast<const T*>(p->v)[(row0 + t0 + i / kRcDv) * p->v_stride +
+                                                         static_cast<int64_t>(h) * p->dv + col0 + i % kRcDv]);
+    __syncthreads();
+#pragma unroll 1
+    for (int t = 0; t < nt; ++t) {
+      const float kt = fk[t * kRcDk + sr], qt = fq[t * kRcDk + sr];
+      float* to = part + (t & 1) * 4 * kRcDv;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        S[i] = fmaf(dec, S[i], kt * fv[t * kRcDv + sc + i]);
+        const float sum = warp_sum(S[i] * qt);
+        if (lane == 0) to[(warp & 3) * kRcDv + sc + i] = sum;
+      }
+      __syncthreads();
+      if (tid < kRcDv)
+        p->o[((row0 + t0 + t) * p->H + h) * static_cast<int64_t>(p->dv) + col0 + tid] =
+            (to[tid] + to[kRcDv + tid]) + (to[2 * kRcDv + tid] + to[3 * kRcDv + tid]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 16; ++i) state[i] = S[i];
+}
+
 // parts (a, b) of the six products, smallest first
 __host__ __device__ constexpr int rc_pa(int i) { return (0x001102 >> (4 * i)) & 15; }  // 2 0 1 1 0 0
 __host__ __device__ constexpr int rc_pb(int i) { return (0x010120 >> (4 * i)) & 15; }  // 0 2 1 0 1 0
 
 template <typename T, int VS>  // VS: bf16 parts of a value as it is stored (1: bf16, 2: fp16)
 __global__ void __launch_bounds__(kRcThreads, 1)
-retention_chunked_kernel(const RetChunkParams p) {
+retention_chunked_kernel(const __grid_constant__ RetChunkParams p) {
   extern __shared__ uint8_t rc_smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(rc_smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -176,6 +251,10 @@ retention_chunked_kernel(const RetChunkParams p) {
     const float4 x = pos0 > 0 ? *reinterpret_cast<const float4*>(st + i) : make_float4(0.f, 0.f, 0.f, 0.f);
     S[i] = x.x; S[i + 1] = x.y; S[i + 2] = x.z; S[i + 3] = x.w;
   }
+  // the same watch over the state a portion starts from; what inputs below 2^32 add to it stays far from fp32's end
+  bool odd_state = false;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) odd_state |= !(fabsf(S[i]) <= 0x1p64f);
   auto put_state = [&]() {
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
@@ -210,21 +289,18 @@ retention_chunked_kernel(const RetChunkParams p) {
     }
   };
   angles(0);
-  int nt = 0;
-  for (int t0 = 0, it = 0; t0 < n; t0 += nt, ++it) {
-    const uint32_t par = it & 1;
-    cp_async_wait<0>();
-    bool odd = false;  // an infinite or NaN value among those this thread has fetched
-    float v8[8];
-    {
-      rc_load8<T>(rv + ut * kRcDv + u * 8, v8);
+  auto store_state = [&]() {
 #pragma unroll
-      for (int e = 0; e < 8; ++e) odd |= !(fabsf(v8[e]) <= 3.4028235e38f);
-    }
+    for (int i = 0; i < 16; i += 4) *reinterpret_cast<float4*>(st + i) = make_float4(S[i], S[i + 1], S[i + 2], S[i + 3]);
+  };
+  int t_odd = n;
+  uint32_t par = 0;
+  for (int t0 = 0; t0 < n; t0 += kRcTok, par ^= 1) {
+    const int nt = min(kRcTok, n - t0);
+    cp_async_wait<0>();
     tc_fence_before_sync();
-    // raw rows visible; the previous chunk's operands and accumulators have been read.  With such a value the zeros of the
-    // masked A would spoil the tokens before it: its chunk is taken one token at a time.
-    nt = __syncthreads_or(odd) ? 1 : min(kRcTok, n - t0);
+    __syncthreads();  // raw rows visible; the previous chunk's operands and accumulators have been read
+    uint32_t z = 0;
     {
       // ---- q, k: rotate, split: 16 channels of a token and of each ----
       const bool live = ut < nt;
@@ -247,11 +323,18 @@ retention_chunked_kernel(const RetChunkParams p) {
           for (int e = 0; e < 8; ++e) x[e] = y[e] = 0.f;
         }
         uint8_t* dst = w ? sK : sQ;
-        rc_split8(x, dst + (d0 >> 6) * kRcV + rc_off(ut, (d0 >> 3) & 7), kRcQ);
-        rc_split8(y, dst + (d1 >> 6) * kRcV + rc_off(ut, (d1 >> 3) & 7), kRcQ);
+        const RcUpper hx = rc_split8(x, dst + (d0 >> 6) * kRcV + rc_off(ut, (d0 >> 3) & 7), kRcQ);
+        const RcUpper hy = rc_split8(y, dst + (d1 >> 6) * kRcV + rc_off(ut, (d1 >> 3) & 7), kRcQ);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          rc_watch(hx.h[e], z);
+          rc_watch(hy.h[e], z);
+        }
       }
       // ---- v, v' ----
       {
+        float v8[8];
+        rc_load8<T>(rv + ut * kRcDv + u * 8, v8);
         if (!live) {
 #pragma unroll
           for (int e = 0; e < 8; ++e) v8[e] = 0.f;
@@ -259,7 +342,10 @@ retention_chunked_kernel(const RetChunkParams p) {
         const uint32_t off = rc_off(ut, u);
         uint32_t hh[4], mm[4], ll;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) rc_split2(v8[2 * e], v8[2 * e + 1], hh[e], mm[e], ll);
+        for (int e = 0; e < 4; ++e) {
+          rc_split2(v8[2 * e], v8[2 * e + 1], hh[e], mm[e], ll);
+          rc_watch(hh[e], z);
+        }
         *reinterpret_cast<uint4*>(sV + off) = make_uint4(hh[0], hh[1], hh[2], hh[3]);
         if constexpr (VS == 2) *reinterpret_cast<uint4*>(sV + kRcV + off) = make_uint4(mm[0], mm[1], mm[2], mm[3]);
         const float f = pw[max(nt - 1 - ut, 0)] * p.k_scale;
@@ -269,7 +355,11 @@ retention_chunked_kernel(const RetChunkParams p) {
       }
     }
     fence_proxy_async_smem();
-    __syncthreads();
+    // the first chunk with a value that has no parts: it and what follows are done again, from this state, behind the loop
+    if (__syncthreads_or(rc_spoilt(z) || odd_state) && t0 < t_odd) {
+      t_odd = t0;
+      store_state();
+    }
     tc_fence_after_sync();
     const uint32_t tm = *tmem_slot;
     const uint32_t tA = tm, tO1 = tm + 64, tO2 = tm + 128, tU = tm + 192;
@@ -398,10 +488,12 @@ retention_chunked_kernel(const RetChunkParams p) {
       }
     }
   }
-#pragma unroll
-  for (int i = 0; i < 16; i += 4) *reinterpret_cast<float4*>(st + i) = make_float4(S[i], S[i + 1], S[i + 2], S[i + 3]);
   tc_fence_before_sync();
   __syncthreads();
+  if (t_odd < n)
+    rc_token_by_token<T>(&p, t_odd, n, pos0, row0, reinterpret_cast<float*>(sQ), st, pw[1]);
+  else
+    store_state();
   if (warp == 0) tmem_dealloc(*tmem_slot, 256);
   if (*dead && tid == 0) atomicAdd(&g_rc_wait_expired, 1u);
 }

@@ -97,6 +97,42 @@ def test_values_that_are_not_finite_leave_the_tokens_before_them_alone():
     assert _rel(o[seen], wo[seen]) < 1e-6
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("what", ["q", "k", "state", "v", "all"])
+def test_values_that_are_not_finite_as_token_by_token(dtype, what):
+    """Infinities and NaNs in q, k, v and the state: finite, infinite (with the sign) and NaN where the token-by-token kernel
+    (taken by portions of one token) has them."""
+    H, dv, pre, ext = 2, 64, [5, 0, 9], [200, 50, 64]
+    q, k, v, state, table, decay = _case(pre, ext, H, dv, 64, dtype, [0.9, 0.5])
+    inf, nan = float("inf"), float("nan")
+    if what in ("q", "all"):  # a channel that is not rotated: 0.7 inf, then inf - inf
+        q[70, 100], q[90, DK + 3], q[249, 100], q[249, 101] = inf, nan, -inf, inf
+    if what in ("k", "all"):
+        k[130, 99], k[220, 5] = -inf, nan
+    if what in ("v", "all"):
+        v[150, 3], v[263, dv + 1], v[300, 9] = inf, -inf, nan
+    if what in ("state", "all"):
+        state[0, 1, 100, 7], state[2, 0, 1, 2] = inf, -inf
+    whole, ws = _run(q, k, v, state, table, decay, pre, ext, H, dv, 64, 1.0)
+    st, rows = state, [[], [], []]
+    starts = [0, 200, 250]
+    for t in range(max(ext)):
+        live = [r for r in range(3) if t < ext[r]]
+        at = [starts[r] + t for r in live]
+        o, s = _run(q[at], k[at], v[at], torch.cat((st[live], st[-1:])).float(), table, decay, [pre[r] + t for r in live],
+                    [1] * len(live), H, dv, 64, 1.0)
+        st = st.clone().double()
+        st[live] = s[:-1]
+        for i, r in enumerate(live):
+            rows[r].append(o[i: i + 1])
+    steps = torch.cat([torch.cat(r) for r in rows])
+    for a, b in ((whole, steps), (ws[:3], st[:3])):
+        fin = b.isfinite()
+        assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isinf(), b.isinf())
+        assert torch.equal(a[b.isinf()], b[b.isinf()])
+        assert _rel(a[fin], b[fin]) < 1e-6
+
+
 def test_strided_rows_and_a_cut_prompt():
     """q, k, v as slices of one projection; a prompt in three portions against the prompt in one."""
     H, dv, n = 2, 128, 333
