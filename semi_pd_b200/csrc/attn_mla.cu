@@ -83,7 +83,11 @@ struct MlaShape {
   static constexpr int N = TQ * kMlaHeads;
   static constexpr int E = kExtend ? 2 : 1;  // what beginning and ending an item costs, in tiles: it counts in the work split
   static constexpr int kQBytes = 9 * N * 128;
-  static constexpr int kPBytes = N * 128;
+  // P as the sum of two 16-bit numbers (decode): rounded to one, its error grew 2.3 % over the warp-level kernel's, whose
+  // shorter tiles and splits had more probabilities that are exactly 1 (extend: 0.1 % of a layer's, and no room for it)
+  static constexpr int kPParts = kExtend ? 1 : 2;
+  static constexpr int kPPart = N * 128;
+  static constexpr int kPBytes = kPParts * kPPart;
   static constexpr int kPairs = kExtend ? 8 : 11;  // ring slots of 16 KB: one pair of 64-column blocks of a tile
   static constexpr int kRopes = kExtend ? 2 : 3;   // ring slots of 8 KB: a tile's rope block
   static constexpr int kRing = kPairs * 2 * kMlaBlk + kRopes * kMlaBlk;
@@ -489,6 +493,10 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
             const uint32_t acc = (!first || k > 0) ? 1u : 0u;
             umma_ss_lo(tmem_O + i * N, v0 + k * 128, p_lo + k * 2, hi, idesc_o, acc);
             umma_ss_lo(tmem_O + (i + 1) * N, v1 + k * 128, p_lo + k * 2, hi, idesc_o, acc);
+            if constexpr (S::kPParts == 2) {
+              umma_ss_lo(tmem_O + i * N, v0 + k * 128, p_lo + (S::kPPart >> 4) + k * 2, hi, idesc_o, 1u);
+              umma_ss_lo(tmem_O + (i + 1) * N, v1 + k * 128, p_lo + (S::kPPart >> 4) + k * 2, hi, idesc_o, 1u);
+            }
           }
           umma_commit(&k_empty[slot0]);
           umma_commit(&k_empty[slot1]);
@@ -646,8 +654,7 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
         if (mla_bar_or(exceed)) {
           // The true running max per column, so that a column's largest P is exactly 1: a reference that lags by up to 2^8
           // saves most of these rescales but rounds that P too (decode: 32.4 instead of 33.8 us and extend 548
-          // instead of 600, but 6 - 14 % more rms error of a decode against 64-bit results; what is left is about 2.5 %, perhaps the
-          // max being taken per 64 keys where the warp-level kernel took it per 32).
+          // instead of 600, but 6 - 14 % more rms error against 64-bit results where P has one part).
 #pragma unroll
           for (int i = 0; i < C; ++i) {
             float m = fmaxf(s[(i >> 1) * 4 + (i & 1)], s[(i >> 1) * 4 + 2 + (i & 1)]);
@@ -687,25 +694,34 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
           mla_bar();  // red / s_col may be written again
         }
         // P^T -> shared memory (B operand, K-major: row = column of the item, 64 kv); sums of what is multiplied
-        uint32_t pk[N / 4];
+        uint32_t pk[N / 4], pk2[S::kPParts == 2 ? N / 4 : 1];
 #pragma unroll
         for (int g = 0; g < N / 8; ++g)
 #pragma unroll
           for (int x = 0; x < 2; ++x) {
             const float m0 = m_ref[2 * g] == -INFINITY ? 0.f : m_ref[2 * g];
             const float m1 = m_ref[2 * g + 1] == -INFINITY ? 0.f : m_ref[2 * g + 1];
-            pk[2 * g + x] = pack2<T>(fast_exp2(s[4 * g + 2 * x] - m0), fast_exp2(s[4 * g + 2 * x + 1] - m1));
+            const float p0 = fast_exp2(s[4 * g + 2 * x] - m0), p1 = fast_exp2(s[4 * g + 2 * x + 1] - m1);
+            pk[2 * g + x] = pack2<T>(p0, p1);
             const float2 v = unpack2<T>(pk[2 * g + x]);
-            l_thr[2 * g] += v.x;
-            l_thr[2 * g + 1] += v.y;
+            if constexpr (S::kPParts == 2) {
+              pk2[2 * g + x] = pack2<T>(p0 - v.x, p1 - v.y);
+              l_thr[2 * g] += p0;
+              l_thr[2 * g + 1] += p1;
+            } else {
+              l_thr[2 * g] += v.x;
+              l_thr[2 * g + 1] += v.y;
+            }
           }
         mbar_wait_bounded(p_empty, (t & 1) ^ 1, dead);
 #pragma unroll
         for (int g = 0; g < N / 8; g += 2) {
           // matrices: (columns 8 g.., kv 0-7), (8 g.., kv 8-15), (8 (g + 1).., kv 0-7), (8 (g + 1).., kv 8-15)
           const int row = 8 * (g + (lane >> 4)) + (lane & 7);
-          mla_stsm_x4_t(smem_u32(sP + mla_off(row, warp * 2 + ((lane >> 3) & 1))), pk[2 * g], pk[2 * g + 1], pk[2 * g + 2],
-                        pk[2 * g + 3]);
+          const uint32_t at = smem_u32(sP + mla_off(row, warp * 2 + ((lane >> 3) & 1)));
+          mla_stsm_x4_t(at, pk[2 * g], pk[2 * g + 1], pk[2 * g + 2], pk[2 * g + 3]);
+          if constexpr (S::kPParts == 2)
+            mla_stsm_x4_t(at + S::kPPart, pk2[2 * g], pk2[2 * g + 1], pk2[2 * g + 2], pk2[2 * g + 3]);
         }
         fence_proxy_async_smem();
         mbar_arrive(p_full);
