@@ -444,10 +444,23 @@ def mla_rotary_store(qa: torch.Tensor, q_lat: torch.Tensor, kv_pool: torch.Tenso
         raise RuntimeError("mla_rotary_store: cos_sin_cache is float32, positions are int64")
     if not (qa.dtype == q_lat.dtype == kv_pool.dtype == norm_weight.dtype):
         raise RuntimeError("mla_rotary_store: qa, q_lat, the pool and the norm weight share a dtype")
+    T, DL = qa.shape[0], kv_lora_rank + rope_dim
+    if qa.dim() != 2 or qa.shape[1] != num_heads * (nope_dim + rope_dim) + DL or qa.stride(1) != 1:
+        raise RuntimeError("mla_rotary_store: qa is [T, H (nope + rope) + kv_lora + rope] with contiguous rows")
+    if tuple(q_lat.shape) != (T, num_heads * DL) or (T and q_lat.stride(1) != 1):
+        raise RuntimeError("mla_rotary_store: q_lat is [T, H (kv_lora + rope)] with contiguous rows")
+    if kv_pool.shape[-1] != DL or not kv_pool.is_contiguous() or kv_pool.numel() != kv_pool.shape[0] * DL:
+        raise RuntimeError("mla_rotary_store: the pool is contiguous rows of kv_lora + rope")
+    if any(tuple(t.shape) != (T,) or not t.is_contiguous() for t in (positions, loc)):
+        raise RuntimeError("mla_rotary_store: one position and one slot per row of qa, contiguous")
+    if tuple(norm_weight.shape) != (kv_lora_rank,) or not norm_weight.is_contiguous():
+        raise RuntimeError("mla_rotary_store: the norm weight is [kv_lora], contiguous")
+    if cos_sin_cache.dim() != 2 or cos_sin_cache.shape[1] != rope_dim or not cos_sin_cache.is_contiguous():
+        raise RuntimeError("mla_rotary_store: cos_sin_cache is [positions, rope], contiguous")
     if loc.dtype != torch.int64:
         loc = loc.long()
     check(lib.spd_mla_rotary_store(q_lat.data_ptr(), qa.data_ptr(), kv_pool.data_ptr(), norm_weight.data_ptr(),
-                                   cos_sin_cache.data_ptr(), positions.data_ptr(), loc.data_ptr(), qa.shape[0], num_heads,
+                                   cos_sin_cache.data_ptr(), positions.data_ptr(), loc.data_ptr(), T, num_heads,
                                    nope_dim, kv_lora_rank, rope_dim, qa.stride(0), q_lat.stride(0), float(eps), _dt(qa),
                                    _stream()), "spd_mla_rotary_store")
 

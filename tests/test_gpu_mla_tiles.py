@@ -171,3 +171,35 @@ def test_rotary_store(dtype, T, H):
     tol = 2 ** -11 * 8 + 1e-5 if dtype == torch.float16 else 2 ** -8 * 8 + 1e-5
     assert (pool.cpu().double()[:, 0] - want).abs().max().item() < tol
     assert (q_lat.cpu().double().view(T, H, -1) - q_want).abs().max().item() < tol
+
+
+def test_rotary_store_refuses_what_it_would_read_past():
+    from semi_pd_b200 import ops
+    H, nope, T = 2, 128, 5
+    good = dict(qa=torch.zeros(T, H * (nope + DR) + R + DR), q_lat=torch.zeros(T, H * (R + DR)), pool=torch.zeros(9, 1, R + DR),
+                pos=torch.zeros(T, dtype=torch.int64), loc=torch.arange(T), w=torch.ones(R), table=torch.zeros(4, DR))
+    bad = [dict(qa=torch.zeros(T, H * (nope + DR) + R)), dict(qa=torch.zeros(H * (nope + DR) + R + DR, T).t()),
+           dict(q_lat=torch.zeros(T - 1, H * (R + DR))), dict(q_lat=torch.zeros(T, H * R)),
+           dict(q_lat=torch.zeros(H * (R + DR), T).t()), dict(pool=torch.zeros(9, 1, R)),
+           dict(pool=torch.zeros(9, 1, 2 * (R + DR))[..., : R + DR]), dict(pos=torch.zeros(T - 1, dtype=torch.int64)),
+           dict(pos=torch.zeros(2 * T, dtype=torch.int64)[::2]), dict(loc=torch.arange(T + 1)),
+           dict(loc=torch.arange(2 * T)[::2]), dict(w=torch.ones(R - 8)), dict(w=torch.ones(2 * R)[::2]),
+           dict(table=torch.zeros(4, DR // 2)), dict(table=torch.zeros(4, 2 * DR)[:, :DR])]
+
+    def call(a):
+        d = {}
+        for n, t in a.items():  # (the layout of the CPU tensor: .to keeps only dense strides)
+            dt = t.dtype if t.dtype == torch.int64 or n == "table" else torch.float16
+            d[n] = torch.empty(t.untyped_storage().nbytes() // t.element_size(), dtype=dt, device=DEV).as_strided(
+                t.shape, t.stride()).copy_(t)
+        ops.mla_rotary_store(d["qa"], d["q_lat"], d["pool"], d["pos"], d["loc"], d["w"], d["table"], H, nope, R, DR, 1e-6)
+
+    call(good)
+    for i, b in enumerate(bad):
+        try:
+            call({**good, **b})
+        except RuntimeError as e:
+            assert "mla_rotary_store" in str(e), (i, e)
+        else:
+            raise AssertionError(f"case {i} was accepted")
+    torch.cuda.synchronize()
