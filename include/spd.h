@@ -659,6 +659,16 @@ int spd_attn_general_keys(void* out, const void* q, const void* k_pool, const vo
                           int qtemp_every, int64_t max_extend_len, float softcap, int num_v_heads,
                           int64_t v_slot_stride, int block_size, int block_run_len, int64_t block_base, int keep_first,
                           const float* dist_bias, int dist_bias_len, int dtype, spd_stream_t stream);
+/* spd_attn_general_keys on sm_budget SMs of the device (0: all), for the forms that run one CTA per SM. */
+int spd_attn_general_sms(void* out, const void* q, const void* k_pool, const void* v_pool,
+                         const int32_t* req_to_token, const int64_t* req_pool_indices, const int64_t* seq_lens,
+                         const int32_t* prefix_lens, const int32_t* extend_lens, const int32_t* extend_start_loc,
+                         int64_t batch, int64_t total_tokens, int num_q_heads, int num_kv_heads, int head_dim,
+                         int v_dim, int64_t q_stride, int64_t out_stride, int64_t req_to_token_stride,
+                         float sm_scale, int window, const float* sinks, const float* slopes, float qtemp_coef,
+                         int qtemp_every, int64_t max_extend_len, float softcap, int num_v_heads,
+                         int64_t v_slot_stride, int block_size, int block_run_len, int64_t block_base, int keep_first,
+                         const float* dist_bias, int dist_bias_len, int dtype, int sm_budget, spd_stream_t stream);
 /* Writes the rows of the blocks that a batch's new tokens complete (their K / V are in the pool already): the mean over
  * the block's token rows of k_pool (rows of k_row_elems) and v_pool (v_row_elems; v_pool NULL: keys only), summed in
  * fp32.  Decode (seq_lens) or ragged extend (max_extend_len: host-side bound of extend_lens); slot 0 is padding. */

@@ -161,6 +161,11 @@ SIGNATURES = {
         [_p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i64, _i64, _i, _i, _i, _i, _i64, _i64, _i64, _f, _i, _p, _p,
          _f, _i, _i64, _f, _i, _i64, _i, _i, _i64, _i, _p, _i, _i, _p],
     ),
+    "spd_attn_general_sms": (
+        _i,
+        [_p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i64, _i64, _i, _i, _i, _i, _i64, _i64, _i64, _f, _i, _p, _p,
+         _f, _i, _i64, _f, _i, _i64, _i, _i, _i64, _i, _p, _i, _i, _i, _p],
+    ),
     "spd_attn_general_blocks": (
         _i,
         [_p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i64, _i64, _i, _i, _i, _i, _i64, _i64, _i64, _f, _i, _p, _p,

@@ -591,7 +591,7 @@ int attn_prefill_window_try(void* out, const void* q, const void* k_pool, const 
                             const int64_t* req_pool_indices, const int32_t* prefix_lens, const int32_t* extend_lens,
                             const int32_t* extend_start_loc, int64_t batch, int64_t total_tokens, int64_t max_extend_len,
                             int H, int G, int64_t q_stride, int64_t out_stride, int64_t r2t_stride, float sm_scale,
-                            int window, const float* sinks, float qtemp_coef, int qtemp_every, int dtype,
+                            int window, const float* sinks, float qtemp_coef, int qtemp_every, int dtype, int sm_budget,
                             cudaStream_t stream);
 
 int attn_general_mma_decode_try(void* out, const void* q, const void* k_pool, const void* v_pool,
@@ -658,7 +658,7 @@ int spd_pool_key_blocks(void* k_pool, void* v_pool, const int32_t* req_to_token,
   return 0;
 }
 
-int spd_attn_general_keys(void* out, const void* q, const void* k_pool, const void* v_pool,
+int spd_attn_general_sms(void* out, const void* q, const void* k_pool, const void* v_pool,
                           const int32_t* req_to_token, const int64_t* req_pool_indices, const int64_t* seq_lens,
                           const int32_t* prefix_lens, const int32_t* extend_lens, const int32_t* extend_start_loc,
                           int64_t batch, int64_t total_tokens, int num_q_heads, int num_kv_heads, int head_dim,
@@ -666,7 +666,8 @@ int spd_attn_general_keys(void* out, const void* q, const void* k_pool, const vo
                           float sm_scale, int window, const float* sinks, const float* slopes, float qtemp_coef,
                           int qtemp_every, int64_t max_extend_len, float softcap, int num_v_heads,
                           int64_t v_slot_stride, int block_size, int block_run_len, int64_t block_base, int keep_first,
-                          const float* dist_bias, int dist_bias_len, int dtype, spd_stream_t stream) {
+                          const float* dist_bias, int dist_bias_len, int dtype, int sm_budget,
+                         spd_stream_t stream) {
   if (num_v_heads <= 0) num_v_heads = num_kv_heads;
   if (v_slot_stride <= 0) v_slot_stride = (int64_t)num_v_heads * v_dim;
   const int Gv = num_v_heads;
@@ -762,7 +763,7 @@ int spd_attn_general_keys(void* out, const void* q, const void* k_pool, const vo
     const int rc = attn_prefill_window_try(out, q, k_pool, v_pool, req_to_token, req_pool_indices, prefix_lens, extend_lens,
                                            extend_start_loc, batch, total_tokens, max_extend_len, num_q_heads, num_kv_heads,
                                            q_stride, out_stride, req_to_token_stride, sm_scale, window, sinks, qtemp_coef,
-                                           qtemp_every, dtype, as_stream(stream));
+                                           qtemp_every, dtype, sm_budget, as_stream(stream));
     if (rc != 1) return rc;
   }
   if (max_extend_len > 0) {  // 16-bit prefill on the tensor cores where the head sizes are instantiated
@@ -785,6 +786,23 @@ int spd_attn_general_keys(void* out, const void* q, const void* k_pool, const vo
                     qtemp_coef, qtemp_every, softcap, Gv, v_slot, kb, db));
   });
   return 0;
+}
+
+int spd_attn_general_keys(void* out, const void* q, const void* k_pool, const void* v_pool,
+                          const int32_t* req_to_token, const int64_t* req_pool_indices, const int64_t* seq_lens,
+                          const int32_t* prefix_lens, const int32_t* extend_lens, const int32_t* extend_start_loc,
+                          int64_t batch, int64_t total_tokens, int num_q_heads, int num_kv_heads, int head_dim,
+                          int v_dim, int64_t q_stride, int64_t out_stride, int64_t req_to_token_stride,
+                          float sm_scale, int window, const float* sinks, const float* slopes, float qtemp_coef,
+                          int qtemp_every, int64_t max_extend_len, float softcap, int num_v_heads,
+                          int64_t v_slot_stride, int block_size, int block_run_len, int64_t block_base, int keep_first,
+                          const float* dist_bias, int dist_bias_len, int dtype, spd_stream_t stream) {
+  return spd_attn_general_sms(out, q, k_pool, v_pool, req_to_token, req_pool_indices, seq_lens, prefix_lens,
+                              extend_lens, extend_start_loc, batch, total_tokens, num_q_heads, num_kv_heads, head_dim,
+                              v_dim, q_stride, out_stride, req_to_token_stride, sm_scale, window, sinks, slopes,
+                              qtemp_coef, qtemp_every, max_extend_len, softcap, num_v_heads, v_slot_stride,
+                              block_size, block_run_len, block_base, keep_first, dist_bias, dist_bias_len, dtype, 0,
+                              stream);
 }
 
 int spd_attn_general_blocks(void* out, const void* q, const void* k_pool, const void* v_pool,

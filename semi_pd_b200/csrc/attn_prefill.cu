@@ -923,7 +923,7 @@ int attn_prefill_window_try(void* out, const void* q, const void* k_pool, const 
                             const int64_t* req_pool_indices, const int32_t* prefix_lens, const int32_t* extend_lens,
                             const int32_t* extend_start_loc, int64_t batch, int64_t total_tokens, int64_t max_extend_len,
                             int H, int G, int64_t q_stride, int64_t out_stride, int64_t r2t_stride, float sm_scale,
-                            int window, const float* sinks, float qtemp_coef, int qtemp_every, int dtype,
+                            int window, const float* sinks, float qtemp_coef, int qtemp_every, int dtype, int sm_budget,
                             cudaStream_t stream) {
   // a reference max of raw scores serves the scaled ones only where the scale is not negative
   if (!(sm_scale >= 0.f) || !(qtemp_every <= 0 || qtemp_coef >= 0.f)) return 1;
@@ -943,7 +943,7 @@ int attn_prefill_window_try(void* out, const void* q, const void* k_pool, const 
   p.sinks = sinks;
   p.qtemp_coef = qtemp_coef;
   p.qtemp_every = qtemp_every > 0 ? qtemp_every : 0;
-  const int sms = device_sm_count_cached();
+  const int sms = sm_budget > 0 ? sm_budget : device_sm_count_cached();  // items are dealt to the CTAs that run at once
   const int grid = p.total_items < sms ? p.total_items : sms;
   SPD_DISPATCH_DTYPE(dtype, {
     auto kern = attn_prefill_kernel<T, 64, false, true>;

@@ -994,14 +994,14 @@ def attn_general(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, re
             raise RuntimeError("attn_general: sinks and slopes are fp32")
     out = torch.empty((T, num_q_heads * v_dim), device=q.device, dtype=q.dtype)
     size, run_len, base = blocks or (0, 0, 0)
-    check(lib.spd_attn_general_keys(out.data_ptr(), q.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(),
+    check(lib.spd_attn_general_sms(out.data_ptr(), q.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(),
                                   req_to_token.data_ptr(), req_pool_indices.data_ptr(), _ptr(seq_lens), _ptr(prefix_lens),
                                   _ptr(extend_lens), _ptr(extend_start_loc), req_pool_indices.numel(), T, num_q_heads,
                                   num_kv_heads, head_dim, v_dim, q.stride(0), out.stride(0), req_to_token.stride(0),
                                   float(sm_scale), int(window), _ptr(sinks), _ptr(slopes), float(qtemp_coef),
                                   int(qtemp_every), int(max_extend_len), float(softcap or 0.0), int(num_v_heads),
                                   int(v_slot_stride), int(size), int(run_len), int(base), int(keep_first), _ptr(dist_bias),
-                                  dist_bias.shape[1] if dist_bias is not None else 0, _dta(q), _stream()),
+                                  dist_bias.shape[1] if dist_bias is not None else 0, _dta(q), get_sm_budget(), _stream()),
           "spd_attn_general")
     return out
 

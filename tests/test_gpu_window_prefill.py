@@ -111,3 +111,34 @@ def test_negative_scale_and_temperature_keep_their_results():
 @pytest.mark.parametrize("ext,window", [(1023, 512), (1024, 512), (1499, 128), (1500, 128)])
 def test_a_request_alone(ext, window):
     _run([77], [ext], 4, 2, window, torch.bfloat16, sinks=1.0)
+
+
+def test_the_sm_budget_bounds_the_grid():
+    """With a budget of 4 SMs a call occupies 4: it takes many times as long as on the whole device."""
+    from semi_pd_b200 import ops
+    H, G, n = 8, 2, 2048
+    k, v = (torch.randn(2 * n + 1, G, D, device=DEV).bfloat16() for _ in range(2))
+    q = torch.randn(2 * n, H * D, device=DEV).bfloat16()
+    rtt = (torch.arange(2 * n, device=DEV, dtype=torch.int32) + 1).view(2, n)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    args = (q, k, v, rtt, torch.arange(2, device=DEV), H, G, D, D, D ** -0.5)
+    more = dict(window=1024, prefix_lens=i32([0, 0]), extend_lens=i32([n, n]), extend_start_loc=i32([0, n]), max_extend_len=n)
+
+    def run(budget):
+        ops.set_sm_budget(budget)
+        try:
+            out = ops.attn_general(*args, **more)
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda.synchronize()
+            a.record()
+            for _ in range(3):
+                ops.attn_general(*args, **more)
+            b.record()
+            torch.cuda.synchronize()
+        finally:
+            ops.set_sm_budget(0)
+        return out, a.elapsed_time(b)
+
+    (whole, t_whole), (few, t_few) = run(0), run(4)
+    assert torch.equal(whole, few)
+    assert t_few > 8 * t_whole  # 64 items on 64 CTAs, or 16 rounds on 4
