@@ -32,6 +32,7 @@ typedef void* spd_stream_t; /* cudaStream_t */
 #define SPD_E_ALIGN (-2)    /* pointer or stride not 16-byte aligned / dim not multiple of 8 */
 #define SPD_E_SHAPE (-3)    /* unsupported shape (head_dim, group size, K multiple …) */
 #define SPD_E_WORKSPACE (-4)/* workspace too small */
+#define SPD_E_TIMEOUT (-6)  /* a wait inside an earlier kernel ran out (spd_wait_status) */
 #define SPD_E_DRIVER (-5)   /* driver entry point missing (green contexts, tensor maps) */
 
 /* ---------------------------------------------------------------------------------------------
@@ -39,6 +40,13 @@ typedef void* spd_stream_t; /* cudaStream_t */
  * ------------------------------------------------------------------------------------------- */
 int spd_version(void);
 const char* spd_last_error_string(void);
+/* Waits inside spd_attn_mla and spd_retention_extend are bounded (seconds).  One that runs out sets a word in host memory
+ * when its kernel ends; what that kernel wrote is not to be trusted (a recurrent state is kept as it was before the tokens
+ * the wait stood for), and those calls return SPD_E_TIMEOUT from then on.  spd_wait_status reads the word without
+ * synchronising: call it where a kernel's results are known to have arrived.  clear != 0 resets it. */
+int spd_wait_status(int* expired, int clear);
+/* A kernel whose one wait runs out after `tries` (1 .. 1000) tries: what spd_wait_status then reports. */
+int spd_wait_selftest(int tries, spd_stream_t stream);
 /* replaces semi_pd_ipc.get_device_sm_count (semi-pd-ipc/ipc.cpp:87-92) */
 int spd_device_sm_count(int device, int* sm_count);
 

@@ -33,6 +33,8 @@ _f = C.c_float
 SIGNATURES = {
     "spd_version": (_i, []),
     "spd_last_error_string": (C.c_char_p, []),
+    "spd_wait_status": (_i, [C.POINTER(_i), _i]),
+    "spd_wait_selftest": (_i, [_i, _p]),
     "spd_device_sm_count": (_i, [_i, C.POINTER(_i)]),
     "spd_partition_create": (_i, [_i, _i, _i, C.POINTER(_p)]),
     "spd_partition_sm_counts": (_i, [_p, C.POINTER(_i), C.POINTER(_i)]),

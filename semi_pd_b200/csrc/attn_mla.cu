@@ -39,7 +39,7 @@
 // short items took twice as long).
 //
 // Every mbarrier wait is bounded: a wait that runs out marks the CTA dead, all later waits fall through, the kernel
-// finishes without waiting and counts itself in g_mla_wait_expired.
+// finishes without waiting and sets the word that spd_wait_status reads.
 #include <cuda.h>
 
 #include "common.cuh"
@@ -54,8 +54,6 @@ constexpr int kMlaHeads = 16;    // heads per item
 constexpr int kMlaDL = 576, kMlaDV = 512;
 constexpr int kMlaBlk = kMlaTile * 128;       // one [64 rows x 64 columns] swizzle block of a tile
 constexpr int kMlaMisc = 2048;
-
-__device__ unsigned int g_mla_wait_expired;
 
 struct MlaParams {
   void* out;             // [items, H, DV]
@@ -75,6 +73,7 @@ struct MlaParams {
   float* o_part;   // [2 * grid][cols][DV]
   float* ml_part;  // [2 * grid][cols][2]
   int* info;       // [grid][8]: see mla_merge_kernel
+  unsigned* wait_expired;
 };
 
 template <bool kExtend>
@@ -889,11 +888,11 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
   griddep_launch_dependents();
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 6) tmem_dealloc(tmem_base, S::kTmem);
-  if (*dead) {  // a wait ran out: let copies in flight land before the shared memory is given back
-    for (int i = 0; i < 1000; ++i) __nanosleep(1000);
-    if (tid == 0) atomicAdd(&g_mla_wait_expired, 1u);
+  if (*dead) {
+    wait_drain();
+    if (tid == 0) wait_report(p.wait_expired);
   }
+  if (warp == 6) tmem_dealloc(tmem_base, S::kTmem);
 }
 
 // Merges the parts of the items that span several CTAs.  Block (c, 4 columns) serves the item that ends in CTA c after
@@ -1058,6 +1057,7 @@ int spd_attn_mla(void* out, const void* q, const void* kv_pool, const int32_t* r
   const int sms = sm_budget > 0 ? sm_budget : device_sms;
   const int grid = sms < device_sms ? sms : device_sms;
   MlaParams p{};
+  if (int rc = wait_flag(&p.wait_expired)) return rc;
   p.out = out;
   p.q = q;
   p.kv_pool = kv_pool;

@@ -77,6 +77,9 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 inline cudaStream_t as_stream(spd_stream_t s) { return reinterpret_cast<cudaStream_t>(s); }
 
 int device_sm_count_cached();
+// The word of host memory that a kernel sets when one of its bounded waits has run out (spd_wait_status); an error also
+// when it is set: the results since then are not to be trusted.
+int wait_flag(unsigned** flag);
 // programmatic dependent launch for the per-layer kernels (SPD_PDL=0 in the environment disables it)
 bool pdl_enabled();
 

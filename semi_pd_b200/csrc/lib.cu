@@ -5,9 +5,11 @@
 #include <cuda.h>
 #include <stdlib.h>
 #include <string.h>
+#include <atomic>
 #include <mutex>
 
 #include "common.cuh"
+#include "ptx.cuh"
 #include "tmap.cuh"
 
 namespace spd {
@@ -98,9 +100,65 @@ int make_tmap_blocks_sw128(CUtensorMap* out, const void* base, uint64_t rows, ui
   return 0;
 }
 
+// Allocated once, on the first call of a kernel with bounded waits; mapped, so that reading it takes no copy and no
+// synchronisation.  (The allocation may fall into a stream capture of this thread, where it is harmless.)
+static std::atomic<unsigned*> g_wait_flag{nullptr};
+
+int wait_flag(unsigned** flag) {
+  unsigned* f = g_wait_flag.load(std::memory_order_acquire);
+  if (f == nullptr) {
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lock(mu);
+    f = g_wait_flag.load(std::memory_order_acquire);
+    if (f == nullptr) {
+      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+      SPD_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+      void* p = nullptr;
+      const cudaError_t e = cudaHostAlloc(&p, 64, cudaHostAllocPortable | cudaHostAllocMapped);
+      SPD_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+      SPD_CUDA(e);
+      f = static_cast<unsigned*>(p);
+      *f = 0;
+      g_wait_flag.store(f, std::memory_order_release);
+    }
+  }
+  SPD_REQUIRE(*static_cast<volatile unsigned*>(f) == 0, SPD_E_TIMEOUT,
+              "a wait inside an earlier kernel ran out: results since then are not to be trusted (spd_wait_status)");
+  *flag = f;
+  return 0;
+}
+
+__global__ void wait_selftest_kernel(unsigned* flag, int tries) {
+  __shared__ uint64_t bar;
+  __shared__ int dead;
+  if (threadIdx.x == 0) {
+    dead = 0;
+    mbar_init(&bar, 1);
+    fence_barrier_init();
+    mbar_wait_bounded(&bar, 0, &dead, tries);  // nothing arrives
+    if (*static_cast<volatile int*>(&dead)) wait_report(flag);
+  }
+}
+
 }  // namespace spd
 
 using namespace spd;
+
+extern "C" int spd_wait_status(int* expired, int clear) {
+  SPD_REQUIRE(expired, SPD_E_BADARG, "spd_wait_status: null pointer");
+  volatile unsigned* f = g_wait_flag.load(std::memory_order_acquire);
+  *expired = f != nullptr && *f != 0;
+  if (f != nullptr && clear) *f = 0;
+  return 0;
+}
+
+extern "C" int spd_wait_selftest(int tries, spd_stream_t stream) {
+  SPD_REQUIRE(tries > 0 && tries <= 1000, SPD_E_BADARG, "spd_wait_selftest: 1 to 1000 tries");
+  unsigned* f;
+  if (int rc = wait_flag(&f)) return rc;
+  SPD_CUDA(launch(wait_selftest_kernel, dim3(1), dim3(32), 0, as_stream(stream), false, f, tries));
+  return 0;
+}
 
 // ------------------------------------------------------------------------------------------------
 // SM partitions

@@ -38,8 +38,6 @@ constexpr int kRcS = kRcDk * 128;        // one part of S: [128 x 128 B]
 constexpr int kRcV = kRcTok * 128;       // one part of v, v', A: [64 x 128 B]
 constexpr int kRcMisc = 1024;
 
-__device__ unsigned int g_rc_wait_expired;
-
 struct RetChunkParams {
   float* o;
   const void *q, *k, *v;
@@ -51,6 +49,7 @@ struct RetChunkParams {
   const float* decay;
   const float* cos_sin;
   float k_scale;
+  unsigned* wait_expired;
 };
 
 __device__ __forceinline__ uint32_t rc_off(int row, int c) { return row * 128 + ((c ^ (row & 7)) << 4); }
@@ -490,12 +489,16 @@ retention_chunked_kernel(const __grid_constant__ RetChunkParams p) {
   }
   tc_fence_before_sync();
   __syncthreads();
-  if (t_odd < n)
+  if (*dead) {  // the request keeps the state it had (or, stored above, had at its first token without parts)
+    wait_drain();
+    if (tid == 0) wait_report(p.wait_expired);
+  } else if (t_odd < n) {
     rc_token_by_token<T>(&p, t_odd, n, pos0, row0, reinterpret_cast<float*>(sQ), st, pw[1]);
-  else
+  } else {
     store_state();
+  }
+  __syncthreads();
   if (warp == 0) tmem_dealloc(*tmem_slot, 256);
-  if (*dead && tid == 0) atomicAdd(&g_rc_wait_expired, 1u);
 }
 
 template <typename T, int VS>
@@ -530,8 +533,10 @@ int retention_chunked_try(float* o, const void* q, const void* k, const void* v,
   if (q_stride % 8 != 0 || k_stride % 8 != 0 || v_stride % 8 != 0 || !aligned16(q) || !aligned16(k) || !aligned16(v) ||
       !aligned16(o) || !aligned16(state) || (rot > 0 && !aligned16(cos_sin)))
     return 1;
+  unsigned* wait_expired;
+  if (int rc = wait_flag(&wait_expired)) return rc;
   const RetChunkParams p{o, q, k, v, state, req_pool_indices, prefix_lens, extend_lens, extend_start_loc, H, dv, rot,
-                         q_stride, k_stride, v_stride, max_positions, decay, cos_sin, k_scale};
+                         q_stride, k_stride, v_stride, max_positions, decay, cos_sin, k_scale, wait_expired};
   return dtype == SPD_BF16 ? rc_launch<__nv_bfloat16, 1>(p, batch, stream) : rc_launch<__half, 2>(p, batch, stream);
 }
 

@@ -1430,6 +1430,15 @@ def get_partition(device: int, prefill_sms: int, decode_sms: int) -> SmPartition
     return part
 
 
+def check_waits() -> None:
+    """Raises if a wait inside a kernel has run out (the kernel ended without hanging the GPU, its results are not to be
+    trusted).  Does not synchronise: call it where results have arrived on the host."""
+    n = _C.c_int()
+    check(lib.spd_wait_status(_C.byref(n), 0), "spd_wait_status")
+    if n.value:
+        raise RuntimeError("a wait inside a kernel ran out: its results are not to be trusted")
+
+
 def device_sm_count(device: int = 0) -> int:
     n = _C.c_int()
     check(lib.spd_device_sm_count(device, _C.byref(n)), "spd_device_sm_count")

@@ -230,6 +230,7 @@ class SemiPDPrefillScheduler(SemiPDScheduler):
         # before their KV exists — otherwise the running decode batch would stall on the device
         # behind this prefill — so the report waits for the event in both arms.
         done.synchronize()
+        ops.check_waits()
         if not self.device_resident:
             ids = ids.tolist()
         self.prefill_busy_s += time.perf_counter() - t0
@@ -549,6 +550,7 @@ class SemiPDDecodeScheduler(SemiPDScheduler):
 
     def process_batch_result_decode(self, reqs: List[Req], pinned: torch.Tensor, bs: int, ev):
         ev.synchronize()
+        ops.check_waits()
         now = time.perf_counter()
         ids = pinned[:bs].tolist() if pinned is not None else [-1] * bs
         for req, tok in zip(reqs, ids):

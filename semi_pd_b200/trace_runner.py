@@ -119,6 +119,7 @@ def main(argv=None) -> int:
     a = ap.parse_args(argv)
     os.makedirs(a.out, exist_ok=True)
     worker = build_worker(a.model, a.dtype, a.max_tokens, a.max_requests, not a.disable_cuda_graph)
+    from . import ops
     session = TraceSession(worker)
     for line in sys.stdin:
         line = line.strip()
@@ -128,6 +129,7 @@ def main(argv=None) -> int:
         logits = session.step(msg.get("entries", []))
         if logits.shape[0]:
             arr = logits.cpu().numpy().astype("<f4", copy=False)
+            ops.check_waits()
             tmp = os.path.join(a.out, f".{msg['step']}.f32.part")
             with open(tmp, "wb") as f:
                 f.write(np.ascontiguousarray(arr).tobytes())

@@ -73,3 +73,10 @@ def test_compute_without_gpu_fails_loudly():
     p16 = (C.addressof(buf) + 15) & ~15
     rc = _lib.lib.spd_rmsnorm(p16, p16 + 1024, p16 + 2048, 1, 128, 128, 128, 1e-6, 0, None)
     assert rc > 0
+
+
+def test_wait_status_without_a_gpu_call():
+    n = C.c_int(7)
+    assert _lib.lib.spd_wait_status(C.byref(n), 0) == 0 and n.value == 0
+    assert _lib.lib.spd_wait_status(None, 0) == -1
+    assert _lib.lib.spd_wait_selftest(0, None) == -1 and _lib.lib.spd_wait_selftest(1001, None) == -1

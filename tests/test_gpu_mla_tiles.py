@@ -203,3 +203,26 @@ def test_rotary_store_refuses_what_it_would_read_past():
         else:
             raise AssertionError(f"case {i} was accepted")
     torch.cuda.synchronize()
+
+
+def test_a_wait_that_ran_out_is_reported():
+    """A kernel whose bounded wait runs out ends, sets the status word, and the calls with such waits refuse from then on."""
+    import ctypes
+
+    from semi_pd_b200 import _lib, ops
+    torch.cuda.synchronize()
+    ops.check_waits()
+    n = ctypes.c_int()
+    try:
+        assert _lib.lib.spd_wait_selftest(2, ops._stream()) == 0
+        torch.cuda.synchronize()
+        with pytest.raises(RuntimeError, match="ran out"):
+            ops.check_waits()
+        with pytest.raises(RuntimeError, match="ran out"):
+            _run([63], [1], 16, torch.bfloat16, "runs", True)
+    finally:
+        torch.cuda.synchronize()
+        assert _lib.lib.spd_wait_status(ctypes.byref(n), 1) == 0
+    assert n.value == 1
+    ops.check_waits()
+    _run([63], [1], 16, torch.bfloat16, "runs", True)
