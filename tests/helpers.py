@@ -5,6 +5,23 @@ import torch
 from oracle import llama_oracle as O
 
 
+# Largest relative error (2-norms, one request's outputs) of attention in 16 bits: rounding P moves an output by at most half
+# an ulp of its terms, rounding the output by half an ulp of itself.  A request that lost one of its tiles is far above.
+ATTN_REL = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}
+
+
+def assert_requests_close(got, want, rows, dtype, keep=None):
+    """got / want [rows, ...]: every request's rows (their counts in `rows`) within ATTN_REL; keep: elements compared."""
+    at = 0
+    for b, n in enumerate(rows):
+        g, w = got[at: at + n].double(), want[at: at + n].double()
+        if keep is not None:
+            g, w = g[keep[at: at + n]], w[keep[at: at + n]]
+        err = (g - w).norm().item()
+        assert err <= ATTN_REL[dtype] * w.norm().item() + 1e-7 * max(w.numel(), 1) ** 0.5, (b, err, w.norm().item())
+        at += n
+
+
 def make_runner(cfg_kwargs, dtype, kv_slots=4096, max_reqs=16, ctx=2048, cuda_graph=False,
                 cuda_graph_bs=None, oracle_mode="fp32", seed=1234, name="tiny-llama-test"):
     from semi_pd_b200.configs import ModelConfig, ServerArgs

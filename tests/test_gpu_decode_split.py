@@ -3,6 +3,8 @@ end on and beside tiles, an empty request, more items than the split takes (whol
 import pytest
 import torch
 
+from tests.helpers import assert_requests_close
+
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
 D = 128
@@ -49,15 +51,17 @@ def _run(lens, Hq, Hk, dtype=torch.bfloat16, sms=0, workspace="own", repeat=1):
     # values N(0, 1): the largest output is that of a request of one token; P and the output are rounded to 16 bits
     err = (outs[0].double().view(B, Hq, D) - want).abs().max().item()
     assert err < (3e-2 if dtype == torch.bfloat16 else 4e-3), err
+    assert_requests_close(outs[0].view(B, Hq, D), want, [1] * B, dtype)
     if untouched:
         assert bool((ws == 255).all())
     assert all(torch.equal(outs[0], o) for o in outs[1:])  # the parts are merged in a fixed order; counters are re-armed
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("Hq,Hk", [(32, 8), (8, 8), (8, 1), (4, 2)])
 @pytest.mark.parametrize("lens", [[1], [5000], [127, 128, 129], [0, 300, 0], [2000, 3, 70, 1], [400 + 37 * i for i in range(12)]])
-def test_cuts(Hq, Hk, lens):
-    _run(lens, Hq, Hk, repeat=3)
+def test_cuts(Hq, Hk, lens, dtype):
+    _run(lens, Hq, Hk, dtype, repeat=3)
 
 
 @pytest.mark.parametrize("sms", [1, 2, 7, 40])
@@ -66,7 +70,8 @@ def test_partitions(sms):
 
 
 def test_many_requests():
-    _run([1 + (53 * i) % 700 for i in range(70)], 32, 8)      # 560 items: cut
+    _run([1 + (53 * i) % 700 for i in range(70)], 32, 8)      # 560 items: whole ones
+    _run([4000 - 53 * i for i in range(20)], 32, 8)           # 160 items: cut
     _run([1 + (53 * i) % 90 for i in range(300)], 32, 8)      # 2400 items: whole ones
 
 

@@ -4,6 +4,8 @@ no group of 16, a workspace of the least size a call has to bring, a batch large
 import pytest
 import torch
 
+from tests.helpers import assert_requests_close
+
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
 R, DR = 512, 64
@@ -78,6 +80,7 @@ def _run(pre, ext, H, dtype, layout, decode, ws_bytes=None, sms=0, odd=()):
     out = out.cpu().double().view(want.shape)
     err = (out - want)[blind].abs().max().item()
     assert err < TOL[dtype], err
+    assert_requests_close(out, want, ext, dtype, blind)
     for b, pos, channel, value in odd:
         at = sum(ext[:b])
         assert not out[at + max(0, pos - pre[b]): at + ext[b], :, channel].isfinite().any()
@@ -97,11 +100,12 @@ def test_head_counts(H, decode):
     _run([300, 64, 700], ext, H, torch.bfloat16, "runs", decode)
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("layout", ["runs", "scattered", "stray"])
 @pytest.mark.parametrize("pre,ext", [([0], [3]), ([0], [64]), ([61], [7]), ([0, 130, 5], [1, 65, 4]), ([2000], [2]),
                                      ([0, 640], [700, 259])])
-def test_extend_tiles(layout, pre, ext):
-    _run(pre, ext, 16, torch.bfloat16, layout, False)
+def test_extend_tiles(layout, pre, ext, dtype):
+    _run(pre, ext, 16, dtype, layout, False)
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])

@@ -4,6 +4,8 @@ head (two token tiles per item) and of several, scattered slots, a sink and scor
 import pytest
 import torch
 
+from tests.helpers import assert_requests_close
+
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
 D = 128
@@ -60,6 +62,7 @@ def _run(pre, ext, H, G, window, dtype, sinks=None, qtemp=(0.0, 0), scattered=Fa
     out = out.cpu().double()
     err = (out - want)[blind].abs().max().item()
     assert err < tol, err
+    assert_requests_close(out, want, ext, dtype, blind)
     assert not out[~blind].isfinite().any()
 
 
