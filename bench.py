@@ -17,11 +17,11 @@ running concurrently on disjoint SM partitions) until the last token of the last
   * `parity_check`: greedy ids the e2e arm returned, compared with the CPU oracle's on the same
                 weights and prompts (outside the timed region);
   * `latency_sweep`: Poisson windows (exponential gaps, bench_serving.py:884-899) at the rates of
-                SURVEY §8d for p50/p99 TTFT and TPOT (TPOT = (t_last - t_first)/(n-1),
+                `--sweep-rates` for p50/p99 TTFT and TPOT (TPOT = (t_last - t_first)/(n-1),
                 bench_serving.py:920-921); `latency` = the window at 60 % of the measured capacity;
   * `gpu_baseline`: the same request mix through flashinfer's paged wrappers + cuBLAS `F.linear`
                 on the same box (scripts/gpu_baseline_flashinfer.py) — the stand-in for the
-                reference's own flashinfer build, which cannot be installed here (DESIGN.md §6).
+                reference's own flashinfer build, which cannot be installed here.
 N > 1: `value` / `e2e` are N independent replicas (one engine per GPU, no data-path collective,
 weak scaling); the `tp` block then serves the same mix with ONE engine sharded TP = N (heads / FFN
 columns per GPU, spd_allreduce / NCCL after o_proj and down_proj), `tp_parity` checks a TP = N
@@ -719,7 +719,7 @@ def main():
                              **latency_stats(reqs)}
         sweep = []
         for r_s in [float(x) for x in args.sweep_rates.split(",") if x.strip()]:
-            # SURVEY §8d rates; each window is bounded to ~6 s of arrivals (at least 32 requests)
+            # the sweep's rates; each window is bounded to ~6 s of arrivals (at least 32 requests)
             n = int(min(args.requests, max(32, round(r_s * 6))))
             wall, reqs, _ = run_window(engine, prompts[:n], dev_prompts[:n], args.output_len, r_s, False)
             sweep.append({"request_rate": r_s, "requests": n, "saturated": r_s > cap,

@@ -345,14 +345,6 @@ int spd_moe_combine(void* out, const void* y, const void* shared, const int32_t*
 int spd_moe_dense_act(void* act, const void* gate_up, const int32_t* topk_ids, const float* topk_w,
                       int64_t tokens, int top_k, int num_experts, int64_t inter, int dtype,
                       spd_stream_t stream);
-/* Absorbed MLA attention (MQA over the latent pool), decode (seq_lens != NULL: one query per request
- * over its seq_lens[b] rows) or ragged extend (seq_lens == NULL: query token j of request r, row
- * extend_start_loc[r] + j of q, attends keys 0 .. prefix_lens[r] + j).  kv_pool [slots, kv_lora_rank +
- * rope_dim] = MLATokenToKVPool rows (S/mem_cache/memory_pool.py:379-452); K = the whole row, V = its
- * first kv_lora_rank columns; q [tokens, H, kv_lora_rank + rope_dim] (q_nope already multiplied by
- * w_kc), out [tokens, H, kv_lora_rank].  replaces DeepseekV2AttentionMLA.forward_absorb's attention
- * call (S/models/deepseek_v2.py:684-700 → S/layers/attention/triton_ops/decode_attention.py:235-470,
- * extend_attention.py:291-410). */
 /* Between the fused projection qa [tokens, heads * (nope + rope) || kv_lora || rope] and spd_attn_mla: RMS norm of the
  * latent and rotation (interleaved pairs, cos_sin [positions, rope] fp32 = cos || sin) of its rope part -> row loc[t] of
  * kv_pool; rotation of every head's rope part -> q_lat [tokens, heads, kv_lora + rope] behind the kv_lora columns, which
@@ -362,6 +354,15 @@ int spd_mla_rotary_store(void* q_lat, const void* qa, void* kv_pool, const void*
                          const int64_t* positions, const int64_t* loc, int64_t tokens, int num_heads, int nope_dim,
                          int kv_lora_rank, int rope_dim, int64_t qa_stride, int64_t q_lat_stride, float eps, int dtype,
                          spd_stream_t stream);
+/* Absorbed MLA attention (MQA over the latent pool), decode (seq_lens != NULL: one query per request
+ * over its seq_lens[b] rows) or ragged extend (seq_lens == NULL: query token j of request r, row
+ * extend_start_loc[r] + j of q, attends keys 0 .. prefix_lens[r] + j).  kv_pool [slots, kv_lora_rank +
+ * rope_dim] = MLATokenToKVPool rows (S/mem_cache/memory_pool.py:379-452); K = the whole row, V = its
+ * first kv_lora_rank columns; q [tokens, H, kv_lora_rank + rope_dim] (q_nope already multiplied by
+ * w_kc), out [tokens, H, kv_lora_rank].  replaces DeepseekV2AttentionMLA.forward_absorb's attention
+ * call (S/models/deepseek_v2.py:684-700 → S/layers/attention/triton_ops/decode_attention.py:235-470,
+ * extend_attention.py:291-410).  The workspace (spd_attn_mla_workspace_bytes() for any batch, not zeroed)
+ * holds parts of requests cut over SMs while the call runs: one call at a time. */
 int64_t spd_attn_mla_workspace_bytes(int num_heads, int kv_lora_rank);
 int spd_attn_mla(void* out, const void* q, const void* kv_pool, const int32_t* req_to_token,
                  const int64_t* req_pool_indices, const int64_t* seq_lens, const int32_t* prefix_lens,

@@ -37,9 +37,8 @@ import threading
 import time
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-# JIT cache prebuilt in the build container travels with the repo (baseline/_ref is git-ignored,
-# not gpurun-ignored).  /root/repo is valid in the build container AND on the GPU box (a symlink
-# to the snapshot there), so the absolute paths ninja recorded stay valid and nothing recompiles.
+# The JIT cache lies in the tree (baseline/_ref, git-ignored) under one fixed path, so that the absolute paths ninja
+# recorded stay valid where the tree is copied to and nothing recompiles.
 _base = "/root/repo" if os.path.isdir("/root/repo/scripts") else ROOT
 os.environ.setdefault("FLASHINFER_WORKSPACE_BASE", os.path.join(_base, "baseline", "_ref", "flashinfer"))
 os.environ.setdefault("FLASHINFER_CUDA_ARCH_LIST", "10.0a")

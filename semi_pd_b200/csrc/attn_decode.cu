@@ -12,12 +12,13 @@
 // real cost is the stream itself.
 //
 // grid = #SMs (or the partition's SM budget).  Work items (request, kv head) are dealt to the CTAs with a static stride, or,
-// where that would leave SMs idle, cut: their 128-token tiles, one after another and with one more unit per item for its
-// epilogue, are one list that the CTAs share in equal contiguous ranges.  Lengths are read on the device.  A CTA keeps its TMEM, barriers and the 3-stage K/V ring alive across items, so the gather of the
-// next item overlaps the epilogue of the current one.  The parts of an item that was cut are merged by the last-arriving
+// where that would leave SMs idle (and the caller owns the workspace, or there are fewer items than SMs), cut: their
+// 128-token tiles, one after another and with one more unit per item for its epilogue, are one list that the CTAs share in
+// equal contiguous ranges.  Lengths are read on the device.  A CTA keeps its TMEM, barriers and the 3-stage K/V ring alive
+// across items, so the gather of the next item overlaps the epilogue of the current one.  The parts of an item that was cut are merged by the last-arriving
 // of its CTAs — no host plan, no second launch, CUDA-graph safe.  (A fixed number of splits per
 // item, for the SMs to be covered, took two rounds for the 160 splits of 5 requests x 8 heads: 7000 tokens each 52 us, 36
-// as ranges; one request of 1000 tokens 19.3 / 13.9 us.)
+// as ranges; one request of 1000 tokens 19.3 / 14.4 us.)
 //
 // Softmax without per-tile reductions: every thread owns one kv token of the tile (a TMEM lane of
 // S^T).  All threads exponentiate against a shared REFERENCE max m_ref that is only raised when
@@ -38,8 +39,7 @@
 // allocator's scattered slots, the ragged last tile of a sequence — takes the gather path:
 // 16-byte cp.async per row chunk through req_to_token into the same swizzled layout.
 // (tile::gather4, 4 rows x 128 B per instruction, was built and measured: correct,
-// but ~1 instruction per 27 clk per SM -> 36 GB/s per SM, below the cp.async gather's 47;
-// profiles/r01_decode_attention_loader_experiments.md.)
+// but ~1 instruction per 27 clk per SM -> 36 GB/s per SM, below the cp.async gather's 47.)
 #include <cuda.h>
 
 #include "common.cuh"

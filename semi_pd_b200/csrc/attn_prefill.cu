@@ -89,7 +89,7 @@ struct PrefillParams {
   int64_t q_stride;
   const float* sinks;
   float qtemp_coef;
-  long long* trace;  // debug timeline of CTA 0 (scripts/debug_attn_prefill_timeline.py); kTrace builds only
+  long long* trace;  // debug timeline of CTA 0; kTrace builds only
   int trace_cap;
 };
 
@@ -225,13 +225,13 @@ __device__ __forceinline__ uint64_t fadd2(uint64_t a, uint64_t b) {
   return d;
 }
 
-// 32 columns of one tile row: p = exp2(s*scale - m_off), packed to 16 bits into pk[0..16)
 // key `kv` of a masked unit is visible: kv <= limit, and with a window (span = its size - 1) limit - kv <= span
 template <bool kWin>
 __device__ __forceinline__ bool pf_visible(int kv, int limit, int span) {
   if constexpr (kWin) return static_cast<uint32_t>(limit - kv) <= static_cast<uint32_t>(span);
   return kv <= limit;
 }
+// 32 columns of one tile row: p = exp2(s*scale - m_off), packed to 16 bits into pk[0..16)
 template <typename T, bool kMask, bool kWin>
 __device__ __forceinline__ void softmax_chunk(const uint32_t* r, int c, uint32_t* pk, uint64_t scale2,
                                               uint64_t neg_m2, int kv0, int limit, int span, uint64_t& ps) {
@@ -310,7 +310,7 @@ __device__ __forceinline__ float softmax_row_max(uint32_t ts, int kv0, int limit
 
 // Output of one query row by a warp, from the keys the row sees alone; before the division by the sum, columns
 // c + 2 lane and c + 2 lane + 1.  (kWin, for rows whose output is not finite: the tiles hold keys that the row does not
-// see, and their P of 0 times an infinite or NaN value is NaN.  Looking for them in the epilogue: 140.6 -> 143.4 us for
+// see, and their P of 0 times an infinite or NaN value is NaN.  Looking for them in the epilogue: 140.2 -> 142.7 us for
 // 4 requests of 2048 new tokens, 16 / 4 heads, window 1024.)
 template <typename T>
 __device__ __noinline__ float2 pf_row_alone(const T* q, const T* k_pool, const T* v_pool, const int32_t* page,
@@ -460,13 +460,12 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         // issued earlier by this thread — tcgen05.mma executes in issue order.
         // (Tried: interleaving the two warpgroups' MMAs instruction by instruction —
         // back-to-back tcgen05.mma on ONE accumulator cost ~43 clk (SS) / ~10 clk (TS) more than
-        // N/2 each, alternating accumulators runs at the shared-memory operand rate,
-        // profiles/r02_tcgen05_2cta_probe.log.  The issuer's time per unit pair did drop from
+        // N/2 each, alternating accumulators runs at the shared-memory operand rate
+        // (rates of unrolled MMAs; from a short loop one of M = 128, N = 64 takes 46 clk on one or several).  The issuer's time per unit pair did drop from
         // 2 x 795 to 1293 clk, but pairing forces both warpgroups' softmax passes into the same
         // phase (1020 -> 1500 clk per pass, XU contention) and the kernel got 2-5 % slower.
         // Second attempt: keep the warpgroups staggered and interleave PV(t) — as two 64-column
-        // halves of O — with S'(t-1), the next tile's S of the chain served one step earlier
-        // (scripts/experiments/attn_prefill_staggered_interleave.cu.txt).  Correct, and 30 %
+        // halves of O — with S'(t-1), the next tile's S of the chain served one step earlier.  Correct, and 30 %
         // SLOWER: the issuer needed 1205 clk per 16-instruction step, 75 clk per instruction —
         // alternating TS- and SS-form MMAs costs more than either stream alone (8 x 42 + 8 x 75
         // by the probe), the alternation benefit exists for SS next to SS only.)

@@ -2,7 +2,7 @@
 // distributed shared memory — for the layers whose N gives fewer 128-row weight tiles than there
 // are SMs (W_qkv: 48 tiles, W_o and W_down: 32 tiles on Llama-3-8B).  One SM streams ~90-100 GB/s
 // however deep its TMA ring is, so those layers need 3-4 SMs per tile to approach HBM speed; a
-// global-memory split-K fix-up costs ~8 us (measured, profiles/r01_gemm_decode_sweep.log), more
+// global-memory split-K fix-up costs ~8 us (measured), more
 // than the 10-20 us the whole GEMM should take.
 //
 // cluster = S CTAs working on the same [128 weight rows] x [BN tokens] output tile (swap-AB as in

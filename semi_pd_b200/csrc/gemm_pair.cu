@@ -6,7 +6,7 @@
 // writes each CTA's 128 x 256 fp32 accumulator into that CTA's own TMEM.  Against the single-CTA
 // 128 x 256 tile (gemm.cu) every CTA stages 32 KB instead of 48 KB per k-block and the tensor
 // core reads a third fewer operand bytes from shared memory per FLOP — on a power-capped B200
-// (scripts/bench_gemm_prefill.py: ~1 kW, SM clock 1.15-1.45 GHz under sustained GEMM load) the
+// (measured: ~1 kW, SM clock 1.15-1.45 GHz under sustained GEMM load) the
 // joules per FLOP are what sets the sustained rate.
 //
 // Pipeline (per CTA: 256 threads; warp 0 = TMA producer, warp 1 = MMA issuer (leader CTA only),

@@ -1,9 +1,8 @@
 // Decode-regime GEMM on CTA PAIRS: C[M,N] = A[M,K] * W[N,K]^T for 32 < M <= 256 tokens, swap-AB
 // with tcgen05.mma.cta_group::2.
 //
-// Why: measured on B200 (profiles/r01_gemm_decode_sweep.log, scripts/bench_kernels.py gd) the
-// single-CTA swap-AB kernel (gemm.cu) delivers a constant ~8-9 TB/s of operand bytes into the SMs
-// whatever M is — the chip-wide L2 -> SM limit — and every 128-row weight tile re-reads the whole
+// Why: measured on B200 the single-CTA swap-AB kernel (gemm.cu) delivers a constant ~8-9 TB/s of
+// operand bytes into the SMs whatever M is — the chip-wide L2 -> SM limit — and every 128-row weight tile re-reads the whole
 // activation matrix, so the weight stream runs at HBM speed only while M is tiny:
 // bytes into the SMs = weights x (1 + M/128).  A CTA pair shares ONE activation tile between 256
 // weight rows (each CTA stages half of the token rows, the 2-SM MMA reads both halves), which

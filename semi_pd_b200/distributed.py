@@ -44,7 +44,7 @@ NCCL_FOR_LARGE = os.environ.get("SPD_TP_NCCL", "0") == "1"
 # the all-reduce after o_proj / down_proj fused with the residual-add RMSNorm that consumes it
 # (decode-sized messages: every rank reads all W slots, so the one-shot form stops paying at ~2 MiB).
 # Bit-identical to the two kernels and tested, but measured NEUTRAL on 2 GPUs (TP = 2 engine, 8B:
-# TPOT p50 at 40 req/s 4.31 ms fused vs 4.22 ms unfused, profiles/r02_bench_n2_fused_ar_norm_ab.txt:
+# TPOT p50 at 40 req/s 4.31 ms fused vs 4.22 ms unfused:
 # the cross-GPU barrier dominates both, and under PDL the separate RMSNorm already starts inside
 # the all-reduce's tail) — so it is opt-in: SPD_FUSE_AR_NORM=1.
 FUSE_AR_NORM = os.environ.get("SPD_FUSE_AR_NORM", "0") == "1"

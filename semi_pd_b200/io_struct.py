@@ -48,7 +48,7 @@ class BatchProcessPrefillResultReq:
     # recorded on the prefill stream after the forward (KV rows of the batch are in the pool)
     done_event: Any = None
     # host timestamps of the prefill worker (batch fetched, forward launched, ids read back):
-    # TTFT breakdown of scripts/debug_ttft_breakdown.py
+    # TTFT breakdown of one request
     timing: Optional[tuple] = None
 
 

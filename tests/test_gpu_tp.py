@@ -1,13 +1,12 @@
 """Tensor-parallel forward path on real GPUs (needs >= 2; skipped otherwise): N ranks, sharded
 heads / FFN columns, SUM all-reduce after o_proj and down_proj only — libspd's peer-memory
 `spd_allreduce` (one-shot / two-shot over IPC-mapped buffers) for decode-sized messages, NCCL above
-8 MiB — and a vocab-sharded lm_head whose greedy ids come from an all-gather of (max, argmax) rows
-(SURVEY §8e).  Every rank must reproduce the unsharded CPU oracle's logits; decode runs both
+8 MiB — and a vocab-sharded lm_head whose greedy ids come from an all-gather of (max, argmax) rows.
+Every rank must reproduce the unsharded CPU oracle's logits; decode runs both
 eagerly and through the captured CUDA graph (the collective is inside the graph); the semi-PD
 engine runs with tp_size = 2 (P and D on separate communicators, rank 0 broadcasting the decode
 scheduler's messages) and must produce the sequential oracle's tokens.
-The driver's GPUTEST box has one GPU: the pass is recorded by `gpurun --gpus 2` logs under
-profiles/ and by `bench.py --gpus N`'s `tp_parity` block in every SCALE run."""
+On one GPU these tests are skipped; `bench.py --gpus N` reports the same check as `tp_parity`."""
 import os
 import socket
 
