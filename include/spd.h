@@ -362,7 +362,9 @@ int spd_mla_rotary_store(void* q_lat, const void* qa, void* kv_pool, const void*
  * w_kc), out [tokens, H, kv_lora_rank].  replaces DeepseekV2AttentionMLA.forward_absorb's attention
  * call (S/models/deepseek_v2.py:684-700 → S/layers/attention/triton_ops/decode_attention.py:235-470,
  * extend_attention.py:291-410).  The workspace (spd_attn_mla_workspace_bytes() for any batch, not zeroed)
- * holds parts of requests cut over SMs while the call runs: one call at a time. */
+ * holds parts of requests cut over SMs while a call runs, one call at a time.  A call whose query tokens x groups of 16 heads
+ * are at least twice the SMs it may occupy does not touch it (it may be NULL), unless it is spd_attn_mla_own: there the
+ * workspace belongs to this stream's calls of every size, which are then cut evenly. */
 int64_t spd_attn_mla_workspace_bytes(int num_heads, int kv_lora_rank);
 int spd_attn_mla(void* out, const void* q, const void* kv_pool, const int32_t* req_to_token,
                  const int64_t* req_pool_indices, const int64_t* seq_lens, const int32_t* prefix_lens,
@@ -370,6 +372,12 @@ int spd_attn_mla(void* out, const void* q, const void* kv_pool, const int32_t* r
                  int kv_lora_rank, int rope_dim, int64_t q_stride, int64_t out_stride,
                  int64_t req_to_token_stride, float sm_scale, int dtype, void* workspace,
                  int64_t workspace_bytes, int sm_budget, spd_stream_t stream);
+int spd_attn_mla_own(void* out, const void* q, const void* kv_pool, const int32_t* req_to_token,
+                     const int64_t* req_pool_indices, const int64_t* seq_lens, const int32_t* prefix_lens,
+                     const int32_t* extend_start_loc, int64_t batch, int64_t total_tokens, int num_heads,
+                     int kv_lora_rank, int rope_dim, int64_t q_stride, int64_t out_stride,
+                     int64_t req_to_token_stride, float sm_scale, int dtype, void* workspace,
+                     int64_t workspace_bytes, int sm_budget, spd_stream_t stream);
 
 /* ---------------------------------------------------------------------------------------------
  * 32-bit capable ops — the operators of the hybrid (windowed attention + retention + MoE) model

@@ -339,7 +339,7 @@ class SpdAttnBackend(AttentionBackend):
         kv = pool.get_key_buffer(layer.layer_id)
         rope = layer.head_dim - layer.v_head_dim
         common = dict(num_heads=layer.tp_q_head_num, kv_lora_rank=layer.v_head_dim, rope_dim=rope,
-                      sm_scale=layer.scaling, workspace=self.mla_workspace)
+                      sm_scale=layer.scaling, workspace=self.mla_workspace, own_workspace=True)
         if forward_batch.forward_mode.is_decode():
             return ops.attn_mla(q_lat, kv, forward_batch.req_to_token_pool.req_to_token,
                                 forward_batch.req_pool_indices, seq_lens=forward_batch.seq_lens, **common)

@@ -1035,12 +1035,14 @@ int64_t spd_attn_mla_workspace_bytes(int num_heads, int kv_lora_rank) {
   return items * num_heads * 8 * (kv_lora_rank + 2) * 4 + 256;
 }
 
-int spd_attn_mla(void* out, const void* q, const void* kv_pool, const int32_t* req_to_token,
-                 const int64_t* req_pool_indices, const int64_t* seq_lens, const int32_t* prefix_lens,
-                 const int32_t* extend_start_loc, int64_t batch, int64_t total_tokens, int num_heads,
-                 int kv_lora_rank, int rope_dim, int64_t q_stride, int64_t out_stride,
-                 int64_t req_to_token_stride, float sm_scale, int dtype, void* workspace,
-                 int64_t workspace_bytes, int sm_budget, spd_stream_t stream) {
+// own_workspace: the workspace is this stream's alone at every batch size (spd_attn_mla_own); otherwise a call that need not
+// bring one leaves it untouched.
+static int attn_mla(void* out, const void* q, const void* kv_pool, const int32_t* req_to_token,
+                    const int64_t* req_pool_indices, const int64_t* seq_lens, const int32_t* prefix_lens,
+                    const int32_t* extend_start_loc, int64_t batch, int64_t total_tokens, int num_heads, int kv_lora_rank,
+                    int rope_dim, int64_t q_stride, int64_t out_stride, int64_t req_to_token_stride, float sm_scale,
+                    int dtype, void* workspace, int64_t workspace_bytes, bool own_workspace, int sm_budget,
+                    spd_stream_t stream) {
   SPD_REQUIRE(out && q && kv_pool && req_to_token && req_pool_indices, SPD_E_BADARG, "spd_attn_mla: null pointer");
   const bool extend = seq_lens == nullptr;
   SPD_REQUIRE(!extend || (prefix_lens && extend_start_loc), SPD_E_BADARG,
@@ -1087,6 +1089,7 @@ int spd_attn_mla(void* out, const void* q, const void* kv_pool, const int32_t* r
   const int64_t least = splits > 1 ? items * num_heads * splits * (kMlaDV + 2) * 4 : 0;
   SPD_REQUIRE(least == 0 || (workspace && workspace_bytes >= least), SPD_E_WORKSPACE,
               "spd_attn_mla: workspace too small (%lld < %lld)", (long long)workspace_bytes, (long long)least);
+  if (least == 0 && !own_workspace) workspace = nullptr;
   p.snap = workspace == nullptr || workspace_bytes < need || groups >= 16ll * grid;
   if (!p.snap) {
     p.o_part = reinterpret_cast<float*>(workspace);
@@ -1098,6 +1101,26 @@ int spd_attn_mla(void* out, const void* q, const void* kv_pool, const int32_t* r
     return extend ? mla_launch<T, true>(p, grid, st) : mla_launch<T, false>(p, grid, st);
   });
   return 0;
+}
+
+int spd_attn_mla(void* out, const void* q, const void* kv_pool, const int32_t* req_to_token, const int64_t* req_pool_indices,
+                 const int64_t* seq_lens, const int32_t* prefix_lens, const int32_t* extend_start_loc, int64_t batch,
+                 int64_t total_tokens, int num_heads, int kv_lora_rank, int rope_dim, int64_t q_stride, int64_t out_stride,
+                 int64_t req_to_token_stride, float sm_scale, int dtype, void* workspace, int64_t workspace_bytes,
+                 int sm_budget, spd_stream_t stream) {
+  return attn_mla(out, q, kv_pool, req_to_token, req_pool_indices, seq_lens, prefix_lens, extend_start_loc, batch, total_tokens,
+                  num_heads, kv_lora_rank, rope_dim, q_stride, out_stride, req_to_token_stride, sm_scale, dtype, workspace,
+                  workspace_bytes, false, sm_budget, stream);
+}
+
+int spd_attn_mla_own(void* out, const void* q, const void* kv_pool, const int32_t* req_to_token, const int64_t* req_pool_indices,
+                     const int64_t* seq_lens, const int32_t* prefix_lens, const int32_t* extend_start_loc, int64_t batch,
+                     int64_t total_tokens, int num_heads, int kv_lora_rank, int rope_dim, int64_t q_stride, int64_t out_stride,
+                     int64_t req_to_token_stride, float sm_scale, int dtype, void* workspace, int64_t workspace_bytes,
+                     int sm_budget, spd_stream_t stream) {
+  return attn_mla(out, q, kv_pool, req_to_token, req_pool_indices, seq_lens, prefix_lens, extend_start_loc, batch, total_tokens,
+                  num_heads, kv_lora_rank, rope_dim, q_stride, out_stride, req_to_token_stride, sm_scale, dtype, workspace,
+                  workspace_bytes, true, sm_budget, stream);
 }
 
 }  // extern "C"

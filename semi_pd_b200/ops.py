@@ -467,21 +467,23 @@ def mla_rotary_store(qa: torch.Tensor, q_lat: torch.Tensor, kv_pool: torch.Tenso
 
 def attn_mla(q: torch.Tensor, kv_pool: torch.Tensor, req_to_token, req_pool_indices, num_heads: int,
              kv_lora_rank: int, rope_dim: int, sm_scale: float, workspace: torch.Tensor, seq_lens=None,
-             prefix_lens=None, extend_start_loc=None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+             prefix_lens=None, extend_start_loc=None, out: Optional[torch.Tensor] = None,
+             own_workspace: bool = False) -> torch.Tensor:
     """Absorbed MLA attention: decode (seq_lens) or ragged extend (prefix_lens + extend_start_loc).
-    q [T, H * (kv_lora + rope)] → out [T, H * kv_lora]."""
+    q [T, H * (kv_lora + rope)] → out [T, H * kv_lora].  own_workspace: `workspace` serves one stream at a time at every
+    batch size; without that promise a batch that fills the SMs twice leaves it untouched (and cuts no request)."""
     _cuda(q, kv_pool, req_to_token, req_pool_indices)
     T = q.shape[0]
     q2 = q.view(T, -1)
     if out is None:
         out = torch.empty((T, num_heads * kv_lora_rank), device=q.device, dtype=q.dtype)
-    check(lib.spd_attn_mla(out.data_ptr(), q2.data_ptr(), kv_pool.data_ptr(), req_to_token.data_ptr(),
-                           req_pool_indices.data_ptr(), seq_lens.data_ptr() if seq_lens is not None else None,
-                           prefix_lens.data_ptr() if prefix_lens is not None else None,
-                           extend_start_loc.data_ptr() if extend_start_loc is not None else None,
-                           req_pool_indices.numel(), T, num_heads, kv_lora_rank, rope_dim, q2.stride(0),
-                           out.stride(0), req_to_token.stride(0), float(sm_scale), _dt(q), workspace.data_ptr(),
-                           workspace.numel(), get_sm_budget(), _stream()), "spd_attn_mla")
+    call = lib.spd_attn_mla_own if own_workspace else lib.spd_attn_mla
+    check(call(out.data_ptr(), q2.data_ptr(), kv_pool.data_ptr(), req_to_token.data_ptr(), req_pool_indices.data_ptr(),
+               seq_lens.data_ptr() if seq_lens is not None else None,
+               prefix_lens.data_ptr() if prefix_lens is not None else None,
+               extend_start_loc.data_ptr() if extend_start_loc is not None else None, req_pool_indices.numel(), T,
+               num_heads, kv_lora_rank, rope_dim, q2.stride(0), out.stride(0), req_to_token.stride(0), float(sm_scale),
+               _dt(q), workspace.data_ptr(), workspace.numel(), get_sm_budget(), _stream()), "spd_attn_mla")
     return out
 
 

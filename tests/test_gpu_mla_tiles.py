@@ -50,7 +50,7 @@ def _reference(q, pool, rtt, pre, ext, scale):
 TOL = {torch.float16: 2e-3, torch.bfloat16: 1.6e-2}
 
 
-def _run(pre, ext, H, dtype, layout, decode, ws_bytes=None, sms=0, odd=()):
+def _run(pre, ext, H, dtype, layout, decode, ws_bytes=None, sms=0, odd=(), own=True):
     from semi_pd_b200 import ops
     g = torch.Generator().manual_seed(sum(ext) + 7 * sum(pre) + H)
     lens = [p + e for p, e in zip(pre, ext)]
@@ -74,9 +74,11 @@ def _run(pre, ext, H, dtype, layout, decode, ws_bytes=None, sms=0, odd=()):
     ops.set_sm_budget(sms)
     try:
         out = ops.attn_mla(q.to(DEV).view(q.shape[0], -1), pool.to(DEV), rtt.to(DEV), torch.arange(len(ext), device=DEV), H,
-                           R, DR, scale, ws, **more)
+                           R, DR, scale, ws, own_workspace=own, **more)
     finally:
         ops.set_sm_budget(0)
+    if not own and q.shape[0] * -(-H // 16) >= 2 * (sms or ops.device_sm_count(0)):
+        assert bool((ws == 255).all())  # another stream may be using it
     out = out.cpu().double().view(want.shape)
     err = (out - want)[blind].abs().max().item()
     assert err < TOL[dtype], err
@@ -130,6 +132,12 @@ def test_small_partition_and_request_starts():
     # 40 requests on 2 SMs: 20 per SM, cut at request starts; on 8 SMs the ranges cut requests
     for sms in (2, 8):
         _run([50 + 9 * i for i in range(40)], [1] * 40, 16, torch.bfloat16, "runs", True, sms=sms)
+
+
+def test_a_shared_workspace():
+    _run([0, 640], [700, 259], 16, torch.float16, "runs", False, own=False)
+    _run([50 + 9 * i for i in range(40)], [1] * 40, 16, torch.bfloat16, "runs", True, sms=8, own=False)
+    _run([300, 64], [40, 5], 16, torch.bfloat16, "runs", False, own=False)  # too small to go without it
 
 
 @pytest.mark.parametrize("decode", [True, False])
