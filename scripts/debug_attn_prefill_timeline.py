@@ -1,6 +1,6 @@
 """In-kernel timeline of the prefill attention (CTA 0): when each softmax warpgroup waits for S /
-publishes P and when the MMA issuer waits for P / issues PV + next S.
-usage: python scripts/debug_attn_prefill_timeline.py [sm_budget] [nreq] [ext_len]   (SPD_ATTN_PF_UNIT=64|128)"""
+publishes P and when the MMA issuers wait for P / issue PV + next S.
+usage: python scripts/debug_attn_prefill_timeline.py [sm_budget] [nreq] [ext_len]"""
 import ctypes as C
 import sys
 
@@ -31,17 +31,17 @@ run = lambda: ops.attn_prefill(q, kp, vp, rtt, rpi, pre, ext, st, E, Hq, Hk, D, 
 run()
 torch.cuda.synchronize()
 cap = 8192
-buf = torch.zeros(3 * cap * 2, dtype=torch.int64, device=dev)
+buf = torch.zeros(4 * cap * 2, dtype=torch.int64, device=dev)
 fn = _lib.lib.spd_debug_attn_prefill_trace
 fn.argtypes = [C.c_void_p, C.c_int64]
 fn(buf.data_ptr(), cap)
 run()
 torch.cuda.synchronize()
 fn(None, 0)
-ev = buf.cpu().numpy().reshape(3, cap, 2)
-t0 = min(int(ev[r, 0, 1]) for r in range(3) if ev[r, 0, 0])
-names = {0: "softmax wg0", 1: "softmax wg1", 2: "mma issuer"}
-for r in range(3):
+ev = buf.cpu().numpy().reshape(4, cap, 2)
+t0 = min(int(ev[r, 0, 1]) for r in range(4) if ev[r, 0, 0])
+names = {0: "softmax wg0", 1: "softmax wg1", 2: "mma issuer 0", 3: "mma issuer 1"}
+for r in range(4):
     e = ev[r][ev[r, :, 0] != 0]
     tags, clk = e[:, 0] >> 8, e[:, 1] - t0
     print(f"-- {names[r]}: {len(e)} events, span {clk[-1] - clk[0]} clk")
@@ -64,7 +64,7 @@ for r in range(3):
         print(f"   units {len(c)}: wait-for-P mean {np.mean(w):.0f} (p50 {np.median(w):.0f}, p90 {np.percentile(w, 90):.0f}), "
               f"V-wait+issue mean {np.mean(c):.0f} (p50 {np.median(c):.0f}, p90 {np.percentile(c, 90):.0f})")
 # merged excerpt from the middle of the run
-allev = sorted((int(ev[r, i, 1]) - t0, r, int(ev[r, i, 0])) for r in range(3) for i in range(cap) if ev[r, i, 0])
+allev = sorted((int(ev[r, i, 1]) - t0, r, int(ev[r, i, 0])) for r in range(4) for i in range(cap) if ev[r, i, 0])
 mid = len(allev) // 2
 lab = {1: "wait", 2: "ready", 3: "done", 4: "epilogue", 5: "drained", 6: "stored"}
 print("-- excerpt (clk, role, event, unit)")

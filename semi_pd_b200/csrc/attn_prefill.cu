@@ -33,13 +33,16 @@
 //                    strided 2-D box of the pool and is fetched with two TMA tensor copies by one
 //                    lane; any other tile (scattered slots, the ragged tail of a sequence) is
 //                    gathered row by row through req_to_token with 16-byte cp.async;
-//   warp 10          MMA issuer: S_w,h = Q_w K_j[h]^T (both K-major in smem), O_w += P_w,h V_j[h] (P
-//                    from TMEM, V MN-major in smem); per warpgroup and half the order is PV(j,h)
-//                    then S(j+1,h) (which overwrites the columns P(j,h) lives in; tcgen05.mma
-//                    executes in order);
-//   warp 11          Q loader (TMA): the next item's Q tiles are fetched as soon as the current
-//                    item's last S MMA has read them.
-// Items are ordered heaviest (latest query tiles) first and dealt to the CTAs in snake order.
+//   warp 10, warp 11 MMA issuer of warpgroup 0 / 1: S_h = Q K_j[h]^T (both K-major in smem), O += P_h V_j[h] (P
+//                    from TMEM, V MN-major in smem); the order is PV(j,h) then S(j+1,h) (which overwrites the columns
+//                    P(j,h) lives in; tcgen05.mma executes in order).  The next item's Q tile is fetched (TMA) before the
+//                    item's last PV goes out.
+// The issuers' own time bounded the kernel while one lane of one warp issued for both warpgroups from unrolled code: 65 clk
+// per MMA and 250 between two units.  Whole warps with uniform operands, short loops and an issuer per warpgroup: 8
+// requests of 1024 new tokens on average, half of them behind 1024 cached ones, 32 / 8 heads: 193 -> 176 us; 4 requests
+// of 2048, 16 / 4 heads, window 1024: 142 -> 132 us.  Slower: S issued 128 keys wide with softmax and PV still per half and
+// one issuer (160 / 128 us against 156 / 112 with the sorted items), or with two (250 us: both warpgroups in one phase).
+// Items are ordered heaviest first (pf_sort) and dealt to the CTAs in snake order.
 // smem: Q0 Q1 + 5 K/V slots = 7 x 32 KB.  TMEM: S0a/P0a S0b/P0b | S1a/P1a S1b/P1b | O0 | O1 = 512 columns.
 #include <cuda.h>
 
@@ -49,7 +52,7 @@
 
 namespace spd {
 
-constexpr int kPfThreads = 384;  // 12 warps -> 168 registers per thread for the softmax warps
+constexpr int kPfThreads = 384;  // 12 warps -> 168 registers per thread
 constexpr int kPfM = 128;    // query rows per warpgroup tile
 constexpr int kPfN = 128;    // kv tokens per tile
 constexpr int kPfH = 64;     // kv tokens per half-tile unit (columns of one S half)
@@ -57,7 +60,10 @@ constexpr int kPfD = 128;    // head dim
 constexpr int kTileBytes = 128 * 128 * 2;  // one [128 x 128] 16-bit tile = two 16 KB swizzle blocks
 constexpr int kPfSlots = 4;
 constexpr int kPfStage = 2 * 16384;  // epilogue staging: one [128 x 64] 16-bit block per warpgroup
-constexpr int kPfSmem = kTileBytes * (2 + kPfSlots) + kPfStage + 1024 + 512;
+constexpr int kPfBars = 512;
+constexpr int kPfList = 768;          // row tiles that the sorted list holds
+constexpr int kPfSmem = kTileBytes * (2 + kPfSlots) + kPfStage + kPfBars + kPfList * 2 + 1024;
+static_assert(kPfSmem <= 232448, "shared memory of one block");
 constexpr float kRescaleTrigger = 256.f;  // a row sum above 2^8 may hide an element above 2^8
 
 struct PrefillParams {
@@ -77,11 +83,12 @@ struct PrefillParams {
   int heads_x;     // item columns along the head axis
   int batch;
   int total_items;
+  int sorted;      // 1: items are dealt from a list of the row tiles by weight (pf_sort)
   int use_tma;  // 0: always gather (SPD_ATTN_TMA=0)
   // n / d for the three launch-constant divisors of the item decode (per_x = heads_x * batch,
   // heads_x, GQA group) as multiply-high + shift: four dependent integer divisions sat on every
   // item boundary of every role
-  uint32_t per_x_m, per_x_s, heads_x_m, heads_x_s, group_m, group_s;
+  uint32_t per_x_m, per_x_s, heads_x_m, heads_x_s, group_m, group_s, tiles_x_m, tiles_x_s;
   // kWin only: keys a query sees up to and with itself; a logit per head in the softmax denominator (nullptr: none); query
   // temperature 1 + coef ln(floor((pos + 1) / every) + 1) (every 0: none)
   int window, qtemp_every;
@@ -97,7 +104,7 @@ struct PrefillParams {
 template <bool kTrace>
 __device__ __forceinline__ void pf_trace(const PrefillParams& p, int region, uint32_t& n, long long tag) {
   if constexpr (kTrace) {
-    if (blockIdx.x == 0 && p.trace && static_cast<int>(n) < p.trace_cap) {
+    if (blockIdx.x == 0 && (threadIdx.x & 31) == 0 && p.trace && static_cast<int>(n) < p.trace_cap) {
       long long* e = p.trace + (static_cast<size_t>(region) * p.trace_cap + n) * 2;
       e[0] = tag;
       e[1] = clock64();
@@ -124,40 +131,64 @@ inline void fastdiv_magic(uint32_t d, uint32_t& m, uint32_t& s) {
   m = static_cast<uint32_t>(((1ull << 32) * ((1ull << s) - d)) / d + 1);
 }
 
-// the three per-request values an item needs from global memory; loaded ONE ITEM AHEAD by every
+// The row tiles of a launch that has more items than CTAs, heaviest first: list[rank] = req * tiles_x + qx.  Every CTA
+// makes the same list in its own shared memory.
+struct PfList {
+  int items;             // items to deal: row tiles x heads_x
+  const uint16_t* list;  // nullptr: no list, items in the order (qx descending, req, head)
+};
+
+// where an item lies, and the three per-request values it needs from global memory; loaded ONE ITEM AHEAD by every
 // role (the dependent loads used to sit between two items: ~1000 clk per item boundary)
 struct PfRaw {
+  int req, qx, hx;
   int ext, pre, start;
 };
-__device__ __forceinline__ PfRaw pf_raw(const PrefillParams& p, int idx) {
-  PfRaw r{0, 0, 0};
-  if (idx < p.total_items) {
-    const int per_x = p.heads_x * p.batch;
-    const int req = fastdiv(idx - fastdiv(idx, p.per_x_m, p.per_x_s) * per_x, p.heads_x_m, p.heads_x_s);
-    r.ext = __ldg(p.extend_lens + req);
-    r.pre = __ldg(p.prefix_lens + req);
-    r.start = __ldg(p.extend_start_loc + req);
+__device__ __forceinline__ PfRaw pf_raw(const PrefillParams& p, const PfList& pl, int idx) {
+  PfRaw r{0, 0, 0, 0, 0, 0};
+  if (idx < pl.items) {
+    if (pl.list != nullptr) {
+      const int e = fastdiv(idx, p.heads_x_m, p.heads_x_s);
+      r.hx = idx - e * p.heads_x;
+      const int slot = pl.list[e];
+      r.req = fastdiv(slot, p.tiles_x_m, p.tiles_x_s);
+      r.qx = slot - r.req * p.tiles_x;
+    } else {
+      const int ix = fastdiv(idx, p.per_x_m, p.per_x_s);
+      const int rest = idx - ix * (p.heads_x * p.batch);
+      r.qx = p.tiles_x - 1 - ix;  // heaviest (latest) query tiles first
+      r.req = fastdiv(rest, p.heads_x_m, p.heads_x_s);
+      r.hx = rest - r.req * p.heads_x;
+    }
+    r.ext = __ldg(p.extend_lens + r.req);
+    r.pre = __ldg(p.prefix_lens + r.req);
+    r.start = __ldg(p.extend_start_loc + r.req);
   }
+  return r;
+}
+// the same in every lane of a warp, and known to be
+__device__ __forceinline__ PfRaw pf_raw_uniform(PfRaw r) {
+  r.req = __shfl_sync(0xffffffffu, r.req, 0);
+  r.qx = __shfl_sync(0xffffffffu, r.qx, 0);
+  r.hx = __shfl_sync(0xffffffffu, r.hx, 0);
+  r.ext = __shfl_sync(0xffffffffu, r.ext, 0);
+  r.pre = __shfl_sync(0xffffffffu, r.pre, 0);
+  r.start = __shfl_sync(0xffffffffu, r.start, 0);
   return r;
 }
 
 template <bool kWin>
-__device__ __forceinline__ PfItem pf_item(const PrefillParams& p, int idx, const PfRaw& raw) {
+__device__ __forceinline__ PfItem pf_item(const PrefillParams& p, const PfRaw& raw) {
   PfItem it;
-  const int per_x = p.heads_x * p.batch;
-  const int ix = fastdiv(idx, p.per_x_m, p.per_x_s);
-  const int qx = p.tiles_x - 1 - ix;  // heaviest (latest) query tiles first
-  const int r = idx - ix * per_x;
-  it.req = fastdiv(r, p.heads_x_m, p.heads_x_s);
-  const int hx = r - it.req * p.heads_x;
+  it.req = raw.req;
   if (p.pair_heads) {
-    it.head[0] = 2 * hx;
-    it.head[1] = 2 * hx + 1;
-    it.m0[0] = it.m0[1] = qx * kPfM;
+    it.head[0] = 2 * raw.hx;
+    it.head[1] = 2 * raw.hx + 1;
+    it.m0[0] = it.m0[1] = raw.qx * kPfM;
   } else {
-    it.head[0] = it.head[1] = hx;
-    it.m0[0] = 2 * qx * kPfM;
-    it.m0[1] = (2 * qx + 1) * kPfM;
+    it.head[0] = it.head[1] = raw.hx;
+    it.m0[0] = 2 * raw.qx * kPfM;
+    it.m0[1] = (2 * raw.qx + 1) * kPfM;
   }
   it.hk = fastdiv(it.head[0], p.group_m, p.group_s);
   const int ext = raw.ext;
@@ -180,6 +211,39 @@ __device__ __forceinline__ PfItem pf_item(const PrefillParams& p, int idx, const
   return it;
 }
 
+// The row tiles with any rows, sorted by the K / V tiles they walk, into `list` (keys: shared memory that nothing uses
+// yet; count: zero before).  Request lengths differ, so the order by query tile alone leaves the CTAs with unequal
+// shares: 8 requests of 512 - 1536 new tokens, four with a prefix of 1024, 102 tiles on the busiest CTA against 79 on
+// average; sorted 81 (176 -> 156 us; with the window, 50 and 37: 132 -> 112 us).
+template <bool kWin>
+__device__ __forceinline__ PfList pf_sort(const PrefillParams& p, uint32_t* keys, uint32_t* count, uint16_t* list) {
+  if (!p.sorted) return PfList{p.total_items, nullptr};
+  for (int slot = threadIdx.x; slot < p.batch * p.tiles_x; slot += kPfThreads) {
+    PfRaw raw{};
+    raw.req = fastdiv(slot, p.tiles_x_m, p.tiles_x_s);
+    raw.qx = slot - raw.req * p.tiles_x;
+    raw.ext = __ldg(p.extend_lens + raw.req);
+    raw.pre = __ldg(p.prefix_lens + raw.req);
+    const PfItem it = pf_item<kWin>(p, raw);
+    if (it.n > 0) {
+      const uint32_t at = atomicAdd(count, 1u);
+      if (at < kPfList) keys[at] = static_cast<uint32_t>(it.n - it.j0) << 16 | static_cast<uint32_t>(slot);
+    }
+  }
+  __syncthreads();
+  const int n = static_cast<int>(*count);
+  if (n > kPfList) return PfList{p.total_items, nullptr};  // more tiles than total_tokens allows
+  for (int e = threadIdx.x; e < n; e += kPfThreads) {
+    const uint32_t key = keys[e];
+    int rank = 0;
+#pragma unroll 8
+    for (int f = 0; f < n; ++f) rank += keys[f] > key;  // keys differ: the order is the same in every CTA
+    list[rank] = static_cast<uint16_t>(key);
+  }
+  __syncthreads();
+  return PfList{n * p.heads_x, list};
+}
+
 // k-th item of CTA c out of G CTAs, snake order over the heaviest-first list
 __device__ __forceinline__ int pf_rank(int k, int c, int G) {
   return k * G + ((k & 1) ? (G - 1 - c) : c);
@@ -191,15 +255,38 @@ __device__ __forceinline__ uint32_t tile_off(int row, int chunk16) {
   return (chunk16 >> 3) * 16384 + row * 128 + (((chunk16 & 7) ^ (row & 7)) << 4);
 }
 
-// D[tmem] (+)= A[tmem] * B[smem]: the A operand (here the 16-bit probabilities, two per 32-bit
-// column, row = TMEM lane) is read from tensor memory
-__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
-                                        uint32_t accumulate) {
+// MMAs and commits issued by the warp's lane for which `on` holds; every lane computes the operands.  Descriptors by
+// halves, as in umma_ss_lo.  umma_ts_if: A (here the 16-bit probabilities, two per 32-bit column, row = TMEM lane) is read
+// from tensor memory.
+__device__ __forceinline__ void umma_ss_if(bool on, uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc,
+                                           uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(tmem_d),
-      "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
+      "mov.b64 da, {%1, %3};\n\t"
+      "mov.b64 db, {%2, %3};\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "setp.ne.b32 q, %6, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t}\n" ::"r"(tmem_d),
+      "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate), "r"(static_cast<uint32_t>(on))
+      : "memory");
+}
+__device__ __forceinline__ void umma_ts_if(bool on, uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t b_hi,
+                                           uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 db;\n\t"
+      "mov.b64 db, {%2, %3};\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "setp.ne.b32 q, %6, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}\n" ::"r"(tmem_d),
+      "r"(tmem_a), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(static_cast<uint32_t>(on))
+      : "memory");
+}
+__device__ __forceinline__ void umma_commit_if(bool on, uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n" ::"r"(smem_u32(bar)),
+      "r"(static_cast<uint32_t>(on))
       : "memory");
 }
 
@@ -250,12 +337,12 @@ __device__ __forceinline__ void softmax_chunk(const uint32_t* r, int c, uint32_t
   }
 }
 
-// One row of one S unit (kU = 64 or 128 columns) for one thread: S (TMEM) -> kU/2 packed 16-bit
+// One row of one S unit (64 columns) for one thread: S (TMEM) -> 32 packed 16-bit
 // pairs in registers.  Returns the row sum of p (masked entries excluded).  Two 32-column TMEM
 // loads are in flight while the previous 32 columns are exponentiated.  kMask is a template
 // parameter so that the unmasked units run the lean loop: FFMA + MUFU.EX2 + FADD + half an F2FP
 // per element.
-template <typename T, bool kMask, int kU, bool kWin>
+template <typename T, bool kMask, bool kWin>
 __device__ __forceinline__ float softmax_row_pass(uint32_t ts, uint32_t* pk, float scale_log2, float m_off,
                                                   int kv0, int limit, int span) {
   const uint64_t scale2 = pack_f32x2(scale_log2, scale_log2);
@@ -266,14 +353,7 @@ __device__ __forceinline__ float softmax_row_pass(uint32_t ts, uint32_t* pk, flo
   tmem_ld_32x32b_x32(ts + 32, rb);
   tmem_ld_wait();
   softmax_chunk<T, kMask, kWin>(ra, 0, pk, scale2, neg_m2, kv0, limit, span, ps);
-  if constexpr (kU == 128) tmem_ld_32x32b_x32(ts + 64, ra);  // in flight under the next chunk
   softmax_chunk<T, kMask, kWin>(rb, 32, pk + 16, scale2, neg_m2, kv0, limit, span, ps);
-  if constexpr (kU == 128) {
-    tmem_ld_32x32b_x32(ts + 96, rb);
-    tmem_ld_wait();
-    softmax_chunk<T, kMask, kWin>(ra, 64, pk + 32, scale2, neg_m2, kv0, limit, span, ps);
-    softmax_chunk<T, kMask, kWin>(rb, 96, pk + 48, scale2, neg_m2, kv0, limit, span, ps);
-  }
   float ps0, ps1;
   unpack_f32x2(ps, ps0, ps1);
   return ps0 + ps1;
@@ -293,18 +373,15 @@ __device__ __forceinline__ void rowmax_chunk(const uint32_t* r, int c, int kv0, 
     m1 = fmaxf(m1, b);
   }
 }
-template <bool kMask, int kU, bool kWin>
+template <bool kMask, bool kWin>
 __device__ __forceinline__ float softmax_row_max(uint32_t ts, int kv0, int limit, int span) {
   float m0 = -INFINITY, m1 = -INFINITY;
-#pragma unroll
-  for (int c = 0; c < kU; c += 64) {
-    uint32_t ra[32], rb[32];
-    tmem_ld_32x32b_x32(ts + c, ra);
-    tmem_ld_32x32b_x32(ts + c + 32, rb);
-    tmem_ld_wait();
-    rowmax_chunk<kMask, kWin>(ra, c, kv0, limit, span, m0, m1);
-    rowmax_chunk<kMask, kWin>(rb, c + 32, kv0, limit, span, m0, m1);
-  }
+  uint32_t ra[32], rb[32];
+  tmem_ld_32x32b_x32(ts, ra);
+  tmem_ld_32x32b_x32(ts + 32, rb);
+  tmem_ld_wait();
+  rowmax_chunk<kMask, kWin>(ra, 0, kv0, limit, span, m0, m1);
+  rowmax_chunk<kMask, kWin>(rb, 32, kv0, limit, span, m0, m1);
   return fmaxf(m0, m1);
 }
 
@@ -346,15 +423,11 @@ __device__ __noinline__ float2 pf_row_alone(const T* q, const T* k_pool, const T
   return acc;
 }
 
-// kU: columns of one softmax / MMA unit.  64: the half-tile pipeline described above.  128: one
-// unit per K/V tile — S = Q K^T goes out as ONE N = 128 group (8 instead of 16 SS-form MMAs per
-// tile, the form whose fixed cost per instruction dominates at N = 64) and the two warpgroups
-// alternate on the tensor core tile by tile.
 // kWin: a sliding window (KV tiles before the item's first visible key are skipped), sinks and a query temperature — the
 // general attention of the hybrid families at head size 128 (see spd::attn_prefill_window_try).
 // 4 requests of 2048 new tokens, 16 / 4 heads, window 1024: 320 us on warp-level MMAs with 64 x 64 tiles, 140 us here
 // (60 GFLOP visible; a query tile of 128 meets nine key tiles, two of them masked).
-template <typename T, int kU, bool kTrace, bool kWin>
+template <typename T, bool kTrace, bool kWin>
 __global__ void __launch_bounds__(kPfThreads, 1)
 attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
@@ -366,8 +439,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   uint8_t* sKV = smem + 2 * kTileBytes;   // ring: position 2t = K of tile t, 2t+1 = V of tile t
   uint8_t* sO = smem + (2 + kPfSlots) * kTileBytes;  // epilogue staging, 16 KB per warpgroup
   uint64_t* bars = reinterpret_cast<uint64_t*>(sO + kPfStage);
-  uint64_t* q_full = bars;                     // 1
-  uint64_t* q_empty = bars + 1;                // 1
+  uint64_t* q_full = bars;                     // 2
   uint64_t* kv_full = bars + 2;                // kPfSlots
   uint64_t* kv_empty = kv_full + kPfSlots;     // kPfSlots
   uint64_t* s_full = kv_empty + kPfSlots;      // 4: [warpgroup][half]
@@ -375,19 +447,21 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   uint64_t* pv_done = p_full + 4;              // 4: [warpgroup][half] (see the parity note in the softmax)
   uint64_t* o_free = pv_done + 4;              // 2
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_free + 2);
+  uint32_t* n_tiles = tmem_slot + 1;
+  uint16_t* list = reinterpret_cast<uint16_t*>(sO + kPfStage + kPfBars);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   const int lane = threadIdx.x & 31;
   const int cta = blockIdx.x, ncta = gridDim.x;
+  constexpr int kU = kPfH;        // columns of one softmax / MMA unit
   constexpr int kNU = kPfN / kU;  // units per K/V tile
 
   if (warp == 10) {
     if (lane == 0) {
-      mbar_init(q_full, 1);
-      mbar_init(q_empty, 1);
+      for (int i = 0; i < 2; ++i) mbar_init(&q_full[i], 1);
       for (int i = 0; i < kPfSlots; ++i) {
         mbar_init(&kv_full[i], 32);
-        mbar_init(&kv_empty[i], 1);
+        mbar_init(&kv_empty[i], 2);
       }
       for (int i = 0; i < 4; ++i) {
         mbar_init(&s_full[i], 1);
@@ -395,6 +469,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         mbar_init(&pv_done[i], 1);
       }
       for (int i = 0; i < 2; ++i) mbar_init(&o_free[i], 4);
+      *n_tiles = 0;
       fence_barrier_init();
     }
     __syncwarp();
@@ -414,126 +489,121 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const uint32_t tmem_O = tmem_base + 256;  // 2 x 128 columns
 
   griddep_wait();
+  const PfList pl = pf_sort<kWin>(p, reinterpret_cast<uint32_t*>(sO), n_tiles, list);
 
-  if (warp == 11) {
-    // ===================== Q loader =====================
-    if (elect_one()) {
-      uint32_t itn = 0;
-      int idx = pf_rank(0, cta, ncta);
-      PfRaw raw = pf_raw(p, idx);
-      for (int k = 0; idx < p.total_items; ++k) {
-        const PfItem it = pf_item<kWin>(p, idx, raw);
-        idx = pf_rank(k + 1, cta, ncta);
-        raw = pf_raw(p, idx);
-        if (it.n == 0) continue;
-        mbar_wait(q_empty, (itn & 1) ^ 1);
-        mbar_expect_tx(q_full, ((it.rows[0] > 0) + (it.rows[1] > 0)) * kTileBytes);
-#pragma unroll
-        for (int w = 0; w < 2; ++w)
-          if (it.rows[w] > 0) {
-            tma_load_2d(sQ + w * kTileBytes, &tmQ, q_full, it.head[w] * kPfD, it.q_row0[w], kEvictFirst);
-            tma_load_2d(sQ + w * kTileBytes + 16384, &tmQ, q_full, it.head[w] * kPfD + 64, it.q_row0[w],
-                        kEvictFirst);
-          }
-        ++itn;
+  if (warp >= 10) {
+    // ===================== MMA issuer of warpgroup 0 (warp 10) / 1 (warp 11) =====================
+    // The whole warp walks the items and one lane issues: descriptors then stay in uniform registers.  Short loops, not
+    // unrolled ones.
+    const bool leader = elect_one();
+    const int w = warp - 10;
+    constexpr uint32_t idesc_qk = umma_idesc<T>(kPfM, kU, 0, 0);    // A, B K-major; N = one unit
+    constexpr uint32_t idesc_pv = umma_idesc<T>(kPfM, kPfD, 0, 1);  // A = P (TMEM), B = V MN-major
+    const uint64_t qd = umma_desc_sw128(smem_u32(sQ + w * kTileBytes), 16, 1024);
+    const uint64_t kd0 = umma_desc_sw128(smem_u32(sKV), 16, 1024);
+    const uint64_t vd0 = umma_desc_sw128(smem_u32(sKV), 16384, 1024);
+    const uint32_t qk_hi = static_cast<uint32_t>(qd >> 32), v_hi = static_cast<uint32_t>(vd0 >> 32);
+    uint32_t t_base = 0;  // tiles of all previous items (ring position / 2)
+    uint32_t pq = 0;      // PV units issued (all items); unit of the tile = pq % kNU
+    uint32_t eq = 0;      // items of the warpgroup (o_free phase)
+    uint32_t tn = 0;
+    bool q_ahead = false;  // the next item's Q is already under way
+    auto load_q = [&](const PfItem& it) {
+      const int head = w == 0 ? it.head[0] : it.head[1], row0 = w == 0 ? it.q_row0[0] : it.q_row0[1];
+      if (leader) {
+        mbar_expect_tx(&q_full[w], kTileBytes);
+        tma_load_2d(sQ + w * kTileBytes, &tmQ, &q_full[w], head * kPfD, row0, kEvictFirst);
+        tma_load_2d(sQ + w * kTileBytes + 16384, &tmQ, &q_full[w], head * kPfD + 64, row0, kEvictFirst);
       }
-    }
-  } else if (warp == 10) {
-    // ===================== MMA issuer =====================
-    if (elect_one()) {
-      constexpr uint32_t idesc_qk = umma_idesc<T>(kPfM, kU, 0, 0);  // A, B K-major; N = one unit
-      constexpr uint32_t idesc_pv = umma_idesc<T>(kPfM, kPfD, 0, 1);  // A = P (TMEM), B = V MN-major
-      uint32_t t_base = 0;          // tiles of all previous items (ring position / 2)
-      uint32_t pq[2] = {0, 0};      // PV units issued per warpgroup (all items); unit of the tile = pq % kNU
-      uint32_t eq[2] = {0, 0};      // items per warpgroup (o_free phase)
-      uint32_t itn = 0;
-      uint32_t tn = 0;
-      int idx = pf_rank(0, cta, ncta);
-      PfRaw raw = pf_raw(p, idx);
-      for (int kk = 0; idx < p.total_items; ++kk) {
-        const PfItem it = pf_item<kWin>(p, idx, raw);
-        idx = pf_rank(kk + 1, cta, ncta);
-        raw = pf_raw(p, idx);
-        if (it.n == 0) continue;
-        mbar_wait(q_full, itn & 1);
-        // S_w(j, h): the warpgroup's previous P in these columns has been consumed by PV(j-1, h),
-        // issued earlier by this thread — tcgen05.mma executes in issue order.
-        // (Tried: interleaving the two warpgroups' MMAs instruction by instruction —
-        // back-to-back tcgen05.mma on ONE accumulator cost ~43 clk (SS) / ~10 clk (TS) more than
-        // N/2 each, alternating accumulators runs at the shared-memory operand rate
-        // (rates of unrolled MMAs; from a short loop one of M = 128, N = 64 takes 46 clk on one or several).  The issuer's time per unit pair did drop from
-        // 2 x 795 to 1293 clk, but pairing forces both warpgroups' softmax passes into the same
-        // phase (1020 -> 1500 clk per pass, XU contention) and the kernel got 2-5 % slower.
-        // Second attempt: keep the warpgroups staggered and interleave PV(t) — as two 64-column
-        // halves of O — with S'(t-1), the next tile's S of the chain served one step earlier.  Correct, and 30 %
-        // SLOWER: the issuer needed 1205 clk per 16-instruction step, 75 clk per instruction —
-        // alternating TS- and SS-form MMAs costs more than either stream alone (8 x 42 + 8 x 75
-        // by the probe), the alternation benefit exists for SS next to SS only.)
-        auto issue_s = [&](int w, int j, int h) {
-          const uint32_t pos = 2 * (t_base + j - it.j0);
-          mbar_wait(&kv_full[pos % kPfSlots], (pos / kPfSlots) & 1);
-          tc_fence_after_sync();
-          const uint32_t q_addr = smem_u32(sQ + w * kTileBytes);
-          const uint32_t k_addr = smem_u32(sKV + (pos % kPfSlots) * kTileBytes) + h * (kU * 128);
+      __syncwarp();
+    };
+    int idx = pf_rank(0, cta, ncta);
+    PfRaw raw = pf_raw_uniform(pf_raw(p, pl, idx));
+    for (int kk = 0; idx < pl.items; ++kk) {
+      const PfItem it = pf_item<kWin>(p, raw);
+      idx = pf_rank(kk + 1, cta, ncta);
+      raw = pf_raw_uniform(pf_raw(p, pl, idx));
+      if (it.n == 0) continue;
+      const int nt = w == 0 ? it.nt[0] : it.nt[1];
+      if (nt > 0) {
+        if (!q_ahead) load_q(it);
+        q_ahead = false;
+        mbar_wait(&q_full[w], eq & 1);
+      }
+      // S(j, h): the warpgroup's previous P in these columns has been consumed by PV(j-1, h),
+      // issued earlier by this thread — tcgen05.mma executes in issue order.
+      auto issue_s = [&](int j, int h) {
+        const uint32_t pos = 2 * (t_base + j - it.j0);
+        mbar_wait(&kv_full[pos % kPfSlots], (pos / kPfSlots) & 1);
+        tc_fence_after_sync();
+        uint32_t qa = static_cast<uint32_t>(qd);
+        uint32_t ka = static_cast<uint32_t>(kd0) + (pos % kPfSlots) * (kTileBytes / 16) + h * (kU * 128 / 16);
+        const uint32_t td = tmem_S + w * kPfN + h * kU;
+#pragma unroll 1
+        for (int k = 0; k < kPfD / 16; ++k) {
+          umma_ss_if(leader, td, qa, ka, qk_hi, idesc_qk, k);
+          const uint32_t step = k == 3 ? (16384 - 96) / 16 : 2;
+          qa += step;
+          ka += step;
+        }
+        umma_commit_if(leader, &s_full[w * 2 + h]);
+      };
+      // K_j (V_j) is released by both issuers, also by one whose warpgroup does not use the tile: it waits for the tile
+      // first, so that its arrivals keep to the ring's phases
+      auto release_k = [&](int j) {
+        const uint32_t pos = 2 * (t_base + j - it.j0);
+        if (j >= nt) mbar_wait(&kv_full[pos % kPfSlots], (pos / kPfSlots) & 1);
+        umma_commit_if(leader, &kv_empty[pos % kPfSlots]);
+      };
+      // the epilogue of the previous item reads O, not S — and its last PVs (reading P in the S
+      // columns) were issued before these, so S(0, .) may go out immediately
+      if (it.j0 < nt) {
 #pragma unroll
-          for (int k = 0; k < kPfD / 16; ++k) {
-            const uint32_t off = (k >> 2) * 16384 + (k & 3) * 32;
-            umma_ss(tmem_S + w * kPfN + h * kU, umma_desc_sw128(q_addr + off, 16, 1024),
-                    umma_desc_sw128(k_addr + off, 16, 1024), idesc_qk, k > 0 ? 1u : 0u);
-          }
-          umma_commit(&s_full[w * 2 + h]);
-        };
-        // after every unit of S(j) of both warpgroups has been issued: release K_j, and Q after
-        // the item's last S
-        auto s_tile_issued = [&](int j) {
-          umma_commit(&kv_empty[(2 * (t_base + j - it.j0)) % kPfSlots]);
-          if (j == it.n - 1) umma_commit(q_empty);
-        };
-        // the epilogue of the previous item reads O, not S — and its last PVs (reading P in the S
-        // columns) were issued before these, so S(0, .) may go out immediately
-#pragma unroll
-        for (int h = 0; h < kNU; ++h)
-#pragma unroll
-          for (int w = 0; w < 2; ++w)
-            if (it.nt[w] > 0) issue_s(w, it.j0, h);
-        s_tile_issued(it.j0);
-        for (int j = it.j0; j < it.n; ++j) {
-          const uint32_t vpos = 2 * (t_base + j - it.j0) + 1;
+        for (int h = 0; h < kNU; ++h) issue_s(it.j0, h);
+      }
+      release_k(it.j0);
+      for (int j = it.j0; j < it.n; ++j) {
+        const uint32_t vpos = 2 * (t_base + j - it.j0) + 1;
+        if (j < nt) {
 #pragma unroll
           for (int h = 0; h < kNU; ++h) {
-#pragma unroll
-            for (int w = 0; w < 2; ++w) {
-              if (j >= it.nt[w]) continue;
-              pf_trace<kTrace>(p, 2, tn, 0x100 + w * 2 + h);  // waiting for P
-              mbar_wait(&p_full[w * 2 + h], (pq[w] / kNU) & 1);
-              pf_trace<kTrace>(p, 2, tn, 0x200 + w * 2 + h);  // P ready
-              mbar_wait(&kv_full[vpos % kPfSlots], (vpos / kPfSlots) & 1);
-              if (j == it.j0 && h == 0) mbar_wait(&o_free[w], (eq[w] & 1) ^ 1);  // previous item's O has been read
-              tc_fence_after_sync();
-              const uint32_t v_addr = smem_u32(sKV + (vpos % kPfSlots) * kTileBytes) + h * (kU * 128);
-#pragma unroll
-              for (int k = 0; k < kU / 16; ++k) {
-                // A = P[128 x 16 kv]: 8 TMEM columns per k-step; B = V[16 kv x 128 d] (MN-major: 2
-                // blocks of 64 d, LBO = 16 KB; kv rows 128 B apart, 8-row groups SBO = 1 KB)
-                umma_ts(tmem_O + w * kPfD, tmem_S + w * kPfN + h * kU + k * 8,
-                        umma_desc_sw128(v_addr + k * 2048, 16384, 1024), idesc_pv,
-                        (j > it.j0 || h > 0 || k > 0) ? 1u : 0u);
-              }
-              umma_commit(&pv_done[w * 2 + h]);
-              ++pq[w];
-              if (j + 1 < it.nt[w]) issue_s(w, j + 1, h);
-              pf_trace<kTrace>(p, 2, tn, 0x300 + w * 2 + h);  // PV (+ next S) issued
+            pf_trace<kTrace>(p, 2 + w, tn, 0x100 + w * 2 + h);  // waiting for P
+            mbar_wait(&p_full[w * 2 + h], (pq / kNU) & 1);
+            pf_trace<kTrace>(p, 2 + w, tn, 0x200 + w * 2 + h);  // P ready
+            mbar_wait(&kv_full[vpos % kPfSlots], (vpos / kPfSlots) & 1);
+            if (j == it.j0 && h == 0) mbar_wait(&o_free[w], (eq & 1) ^ 1);  // previous item's O has been read
+            if (j == nt - 1 && h == kNU - 1 && idx < pl.items) {
+              // every S of the item is complete: its P has arrived.  Q's memory is free for the next item.
+              const PfItem next = pf_item<kWin>(p, raw);
+              q_ahead = (w == 0 ? next.nt[0] : next.nt[1]) > 0;
+              if (q_ahead) load_q(next);
             }
+            tc_fence_after_sync();
+            uint32_t va = static_cast<uint32_t>(vd0) + (vpos % kPfSlots) * (kTileBytes / 16) + h * (kU * 128 / 16);
+            uint32_t pa = tmem_S + w * kPfN + h * kU;
+            uint32_t acc = (j > it.j0 || h > 0) ? 1u : 0u;
+#pragma unroll 1
+            for (int k = 0; k < kU / 16; ++k) {
+              // A = P[128 x 16 kv]: 8 TMEM columns per k-step; B = V[16 kv x 128 d] (MN-major: 2
+              // blocks of 64 d, LBO = 16 KB; kv rows 128 B apart, 8-row groups SBO = 1 KB)
+              umma_ts_if(leader, tmem_O + w * kPfD, pa, va, v_hi, idesc_pv, acc);
+              pa += 8;
+              va += 2048 / 16;
+              acc = 1;
+            }
+            umma_commit_if(leader, &pv_done[w * 2 + h]);
+            ++pq;
+            if (j + 1 < nt) issue_s(j + 1, h);
+            pf_trace<kTrace>(p, 2 + w, tn, 0x300 + w * 2 + h);  // PV (+ next S) issued
           }
-          umma_commit(&kv_empty[vpos % kPfSlots]);  // V_j: all PVs issued
-          if (j + 1 < it.n) s_tile_issued(j + 1);
+        } else {
+          mbar_wait(&kv_full[vpos % kPfSlots], (vpos / kPfSlots) & 1);
         }
-#pragma unroll
-        for (int w = 0; w < 2; ++w)
-          if (it.nt[w] > 0) ++eq[w];
-        t_base += it.n - it.j0;
-        ++itn;
+        umma_commit_if(leader, &kv_empty[vpos % kPfSlots]);  // V_j: all PVs issued
+        if (j + 1 < it.n) release_k(j + 1);
       }
+      if (nt > 0) ++eq;
+      t_base += it.n - it.j0;
     }
   } else if (warp >= 8) {
     // ===================== K loader (warp 8) / V loader (warp 9) =====================
@@ -545,11 +615,11 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     uint32_t t = 0;        // tiles loaded so far (all items)
     int pending = -1;      // slot whose cp.async group is committed but not yet published
     int idx = pf_rank(0, cta, ncta);
-    PfRaw raw = pf_raw(p, idx);
-    for (int k = 0; idx < p.total_items; ++k) {
-      const PfItem it = pf_item<kWin>(p, idx, raw);
+    PfRaw raw = pf_raw(p, pl, idx);
+    for (int k = 0; idx < pl.items; ++k) {
+      const PfItem it = pf_item<kWin>(p, raw);
       idx = pf_rank(k + 1, cta, ncta);
-      raw = pf_raw(p, idx);
+      raw = pf_raw(p, pl, idx);
       if (it.n == 0) continue;
       const int32_t* rtt = p.req_to_token + p.req_pool_indices[it.req] * p.rtt_stride;
       const int64_t col = static_cast<int64_t>(it.hk) * kPfD + chunk * 8;
@@ -764,11 +834,11 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       }
     };
     int idx = pf_rank(0, cta, ncta);
-    PfRaw raw = pf_raw(p, idx);
-    for (int k = 0; idx < p.total_items; ++k) {
-      const PfItem it = pf_item<kWin>(p, idx, raw);
+    PfRaw raw = pf_raw(p, pl, idx);
+    for (int k = 0; idx < pl.items; ++k) {
+      const PfItem it = pf_item<kWin>(p, raw);
       idx = pf_rank(k + 1, cta, ncta);
-      raw = pf_raw(p, idx);
+      raw = pf_raw(p, pl, idx);
       const int nt = w == 0 ? it.nt[0] : it.nt[1];
       if (nt == 0) continue;
       const int m0 = w == 0 ? it.m0[0] : it.m0[1];
@@ -799,8 +869,8 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           // The true running max, raised at every unit: the largest P of a row is then exactly 1, as in the warp-level kernel
           // that serves the other calls.  (A reference that lags, as below, rounds that P too: 113 us instead of 140, but
           // 9 - 15 % more rms error against 64-bit results.)
-          const float mx = need_mask ? softmax_row_max<true, kU, kWin>(tsh, kv0, limit, span)
-                                     : softmax_row_max<false, kU, kWin>(tsh, kv0, limit, span);
+          const float mx = need_mask ? softmax_row_max<true, kWin>(tsh, kv0, limit, span)
+                                     : softmax_row_max<false, kWin>(tsh, kv0, limit, span);
           if (__any_sync(0xffffffffu, mx > m_used)) {
             const float m_new = fmaxf(m_used, mx);
             const float alpha = (m_used == -INFINITY) ? 0.f : fast_exp2((m_used - m_new) * scale);
@@ -810,32 +880,31 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           }
         } else if (jh == 0) {
           // first unit of the item: establish the reference max with a max-only pre-pass
-          m_used = need_mask ? softmax_row_max<true, kU, kWin>(tsh, kv0, limit, span)
-                             : softmax_row_max<false, kU, kWin>(tsh, kv0, limit, span);
+          m_used = need_mask ? softmax_row_max<true, kWin>(tsh, kv0, limit, span)
+                             : softmax_row_max<false, kWin>(tsh, kv0, limit, span);
         }
         float m_off = (m_used == -INFINITY) ? 0.f : m_used * scale;
         uint32_t pk[kU / 2];
-        float psum = need_mask ? softmax_row_pass<T, true, kU, kWin>(tsh, pk, scale, m_off, kv0, limit, span)
-                               : softmax_row_pass<T, false, kU, kWin>(tsh, pk, scale, m_off, kv0, limit, span);
+        float psum = need_mask ? softmax_row_pass<T, true, kWin>(tsh, pk, scale, m_off, kv0, limit, span)
+                               : softmax_row_pass<T, false, kWin>(tsh, pk, scale, m_off, kv0, limit, span);
         // raise the reference max only when some row may have outgrown it by > 2^8 (an element
         // above 2^8 implies a row sum above 2^8; warp-uniform decision: tcgen05.ld/st are
         // warp-collective); S is still intact (P is stored below), so the unit is simply redone
         if (!kWin && __any_sync(0xffffffffu, psum > kRescaleTrigger)) {
-          const float mx = need_mask ? softmax_row_max<true, kU, kWin>(tsh, kv0, limit, span)
-                                     : softmax_row_max<false, kU, kWin>(tsh, kv0, limit, span);
+          const float mx = need_mask ? softmax_row_max<true, kWin>(tsh, kv0, limit, span)
+                                     : softmax_row_max<false, kWin>(tsh, kv0, limit, span);
           const float m_new = fmaxf(m_used, mx);
           const float alpha = (m_used == -INFINITY) ? 0.f : fast_exp2((m_used - m_new) * scale);
           l *= alpha;
           m_used = m_new;
           m_off = (m_used == -INFINITY) ? 0.f : m_used * scale;
           if (jh > 0) rescale_o(alpha, u);
-          psum = need_mask ? softmax_row_pass<T, true, kU, kWin>(tsh, pk, scale, m_off, kv0, limit, span)
-                           : softmax_row_pass<T, false, kU, kWin>(tsh, pk, scale, m_off, kv0, limit, span);
+          psum = need_mask ? softmax_row_pass<T, true, kWin>(tsh, pk, scale, m_off, kv0, limit, span)
+                           : softmax_row_pass<T, false, kWin>(tsh, pk, scale, m_off, kv0, limit, span);
         }
         l += psum;
         // P over the first kU/2 columns of this S unit (every column of it is in registers by now)
         tmem_st_32x32b_x32(tsh, pk);
-        if constexpr (kU == 128) tmem_st_32x32b_x32(tsh + 32, pk + 32);
         tmem_st_wait();
         tc_fence_before_sync();
         __syncwarp();
@@ -897,6 +966,7 @@ static int pf_setup(PrefillParams& p, CUtensorMap& tq, CUtensorMap& tk, CUtensor
   SPD_REQUIRE(total < (1ll << 30), SPD_E_SHAPE, "prefill attention: too many work items");
   p.total_items = static_cast<int>(total);
   fastdiv_magic(static_cast<uint32_t>(p.heads_x) * static_cast<uint32_t>(p.batch), p.per_x_m, p.per_x_s);
+  fastdiv_magic(static_cast<uint32_t>(p.tiles_x), p.tiles_x_m, p.tiles_x_s);
   fastdiv_magic(static_cast<uint32_t>(p.heads_x), p.heads_x_m, p.heads_x_s);
   fastdiv_magic(static_cast<uint32_t>(num_q_heads / num_kv_heads), p.group_m, p.group_s);
   if (int rc = get_tmap(&tq, q, static_cast<uint64_t>(total_tokens),
@@ -914,6 +984,16 @@ static int pf_setup(PrefillParams& p, CUtensorMap& tq, CUtensorMap& tk, CUtensor
   if (int rc = get_tmap(&tk, k_pool, 1ull << 31, row_elems, row_elems, kPfN)) return rc;
   if (int rc = get_tmap(&tv, v_pool, 1ull << 31, row_elems, row_elems, kPfN)) return rc;
   return 0;
+}
+
+// A list of the row tiles by weight serves where some CTA gets more than one item; it holds kPfList tiles, named by 16 bits
+// (kv lengths below 2^23, so that a weight fits the key's other half).
+static int pf_wants_list(const PrefillParams& p, int64_t total_tokens, int grid) {
+  const int64_t rows = p.pair_heads ? kPfM : 2 * kPfM;
+  return p.total_items > grid && total_tokens / rows + p.batch <= kPfList &&
+                 static_cast<int64_t>(p.batch) * p.tiles_x <= 65536 && p.rtt_stride < (1 << 23)
+             ? 1
+             : 0;
 }
 
 // Ragged extend of the general attention at head size 128 with a window, sinks and a query temperature (no distance bias,
@@ -944,8 +1024,9 @@ int attn_prefill_window_try(void* out, const void* q, const void* k_pool, const 
   p.qtemp_every = qtemp_every > 0 ? qtemp_every : 0;
   const int sms = sm_budget > 0 ? sm_budget : device_sm_count_cached();  // items are dealt to the CTAs that run at once
   const int grid = p.total_items < sms ? p.total_items : sms;
+  p.sorted = pf_wants_list(p, total_tokens, grid);
   SPD_DISPATCH_DTYPE(dtype, {
-    auto kern = attn_prefill_kernel<T, 64, false, true>;
+    auto kern = attn_prefill_kernel<T, false, true>;
     static bool configured = false;
     if (!configured) {
       SPD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmem));
@@ -965,7 +1046,7 @@ int check_attn_args(const char* fn, const void* out, const void* q, const void* 
 using namespace spd;
 
 // debug only (not part of include/spd.h): subsequent launches run the traced build and CTA 0 writes
-// its timeline — 3 regions (softmax warpgroup 0, 1, MMA issuer) of `cap` (tag, clock) pairs
+// its timeline — 4 regions (softmax warpgroup 0, 1, MMA issuer 0, 1) of `cap` (tag, clock) pairs
 static long long* g_pf_trace = nullptr;
 static int g_pf_trace_cap = 0;
 extern "C" int spd_debug_attn_prefill_trace(void* buf, int64_t cap) {
@@ -1000,11 +1081,10 @@ extern "C" int spd_attn_prefill_ragged(void* out, const void* q, const void* k_p
     return rc;
   const int sms = sm_budget > 0 ? sm_budget : device_sm_count_cached();
   const int grid = p.total_items < sms ? p.total_items : sms;
-  // SPD_ATTN_PF_UNIT = 64 | 128: width of a softmax / MMA unit (see the kernel's kU)
-  static const int unit = []() { const char* e = getenv("SPD_ATTN_PF_UNIT"); return (e && atoi(e) == 128) ? 128 : 64; }();
-#define SPD_PF_LAUNCH(U, TR)                                                                           \
+  p.sorted = pf_wants_list(p, total_tokens, grid);
+#define SPD_PF_LAUNCH(TR)                                                                              \
   do {                                                                                                 \
-    auto kern = attn_prefill_kernel<T, U, TR, false>;                                                       \
+    auto kern = attn_prefill_kernel<T, TR, false>;                                                             \
     static bool configured = false;                                                                    \
     if (!configured) {                                                                                 \
       SPD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmem));      \
@@ -1016,12 +1096,9 @@ extern "C" int spd_attn_prefill_ragged(void* out, const void* q, const void* k_p
     if (g_pf_trace) {
       p.trace = g_pf_trace;
       p.trace_cap = g_pf_trace_cap;
-      if (unit == 64) SPD_PF_LAUNCH(64, true);
-      else SPD_PF_LAUNCH(128, true);
-    } else if (unit == 64) {
-      SPD_PF_LAUNCH(64, false);
+      SPD_PF_LAUNCH(true);
     } else {
-      SPD_PF_LAUNCH(128, false);
+      SPD_PF_LAUNCH(false);
     }
   });
 #undef SPD_PF_LAUNCH
