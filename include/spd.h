@@ -40,7 +40,7 @@ typedef void* spd_stream_t; /* cudaStream_t */
  * ------------------------------------------------------------------------------------------- */
 int spd_version(void);
 const char* spd_last_error_string(void);
-/* Waits inside spd_attn_mla and spd_retention_extend are bounded (seconds).  One that runs out sets a word in host memory
+/* Waits inside spd_attn_mla, spd_attn_mla_prefill and spd_retention_extend are bounded (seconds).  One that runs out sets a word in host memory
  * when its kernel ends; what that kernel wrote is not to be trusted (a recurrent state is kept as it was before the tokens
  * the wait stood for), and those calls return SPD_E_TIMEOUT from then on.  spd_wait_status reads the word without
  * synchronising: call it where a kernel's results are known to have arrived.  clear != 0 resets it. */
@@ -354,6 +354,26 @@ int spd_mla_rotary_store(void* q_lat, const void* qa, void* kv_pool, const void*
                          const int64_t* positions, const int64_t* loc, int64_t tokens, int num_heads, int nope_dim,
                          int kv_lora_rank, int rope_dim, int64_t qa_stride, int64_t q_lat_stride, float eps, int dtype,
                          spd_stream_t stream);
+/* The same with the heads' rotated parts left where they were in qa: the queries of spd_attn_mla_prefill. */
+int spd_mla_rotary_store_inplace(void* qa, void* kv_pool, const void* norm_weight, const float* cos_sin_cache,
+                                 const int64_t* positions, const int64_t* loc, int64_t tokens, int num_heads, int nope_dim,
+                                 int kv_lora_rank, int rope_dim, int64_t qa_stride, float eps, int dtype,
+                                 spd_stream_t stream);
+/* rows [total_kv, kv_lora + rope] = the latent rows of every request's prefix_lens[r] + extend_lens[r] keys, one request
+ * after another; kv_start[r] = the first row of request r. */
+int spd_mla_gather(void* rows, int32_t* kv_start, const void* kv_pool, const int32_t* req_to_token,
+                   const int64_t* req_pool_indices, const int32_t* prefix_lens, const int32_t* extend_lens, int64_t batch,
+                   int64_t total_kv, int64_t max_kv_len, int kv_lora_rank, int rope_dim, int64_t req_to_token_stride,
+                   int dtype, spd_stream_t stream);
+/* MLA ragged extend with expanded heads: q [tokens, H, nope + rope] (rotated), kv [total_kv, H, nope + v] = the rows of
+ * spd_mla_gather times kv_b_proj, rows = those rows (their last rope columns are shared by all heads' keys), out
+ * [tokens, H, v].  replaces DeepseekV2AttentionMLA.forward_normal's attention (models/deepseek_v2.py:591-631), with cached
+ * prefixes as well. */
+int spd_attn_mla_prefill(void* out, const void* q, const void* kv, const void* rows, const int32_t* kv_start,
+                         const int32_t* prefix_lens, const int32_t* extend_lens, const int32_t* extend_start_loc,
+                         int64_t batch, int64_t total_tokens, int64_t total_kv, int64_t max_extend_len, int64_t max_kv_len,
+                         int num_heads, int nope_dim, int rope_dim, int v_dim, int64_t q_stride, int64_t out_stride,
+                         float sm_scale, int dtype, int sm_budget, spd_stream_t stream);
 /* Absorbed MLA attention (MQA over the latent pool), decode (seq_lens != NULL: one query per request
  * over its seq_lens[b] rows) or ragged extend (seq_lens == NULL: query token j of request r, row
  * extend_start_loc[r] + j of q, attends keys 0 .. prefix_lens[r] + j).  kv_pool [slots, kv_lora_rank +

@@ -94,6 +94,10 @@ SIGNATURES = {
     "spd_moe_combine": (_i, [_p, _p, _p, _p, _p, _i64, _i, _i64, _i, _p]),
     "spd_moe_dense_act": (_i, [_p, _p, _p, _p, _i64, _i, _i, _i64, _i, _p]),
     "spd_mla_rotary_store": (_i, [_p, _p, _p, _p, _p, _p, _p, _i64, _i, _i, _i, _i, _i64, _i64, _f, _i, _p]),
+    "spd_mla_rotary_store_inplace": (_i, [_p, _p, _p, _p, _p, _p, _i64, _i, _i, _i, _i, _i64, _f, _i, _p]),
+    "spd_mla_gather": (_i, [_p, _p, _p, _p, _p, _p, _p, _i64, _i64, _i64, _i, _i, _i64, _i, _p]),
+    "spd_attn_mla_prefill": (_i, [_p, _p, _p, _p, _p, _p, _p, _p, _i64, _i64, _i64, _i64, _i64, _i, _i, _i, _i, _i64, _i64,
+                                  _f, _i, _i, _p]),
     "spd_attn_mla_workspace_bytes": (_i64, [_i, _i]),
     "spd_attn_mla": (_i, [_p, _p, _p, _p, _p, _p, _p, _p, _i64, _i64, _i, _i, _i, _i64, _i64, _i64, _f, _i, _p,
                           _i64, _i, _p]),

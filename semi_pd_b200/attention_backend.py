@@ -346,3 +346,21 @@ class SpdAttnBackend(AttentionBackend):
         return ops.attn_mla(q_lat, kv, forward_batch.req_to_token_pool.req_to_token,
                             forward_batch.req_pool_indices, prefix_lens=forward_batch.extend_prefix_lens,
                             extend_start_loc=forward_batch.extend_start_loc, **common)
+
+    def forward_mla_expanded(self, q, w_kv_b, layer: RadixAttention, nope_dim: int, v_dim: int, forward_batch: ForwardBatch):
+        """MLA extend with expanded heads (DeepseekV2AttentionMLA.forward_normal, models/deepseek_v2.py:591-631): q
+        [T, H * (nope + rope)], rotated → [T, H * v].  K and V of all keys, cached ones too, are made from the pool's latent
+        rows by one GEMM.  The latent rows of this batch are already in the pool."""
+        kv_pool = forward_batch.token_to_kv_pool.get_key_buffer(layer.layer_id)
+        rank, H = layer.v_head_dim, layer.tp_q_head_num
+        rope = layer.head_dim - rank
+        ext, pre = forward_batch.extend_seq_lens_cpu, forward_batch.extend_prefix_lens_cpu
+        max_kv = max((a + b for a, b in zip(ext, pre)), default=0)
+        rows, start = ops.mla_gather(kv_pool, forward_batch.req_to_token_pool.req_to_token, forward_batch.req_pool_indices,
+                                     forward_batch.extend_prefix_lens, forward_batch.extend_seq_lens, sum(ext) + sum(pre),
+                                     max_kv, rank, rope)
+        kv = ops.linear(rows[:, :rank], w_kv_b)
+        return ops.attn_mla_prefill(q, kv, rows, start, forward_batch.extend_prefix_lens, forward_batch.extend_seq_lens,
+                                    forward_batch.extend_start_loc, max(ext, default=0), max_kv, H, nope_dim, rope, v_dim,
+                                    layer.scaling)
+

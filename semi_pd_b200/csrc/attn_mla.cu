@@ -933,14 +933,14 @@ mla_merge_kernel(const MlaParams p) {
 
 // What stands between the fused q / latent projection and the attention, one CTA per token: the latent row (RMS norm of
 // its 512 columns, rotation of its 64) goes to its cache slot, the rotated part of every query head to its place behind
-// the absorbed part.  Replaces four launches (norm in place, rotation in place, cache write, a strided copy of the rotated
+// the absorbed part, or back to where it was (q_rot: head 0's, in either case).  Replaces four launches (norm in place, rotation in place, cache write, a strided copy of the rotated
 // queries: 8.2 + 7.9 + 5.5 + 12.5 us at 4096 tokens); it moves 13 KB a token, what bounds it is latency at small batches.
 template <typename T>
 __global__ void __launch_bounds__(256)
-mla_rotary_store_kernel(T* __restrict__ q_lat, const T* __restrict__ qa, T* __restrict__ pool, const T* __restrict__ w,
+mla_rotary_store_kernel(T* q_rot, const T* qa, T* __restrict__ pool, const T* __restrict__ w,
                         const float* __restrict__ cos_sin, const int64_t* __restrict__ positions,
-                        const int64_t* __restrict__ loc, int H, int nope, int64_t qa_stride, int64_t q_lat_stride,
-                        float eps) {
+                        const int64_t* __restrict__ loc, int H, int nope, int64_t qa_stride, int64_t q_rot_stride,
+                        int q_head_stride, float eps) {
   constexpr int kRot = kMlaDL - kMlaDV;
   __shared__ float part[2];
   griddep_launch_dependents();
@@ -980,7 +980,7 @@ mla_rotary_store_kernel(T* __restrict__ q_lat, const T* __restrict__ qa, T* __re
       o.e()[2 * j] = from_f32<T>(a * co[j] - b * si[j]);
       o.e()[2 * j + 1] = from_f32<T>(b * co[j] + a * si[j]);
     }
-    stv(h < H ? q_lat + t * q_lat_stride + h * kMlaDL + kMlaDV + c * 8 : dst + kMlaDV + c * 8, o);
+    stv(h < H ? q_rot + t * q_rot_stride + static_cast<int64_t>(h) * q_head_stride + c * 8 : dst + kMlaDV + c * 8, o);
   }
 }
 
@@ -1007,25 +1007,47 @@ using namespace spd;
 
 extern "C" {
 
+static int mla_rotary_store(const char* fn, void* q_rot, int64_t q_rot_stride, int q_head_stride, const void* qa, void* kv_pool,
+                            const void* norm_weight, const float* cos_sin_cache, const int64_t* positions,
+                            const int64_t* loc, int64_t tokens, int num_heads, int nope_dim, int kv_lora_rank, int rope_dim,
+                            int64_t qa_stride, float eps, int dtype, spd_stream_t stream) {
+  SPD_REQUIRE(kv_lora_rank == kMlaDV && rope_dim == kMlaDL - kMlaDV, SPD_E_SHAPE,
+              "%s: built for kv_lora_rank 512 + rope 64 (got %d + %d)", fn, kv_lora_rank, rope_dim);
+  SPD_REQUIRE(tokens >= 0 && tokens < (1ll << 31) && num_heads > 0 && nope_dim >= 0, SPD_E_BADARG, "%s: bad sizes", fn);
+  SPD_REQUIRE(nope_dim % 8 == 0 && qa_stride % 8 == 0 && q_rot_stride % 8 == 0 && aligned16(q_rot) && aligned16(qa) &&
+                  aligned16(kv_pool) && aligned16(norm_weight) && aligned16(cos_sin_cache),
+              SPD_E_ALIGN, "%s: strides must be multiples of 8 and pointers 16-B aligned", fn);
+  if (tokens == 0) return 0;
+  SPD_DISPATCH_DTYPE(dtype, {
+    SPD_CUDA(launch(mla_rotary_store_kernel<T>, dim3((unsigned)tokens), dim3(256), 0, as_stream(stream), pdl_enabled(),
+                    (T*)q_rot, (const T*)qa, (T*)kv_pool, (const T*)norm_weight, cos_sin_cache, positions, loc, num_heads,
+                    nope_dim, qa_stride, q_rot_stride, q_head_stride, eps));
+  });
+  return 0;
+}
+
 int spd_mla_rotary_store(void* q_lat, const void* qa, void* kv_pool, const void* norm_weight, const float* cos_sin_cache,
                          const int64_t* positions, const int64_t* loc, int64_t tokens, int num_heads, int nope_dim,
                          int kv_lora_rank, int rope_dim, int64_t qa_stride, int64_t q_lat_stride, float eps, int dtype,
                          spd_stream_t stream) {
   SPD_REQUIRE(q_lat && qa && kv_pool && norm_weight && cos_sin_cache && positions && loc, SPD_E_BADARG,
               "spd_mla_rotary_store: null pointer");
-  SPD_REQUIRE(kv_lora_rank == kMlaDV && rope_dim == kMlaDL - kMlaDV, SPD_E_SHAPE,
-              "spd_mla_rotary_store: built for kv_lora_rank 512 + rope 64 (got %d + %d)", kv_lora_rank, rope_dim);
-  SPD_REQUIRE(tokens >= 0 && tokens < (1ll << 31) && num_heads > 0 && nope_dim >= 0, SPD_E_BADARG, "spd_mla_rotary_store: bad sizes");
-  SPD_REQUIRE(nope_dim % 8 == 0 && qa_stride % 8 == 0 && q_lat_stride % 8 == 0 && aligned16(q_lat) && aligned16(qa) &&
-                  aligned16(kv_pool) && aligned16(norm_weight) && aligned16(cos_sin_cache),
-              SPD_E_ALIGN, "spd_mla_rotary_store: strides must be multiples of 8 and pointers 16-B aligned");
-  if (tokens == 0) return 0;
-  SPD_DISPATCH_DTYPE(dtype, {
-    SPD_CUDA(launch(mla_rotary_store_kernel<T>, dim3((unsigned)tokens), dim3(256), 0, as_stream(stream), pdl_enabled(),
-                    (T*)q_lat, (const T*)qa, (T*)kv_pool, (const T*)norm_weight, cos_sin_cache, positions, loc, num_heads,
-                    nope_dim, qa_stride, q_lat_stride, eps));
-  });
-  return 0;
+  return mla_rotary_store("spd_mla_rotary_store", static_cast<char*>(q_lat) + 2 * kMlaDV, q_lat_stride, kMlaDL, qa, kv_pool,
+                          norm_weight, cos_sin_cache, positions, loc, tokens, num_heads, nope_dim, kv_lora_rank, rope_dim,
+                          qa_stride, eps, dtype, stream);
+}
+
+int spd_mla_rotary_store_inplace(void* qa, void* kv_pool, const void* norm_weight, const float* cos_sin_cache,
+                                 const int64_t* positions, const int64_t* loc, int64_t tokens, int num_heads, int nope_dim,
+                                 int kv_lora_rank, int rope_dim, int64_t qa_stride, float eps, int dtype,
+                                 spd_stream_t stream) {
+  SPD_REQUIRE(qa && kv_pool && norm_weight && cos_sin_cache && positions && loc, SPD_E_BADARG,
+              "spd_mla_rotary_store_inplace: null pointer");
+  SPD_REQUIRE(nope_dim >= 0 && rope_dim >= 0 && nope_dim < (1 << 20) && rope_dim < (1 << 20), SPD_E_BADARG,
+              "spd_mla_rotary_store_inplace: bad sizes");
+  return mla_rotary_store("spd_mla_rotary_store_inplace", static_cast<char*>(qa) + 2ll * nope_dim, qa_stride,
+                          nope_dim + rope_dim, qa, kv_pool, norm_weight, cos_sin_cache, positions, loc, tokens, num_heads,
+                          nope_dim, kv_lora_rank, rope_dim, qa_stride, eps, dtype, stream);
 }
 
 int64_t spd_attn_mla_workspace_bytes(int num_heads, int kv_lora_rank) {

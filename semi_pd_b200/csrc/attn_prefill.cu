@@ -47,6 +47,7 @@
 #include <cuda.h>
 
 #include "common.cuh"
+#include "prefill_tiles.cuh"
 #include "ptx.cuh"
 #include "tmap.cuh"
 
@@ -61,10 +62,8 @@ constexpr int kTileBytes = 128 * 128 * 2;  // one [128 x 128] 16-bit tile = two 
 constexpr int kPfSlots = 4;
 constexpr int kPfStage = 2 * 16384;  // epilogue staging: one [128 x 64] 16-bit block per warpgroup
 constexpr int kPfBars = 512;
-constexpr int kPfList = 768;          // row tiles that the sorted list holds
-constexpr int kPfSmem = kTileBytes * (2 + kPfSlots) + kPfStage + kPfBars + kPfList * 2 + 1024;
+constexpr int kPfSmem = kTileBytes * (2 + kPfSlots) + kPfStage + kPfBars + kTileList * 2 + 1024;
 static_assert(kPfSmem <= 232448, "shared memory of one block");
-constexpr float kRescaleTrigger = 256.f;  // a row sum above 2^8 may hide an element above 2^8
 
 struct PrefillParams {
   void* out;
@@ -120,31 +119,13 @@ struct PfItem {
   int kv_len;
 };
 
-// floor(n / d), n < 2^31, with (m, s) from fastdiv_magic(d)
-__device__ __forceinline__ int fastdiv(int n, uint32_t m, uint32_t s) {
-  return static_cast<int>((static_cast<uint64_t>(__umulhi(static_cast<uint32_t>(n), m)) + static_cast<uint32_t>(n)) >> s);
-}
-// Granlund-Montgomery round-up magic: s = ceil(log2 d), m = floor(2^32 * (2^s - d) / d) + 1
-inline void fastdiv_magic(uint32_t d, uint32_t& m, uint32_t& s) {
-  s = 0;
-  while ((1ull << s) < d) ++s;
-  m = static_cast<uint32_t>(((1ull << 32) * ((1ull << s) - d)) / d + 1);
-}
-
-// The row tiles of a launch that has more items than CTAs, heaviest first: list[rank] = req * tiles_x + qx.  Every CTA
-// makes the same list in its own shared memory.
-struct PfList {
-  int items;             // items to deal: row tiles x heads_x
-  const uint16_t* list;  // nullptr: no list, items in the order (qx descending, req, head)
-};
-
 // where an item lies, and the three per-request values it needs from global memory; loaded ONE ITEM AHEAD by every
 // role (the dependent loads used to sit between two items: ~1000 clk per item boundary)
 struct PfRaw {
   int req, qx, hx;
   int ext, pre, start;
 };
-__device__ __forceinline__ PfRaw pf_raw(const PrefillParams& p, const PfList& pl, int idx) {
+__device__ __forceinline__ PfRaw pf_raw(const PrefillParams& p, const TileList& pl, int idx) {
   PfRaw r{0, 0, 0, 0, 0, 0};
   if (idx < pl.items) {
     if (pl.list != nullptr) {
@@ -211,178 +192,30 @@ __device__ __forceinline__ PfItem pf_item(const PrefillParams& p, const PfRaw& r
   return it;
 }
 
-// The row tiles with any rows, sorted by the K / V tiles they walk, into `list` (keys: shared memory that nothing uses
-// yet; count: zero before).  Request lengths differ, so the order by query tile alone leaves the CTAs with unequal
-// shares: 8 requests of 512 - 1536 new tokens, four with a prefix of 1024, 102 tiles on the busiest CTA against 79 on
-// average; sorted 81 (176 -> 156 us; with the window, 50 and 37: 132 -> 112 us).
+// The row tiles with any rows, by the K / V tiles they walk (see tile_list).  Request lengths differ, so the order by query
+// tile alone leaves the CTAs with unequal shares: 8 requests of 512 - 1536 new tokens, four with a prefix of 1024, 102
+// tiles on the busiest CTA against 79 on average; sorted 81 (176 -> 156 us; with the window, 50 and 37: 132 -> 112 us).
 template <bool kWin>
-__device__ __forceinline__ PfList pf_sort(const PrefillParams& p, uint32_t* keys, uint32_t* count, uint16_t* list) {
-  if (!p.sorted) return PfList{p.total_items, nullptr};
-  for (int slot = threadIdx.x; slot < p.batch * p.tiles_x; slot += kPfThreads) {
-    PfRaw raw{};
-    raw.req = fastdiv(slot, p.tiles_x_m, p.tiles_x_s);
-    raw.qx = slot - raw.req * p.tiles_x;
-    raw.ext = __ldg(p.extend_lens + raw.req);
-    raw.pre = __ldg(p.prefix_lens + raw.req);
-    const PfItem it = pf_item<kWin>(p, raw);
-    if (it.n > 0) {
-      const uint32_t at = atomicAdd(count, 1u);
-      if (at < kPfList) keys[at] = static_cast<uint32_t>(it.n - it.j0) << 16 | static_cast<uint32_t>(slot);
-    }
-  }
-  __syncthreads();
-  const int n = static_cast<int>(*count);
-  if (n > kPfList) return PfList{p.total_items, nullptr};  // more tiles than total_tokens allows
-  for (int e = threadIdx.x; e < n; e += kPfThreads) {
-    const uint32_t key = keys[e];
-    int rank = 0;
-#pragma unroll 8
-    for (int f = 0; f < n; ++f) rank += keys[f] > key;  // keys differ: the order is the same in every CTA
-    list[rank] = static_cast<uint16_t>(key);
-  }
-  __syncthreads();
-  return PfList{n * p.heads_x, list};
-}
-
-// k-th item of CTA c out of G CTAs, snake order over the heaviest-first list
-__device__ __forceinline__ int pf_rank(int k, int c, int G) {
-  return k * G + ((k & 1) ? (G - 1 - c) : c);
+__device__ __forceinline__ TileList pf_sort(const PrefillParams& p, uint32_t* keys, uint32_t* count, uint16_t* list) {
+  if (!p.sorted) return TileList{p.total_items, nullptr};
+  return tile_list<kPfThreads>(
+      p.batch * p.tiles_x, p.heads_x, p.total_items,
+      [&](int slot) {
+        PfRaw raw{};
+        raw.req = fastdiv(slot, p.tiles_x_m, p.tiles_x_s);
+        raw.qx = slot - raw.req * p.tiles_x;
+        raw.ext = __ldg(p.extend_lens + raw.req);
+        raw.pre = __ldg(p.prefix_lens + raw.req);
+        const PfItem it = pf_item<kWin>(p, raw);
+        return it.n > 0 ? it.n - it.j0 : 0;
+      },
+      keys, count, list);
 }
 
 // byte offset of (row, 16-byte chunk) inside a [128 x 128] 16-bit tile stored as two
 // [128 rows x 128 B] blocks with the 128-byte swizzle (chunk index XOR row%8)
 __device__ __forceinline__ uint32_t tile_off(int row, int chunk16) {
   return (chunk16 >> 3) * 16384 + row * 128 + (((chunk16 & 7) ^ (row & 7)) << 4);
-}
-
-// MMAs and commits issued by the warp's lane for which `on` holds; every lane computes the operands.  Descriptors by
-// halves, as in umma_ss_lo.  umma_ts_if: A (here the 16-bit probabilities, two per 32-bit column, row = TMEM lane) is read
-// from tensor memory.
-__device__ __forceinline__ void umma_ss_if(bool on, uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc,
-                                           uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
-      "mov.b64 da, {%1, %3};\n\t"
-      "mov.b64 db, {%2, %3};\n\t"
-      "setp.ne.b32 p, %5, 0;\n\t"
-      "setp.ne.b32 q, %6, 0;\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t}\n" ::"r"(tmem_d),
-      "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate), "r"(static_cast<uint32_t>(on))
-      : "memory");
-}
-__device__ __forceinline__ void umma_ts_if(bool on, uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t b_hi,
-                                           uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t.reg .b64 db;\n\t"
-      "mov.b64 db, {%2, %3};\n\t"
-      "setp.ne.b32 p, %5, 0;\n\t"
-      "setp.ne.b32 q, %6, 0;\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}\n" ::"r"(tmem_d),
-      "r"(tmem_a), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(static_cast<uint32_t>(on))
-      : "memory");
-}
-__device__ __forceinline__ void umma_commit_if(bool on, uint64_t* bar) {
-  asm volatile(
-      "{\n\t.reg .pred q;\n\t"
-      "setp.ne.b32 q, %1, 0;\n\t"
-      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n" ::"r"(smem_u32(bar)),
-      "r"(static_cast<uint32_t>(on))
-      : "memory");
-}
-
-// Packed fp32 pairs (sm_100 FFMA2 / FADD2): one instruction per two elements.  The softmax warps
-// are issue-bound around the MUFU stream (one warp per scheduler and warpgroup), so halving the
-// FFMA / FADD count is what shortens a row pass.
-__device__ __forceinline__ uint64_t pack_f32x2(float lo, float hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void unpack_f32x2(uint64_t v, float& lo, float& hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ uint64_t ffma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ uint64_t fadd2(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-
-// key `kv` of a masked unit is visible: kv <= limit, and with a window (span = its size - 1) limit - kv <= span
-template <bool kWin>
-__device__ __forceinline__ bool pf_visible(int kv, int limit, int span) {
-  if constexpr (kWin) return static_cast<uint32_t>(limit - kv) <= static_cast<uint32_t>(span);
-  return kv <= limit;
-}
-// 32 columns of one tile row: p = exp2(s*scale - m_off), packed to 16 bits into pk[0..16)
-template <typename T, bool kMask, bool kWin>
-__device__ __forceinline__ void softmax_chunk(const uint32_t* r, int c, uint32_t* pk, uint64_t scale2,
-                                              uint64_t neg_m2, int kv0, int limit, int span, uint64_t& ps) {
-#pragma unroll
-  for (int i = 0; i < 32; i += 2) {
-    float x0, x1;
-    unpack_f32x2(ffma2(pack_f32x2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), scale2, neg_m2), x0, x1);
-    float p0 = fast_exp2(x0);
-    float p1 = fast_exp2(x1);
-    if constexpr (kMask) {
-      p0 = pf_visible<kWin>(kv0 + c + i, limit, span) ? p0 : 0.f;
-      p1 = pf_visible<kWin>(kv0 + c + i + 1, limit, span) ? p1 : 0.f;
-    }
-    ps = fadd2(ps, pack_f32x2(p0, p1));
-    pk[i >> 1] = pack2<T>(p0, p1);
-  }
-}
-
-// One row of one S unit (64 columns) for one thread: S (TMEM) -> 32 packed 16-bit
-// pairs in registers.  Returns the row sum of p (masked entries excluded).  Two 32-column TMEM
-// loads are in flight while the previous 32 columns are exponentiated.  kMask is a template
-// parameter so that the unmasked units run the lean loop: FFMA + MUFU.EX2 + FADD + half an F2FP
-// per element.
-template <typename T, bool kMask, bool kWin>
-__device__ __forceinline__ float softmax_row_pass(uint32_t ts, uint32_t* pk, float scale_log2, float m_off,
-                                                  int kv0, int limit, int span) {
-  const uint64_t scale2 = pack_f32x2(scale_log2, scale_log2);
-  const uint64_t neg_m2 = pack_f32x2(-m_off, -m_off);
-  uint64_t ps = pack_f32x2(0.f, 0.f);
-  uint32_t ra[32], rb[32];
-  tmem_ld_32x32b_x32(ts, ra);
-  tmem_ld_32x32b_x32(ts + 32, rb);
-  tmem_ld_wait();
-  softmax_chunk<T, kMask, kWin>(ra, 0, pk, scale2, neg_m2, kv0, limit, span, ps);
-  softmax_chunk<T, kMask, kWin>(rb, 32, pk + 16, scale2, neg_m2, kv0, limit, span, ps);
-  float ps0, ps1;
-  unpack_f32x2(ps, ps0, ps1);
-  return ps0 + ps1;
-}
-
-// max of the visible raw scores of one row of an S unit (TMEM)
-template <bool kMask, bool kWin>
-__device__ __forceinline__ void rowmax_chunk(const uint32_t* r, int c, int kv0, int limit, int span, float& m0, float& m1) {
-#pragma unroll
-  for (int i = 0; i < 32; i += 2) {
-    float a = __uint_as_float(r[i]), b = __uint_as_float(r[i + 1]);
-    if constexpr (kMask) {
-      a = pf_visible<kWin>(kv0 + c + i, limit, span) ? a : -INFINITY;
-      b = pf_visible<kWin>(kv0 + c + i + 1, limit, span) ? b : -INFINITY;
-    }
-    m0 = fmaxf(m0, a);
-    m1 = fmaxf(m1, b);
-  }
-}
-template <bool kMask, bool kWin>
-__device__ __forceinline__ float softmax_row_max(uint32_t ts, int kv0, int limit, int span) {
-  float m0 = -INFINITY, m1 = -INFINITY;
-  uint32_t ra[32], rb[32];
-  tmem_ld_32x32b_x32(ts, ra);
-  tmem_ld_32x32b_x32(ts + 32, rb);
-  tmem_ld_wait();
-  rowmax_chunk<kMask, kWin>(ra, 0, kv0, limit, span, m0, m1);
-  rowmax_chunk<kMask, kWin>(rb, 32, kv0, limit, span, m0, m1);
-  return fmaxf(m0, m1);
 }
 
 // Output of one query row by a warp, from the keys the row sees alone; before the division by the sum, columns
@@ -489,7 +322,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const uint32_t tmem_O = tmem_base + 256;  // 2 x 128 columns
 
   griddep_wait();
-  const PfList pl = pf_sort<kWin>(p, reinterpret_cast<uint32_t*>(sO), n_tiles, list);
+  const TileList pl = pf_sort<kWin>(p, reinterpret_cast<uint32_t*>(sO), n_tiles, list);
 
   if (warp >= 10) {
     // ===================== MMA issuer of warpgroup 0 (warp 10) / 1 (warp 11) =====================
@@ -823,15 +656,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       // the current phase from the one before it).
       mbar_wait(&pv_done[w * 2 + ((unit - 1) % kNU)], ((unit - 1) / kNU) & 1);
       tc_fence_after_sync();
-#pragma unroll 1
-      for (int c = 0; c < kPfD; c += 32) {
-        uint32_t r[32];
-        tmem_ld_32x32b_x32(to + c, r);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * alpha);
-        tmem_st_32x32b_x32(to + c, r);
-      }
+      rescale_row128(to, alpha);
     };
     int idx = pf_rank(0, cta, ncta);
     PfRaw raw = pf_raw(p, pl, idx);
@@ -865,46 +690,53 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         mbar_wait(&s_full[w * 2 + h], (u / kNU) & 1);
         tc_fence_after_sync();
         if (tracer) pf_trace<kTrace>(p, w, tn, 0x200 + h);  // S ready
+        uint32_t pk[kU / 2];
+        bool raise = false;  // kWin: the reference max has been raised, O is rescaled below
+        float alpha = 1.f;
         if constexpr (kWin) {
-          // The true running max, raised at every unit: the largest P of a row is then exactly 1, as in the warp-level kernel
-          // that serves the other calls.  (A reference that lags, as below, rounds that P too: 113 us instead of 140, but
-          // 9 - 15 % more rms error against 64-bit results.)
-          const float mx = need_mask ? softmax_row_max<true, kWin>(tsh, kv0, limit, span)
-                                     : softmax_row_max<false, kWin>(tsh, kv0, limit, span);
-          if (__any_sync(0xffffffffu, mx > m_used)) {
+          // The true running max: the largest P of a row is then exactly 1, as in the warp-level kernel that serves the
+          // other calls.  (A reference that lags, as below, rounds that P too: 9 - 15 % more rms error against 64-bit results.)
+          // One read of the unit for the max and the P, and O rescaled after the exponentials: 112 -> 101 us for 4
+          // requests of 2048 new tokens, 16 / 4 heads, window 1024; the sum of the rounded P: 0.6 % less rms error.
+          uint32_t ra[32], rb[32];
+          const float mx = need_mask ? softmax_load_max<true, kWin>(tsh, ra, rb, kv0, limit, span)
+                                     : softmax_load_max<false, kWin>(tsh, ra, rb, kv0, limit, span);
+          raise = __any_sync(0xffffffffu, mx > m_used);
+          if (raise) {
             const float m_new = fmaxf(m_used, mx);
-            const float alpha = (m_used == -INFINITY) ? 0.f : fast_exp2((m_used - m_new) * scale);
+            alpha = (m_used == -INFINITY) ? 0.f : fast_exp2((m_used - m_new) * scale);
             l *= alpha;
             m_used = m_new;
-            if (jh > 0) rescale_o(alpha, u);
+            raise = jh > 0;
           }
-        } else if (jh == 0) {
-          // first unit of the item: establish the reference max with a max-only pre-pass
-          m_used = need_mask ? softmax_row_max<true, kWin>(tsh, kv0, limit, span)
-                             : softmax_row_max<false, kWin>(tsh, kv0, limit, span);
+          l += softmax_unit<T>(ra, rb, pk, scale, (m_used == -INFINITY) ? 0.f : m_used * scale);
+        } else {
+          if (jh == 0)  // first unit of the item: establish the reference max with a max-only pre-pass
+            m_used = need_mask ? softmax_row_max<true, kWin>(tsh, kv0, limit, span)
+                               : softmax_row_max<false, kWin>(tsh, kv0, limit, span);
+          float m_off = (m_used == -INFINITY) ? 0.f : m_used * scale;
+          float psum = need_mask ? softmax_row_pass<T, true, kWin>(tsh, pk, scale, m_off, kv0, limit, span)
+                                 : softmax_row_pass<T, false, kWin>(tsh, pk, scale, m_off, kv0, limit, span);
+          // raise the reference max only when some row may have outgrown it by > 2^8 (an element
+          // above 2^8 implies a row sum above 2^8; warp-uniform decision: tcgen05.ld/st are
+          // warp-collective); S is still intact (P is stored below), so the unit is simply redone
+          if (__any_sync(0xffffffffu, psum > kRescaleTrigger)) {
+            const float mx = need_mask ? softmax_row_max<true, kWin>(tsh, kv0, limit, span)
+                                       : softmax_row_max<false, kWin>(tsh, kv0, limit, span);
+            const float m_new = fmaxf(m_used, mx);
+            alpha = (m_used == -INFINITY) ? 0.f : fast_exp2((m_used - m_new) * scale);
+            l *= alpha;
+            m_used = m_new;
+            m_off = (m_used == -INFINITY) ? 0.f : m_used * scale;
+            if (jh > 0) rescale_o(alpha, u);
+            psum = need_mask ? softmax_row_pass<T, true, kWin>(tsh, pk, scale, m_off, kv0, limit, span)
+                             : softmax_row_pass<T, false, kWin>(tsh, pk, scale, m_off, kv0, limit, span);
+          }
+          l += psum;
         }
-        float m_off = (m_used == -INFINITY) ? 0.f : m_used * scale;
-        uint32_t pk[kU / 2];
-        float psum = need_mask ? softmax_row_pass<T, true, kWin>(tsh, pk, scale, m_off, kv0, limit, span)
-                               : softmax_row_pass<T, false, kWin>(tsh, pk, scale, m_off, kv0, limit, span);
-        // raise the reference max only when some row may have outgrown it by > 2^8 (an element
-        // above 2^8 implies a row sum above 2^8; warp-uniform decision: tcgen05.ld/st are
-        // warp-collective); S is still intact (P is stored below), so the unit is simply redone
-        if (!kWin && __any_sync(0xffffffffu, psum > kRescaleTrigger)) {
-          const float mx = need_mask ? softmax_row_max<true, kWin>(tsh, kv0, limit, span)
-                                     : softmax_row_max<false, kWin>(tsh, kv0, limit, span);
-          const float m_new = fmaxf(m_used, mx);
-          const float alpha = (m_used == -INFINITY) ? 0.f : fast_exp2((m_used - m_new) * scale);
-          l *= alpha;
-          m_used = m_new;
-          m_off = (m_used == -INFINITY) ? 0.f : m_used * scale;
-          if (jh > 0) rescale_o(alpha, u);
-          psum = need_mask ? softmax_row_pass<T, true, kWin>(tsh, pk, scale, m_off, kv0, limit, span)
-                           : softmax_row_pass<T, false, kWin>(tsh, pk, scale, m_off, kv0, limit, span);
-        }
-        l += psum;
         // P over the first kU/2 columns of this S unit (every column of it is in registers by now)
         tmem_st_32x32b_x32(tsh, pk);
+        if (kWin && raise) rescale_o(alpha, u);
         tmem_st_wait();
         tc_fence_before_sync();
         __syncwarp();
@@ -986,11 +818,11 @@ static int pf_setup(PrefillParams& p, CUtensorMap& tq, CUtensorMap& tk, CUtensor
   return 0;
 }
 
-// A list of the row tiles by weight serves where some CTA gets more than one item; it holds kPfList tiles, named by 16 bits
+// A list of the row tiles by weight serves where some CTA gets more than one item; it holds kTileList tiles, named by 16 bits
 // (kv lengths below 2^23, so that a weight fits the key's other half).
 static int pf_wants_list(const PrefillParams& p, int64_t total_tokens, int grid) {
   const int64_t rows = p.pair_heads ? kPfM : 2 * kPfM;
-  return p.total_items > grid && total_tokens / rows + p.batch <= kPfList &&
+  return p.total_items > grid && total_tokens / rows + p.batch <= kTileList &&
                  static_cast<int64_t>(p.batch) * p.tiles_x <= 65536 && p.rtt_stride < (1 << 23)
              ? 1
              : 0;
@@ -1004,8 +836,8 @@ int attn_prefill_window_try(void* out, const void* q, const void* k_pool, const 
                             int H, int G, int64_t q_stride, int64_t out_stride, int64_t r2t_stride, float sm_scale,
                             int window, const float* sinks, float qtemp_coef, int qtemp_every, int dtype, int sm_budget,
                             cudaStream_t stream) {
-  // a reference max of raw scores serves the scaled ones only where the scale is not negative
-  if (!(sm_scale >= 0.f) || !(qtemp_every <= 0 || qtemp_coef >= 0.f)) return 1;
+  // a max of raw scores serves the scaled ones only where the scale is positive
+  if (!(sm_scale > 0.f) || !(qtemp_every <= 0 || qtemp_coef >= 0.f)) return 1;
   if (q_stride % 8 != 0 || out_stride % 8 != 0 || !aligned16(out) || !aligned16(q) || !aligned16(k_pool) || !aligned16(v_pool))
     return 1;
   const int64_t items = (max_extend_len + kPfM - 1) / kPfM * H * batch;

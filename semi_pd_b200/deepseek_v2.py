@@ -4,11 +4,11 @@ names: `DeepseekV2MLP` (:70-111), `MoEGate` (:114-138), `DeepseekV2MoE` (:141-21
 `DeepseekV2ForCausalLM` (:993-1267).  BASELINE configs[3].
 
 What differs from the reference, all on the kernel side:
-  * attention always takes the ABSORBED form (forward_absorb, :633-706): q_nope is multiplied into
-    the latent space (w_kc), one MQA pass over the latent pool (`spd_attn_mla`), and the result
+  * attention takes the ABSORBED form (forward_absorb, :633-706) for decode and small prefill batches: q_nope is
+    multiplied into the latent space (w_kc), one MQA pass over the latent pool (`spd_attn_mla`), and the result
     comes back through w_vc.  The reference uses the plain-MHA form for prefill batches without a
-    cached prefix (:555-561, 591-631) — the same function of the same inputs; one kernel family
-    here serves prefill, chunked prefill and decode.
+    cached prefix (:555-561, 591-631) — the same function of the same inputs; here prefill batches with or without one
+    take it where it is faster (`mla_expanded_pays`, `spd_attn_mla_prefill`).
   * q_proj and kv_a_proj_with_mqa run as ONE GEMM (their weights stacked), the two per-head BMMs
     as one block-diagonal `spd_gemm_grouped` launch each.
   * the routed experts run either as two grouped GEMMs over expert-sorted 128-row tiles
@@ -33,6 +33,32 @@ _FUSED_SILU_MIN_TOKENS = 257
 # batches in [lo, hi] run all experts densely (see module docstring)
 _MOE_DENSE_MIN_TOKENS = 16
 _MOE_DENSE_MAX_TOKENS = 256
+
+
+# The expanded form of MLA prefill keeps K and V of every key while a layer runs: 8 KB per key at 16 heads.
+_MLA_EXPANDED_MAX_KEYS = 32768
+
+
+def mla_expanded_pays(extend_lens, prefix_lens, num_heads: int, sms: int) -> bool:
+    """Whether a prefill batch is faster with K and V of every head made from the latent rows (attn_mla_prefill) than in the
+    absorbed form (attn_mla).  Estimates in us on 148 SMs at 16 heads, from whole layers: absorbed, 0.12 per 1000 pairs of
+    query and key and 13 per 1000 tokens for the two per-head products; expanded, 7 per 1000 keys and 1 per tile of 64 keys
+    of an item of 256 queries, of the longest item or of an SM's share, and 15 of host time.  Measured (absorbed, expanded):
+    1 x 512 tokens 118, 123; 1 x 1024 167, 150; 4 x 1024 behind 512 610, 175; 1 x 128 behind 4000 125, 132; 1 x 256 behind
+    4000 197, 175; 8 x 64, half of them behind 4000, 187, 205; 8 x 128 likewise 316, 226; 1 x 128 behind 16000 273, 372."""
+    keys = sum(extend_lens) + sum(prefix_lens)
+    if keys > _MLA_EXPANDED_MAX_KEYS:
+        return False
+    tokens = sum(extend_lens)
+    pairs = sum(e * p + e * (e + 1) // 2 for e, p in zip(extend_lens, prefix_lens))
+    groups, few = -(-num_heads // 16), 148.0 / max(1, sms)
+    absorbed = (0.12e-3 * pairs * groups + 13e-3 * tokens * num_heads / 16) * few
+    if absorbed < 15:
+        return False
+    longest = max((e + p + 63) // 64 for e, p in zip(extend_lens, prefix_lens))
+    tiles = sum(sum((min(e, i + 256) + p + 63) // 64 for i in range(0, e, 256)) for e, p in zip(extend_lens, prefix_lens))
+    expanded = 7e-3 * keys * num_heads / 16 * few + max(longest, tiles * num_heads / max(1, sms)) + 15
+    return expanded < absorbed
 
 
 def yarn_get_mscale(scale: float = 1, mscale: float = 1) -> float:
@@ -175,6 +201,7 @@ class DeepseekV2AttentionMLA:
         self.o_proj = LinearBase(self.num_heads * self.v_head_dim, self.hidden_size)
         self.w_kc_t: torch.Tensor = None   # [H * kv_lora, nope]: head h = rows [h*kv_lora, ...) = W_kc[h]^T
         self.w_vc: torch.Tensor = None     # [H * v_head_dim, kv_lora]
+        self.w_kv_b: torch.Tensor = None   # [H * (nope + v_head_dim), kv_lora], as in the checkpoint: the expanded form
         self.cos_sin_cache = deepseek_cos_sin_cache(self.qk_rope_head_dim, config.max_position_embeddings,
                                                     config.rope_theta, rs, device)
         # RadixAttention descriptor as the reference builds it for the absorbed form (:478-489):
@@ -188,12 +215,32 @@ class DeepseekV2AttentionMLA:
         w = kv_b.view(H, self.qk_nope_head_dim + self.v_head_dim, R)
         self.w_kc_t = w[:, : self.qk_nope_head_dim, :].transpose(1, 2).contiguous().view(H * R, self.qk_nope_head_dim)
         self.w_vc = w[:, self.qk_nope_head_dim:, :].contiguous().view(H * self.v_head_dim, R)
+        self.w_kv_b = w.contiguous().view(H * (self.qk_nope_head_dim + self.v_head_dim), R)
+
+    def expands(self, forward_batch: ForwardBatch) -> bool:
+        """Whether this batch takes the expanded form (forward_normal); decided once per batch."""
+        if (forward_batch.forward_mode.is_decode() or self.w_kv_b is None or forward_batch.extend_seq_lens_cpu is None
+                or forward_batch.extend_prefix_lens_cpu is None
+                or (self.qk_nope_head_dim, self.qk_rope_head_dim, self.v_head_dim, self.kv_lora_rank) != (128, 64, 128, 512)):
+            return False
+        if forward_batch.mla_expanded is None:
+            forward_batch.mla_expanded = mla_expanded_pays(forward_batch.extend_seq_lens_cpu, forward_batch.extend_prefix_lens_cpu,
+                                                           self.num_heads, ops.get_sm_budget() or ops.device_sm_count(0))
+        return forward_batch.mla_expanded
 
     def forward(self, positions: torch.Tensor, hidden_states: torch.Tensor, forward_batch: ForwardBatch):
         T = hidden_states.shape[0]
         H, DL, R = self.num_heads, self.latent_dim, self.kv_lora_rank
         qa = ops.linear(hidden_states, self.q_kv_a_proj.weight)          # [T, H*192 + 576]
         q = qa[:, : self.q_size]
+        if self.expands(forward_batch):
+            ops.mla_rotary_store_inplace(qa, forward_batch.token_to_kv_pool.get_key_buffer(self.layer_id), positions,
+                                         forward_batch.out_cache_loc, self.kv_a_layernorm.weight, self.cos_sin_cache, H,
+                                         self.qk_nope_head_dim, R, self.qk_rope_head_dim,
+                                         self.kv_a_layernorm.variance_epsilon)
+            attn_out = forward_batch.attn_backend.forward_mla_expanded(q, self.w_kv_b, self.attn_mqa, self.qk_nope_head_dim,
+                                                                       self.v_head_dim, forward_batch)
+            return ops.linear(attn_out, self.o_proj.weight)
         # latent row (RMSNorm on the kv_lora part, interleaved RoPE on the rope part) into its pool slot, and every head's
         # rotated q_pe behind its absorbed query [q_nope W_kc || q_pe]
         pool = forward_batch.token_to_kv_pool

@@ -118,6 +118,7 @@ class ForwardBatch:
     extend_prefix_lens_cpu: Optional[List[int]] = None
     extend_seq_lens_cpu: Optional[List[int]] = None
     extend_logprob_start_lens_cpu: Optional[List[int]] = None
+    mla_expanded: Optional[bool] = None  # MLA prefill with expanded heads, decided by the first layer
 
     sampling_info: object = None
 

@@ -440,29 +440,96 @@ def mla_rotary_store(qa: torch.Tensor, q_lat: torch.Tensor, kv_pool: torch.Tenso
     """qa [T, H (nope + rope) + kv_lora + rope], the fused projection: kv_pool[loc[t]] = normed latent || rotated rope part;
     q_lat [T, H (kv_lora + rope)] gets every head's rotated rope part (its kv_lora columns are the caller's)."""
     _cuda(qa, q_lat, kv_pool, positions, loc, norm_weight, cos_sin_cache)
-    if cos_sin_cache.dtype != torch.float32 or positions.dtype != torch.int64:
-        raise RuntimeError("mla_rotary_store: cos_sin_cache is float32, positions are int64")
-    if not (qa.dtype == q_lat.dtype == kv_pool.dtype == norm_weight.dtype):
-        raise RuntimeError("mla_rotary_store: qa, q_lat, the pool and the norm weight share a dtype")
     T, DL = qa.shape[0], kv_lora_rank + rope_dim
-    if qa.dim() != 2 or qa.shape[1] != num_heads * (nope_dim + rope_dim) + DL or qa.stride(1) != 1:
-        raise RuntimeError("mla_rotary_store: qa is [T, H (nope + rope) + kv_lora + rope] with contiguous rows")
+    loc = _mla_rotary_args("mla_rotary_store", qa, kv_pool, positions, loc, norm_weight, cos_sin_cache, num_heads, nope_dim,
+                           kv_lora_rank, rope_dim)
+    if q_lat.dtype != qa.dtype:
+        raise RuntimeError("mla_rotary_store: qa, q_lat, the pool and the norm weight share a dtype")
     if tuple(q_lat.shape) != (T, num_heads * DL) or (T and q_lat.stride(1) != 1):
         raise RuntimeError("mla_rotary_store: q_lat is [T, H (kv_lora + rope)] with contiguous rows")
-    if kv_pool.shape[-1] != DL or not kv_pool.is_contiguous() or kv_pool.numel() != kv_pool.shape[0] * DL:
-        raise RuntimeError("mla_rotary_store: the pool is contiguous rows of kv_lora + rope")
-    if any(tuple(t.shape) != (T,) or not t.is_contiguous() for t in (positions, loc)):
-        raise RuntimeError("mla_rotary_store: one position and one slot per row of qa, contiguous")
-    if tuple(norm_weight.shape) != (kv_lora_rank,) or not norm_weight.is_contiguous():
-        raise RuntimeError("mla_rotary_store: the norm weight is [kv_lora], contiguous")
-    if cos_sin_cache.dim() != 2 or cos_sin_cache.shape[1] != rope_dim or not cos_sin_cache.is_contiguous():
-        raise RuntimeError("mla_rotary_store: cos_sin_cache is [positions, rope], contiguous")
-    if loc.dtype != torch.int64:
-        loc = loc.long()
     check(lib.spd_mla_rotary_store(q_lat.data_ptr(), qa.data_ptr(), kv_pool.data_ptr(), norm_weight.data_ptr(),
                                    cos_sin_cache.data_ptr(), positions.data_ptr(), loc.data_ptr(), T, num_heads,
                                    nope_dim, kv_lora_rank, rope_dim, qa.stride(0), q_lat.stride(0), float(eps), _dt(qa),
                                    _stream()), "spd_mla_rotary_store")
+
+
+def _mla_rotary_args(fn: str, qa, kv_pool, positions, loc, norm_weight, cos_sin_cache, num_heads: int, nope_dim: int,
+                     kv_lora_rank: int, rope_dim: int) -> torch.Tensor:
+    """Shapes and strides that the kernel relies on; → loc as int64."""
+    if cos_sin_cache.dtype != torch.float32 or positions.dtype != torch.int64:
+        raise RuntimeError(f"{fn}: cos_sin_cache is float32, positions are int64")
+    if not (qa.dtype == kv_pool.dtype == norm_weight.dtype):
+        raise RuntimeError(f"{fn}: qa, the pool and the norm weight share a dtype")
+    T, DL = qa.shape[0], kv_lora_rank + rope_dim
+    if qa.dim() != 2 or qa.shape[1] != num_heads * (nope_dim + rope_dim) + DL or qa.stride(1) != 1:
+        raise RuntimeError(f"{fn}: qa is [T, H (nope + rope) + kv_lora + rope] with contiguous rows")
+    if kv_pool.shape[-1] != DL or not kv_pool.is_contiguous() or kv_pool.numel() != kv_pool.shape[0] * DL:
+        raise RuntimeError(f"{fn}: the pool is contiguous rows of kv_lora + rope")
+    if any(tuple(t.shape) != (T,) or not t.is_contiguous() for t in (positions, loc)):
+        raise RuntimeError(f"{fn}: one position and one slot per row of qa, contiguous")
+    if tuple(norm_weight.shape) != (kv_lora_rank,) or not norm_weight.is_contiguous():
+        raise RuntimeError(f"{fn}: the norm weight is [kv_lora], contiguous")
+    if cos_sin_cache.dim() != 2 or cos_sin_cache.shape[1] != rope_dim or not cos_sin_cache.is_contiguous():
+        raise RuntimeError(f"{fn}: cos_sin_cache is [positions, rope], contiguous")
+    return loc if loc.dtype == torch.int64 else loc.long()
+
+
+def mla_rotary_store_inplace(qa: torch.Tensor, kv_pool: torch.Tensor, positions: torch.Tensor, loc: torch.Tensor,
+                             norm_weight: torch.Tensor, cos_sin_cache: torch.Tensor, num_heads: int, nope_dim: int,
+                             kv_lora_rank: int, rope_dim: int, eps: float) -> None:
+    """mla_rotary_store with the heads' rotated parts left where they were in qa (the queries of attn_mla_prefill)."""
+    _cuda(qa, kv_pool, positions, loc, norm_weight, cos_sin_cache)
+    loc = _mla_rotary_args("mla_rotary_store_inplace", qa, kv_pool, positions, loc, norm_weight, cos_sin_cache, num_heads,
+                           nope_dim, kv_lora_rank, rope_dim)
+    check(lib.spd_mla_rotary_store_inplace(qa.data_ptr(), kv_pool.data_ptr(), norm_weight.data_ptr(),
+                                           cos_sin_cache.data_ptr(), positions.data_ptr(), loc.data_ptr(), qa.shape[0],
+                                           num_heads, nope_dim, kv_lora_rank, rope_dim, qa.stride(0), float(eps), _dt(qa),
+                                           _stream()), "spd_mla_rotary_store_inplace")
+
+
+def mla_gather(kv_pool: torch.Tensor, req_to_token: torch.Tensor, req_pool_indices: torch.Tensor, prefix_lens: torch.Tensor,
+               extend_lens: torch.Tensor, total_kv: int, max_kv_len: int, kv_lora_rank: int, rope_dim: int):
+    """The latent rows of every request's prefix_lens + extend_lens keys, one request after another.
+    → (rows [total_kv, kv_lora + rope], first row of every request int32)."""
+    _cuda(kv_pool, req_to_token, req_pool_indices, prefix_lens, extend_lens)
+    DL, B = kv_lora_rank + rope_dim, req_pool_indices.numel()
+    if kv_pool.shape[-1] != DL or not kv_pool.is_contiguous() or kv_pool.numel() != kv_pool.shape[0] * DL:
+        raise RuntimeError("mla_gather: the pool is contiguous rows of kv_lora + rope")
+    if any(t.numel() != B or t.dtype != torch.int32 or not t.is_contiguous() for t in (prefix_lens, extend_lens)):
+        raise RuntimeError("mla_gather: prefix_lens and extend_lens are int32, one per request")
+    rows = torch.empty((total_kv, DL), device=kv_pool.device, dtype=kv_pool.dtype)
+    start = torch.empty((B,), device=kv_pool.device, dtype=torch.int32)
+    check(lib.spd_mla_gather(rows.data_ptr(), start.data_ptr(), kv_pool.data_ptr(), req_to_token.data_ptr(),
+                             req_pool_indices.data_ptr(), prefix_lens.data_ptr(), extend_lens.data_ptr(), B, total_kv,
+                             max_kv_len, kv_lora_rank, rope_dim, req_to_token.stride(0), _dt(kv_pool), _stream()),
+          "spd_mla_gather")
+    return rows, start
+
+
+def attn_mla_prefill(q: torch.Tensor, kv: torch.Tensor, rows: torch.Tensor, kv_start: torch.Tensor,
+                     prefix_lens: torch.Tensor, extend_lens: torch.Tensor, extend_start_loc: torch.Tensor,
+                     max_extend_len: int, max_kv_len: int, num_heads: int, nope_dim: int, rope_dim: int, v_dim: int,
+                     sm_scale: float) -> torch.Tensor:
+    """MLA ragged extend with expanded heads: q [T, H (nope + rope)] (row-strided), kv [rows, H (nope + v)], rows and
+    kv_start as mla_gather gives them → [T, H v]."""
+    _cuda(q, kv, rows, kv_start, prefix_lens, extend_lens, extend_start_loc)
+    T, B = q.shape[0], kv_start.numel()
+    if q.dim() != 2 or q.shape[1] != num_heads * (nope_dim + rope_dim) or q.stride(1) != 1:
+        raise RuntimeError("attn_mla_prefill: q is [T, H (nope + rope)] with contiguous rows")
+    if tuple(kv.shape) != (rows.shape[0], num_heads * (nope_dim + v_dim)) or not kv.is_contiguous() or not rows.is_contiguous():
+        raise RuntimeError("attn_mla_prefill: kv is [rows, H (nope + v)], kv and rows contiguous")
+    if not (q.dtype == kv.dtype == rows.dtype):
+        raise RuntimeError("attn_mla_prefill: q, kv and rows share a dtype")
+    if any(t.numel() != B or t.dtype != torch.int32 or not t.is_contiguous()
+           for t in (kv_start, prefix_lens, extend_lens, extend_start_loc)):
+        raise RuntimeError("attn_mla_prefill: kv_start, prefix_lens, extend_lens and extend_start_loc are int32, one per request")
+    out = torch.empty((T, num_heads * v_dim), device=q.device, dtype=q.dtype)
+    check(lib.spd_attn_mla_prefill(out.data_ptr(), q.data_ptr(), kv.data_ptr(), rows.data_ptr(), kv_start.data_ptr(),
+                                   prefix_lens.data_ptr(), extend_lens.data_ptr(), extend_start_loc.data_ptr(), B, T,
+                                   rows.shape[0], max_extend_len, max_kv_len, num_heads, nope_dim, rope_dim, v_dim,
+                                   q.stride(0), out.stride(0), float(sm_scale), _dt(q), get_sm_budget(), _stream()),
+          "spd_attn_mla_prefill")
+    return out
 
 
 def attn_mla(q: torch.Tensor, kv_pool: torch.Tensor, req_to_token, req_pool_indices, num_heads: int,
