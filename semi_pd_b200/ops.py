@@ -8,6 +8,7 @@ torch is plumbing here (device memory + streams); every computation runs in libs
 """
 from __future__ import annotations
 
+import contextlib
 import os
 from typing import Optional
 
@@ -302,13 +303,30 @@ def write_req_to_token_pool(req_to_token: torch.Tensor, req_pool_indices: torch.
 _gemm_ws = {}
 
 
+def new_gemm_workspace(device) -> torch.Tensor:
+    return torch.zeros((lib.spd_gemm_workspace_bytes(),), dtype=torch.uint8, device=device)
+
+
+@contextlib.contextmanager
+def gemm_workspace(ws: torch.Tensor):
+    """This thread's GEMMs on ws.device use `ws` (zeroed once; one stream at a time) instead of their stream's."""
+    before = getattr(_tls, "gemm_ws", None)
+    _tls.gemm_ws = ws
+    try:
+        yield
+    finally:
+        _tls.gemm_ws = before
+
+
 def _gemm_workspace(device: torch.device) -> torch.Tensor:
     """Split-K scratch, one per (device, stream) so the prefill and decode workers never share it."""
+    own = getattr(_tls, "gemm_ws", None)
+    if own is not None and own.device == device:
+        return own
     key = (device.index, _stream())
     ws = _gemm_ws.get(key)
     if ws is None:
-        ws = torch.zeros((lib.spd_gemm_workspace_bytes(),), dtype=torch.uint8, device=device)
-        _gemm_ws[key] = ws
+        ws = _gemm_ws[key] = new_gemm_workspace(device)
     return ws
 
 
