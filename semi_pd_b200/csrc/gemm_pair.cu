@@ -1,7 +1,7 @@
 // Prefill-regime GEMM on CTA PAIRS: C[M,N] = A[M,K] * W[N,K]^T with tcgen05.mma.cta_group::2.
 //
-// Two CTAs on the two SMs of one TPC (cluster of 2) own one 256 x 256 output tile.  CTA r holds
-// the A rows [r*128, r*128+128) of the tile and HALF of the W tile (128 of its 256 rows); one
+// Two CTAs on the two SMs of one TPC (cluster of 2) own one 256 x BN output tile (BN = 256, see pair_tile_cols for the
+// others).  CTA r holds the A rows [r*128, r*128+128) of the tile and HALF of the W tile (128 of its 256 rows); one
 // UMMA of shape M=256, N=256, K=16 issued by the leader CTA reads both CTAs' shared memory and
 // writes each CTA's 128 x 256 fp32 accumulator into that CTA's own TMEM.  Against the single-CTA
 // 128 x 256 tile (gemm.cu) every CTA stages 32 KB instead of 48 KB per k-block and the tensor
@@ -31,12 +31,16 @@ namespace spd {
 
 constexpr int kPgThreads = 256;
 constexpr int kPgBM = 128;   // rows per CTA (pair tile = 256)
-constexpr int kPgBN = 256;
+constexpr int kPgBN = 256;   // the widest tile
 constexpr int kPgBK = 64;
-constexpr int kPgStages = 6;
-constexpr int kPgABytes = kPgBM * kPgBK * 2;        // 16 KB
-constexpr int kPgBBytes = (kPgBN / 2) * kPgBK * 2;  // 16 KB: this CTA's half of the W tile
-constexpr int kPgSmemBytes = kPgStages * (kPgABytes + kPgBBytes) + 1024 + 256;
+constexpr int kPgABytes = kPgBM * kPgBK * 2;  // 16 KB
+template <int BN>
+struct PairShape {
+  static constexpr int kBBytes = (BN / 2) * kPgBK * 2;  // this CTA's half of the W tile
+  static constexpr int kStages = BN >= 224 ? 6 : 7;
+  static constexpr int kSmem = kStages * (kPgABytes + kBBytes) + 1024 + 256;
+  static_assert(BN % 32 == 0 && kSmem <= 232448, "tile shape");
+};
 
 struct PairGemmParams {
   void* C;
@@ -104,24 +108,27 @@ __device__ __forceinline__ void umma_commit_2cta_mc(uint64_t* bar, uint16_t mask
       : "memory");
 }
 
-template <typename T, int kEpi>
+template <typename T, int kEpi, int BN>
 __global__ void __launch_bounds__(kPgThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW,
                  const PairGemmParams p) {
-  constexpr int kBNOut = (kEpi == SPD_EPI_SILU_MUL) ? kPgBN / 2 : kPgBN;
-  constexpr int kTmemCols = 2 * kPgBN;  // two accumulator stages
+  constexpr int kStages = PairShape<BN>::kStages, kBBytes = PairShape<BN>::kBBytes;
+  constexpr int kBNOut = (kEpi == SPD_EPI_SILU_MUL) ? BN / 2 : BN;
+  constexpr int kTmemStage = 256;
+  constexpr int kTmemCols = 2 * kTmemStage;  // two accumulator stages
+  static_assert(kBNOut % 32 == 0, "the epilogue goes by 32 columns");
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
   uint8_t* sA = smem;
-  uint8_t* sB = smem + kPgStages * kPgABytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kPgStages * (kPgABytes + kPgBBytes));
-  uint64_t* full = bars;                        // [kPgStages]  (leader's are the live ones)
-  uint64_t* empty = bars + kPgStages;           // [kPgStages]
-  uint64_t* tfull = bars + 2 * kPgStages;       // [2]
-  uint64_t* tempty = bars + 2 * kPgStages + 2;  // [2]          (leader's are the live ones)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kPgStages + 4);
+  uint8_t* sB = smem + kStages * kPgABytes;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kStages * (kPgABytes + kBBytes));
+  uint64_t* full = bars;                        // [kStages]  (leader's are the live ones)
+  uint64_t* empty = bars + kStages;           // [kStages]
+  uint64_t* tfull = bars + 2 * kStages;       // [2]
+  uint64_t* tempty = bars + 2 * kStages + 2;  // [2]          (leader's are the live ones)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kStages + 4);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -135,7 +142,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     tma_prefetch_desc(&tmW);
   }
   if (warp == 1 && lane == 0) {
-    for (int i = 0; i < kPgStages; ++i) {
+    for (int i = 0; i < kStages; ++i) {
       mbar_init(&full[i], 1);
       mbar_init(&empty[i], 1);
     }
@@ -166,38 +173,38 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         const int a_row = xt * (2 * kPgBM) + static_cast<int>(rank) * kPgBM;
         const int w_row = (kEpi == SPD_EPI_SILU_MUL)
                               ? (rank == 0 ? yt * kBNOut : static_cast<int>(p.up_row0) + yt * kBNOut)
-                              : yt * kPgBN + static_cast<int>(rank) * (kPgBN / 2);
+                              : yt * BN + static_cast<int>(rank) * (BN / 2);
         for (int kb = 0; kb < p.kblocks; ++kb) {
           mbar_wait(&empty[stage], phase ^ 1);
-          if (rank == 0) mbar_expect_tx(&full[stage], 2 * (kPgABytes + kPgBBytes));
+          if (rank == 0) mbar_expect_tx(&full[stage], 2 * (kPgABytes + kBBytes));
           const uint32_t lead_full = map_to_rank(smem_u32(&full[stage]), 0);
           tma_load_2d_2cta(sA + stage * kPgABytes, &tmA, lead_full, kb * kPgBK, a_row, kEvictNormal);
-          tma_load_2d_2cta(sB + stage * kPgBBytes, &tmW, lead_full, kb * kPgBK, w_row, kEvictNormal);
-          if (++stage == kPgStages) { stage = 0; phase ^= 1; }
+          tma_load_2d_2cta(sB + stage * kBBytes, &tmW, lead_full, kb * kPgBK, w_row, kEvictNormal);
+          if (++stage == kStages) { stage = 0; phase ^= 1; }
         }
       }
     }
   } else if (warp == 1) {
     if (rank == 0 && elect_one()) {
-      constexpr uint32_t idesc = umma_idesc<T>(2 * kPgBM, kPgBN, 0, 0);
+      constexpr uint32_t idesc = umma_idesc<T>(2 * kPgBM, BN, 0, 0);
       int stage = 0, phase = 0, n = 0;
       for (int tile = pair; tile < num_tiles; tile += npairs) {
         const int as = n & 1, aphase = (n >> 1) & 1;
         ++n;
         mbar_wait_cluster_acquire(&tempty[as], aphase ^ 1);  // both CTAs drained this accumulator
         tc_fence_after_sync();
-        const uint32_t d_tmem = tmem_base + as * kPgBN;
+        const uint32_t d_tmem = tmem_base + as * kTmemStage;
         for (int kb = 0; kb < p.kblocks; ++kb) {
           mbar_wait(&full[stage], phase);
           tc_fence_after_sync();
           const uint32_t aa = smem_u32(sA + stage * kPgABytes);
-          const uint32_t ba = smem_u32(sB + stage * kPgBBytes);
+          const uint32_t ba = smem_u32(sB + stage * kBBytes);
 #pragma unroll
           for (int k = 0; k < kPgBK / 16; ++k)
             umma_ss_2cta(d_tmem, umma_desc_sw128(aa + k * 32, 16, 1024), umma_desc_sw128(ba + k * 32, 16, 1024),
                          idesc, (kb > 0 || k > 0) ? 1u : 0u);
           umma_commit_2cta_mc(&empty[stage], 0b11);  // both CTAs' slots are free once these MMAs are done
-          if (++stage == kPgStages) { stage = 0; phase ^= 1; }
+          if (++stage == kStages) { stage = 0; phase ^= 1; }
         }
         umma_commit_2cta_mc(&tfull[as], 0b11);
       }
@@ -214,7 +221,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       ++n;
       mbar_wait(&tfull[as], aphase);
       tc_fence_after_sync();
-      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + as * kPgBN;
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + as * kTmemStage;
       const int64_t m = static_cast<int64_t>(xt) * (2 * kPgBM) + rank * kPgBM + row;
 #pragma unroll 1
       for (int c = 0; c < kBNOut; c += 32) {
@@ -282,19 +289,19 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   if (warp == 2) tmem_dealloc_2cta(tmem_base, kTmemCols);
 }
 
-template <typename T, int kEpi>
+template <typename T, int kEpi, int BN>
 static int launch_pair_gemm(const CUtensorMap& ta, const CUtensorMap& tw, const PairGemmParams& p, int pairs,
                             cudaStream_t stream) {
-  auto kern = gemm_pair_kernel<T, kEpi>;
+  auto kern = gemm_pair_kernel<T, kEpi, BN>;
   static bool configured = false;
   if (!configured) {
-    SPD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPgSmemBytes));
+    SPD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PairShape<BN>::kSmem));
     configured = true;
   }
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(2 * pairs);
   cfg.blockDim = dim3(kPgThreads);
-  cfg.dynamicSmemBytes = kPgSmemBytes;
+  cfg.dynamicSmemBytes = PairShape<BN>::kSmem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -309,6 +316,25 @@ static int launch_pair_gemm(const CUtensorMap& ta, const CUtensorMap& tw, const 
   return 0;
 }
 
+// Columns of a pair tile: the width whose waves take least.  A wave of BN columns takes about BN + 100 units (a tile's A rows,
+// its beginning and end do not shrink with it), so a narrower tile serves where the widest leaves a last wave nearly empty.
+// 256 / the one chosen, us: 4096 x 14336 weights, M = 700 84.9 / 67.3 (192), 1300 147 / 127 (192); 4096 x 4096, 700 31.1 /
+// 24.9 (192), 1300 49.7 / 41.0 (192); 3648 x 2048, 4096 54.1 / 48.0 (224).  160 and 128 were never the fastest; SiLU tiles
+// (gate and up rows in one) gained nothing from 192.
+static int pair_tile_cols(int64_t N, int64_t x_tiles, int epilogue, int pairs, int64_t* cost) {
+  int best = 0;
+  for (int bn : {256, 224, 192}) {
+    const int64_t n_out = epilogue == SPD_EPI_SILU_MUL ? bn / 2 : bn;
+    const int64_t waves = (x_tiles * ((N + n_out - 1) / n_out) + pairs - 1) / pairs;
+    if (best == 0 || waves * (bn + 100) < *cost) {
+      best = bn;
+      *cost = waves * (bn + 100);
+    }
+    if (epilogue != SPD_EPI_NONE) break;
+  }
+  return best;
+}
+
 // Called by spd_gemm for the prefill regime.  Returns 1 if this path does not apply (the caller
 // falls through to the single-CTA kernel), 0 on launch, else an error code.
 int gemm_pair_try(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_t K, int64_t lda,
@@ -321,12 +347,13 @@ int gemm_pair_try(void* C, const void* A, const void* W, int64_t M, int64_t N, i
   // all waves) that the pair's longer start and end decide.  4096 x 14336 weights: M = 300 87 -> 70 us, 600 87 -> 72,
   // 1300 167 -> 156; 3648 x 2048, M = 600: 15.7 us single, 17.9 pair, 1300: 35 single, 28 pair.
   const int64_t rows_pair = (M + 255) / 256 * 256, rows_single = (M + 127) / 128 * 128;
+  int64_t cost;
+  const int bn = pair_tile_cols(N, rows_pair / 256, epilogue, sms / 2, &cost);
   if (rows_pair != rows_single && M < 2048) {
     const int n_tile = epilogue == SPD_EPI_SILU_MUL ? kPgBN / 2 : kPgBN;
     const int64_t cols = (N + n_tile - 1) / n_tile, kblocks = (K + kPgBK - 1) / kPgBK;
-    const int64_t waves_pair = (rows_pair / 256 * cols + sms / 2 - 1) / (sms / 2);
     const int64_t waves_single = (rows_single / 128 * cols + sms - 1) / sms;
-    if (waves_pair * 9 >= waves_single * 10 || waves_single * kblocks < 48) return 1;
+    if (cost * 9 >= waves_single * (kPgBN + 100) * 10 || waves_single * kblocks < 48) return 1;
   }
   PairGemmParams p{};
   p.C = C;
@@ -337,9 +364,9 @@ int gemm_pair_try(void* C, const void* A, const void* W, int64_t M, int64_t N, i
   p.out_f32 = out_f32;
   p.kblocks = static_cast<int>((K + kPgBK - 1) / kPgBK);
   p.x_tiles = static_cast<int>((M + 255) / 256);
-  const int n_out = epilogue == SPD_EPI_SILU_MUL ? kPgBN / 2 : kPgBN;
+  const int n_out = epilogue == SPD_EPI_SILU_MUL ? bn / 2 : bn;
   p.y_tiles = static_cast<int>((N + n_out - 1) / n_out);
-  const long long tile_bytes = static_cast<long long>(kPgBN) * K * 2;
+  const long long tile_bytes = static_cast<long long>(bn) * K * 2;
   const long long q = (static_cast<long long>(panel_mb) << 20) / tile_bytes;
   p.panel = static_cast<int>(q < 1 ? 1 : q);
   const int total = p.x_tiles * p.y_tiles;
@@ -347,14 +374,15 @@ int gemm_pair_try(void* C, const void* A, const void* W, int64_t M, int64_t N, i
   CUtensorMap ta, tw;
   int rc;
   if ((rc = get_tmap(&ta, A, M, K, lda, kPgBM))) return rc;
-  if ((rc = get_tmap(&tw, W, epilogue == SPD_EPI_SILU_MUL ? 2 * N : N, K, ldw, kPgBN / 2))) return rc;
-  if (epilogue == SPD_EPI_SILU_MUL) {
-    SPD_DISPATCH_DTYPE(dtype, { return launch_pair_gemm<T, SPD_EPI_SILU_MUL>(ta, tw, p, pairs, stream); });
-  } else if (epilogue == SPD_EPI_GELU) {
-    SPD_DISPATCH_DTYPE(dtype, { return launch_pair_gemm<T, SPD_EPI_GELU>(ta, tw, p, pairs, stream); });
-  } else {
-    SPD_DISPATCH_DTYPE(dtype, { return launch_pair_gemm<T, SPD_EPI_NONE>(ta, tw, p, pairs, stream); });
-  }
+  if ((rc = get_tmap(&tw, W, epilogue == SPD_EPI_SILU_MUL ? 2 * N : N, K, ldw, bn / 2))) return rc;
+#define SPD_PAIR(EPI, BN) \
+  if (epilogue == EPI && bn == BN) SPD_DISPATCH_DTYPE(dtype, { return launch_pair_gemm<T, EPI, BN>(ta, tw, p, pairs, stream); })
+  SPD_PAIR(SPD_EPI_SILU_MUL, 256);
+  SPD_PAIR(SPD_EPI_GELU, 256);
+  SPD_PAIR(SPD_EPI_NONE, 256);
+  SPD_PAIR(SPD_EPI_NONE, 224);
+  SPD_PAIR(SPD_EPI_NONE, 192);
+#undef SPD_PAIR
   return 1;
 }
 
