@@ -40,8 +40,8 @@ typedef void* spd_stream_t; /* cudaStream_t */
  * ------------------------------------------------------------------------------------------- */
 int spd_version(void);
 const char* spd_last_error_string(void);
-/* Waits inside spd_attn_mla, spd_attn_mla_prefill and spd_retention_extend are bounded (seconds).  One that runs out sets a word in host memory
- * when its kernel ends; what that kernel wrote is not to be trusted (a recurrent state is kept as it was before the tokens
+/* Waits inside spd_attn_mla, spd_attn_mla_prefill and spd_retention_extend are bounded (seconds).  One that runs out sets a
+ * word in host memory when its kernel ends; what that kernel wrote is not to be trusted (a recurrent state is kept as it was before the tokens
  * the wait stood for), and those calls return SPD_E_TIMEOUT from then on.  spd_wait_status reads the word without
  * synchronising: call it where a kernel's results are known to have arrived.  clear != 0 resets it. */
 int spd_wait_status(int* expired, int clear);
@@ -497,6 +497,17 @@ int spd_retention_extend(float* o, const void* q, const void* k, const void* v, 
                          int v_dim, int64_t q_stride, int64_t k_stride, int64_t v_stride, const float* decay,
                          const float* cos_sin, int rot_dims, int64_t max_positions, float k_scale, int in_act, int dtype,
                          spd_stream_t stream);
+/* The same with a workspace of spd_retention_workspace_bytes (0: none would be used) for the same sizes and sm_budget, not
+ * zeroed, one call at a time: long portions of few requests are then cut into segments that run side by side. */
+int64_t spd_retention_workspace_bytes(int64_t batch, int64_t total_tokens, int num_heads, int head_dim, int v_dim,
+                                      int rot_dims, int in_act, int dtype, int sm_budget);
+int spd_retention_extend_ws(float* o, const void* q, const void* k, const void* v, float* state,
+                            const int64_t* req_pool_indices, const int32_t* prefix_lens, const int32_t* extend_lens,
+                            const int32_t* extend_start_loc, int64_t batch, int64_t total_tokens, int num_heads,
+                            int head_dim, int v_dim, int64_t q_stride, int64_t k_stride, int64_t v_stride,
+                            const float* decay, const float* cos_sin, int rot_dims, int64_t max_positions, float k_scale,
+                            int in_act, int dtype, void* workspace, int64_t workspace_bytes, int sm_budget,
+                            spd_stream_t stream);
 
 /* spd_residual_rmsnorm with a second weight: out2 = the same normed row times (weight_offset + w2)
  * (out2 and w2 both NULL or both given) */

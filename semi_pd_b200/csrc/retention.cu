@@ -212,7 +212,9 @@ int retention_chunked_try(float* o, const void* q, const void* k, const void* v,
                           const int32_t* extend_start_loc, int64_t batch, int H, int dk, int dv, int64_t q_stride,
                           int64_t k_stride, int64_t v_stride, const float* decay, const float* cos_sin, int rot,
                           int64_t max_positions, float k_scale, int in_act, int dtype, int64_t total_tokens,
-                          cudaStream_t stream);
+                          void* workspace, int64_t workspace_bytes, int sms, cudaStream_t stream);
+int64_t retention_chunked_workspace(int64_t batch, int64_t total_tokens, int H, int dk, int dv, int rot, int in_act, int dtype,
+                                    int sms);
 
 template <typename T, int W, int ROWS, bool ASYNC, int TOK>
 int retention_launch(dim3 grid, size_t smem, cudaStream_t stream, float* o, const void* q, const void* k, const void* v,
@@ -289,24 +291,43 @@ int spd_retention(float* o, const void* q, const void* k, const void* v, float* 
   return 0;
 }
 
-int spd_retention_extend(float* o, const void* q, const void* k, const void* v, float* state,
+int64_t spd_retention_workspace_bytes(int64_t batch, int64_t total_tokens, int num_heads, int head_dim, int v_dim,
+                                      int rot_dims, int in_act, int dtype, int sm_budget) {
+  return retention_chunked_workspace(batch, total_tokens, num_heads, head_dim, v_dim, rot_dims, in_act, dtype,
+                                     sm_budget > 0 ? sm_budget : device_sm_count_cached());
+}
+
+int spd_retention_extend_ws(float* o, const void* q, const void* k, const void* v, float* state,
                          const int64_t* req_pool_indices, const int32_t* prefix_lens, const int32_t* extend_lens,
                          const int32_t* extend_start_loc, int64_t batch, int64_t total_tokens, int num_heads, int head_dim,
                          int v_dim, int64_t q_stride, int64_t k_stride, int64_t v_stride, const float* decay,
                          const float* cos_sin, int rot_dims, int64_t max_positions, float k_scale, int in_act, int dtype,
-                         spd_stream_t stream) {
+                         void* workspace,
+                            int64_t workspace_bytes, int sm_budget, spd_stream_t stream) {
   const bool checked = o && q && k && v && state && req_pool_indices && decay && prefix_lens && extend_lens &&
                        extend_start_loc && num_heads > 0 && head_dim > 0 && v_dim > 0 && rot_dims >= 0 &&
                        rot_dims <= head_dim && (rot_dims == 0 || (cos_sin && max_positions > 0)) && batch > 0;
   if (checked) {  // (what is not is reported by the call below)
     const int rc = retention_chunked_try(o, q, k, v, state, req_pool_indices, prefix_lens, extend_lens, extend_start_loc,
                                          batch, num_heads, head_dim, v_dim, q_stride, k_stride, v_stride, decay, cos_sin,
-                                         rot_dims, max_positions, k_scale, in_act, dtype, total_tokens, as_stream(stream));
+                                         rot_dims, max_positions, k_scale, in_act, dtype, total_tokens, workspace, workspace_bytes,
+                                         sm_budget > 0 ? sm_budget : device_sm_count_cached(), as_stream(stream));
     if (rc != 1) return rc;
   }
   return spd_retention(o, q, k, v, state, req_pool_indices, nullptr, nullptr, prefix_lens, extend_lens, extend_start_loc,
                        batch, num_heads, head_dim, v_dim, q_stride, k_stride, v_stride, decay, cos_sin, rot_dims,
                        max_positions, k_scale, in_act, dtype, stream);
+}
+
+int spd_retention_extend(float* o, const void* q, const void* k, const void* v, float* state,
+                         const int64_t* req_pool_indices, const int32_t* prefix_lens, const int32_t* extend_lens,
+                         const int32_t* extend_start_loc, int64_t batch, int64_t total_tokens, int num_heads, int head_dim,
+                         int v_dim, int64_t q_stride, int64_t k_stride, int64_t v_stride, const float* decay,
+                         const float* cos_sin, int rot_dims, int64_t max_positions, float k_scale, int in_act, int dtype,
+                         spd_stream_t stream) {
+  return spd_retention_extend_ws(o, q, k, v, state, req_pool_indices, prefix_lens, extend_lens, extend_start_loc, batch,
+                                 total_tokens, num_heads, head_dim, v_dim, q_stride, k_stride, v_stride, decay, cos_sin,
+                                 rot_dims, max_positions, k_scale, in_act, dtype, nullptr, 0, 0, stream);
 }
 
 }  // extern "C"

@@ -1129,12 +1129,15 @@ def retention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.Te
         raise RuntimeError("retention: q / k / v need contiguous rows and one dtype")
     o = torch.empty((T, num_heads * v_dim), device=q.device, dtype=torch.float32)
     if seq_lens is None:
-        check(lib.spd_retention_extend(o.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), state.data_ptr(),
-                                       req_pool_indices.data_ptr(), _ptr(prefix_lens), _ptr(extend_lens),
-                                       _ptr(extend_start_loc), req_pool_indices.numel(), T, num_heads, head_dim, v_dim,
-                                       q.stride(0), k.stride(0), v.stride(0), decay.data_ptr(), _ptr(cos_sin),
-                                       int(rot_dims), cos_sin.shape[0] if cos_sin is not None else 0, float(k_scale),
-                                       {None: 0, "silu": 1}[in_act], _dta(q), _stream()), "spd_retention")
+        act, B = {None: 0, "silu": 1}[in_act], req_pool_indices.numel()
+        room = lib.spd_retention_workspace_bytes(B, T, num_heads, head_dim, v_dim, int(rot_dims), act, _dta(q), get_sm_budget())
+        ws = torch.empty((room,), device=q.device, dtype=torch.uint8) if room > 0 else None
+        check(lib.spd_retention_extend_ws(o.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), state.data_ptr(),
+                                          req_pool_indices.data_ptr(), _ptr(prefix_lens), _ptr(extend_lens),
+                                          _ptr(extend_start_loc), B, T, num_heads, head_dim, v_dim, q.stride(0), k.stride(0),
+                                          v.stride(0), decay.data_ptr(), _ptr(cos_sin), int(rot_dims),
+                                          cos_sin.shape[0] if cos_sin is not None else 0, float(k_scale), act, _dta(q),
+                                          _ptr(ws), room, get_sm_budget(), _stream()), "spd_retention")
         return o
     check(lib.spd_retention(o.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), state.data_ptr(),
                             req_pool_indices.data_ptr(), _ptr(seq_lens), _ptr(out_cache_loc), _ptr(prefix_lens),
