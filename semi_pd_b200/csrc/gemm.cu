@@ -34,6 +34,7 @@
 
 #include "common.cuh"
 #include "ptx.cuh"
+#include "row_stage.cuh"
 #include "tmap.cuh"
 
 namespace spd {
@@ -89,9 +90,9 @@ __host__ __device__ constexpr int gemm_stages() {
   return (kSmemBudget / gemm_stage_bytes<BN>()) < kMaxStages ? (kSmemBudget / gemm_stage_bytes<BN>())
                                                              : kMaxStages;
 }
-template <int BN>
+template <int BN, bool kSwap>
 __host__ __device__ constexpr int gemm_smem_bytes() {
-  return gemm_stages<BN>() * gemm_stage_bytes<BN>() + 1024 /*align*/ + 256 /*barriers*/;
+  return gemm_stages<BN>() * gemm_stage_bytes<BN>() + (kSwap ? 0 : 4 * kStageWarp) + 1024 /*align*/ + 256 /*barriers*/;
 }
 
 // Tile index -> (x tile, y tile).  Tiles are walked panel by panel: a panel is `panel` consecutive
@@ -177,7 +178,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
                                              ~static_cast<uintptr_t>(1023));
   uint8_t* sX = smem;
   uint8_t* sY = smem + kStages * kXBytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kStages * (kXBytes + kYBytes));
+  uint8_t* sOut = smem + kStages * (kXBytes + kYBytes);  // !kSwap: kStageWarp per epilogue warp
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sOut + (kSwap ? 0 : 4 * kStageWarp));
   uint64_t* full = bars;                     // [kStages]
   uint64_t* empty = bars + kStages;          // [kStages]
   uint64_t* tfull = bars + 2 * kStages;      // [2]
@@ -313,16 +315,20 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
     const int n_cols = kSwap ? static_cast<int>(((p.y_rows + kChunk - 1) / kChunk) * kChunk) : BN;
     const int cols_used = n_cols < BN ? n_cols : BN;
 
+    // column of C where column c of y tile yt lands
+    auto out_col = [&](int yt, int c) -> int64_t {
+      if (p.c_group_cols > 0) {  // cols mode with strided output groups
+        const int g = yt / p.y_tiles_per_group;
+        return g * p.c_group_cols + static_cast<int64_t>(yt - g * p.y_tiles_per_group) * kBNOut + c;
+      }
+      return static_cast<int64_t>(yt) * kBNOut + c;
+    };
     // v[0..kChunk) of output chunk c of tile (xt, yt) -> C
     auto store_chunk = [&](int xt, int yt, int c, const float* v) {
       if constexpr (!kSwap) {
         const int64_t m = static_cast<int64_t>(xt) * kBM + row;
         const int64_t nl = static_cast<int64_t>(yt) * kBNOut + c;  // logical column: bounds; n0: where it lands
-        int64_t n0 = nl;
-        if (p.c_group_cols > 0) {  // cols mode with strided output groups
-          const int g = yt / p.y_tiles_per_group;
-          n0 = g * p.c_group_cols + static_cast<int64_t>(yt - g * p.y_tiles_per_group) * kBNOut + c;
-        }
+        const int64_t n0 = out_col(yt, c);
         if (m < p.x_rows) {
           if (p.out_f32) {
             float* dst = reinterpret_cast<float*>(p.C) + m * p.ldc + n0;
@@ -424,9 +430,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
         continue;
       }
 
-#pragma unroll 1
-      for (int c = 0; c < (kSwap ? cols_used : kBNOut); c += kChunk) {
-        float v[kChunk];
+      auto values = [&](int c, float (&v)[kChunk]) {
         uint32_t r[kChunk];
         if constexpr (kChunk == 32) tmem_ld_32x32b_x32(taddr + c, r);
         else tmem_ld_32x32b_x16(taddr + c, r);
@@ -447,7 +451,37 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
           for (int j = 0; j < kChunk; ++j)
             v[j] = kEpi == SPD_EPI_GELU ? gelu_fast_f32(to_f32<T>(from_f32<T>(__uint_as_float(r[j])))) : __uint_as_float(r[j]);
         }
-        store_chunk(xt, yt, c, v);
+      };
+      if constexpr (kSwap) {
+#pragma unroll 1
+        for (int c = 0; c < cols_used; c += kChunk) {
+          float v[kChunk];
+          values(c, v);
+          store_chunk(xt, yt, c, v);
+        }
+      } else {
+        static_assert(kBNOut % 64 == 0 && kChunk == 32, "rows are staged by 64 columns");
+        uint8_t* stage = sOut + q * kStageWarp;
+        const int64_t m0 = static_cast<int64_t>(xt) * kBM + q * 32;
+        const int rows = static_cast<int>(min(static_cast<int64_t>(32), p.x_rows - m0));
+        const int step = p.out_f32 ? 32 : 64;
+#pragma unroll 1
+        for (int c = 0; c < kBNOut; c += step) {
+          const int64_t nl = static_cast<int64_t>(yt) * kBNOut + c;
+          const int64_t n0 = out_col(yt, c);
+          const int cols = static_cast<int>(min(static_cast<int64_t>(step), p.y_rows - nl));
+          float v[kChunk];
+          values(c, v);
+          if (p.out_f32) {
+            stage_put32<T>(stage, lane, v, p.out_f32);
+            stage_out(stage, lane, reinterpret_cast<uint8_t*>(p.C) + (m0 * p.ldc + n0) * 4, p.ldc * 4, rows, cols * 4);
+          } else {
+            stage_put16<T>(stage, lane, 0, v);
+            values(c + 32, v);
+            stage_put16<T>(stage, lane, 1, v);
+            stage_out(stage, lane, reinterpret_cast<uint8_t*>(p.C) + (m0 * p.ldc + n0) * 2, p.ldc * 2, rows, cols * 2);
+          }
+        }
       }
       tc_fence_before_sync();
       __syncwarp();
@@ -591,10 +625,10 @@ static int launch_gemm(const CUtensorMap& tx, const CUtensorMap& ty, const GemmP
   static bool configured = false;  // per instantiation
   if (!configured) {
     SPD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  gemm_smem_bytes<BN>()));
+                                  gemm_smem_bytes<BN, kSwap>()));
     configured = true;
   }
-  SPD_CUDA(launch(kern, dim3(grid), dim3(kGemmThreads), gemm_smem_bytes<BN>(), stream,
+  SPD_CUDA(launch(kern, dim3(grid), dim3(kGemmThreads), gemm_smem_bytes<BN, kSwap>(), stream,
                   pdl_enabled(), tx, ty, p));
   return 0;
 }

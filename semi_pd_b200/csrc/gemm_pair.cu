@@ -25,6 +25,7 @@
 
 #include "common.cuh"
 #include "ptx.cuh"
+#include "row_stage.cuh"
 #include "tmap.cuh"
 
 namespace spd {
@@ -38,7 +39,7 @@ template <int BN>
 struct PairShape {
   static constexpr int kBBytes = (BN / 2) * kPgBK * 2;  // this CTA's half of the W tile
   static constexpr int kStages = BN >= 224 ? 6 : 7;
-  static constexpr int kSmem = kStages * (kPgABytes + kBBytes) + 1024 + 256;
+  static constexpr int kSmem = kStages * (kPgABytes + kBBytes) + 4 * kStageWarp + 1024 + 256;
   static_assert(BN % 32 == 0 && kSmem <= 232448, "tile shape");
 };
 
@@ -123,7 +124,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                                              ~static_cast<uintptr_t>(1023));
   uint8_t* sA = smem;
   uint8_t* sB = smem + kStages * kPgABytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kStages * (kPgABytes + kBBytes));
+  uint8_t* sOut = smem + kStages * (kPgABytes + kBBytes);  // kStageWarp per epilogue warp
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sOut + 4 * kStageWarp);
   uint64_t* full = bars;                        // [kStages]  (leader's are the live ones)
   uint64_t* empty = bars + kStages;           // [kStages]
   uint64_t* tfull = bars + 2 * kStages;       // [2]
@@ -211,7 +213,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
   } else if (warp >= 4) {
     const int q = warp & 3;
-    const int row = q * 32 + lane;
+    uint8_t* stage = sOut + q * kStageWarp;
     const uint32_t lead_tempty0 = map_to_rank(smem_u32(&tempty[0]), 0);
     int n = 0;
     for (int tile = pair; tile < num_tiles; tile += npairs) {
@@ -222,11 +224,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       mbar_wait(&tfull[as], aphase);
       tc_fence_after_sync();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + as * kTmemStage;
-      const int64_t m = static_cast<int64_t>(xt) * (2 * kPgBM) + rank * kPgBM + row;
-#pragma unroll 1
-      for (int c = 0; c < kBNOut; c += 32) {
+      const int64_t m0 = static_cast<int64_t>(xt) * (2 * kPgBM) + rank * kPgBM + q * 32;
+      const int rows = static_cast<int>(min(static_cast<int64_t>(32), p.m_rows - m0));
+      auto values = [&](int c, float (&v)[32]) {
         uint32_t r[32];
-        float v[32];
         tmem_ld_32x32b_x32(taddr + c, r);
         if constexpr (kEpi == SPD_EPI_SILU_MUL) {
           uint32_t u[32];
@@ -245,35 +246,24 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           for (int j = 0; j < 32; ++j)
             v[j] = kEpi == SPD_EPI_GELU ? gelu_fast_f32(to_f32<T>(from_f32<T>(__uint_as_float(r[j])))) : __uint_as_float(r[j]);
         }
+      };
+      const int step = p.out_f32 ? 32 : 64;
+#pragma unroll 1
+      for (int c = 0; c < kBNOut; c += step) {
         const int64_t n0 = static_cast<int64_t>(yt) * kBNOut + c;
-        if (m < p.m_rows) {
-          if (p.out_f32) {
-            float* dst = reinterpret_cast<float*>(p.C) + m * p.ldc + n0;
-#pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-              if (n0 + j < p.n_cols) {
-                float4 o;
-                o.x = f32_result<T>(v[j], p.out_f32);
-                o.y = f32_result<T>(v[j + 1], p.out_f32);
-                o.z = f32_result<T>(v[j + 2], p.out_f32);
-                o.w = f32_result<T>(v[j + 3], p.out_f32);
-                *reinterpret_cast<float4*>(dst + j) = o;
-              }
-            }
-          } else {
-            T* dst = reinterpret_cast<T*>(p.C) + m * p.ldc + n0;
-#pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-              if (n0 + j < p.n_cols) {
-                uint4 o;
-                o.x = pack2<T>(v[j], v[j + 1]);
-                o.y = pack2<T>(v[j + 2], v[j + 3]);
-                o.z = pack2<T>(v[j + 4], v[j + 5]);
-                o.w = pack2<T>(v[j + 6], v[j + 7]);
-                *reinterpret_cast<uint4*>(dst + j) = o;
-              }
-            }
+        const int cols = static_cast<int>(min(static_cast<int64_t>(min(step, kBNOut - c)), p.n_cols - n0));
+        float v[32];
+        values(c, v);
+        if (p.out_f32) {
+          stage_put32<T>(stage, lane, v, p.out_f32);
+          stage_out(stage, lane, reinterpret_cast<uint8_t*>(p.C) + (m0 * p.ldc + n0) * 4, p.ldc * 4, rows, cols * 4);
+        } else {
+          stage_put16<T>(stage, lane, 0, v);
+          if (c + 32 < kBNOut) {
+            values(c + 32, v);
+            stage_put16<T>(stage, lane, 1, v);
           }
+          stage_out(stage, lane, reinterpret_cast<uint8_t*>(p.C) + (m0 * p.ldc + n0) * 2, p.ldc * 2, rows, cols * 2);
         }
       }
       tc_fence_before_sync();
