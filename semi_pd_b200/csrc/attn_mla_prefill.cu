@@ -6,7 +6,7 @@
 // prefill batches without a cached prefix; here it serves prefixes as well, as long as a latent row is met by enough
 // queries to pay for its expansion.  The absorbed form (attn_mla.cu) needs 1088 multiply-adds per query, key and head and
 // this one 320, plus 131072 per key and head.  4096 new tokens in 4 requests, two of them behind 515 cached tokens, 16
-// heads, whole attention layer: 606 us absorbed, 180 here (this kernel 68, the rows 5 - 10, the GEMM 31).
+// heads, whole attention layer: 606 us absorbed, 166 here (this kernel 67, the rows 6, the GEMM 26).
 //
 // Items are two consecutive 128-query tiles of one head that share every K / V tile of 64 keys, one tile per softmax
 // warpgroup; they are dealt to one persistent CTA per SM by weight (tile_list).  Roles as in attn_prefill.cu (384 threads):
@@ -489,8 +489,10 @@ attn_mla_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   if (warp == 10) tmem_dealloc(tmem_S, 512);
 }
 
-// The latent rows of every request's keys, one request after another, and where each begins.  Block (request, 64 rows); it
-// moves 2.3 KB per row: 5.1 k rows 4.5 us.
+// The latent rows of every request's keys, one request after another, and where each begins.  Block (request, 16 rows), a
+// thread's pieces all in flight: latency is what it costs (5.2 k rows, 12 MB: 64 rows a block, piece after piece, 10.2 us;
+// 5.7 here).
+constexpr int kGatherRows = 16;
 template <typename T>
 __global__ void __launch_bounds__(256)
 mla_gather_kernel(T* __restrict__ rows, int32_t* __restrict__ kv_start, const T* __restrict__ pool,
@@ -499,9 +501,9 @@ mla_gather_kernel(T* __restrict__ rows, int32_t* __restrict__ kv_start, const T*
                   int64_t rtt_stride) {
   constexpr int kChunks = (kMpRank + kMpRope) / 8;  // 16-byte pieces of a row
   __shared__ int part[8];
-  __shared__ int slots[64];
+  __shared__ int slots[kGatherRows];
   griddep_wait();
-  const int req = blockIdx.x, tid = threadIdx.x, at = blockIdx.y * 64;
+  const int req = blockIdx.x, tid = threadIdx.x, at = blockIdx.y * kGatherRows;
   const int len = prefix_lens[req] + extend_lens[req];
   if (at >= len && blockIdx.y > 0) return;
   int before = 0;
@@ -509,19 +511,25 @@ mla_gather_kernel(T* __restrict__ rows, int32_t* __restrict__ kv_start, const T*
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
   if ((tid & 31) == 0) part[tid >> 5] = before;
-  if (tid < 64 && at + tid < len) slots[tid] = req_to_token[req_pool_indices[req] * rtt_stride + at + tid];
+  if (tid < kGatherRows && at + tid < len) slots[tid] = req_to_token[req_pool_indices[req] * rtt_stride + at + tid];
   __syncthreads();
   int start = 0;
 #pragma unroll
   for (int i = 0; i < 8; ++i) start += part[i];
   if (blockIdx.y == 0 && tid == 0) kv_start[req] = start;
   // (rows past `total`, what the caller says the lengths add up to, are not written)
-  const int64_t n = min(static_cast<int64_t>(min(64, len - at)), total - start - at);
+  const int64_t n = min(static_cast<int64_t>(min(kGatherRows, len - at)), total - start - at);
   T* dst = rows + (static_cast<int64_t>(start) + at) * (kMpRank + kMpRope);
-  for (int i = tid; i < n * kChunks; i += 256) {
-    const int r = i / kChunks, c = i - r * kChunks;
-    stv(dst + i * 8, ldv(pool + static_cast<int64_t>(slots[r]) * (kMpRank + kMpRope) + c * 8));
+  constexpr int kPer = (kGatherRows * kChunks + 255) / 256;
+  Vec16<T> v[kPer];
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    const int i = tid + 256 * k, r = i / kChunks, c = i - r * kChunks;
+    if (i < n * kChunks) v[k] = ldv(pool + static_cast<int64_t>(slots[r]) * (kMpRank + kMpRope) + c * 8);
   }
+#pragma unroll
+  for (int k = 0; k < kPer; ++k)
+    if (tid + 256 * k < n * kChunks) stv(dst + (tid + 256 * k) * 8, v[k]);
   griddep_launch_dependents();
 }
 
@@ -539,11 +547,11 @@ int spd_mla_gather(void* rows, int32_t* kv_start, const void* kv_pool, const int
               "spd_mla_gather: null pointer");
   SPD_REQUIRE(kv_lora_rank == kMpRank && rope_dim == kMpRope, SPD_E_SHAPE,
               "spd_mla_gather: built for kv_lora_rank 512 + rope 64 (got %d + %d)", kv_lora_rank, rope_dim);
-  SPD_REQUIRE(batch >= 0 && total_kv >= 0 && total_kv < (1ll << 31) && max_kv_len >= 0 && max_kv_len <= 64ll * 65535,
+  SPD_REQUIRE(batch >= 0 && total_kv >= 0 && total_kv < (1ll << 31) && max_kv_len >= 0 && max_kv_len <= static_cast<int64_t>(kGatherRows) * 65535,
               SPD_E_BADARG, "spd_mla_gather: bad sizes");
   SPD_REQUIRE(aligned16(rows) && aligned16(kv_pool), SPD_E_ALIGN, "spd_mla_gather: pointers must be 16-B aligned");
   if (batch == 0) return 0;
-  const unsigned chunks = static_cast<unsigned>((max_kv_len + 63) / 64);
+  const unsigned chunks = static_cast<unsigned>((max_kv_len + kGatherRows - 1) / kGatherRows);
   SPD_DISPATCH_DTYPE(dtype, {
     SPD_CUDA(launch(mla_gather_kernel<T>, dim3((unsigned)batch, chunks > 0 ? chunks : 1), dim3(256), 0, as_stream(stream),
                     pdl_enabled(), (T*)rows, kv_start, (const T*)kv_pool, req_to_token, req_pool_indices, prefix_lens,

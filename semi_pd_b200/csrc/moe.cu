@@ -190,23 +190,30 @@ moe_align_kernel(int32_t* __restrict__ row_token, int32_t* __restrict__ inv_pos,
   }
 }
 
-// xs[r, :] = x[row_token[r], :]  (zeros for padding rows)
+// xs[r, :] = x[row_token[r], :]  (zeros for padding rows).  A warp per row, eight pieces of a lane in flight: 32768 rows of
+// 4 KB 34 us with a block and one piece per thread for each, 23.9 here.
 template <typename T>
 __global__ void __launch_bounds__(256)
-moe_gather_kernel(T* __restrict__ xs, const T* __restrict__ x, const int32_t* __restrict__ row_token, int64_t dim,
-                  int64_t x_stride) {
+moe_gather_kernel(T* __restrict__ xs, const T* __restrict__ x, const int32_t* __restrict__ row_token, int64_t rows,
+                  int64_t dim, int64_t x_stride) {
   griddep_wait();
-  const int64_t r = blockIdx.x;
+  const int64_t r = blockIdx.x * 8ll + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (r >= rows) return;
   const int tok = row_token[r];
-  MVec8* dst = reinterpret_cast<MVec8*>(xs + r * dim);
   const int nv = static_cast<int>(dim >> 3);
-  if (tok < 0) {
-    MVec8 z;
-    z.w[0] = z.w[1] = z.w[2] = z.w[3] = 0u;
-    for (int i = threadIdx.x; i < nv; i += 256) dst[i] = z;
-  } else {
-    const MVec8* src = reinterpret_cast<const MVec8*>(x + tok * x_stride);
-    for (int i = threadIdx.x; i < nv; i += 256) dst[i] = src[i];
+  uint4* dst = reinterpret_cast<uint4*>(xs + r * dim);
+  const uint4* src = reinterpret_cast<const uint4*>(x + static_cast<int64_t>(tok < 0 ? 0 : tok) * x_stride);
+  for (int i0 = lane; i0 < nv; i0 += 256) {
+    uint4 v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      v[k] = make_uint4(0, 0, 0, 0);
+      if (tok >= 0 && i0 + 32 * k < nv) v[k] = __ldg(src + i0 + 32 * k);
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (i0 + 32 * k < nv) dst[i0 + 32 * k] = v[k];
   }
 }
 
@@ -351,8 +358,8 @@ int spd_moe_gather(void* xs, const void* x, const int32_t* row_token, int64_t ro
               "spd_moe_gather: rows must be multiples of 8 elements, pointers 16-B aligned");
   if (rows == 0) return 0;
   SPD_DISPATCH_DTYPE(dtype, {
-    SPD_CUDA(launch(moe_gather_kernel<T>, dim3((unsigned)rows), dim3(256), 0, as_stream(stream), pdl_enabled(),
-                    (T*)xs, (const T*)x, row_token, dim, x_stride));
+    SPD_CUDA(launch(moe_gather_kernel<T>, dim3((unsigned)((rows + 7) / 8)), dim3(256), 0, as_stream(stream), pdl_enabled(),
+                    (T*)xs, (const T*)x, row_token, rows, dim, x_stride));
   });
   return 0;
 }
