@@ -569,14 +569,30 @@ pool_key_blocks_kernel(T* __restrict__ k_pool, T* __restrict__ v_pool, const int
   }
 }
 
-// Whether portions of at most `ext` new tokens take the tcgen05 prefill kernel (tiles of 128 queries x 128 keys) rather
-// than the mma.sync one (64 x 64): a query tile has to meet several whole key tiles, and a request alone, whose few tiles
-// leave SMs idle either way, has to be longer.  16 / 4 heads, mma.sync / tcgen05: 4 requests of 192 tokens, window 1024
-// 17.0 / 12.4 us, after 1500 tokens, window 512 29.4 / 23.7; of 1024, window 128 46.6 / 33.9.  One request of 192, window
-// 1024 9.8 / 10.2, of 500 after 1500, window 512 22.0 / 23.5, of 1024 29.4 / 23.3; window 128: of 1024 13.6 / 15.1, of 1500
-// 21.9 / 17.1.  The prefixes are on the device, so they do not enter the rule.
-inline bool window_tc_wins(int64_t batch, int64_t ext, int window) {
-  if (window <= 0 || window >= 512) return ext >= (batch > 1 ? 192 : 1024);
+// Whether a prefill takes the tcgen05 kernel (tiles of 128 queries x 128 keys) rather than the mma.sync one (64 x 64, two
+// blocks an SM).  What decides is how many waves the latter needs, so its blocks are estimated from what the host knows:
+// the tokens, and half a tile a request for the last one.  The prefixes are on the device and do not enter the rule.  Up to
+// 128 tokens a request the big tiles are mostly padding (two of 128, no prefix, 16 heads: 8.0 / 9.2 us, mma.sync / tcgen05).
+// - More than two blocks an SM: tcgen05 at every window.  128: 2 x 600 after 8000, 16 heads 21.1 / 16.2, 4 x 300, 32 heads
+//   27.8 / 19.0, 16 x 260, 64 heads 197 / 116; below, 1 x 1020, 16 heads 13.6 / 15.8, 2 x 1000, 8 heads 13.6 / 15.8.
+// - More than one: from windows of two key tiles.  256: 4 x 400, 8 heads 18.7 / 18.2; 384: 1 x 700, 16 heads 24.0 / 20.3;
+//   512: 1 x 600, 16 heads 29.0 / 22.9, 2 x 129, 32 heads 29.3 / 23.0; no window: 4 x 129, 16 heads 12.5 / 10.3.
+// - Fewer: a block's own time decides, 2.0 us a 64-key step against 2.4 us a 128-key one after a longer start.  No window and
+//   1024 on: 1 x 257 without a prefix, 8 heads 13.9 / 9.8, 1 x 384 after 8000, 16 heads 251 / 153, but 1 x 192, 16 heads 9.8 /
+//   10.8.  At 512 they are within 5 % of each other after a prefix (1 x 1000, 8 heads 22.0 / 23.0), but ragged portions are
+//   not (2 of at most 260 after 1500, 16 heads 28.4 / 23.7).  Below 512 mma.sync is ahead (128: 2 x 1000, 4 heads 10.5 /
+//   15.1); long portions still go to tcgen05, which keeps infinities and NaN out of the rows that do not see them.
+// The first two lines ask for portions that fill the big tiles on average: 16 heads of 4, [129] + 23 x [32], window 128 14.1 /
+// 15.9, after 3000, window 64 18.3 / 21.4, 12 x 129 15.7 / 12.2; more with one head a group, whose items hold two of the tiles
+// (8 heads, [140] + 31 x [64] 11.7 / 13.7); less from windows of 256 on, where most keys are the prefixes' ([129] + 15 x [1]
+// after 3000, 16 heads of 4 29.3 / 24.5; 64 x 129 or 1 without prefixes 25.4 / 25.7).
+inline bool window_tc_wins(int64_t batch, int64_t tokens, int64_t ext, int heads, int groups, int window) {
+  if (ext <= 128) return false;
+  if (window <= 0) window = 1 << 30;
+  const int64_t blocks = (tokens + batch * 32) * heads / 64, sms = device_sm_count_cached();
+  const int64_t mean = heads == groups ? 128 : window >= 256 ? 8 : 96;
+  if (tokens >= batch * mean && (blocks >= 2 * sms || (blocks >= sms && window >= 256))) return true;
+  if (window >= 512) return ext >= (batch > 1 ? 192 : window >= 1024 ? 256 : 1024);
   return ext >= (batch > 1 ? 1024 : 1500);
 }
 
@@ -757,7 +773,7 @@ int spd_attn_general_sms(void* out, const void* q, const void* k_pool, const voi
     return 0;
   }
   // 16-bit prefill at head size 128 on tcgen05, for the options that kernel has
-  if (window_tc_wins(batch, max_extend_len, window) && dtype != SPD_F32 && head_dim == 128 && v_dim == 128 && slopes == nullptr &&
+  if (window_tc_wins(batch, total_tokens, max_extend_len, num_q_heads, num_kv_heads, window) && dtype != SPD_F32 && head_dim == 128 && v_dim == 128 && slopes == nullptr &&
       db.table == nullptr && !(softcap > 0.f) && kb.size == 0 && kb.keep == 0 && Gv == num_kv_heads &&
       v_slot == (int64_t)num_kv_heads * 128) {
     const int rc = attn_prefill_window_try(out, q, k_pool, v_pool, req_to_token, req_pool_indices, prefix_lens, extend_lens,

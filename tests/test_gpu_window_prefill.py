@@ -145,3 +145,18 @@ def test_the_sm_budget_bounds_the_grid():
     (whole, t_whole), (few, t_few) = run(0), run(4)
     assert torch.equal(whole, few)
     assert t_few > 8 * t_whole  # 64 items on 64 CTAs, or 16 rounds on 4
+
+
+# the three lines of the choice between this kernel and the mma.sync one, a case on each side: portions of 128 tokens, two
+# (window below 256) and one block of 64 queries an SM, portions alone that fill less (148 SMs, 8 heads), and 8 tokens a
+# request on average
+@pytest.mark.parametrize("pre,ext,window", [([900] + [0] * 9, [128] * 10, 512), ([900] + [0] * 9, [129] * 10, 512),
+                                            ([40, 0, 0], [770, 770, 667], 128), ([40, 0, 0], [770, 770, 733], 128),
+                                            ([300, 0], [192, 927], 300), ([300, 0], [192, 930], 300),
+                                            ([300, 0], [192, 930], 255),
+                                            ([700], [255], 1024), ([700], [256], 1024), ([700], [256], -1), ([0], [1023], 600),
+                                            ([0], [1024], 600), ([0, 9], [5, 191], 600), ([0, 9], [5, 192], 600),
+                                            ([0] * 80, [580] + [1] * 58 + [0] * 21, 256),
+                                            ([0] * 80, [580] + [1] * 60 + [0] * 19, 256)])
+def test_both_sides_of_the_choice_of_kernel(pre, ext, window):
+    _run(pre, ext, 8, 2, window, torch.bfloat16, sinks=1.0, qtemp=(0.3, 128))
