@@ -26,7 +26,7 @@
 //                    into TMEM over the first 32 columns of the S half they came from
 //                    (tcgen05.st) and feed the PV MMA as its A operand from TMEM;
 //                    epilogue O / l straight from TMEM to global memory;
-//   warp 8, warp 9   K / V loader into 128-byte-swizzled smem; one 5-slot ring K_j V_j K_{j+1} ...
+//   warp 8, warp 9   K / V loader into 128-byte-swizzled smem; one 4-slot ring K_j V_j K_{j+1} ...
 //                    runs ahead of the consumer ACROSS items, so an item's first tiles are in
 //                    flight while the previous item drains.  A tile whose 128 page-table entries
 //                    are consecutive slots (what the run allocator produces, memory_pool.py) is a
@@ -35,13 +35,16 @@
 //                    gathered row by row through req_to_token with 16-byte cp.async;
 //   warp 10, warp 11 MMA issuer of warpgroup 0 / 1: S_h = Q K_j[h]^T (both K-major in smem), O += P_h V_j[h] (P
 //                    from TMEM, V MN-major in smem); the order is PV(j,h) then S(j+1,h) (which overwrites the columns
-//                    P(j,h) lives in; tcgen05.mma executes in order).  The next item's Q tile is fetched (TMA) before the
-//                    item's last PV goes out.
+//                    P(j,h) lives in; tcgen05.mma executes in order).  The next item's Q tile is fetched (TMA) when the
+//                    item's last S is complete.
 // The issuers' own time bounded the kernel while one lane of one warp issued for both warpgroups from unrolled code: 65 clk
 // per MMA and 250 between two units.  Whole warps with uniform operands, short loops and an issuer per warpgroup: 8
 // requests of 1024 new tokens on average, half of them behind 1024 cached ones, 32 / 8 heads: 193 -> 176 us; 4 requests
 // of 2048, 16 / 4 heads, window 1024: 142 -> 132 us.  Slower: S issued 128 keys wide with softmax and PV still per half and
 // one issuer (160 / 128 us against 156 / 112 with the sorted items), or with two (250 us: both warpgroups in one phase).
+// With an issuer each nothing keeps the warpgroups apart, and on half of the CTAs they fell into one phase: warpgroup 1
+// starts every item behind warpgroup 0 (`turn`).  64 requests of 128 tokens, 32 / 8 heads: 36.1 us with one issuer, 41.5 with
+// two, 36.2 here; 8 of 1024: 80.1, 82.8, 80.9; 16 of 500: 58.0, 62.1, 61.4 (of unequal lengths 96, 75, 75).
 // Items are ordered heaviest first (pf_sort) and dealt to the CTAs in snake order.
 // smem: Q0 Q1 + 5 K/V slots = 7 x 32 KB.  TMEM: S0a/P0a S0b/P0b | S1a/P1a S1b/P1b | O0 | O1 = 512 columns.
 #include <cuda.h>
@@ -281,6 +284,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   uint64_t* o_free = pv_done + 4;              // 2
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_free + 2);
   uint32_t* n_tiles = tmem_slot + 1;
+  volatile uint32_t* turn = tmem_slot + 2;  // items whose first S warpgroup 0's issuer has handed in
   uint16_t* list = reinterpret_cast<uint16_t*>(sO + kPfStage + kPfBars);
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
@@ -303,6 +307,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       }
       for (int i = 0; i < 2; ++i) mbar_init(&o_free[i], 4);
       *n_tiles = 0;
+      *turn = 0;
       fence_barrier_init();
     }
     __syncwarp();
@@ -339,6 +344,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     uint32_t t_base = 0;  // tiles of all previous items (ring position / 2)
     uint32_t pq = 0;      // PV units issued (all items); unit of the tile = pq % kNU
     uint32_t eq = 0;      // items of the warpgroup (o_free phase)
+    uint32_t items = 0;   // items begun
     uint32_t tn = 0;
     bool q_ahead = false;  // the next item's Q is already under way
     auto load_q = [&](const PfItem& it) {
@@ -351,11 +357,11 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       __syncwarp();
     };
     int idx = pf_rank(0, cta, ncta);
-    PfRaw raw = pf_raw_uniform(pf_raw(p, pl, idx));
+    PfRaw raw = pf_raw(p, pl, idx);
     for (int kk = 0; idx < pl.items; ++kk) {
-      const PfItem it = pf_item<kWin>(p, raw);
+      const PfItem it = pf_item<kWin>(p, pf_raw_uniform(raw));
       idx = pf_rank(kk + 1, cta, ncta);
-      raw = pf_raw_uniform(pf_raw(p, pl, idx));
+      raw = pf_raw(p, pl, idx);
       if (it.n == 0) continue;
       const int nt = w == 0 ? it.nt[0] : it.nt[1];
       if (nt > 0) {
@@ -390,9 +396,18 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       };
       // the epilogue of the previous item reads O, not S — and its last PVs (reading P in the S
       // columns) were issued before these, so S(0, .) may go out immediately
+      // Warpgroup 1 starts an item behind the first S of warpgroup 0: in one phase the two meet at the exponentials and at
+      // the output (5.7 us instead of 5.0 per item of one tile).  (The count only grows and warpgroup 0's issuer waits for
+      // nothing that comes later here; a start that is not seen costs the phase, no result.)
+      ++items;
+      if (w == 1 && nt > 0) {
+        for (int i = 0; i < 1024 && *turn < items; ++i) {}
+        __syncwarp();
+      }
       if (it.j0 < nt) {
 #pragma unroll
         for (int h = 0; h < kNU; ++h) issue_s(it.j0, h);
+        if (w == 0 && leader) *turn = items;
       }
       release_k(it.j0);
       for (int j = it.j0; j < it.n; ++j) {
@@ -400,17 +415,21 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         if (j < nt) {
 #pragma unroll
           for (int h = 0; h < kNU; ++h) {
+            if (j == nt - 1 && h == 0 && idx < pl.items) {
+              // The item's last S is under way, and nothing goes out before P arrives: once it is complete, Q's memory
+              // is free for the next item
+              const PfItem next = pf_item<kWin>(p, pf_raw_uniform(raw));
+              q_ahead = (w == 0 ? next.nt[0] : next.nt[1]) > 0;
+              if (q_ahead) {
+                mbar_wait(&s_full[w * 2 + kNU - 1], (pq / kNU) & 1);
+                load_q(next);
+              }
+            }
             pf_trace<kTrace>(p, 2 + w, tn, 0x100 + w * 2 + h);  // waiting for P
             mbar_wait(&p_full[w * 2 + h], (pq / kNU) & 1);
             pf_trace<kTrace>(p, 2 + w, tn, 0x200 + w * 2 + h);  // P ready
             mbar_wait(&kv_full[vpos % kPfSlots], (vpos / kPfSlots) & 1);
             if (j == it.j0 && h == 0) mbar_wait(&o_free[w], (eq & 1) ^ 1);  // previous item's O has been read
-            if (j == nt - 1 && h == kNU - 1 && idx < pl.items) {
-              // every S of the item is complete: its P has arrived.  Q's memory is free for the next item.
-              const PfItem next = pf_item<kWin>(p, raw);
-              q_ahead = (w == 0 ? next.nt[0] : next.nt[1]) > 0;
-              if (q_ahead) load_q(next);
-            }
             tc_fence_after_sync();
             uint32_t va = static_cast<uint32_t>(vd0) + (vpos % kPfSlots) * (kTileBytes / 16) + h * (kU * 128 / 16);
             uint32_t pa = tmem_S + w * kPfN + h * kU;

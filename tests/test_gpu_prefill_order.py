@@ -50,3 +50,23 @@ def test_sorted_and_unsorted_items(H, G, n, most, prefix):
         assert torch.equal(ops.attn_prefill(*args), out)
     finally:
         ops.set_sm_budget(0)
+
+
+# up to 384 row tiles the list is made with a tile per thread, past that by compaction; portions of exactly one K / V tile and
+# of whole tiles (both warpgroups begin every item together), CTAs with many items of one tile
+@pytest.mark.parametrize("H,G", [(4, 2), (3, 3)])
+@pytest.mark.parametrize("pre,ext", [([0] * 384, [1, 2, 3] * 128), ([7] * 385, [2] * 385), ([0] * 128, [300] + [0] * 126 + [257]),
+                                     ([0] * 130, [260] + [0] * 128 + [1]), ([0] * 64, [128] * 64), ([128, 0] * 20, [128] * 40),
+                                     ([0, 256, 0], [384] * 3)])
+def test_list_of_tiles(H, G, pre, ext):
+    from semi_pd_b200 import ops
+    args = _args(pre, ext, H, G, torch.float16)
+    want = ops.attn_prefill(*args, impl="simt").float()
+    out = ops.attn_prefill(*args)
+    # both round the output to 16 bits (2^-12 of |o| < 5), the tensor-core kernel its probabilities as well
+    assert (out.float() - want).abs().max().item() < 4e-3
+    try:
+        ops.set_sm_budget(3)
+        assert torch.equal(ops.attn_prefill(*args), out)
+    finally:
+        ops.set_sm_budget(0)
