@@ -43,3 +43,17 @@ def test_dense_act(T, E, k, inter):
     # the product is rounded to bf16 before and after the weight: 2^-9 each of values up to 5 x 5 x 1.1
     assert (got - want * dense[..., None]).abs().max().item() < 2 * 2 ** -9 * 28
     assert (got[dense == 0] == 0).all()
+
+
+@pytest.mark.parametrize("T,E,k", [(1, 1, 1), (1, 256, 8), (40, 64, 6), (256, 256, 8), (257, 256, 8), (2048, 3, 1)])
+def test_one_cta_keeps_every_entry_in_its_experts_rows(T, E, k):
+    """Up to 2048 entries one CTA does it alone, without a cluster (257 x 8: four)."""
+    from semi_pd_b200 import ops
+    g = torch.Generator().manual_seed(T + E)
+    ids = torch.randint(0, E, (T, k), generator=g, dtype=torch.int32)
+    for _ in range(3):  # its places come from atomics: any order inside an expert
+        row_token, inv_pos, tile_group = (t.cpu().long() for t in ops.moe_align(ids.to(DEV), E))
+        assert inv_pos.unique().numel() == T * k
+        assert torch.equal(row_token[inv_pos], torch.arange(T * k) // k)
+        assert torch.equal(tile_group[inv_pos // 128], ids.view(-1).long())
+        assert int((row_token >= 0).sum()) == T * k
