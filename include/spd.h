@@ -182,6 +182,9 @@ int spd_bias_act_residual(void* out, const void* x, const void* bias, const void
 #define SPD_EPI_SILU_MUL 1
 #define SPD_EPI_GELU 2
 int64_t spd_gemm_workspace_bytes(void);
+/* CTAs (pairs of CTAs) over which a decode GEMM that splits along K cuts its tiles x kblocks units, of `slots` that run at
+ * once; split: contributors per tile that it aims at (4). */
+int64_t spd_gemm_streamk_ctas(int64_t tiles, int kblocks, int split, int64_t slots);
 int spd_gemm(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_t K, int64_t lda,
              int64_t ldw, int64_t ldc, int dtype, int out_f32, int epilogue, void* workspace,
              int64_t workspace_bytes, int sm_budget, spd_stream_t stream);

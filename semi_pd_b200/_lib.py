@@ -58,6 +58,7 @@ SIGNATURES = {
     "spd_build_kv_indices": (_i, [_p, _p, _p, _p, _p, _p, _i64, _i64, _p]),
     "spd_write_req_to_token": (_i, [_p, _p, _p, _p, _p, _p, _i64, _i64, _p]),
     "spd_gemm_workspace_bytes": (_i64, []),
+    "spd_gemm_streamk_ctas": (_i64, [_i64, _i, _i, _i64]),
     "spd_gemm": (
         _i,
         [_p, _p, _p, _i64, _i64, _i64, _i64, _i64, _i64, _i, _i, _i, _p, _i64, _i, _p],

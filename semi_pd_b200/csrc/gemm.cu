@@ -604,11 +604,19 @@ int get_tmap(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, u
   return 0;
 }
 
-// Fewest k-blocks of a CTA's share: about `split` CTAs per tile, each partial being read once more; shares of 64 k-blocks are
-// long enough whatever a tile's length (K = 90112, 2048 rows, 40 tokens: 32 pairs of CTAs 75 us, all 74 70; 20 tokens, the layer 266 -> 221).
-long long streamk_min_units(int kblocks, int split) {
-  const long long n = kblocks / split < 64 ? kblocks / split : 64;
-  return n > 4 ? n : 4;
+// How many CTAs (or pairs) a stream-K call cuts its units (tiles x k-blocks) over, of `slots` that run at once: as many as
+// leave a tile about `split` contributors (every partial is read once more) and a share 4 k-blocks.  Long rows in few tiles
+// leave most of the slots idle that way; a share of 64 k-blocks then pays whatever the tile's length, up to a quarter of the
+// slots in use, and one of 96 up to half of them.  Pairs, 40 / 160 tokens, us: 1 tile of 448 k-blocks 4 pairs 24 / 32, 7 pairs 18 / 30;
+// 4 x 1408 (16, 74) 61 / 76, 40 / 62; 8 x 1408 (32, 74) 69 / 83, 62 / 78; 8 x 1024 (32, 74) 51 / 62, 49 / 62.  No gain: 8 x 512 (32, 64)
+// 29 / 38, 29 / 39; 12 x 448 (48, 74) 31 / 40, 32 / 43; 16 x 448 (64, 74) 39 / 47, 39 / 49, 256 tokens 58, 61; 4 x 272 (16, 17) 18 / 25, 18 / 26.
+long long streamk_ctas(long long tiles, int kblocks, int split, long long slots) {
+  const long long units = tiles * kblocks, base = kblocks / split > 4 ? kblocks / split : 4;
+  auto ctas = [&](long long share) { return units / slots >= share ? slots : units / share > 0 ? units / share : 1; };
+  const long long g = ctas(base);
+  if (4 * g <= slots && 4 * ctas(64) >= 5 * g) return ctas(64);
+  if (2 * g <= slots && units / slots >= 96) return slots;
+  return g;
 }
 
 int gemm_cluster_try(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_t K, int64_t lda,
@@ -646,6 +654,11 @@ using namespace spd;
 
 extern "C" {
 
+int64_t spd_gemm_streamk_ctas(int64_t tiles, int kblocks, int split, int64_t slots) {
+  if (tiles <= 0 || kblocks <= 0 || split <= 0 || slots <= 0) return SPD_E_BADARG;
+  return streamk_ctas(tiles, kblocks, split, slots);
+}
+
 int64_t spd_gemm_workspace_bytes(void) { return kGemmWsBytes + kGemmCounters * 4; }
 
 int spd_gemm(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_t K, int64_t lda,
@@ -679,21 +692,16 @@ int spd_gemm(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_
   CUtensorMap tx, ty;
   int rc;
 
-  // stream-K grid: one equal unit range per SM, but never so thin that a tile is shared by more
-  // than ~SPD_GEMM_SPLIT CTAs (the owner reads one partial per contributor) or a CTA gets < 4
-  // k-blocks.  Tuning knobs (experiments only): SPD_GEMM_STREAMK=0 disables stream-K, =2 forces it;
-  // SPD_GEMM_SPLIT=d caps the contributors per tile at ~d; SPD_GEMM_SWAPMAX=m is the largest M
-  // routed to swap-AB; SPD_GEMM_CLUSTER=1 routes few-tile layers at M <= 128 to the cluster
+  // stream-K grid: equal unit ranges (streamk_ctas).  Tuning knobs (experiments only):
+  // SPD_GEMM_STREAMK=0 disables stream-K, =2 forces it; SPD_GEMM_SPLIT=d aims at ~d contributors per
+  // tile where that does not leave most SMs idle; SPD_GEMM_SWAPMAX=m is the largest M routed to swap-AB; SPD_GEMM_CLUSTER=1 routes few-tile layers at M <= 128 to the cluster
   // split-K kernel (gemm_cluster.cu) instead.
   static const int env_streamk = getenv("SPD_GEMM_STREAMK") ? atoi(getenv("SPD_GEMM_STREAMK")) : 1;
   static const int env_split = getenv("SPD_GEMM_SPLIT") ? atoi(getenv("SPD_GEMM_SPLIT")) : 4;
   static const int env_swapmax = getenv("SPD_GEMM_SWAPMAX") ? atoi(getenv("SPD_GEMM_SWAPMAX")) : 256;
   const bool ws_ok = env_streamk && workspace && workspace_bytes >= spd_gemm_workspace_bytes();
   auto streamk_grid = [&](long long tiles, int BN) -> int {
-    const long long units = tiles * kblocks;
-    long long g = sms;
-    const long long min_units = streamk_min_units(kblocks, env_split);
-    if (units / g < min_units) g = units / min_units > 0 ? units / min_units : 1;
+    long long g = streamk_ctas(tiles, kblocks, env_split, sms);
     if (g * kBM * BN * 4 > kGemmWsBytes) g = kGemmWsBytes / (1ll * kBM * BN * 4);
     if (g > kGemmCounters) g = kGemmCounters;
     return static_cast<int>(g);

@@ -501,7 +501,7 @@ static int launch_pair_decode(const CUtensorMap& tw, const CUtensorMap& ta, cons
   return 0;
 }
 
-long long streamk_min_units(int kblocks, int split);  // gemm.cu
+long long streamk_ctas(long long tiles, int kblocks, int split, long long slots);  // gemm.cu
 
 // Called by spd_gemm for the swap-AB regime.  Returns 1 if this path does not apply (the caller
 // falls through to the single-CTA kernel), 0 on launch, else an error code.
@@ -532,10 +532,7 @@ int gemm_pair_decode_try(void* C, const void* A, const void* W, int64_t M, int64
   const long long waves = (p.tiles + max_pairs - 1) / max_pairs;
   const bool ws_ok = ws && flags && p.kblocks >= 8;
   if (ws_ok && static_cast<long long>(p.tiles) * 10 < waves * max_pairs * 9) {
-    const long long units = static_cast<long long>(p.tiles) * p.kblocks;
-    long long g = max_pairs;
-    const long long min_units = streamk_min_units(p.kblocks, max_split);
-    if (units / g < min_units) g = units / min_units > 0 ? units / min_units : 1;
+    long long g = streamk_ctas(p.tiles, p.kblocks, max_split, max_pairs);
     const long long per_cta = static_cast<long long>(kPdBM) * BN * 4;
     if (2 * g * per_cta > ws_bytes) g = ws_bytes / (2 * per_cta);
     if (2 * g > n_flags) g = n_flags / 2;
