@@ -319,6 +319,42 @@ retention_chunked_kernel(const __grid_constant__ RetChunkParams p) {
   };
   fetch(begin);
 
+  // what the first chunk needs besides its rows, before anything waits for the state: what a CTA does before its first MMA
+  // counts for short portions and for every wave of segments (60 tokens 12.9 us with the angles requested after the state had
+  // arrived, 12.5 here; 8000 tokens of 4 heads in segments of two chunks 116, 82)
+  const int half = p.rot >> 1;
+  const int rot_steps = sizeof(T) == 2 && VS == 1 ? p.rot / 16 : kRcDk / 16;  // k-steps whose q, k need three parts
+  const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
+  const int ar = (warp & 3) * 16 + (lane >> 2), ac = (warp >> 2) * 16 + 2 * (lane & 3);  // fragment row (+ 8), column
+
+  // this thread's part of a chunk's preparation: token t, eight pairs (8 g .., 8 g + half ..) of q or k where they are rotated
+  // (of both, where more than 64 channels are), pieces of eight channels of what is not rotated, value columns 8 u ..
+  const int t = tid & 63, t8 = tid >> 6, ut = tid >> 3, u = tid & 7;
+  const int groups = p.rot >> 4;
+  const bool both = groups > 4, rotates = t8 < (both ? groups : 2 * groups);
+  const int w0 = !both && t8 >= groups ? 1 : 0, d0 = 8 * (t8 - w0 * groups), d1 = d0 + half;
+  const int plain = (kRcDk - p.rot) >> 3;  // pieces of a row that are not rotated
+  float cs[8], sn[8];
+  auto angles = [&](int t0) {  // cos / sin of this thread's token and channels, loaded a chunk ahead; zeros past the portion
+    if (!rotates) return;
+    int64_t pos = pos0 + t0 + t;
+    pos = pos < p.max_positions ? pos : p.max_positions - 1;
+    const bool live = t0 + t < n;
+    const float4* cp = reinterpret_cast<const float4*>(p.cos_sin + pos * p.rot + d0);
+    const float4* sp = reinterpret_cast<const float4*>(p.cos_sin + pos * p.rot + half + d0);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f), a = live ? __ldg(cp + e) : zero, b = live ? __ldg(sp + e) : zero;
+      cs[4 * e] = a.x; cs[4 * e + 1] = a.y; cs[4 * e + 2] = a.z; cs[4 * e + 3] = a.w;
+      sn[4 * e] = b.x; sn[4 * e + 1] = b.y; sn[4 * e + 2] = b.z; sn[4 * e + 3] = b.w;
+    }
+  };
+  if constexpr (VS == 1) {
+    // bf16 channels that are not rotated have one part: the others' rows in K^T V' are zeros
+    for (int i = tid; i < 2 * kRcQ / 16; i += kRcThreads) reinterpret_cast<uint4*>(sK + kRcQ)[i] = make_uint4(0, 0, 0, 0);
+  }
+  angles(begin);
+
   // this thread's piece of the state: channel sr, value columns sc .. sc + 15
   const int sr = (warp & 3) * 32 + lane, sc = (warp >> 2) * 16;
   float* st = p.state + (p.req_pool_indices[r] * p.H + h) * static_cast<int64_t>(kRcDk) * p.dv +
@@ -358,38 +394,6 @@ retention_chunked_kernel(const __grid_constant__ RetChunkParams p) {
     }
   };
   put_state();
-  const int half = p.rot >> 1;
-  const int rot_steps = sizeof(T) == 2 && VS == 1 ? p.rot / 16 : kRcDk / 16;  // k-steps whose q, k need three parts
-  const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
-  const int ar = (warp & 3) * 16 + (lane >> 2), ac = (warp >> 2) * 16 + 2 * (lane & 3);  // fragment row (+ 8), column
-
-  // this thread's part of a chunk's preparation: token t, eight pairs (8 g .., 8 g + half ..) of q or k where they are rotated
-  // (of both, where more than 64 channels are), pieces of eight channels of what is not rotated, value columns 8 u ..
-  const int t = tid & 63, t8 = tid >> 6, ut = tid >> 3, u = tid & 7;
-  const int groups = p.rot >> 4;
-  const bool both = groups > 4, rotates = t8 < (both ? groups : 2 * groups);
-  const int w0 = !both && t8 >= groups ? 1 : 0, d0 = 8 * (t8 - w0 * groups), d1 = d0 + half;
-  const int plain = (kRcDk - p.rot) >> 3;  // pieces of a row that are not rotated
-  float cs[8], sn[8];
-  auto angles = [&](int t0) {  // cos / sin of this thread's token and channels, loaded a chunk ahead; zeros past the portion
-    if (!rotates) return;
-    int64_t pos = pos0 + t0 + t;
-    pos = pos < p.max_positions ? pos : p.max_positions - 1;
-    const bool live = t0 + t < n;
-    const float4* cp = reinterpret_cast<const float4*>(p.cos_sin + pos * p.rot + d0);
-    const float4* sp = reinterpret_cast<const float4*>(p.cos_sin + pos * p.rot + half + d0);
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f), a = live ? __ldg(cp + e) : zero, b = live ? __ldg(sp + e) : zero;
-      cs[4 * e] = a.x; cs[4 * e + 1] = a.y; cs[4 * e + 2] = a.z; cs[4 * e + 3] = a.w;
-      sn[4 * e] = b.x; sn[4 * e + 1] = b.y; sn[4 * e + 2] = b.z; sn[4 * e + 3] = b.w;
-    }
-  };
-  if constexpr (VS == 1) {
-    // bf16 channels that are not rotated have one part: the others' rows in K^T V' are zeros
-    for (int i = tid; i < 2 * kRcQ / 16; i += kRcThreads) reinterpret_cast<uint4*>(sK + kRcQ)[i] = make_uint4(0, 0, 0, 0);
-  }
-  angles(begin);
   cp_async_wait<0>();
   tc_fence_before_sync();
   __syncthreads();
