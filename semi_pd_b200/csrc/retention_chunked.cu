@@ -984,21 +984,22 @@ static int rc_launch(const RetChunkParams& p, int64_t segments, cudaStream_t str
 
 // Tokens of a segment (a multiple of 64), or 0: portions are not cut.  Estimates in us.  Not cut: the longest portion (which
 // only the device knows: 1.25 times the mean) at 5.6 per chunk.  Cut: the waves of CTAs of the segments' sums (4.5 per chunk,
-// two CTAs an SM, 128 columns each), 10 for the scan and the launches, the waves of the chunks' own CTAs.  16 heads, not cut /
-// cut: 1 x 500 tokens 55 / 42 (segments of 2 chunks), 1 x 1500 145 / 76 (6), 1 x 8000 728 / 260 (10), 2 x 3000 327 / 214 (6),
-// 3 x 2000 210 / 216.
+// two CTAs an SM, 128 columns each), 10 for the scan and the launches, the waves of the chunks' own CTAs and 6 for each
+// but the first (a CTA begins when one before it has ended).  16 heads, not cut /
+// cut: 1 x 500 tokens 52 / 37 (segments of 2 chunks), 1 x 1500 139 / 71 (3), 1 x 8000 728 / 241 (7), 2 x 1000 97 / 85 (4),
+// 2 x 3000 277 / 208 (8), 3 x 2000 190 / 216 (6); 32 heads, 3 x 2000 377 / 418 (5), 371 (12).
 static int rc_seg_tokens(int64_t batch, int64_t total_tokens, int H, int dv, int sms) {
   const int64_t chunks = (total_tokens + kRcTok - 1) / kRcTok, ctas = static_cast<int64_t>(H) * (dv / kRcDv);
   auto waves = [](int64_t n, int64_t slots) { return static_cast<double>((n + slots - 1) / slots); };
   const double mean = static_cast<double>(chunks) / static_cast<double>(batch);
   const double whole = waves(batch * ctas, sms) * 5.6 * (batch > 1 ? 1.25 : 1.0) * mean + 4;
-  double best = 0.8 * whole;
+  double best = 0.9 * whole;
   int seg = 0;
   for (int n = 2; n <= 16; ++n) {
     const int64_t segs = (chunks + n - 1) / n + batch / 2;
     if (segs <= batch) break;
-    const double t = waves(segs * ctas, sms) * (5.6 * n + 4) + 10 +
-                     waves((segs - batch) * ((ctas + 1) / 2), 2 * sms) * (4.5 * n + 5);
+    const double w = waves(segs * ctas, sms);
+    const double t = w * (5.6 * n + 4) + (w - 1) * 6 + 10 + waves((segs - batch) * ((ctas + 1) / 2), 2 * sms) * (4.5 * n + 5);
     if (t < best) {
       best = t;
       seg = n;
