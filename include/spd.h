@@ -710,6 +710,10 @@ int spd_attn_general_keys(void* out, const void* q, const void* k_pool, const vo
                           int qtemp_every, int64_t max_extend_len, float softcap, int num_v_heads,
                           int64_t v_slot_stride, int block_size, int block_run_len, int64_t block_base, int keep_first,
                           const float* dist_bias, int dist_bias_len, int dtype, spd_stream_t stream);
+/* Whether a 16-bit prefill at head size 128 (without distance bias, score cap, pooled blocks or kept first tokens) goes by its
+ * sizes to the tcgen05 kernel (1) or to the mma.sync one (0). */
+int spd_attn_general_tcgen05(int64_t batch, int64_t total_tokens, int64_t max_extend_len, int num_q_heads, int num_kv_heads,
+                             int window, int sm_budget);
 /* spd_attn_general_keys on sm_budget SMs of the device (0: all), for the forms that run one CTA per SM. */
 int spd_attn_general_sms(void* out, const void* q, const void* k_pool, const void* v_pool,
                          const int32_t* req_to_token, const int64_t* req_pool_indices, const int64_t* seq_lens,

@@ -586,10 +586,12 @@ pool_key_blocks_kernel(T* __restrict__ k_pool, T* __restrict__ v_pool, const int
 // 15.9, after 3000, window 64 18.3 / 21.4, 12 x 129 15.7 / 12.2; more with one head a group, whose items hold two of the tiles
 // (8 heads, [140] + 31 x [64] 11.7 / 13.7); less from windows of 256 on, where most keys are the prefixes' ([129] + 15 x [1]
 // after 3000, 16 heads of 4 29.3 / 24.5; 64 x 129 or 1 without prefixes 25.4 / 25.7).
-inline bool window_tc_wins(int64_t batch, int64_t tokens, int64_t ext, int heads, int groups, int window) {
+// The SMs are the caller's.  Counted against the device's on a partition of 40: 1 x 500, 16 heads, window 512 37.8 / 16.7 us, 4 x 200
+// after 1500, window 128 39.6 / 20.7; of 72: 1 x 500, 16 heads, window 512 27.3 / 16.9.
+inline bool window_tc_wins(int64_t batch, int64_t tokens, int64_t ext, int heads, int groups, int window, int64_t sms) {
   if (ext <= 128) return false;
   if (window <= 0) window = 1 << 30;
-  const int64_t blocks = (tokens + batch * 32) * heads / 64, sms = device_sm_count_cached();
+  const int64_t blocks = (tokens + batch * 32) * heads / 64;
   const int64_t mean = heads == groups ? 128 : window >= 256 ? 8 : 96;
   if (tokens >= batch * mean && (blocks >= 2 * sms || (blocks >= sms && window >= 256))) return true;
   if (window >= 512) return ext >= (batch > 1 ? 192 : window >= 1024 ? 256 : 1024);
@@ -672,6 +674,14 @@ int spd_pool_key_blocks(void* k_pool, void* v_pool, const int32_t* req_to_token,
                     v_row_elems, tl, kb));
   });
   return 0;
+}
+
+int spd_attn_general_tcgen05(int64_t batch, int64_t total_tokens, int64_t max_extend_len, int num_q_heads, int num_kv_heads,
+                             int window, int sm_budget) {
+  return window_tc_wins(batch, total_tokens, max_extend_len, num_q_heads, num_kv_heads, window,
+                        sm_budget > 0 ? sm_budget : device_sm_count_cached())
+             ? 1
+             : 0;
 }
 
 int spd_attn_general_sms(void* out, const void* q, const void* k_pool, const void* v_pool,
@@ -773,7 +783,9 @@ int spd_attn_general_sms(void* out, const void* q, const void* k_pool, const voi
     return 0;
   }
   // 16-bit prefill at head size 128 on tcgen05, for the options that kernel has
-  if (window_tc_wins(batch, total_tokens, max_extend_len, num_q_heads, num_kv_heads, window) && dtype != SPD_F32 && head_dim == 128 && v_dim == 128 && slopes == nullptr &&
+  if (dtype != SPD_F32 && head_dim == 128 && v_dim == 128 && slopes == nullptr &&
+      window_tc_wins(batch, total_tokens, max_extend_len, num_q_heads, num_kv_heads, window,
+                     sm_budget > 0 ? sm_budget : device_sm_count_cached()) &&
       db.table == nullptr && !(softcap > 0.f) && kb.size == 0 && kb.keep == 0 && Gv == num_kv_heads &&
       v_slot == (int64_t)num_kv_heads * 128) {
     const int rc = attn_prefill_window_try(out, q, k_pool, v_pool, req_to_token, req_pool_indices, prefix_lens, extend_lens,
