@@ -185,6 +185,8 @@ int64_t spd_gemm_workspace_bytes(void);
 /* CTAs (pairs of CTAs) over which a decode GEMM that splits along K cuts its tiles x kblocks units, of `slots` that run at
  * once; split: contributors per tile that it aims at (4). */
 int64_t spd_gemm_streamk_ctas(int64_t tiles, int kblocks, int split, int64_t slots);
+/* Columns (256, 224, 192) of the tiles on CTA pairs that a GEMM of these sizes takes; 0: tiles of one CTA. */
+int spd_gemm_pair_cols(int64_t M, int64_t N, int64_t K, int epilogue, int sm_budget);
 int spd_gemm(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_t K, int64_t lda,
              int64_t ldw, int64_t ldc, int dtype, int out_f32, int epilogue, void* workspace,
              int64_t workspace_bytes, int sm_budget, spd_stream_t stream);

@@ -59,6 +59,7 @@ SIGNATURES = {
     "spd_write_req_to_token": (_i, [_p, _p, _p, _p, _p, _p, _i64, _i64, _p]),
     "spd_gemm_workspace_bytes": (_i64, []),
     "spd_gemm_streamk_ctas": (_i64, [_i64, _i, _i, _i64]),
+    "spd_gemm_pair_cols": (_i, [_i64, _i64, _i64, _i, _i]),
     "spd_attn_general_tcgen05": (_i, [_i64, _i64, _i64, _i, _i, _i, _i]),
     "spd_gemm": (
         _i,

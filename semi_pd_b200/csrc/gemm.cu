@@ -622,6 +622,7 @@ long long streamk_ctas(long long tiles, int kblocks, int split, long long slots)
 int gemm_cluster_try(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_t K, int64_t lda,
                      int64_t ldw, int64_t ldc, int dtype, int out_f32, int sms, cudaStream_t stream);
 
+int gemm_pair_cols(int64_t M, int64_t N, int64_t K, int epilogue, int sms);
 int gemm_pair_try(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_t K, int64_t lda,
                   int64_t ldw, int64_t ldc, int dtype, int out_f32, int epilogue, int sms, int panel_mb,
                   cudaStream_t stream);
@@ -657,6 +658,11 @@ extern "C" {
 int64_t spd_gemm_streamk_ctas(int64_t tiles, int kblocks, int split, int64_t slots) {
   if (tiles <= 0 || kblocks <= 0 || split <= 0 || slots <= 0) return SPD_E_BADARG;
   return streamk_ctas(tiles, kblocks, split, slots);
+}
+
+int spd_gemm_pair_cols(int64_t M, int64_t N, int64_t K, int epilogue, int sm_budget) {
+  if (M <= 0 || N <= 0 || K <= 0) return SPD_E_BADARG;
+  return gemm_pair_cols(M, N, K, epilogue, sm_budget > 0 ? sm_budget : device_sm_count_cached());
 }
 
 int64_t spd_gemm_workspace_bytes(void) { return kGemmWsBytes + kGemmCounters * 4; }

@@ -325,13 +325,10 @@ static int pair_tile_cols(int64_t N, int64_t x_tiles, int epilogue, int pairs, i
   return best;
 }
 
-// Called by spd_gemm for the prefill regime.  Returns 1 if this path does not apply (the caller
-// falls through to the single-CTA kernel), 0 on launch, else an error code.
-int gemm_pair_try(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_t K, int64_t lda,
-                  int64_t ldw, int64_t ldc, int dtype, int out_f32, int epilogue, int sms, int panel_mb,
-                  cudaStream_t stream) {
+// Columns of the pair tiles that a GEMM of these sizes takes, 0: single-CTA tiles.
+int gemm_pair_cols(int64_t M, int64_t N, int64_t K, int epilogue, int sms) {
   static const int enabled = getenv("SPD_GEMM_2CTA") ? atoi(getenv("SPD_GEMM_2CTA")) : 1;
-  if (!enabled || M <= 256 || sms < 2) return 1;
+  if (!enabled || M <= 256 || sms < 2) return 0;
   // A wave of 256 x 256 pair tiles takes about 0.9 of the time of a wave of 128 x 256 single tiles, so the pair serves also
   // where its taller tiles pad M more, unless that costs it another wave — or the call is so short (under 48 k-blocks in
   // all waves) that the pair's longer start and end decide.  4096 x 14336 weights: M = 300 87 -> 70 us, 600 87 -> 72,
@@ -343,8 +340,18 @@ int gemm_pair_try(void* C, const void* A, const void* W, int64_t M, int64_t N, i
     const int n_tile = epilogue == SPD_EPI_SILU_MUL ? kPgBN / 2 : kPgBN;
     const int64_t cols = (N + n_tile - 1) / n_tile, kblocks = (K + kPgBK - 1) / kPgBK;
     const int64_t waves_single = (rows_single / 128 * cols + sms - 1) / sms;
-    if (cost * 9 >= waves_single * (kPgBN + 100) * 10 || waves_single * kblocks < 48) return 1;
+    if (cost * 9 >= waves_single * (kPgBN + 100) * 10 || waves_single * kblocks < 48) return 0;
   }
+  return bn;
+}
+
+// Called by spd_gemm for the prefill regime.  Returns 1 if this path does not apply (the caller
+// falls through to the single-CTA kernel), 0 on launch, else an error code.
+int gemm_pair_try(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_t K, int64_t lda,
+                  int64_t ldw, int64_t ldc, int dtype, int out_f32, int epilogue, int sms, int panel_mb,
+                  cudaStream_t stream) {
+  const int bn = gemm_pair_cols(M, N, K, epilogue, sms);
+  if (bn == 0) return 1;
   PairGemmParams p{};
   p.C = C;
   p.ldc = ldc;

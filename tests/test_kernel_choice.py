@@ -1,8 +1,24 @@
-"""Which kernel a call's sizes choose, at the sizes that the GPU tests of those kernels run: tcgen05 or mma.sync for the windowed
-prefill attention, on the whole GPU and on a partition."""
+"""Which kernel a call's sizes choose, at the sizes that the GPU tests of those kernels run: the width of a prefill GEMM's tiles
+on CTA pairs, and tcgen05 or mma.sync for the windowed prefill attention, on the whole GPU and on a partition."""
 import pytest
 
-from semi_pd_b200._lib import lib
+from semi_pd_b200._lib import SPD_EPI_GELU, SPD_EPI_NONE, SPD_EPI_SILU_MUL, lib
+
+
+@pytest.mark.parametrize("M,N,cols", [(768, 4096, 192), (768, 4104, 192), (700, 4000, 192), (768, 4224, 192), (4096, 3648, 224),
+                                      (4000, 3592, 224), (2048, 6144, 256), (2048, 6080, 256)])
+@pytest.mark.parametrize("K", [64, 200, 1024])
+def test_pair_tile_columns(M, N, K, cols):
+    assert lib.spd_gemm_pair_cols(M, N, K, SPD_EPI_NONE, 148) == cols
+    for epilogue in (SPD_EPI_SILU_MUL, SPD_EPI_GELU):
+        assert lib.spd_gemm_pair_cols(M, N, K, epilogue, 148) in (0, 256)
+
+
+def test_single_cta_tiles():
+    assert lib.spd_gemm_pair_cols(256, 4096, 4096, SPD_EPI_NONE, 148) == 0   # decode
+    assert lib.spd_gemm_pair_cols(600, 3648, 2048, SPD_EPI_NONE, 148) == 0   # a call too short for the rows a pair pads
+    assert lib.spd_gemm_pair_cols(4096, 4096, 4096, SPD_EPI_NONE, 1) == 0    # no pair of SMs
+    assert lib.spd_gemm_pair_cols(4096, 4096, 4096, SPD_EPI_NONE, 2) == 256
 
 
 def _tcgen05(ext, window, sms, heads=8, groups=2):
