@@ -4,7 +4,7 @@
 Contract (driver): `python bench.py --gpus N --steps K --warmup W [--impl reference]`; for N > 1 it
 is launched under torch.distributed.run, one rank per GPU.  Rank 0 prints ONE JSON line.
 
-Workload (BASELINE.json configs[1]): Llama-3-8B, TP = 1, semi-PD with a 50/50 SM split, synthetic
+Workload: Llama-3-8B, TP = 1, semi-PD with a 50/50 SM split, synthetic
 requests of 1024 input / 128 output tokens (token ids as python/sglang/bench_serving.py:772-783,
 np.random.seed(1); ignore_eos), random-init weights of that architecture.
 A STEP = one serving window: R requests pushed through the engine (prefill worker and decode worker
@@ -26,7 +26,7 @@ N > 1: `value` / `e2e` are N independent replicas (one engine per GPU, no data-p
 weak scaling); the `tp` block then serves the same mix with ONE engine sharded TP = N (heads / FFN
 columns per GPU, spd_allreduce / NCCL after o_proj and down_proj), `tp_parity` checks a TP = N
 model against the unsharded oracle in this very run, and at N = 8 `tp_70b` runs Llama-3-70B TP = 8
-(BASELINE.json configs[4]).
+(tensor parallelism).
 `--impl reference` times the CPU restatement of the reference forward (oracle/) on the host cores.
 """
 from __future__ import annotations

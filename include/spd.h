@@ -147,7 +147,7 @@ int spd_write_req_to_token(int32_t* req_to_token, const int64_t* req_pool_indice
                            int64_t req_to_token_stride, spd_stream_t stream);
 
 /* ---------------------------------------------------------------------------------------------
- * OPT-family ops (opt-125m plumbing + logit check).  The reference has no OPT
+ * OPT-family ops (opt-125m: plumbing + logit check).  The reference has no OPT
  * model; these follow torch.nn.LayerNorm / F.relu / the `residual + hidden_states` adds of
  * transformers' modeling_opt.py (OPTDecoderLayer.forward), fp32 math, 16-bit I/O.
  * spd_layernorm: out = (x - mean) / sqrt(var + eps) * gamma + beta per row (dim <= 8192).
@@ -251,7 +251,7 @@ int spd_attn_decode_simt(void* out, const void* q, const void* k_pool, const voi
 
 /* ---------------------------------------------------------------------------------------------
  * tensor-parallel all-reduce over NVLink peer memory (one process per GPU) — the `spd_allreduce`
- * of SURVEY §8b's export list.  Replaces the custom all-reduce the reference sends every
+ * of the exported operators.  Replaces the custom all-reduce the reference sends every
  * RowParallelLinear output below 8 MiB through (S/layers/linear.py:1265-1266 →
  * S/distributed/parallel_state.py:376-436 → device_communicators/custom_all_reduce.py:147-160,
  * 447-480; alternative K/csrc/allreduce/trt_reduce_internal.cu:190-300); the reference sends larger
@@ -302,7 +302,7 @@ int spd_allgather(spd_comm_t* comm, void* out, const void* in, int64_t bytes_per
 int spd_comm_destroy(spd_comm_t* comm);
 
 /* ---------------------------------------------------------------------------------------------
- * DeepSeek-V2-Lite path (BASELINE configs[3]): absorbed MLA attention over the latent KV pool,
+ * DeepSeek-V2-Lite path: absorbed MLA attention over the latent KV pool,
  * grouped GEMMs and the MoE plumbing.
  * ------------------------------------------------------------------------------------------- */
 /* Grouped GEMM on the tcgen05 kernel of spd_gemm (normal regime, 128-row tiles).

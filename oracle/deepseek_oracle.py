@@ -1,4 +1,4 @@
-"""CPU oracle for BASELINE configs[3] (DeepSeek-V2-Lite: MLA attention + MoE) — TEST INFRASTRUCTURE
+"""CPU oracle for DeepSeek-V2-Lite (MLA attention + MoE) — TEST INFRASTRUCTURE
 ONLY.
 
 Restates, in fp32 torch, what the reference computes (infinigence/Semi-PD @ 2565f9f, paths relative

@@ -86,7 +86,7 @@ def weight_shapes(cfg) -> Dict[str, Tuple[int, ...]]:
 def make_weights(cfg, dtype=torch.bfloat16, seed: int = 1234, device="cpu") -> Dict[str, torch.Tensor]:
     """Synthetic weights: one torch.Generator per parameter (model_loader/weight_utils.py:606-617
     seeds each parameter's generator the same way) but N(0, sigma) with fan-in scaling instead of
-    U(-1e-3, 1e-3), so that logits are O(1) and greedy argmax is meaningful (SURVEY §7 'hard parts').
+    U(-1e-3, 1e-3), so that logits are O(1) and greedy argmax is meaningful.
     Norm weights are 1 + N(0, 0.1)."""
     out = {}
     for idx, (name, shape) in enumerate(weight_shapes(cfg).items()):

@@ -1,12 +1,12 @@
-"""CPU oracle for BASELINE configs[0] (opt-125m plumbing + logit check) — TEST INFRASTRUCTURE ONLY.
+"""CPU oracle for opt-125m (plumbing + logit check) — TEST INFRASTRUCTURE ONLY.
 
 PARITY UNPINNED against the reference: infinigence/Semi-PD has no OPT model
-(python/sglang/srt/models/ holds gpt2.py but no opt.py; SURVEY.md §8c), so there is nothing of the
+(python/sglang/srt/models/ holds gpt2.py but no opt.py), so there is nothing of the
 reference's to restate or to run.  The oracle for this config is HuggingFace transformers'
 `OPTForCausalLM` (the implementation any SGLang OPT port would be validated against,
 test/srt/models/test_generation_models.py) built from a hand-written `OPTConfig` of
 facebook/opt-125m — no weights exist offline, so they are synthetic (N(0, 0.02), LayerNorm 1 / 0,
-SURVEY §8d config 1) and shared bit for bit with the CUDA path."""
+opt-125m) and shared bit for bit with the CUDA path."""
 from __future__ import annotations
 
 from typing import Dict, List

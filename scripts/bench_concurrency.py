@@ -1,5 +1,5 @@
-"""Isolated vs concurrent timing of the two halves of the semi-PD path on their SM partitions
-("report every fraction both isolated and concurrent").
+"""Isolated vs concurrent timing of the two halves of the semi-PD path on their SM partitions,
+alone and at the same time.
   * prefill forward: one 8 x 1024-token extend batch through ModelRunner.forward on the prefill
     partition (eager, as the engine runs it);
   * decode step: one CUDA-graph replay at B requests, context ~1088, on the decode partition.

@@ -1,4 +1,4 @@
-"""BASELINE configs[3]: DeepSeek-V2-Lite (MLA + MoE) TP=1 under semi-PD, synthetic requests —
+"""DeepSeek-V2-Lite (MLA + MoE) TP=1 under semi-PD, synthetic requests —
 mirrors evaluation/benchmark_deepseek_v2_lite_semi_pd.sh:17-36 of the reference (bench_serving
 against a --enable-semi-pd server; ShareGPT there, synthetic here: no datasets offline).  One
 saturated window (all requests at t = 0) and one Poisson window at --rate req/s (the reference's
@@ -24,7 +24,7 @@ ap.add_argument("--rate", type=float, default=14.0)
 ap.add_argument("--sharegpt-like", type=int, default=0,
                 help="N > 0: additionally serve N prompts whose lengths follow a fixed-seed log-normal fitted to "
                      "ShareGPT-like statistics (in 220 +- 240, out 190 +- 200 tokens, clipped to [4, 2048]) at "
-                     "--rate req/s — SURVEY §8d config 4 (ShareGPT itself is not available offline)")
+                     "--rate req/s (ShareGPT itself is not available offline)")
 ap.add_argument("--prefill-sm-pct", type=int, default=50)
 ap.add_argument("--decode-sm-pct", type=int, default=50)
 a = ap.parse_args()
@@ -77,6 +77,6 @@ if a.sharegpt_like:
     w3 = time.perf_counter() - t0
     out["sharegpt_like"] = {"requests": n, "request_rate": a.rate, "mean_in": float(lin.mean()), "mean_out": float(lout.mean()),
                             "output_tok_per_s": float(lout.sum()) / w3, **latency_stats(reqs3),
-                            "note": "lengths: fixed-seed log-normal substitution for ShareGPT (SURVEY §8d config 4)"}
+                            "note": "lengths: fixed-seed log-normal substitution for ShareGPT"}
 eng.shutdown()
 print(json.dumps(out))

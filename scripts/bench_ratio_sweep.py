@@ -1,7 +1,7 @@
-"""BASELINE.json configs[2]: Llama-3-8B TP=1, prefill:decode SM-ratio sweep under bursty arrivals.
+"""Llama-3-8B TP=1, prefill:decode SM-ratio sweep under bursty arrivals.
 One process per ratio (green contexts live until process exit):
     for p in 20 35 50 65 80; do python scripts/bench_ratio_sweep.py $p; done
-Arrivals (SURVEY §8d config 3): bursts of 16 requests, exponential gaps between bursts with mean
+Arrivals: bursts of 16 requests, exponential gaps between bursts with mean
 16/rate seconds (inter-arrival CV = 4), seed 2; 1024-in / 128-out, ignore_eos.
 Prints one JSON line: output tok/s, p50/p99 TTFT and TPOT, the SM split actually granted."""
 import json

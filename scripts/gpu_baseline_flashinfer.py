@@ -2,7 +2,7 @@
 """GPU stand-in baseline: the reference's forward path rebuilt from the LIBRARY kernels it calls.
 
 The reference's own `--enable-semi-pd` build (torch 2.5.1 / flashinfer 0.2.3 / sgl-kernel 0.0.5 /
-vllm <= 0.7.2 pins, MPS) cannot be installed in this image (SURVEY §8c/§8d).  What the image does
+vllm <= 0.7.2 pins, MPS) cannot be installed in this image.  What the image does
 carry is flashinfer 0.6.11 — the same wrapper API the reference calls — and cuBLAS.  This script
 serves the bench's request mix (R x 1024-in / 128-out, saturated) with exactly the kernel sequence
 of the reference's Llama layer (python/sglang/srt/models/llama.py:172-183,237-259):
@@ -37,9 +37,15 @@ import threading
 import time
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-# The JIT cache lies in the tree (baseline/_ref, git-ignored) under one fixed path, so that the absolute paths ninja
-# recorded stay valid where the tree is copied to and nothing recompiles.
-_base = "/root/repo" if os.path.isdir("/root/repo/scripts") else ROOT
+# The JIT cache lies in the tree (baseline/_ref, git-ignored).  ninja records absolute paths: where the tree was copied and the
+# place it was built in leads here too, that path is used, so that nothing recompiles.
+_built_under = os.path.join(ROOT, "baseline", "_ref", "built_under")
+_base = ROOT
+if os.path.exists(_built_under):
+    with open(_built_under) as f:
+        _at = f.read().strip()
+    if os.path.exists(os.path.join(_at, "baseline", "_ref", "built_under")):
+        _base = _at
 os.environ.setdefault("FLASHINFER_WORKSPACE_BASE", os.path.join(_base, "baseline", "_ref", "flashinfer"))
 os.environ.setdefault("FLASHINFER_CUDA_ARCH_LIST", "10.0a")
 
@@ -82,6 +88,8 @@ def build_only(dtype):
     get_rope_module()
     get_batch_decode_module(dtype, dtype, dtype, torch.int32, D, D, 0, False, False)
     get_batch_prefill_module("fa2", dtype, dtype, dtype, torch.int32, D, D, 0, False, False, False)
+    with open(_built_under, "w") as f:
+        f.write(_base)
     print(f"flashinfer modules built in {time.time() - t0:.0f} s under {os.environ['FLASHINFER_WORKSPACE_BASE']}")
 
 

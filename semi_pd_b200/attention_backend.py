@@ -133,7 +133,7 @@ class SpdAttnBackend(AttentionBackend):
             self.max_extend_len = 0
             return
         # "tc" = tcgen05 kernels (the product path, head_dim 128); "simt" exists for bring-up /
-        # cross-checks and serves the head_dim-64 plumbing model (OPT-125m, BASELINE configs[0])
+        # cross-checks and serves the head_dim-64 plumbing model (OPT-125m)
         self.impl = os.environ.get("SPD_ATTN_IMPL", "tc" if self.head_dim == 128 else "simt")
         self.max_extend_len = 0
         # Scratch of the decode kernel: 64 KB of arrival counters, zeroed here and left at zero by every call, and two

@@ -42,7 +42,7 @@ class ModelConfig:
     tie_word_embeddings: bool = False
     hidden_act: str = "silu"
     is_encoder_decoder: bool = False
-    # "llama" (models/llama.py) or "opt" (BASELINE configs[0]: pre-LN, learned positions, ReLU, biases)
+    # "llama" (models/llama.py) or "opt" (pre-LN, learned positions, ReLU, biases)
     model_type: str = "llama"
     layer_norm_eps: float = 1e-5
     # hf_eos_token_id of the reference's ModelConfig (honoured when a request sets ignore_eos=False)
@@ -101,11 +101,11 @@ _PRESETS = {
     "tiny-llama-test": dict(hidden_size=256, intermediate_size=512, num_hidden_layers=2,
                             num_attention_heads=4, num_key_value_heads=2, head_dim=128,
                             vocab_size=1024, max_position_embeddings=2048),
-    # BASELINE configs[0]: facebook/opt-125m (hand-written config, no weights offline)
+    # facebook/opt-125m (hand-written config, no weights offline)
     "opt-125m": dict(model_type="opt", hidden_size=768, intermediate_size=3072, num_hidden_layers=12,
                      num_attention_heads=12, num_key_value_heads=12, head_dim=64, vocab_size=50272,
                      max_position_embeddings=2048, hidden_act="relu", tie_word_embeddings=True),
-    # BASELINE configs[3]: deepseek-ai/DeepSeek-V2-Lite (15.7 B parameters, 2.4 B active)
+    # deepseek-ai/DeepSeek-V2-Lite (15.7 B parameters, 2.4 B active)
     "deepseek-v2-lite": dict(model_type="deepseek_v2", hidden_size=2048, intermediate_size=10944,
                              num_hidden_layers=27, num_attention_heads=16, num_key_value_heads=16,
                              head_dim=192, vocab_size=102400, rms_norm_eps=1e-6, rope_theta=10000.0,
@@ -115,7 +115,7 @@ _PRESETS = {
                              routed_scaling_factor=1.0, norm_topk_prob=False, eos_token_ids=[100001],
                              rope_scaling=dict(type="yarn", factor=40.0, beta_fast=32, beta_slow=1, mscale=0.707,
                                                mscale_all_dim=0.707, original_max_position_embeddings=4096)),
-    # one 8B-shaped layer pair: exhaustive parity at real head/FFN shapes (SURVEY §8d)
+    # one 8B-shaped layer pair: exhaustive parity at real head/FFN shapes
     "llama-3-8b-2layer": dict(num_hidden_layers=2, vocab_size=4096),
 }
 

@@ -487,7 +487,7 @@ write_req_to_token_kernel(int32_t* __restrict__ req_to_token, const int64_t* __r
 }
 
 // ------------------------------------------------------------------------------------------------
-// OPT-family ops (BASELINE configs[0], the plumbing model): LayerNorm with bias, and
+// OPT-family ops (the plumbing model): LayerNorm with bias, and
 // y = act(x + bias) + residual.  fp32 math, 16-bit I/O, 16-byte vectors.
 // ------------------------------------------------------------------------------------------------
 template <typename T, int kMaxVec>

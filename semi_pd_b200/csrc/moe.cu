@@ -1,4 +1,4 @@
-// Mixture-of-experts plumbing for the DeepSeek-V2-Lite path (BASELINE configs[3]): routing,
+// Mixture-of-experts plumbing for the DeepSeek-V2-Lite path: routing,
 // token -> expert alignment, gather / combine, and the dense-decode activation.  The expert
 // GEMMs themselves run on the tcgen05 kernels of gemm.cu (spd_gemm_grouped rows mode for
 // prefill-sized batches, plain spd_gemm over the stacked expert weights for decode-sized ones).

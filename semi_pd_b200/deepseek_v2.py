@@ -1,7 +1,7 @@
 """DeepSeek-V2(-Lite) wiring — python/sglang/srt/models/deepseek_v2.py with the reference's class
 names: `DeepseekV2MLP` (:70-111), `MoEGate` (:114-138), `DeepseekV2MoE` (:141-218),
 `DeepseekV2AttentionMLA` (:393-706), `DeepseekV2DecoderLayer` (:843-990), `DeepseekV2Model`,
-`DeepseekV2ForCausalLM` (:993-1267).  BASELINE configs[3].
+`DeepseekV2ForCausalLM` (:993-1267).
 
 What differs from the reference, all on the kernel side:
   * attention takes the ABSORBED form (forward_absorb, :633-706) for decode and small prefill batches: q_nope is
@@ -140,7 +140,7 @@ class MoEGate:
 class DeepseekV2MoE:
     def __init__(self, config):
         if get_tensor_model_parallel_world_size() != 1:
-            raise NotImplementedError("the MoE config runs TP = 1 (BASELINE configs[3])")
+            raise NotImplementedError("the MoE config runs TP = 1")
         self.config = config
         self.n_experts = config.n_routed_experts
         self.top_k = config.num_experts_per_tok

@@ -3,7 +3,7 @@ python/sglang/srt/managers/io_struct.py (`TokenizedGenerateReqInput` :269-318, s
 :734-755).  In the reference they are pickled over ZMQ ipc:// sockets between processes; here
 they travel through in-process queues, and the two batch messages additionally carry a CUDA
 event so the hand-off is ordered ON THE DEVICE (the reference relies on the ZMQ round trip being
-slower than the req_to_token kernel, SURVEY §3.2).
+slower than the req_to_token kernel).
 """
 from __future__ import annotations
 

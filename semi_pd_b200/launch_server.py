@@ -3,7 +3,7 @@ Builds the semi-PD engine and serves `/generate` in TOKEN-ID space (there is no 
 offline: requests carry `input_ids`, responses carry `output_ids`, as `bench_serving
 --dataset-name random` effectively exercises the reference, bench_serving.py:772-783), plus
 `/health` and `/get_server_info`.  HTTP, OpenAI protocol and detokenisation are outside the hot
-path (SURVEY §2) and intentionally minimal.
+path and intentionally minimal.
 """
 from __future__ import annotations
 

@@ -1,5 +1,5 @@
 """Llama wiring — python/sglang/srt/models/llama.py:58-409 with the same class names and call
-order.  Differences, all fusions that remove HBM round trips (SURVEY §7 step 5):
+order.  Differences, all fusions that remove HBM round trips:
   * RoPE + KV-cache write are one kernel (`RotaryEmbedding.forward_kvwrite`); attention is then
     called with save_kv_cache=False;
   * in the prefill regime the gate_up GEMM applies SiLU·mul in its epilogue;

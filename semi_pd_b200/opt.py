@@ -1,4 +1,4 @@
-"""OPT wiring (opt-125m single-prompt greedy decode, plumbing + logit check).
+"""OPT wiring (opt-125m: single-prompt greedy decode, plumbing + logit check).
 
 The reference has no OPT model (python/sglang/srt/models/ holds gpt2.py but no opt.py), so the
 structure follows transformers' modeling_opt.py (OPTDecoderLayer / OPTDecoder / OPTForCausalLM,
@@ -123,7 +123,7 @@ class OPTForCausalLM:
                 ours.weight, ours.bias = put(w[p + theirs + ".weight"]), put(w[p + theirs + ".bias"])
 
     def init_dummy_weights(self, seed: int = 1234):
-        """weights N(0, 0.02), LayerNorm gamma = 1, beta = 0, one generator
+        """Weights N(0, 0.02), LayerNorm gamma = 1, beta = 0, one generator
         per parameter seeded like model_loader/weight_utils.py:606-617."""
         out = {}
         for idx, (name, shape) in enumerate(self.full_shapes().items()):

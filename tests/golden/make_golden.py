@@ -7,7 +7,7 @@ Reference modules exercised (python/sglang/srt/…):
   layers/radix_attention.py                 RadixAttention
   layers/rotary_embedding.py                RotaryEmbedding.forward_native, Llama3RotaryEmbedding
   model_executor/forward_batch_info.py      compute_position_torch, ForwardMode
-They need three import shims because of version drift in this image (SURVEY §8c): an `IPython`
+They need three import shims because of version drift in this image: an `IPython`
 stub, a `semi_pd_ipc` stub and three `triton.runtime.cache` names.
 """
 import os

@@ -1,6 +1,6 @@
 """Pins oracle/deepseek_oracle.py (the restatement of the reference's MLA normal / absorbed attention
 over a latent KV pool, and its MoE) against transformers' DeepseekV2ForCausalLM on identical random
-weights.  CPU only; prepares BASELINE configs[3] for the next round (no CUDA path yet)."""
+weights.  CPU only."""
 import pytest
 import torch
 

@@ -1,8 +1,8 @@
-"""DeepSeek-V2-Lite path (BASELINE configs[3]) on the GPU: absorbed MLA attention over the latent
+"""DeepSeek-V2-Lite path on the GPU: absorbed MLA attention over the latent
 pool, block-diagonal / grouped GEMMs, MoE routing + expert dispatch, and the whole model against
 oracle/deepseek_oracle.py (the restatement of the reference's models/deepseek_v2.py, pinned to
 transformers' DeepseekV2ForCausalLM by tests/test_deepseek_oracle.py — "parity unpinned" against
-the reference itself, whose module does not import in this image, SURVEY §8c)."""
+the reference itself, whose module does not import in this image)."""
 import math
 
 import pytest
@@ -338,7 +338,7 @@ def test_deepseek_decode_dense_moe_path_and_cuda_graph():
 
 
 def test_deepseek_semi_pd_engine_matches_sequential_oracle():
-    """BASELINE configs[3] end to end: the semi-PD engine (prefill and decode workers on disjoint SM
+    """DeepSeek-V2-Lite end to end: the semi-PD engine (prefill and decode workers on disjoint SM
     partitions, chunked prefill, decode CUDA graphs over the latent pool) serving the mini
     DeepSeek-V2 model produces the sequential oracle's greedy tokens.  A step is compared only
     where the oracle's top-1 / top-2 margin exceeds 2e-2 and no router decision of that forward

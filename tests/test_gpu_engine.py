@@ -2,7 +2,7 @@
 decode worker running CONCURRENTLY on disjoint green-context SM partitions, CUDA-graph decode,
 chunked prefill, overlap scheduling) must produce exactly the greedy token ids the CPU oracle
 produces one request at a time — wherever the oracle's top-1/top-2 margin exceeds 2e-2.
-This is the property the reference never tests ("no Semi-PD tests"): P‖D output ==
+This is the property the reference never tests (it has no Semi-PD tests): P‖D output ==
 sequential output."""
 import pytest
 import torch
@@ -175,7 +175,7 @@ def test_decode_oom_retraction_reprefill_same_tokens():
 
 
 def test_eager_steps_above_graph_bs_do_not_corrupt_small_graph_replays():
-    """the split-KV workspace captured by the small-bs decode graphs must
+    """The split-KV workspace captured by the small-bs decode graphs must
     survive eager decode steps with bs > cuda_graph_max_bs.  10 requests run with graphs captured
     for bs <= 4 only: the batch decodes eagerly while it is large, and through the bs 4/2/1 graphs
     (which split the KV across CTAs and use the workspace) once the short requests have finished."""
@@ -212,7 +212,7 @@ def test_eager_steps_above_graph_bs_do_not_corrupt_small_graph_replays():
 
 
 def test_request_validation_and_two_engines_in_one_process():
-    """over-long inputs are rejected at the engine front, max_new_tokens is
+    """Over-long inputs are rejected at the engine front, max_new_tokens is
     clipped to the context, and the queue keeps moving.  Also: shutdown() releases the engine's
     device memory and a second engine built afterwards reuses the pooled SM partition."""
     dtype = torch.float16

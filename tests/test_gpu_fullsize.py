@@ -1,4 +1,4 @@
-"""Parity at the HEADLINE shape (SURVEY §8d "parity workload"): the real 32-layer, vocab-128256
+"""Parity at the headline shape: the real 32-layer, vocab-128256
 Llama-3-8B with `--load-format dummy` weights generated on the device, one prompt of 128 tokens and
 8 greedy steps, against the CPU oracle on the SAME 16-bit weights (copied off the device).
 
@@ -8,8 +8,8 @@ Two yardsticks:
     1.3e-2 .. 1.8e-2 per forward — above the 1e-2 that the 2-layer models of test_gpu_model.py
     meet, because 32 layers of fp16 activations (one rounding per op boundary, the reference's
     arithmetic as well) accumulate ~4 fp16 ulps on logits of magnitude ~7;
-  * the reference's own arithmetic, `compute="native"` (torch-eager CPU in fp16, BASELINE.json's
-    "torch-eager CPU forward"): its distance from the fp32 oracle is the error the reference
+  * the reference's own arithmetic, `compute="native"` (a torch-eager CPU
+    forward in fp16): its distance from the fp32 oracle is the error the reference
     itself carries at this depth.  The CUDA path must not be less accurate than that (factor 2
     for the independent random walks of two different summation orders), with 3e-2 as the
     absolute bound stated for fp16 at 32 layers."""

@@ -1,5 +1,5 @@
 """End-to-end parity of the CUDA path (through ModelRunner.forward, i.e. through the C-ABI) with
-the CPU oracle on identical synthetic weights and inputs.  Criterion (BASELINE.json north_star):
+the CPU oracle on identical synthetic weights and inputs.  Criterion:
 max-abs(logits_gpu - logits_cpu_fp32) < 1e-2 in fp16, greedy ids exact where the oracle's
 top-1/top-2 margin exceeds 2e-2.  bf16 is held to 6e-2 (its 8-bit mantissa alone moves O(1)
 logits by ~2^-8 per rounding point)."""
@@ -13,10 +13,10 @@ pytestmark = pytest.mark.gpu
 
 TINY = dict(hidden_size=256, intermediate_size=512, num_hidden_layers=2, num_attention_heads=4,
             num_key_value_heads=2, head_dim=128, vocab_size=1024, max_position_embeddings=2048)
-# Llama-3-8B head / FFN shapes, 2 layers, small vocab (SURVEY §8d "exhaustive parity" model)
+# Llama-3-8B head / FFN shapes, 2 layers, small vocab (exhaustive parity)
 L8B2 = dict(hidden_size=4096, intermediate_size=14336, num_hidden_layers=2, num_attention_heads=32,
             num_key_value_heads=8, head_dim=128, vocab_size=4096, max_position_embeddings=4096)
-# what ONE RANK of Llama-3-70B at TP = 8 runs (BASELINE configs[4]): 64 / 8 = 8 query heads over
+# what ONE RANK of Llama-3-70B at TP = 8 runs: 64 / 8 = 8 query heads over
 # 8 / 8 = 1 kv head, hidden 8192, 28672 / 8 = 3584 FFN columns — the GEMM / attention shapes the
 # 8-GPU arm of bench.py launches, checked here on one GPU as a 2-layer model of that geometry
 # (the cross-rank sum itself is covered by tests/test_gpu_tp.py and bench.py's tp_parity)

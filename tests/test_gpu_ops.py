@@ -404,7 +404,7 @@ def test_attention_on_reference_golden_vectors(ops, golden):
 
 
 def test_attn_properties_full_size(ops):
-    """Size-independent properties at BASELINE sizes (Llama-3-8B heads, B = 64, S ≈ 1088):
+    """Size-independent properties at the benchmark's sizes (Llama-3-8B heads, B = 64, S ≈ 1088):
     (1) tcgen05 == SIMT kernel on the same inputs; (2) softmax convexity: every output lies inside
     [min V, max V] of its kv head; (3) permuting the slot assignment (a different page table over
     the same logical sequence) does not change the result."""

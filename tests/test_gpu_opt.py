@@ -1,4 +1,4 @@
-"""opt-125m single-prompt greedy decode — plumbing + logit check.
+"""opt-125m: single-prompt greedy decode — plumbing + logit check.
 CUDA path (libspd: GEMM, LayerNorm, bias/ReLU/residual, SIMT attention at head_dim 64, greedy
 sampling, paged KV pool) vs the HF-transformers fp32 oracle on identical fp16 weights."""
 import pytest
@@ -31,7 +31,7 @@ def test_opt125m_greedy_decode_matches_hf(cuda_graph):
     mr, weights = _runner(cuda_graph)
     oracle = OptOracle(opt125m_config(), weights)
     gs = GpuSession(mr)
-    prompt = [(7 + 13 * i) % 50272 for i in range(16)]  # SURVEY §8d config 1
+    prompt = [(7 + 13 * i) % 50272 for i in range(16)]
     reqs, logits, ids = gs.extend([prompt])
     seq = list(prompt)
     worst = 0.0
@@ -44,7 +44,7 @@ def test_opt125m_greedy_decode_matches_hf(cuda_graph):
         tok = int(ref.argmax(-1)[0])
         seq.append(tok)
         logits, ids = gs.decode(reqs, [tok])
-    assert worst < 1e-2, worst  # fp16, max-abs logit error (north_star tolerance)
+    assert worst < 1e-2, worst  # fp16, max-abs logit error
 
 
 def test_opt_elementwise_ops_match_torch():
