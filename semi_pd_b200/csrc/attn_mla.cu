@@ -7,8 +7,9 @@
 // (layers/attention/triton_ops/decode_attention.py:235-470, extend_attention.py:291-410): all H
 // query heads share ONE latent K/V stream (MQA), K = the whole latent row (DL = kv_lora + rope),
 // V = its first DV = kv_lora columns.  The reference switches to a plain MHA (forward_normal) for
-// prefill batches without a cached prefix; the absorbed form used here for every batch is the same
-// function of the same inputs (oracle/deepseek_oracle.py checks both against each other).
+// prefill batches without a cached prefix; the absorbed form, the same function of the same inputs
+// (oracle/deepseek_oracle.py checks both against each other), serves decode here and the prefill
+// batches for which expanded heads (attn_mla_prefill.cu) would not be faster.
 //
 // Swap-AB formulation: an item is TQ query tokens x 16 heads = N columns (decode: 1 x 16, extend: 4 x 16),
 //     S^T[64 kv x N]  = K_tile[64 x 576] * Q^T           (36 MMAs, M = 64)
@@ -33,7 +34,8 @@
 // Decode streams each latent row once, 64 requests of 1088 keys (83 MB) in 34 us with the merge launch; one CTA per token,
 // head group and split with warp-level MMAs took 62 us.  About 9000 clk pass until the first tile has landed, then 3000 clk
 // per 72 KB tile and SM.  MMAs (M = 64: 23 clk at N = 16, 31 at N = 64) are hidden as long as the issuer's code stays a
-// short loop.  Extend, 4096 new tokens in 4 requests (two with 515 cached), whole layer: 1645 -> 600 us; bounded by the
+// short loop.  Extend, 4096 new tokens in 4 requests (two with 515 cached), whole layer: 1645 -> 600 us (a batch that takes
+// expanded heads now: 185 us); bounded by the
 // ring of two tiles (a tile's copies start when the PV before last has finished), by the rescale of O^T whenever a tile
 // raises one of 64 columns, and by beginning and ending items, which therefore count in the split (without that, SMs with
 // short items took twice as long).

@@ -6,7 +6,8 @@
 // prefill batches without a cached prefix; here it serves prefixes as well, as long as a latent row is met by enough
 // queries to pay for its expansion.  The absorbed form (attn_mla.cu) needs 1088 multiply-adds per query, key and head and
 // this one 320, plus 131072 per key and head.  4096 new tokens in 4 requests, two of them behind 515 cached tokens, 16
-// heads, whole attention layer: 606 us absorbed, 166 here (this kernel 67, the rows 6, the GEMM 26).
+// heads, whole attention layer called after other work: 606 us absorbed, 185 here; warm and alone this kernel 67, the rows 6, the
+// expanding GEMM 26.
 //
 // Items are two consecutive 128-query tiles of one head that share every K / V tile of 64 keys, one tile per softmax
 // warpgroup; they are dealt to one persistent CTA per SM by weight (tile_list).  Roles as in attn_prefill.cu (384 threads):

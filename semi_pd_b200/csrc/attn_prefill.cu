@@ -25,7 +25,7 @@
 //                    P never touches shared memory: the 16-bit probabilities are written back
 //                    into TMEM over the first 32 columns of the S half they came from
 //                    (tcgen05.st) and feed the PV MMA as its A operand from TMEM;
-//                    epilogue O / l straight from TMEM to global memory;
+//                    epilogue O / l from TMEM through shared memory and TMA stores (a ragged last tile: from registers);
 //   warp 8, warp 9   K / V loader into 128-byte-swizzled smem; one 4-slot ring K_j V_j K_{j+1} ...
 //                    runs ahead of the consumer ACROSS items, so an item's first tiles are in
 //                    flight while the previous item drains.  A tile whose 128 page-table entries
@@ -38,15 +38,15 @@
 //                    P(j,h) lives in; tcgen05.mma executes in order).  The next item's Q tile is fetched (TMA) when the
 //                    item's last S is complete.
 // The issuers' own time bounded the kernel while one lane of one warp issued for both warpgroups from unrolled code: 65 clk
-// per MMA and 250 between two units.  Whole warps with uniform operands, short loops and an issuer per warpgroup: 8
-// requests of 1024 new tokens on average, half of them behind 1024 cached ones, 32 / 8 heads: 193 -> 176 us; 4 requests
-// of 2048, 16 / 4 heads, window 1024: 142 -> 132 us.  Slower: S issued 128 keys wide with softmax and PV still per half and
+// per MMA and 250 between two units.  Whole warps with uniform operands, short loops and an issuer per warpgroup (warm, the
+// kernel alone): 8 requests of 1024 new tokens on average, half of them behind 1024 cached ones, 32 / 8 heads: 193 -> 176 us;
+// 4 requests of 2048, 16 / 4 heads, window 1024: 142 -> 132 us.  Slower: S issued 128 keys wide with softmax and PV still per half and
 // one issuer (160 / 128 us against 156 / 112 with the sorted items), or with two (250 us: both warpgroups in one phase).
 // With an issuer each nothing keeps the warpgroups apart, and on half of the CTAs they fell into one phase: warpgroup 1
 // starts every item behind warpgroup 0 (`turn`).  64 requests of 128 tokens, 32 / 8 heads: 36.1 us with one issuer, 41.5 with
 // two, 36.2 here; 8 of 1024: 80.1, 82.8, 80.9; 16 of 500: 58.0, 62.1, 61.4 (of unequal lengths 96, 75, 75).
 // Items are ordered heaviest first (pf_sort) and dealt to the CTAs in snake order.
-// smem: Q0 Q1 + 5 K/V slots = 7 x 32 KB.  TMEM: S0a/P0a S0b/P0b | S1a/P1a S1b/P1b | O0 | O1 = 512 columns.
+// smem: Q0 Q1 + 4 K/V slots + output staging = 7 x 32 KB, the list of tiles.  TMEM: S0a/P0a S0b/P0b | S1a/P1a S1b/P1b | O0 | O1 = 512 columns.
 #include <cuda.h>
 
 #include "common.cuh"
@@ -261,8 +261,8 @@ __device__ __noinline__ float2 pf_row_alone(const T* q, const T* k_pool, const T
 
 // kWin: a sliding window (KV tiles before the item's first visible key are skipped), sinks and a query temperature — the
 // general attention of the hybrid families at head size 128 (see spd::attn_prefill_window_try).
-// 4 requests of 2048 new tokens, 16 / 4 heads, window 1024: 320 us on warp-level MMAs with 64 x 64 tiles, 140 us here
-// (60 GFLOP visible; a query tile of 128 meets nine key tiles, two of them masked).
+// 4 requests of 2048 new tokens, 16 / 4 heads, window 1024: 320 us on warp-level MMAs with 64 x 64 tiles, 101 us here,
+// warm (60 GFLOP visible; a query tile of 128 meets nine key tiles, two of them masked).
 template <typename T, bool kTrace, bool kWin>
 __global__ void __launch_bounds__(kPfThreads, 1)
 attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -731,25 +731,25 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           l += softmax_unit<T>(ra, rb, pk, scale, (m_used == -INFINITY) ? 0.f : m_used * scale);
         } else {
           if (jh == 0)  // first unit of the item: establish the reference max with a max-only pre-pass
-            m_used = need_mask ? softmax_row_max<true, kWin>(tsh, kv0, limit, span)
-                               : softmax_row_max<false, kWin>(tsh, kv0, limit, span);
+            m_used = need_mask ? softmax_row_max<true>(tsh, kv0, limit)
+                               : softmax_row_max<false>(tsh, kv0, limit);
           float m_off = (m_used == -INFINITY) ? 0.f : m_used * scale;
-          float psum = need_mask ? softmax_row_pass<T, true, kWin>(tsh, pk, scale, m_off, kv0, limit, span)
-                                 : softmax_row_pass<T, false, kWin>(tsh, pk, scale, m_off, kv0, limit, span);
+          float psum = need_mask ? softmax_row_pass<T, true>(tsh, pk, scale, m_off, kv0, limit)
+                                 : softmax_row_pass<T, false>(tsh, pk, scale, m_off, kv0, limit);
           // raise the reference max only when some row may have outgrown it by > 2^8 (an element
           // above 2^8 implies a row sum above 2^8; warp-uniform decision: tcgen05.ld/st are
           // warp-collective); S is still intact (P is stored below), so the unit is simply redone
           if (__any_sync(0xffffffffu, psum > kRescaleTrigger)) {
-            const float mx = need_mask ? softmax_row_max<true, kWin>(tsh, kv0, limit, span)
-                                       : softmax_row_max<false, kWin>(tsh, kv0, limit, span);
+            const float mx = need_mask ? softmax_row_max<true>(tsh, kv0, limit)
+                                       : softmax_row_max<false>(tsh, kv0, limit);
             const float m_new = fmaxf(m_used, mx);
             alpha = (m_used == -INFINITY) ? 0.f : fast_exp2((m_used - m_new) * scale);
             l *= alpha;
             m_used = m_new;
             m_off = (m_used == -INFINITY) ? 0.f : m_used * scale;
             if (jh > 0) rescale_o(alpha, u);
-            psum = need_mask ? softmax_row_pass<T, true, kWin>(tsh, pk, scale, m_off, kv0, limit, span)
-                             : softmax_row_pass<T, false, kWin>(tsh, pk, scale, m_off, kv0, limit, span);
+            psum = need_mask ? softmax_row_pass<T, true>(tsh, pk, scale, m_off, kv0, limit)
+                             : softmax_row_pass<T, false>(tsh, pk, scale, m_off, kv0, limit);
           }
           l += psum;
         }

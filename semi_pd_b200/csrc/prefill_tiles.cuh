@@ -156,9 +156,9 @@ __device__ __forceinline__ bool pf_visible(int kv, int limit, int span) {
 // 32 columns of one tile row: p = exp2(s*scale - m_off), packed to 16 bits into pk[0..16), and their sum.
 // kRound: the sum of the rounded p, the weights that the products use: sum(p v) / sum(p) is then a true mean of the v, and
 // the rounding of a p that outweighs the others cancels.
-template <typename T, bool kMask, bool kWin, bool kRound = false>
+template <typename T, bool kMask, bool kRound>
 __device__ __forceinline__ void softmax_chunk(const uint32_t* r, int c, uint32_t* pk, uint64_t scale2,
-                                              uint64_t neg_m2, int kv0, int limit, int span, uint64_t& ps) {
+                                              uint64_t neg_m2, int kv0, int limit, uint64_t& ps) {
 #pragma unroll
   for (int i = 0; i < 32; i += 2) {
     float x0, x1;
@@ -166,8 +166,8 @@ __device__ __forceinline__ void softmax_chunk(const uint32_t* r, int c, uint32_t
     float p0 = fast_exp2(x0);
     float p1 = fast_exp2(x1);
     if constexpr (kMask) {
-      p0 = pf_visible<kWin>(kv0 + c + i, limit, span) ? p0 : 0.f;
-      p1 = pf_visible<kWin>(kv0 + c + i + 1, limit, span) ? p1 : 0.f;
+      p0 = kv0 + c + i <= limit ? p0 : 0.f;
+      p1 = kv0 + c + i + 1 <= limit ? p1 : 0.f;
     }
     pk[i >> 1] = pack2<T>(p0, p1);
     if constexpr (kRound) {
@@ -184,9 +184,9 @@ __device__ __forceinline__ void softmax_chunk(const uint32_t* r, int c, uint32_t
 // loads are in flight while the previous 32 columns are exponentiated.  kMask is a template
 // parameter so that the unmasked units run the lean loop: FFMA + MUFU.EX2 + FADD + half an F2FP
 // per element.
-template <typename T, bool kMask, bool kWin, bool kRound = false>
+template <typename T, bool kMask>
 __device__ __forceinline__ float softmax_row_pass(uint32_t ts, uint32_t* pk, float scale_log2, float m_off,
-                                                  int kv0, int limit, int span) {
+                                                  int kv0, int limit) {
   const uint64_t scale2 = pack_f32x2(scale_log2, scale_log2);
   const uint64_t neg_m2 = pack_f32x2(-m_off, -m_off);
   uint64_t ps = pack_f32x2(0.f, 0.f);
@@ -194,8 +194,8 @@ __device__ __forceinline__ float softmax_row_pass(uint32_t ts, uint32_t* pk, flo
   tmem_ld_32x32b_x32(ts, ra);
   tmem_ld_32x32b_x32(ts + 32, rb);
   tmem_ld_wait();
-  softmax_chunk<T, kMask, kWin, kRound>(ra, 0, pk, scale2, neg_m2, kv0, limit, span, ps);
-  softmax_chunk<T, kMask, kWin, kRound>(rb, 32, pk + 16, scale2, neg_m2, kv0, limit, span, ps);
+  softmax_chunk<T, kMask, false>(ra, 0, pk, scale2, neg_m2, kv0, limit, ps);
+  softmax_chunk<T, kMask, false>(rb, 32, pk + 16, scale2, neg_m2, kv0, limit, ps);
   float ps0, ps1;
   unpack_f32x2(ps, ps0, ps1);
   return ps0 + ps1;
@@ -226,8 +226,8 @@ __device__ __forceinline__ float softmax_unit(const uint32_t* ra, const uint32_t
   const uint64_t scale2 = pack_f32x2(scale_log2, scale_log2);
   const uint64_t neg_m2 = pack_f32x2(-m_off, -m_off);
   uint64_t ps = pack_f32x2(0.f, 0.f);
-  softmax_chunk<T, false, false, true>(ra, 0, pk, scale2, neg_m2, 0, 0, 0, ps);
-  softmax_chunk<T, false, false, true>(rb, 32, pk + 16, scale2, neg_m2, 0, 0, 0, ps);
+  softmax_chunk<T, false, true>(ra, 0, pk, scale2, neg_m2, 0, 0, ps);
+  softmax_chunk<T, false, true>(rb, 32, pk + 16, scale2, neg_m2, 0, 0, ps);
   float ps0, ps1;
   unpack_f32x2(ps, ps0, ps1);
   return ps0 + ps1;
@@ -259,28 +259,28 @@ __device__ __forceinline__ void rescale_row128(uint32_t to, float alpha) {
 constexpr float kRescaleTrigger = 256.f;  // a row sum above 2^8 may hide an element above 2^8
 
 // max of the visible raw scores of one row of an S unit (TMEM)
-template <bool kMask, bool kWin>
-__device__ __forceinline__ void rowmax_chunk(const uint32_t* r, int c, int kv0, int limit, int span, float& m0, float& m1) {
+template <bool kMask>
+__device__ __forceinline__ void rowmax_chunk(const uint32_t* r, int c, int kv0, int limit, float& m0, float& m1) {
 #pragma unroll
   for (int i = 0; i < 32; i += 2) {
     float a = __uint_as_float(r[i]), b = __uint_as_float(r[i + 1]);
     if constexpr (kMask) {
-      a = pf_visible<kWin>(kv0 + c + i, limit, span) ? a : -INFINITY;
-      b = pf_visible<kWin>(kv0 + c + i + 1, limit, span) ? b : -INFINITY;
+      a = kv0 + c + i <= limit ? a : -INFINITY;
+      b = kv0 + c + i + 1 <= limit ? b : -INFINITY;
     }
     m0 = fmaxf(m0, a);
     m1 = fmaxf(m1, b);
   }
 }
-template <bool kMask, bool kWin>
-__device__ __forceinline__ float softmax_row_max(uint32_t ts, int kv0, int limit, int span) {
+template <bool kMask>
+__device__ __forceinline__ float softmax_row_max(uint32_t ts, int kv0, int limit) {
   float m0 = -INFINITY, m1 = -INFINITY;
   uint32_t ra[32], rb[32];
   tmem_ld_32x32b_x32(ts, ra);
   tmem_ld_32x32b_x32(ts + 32, rb);
   tmem_ld_wait();
-  rowmax_chunk<kMask, kWin>(ra, 0, kv0, limit, span, m0, m1);
-  rowmax_chunk<kMask, kWin>(rb, 32, kv0, limit, span, m0, m1);
+  rowmax_chunk<kMask>(ra, 0, kv0, limit, m0, m1);
+  rowmax_chunk<kMask>(rb, 32, kv0, limit, m0, m1);
   return fmaxf(m0, m1);
 }
 

@@ -234,10 +234,10 @@ retention_chunked_kernel(const __grid_constant__ RetChunkParams p) {
   extern __shared__ uint8_t rc_smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(rc_smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
-  uint8_t* sQ = smem;               // 3 parts; A's three parts once Q has been read
+  uint8_t* sQ = smem;               // 3 parts
   uint8_t* sK = sQ + 3 * kRcQ;      // 3 parts
   uint8_t* sS = sK + 3 * kRcQ;      // 3 parts
-  uint8_t* sW = sS + 3 * kRcS;      // 3 parts of v'
+  uint8_t* sW = sS + 3 * kRcS;      // 3 parts of v'; A's three parts once K^T V' has been read
   uint8_t* sV = sW + 3 * kRcV;      // VS parts of v
   T* rq = reinterpret_cast<T*>(sV + VS * kRcV);  // raw rows of the next chunk: q, k [64][128], v [64][64]
   T* rk = rq + kRcTok * kRcDk;
