@@ -516,6 +516,10 @@ def mla_gather(kv_pool: torch.Tensor, req_to_token: torch.Tensor, req_pool_indic
         raise RuntimeError("mla_gather: the pool is contiguous rows of kv_lora + rope")
     if any(t.numel() != B or t.dtype != torch.int32 or not t.is_contiguous() for t in (prefix_lens, extend_lens)):
         raise RuntimeError("mla_gather: prefix_lens and extend_lens are int32, one per request")
+    if req_pool_indices.dtype != torch.int64 or not req_pool_indices.is_contiguous():
+        raise RuntimeError("mla_gather: req_pool_indices are int64, contiguous")
+    if req_to_token.dtype != torch.int32 or req_to_token.dim() != 2 or req_to_token.stride(1) != 1:
+        raise RuntimeError("mla_gather: req_to_token is int32 with contiguous rows")
     rows = torch.empty(total_kv, DL, device=kv_pool.device, dtype=kv_pool.dtype)
     start = torch.empty(B, device=kv_pool.device, dtype=torch.int32)
     check(lib.spd_mla_gather(rows.data_ptr(), start.data_ptr(), kv_pool.data_ptr(), req_to_token.data_ptr(),

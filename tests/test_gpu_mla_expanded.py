@@ -116,3 +116,20 @@ def test_rotated_queries_in_place(dtype):
     assert torch.equal(heads(inplace)[..., NOPE:], q_lat.view(T, H, R + DR)[..., R:])
     assert torch.equal(heads(inplace)[..., :NOPE], heads(qa)[..., :NOPE])
     assert torch.equal(inplace[:, H * (NOPE + DR):], qa[:, H * (NOPE + DR):])
+
+
+def test_gather_refuses_what_it_would_read_wrongly():
+    from semi_pd_b200 import ops
+    pool = torch.randn(65, 1, R + DR, device=DEV).bfloat16()
+    rtt, idx = torch.arange(64, dtype=torch.int32, device=DEV).view(2, 32), torch.tensor([1, 0], device=DEV)
+    lens = torch.tensor([3, 5], dtype=torch.int32, device=DEV)
+
+    def call(rtt=rtt, idx=idx, pre=lens, ext=lens):
+        return ops.mla_gather(pool, rtt, idx, pre, ext, 16, 10, R, DR)
+
+    rows, start = call()
+    assert start.tolist() == [0, 6] and torch.equal(rows, pool[torch.cat((rtt[1, :6], rtt[0, :10])).long(), 0])
+    for wrong in (dict(idx=idx.int()), dict(idx=torch.tensor([[1, 5], [0, 5]], device=DEV)[:, 0]), dict(rtt=rtt.long()),
+                  dict(rtt=rtt.T), dict(rtt=rtt.flatten()), dict(pre=lens.long()), dict(ext=lens[:1])):
+        with pytest.raises(RuntimeError, match="mla_gather"):
+            call(**wrong)
