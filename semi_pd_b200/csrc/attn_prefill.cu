@@ -32,7 +32,8 @@
 //                    are consecutive slots (what the run allocator produces, memory_pool.py) is a
 //                    strided 2-D box of the pool and is fetched with two TMA tensor copies by one
 //                    lane; any other tile (scattered slots, the ragged tail of a sequence) is
-//                    gathered row by row through req_to_token with 16-byte cp.async;
+//                    gathered row by row through req_to_token with 16-byte cp.async, whose completion arrives on
+//                    the slot's barrier by itself;
 //   warp 10, warp 11 MMA issuer of warpgroup 0 / 1: S_h = Q K_j[h]^T (both K-major in smem), O += P_h V_j[h] (P
 //                    from TMEM, V MN-major in smem); the order is PV(j,h) then S(j+1,h) (which overwrites the columns
 //                    P(j,h) lives in; tcgen05.mma executes in order).  The next item's Q tile is fetched (TMA) when the
@@ -44,7 +45,7 @@
 // one issuer (160 / 128 us against 156 / 112 with the sorted items), or with two (250 us: both warpgroups in one phase).
 // With an issuer each nothing keeps the warpgroups apart, and on half of the CTAs they fell into one phase: warpgroup 1
 // starts every item behind warpgroup 0 (`turn`).  64 requests of 128 tokens, 32 / 8 heads: 36.1 us with one issuer, 41.5 with
-// two, 36.2 here; 8 of 1024: 80.1, 82.8, 80.9; 16 of 500: 58.0, 62.1, 61.4 (of unequal lengths 96, 75, 75).
+// two, 36.2 here; 8 of 1024: 80.1, 82.8, 80.9; 16 of 500: 58.0, 62.1, 60.4 (of unequal lengths 96, 75, 74).
 // Items are ordered heaviest first (pf_sort) and dealt to the CTAs in snake order.
 // smem: Q0 Q1 + 4 K/V slots + output staging = 7 x 32 KB, the list of tiles.  TMEM: S0a/P0a S0b/P0b | S1a/P1a S1b/P1b | O0 | O1 = 512 columns.
 #include <cuda.h>
@@ -374,6 +375,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       auto issue_s = [&](int j, int h) {
         const uint32_t pos = 2 * (t_base + j - it.j0);
         mbar_wait(&kv_full[pos % kPfSlots], (pos / kPfSlots) & 1);
+        if (h == 0) fence_proxy_async_smem();
         tc_fence_after_sync();
         uint32_t qa = static_cast<uint32_t>(qd);
         uint32_t ka = static_cast<uint32_t>(kd0) + (pos % kPfSlots) * (kTileBytes / 16) + h * (kU * 128 / 16);
@@ -429,6 +431,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             mbar_wait(&p_full[w * 2 + h], (pq / kNU) & 1);
             pf_trace<kTrace>(p, 2 + w, tn, 0x200 + w * 2 + h);  // P ready
             mbar_wait(&kv_full[vpos % kPfSlots], (vpos / kPfSlots) & 1);
+            if (h == 0) fence_proxy_async_smem();
             if (j == it.j0 && h == 0) mbar_wait(&o_free[w], (eq & 1) ^ 1);  // previous item's O has been read
             tc_fence_after_sync();
             uint32_t va = static_cast<uint32_t>(vd0) + (vpos % kPfSlots) * (kTileBytes / 16) + h * (kU * 128 / 16);
@@ -465,7 +468,6 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     const T* pool = reinterpret_cast<const T*>(is_v ? p.v_pool : p.k_pool);
     const int64_t row_elems = static_cast<int64_t>(p.Hk) * kPfD;
     uint32_t t = 0;        // tiles loaded so far (all items)
-    int pending = -1;      // slot whose cp.async group is committed but not yet published
     int idx = pf_rank(0, cta, ncta);
     PfRaw raw = pf_raw(p, pl, idx);
     for (int k = 0; idx < pl.items; ++k) {
@@ -493,17 +495,6 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         const uint32_t pos = 2 * t + is_v;
         const int st = pos % kPfSlots;
         const uint32_t epar = ((pos / kPfSlots) & 1) ^ 1;
-        // Keep two tiles in flight when the ring has room.  If this tile's slot is still in use,
-        // publish the previous tile BEFORE blocking on the slot: the consumer of the previous
-        // tile must never wait on a producer that waits on the consumer.
-        bool publish_after = true;
-        if (pending >= 0 && !mbar_try_wait(&kv_empty[st], epar)) {
-          cp_async_wait<0>();
-          fence_proxy_async_smem();
-          mbar_arrive(&kv_full[pending]);
-          pending = -1;
-          publish_after = false;
-        }
         mbar_wait(&kv_empty[st], epar);
         if (contig) {
           // TMA: rows base .. base+127 of the pool, the 128 columns of kv head hk, as the slot's
@@ -518,12 +509,6 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           }
           __syncwarp();
           mbar_arrive(&kv_full[st]);
-          if (pending >= 0) {  // a gathered tile is still unpublished: no later group will cover it
-            cp_async_wait<0>();
-            fence_proxy_async_smem();
-            mbar_arrive(&kv_full[pending]);
-            pending = -1;
-          }
           continue;
         }
         const uint32_t dst = smem_u32(sKV + st * kTileBytes);
@@ -534,19 +519,12 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           const int64_t s64 = valid ? slot[i] : 0;
           cp_async16(dst + tile_off(row, chunk), pool + s64 * row_elems + col, valid);
         }
-        cp_async_commit();
-        if (publish_after && pending >= 0) {
-          cp_async_wait<1>();  // everything but the group just committed has landed
-          fence_proxy_async_smem();
-          mbar_arrive(&kv_full[pending]);
-        }
-        pending = st;
+        // each lane's arrival comes when its copies have landed: nothing here waits for them, and the next tile's lookups
+        // and copies follow at once.  (The MMA issuers, who read what these wrote, fence between the two proxies.)  Handed
+        // over by the loader, a tile waited for the next one's page-table lookups: 40 portions of 16 tokens 25.3 -> 23.7 us,
+        // 16 of 500 61.4 -> 60.4, 8 of 250 18.1 -> 17.4.
+        cp_async_mbar_arrive_noinc(&kv_full[st]);
       }
-    }
-    if (pending >= 0) {
-      cp_async_wait<0>();
-      fence_proxy_async_smem();
-      mbar_arrive(&kv_full[pending]);
     }
   } else {
     // ===================== softmax warpgroups (one thread per query row) =====================
