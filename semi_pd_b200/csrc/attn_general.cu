@@ -586,8 +586,8 @@ pool_key_blocks_kernel(T* __restrict__ k_pool, T* __restrict__ v_pool, const int
 // 15.9, after 3000, window 64 18.3 / 21.4, 12 x 129 15.7 / 12.2; more with one head a group, whose items hold two of the tiles
 // (8 heads, [140] + 31 x [64] 11.7 / 13.7); less from windows of 256 on, where most keys are the prefixes' ([129] + 15 x [1]
 // after 3000, 16 heads of 4 29.3 / 24.5; 64 x 129 or 1 without prefixes 25.4 / 25.7).
-// The SMs are the caller's.  Counted against the device's on a partition of 40: 1 x 500, 16 heads, window 512 37.8 / 16.7 us, 4 x 200
-// after 1500, window 128 39.6 / 20.7; of 72: 1 x 500, 16 heads, window 512 27.3 / 16.9.
+// The SMs are the caller's.  Counted against the device's, on a partition of 40 SMs mma.sync took 1 x 500, 16 heads, window
+// 512 (37.8 / 16.7 us) and 4 x 200 after 1500, window 128 (39.6 / 20.7); on 72 1 x 500, 16 heads, window 512 (27.3 / 16.9).
 inline bool window_tc_wins(int64_t batch, int64_t tokens, int64_t ext, int heads, int groups, int window, int64_t sms) {
   if (ext <= 128) return false;
   if (window <= 0) window = 1 << 30;

@@ -41,13 +41,14 @@
 // The issuers' own time bounded the kernel while one lane of one warp issued for both warpgroups from unrolled code: 65 clk
 // per MMA and 250 between two units.  Whole warps with uniform operands, short loops and an issuer per warpgroup (warm, the
 // kernel alone): 8 requests of 1024 new tokens on average, half of them behind 1024 cached ones, 32 / 8 heads: 193 -> 176 us;
-// 4 requests of 2048, 16 / 4 heads, window 1024: 142 -> 132 us.  Slower: S issued 128 keys wide with softmax and PV still per half and
-// one issuer (160 / 128 us against 156 / 112 with the sorted items), or with two (250 us: both warpgroups in one phase).
+// 4 requests of 2048, 16 / 4 heads, window 1024: 142 -> 132 us.  Slower: S issued 128 keys wide with softmax and PV still
+// per half and one issuer (160 / 128 us against 156 / 112 with the sorted items), or with two (250 us: both warpgroups in one phase).
 // With an issuer each nothing keeps the warpgroups apart, and on half of the CTAs they fell into one phase: warpgroup 1
 // starts every item behind warpgroup 0 (`turn`).  64 requests of 128 tokens, 32 / 8 heads: 36.1 us with one issuer, 41.5 with
 // two, 36.2 here; 8 of 1024: 80.1, 82.8, 80.9; 16 of 500: 58.0, 62.1, 60.4 (of unequal lengths 96, 75, 74).
 // Items are ordered heaviest first (pf_sort) and dealt to the CTAs in snake order.
-// smem: Q0 Q1 + 4 K/V slots + output staging = 7 x 32 KB, the list of tiles.  TMEM: S0a/P0a S0b/P0b | S1a/P1a S1b/P1b | O0 | O1 = 512 columns.
+// smem: Q0 Q1 + 4 K/V slots + output staging = 7 x 32 KB, the list of tiles.
+// TMEM: S0a/P0a S0b/P0b | S1a/P1a S1b/P1b | O0 | O1 = 512 columns.
 #include <cuda.h>
 
 #include "common.cuh"

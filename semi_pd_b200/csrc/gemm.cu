@@ -605,11 +605,12 @@ int get_tmap(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, u
 }
 
 // How many CTAs (or pairs) a stream-K call cuts its units (tiles x k-blocks) over, of `slots` that run at once: as many as
-// leave a tile about `split` contributors (every partial is read once more) and a share 4 k-blocks.  Long rows in few tiles
-// leave most of the slots idle that way; a share of 64 k-blocks then pays whatever the tile's length, up to a quarter of the
-// slots in use, and one of 96 up to half of them.  Pairs, 40 / 160 tokens, us: 1 tile of 448 k-blocks 4 pairs 24 / 32, 7 pairs 18 / 30;
-// 4 x 1408 (16, 74) 61 / 76, 40 / 62; 8 x 1408 (32, 74) 69 / 83, 62 / 78; 8 x 1024 (32, 74) 51 / 62, 49 / 62.  No gain: 8 x 512 (32, 64)
-// 29 / 38, 29 / 39; 12 x 448 (48, 74) 31 / 40, 32 / 43; 16 x 448 (64, 74) 39 / 47, 39 / 49, 256 tokens 58, 61; 4 x 272 (16, 17) 18 / 25, 18 / 26.
+// leave a tile about `split` contributors (every partial is read once more) and a share 4 k-blocks.  Long rows in few
+// tiles leave most of the slots idle that way; a share of 64 k-blocks then pays whatever the tile's length, up to a quarter
+// of the slots in use, and one of 96 up to half of them.  tiles x k-blocks: pairs, 40 / 160 tokens in us:
+//   1 x 448: 4 24 / 32, 7 18 / 30;  4 x 1408: 16 61 / 76, 74 40 / 62;  8 x 1408: 32 69 / 83, 74 62 / 78;
+//   8 x 1024: 32 51 / 62, 74 49 / 62.  No gain: 8 x 512: 32 29 / 38, 64 29 / 39;  12 x 448: 48 31 / 40, 74 32 / 43;
+//   16 x 448: 64 39 / 47, 74 39 / 49;  4 x 272: 16 18 / 25, 17 18 / 26.
 long long streamk_ctas(long long tiles, int kblocks, int split, long long slots) {
   const long long units = tiles * kblocks, base = kblocks / split > 4 ? kblocks / split : 4;
   auto ctas = [&](long long share) { return units / slots >= share ? slots : units / share > 0 ? units / share : 1; };
@@ -700,8 +701,9 @@ int spd_gemm(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_
 
   // stream-K grid: equal unit ranges (streamk_ctas).  Tuning knobs (experiments only):
   // SPD_GEMM_STREAMK=0 disables stream-K, =2 forces it; SPD_GEMM_SPLIT=d aims at ~d contributors per
-  // tile where that does not leave most SMs idle; SPD_GEMM_SWAPMAX=m is the largest M routed to swap-AB; SPD_GEMM_CLUSTER=1 routes few-tile layers at M <= 128 to the cluster
-  // split-K kernel (gemm_cluster.cu) instead.
+  // tile where that does not leave most SMs idle; SPD_GEMM_SWAPMAX=m is the largest M routed to
+  // swap-AB; SPD_GEMM_CLUSTER=1 routes few-tile layers at M <= 128 to the cluster split-K kernel
+  // (gemm_cluster.cu) instead.
   static const int env_streamk = getenv("SPD_GEMM_STREAMK") ? atoi(getenv("SPD_GEMM_STREAMK")) : 1;
   static const int env_split = getenv("SPD_GEMM_SPLIT") ? atoi(getenv("SPD_GEMM_SPLIT")) : 4;
   static const int env_swapmax = getenv("SPD_GEMM_SWAPMAX") ? atoi(getenv("SPD_GEMM_SWAPMAX")) : 256;
