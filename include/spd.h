@@ -185,8 +185,12 @@ int64_t spd_gemm_workspace_bytes(void);
 /* CTAs (pairs of CTAs) over which a decode GEMM that splits along K cuts its tiles x kblocks units, of `slots` that run at
  * once; split: contributors per tile that it aims at (4). */
 int64_t spd_gemm_streamk_ctas(int64_t tiles, int kblocks, int split, int64_t slots);
-/* Columns (256, 224, 192) of the tiles on CTA pairs that a GEMM of these sizes takes; 0: tiles of one CTA. */
+/* Columns (256, 224, 192) of the tiles of 256 token rows on CTA pairs that a GEMM of these sizes takes, 0: tiles of one CTA —
+ * where it does not take tiles of 256 weight rows: */
 int spd_gemm_pair_cols(int64_t M, int64_t N, int64_t K, int epilogue, int sm_budget);
+/* Token rows of the widest of the tiles with 256 weight rows that a GEMM of these sizes with 16-bit results takes, 0: the
+ * tiles above. */
+int spd_gemm_swap_rows(int64_t M, int64_t N, int64_t K, int epilogue, int sm_budget);
 int spd_gemm(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_t K, int64_t lda,
              int64_t ldw, int64_t ldc, int dtype, int out_f32, int epilogue, void* workspace,
              int64_t workspace_bytes, int sm_budget, spd_stream_t stream);
@@ -324,6 +328,12 @@ int spd_gemm_grouped(void* C, const void* A, const void* W, int64_t M, int64_t N
                      int64_t ldw, int64_t ldc, int num_groups, const int32_t* tile_group,
                      int64_t a_group_stride, int64_t a_cols, int64_t c_group_stride, int64_t w_group_col_stride,
                      int dtype, int epilogue, int sm_budget, spd_stream_t stream);
+/* rows mode over the rows that exist: group_rows [num_groups][2] (spd_moe_align_groups) = first row and number of rows of
+ * every group; the other rows of C are not written.  Epilogues SPD_EPI_NONE (stacked or K-concatenated weights, as above) and
+ * SPD_EPI_SILU_MUL.  At most 256 groups, M / 256 + num_groups <= 512. */
+int spd_gemm_grouped_rows(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_t K, int64_t lda,
+                          int64_t ldw, int64_t ldc, int num_groups, const int32_t* group_rows,
+                          int64_t w_group_col_stride, int dtype, int epilogue, int sm_budget, spd_stream_t stream);
 /* Router: softmax over the experts (fp32) + greedy top-k; weights = prob (renormalised over the k
  * if renormalize) * scale.  logits [tokens, num_experts] 16-bit.  replaces select_experts /
  * fused_topk (S/layers/moe/topk.py:79-120,128-163). */
@@ -337,6 +347,11 @@ int spd_moe_route(int32_t* topk_ids, float* topk_w, const void* logits, int64_t 
 int64_t spd_moe_align_rows(int64_t tokens, int top_k, int num_experts);
 int spd_moe_align(int32_t* row_token, int32_t* inv_pos, int32_t* tile_group, const int32_t* topk_ids,
                   int64_t tokens, int top_k, int num_experts, int64_t max_rows, spd_stream_t stream);
+/* the same, and group_rows [num_experts][2] (nullable, 8-byte aligned): first sorted row of every expert and its rows
+ * without the padding */
+int spd_moe_align_groups(int32_t* row_token, int32_t* inv_pos, int32_t* tile_group, int32_t* group_rows,
+                         const int32_t* topk_ids, int64_t tokens, int top_k, int num_experts, int64_t max_rows,
+                         spd_stream_t stream);
 /* xs[r, :] = x[row_token[r], :] (zeros for padding rows) */
 int spd_moe_gather(void* xs, const void* x, const int32_t* row_token, int64_t rows, int64_t dim,
                    int64_t x_stride, int dtype, spd_stream_t stream);

@@ -60,6 +60,7 @@ SIGNATURES = {
     "spd_gemm_workspace_bytes": (_i64, []),
     "spd_gemm_streamk_ctas": (_i64, [_i64, _i, _i, _i64]),
     "spd_gemm_pair_cols": (_i, [_i64, _i64, _i64, _i, _i]),
+    "spd_gemm_swap_rows": (_i, [_i64, _i64, _i64, _i, _i]),
     "spd_attn_general_tcgen05": (_i, [_i64, _i64, _i64, _i, _i, _i, _i]),
     "spd_gemm": (
         _i,
@@ -93,6 +94,8 @@ SIGNATURES = {
     "spd_moe_route": (_i, [_p, _p, _p, _i64, _i, _i, _f, _i, _i, _p]),
     "spd_moe_align_rows": (_i64, [_i64, _i, _i]),
     "spd_moe_align": (_i, [_p, _p, _p, _p, _i64, _i, _i, _i64, _p]),
+    "spd_moe_align_groups": (_i, [_p, _p, _p, _p, _p, _i64, _i, _i, _i64, _p]),
+    "spd_gemm_grouped_rows": (_i, [_p, _p, _p, _i64, _i64, _i64, _i64, _i64, _i64, _i, _p, _i64, _i, _i, _i, _p]),
     "spd_moe_gather": (_i, [_p, _p, _p, _i64, _i64, _i64, _i, _p]),
     "spd_moe_combine": (_i, [_p, _p, _p, _p, _p, _i64, _i, _i64, _i, _p]),
     "spd_moe_dense_act": (_i, [_p, _p, _p, _p, _i64, _i, _i, _i64, _i, _p]),

@@ -623,10 +623,14 @@ long long streamk_ctas(long long tiles, int kblocks, int split, long long slots)
 int gemm_cluster_try(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_t K, int64_t lda,
                      int64_t ldw, int64_t ldc, int dtype, int out_f32, int sms, cudaStream_t stream);
 
-int gemm_pair_cols(int64_t M, int64_t N, int64_t K, int epilogue, int sms);
+int gemm_pair_cols(int64_t M, int64_t N, int64_t K, int epilogue, int sms, int64_t* cost = nullptr);
 int gemm_pair_try(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_t K, int64_t lda,
                   int64_t ldw, int64_t ldc, int dtype, int out_f32, int epilogue, int sms, int panel_mb,
                   cudaStream_t stream);
+
+int gemm_swap_tiles(int64_t M, int64_t N, int64_t K, int epilogue, int sms);
+int gemm_pair_swap(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldw, int64_t ldc,
+                   int dtype, int epilogue, int sms, int tok_tiles, int panel_mb, cudaStream_t stream);
 
 int gemm_pair_decode_try(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_t K, int64_t lda,
                          int64_t ldw, int64_t ldc, int dtype, int out_f32, int sms, float* ws, int64_t ws_bytes,
@@ -664,6 +668,12 @@ int64_t spd_gemm_streamk_ctas(int64_t tiles, int kblocks, int split, int64_t slo
 int spd_gemm_pair_cols(int64_t M, int64_t N, int64_t K, int epilogue, int sm_budget) {
   if (M <= 0 || N <= 0 || K <= 0) return SPD_E_BADARG;
   return gemm_pair_cols(M, N, K, epilogue, sm_budget > 0 ? sm_budget : device_sm_count_cached());
+}
+
+int spd_gemm_swap_rows(int64_t M, int64_t N, int64_t K, int epilogue, int sm_budget) {
+  if (M <= 0 || N <= 0 || K <= 0) return SPD_E_BADARG;
+  const int64_t t = gemm_swap_tiles(M, N, K, epilogue, sm_budget > 0 ? sm_budget : device_sm_count_cached());
+  return t ? static_cast<int>(32 * (((M + 31) / 32 + t - 1) / t)) : 0;
 }
 
 int64_t spd_gemm_workspace_bytes(void) { return kGemmWsBytes + kGemmCounters * 4; }
@@ -779,7 +789,10 @@ int spd_gemm(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_
     return set_error(SPD_E_SHAPE, "spd_gemm: unreachable BN=%d", BN);
   }
 
-  // prefill regime proper: 256 x 256 tiles on CTA pairs (tcgen05.mma.cta_group::2, gemm_pair.cu)
+  // prefill regime: token tiles of any width where those take fewer or shorter waves (gemm_pair_swap.cu)
+  if (const int tiles = out_f32 ? 0 : gemm_swap_tiles(M, N, K, epilogue, sms))
+    return gemm_pair_swap(C, A, W, M, N, K, lda, ldw, ldc, dtype, epilogue, sms, tiles, env_panel_mb, st);
+  // else 256 x 256 tiles on CTA pairs (tcgen05.mma.cta_group::2, gemm_pair.cu)
   rc = gemm_pair_try(C, A, W, M, N, K, lda, ldw, ldc, dtype, out_f32, epilogue, sms, env_panel_mb, st);
   if (rc != 1) return rc;
 

@@ -24,6 +24,7 @@
 #include <stdlib.h>
 
 #include "common.cuh"
+#include "pair.cuh"
 #include "ptx.cuh"
 #include "row_stage.cuh"
 #include "tmap.cuh"
@@ -67,46 +68,6 @@ __device__ __forceinline__ void pair_tile_coords(const PairGemmParams& p, int ti
   const int q = min(p.panel, p.y_tiles - y0);
   xt = r / q;
   yt = y0 + r - xt * q;
-}
-
-// --- cta_group::2 forms of the tcgen05 / TMA instructions ---
-__device__ __forceinline__ void tmem_alloc_2cta(uint32_t* smem_result, uint32_t ncols) {
-  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_result)),
-               "r"(ncols)
-               : "memory");
-}
-__device__ __forceinline__ void tmem_relinquish_2cta() {
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc_2cta(uint32_t taddr, uint32_t ncols) {
-  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-// the mbarrier operand is a shared::cluster address (the LEADER's full barrier)
-__device__ __forceinline__ void tma_load_2d_2cta(void* smem_dst, const void* tmap, uint32_t bar_cluster_addr,
-                                                 int32_t c_inner, int32_t c_outer, uint64_t policy) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint"
-      " [%0], [%1, {%3, %4}], [%2], %5;" ::"r"(smem_u32(smem_dst)),
-      "l"(tmap), "r"(bar_cluster_addr), "r"(c_inner), "r"(c_outer), "l"(policy)
-      : "memory");
-}
-__device__ __forceinline__ void umma_ss_2cta(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                             uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// arrive on the barrier at this shared-memory offset in every CTA of `mask` once all MMAs issued
-// so far by this thread have completed
-__device__ __forceinline__ void umma_commit_2cta_mc(uint64_t* bar, uint16_t mask) {
-  asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
-          smem_u32(bar)),
-      "h"(mask)
-      : "memory");
 }
 
 template <typename T, int kEpi, int BN>
@@ -325,8 +286,10 @@ static int pair_tile_cols(int64_t N, int64_t x_tiles, int epilogue, int pairs, i
   return best;
 }
 
-// Columns of the pair tiles that a GEMM of these sizes takes, 0: single-CTA tiles.
-int gemm_pair_cols(int64_t M, int64_t N, int64_t K, int epilogue, int sms) {
+// Columns of the pair tiles that a GEMM of these sizes takes, 0: single-CTA tiles.  *cost: what either takes, in the units
+// of pair_tile_cols.
+int gemm_pair_cols(int64_t M, int64_t N, int64_t K, int epilogue, int sms, int64_t* cost_out) {
+  if (cost_out) *cost_out = 0;
   static const int enabled = getenv("SPD_GEMM_2CTA") ? atoi(getenv("SPD_GEMM_2CTA")) : 1;
   if (!enabled || M <= 256 || sms < 2) return 0;
   // A wave of 256 x 256 pair tiles takes about 0.9 of the time of a wave of 128 x 256 single tiles, so the pair serves also
@@ -336,11 +299,15 @@ int gemm_pair_cols(int64_t M, int64_t N, int64_t K, int epilogue, int sms) {
   const int64_t rows_pair = (M + 255) / 256 * 256, rows_single = (M + 127) / 128 * 128;
   int64_t cost;
   const int bn = pair_tile_cols(N, rows_pair / 256, epilogue, sms / 2, &cost);
+  if (cost_out) *cost_out = cost;
   if (rows_pair != rows_single && M < 2048) {
     const int n_tile = epilogue == SPD_EPI_SILU_MUL ? kPgBN / 2 : kPgBN;
     const int64_t cols = (N + n_tile - 1) / n_tile, kblocks = (K + kPgBK - 1) / kPgBK;
     const int64_t waves_single = (rows_single / 128 * cols + sms - 1) / sms;
-    if (cost * 9 >= waves_single * (kPgBN + 100) * 10 || waves_single * kblocks < 48) return 0;
+    if (cost * 9 >= waves_single * (kPgBN + 100) * 10 || waves_single * kblocks < 48) {
+      if (cost_out) *cost_out = waves_single * (kPgBN + 100) * 10 / 9;
+      return 0;
+    }
   }
   return bn;
 }
@@ -350,7 +317,7 @@ int gemm_pair_cols(int64_t M, int64_t N, int64_t K, int epilogue, int sms) {
 int gemm_pair_try(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_t K, int64_t lda,
                   int64_t ldw, int64_t ldc, int dtype, int out_f32, int epilogue, int sms, int panel_mb,
                   cudaStream_t stream) {
-  const int bn = gemm_pair_cols(M, N, K, epilogue, sms);
+  const int bn = gemm_pair_cols(M, N, K, epilogue, sms, nullptr);
   if (bn == 0) return 1;
   PairGemmParams p{};
   p.C = C;

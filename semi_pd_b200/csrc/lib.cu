@@ -52,52 +52,47 @@ static Fn driver_fn(const char* name) {
 }
 
 // ------------------------------------------------------------------------------------------------
-// TMA descriptors: 2-D, 16-bit elements, 128-byte swizzle, box = {64 elements, box_rows}
+// TMA descriptors: 16-bit elements, 128-byte swizzle, innermost box side 64 elements
 // ------------------------------------------------------------------------------------------------
-int make_tmap_2d_sw128(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols,
-                       uint64_t row_stride_elems, uint32_t box_rows, uint32_t box_cols) {
+int make_tmap_sw128(CUtensorMap* out, const void* base, int rank, const uint64_t* dims, const uint64_t* strides,
+                    const uint32_t* box) {
   using Fn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                           const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
                           CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
                           CUtensorMapFloatOOBfill);
   static Fn fn = driver_fn<Fn>("cuTensorMapEncodeTiled");
   if (!fn) return set_error(SPD_E_DRIVER, "cuTensorMapEncodeTiled not available from the driver");
-  cuuint64_t gdim[2] = {cols, rows};
-  cuuint64_t gstride[1] = {row_stride_elems * 2};
-  cuuint32_t box[2] = {box_cols, box_rows};
-  cuuint32_t estr[2] = {1, 1};
+  cuuint64_t gdim[5], gstride[4];
+  cuuint32_t gbox[5], estr[5];
+  for (int i = 0; i < rank; ++i) {
+    gdim[i] = dims[i];
+    gbox[i] = box[i];
+    estr[i] = 1;
+    if (i > 0) gstride[i - 1] = strides[i - 1] * 2;
+  }
   // 16-bit payload moved as raw bits (no conversion), so one encoding serves bf16 and fp16
-  CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), gdim, gstride,
-                  box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+  CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, const_cast<void*>(base), gdim, gstride,
+                  gbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS)
-    return set_error(SPD_E_DRIVER,
-                     "cuTensorMapEncodeTiled failed (%d): base=%p rows=%llu cols=%llu stride=%llu box=%ux%u",
-                     (int)r, base, (unsigned long long)rows, (unsigned long long)cols,
-                     (unsigned long long)row_stride_elems, box_rows, box_cols);
+    return set_error(SPD_E_DRIVER, "cuTensorMapEncodeTiled failed (%d): base=%p rank=%d dims=%llu,%llu,.. stride=%llu box=%ux%u..",
+                     (int)r, base, rank, (unsigned long long)dims[0], (unsigned long long)dims[1],
+                     (unsigned long long)strides[0], box[0], box[1]);
   return 0;
+}
+
+int make_tmap_2d_sw128(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols,
+                       uint64_t row_stride_elems, uint32_t box_rows, uint32_t box_cols) {
+  const uint64_t dims[2] = {cols, rows};
+  const uint32_t box[2] = {box_cols, box_rows};
+  return make_tmap_sw128(out, base, 2, dims, &row_stride_elems, box);
 }
 
 int make_tmap_blocks_sw128(CUtensorMap* out, const void* base, uint64_t rows, uint64_t blocks, uint64_t row_stride_elems,
                            uint32_t box_rows, uint32_t box_blocks) {
-  using Fn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                          const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
-                          CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
-                          CUtensorMapFloatOOBfill);
-  static Fn fn = driver_fn<Fn>("cuTensorMapEncodeTiled");
-  if (!fn) return set_error(SPD_E_DRIVER, "cuTensorMapEncodeTiled not available from the driver");
-  cuuint64_t gdim[3] = {64, rows, blocks};
-  cuuint64_t gstride[2] = {row_stride_elems * 2, 128};
-  cuuint32_t box[3] = {64, box_rows, box_blocks};
-  cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), gdim, gstride,
-                  box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS)
-    return set_error(SPD_E_DRIVER, "cuTensorMapEncodeTiled failed (%d): base=%p rows=%llu blocks=%llu stride=%llu box=%ux%u",
-                     (int)r, base, (unsigned long long)rows, (unsigned long long)blocks,
-                     (unsigned long long)row_stride_elems, box_rows, box_blocks);
-  return 0;
+  const uint64_t dims[3] = {64, rows, blocks}, strides[2] = {row_stride_elems, 64};
+  const uint32_t box[3] = {64, box_rows, box_blocks};
+  return make_tmap_sw128(out, base, 3, dims, strides, box);
 }
 
 // Allocated once, on the first call of a kernel with bounded waits; mapped, so that reading it takes no copy and no

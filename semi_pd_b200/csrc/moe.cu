@@ -93,6 +93,7 @@ moe_route_kernel(int32_t* __restrict__ topk_ids, float* __restrict__ topk_w, con
 //   row_token[r]  token feeding sorted row r (-1 = padding row)
 //   inv_pos[i]    sorted row of routing entry i = token * k + j (-1: a choice outside the E experts, which owns no row)
 //   tile_group[x] expert of 128-row tile x (-1 = unused tile)
+//   group_rows[e] first sorted row and number of rows of expert e, without the padding (may be null)
 // One cluster of 1 or 4 CTAs, each with its share of the entries: counts in shared memory, the peers' counts through the
 // cluster, then places.  What took the time was latency: entries are read eight at a time per thread, the first round of a
 // share once for both passes.  24576 entries, 64 experts: 23.4 us in one CTA that read them one at a time, twice; 10.7
@@ -102,7 +103,7 @@ constexpr int kMoeAlignEntries = 8;  // per thread and round
 template <int kCtas>
 __global__ void __launch_bounds__(1024)
 moe_align_kernel(int32_t* __restrict__ row_token, int32_t* __restrict__ inv_pos, int32_t* __restrict__ tile_group,
-                 const int32_t* __restrict__ topk_ids, int64_t entries, int k, int E, int64_t max_rows) {
+                 int2* __restrict__ group_rows, const int32_t* __restrict__ topk_ids, int64_t entries, int k, int E, int64_t max_rows) {
   __shared__ int cnt[kMoeMaxExperts];  // this CTA's entries per expert
   __shared__ int off[kMoeMaxExperts + 1];
   __shared__ int cur[kMoeMaxExperts];  // the next place
@@ -160,7 +161,10 @@ moe_align_kernel(int32_t* __restrict__ row_token, int32_t* __restrict__ inv_pos,
         if (tid >= o) incl += v;
       }
       __syncwarp();
-      if (e < E) off[e] = base + incl - n;
+      if (e < E) {
+        if (rank == 0 && group_rows) group_rows[e] = make_int2(base + incl - n, kCtas > 1 ? off[e] : cnt[e]);
+        off[e] = base + incl - n;
+      }
       base += __shfl_sync(0xffffffffu, incl, 31);
     }
     if (tid == 0) off[E] = base;
@@ -332,14 +336,21 @@ int64_t spd_moe_align_rows(int64_t tokens, int top_k, int num_experts) {
 
 int spd_moe_align(int32_t* row_token, int32_t* inv_pos, int32_t* tile_group, const int32_t* topk_ids,
                   int64_t tokens, int top_k, int num_experts, int64_t max_rows, spd_stream_t stream) {
+  return spd_moe_align_groups(row_token, inv_pos, tile_group, nullptr, topk_ids, tokens, top_k, num_experts, max_rows, stream);
+}
+
+int spd_moe_align_groups(int32_t* row_token, int32_t* inv_pos, int32_t* tile_group, int32_t* group_rows, const int32_t* topk_ids,
+                         int64_t tokens, int top_k, int num_experts, int64_t max_rows, spd_stream_t stream) {
   SPD_REQUIRE(row_token && inv_pos && tile_group && topk_ids, SPD_E_BADARG, "spd_moe_align: null pointer");
   SPD_REQUIRE(num_experts > 0 && num_experts <= kMoeMaxExperts && top_k > 0, SPD_E_SHAPE, "spd_moe_align: bad sizes");
   SPD_REQUIRE(max_rows >= spd_moe_align_rows(tokens, top_k, num_experts) && max_rows % kMoeTile == 0,
               SPD_E_WORKSPACE, "spd_moe_align: max_rows too small (need spd_moe_align_rows())");
+  int2* groups = reinterpret_cast<int2*>(group_rows);
+  SPD_REQUIRE((reinterpret_cast<uintptr_t>(groups) & 7u) == 0, SPD_E_ALIGN, "spd_moe_align: group_rows must be 8-byte aligned");
   const int64_t entries = tokens * top_k;
   if (entries <= 2048) {
     SPD_CUDA(launch(moe_align_kernel<1>, dim3(1), dim3(1024), 0, as_stream(stream), pdl_enabled(), row_token, inv_pos,
-                    tile_group, topk_ids, entries, top_k, num_experts, max_rows));
+                    tile_group, groups, topk_ids, entries, top_k, num_experts, max_rows));
     return 0;
   }
   cudaLaunchConfig_t cfg{};
@@ -355,7 +366,7 @@ int spd_moe_align(int32_t* row_token, int32_t* inv_pos, int32_t* tile_group, con
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 2 : 1;
-  SPD_CUDA(cudaLaunchKernelEx(&cfg, moe_align_kernel<4>, row_token, inv_pos, tile_group, topk_ids, entries, top_k,
+  SPD_CUDA(cudaLaunchKernelEx(&cfg, moe_align_kernel<4>, row_token, inv_pos, tile_group, groups, topk_ids, entries, top_k,
                               num_experts, max_rows));
   return 0;
 }

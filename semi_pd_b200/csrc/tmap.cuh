@@ -5,6 +5,11 @@
 
 namespace spd {
 
+// A tensor of 16-bit elements in `rank` (at most 5) dimensions, innermost first; strides in elements, from the second
+// dimension on.
+int make_tmap_sw128(CUtensorMap* out, const void* base, int rank, const uint64_t* dims, const uint64_t* strides,
+                    const uint32_t* box);
+
 // 2-D row-major tensor of 16-bit elements [rows, cols] with `row_stride_elems` between rows;
 // box = box_rows x box_cols (box_cols * 2 bytes must be 128 for the 128-byte swizzle).
 // Out-of-bounds parts of a box are zero-filled by the hardware.

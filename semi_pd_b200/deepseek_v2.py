@@ -167,10 +167,10 @@ class DeepseekV2MoE:
             act = ops.moe_dense_act(gu, ids, w, E, inter)             # [T, E * I], routing weight folded in
             y = ops.linear(act, self.w_down_cat)                      # [T, hidden]
             return ops.bias_act_residual(y, None, shared) if shared is not None else y
-        row_token, inv_pos, tile_group = ops.moe_align(ids, E)
+        row_token, inv_pos, tile_group, rows = ops.moe_align_groups(ids, E)
         xs = ops.moe_gather(x, row_token)
-        act = ops.linear_grouped_rows(xs, self.w_gate_up, tile_group, E, inter, epilogue=ops.SPD_EPI_SILU_MUL)
-        y = ops.linear_grouped_rows(act, self.w_down_cat, tile_group, E, x.shape[1], k_concat=True)
+        act = ops.linear_grouped_rows(xs, self.w_gate_up, tile_group, E, inter, epilogue=ops.SPD_EPI_SILU_MUL, group_rows=rows)
+        y = ops.linear_grouped_rows(act, self.w_down_cat, tile_group, E, x.shape[1], k_concat=True, group_rows=rows)
         return ops.moe_combine(y, inv_pos, w, shared)
 
     __call__ = forward

@@ -372,12 +372,21 @@ def linear_block_diag(x: torch.Tensor, weight: torch.Tensor, num_groups: int, k:
 
 
 def linear_grouped_rows(x_sorted: torch.Tensor, weight: torch.Tensor, tile_group: torch.Tensor, num_groups: int,
-                        n: int, epilogue: int = SPD_EPI_NONE, k_concat: bool = False) -> torch.Tensor:
+                        n: int, epilogue: int = SPD_EPI_NONE, k_concat: bool = False,
+                        group_rows: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Rows of x_sorted are grouped by expert in 128-row tiles; weight = the experts' [n (or 2n), K]
-    matrices stacked along the rows — or, k_concat, [n, E * K] concatenated along K.  → [rows, n]."""
+    matrices stacked along the rows — or, k_concat, [n, E * K] concatenated along K.  → [rows, n].  With group_rows
+    (moe_align_groups) padding rows may be left out: what they hold then is undefined."""
     _cuda(x_sorted, weight, tile_group)
     M, K = x_sorted.shape
     out = torch.empty(M, n, device=x_sorted.device, dtype=x_sorted.dtype)
+    if (group_rows is not None and epilogue in (SPD_EPI_NONE, SPD_EPI_SILU_MUL) and num_groups <= 256
+            and M // 256 + num_groups <= 512):
+        check(lib.spd_gemm_grouped_rows(out.data_ptr(), x_sorted.data_ptr(), weight.data_ptr(), M, n, K, x_sorted.stride(0),
+                                        weight.stride(0), out.stride(0), num_groups, group_rows.data_ptr(),
+                                        K if k_concat else 0, _dt(x_sorted), epilogue, get_sm_budget(), _stream()),
+              "spd_gemm_grouped_rows")
+        return out
     check(lib.spd_gemm_grouped(out.data_ptr(), x_sorted.data_ptr(), weight.data_ptr(), M, n, K, x_sorted.stride(0),
                                weight.stride(0), out.stride(0), num_groups, tile_group.data_ptr(), 0, K, 0,
                                K if k_concat else 0, _dt(x_sorted), epilogue, get_sm_budget(), _stream()),
@@ -409,6 +418,22 @@ def moe_align(topk_ids: torch.Tensor, num_experts: int):
     check(lib.spd_moe_align(row_token.data_ptr(), inv_pos.data_ptr(), tile_group.data_ptr(), topk_ids.data_ptr(),
                             T, k, num_experts, R, _stream()), "spd_moe_align")
     return row_token, inv_pos, tile_group
+
+
+def moe_align_groups(topk_ids: torch.Tensor, num_experts: int):
+    """→ (row_token, inv_pos, tile_group, group_rows): moe_align and, int32 [E, 2], every expert's first row and number of
+    rows without the padding."""
+    _cuda(topk_ids)
+    T, k = topk_ids.shape
+    R = lib.spd_moe_align_rows(T, k, num_experts)
+    dev = topk_ids.device
+    row_token = torch.empty(R, device=dev, dtype=torch.int32)
+    inv_pos = torch.empty(T * k, device=dev, dtype=torch.int32)
+    tile_group = torch.empty(R // 128, device=dev, dtype=torch.int32)
+    group_rows = torch.empty(num_experts, 2, device=dev, dtype=torch.int32)
+    check(lib.spd_moe_align_groups(row_token.data_ptr(), inv_pos.data_ptr(), tile_group.data_ptr(), group_rows.data_ptr(),
+                                   topk_ids.data_ptr(), T, k, num_experts, R, _stream()), "spd_moe_align_groups")
+    return row_token, inv_pos, tile_group, group_rows
 
 
 def moe_gather(x: torch.Tensor, row_token: torch.Tensor) -> torch.Tensor:
