@@ -191,6 +191,11 @@ int spd_gemm_pair_cols(int64_t M, int64_t N, int64_t K, int epilogue, int sm_bud
 /* Token rows of the widest of the tiles with 256 weight rows that a GEMM of these sizes with 16-bit results takes, 0: the
  * tiles above. */
 int spd_gemm_swap_rows(int64_t M, int64_t N, int64_t K, int epilogue, int sm_budget);
+/* Before both: token tiles of a GEMM on few weight rows, 0: the forms above and those for up to 256 tokens that split K over
+ * global memory.  *split: pairs of CTAs over which a cluster cuts K, 0: K uncut, all tiles beside one another. */
+int spd_gemm_split_tiles(int64_t M, int64_t N, int64_t K, int epilogue, int out_f32, int sm_budget, int* split);
+/* Whether SPD_EPI_SILU_MUL serves M tokens at least as well as the plain GEMM and spd_silu_and_mul (N: output columns). */
+int spd_gemm_silu_fused(int64_t M, int64_t N, int64_t K, int sm_budget);
 int spd_gemm(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_t K, int64_t lda,
              int64_t ldw, int64_t ldc, int dtype, int out_f32, int epilogue, void* workspace,
              int64_t workspace_bytes, int sm_budget, spd_stream_t stream);

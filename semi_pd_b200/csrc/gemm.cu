@@ -632,6 +632,10 @@ int gemm_swap_tiles(int64_t M, int64_t N, int64_t K, int epilogue, int sms);
 int gemm_pair_swap(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldw, int64_t ldc,
                    int dtype, int epilogue, int sms, int tok_tiles, int panel_mb, cudaStream_t stream);
 
+int gemm_split_tiles(int64_t M, int64_t N, int64_t K, int epilogue, int out_f32, int sms, int* split);
+int gemm_pair_split(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldw, int64_t ldc,
+                    int dtype, int out_f32, int epilogue, int tok_tiles, int split, cudaStream_t stream);
+
 int gemm_pair_decode_try(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_t K, int64_t lda,
                          int64_t ldw, int64_t ldc, int dtype, int out_f32, int sms, float* ws, int64_t ws_bytes,
                          int* flags, int n_flags, int max_split, cudaStream_t stream);
@@ -668,6 +672,26 @@ int64_t spd_gemm_streamk_ctas(int64_t tiles, int kblocks, int split, int64_t slo
 int spd_gemm_pair_cols(int64_t M, int64_t N, int64_t K, int epilogue, int sm_budget) {
   if (M <= 0 || N <= 0 || K <= 0) return SPD_E_BADARG;
   return gemm_pair_cols(M, N, K, epilogue, sm_budget > 0 ? sm_budget : device_sm_count_cached());
+}
+
+int spd_gemm_silu_fused(int64_t M, int64_t N, int64_t K, int sm_budget) {
+  if (M <= 0 || N <= 0 || K <= 0) return SPD_E_BADARG;
+  const int sms = sm_budget > 0 ? sm_budget : device_sm_count_cached();
+  if (M > 256) return 1;
+  if (sms < 2) return 0;
+  const int64_t tiles = (N + 127) / 128, pairs = sms / 2;
+  if (tiles <= pairs) return 1;
+  // More weight tiles than pairs: fused, every pair has whole tiles; unfused, stream-K deals k-blocks evenly, for 4 us of
+  // fix-up and 3 of activation kernel.  A k-block of a pair takes 0.175 us, the weights at least their time from HBM.  2 x 14336
+  // rows, K = 4096, on 74 pairs: 64 tokens 43.0 unfused / 41.6 fused, 128 46.8 / 43.2, 256 59.7 / 54.6.
+  const double kb = static_cast<double>((K + kBK - 1) / kBK), hbm = 4.0 * N * K / 6.2e6;
+  const double whole = (tiles + pairs - 1) / pairs * kb * 0.175, even = kb * tiles / pairs * 0.175 + 4;
+  return (whole > hbm ? whole : hbm) <= (even > hbm ? even : hbm) + 3;
+}
+
+int spd_gemm_split_tiles(int64_t M, int64_t N, int64_t K, int epilogue, int out_f32, int sm_budget, int* split) {
+  SPD_REQUIRE(split && M > 0 && N > 0 && K > 0, SPD_E_BADARG, "spd_gemm_split_tiles: bad arguments");
+  return gemm_split_tiles(M, N, K, epilogue, out_f32, sm_budget > 0 ? sm_budget : device_sm_count_cached(), split);
 }
 
 int spd_gemm_swap_rows(int64_t M, int64_t N, int64_t K, int epilogue, int sm_budget) {
@@ -712,8 +736,7 @@ int spd_gemm(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_
   // stream-K grid: equal unit ranges (streamk_ctas).  Tuning knobs (experiments only):
   // SPD_GEMM_STREAMK=0 disables stream-K, =2 forces it; SPD_GEMM_SPLIT=d aims at ~d contributors per
   // tile where that does not leave most SMs idle; SPD_GEMM_SWAPMAX=m is the largest M routed to
-  // swap-AB; SPD_GEMM_CLUSTER=1 routes few-tile layers at M <= 128 to the cluster split-K kernel
-  // (gemm_cluster.cu) instead.
+  // swap-AB; SPD_GEMM_CLUSTER=0 leaves the cluster of single CTAs (gemm_cluster.cu) out.
   static const int env_streamk = getenv("SPD_GEMM_STREAMK") ? atoi(getenv("SPD_GEMM_STREAMK")) : 1;
   static const int env_split = getenv("SPD_GEMM_SPLIT") ? atoi(getenv("SPD_GEMM_SPLIT")) : 4;
   static const int env_swapmax = getenv("SPD_GEMM_SWAPMAX") ? atoi(getenv("SPD_GEMM_SWAPMAX")) : 256;
@@ -743,15 +766,15 @@ int spd_gemm(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_
   // Decode regime, M <= 256: swap-AB.  The token dimension feeds UMMA-N (16, or M rounded up to a
   // multiple of 32), each 128-row weight tile is read once, and no MMA work is spent on padding
   // rows (the un-swapped form would pad 160 tokens to 2 x 128 and read W twice from L2).
+  // few weight tiles: clusters of pairs that cut K, or token tiles beside one another (gemm_split_tiles)
+  int split = 0;
+  if (const int tiles = gemm_split_tiles(M, N, K, epilogue, out_f32, sms, &split))
+    return split ? gemm_pair_split(C, A, W, M, N, K, lda, ldw, ldc, dtype, out_f32, epilogue, tiles, split, st)
+                 : gemm_pair_swap(C, A, W, M, N, K, lda, ldw, ldc, dtype, epilogue, sms, tiles, env_panel_mb, st);
+  if (epilogue == SPD_EPI_SILU_MUL && M <= 256 && !out_f32 && sms >= 2)
+    return gemm_pair_swap(C, A, W, M, N, K, lda, ldw, ldc, dtype, epilogue, sms, 1, env_panel_mb, st);
   const bool swap = (M <= env_swapmax) && epilogue == SPD_EPI_NONE;
   if (swap) {
-    // experiment knob: SPD_GEMM_PREFER_CLUSTER=1 routes few-tile layers at M <= 128 to the DSMEM
-    // split-K kernel before the pair kernel is considered
-    static const int env_prefer_cluster = getenv("SPD_GEMM_PREFER_CLUSTER") ? atoi(getenv("SPD_GEMM_PREFER_CLUSTER")) : 0;
-    if (env_prefer_cluster && M > 32 && (N + kBM - 1) / kBM <= sms / 2) {
-      rc = gemm_cluster_try(C, A, W, M, N, K, lda, ldw, ldc, dtype, out_f32, sms, st);
-      if (rc != 1) return rc;
-    }
     // 32 < M <= 256: CTA pairs share one activation tile between 256 weight rows (gemm_pair_decode.cu)
     rc = gemm_pair_decode_try(C, A, W, M, N, K, lda, ldw, ldc, dtype, out_f32, sms, ws_ok ? p.ws : nullptr,
                               kGemmWsBytes, ws_ok ? p.counters : nullptr, kGemmCounters, env_split, st);

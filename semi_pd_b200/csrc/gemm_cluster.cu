@@ -1,4 +1,4 @@
-// Decode-regime GEMM with split-K across a THREAD-BLOCK CLUSTER, reduced on chip through
+// GEMM of up to 16 tokens (gemm_pair_split.cu says which) with split-K across a THREAD-BLOCK CLUSTER, reduced on chip through
 // distributed shared memory — for the layers whose N gives fewer 128-row weight tiles than there
 // are SMs (W_qkv: 48 tiles, W_o and W_down: 32 tiles on Llama-3-8B).  One SM streams ~90-100 GB/s
 // however deep its TMA ring is, so those layers need 3-4 SMs per tile to approach HBM speed; a
@@ -239,25 +239,31 @@ static int launch_cluster_gemm(const CUtensorMap& tw, const CUtensorMap& ta, con
   return 0;
 }
 
+// CTAs per tile
+static int cluster_split(int64_t tiles, int64_t kblocks, int sms) {
+  int64_t S = sms / tiles;            // that still fit the partition in one wave
+  S = S >= 4 ? 4 : (S >= 2 ? 2 : 1);  // clusters of 3 schedule poorly on the 16-20-SM GPCs (measured)
+  return static_cast<int>(S > kblocks / 8 ? kblocks / 8 : S);  // >= 8 k-blocks per rank
+}
+
+// CTAs of a GEMM of up to 16 tokens here, 0: not taken.
+int gemm_cluster_ctas(int64_t N, int64_t K, int sms) {
+  const int64_t tiles = (N + kCgBM - 1) / kCgBM;
+  const int S = cluster_split(tiles, (K + kCgBK - 1) / kCgBK, sms);
+  return S < 2 ? 0 : static_cast<int>(tiles * S);
+}
+
 // Called by spd_gemm for the swap-AB regime.  Returns 1 if this path does not apply (caller falls
 // through to the single-CTA-per-tile kernel), 0 on launch, else an error code.
 int gemm_cluster_try(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_t K, int64_t lda,
                      int64_t ldw, int64_t ldc, int dtype, int out_f32, int sms, cudaStream_t stream) {
   static const int enabled = getenv("SPD_GEMM_CLUSTER") ? atoi(getenv("SPD_GEMM_CLUSTER")) : 1;
-  if (!enabled || M > 128) return 1;
+  if (!enabled || M > 16) return 1;  // more tokens: gemm_pair_split.cu
   const int tiles = static_cast<int>((N + kCgBM - 1) / kCgBM);
   const int kblocks = static_cast<int>((K + kCgBK - 1) / kCgBK);
-  int BN = 16;
-  while (BN < M) BN <<= 1;
-  int S = sms / tiles;            // CTAs per tile that still fit the partition in one wave
-  S = S >= 4 ? 4 : (S >= 2 ? 2 : 1);  // clusters of 3 schedule poorly on the 16-20-SM GPCs (measured)
-  if (S > kblocks / 8) S = kblocks / 8;   // >= 8 k-blocks per rank
-  const int stage_area = (BN == 16 ? cg_stages<16>() * cg_stage_bytes<16>()
-                          : BN == 32 ? cg_stages<32>() * cg_stage_bytes<32>()
-                          : BN == 64 ? cg_stages<64>() * cg_stage_bytes<64>()
-                                     : cg_stages<128>() * cg_stage_bytes<128>());
-  const int part = kCgBM * (BN * 4 + 16);
-  while (S > 1 && (S - 1) * part > stage_area) --S;
+  constexpr int BN = 16;
+  const int S = cluster_split(tiles, kblocks, sms);
+  static_assert(3 * cg_part_bytes<BN>() <= cg_stages<BN>() * cg_stage_bytes<BN>(), "the partial sums of a tile fit the ring");
   if (S < 2) return 1;
   ClusterGemmParams p{};
   p.C = C;
@@ -270,17 +276,7 @@ int gemm_cluster_try(void* C, const void* A, const void* W, int64_t M, int64_t N
   int rc;
   if ((rc = get_tmap(&tw, W, N, K, ldw, kCgBM))) return rc;
   if ((rc = get_tmap(&ta, A, M, K, lda, BN))) return rc;
-#define SPD_CG(BN_)                                                                              \
-  case BN_:                                                                                      \
-    SPD_DISPATCH_DTYPE(dtype, { return launch_cluster_gemm<T, BN_>(tw, ta, p, tiles, S, stream); }); \
-    break;
-  switch (BN) {
-    SPD_CG(16)
-    SPD_CG(32)
-    SPD_CG(64)
-    SPD_CG(128)
-  }
-#undef SPD_CG
+  SPD_DISPATCH_DTYPE(dtype, { return launch_cluster_gemm<T, BN>(tw, ta, p, tiles, S, stream); });
   return 1;
 }
 

@@ -1,5 +1,5 @@
 // Decode-regime GEMM on CTA PAIRS: C[M,N] = A[M,K] * W[N,K]^T for 32 < M <= 256 tokens, swap-AB
-// with tcgen05.mma.cta_group::2.
+// with tcgen05.mma.cta_group::2.  (Few weight tiles: gemm_pair_split.cu.)
 //
 // Why: measured on B200 the single-CTA swap-AB kernel (gemm.cu) delivers a constant ~8-9 TB/s of
 // operand bytes into the SMs whatever M is — the chip-wide L2 -> SM limit — and every 128-row weight tile re-reads the whole

@@ -28,7 +28,7 @@ namespace spd {
 
 constexpr int kPsThreads = 256;
 constexpr int kPsBK = 64;
-constexpr int kPsStages = 8;                   // at most
+constexpr int kPsStages = 12;                  // at most
 constexpr int kPsHalfBytes = 128 * kPsBK * 2;  // 128 rows of one operand
 constexpr int kPsTokens = 64;                  // tokens staged at a time
 constexpr int kPsMaxTiles = 512;               // token tiles of a call
@@ -46,6 +46,7 @@ struct SwapGemmParams {
   int units, tok_tiles;        // one group: 32-row units, token tiles
   int stages, slot;            // ring: slots and bytes of each (128 weight rows, half of the widest token tile)
   int list;                    // token tiles that the list has room for
+  int decode;                  // one group: a batch that streams the weights once (see the launch)
   int panel;                   // one group: token tiles of a rasterisation panel
   const int2* group_rows;      // (first row, rows) of every group, null: one group
   int num_groups;
@@ -153,6 +154,7 @@ gemm_pair_swap_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
 
+  if (p.decode) griddep_launch_dependents();
   // (one group: the weights do not depend on the kernel before, so the copies of the first ones precede the wait)
   if (p.group_rows || warp != 0) griddep_wait();
   // the token tiles of all groups, one behind the other
@@ -200,13 +202,14 @@ gemm_pair_swap_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
   if (warp == 0) {
     if (elect_one()) {
       int stage = 0, phase = 0, ahead = 0;
+      const uint64_t policy = p.decode ? kEvictFirst : kEvictNormal;  // of the weights
       auto load_w = [&](int slot, uint32_t lead_full, int kb, int wt, int group) {
         if constexpr (kSilu)
           tma_load_5d_2cta(smem + slot * p.slot, &tmW, lead_full, kb * kPsBK, 0, 0, wt * 16 + static_cast<int>(rank) * 8, group,
-                           kEvictNormal);
+                           policy);
         else
           tma_load_2d_2cta(smem + slot * p.slot, &tmW, lead_full, static_cast<int>(group * p.w_group_cols) + kb * kPsBK,
-                           static_cast<int>(group * p.w_group_rows) + wt * 256 + static_cast<int>(rank) * 128, kEvictNormal);
+                           static_cast<int>(group * p.w_group_rows) + wt * 256 + static_cast<int>(rank) * 128, policy);
       };
       if (!p.group_rows) {
         int wt, tt;
@@ -330,7 +333,7 @@ gemm_pair_swap_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
     }
   }
 
-  griddep_launch_dependents();
+  if (!p.decode) griddep_launch_dependents();
   tc_fence_before_sync();
   __syncthreads();
   if (*dead) {
@@ -342,7 +345,7 @@ gemm_pair_swap_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
 }
 
 // Gate and up rows of all groups as [group][8-row group][gate / up][8 rows][64 columns]
-static int get_gate_up_tmap(CUtensorMap* out, const void* W, uint64_t groups, uint64_t inter, uint64_t cols, uint64_t ldw) {
+int get_gate_up_tmap(CUtensorMap* out, const void* W, uint64_t groups, uint64_t inter, uint64_t cols, uint64_t ldw) {
   struct Key {
     const void* base;
     uint64_t groups, inter, cols, ldw;
@@ -461,6 +464,8 @@ int gemm_pair_swap(void* C, const void* A, const void* W, int64_t M, int64_t N, 
   const int64_t total = static_cast<int64_t>(p.w_tiles) * tok_tiles;
   const int pairs = static_cast<int>(total < sms / 2 ? total : sms / 2);
   p.list = tok_tiles;
+  // as the other decode kernels (gemm_pair_decode.cu): the next kernel's weights come under this one's tail
+  p.decode = M <= 256;
   return run_swap(p, A, M, K, lda, W, 1, ldw, silu, silu ? 2 * N : N, K, 32 * ((p.units + tok_tiles - 1) / tok_tiles), dtype, pairs, stream);
 }
 

@@ -29,7 +29,6 @@ from .distributed import get_tensor_model_parallel_world_size
 from .forward_batch_info import ForwardBatch, LogitsProcessorOutput
 from .layers import LinearBase, LogitsProcessor, ParallelLMHead, RMSNorm, SiluAndMul, VocabParallelEmbedding
 
-_FUSED_SILU_MIN_TOKENS = 257
 # batches in [lo, hi] run all experts densely (see module docstring)
 _MOE_DENSE_MIN_TOKENS = 16
 _MOE_DENSE_MAX_TOKENS = 256
@@ -118,7 +117,7 @@ class DeepseekV2MLP:
         self.act_fn = SiluAndMul()
 
     def forward(self, x):
-        if x.shape[0] >= _FUSED_SILU_MIN_TOKENS:
+        if ops.silu_fused(x, self.gate_up_proj.weight):
             h = ops.linear(x, self.gate_up_proj.weight, epilogue=ops.SPD_EPI_SILU_MUL)
         else:
             h = self.act_fn(ops.linear(x, self.gate_up_proj.weight))

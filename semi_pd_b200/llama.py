@@ -13,15 +13,15 @@ from typing import Dict, Iterable, Optional, Tuple
 
 import torch
 
+from . import ops
 from .attention_backend import RadixAttention
 from .distributed import get_tensor_model_parallel_rank, get_tensor_model_parallel_world_size
 from .forward_batch_info import ForwardBatch, LogitsProcessorOutput
 from .layers import (LogitsProcessor, MergedColumnParallelLinear, ParallelLMHead, QKVParallelLinear,
                      RMSNorm, RowParallelLinear, SiluAndMul, VocabParallelEmbedding, get_rope)
 
-# tokens above which the gate_up GEMM runs in the (non-swapped) prefill regime and can fuse SiLU·mul
-# SPD_FUSED_SILU_MIN_TOKENS: A/B knob (a huge value routes prefill through the plain GEMM + SiLU·mul kernel)
-_FUSED_SILU_MIN_TOKENS = int(os.environ.get("SPD_FUSED_SILU_MIN_TOKENS", 257))
+# SPD_FUSED_SILU_MIN_TOKENS: A/B knob (smaller batches go through the plain GEMM + SiLU·mul kernel)
+_FUSED_SILU_MIN_TOKENS = int(os.environ.get("SPD_FUSED_SILU_MIN_TOKENS", 1))
 
 
 class LlamaMLP:
@@ -33,7 +33,7 @@ class LlamaMLP:
         self.act_fn = SiluAndMul()
 
     def forward(self, x):
-        if x.shape[0] >= _FUSED_SILU_MIN_TOKENS:
+        if x.shape[0] >= _FUSED_SILU_MIN_TOKENS and ops.silu_fused(x, self.gate_up_proj.weight):
             x = self.gate_up_proj.forward_silu_mul(x)
         else:
             gate_up, _ = self.gate_up_proj(x)

@@ -9,6 +9,7 @@ torch is plumbing here (device memory + streams); every computation runs in libs
 from __future__ import annotations
 
 import contextlib
+import functools
 import os
 from typing import Optional
 
@@ -351,6 +352,16 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = 
                        weight.stride(0), out.stride(0), _dt(x), (2 if exact_f32 else 1) if out_f32 else 0, epilogue,
                        ws.data_ptr(), ws.numel(), get_sm_budget(), _stream()), "spd_gemm")
     return out
+
+
+@functools.lru_cache(maxsize=1024)
+def _silu_fused(M: int, N: int, K: int, sm_budget: int) -> bool:
+    return lib.spd_gemm_silu_fused(M, N, K, sm_budget) == 1
+
+
+def silu_fused(x: torch.Tensor, weight: torch.Tensor) -> bool:
+    """Whether linear(x, weight, epilogue=SPD_EPI_SILU_MUL) serves as well as linear and silu_and_mul."""
+    return _silu_fused(x.shape[0], weight.shape[0] // 2, x.shape[1], get_sm_budget())
 
 
 def linear_block_diag(x: torch.Tensor, weight: torch.Tensor, num_groups: int, k: int, n: int,
