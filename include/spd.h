@@ -534,6 +534,19 @@ int spd_retention_extend_ws(float* o, const void* q, const void* k, const void* 
                             int in_act, int dtype, void* workspace, int64_t workspace_bytes, int sm_budget,
                             spd_stream_t stream);
 
+/* The same in tiles of 128 tokens that all run at once, for batches of some hundred tokens and more; workspace of
+ * spd_retention_tiles_workspace_bytes (0: not for these sizes), not zeroed, one call at a time.  Everything 16-byte aligned,
+ * strides multiples of 8. */
+int64_t spd_retention_tiles_workspace_bytes(int64_t batch, int64_t total_tokens, int num_heads, int head_dim, int v_dim,
+                                            int rot_dims, int in_act, int dtype, int sm_budget);
+int spd_retention_extend_tiles(float* o, const void* q, const void* k, const void* v, float* state,
+                               const int64_t* req_pool_indices, const int32_t* prefix_lens, const int32_t* extend_lens,
+                               const int32_t* extend_start_loc, int64_t batch, int64_t total_tokens, int num_heads,
+                               int head_dim, int v_dim, int64_t q_stride, int64_t k_stride, int64_t v_stride,
+                               const float* decay, const float* cos_sin, int rot_dims, int64_t max_positions, float k_scale,
+                               int in_act, int dtype, void* workspace, int64_t workspace_bytes, int sm_budget,
+                               spd_stream_t stream);
+
 /* spd_residual_rmsnorm with a second weight: out2 = the same normed row times (weight_offset + w2)
  * (out2 and w2 both NULL or both given) */
 int spd_residual_rmsnorm2(void* out, void* out2, float* x, const void* a, const void* b, const void* w,

@@ -152,6 +152,12 @@ SIGNATURES = {
         [_p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i64, _i64, _i, _i, _i, _i, _i64, _i64, _i64, _f, _i, _p, _p,
          _f, _i, _i64, _i, _p],
     ),
+    "spd_retention_tiles_workspace_bytes": (_i64, [_i64, _i64, _i, _i, _i, _i, _i, _i, _i]),
+    "spd_retention_extend_tiles": (
+        _i,
+        [_p, _p, _p, _p, _p, _p, _p, _p, _p, _i64, _i64, _i, _i, _i, _i64, _i64, _i64, _p, _p, _i, _i64, _f, _i, _i, _p, _i64,
+         _i, _p],
+    ),
     "spd_retention_workspace_bytes": (_i64, [_i64, _i64, _i, _i, _i, _i, _i, _i, _i]),
     "spd_retention_extend_ws": (
         _i,

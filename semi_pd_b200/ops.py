@@ -1171,9 +1171,15 @@ def retention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.Te
     o = torch.empty(T, num_heads * v_dim, device=q.device, dtype=torch.float32)
     if seq_lens is None:
         act, B = {None: 0, "silu": 1}[in_act], req_pool_indices.numel()
-        room = lib.spd_retention_workspace_bytes(B, T, num_heads, head_dim, v_dim, int(rot_dims), act, _dta(q), get_sm_budget())
+        sizes = (B, T, num_heads, head_dim, v_dim, int(rot_dims), act, _dta(q), get_sm_budget())
+        room, extend = 0, lib.spd_retention_extend_tiles
+        if all(x % 8 == 0 for x in (q.stride(0), k.stride(0), v.stride(0))) and all(
+                x is None or x.data_ptr() % 16 == 0 for x in (q, k, v, o, state, cos_sin)):
+            room = lib.spd_retention_tiles_workspace_bytes(*sizes)
+        if room == 0:
+            room, extend = lib.spd_retention_workspace_bytes(*sizes), lib.spd_retention_extend_ws
         ws = torch.empty(room, device=q.device, dtype=torch.uint8) if room > 0 else None
-        check(lib.spd_retention_extend_ws(o.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), state.data_ptr(),
+        check(extend(o.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), state.data_ptr(),
                                           req_pool_indices.data_ptr(), _ptr(prefix_lens), _ptr(extend_lens),
                                           _ptr(extend_start_loc), B, T, num_heads, head_dim, v_dim, q.stride(0), k.stride(0),
                                           v.stride(0), decay.data_ptr(), _ptr(cos_sin), int(rot_dims),
