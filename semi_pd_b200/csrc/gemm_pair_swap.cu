@@ -444,6 +444,8 @@ int gemm_swap_tiles(int64_t M, int64_t N, int64_t K, int epilogue, int sms) {
     }
   }
   const bool fewer_rows = waves >= 3 && 32 * units * 105 <= (M + 255) / 256 * 256 * 100;
+  // (up to 16 k-blocks the tiles' ends decide, which take longer here: 5140 x 4096, K = 512 25.9 / 26.5 us for 6 % fewer units)
+  if (K <= 16 * kPsBK) return cost * 10 < other * 9 ? static_cast<int>(best) : 0;
   return cost < other || (cost == other && fewer_rows) ? static_cast<int>(best) : 0;
 }
 

@@ -11,7 +11,7 @@ What differs from the reference, all on the kernel side:
     take it where it is faster (`mla_expanded_pays`, `spd_attn_mla_prefill`).
   * q_proj and kv_a_proj_with_mqa run as ONE GEMM (their weights stacked), the two per-head BMMs
     as one block-diagonal `spd_gemm_grouped` launch each.
-  * the routed experts run either as two grouped GEMMs over expert-sorted 128-row tiles
+  * the routed experts run either as two grouped GEMMs over expert-sorted rows
     (prefill-sized batches, and tiny ones that touch few experts) or, for decode-sized batches
     that hit nearly every expert anyway, as two plain GEMMs over ALL experts' stacked weights with
     the routing weights folded into the activation (`spd_moe_dense_act`).
@@ -29,9 +29,10 @@ from .distributed import get_tensor_model_parallel_world_size
 from .forward_batch_info import ForwardBatch, LogitsProcessorOutput
 from .layers import LinearBase, LogitsProcessor, ParallelLMHead, RMSNorm, SiluAndMul, VocabParallelEmbedding
 
-# batches in [lo, hi] run all experts densely (see module docstring)
-_MOE_DENSE_MIN_TOKENS = 16
-_MOE_DENSE_MAX_TOKENS = 256
+# Batches in [lo, hi] run all experts densely (see module docstring).  Dense / grouped, us a layer: 16 tokens 206 / 202, 24
+# 216 / 214, 32 219 / 223, 64 224 / 226, 96 232 / 233, 128 242 / 236, 256 317 / 250.
+_MOE_DENSE_MIN_TOKENS = 28
+_MOE_DENSE_MAX_TOKENS = 112
 
 
 # The expanded form of MLA prefill keeps K and V of every key while a layer runs: 8 KB per key at 16 heads.
