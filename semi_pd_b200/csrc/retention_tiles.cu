@@ -12,7 +12,7 @@
 // head's values split q and k again, and the longest portion decides (41 chunks of 5.6 us of the 8192 tokens below).  Tiles
 // of 128 rows and 128 value columns are independent, q lies in tensor memory (its products read only their other operand
 // from shared memory), and the state is split once per 128 tokens.  4 requests, 8192 tokens, 16 heads of 128 x 128, bf16:
-// 240 us in chunks, 172 here (sums 48, scan 28, outputs 90); one request of 8000 tokens 242 -> 156.  Against 64 bits the
+// 240 us in chunks, 168 here (sums 46, scan 28, outputs 88); one request of 8000 tokens 242 -> 153.  Against 64 bits the
 // outputs' error is 2.47e-7 -> 2.10e-7, the state's 2.18e-7 -> 1.21e-7 (300 tokens: 2.01e-7 -> 2.04e-7, 1.05e-7 -> 1.07e-7).
 // What bounds it: an output tile's phases (16 k clk: splitting q and k 3.3, Q K^T 2.4, Q S with A's split beside it 3.3, A V
 // 1.7, outputs 1.7) that still follow one another for want of shared memory, issue slots 40 % busy, tensor core 29 %; the
@@ -149,21 +149,18 @@ retention_tile_sums_kernel(const __grid_constant__ RetTileParams t) {
     if (there && sg.seg == 0 && tid == 0) t.odd[static_cast<int64_t>(sg.r) * per_tile + hz] = 0x7fffffff;
   };
   auto fetch = [&](uint32_t buf) {  // zeros past the portion
-    const T* kg = reinterpret_cast<const T*>(p.k) + row0 * p.k_stride + static_cast<int64_t>(next.h) * kRcDk;
-    const T* vg = reinterpret_cast<const T*>(p.v) + row0 * p.v_stride + static_cast<int64_t>(next.h) * p.dv + next.z * NC;
-    const uint32_t kd = smem_u32(raw), vd = VS == 1 ? smem_u32(sV) + buf * kV : kd + kRcQ;
+    constexpr int kKRows = kRtSumThreads / 16, kVRows = kRtSumThreads / (NC / 8);  // rows that the CTA takes at once
+    const int kr = tid >> 4, kc = tid & 15, vr = tid / (NC / 8), vc = tid % (NC / 8);
+    const T* kg = reinterpret_cast<const T*>(p.k) + (row0 + next.t0 + kr) * p.k_stride + next.h * kRcDk + kc * 8;
+    const T* vg = reinterpret_cast<const T*>(p.v) + (row0 + next.t0 + vr) * p.v_stride + next.h * p.dv + next.z * NC + vc * 8;
+    const uint32_t kd = smem_u32(raw), vd = (VS == 1 ? smem_u32(sV) + buf * kV : kd + kRcQ) + (vc >> 3) * kRcV;
+    const int left = next.n - next.t0;
 #pragma unroll
-    for (int j = 0; j < kRcTok * 16 / kRtSumThreads; ++j) {
-      const int i = j * kRtSumThreads + tid, r = i >> 4, c = i & 15;
-      const bool ok = next.t0 + r < next.n;
-      cp_async16(kd + rc_raw(r, c), kg + static_cast<int64_t>(ok ? next.t0 + r : 0) * p.k_stride + c * 8, ok);
-    }
+    for (int r = 0; r < kRcTok; r += kKRows, kg += kKRows * p.k_stride)
+      cp_async16(kd + rc_raw(kr + r, kc), kr + r < left ? kg : reinterpret_cast<const T*>(p.k), kr + r < left);
 #pragma unroll
-    for (int j = 0; j < kRcTok * (NC / 8) / kRtSumThreads; ++j) {
-      const int i = j * kRtSumThreads + tid, r = i / (NC / 8), c = i % (NC / 8);
-      const bool ok = next.t0 + r < next.n;
-      cp_async16(vd + (c >> 3) * kRcV + rc_off(r, c & 7), vg + static_cast<int64_t>(ok ? next.t0 + r : 0) * p.v_stride + c * 8, ok);
-    }
+    for (int r = 0; r < kRcTok; r += kVRows, vg += kVRows * p.v_stride)
+      cp_async16(vd + rc_off(vr + r, vc & 7), vr + r < left ? vg : reinterpret_cast<const T*>(p.v), vr + r < left);
     cp_async_commit();
   };
   float4 ang[2][4];  // cos and sin of the fetched rows' pieces u (of u and u + 8, where both are rotated: of u + 8 later)
@@ -609,15 +606,16 @@ retention_tile_kernel(const __grid_constant__ RetTileParams t) {
   } else {
   asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
   auto fetch = [&](int h, const int4& b) {  // raw q, k; zeros past the portion
-    const T* qg = reinterpret_cast<const T*>(p.q) + b.w * p.q_stride + static_cast<int64_t>(h) * kRcDk;
-    const T* kg = reinterpret_cast<const T*>(p.k) + b.w * p.k_stride + static_cast<int64_t>(h) * kRcDk;
+    constexpr int kRows = kRtThreads / 16;  // at once
+    const int r0 = tid >> 4, c = tid & 15;
+    const T* qg = reinterpret_cast<const T*>(p.q) + (b.w + r0) * p.q_stride + h * kRcDk + c * 8;
+    const T* kg = reinterpret_cast<const T*>(p.k) + (b.w + r0) * p.k_stride + h * kRcDk + c * 8;
+    const uint32_t dst = smem_u32(sY);
 #pragma unroll
-    for (int j = 0; j < kRtTok * 16 / kRtThreads; ++j) {
-      const int i = j * kRtThreads + tid, tok = i >> 4, ch = i & 15;
-      const bool ok = tok < b.x;
-      const int64_t at = ok ? tok : 0;
-      cp_async16(smem_u32(sY) + rc_raw(tok, ch), qg + at * p.q_stride + ch * 8, ok);
-      cp_async16(smem_u32(sY) + kRtPart + rc_raw(tok, ch), kg + at * p.k_stride + ch * 8, ok);
+    for (int r = 0; r < kRtTok; r += kRows, qg += kRows * p.q_stride, kg += kRows * p.k_stride) {
+      const bool ok = r0 + r < b.x;
+      cp_async16(dst + rc_raw(r0 + r, c), ok ? qg : reinterpret_cast<const T*>(p.q), ok);
+      cp_async16(dst + kRtPart + rc_raw(r0 + r, c), ok ? kg : reinterpret_cast<const T*>(p.k), ok);
     }
     cp_async_commit();
   };
@@ -645,26 +643,22 @@ retention_tile_kernel(const __grid_constant__ RetTileParams t) {
     const int n = b4.x;
     const uint8_t* state = rt_state(t, h, tile, col0 / NC);
     // v's memory is free since the last A V
-    const T* vg = reinterpret_cast<const T*>(p.v) + b4.w * p.v_stride + static_cast<int64_t>(h) * p.dv + col0;
-    uint4 rv[VS == 2 ? kRtTok * (NC / 8) / kRtThreads : 1];
-    if constexpr (VS == 1) {
+    constexpr int kVRows = kRtThreads / (NC / 8);
+    const int vr = tid / (NC / 8), vc = tid % (NC / 8);
+    const T* vg = reinterpret_cast<const T*>(p.v) + (b4.w + vr) * p.v_stride + h * p.dv + col0 + vc * 8;
+    uint4 rv[VS == 2 ? kRtTok / kVRows : 1];
 #pragma unroll
-      for (int j = 0; j < kRtTok * (NC / 8) / kRtThreads; ++j) {
-        const int i = j * kRtThreads + tid, tok = i / (NC / 8), c = i % (NC / 8);
-        const bool ok = tok < n;
-        cp_async16(smem_u32(sV) + (c >> 3) * kRtBlock + rc_off(tok, c & 7), vg + (ok ? tok : 0) * p.v_stride + c * 8, ok);
-      }
-      cp_async_commit();
-    } else {
-#pragma unroll
-      for (int j = 0; j < kRtTok * (NC / 8) / kRtThreads; ++j) {
-        const int i = j * kRtThreads + tid, tok = i / (NC / 8), c = i % (NC / 8);
-        rv[j] = tok < n ? __ldg(reinterpret_cast<const uint4*>(vg + static_cast<int64_t>(tok) * p.v_stride + c * 8)) : make_uint4(0, 0, 0, 0);
-      }
+    for (int j = 0; j < kRtTok / kVRows; ++j, vg += kVRows * p.v_stride) {
+      const int tok = vr + j * kVRows;
+      if constexpr (VS == 1)
+        cp_async16(smem_u32(sV) + (vc >> 3) * kRtBlock + rc_off(tok, vc & 7), tok < n ? vg : reinterpret_cast<const T*>(p.v), tok < n);
+      else
+        rv[j] = tok < n ? __ldg(reinterpret_cast<const uint4*>(vg)) : make_uint4(0, 0, 0, 0);
     }
+    if constexpr (VS == 1) cp_async_commit();
     const int odd_tile = t.odd[(static_cast<int64_t>(a4.x) * p.H + h) * (p.dv / t.cols) + col0 / t.cols];
     float* pw = powers + par * 132;
-    if (tid <= kRtTok) pw[tid] = power;
+    if (tid <= kRtTok) pw[tid] = power * p.k_scale;  // c d^i
     if (tid == 0) spoilt[par] = 0;
     if constexpr (VS == 1) cp_async_wait<1>();  // (v's copies may still be on their way)
     else cp_async_wait<0>();
@@ -759,24 +753,36 @@ retention_tile_kernel(const __grid_constant__ RetTileParams t) {
     }
     int4 a_next = a4, b_next = b4;
     look(next_tile, a_next, b_next);
+    float back[4];  // d^(i + 1) of the rows that this thread writes
+#pragma unroll
+    for (int e = 0; e < 4; ++e) back[e] = t.powers[h * (kRtTok + 1) + (warp & 3) * 32 + 8 * e + (lane >> 2) + 1];
     // ---- A: decay, mask, split, over k's parts ----
     rt_wait(&done[0], par, warp, dead);
     tc_fence_after_sync();
+    // (rows of a warp: 32 from a multiple of 32 on; columns likewise: whole blocks above the diagonal are zeros)
+    if (quarter > (warp & 3)) {
+#pragma unroll
+      for (int g = 0; g < 4; ++g)
+#pragma unroll
+        for (int q = 0; q < 3; ++q)
+          *reinterpret_cast<uint4*>(sX + q * kRtPart + (quarter >> 1) * kRtBlock + rc_off(row, (quarter * 4 + g) & 7)) = make_uint4(0, 0, 0, 0);
+    } else {
 #pragma unroll 1
-    for (int c = 0; c < 2; ++c) {
-      const int j0 = quarter * 32 + c * 16;
-      uint32_t x[16];
-      tmem_ld_32x32b_x16(tA + lane_base + j0, x);
-      tmem_ld_wait();
+      for (int c = 0; c < 2; ++c) {
+        const int j0 = quarter * 32 + c * 16;
+        uint32_t x[16];
+        tmem_ld_32x32b_x16(tA + lane_base + j0, x);
+        tmem_ld_wait();
 #pragma unroll
-      for (int g = 0; g < 2; ++g) {
-        float y[8];
+        for (int g = 0; g < 2; ++g) {
+          float y[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const int j = j0 + 8 * g + e;
-          y[e] = j <= row ? __uint_as_float(x[8 * g + e]) * (pw[max(row - j, 0)] * p.k_scale) : 0.f;
+          for (int e = 0; e < 8; ++e) {
+            const int age = row - j0 - 8 * g - e;
+            y[e] = age >= 0 ? __uint_as_float(x[8 * g + e]) * pw[max(age, 0)] : 0.f;
+          }
+          rc_split8(y, sX + (quarter >> 1) * kRtBlock + rc_off(row, ((j0 >> 3) + g) & 7), kRtPart);
         }
-        rc_split8(y, sX + ((j0 >> 3) + g >= 8 ? kRtBlock : 0) + rc_off(row, ((j0 >> 3) + g) & 7), kRtPart);
       }
     }
     if constexpr (VS == 1) cp_async_wait<0>();  // v
@@ -814,7 +820,7 @@ retention_tile_kernel(const __grid_constant__ RetTileParams t) {
       for (int e = 0; e < 2; ++e) {
         const int i = (warp & 3) * 32 + hf * 16 + fr + 8 * e;
         if (i < n && mine) {
-          const float f = pw[i + 1];
+          const float f = hf == 0 ? back[e] : back[2 + e];
           float* dst = og + static_cast<int64_t>(i) * p.H * p.dv + fc;
 #pragma unroll
           for (int g = 0; g < kCols / 8; ++g)
