@@ -260,6 +260,14 @@ def _load():
         fn = getattr(lib, name)  # AttributeError if the .so does not export it
         fn.restype = res
         fn.argtypes = args
+    # the per-layer calls without ctypes (csrc/pycalls.cpp): the same functions of the same library
+    try:
+        from . import _calls
+    except ImportError:  # not built, or for another interpreter: ctypes does all
+        return lib
+    functions = {name: (C.cast(getattr(lib, name), _p).value, getattr(lib, name)) for name in SIGNATURES}
+    for name, fn in _calls.bind(functions).items():
+        setattr(lib, name, fn)
     return lib
 
 
