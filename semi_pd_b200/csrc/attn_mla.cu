@@ -31,9 +31,13 @@
 // softmax keeps the true running max per column (see there): scores are read from TMEM in the 16x256b fragment layout (all
 // 32 lanes of a warp busy although M = 64 fills 16 lanes per warp), P goes back as stmatrix-transposed K-major rows.
 //
-// Decode streams each latent row once, 64 requests of 1088 keys (83 MB) in 34 us with the merge launch; one CTA per token,
-// head group and split with warp-level MMAs took 62 us.  About 9000 clk pass until the first tile has landed, then 3000 clk
-// per 72 KB tile and SM.  MMAs (M = 64: 23 clk at N = 16, 31 at N = 64) are hidden as long as the issuer's code stays a
+// Decode streams each latent row once, 64 requests of 1088 keys (83 MB) in 26.3 us with the merge launch, 160 of 1000 in
+// 44.5 in a row; one CTA per token, head group and split with warp-level MMAs took 62 us.  Start, last tile and merge are 14
+// of the 26 us; between them a 72 KB tile takes 1.67 us per SM, which is what its copies alone take.  It took 2.7 us (34.3
+// for the 64 requests) while a tile held its slots for 4000 clk after landing and its copies were issued one after the
+// other: what counts is the time from landing to the last PV (S 1130 clk, softmax 600, PV 700), so the reference of the
+// softmax lags in decode, the two parts of P are columns of one product (V passes once), and Q's copies and a tile's five
+// go out in parallel.  MMAs (M = 64: 23 clk at N = 16, 31 at N = 64) are hidden as long as the issuer's code stays a
 // short loop.  Extend, 4096 new tokens in 4 requests (two with 515 cached), whole layer: 1645 -> 600 us (a batch that takes
 // expanded heads now: 185 us); bounded by the
 // ring of two tiles (a tile's copies start when the PV before last has finished), by the rescale of O^T whenever a tile
@@ -68,12 +72,14 @@ struct MlaParams {
   const int32_t* extend_start_loc;  // extend
   int batch, total, H, hgs;         // total: query tokens (extend); hgs: groups of 16 heads
   int64_t q_stride, out_stride, rtt_stride;
+  int q_row0, q_dir;  // decode: token i is row q_row0 + q_dir i of Q's tensor map
   float scale_log2;
   int min_tiles;   // fewest tiles a CTA takes
   int snap;        // 1: CTA ranges start at item starts, nothing is split
   int cols;        // columns of a partial: TQ x min(H, 16)
   float* o_part;   // [2 * grid][cols][DV]
   float* ml_part;  // [2 * grid][cols][2]
+  int by_item;     // 1: info by item (few of them, see mla_merge_many_kernel), not by the CTA that an item ends in
   int* info;       // [grid][8]: see mla_merge_kernel
   unsigned* wait_expired;
 };
@@ -87,6 +93,7 @@ struct MlaShape {
   // P as the sum of two 16-bit numbers (decode): rounded to one, its error grew 2.3 % over the warp-level kernel's, whose
   // shorter tiles and splits had more probabilities that are exactly 1 (extend: 0.1 % of a layer's, and no room for it)
   static constexpr int kPParts = kExtend ? 1 : 2;
+  static constexpr float kLag = kExtend ? 0.f : 8.f;  // how far (log2) a score may exceed its column's reference
   static constexpr int kPPart = N * 128;
   static constexpr int kPBytes = kPParts * kPPart;
   static constexpr int kPairs = kExtend ? 8 : 11;  // ring slots of 16 KB: one pair of 64-column blocks of a tile
@@ -94,8 +101,9 @@ struct MlaShape {
   static constexpr int kRing = kPairs * 2 * kMlaBlk + kRopes * kMlaBlk;
   static constexpr int kBars = kPairs + kRopes + 4 + 9;
   static constexpr int kSmem = kQBytes + kRing + kPBytes + kMlaMisc + 1024;
-  static constexpr int kOCols = 4 * N;             // TMEM columns of O^T, then two S^T of two halves
-  static constexpr int kTmem = 8 * N;
+  static constexpr int kON = kPParts * N;          // columns of an O^T block: one set for each part of P
+  static constexpr int kOCols = 4 * kON;           // TMEM columns of O^T, then two S^T of two halves
+  static constexpr int kTmem = kExtend ? 512 : 256;
 };
 static_assert(MlaShape<true>::kSmem <= 232448 && MlaShape<false>::kSmem <= 232448 && MlaShape<true>::kTmem <= 512,
               "does not fit an SM");
@@ -309,7 +317,8 @@ __device__ __forceinline__ void mla_stsm_x4_t(uint32_t addr, uint32_t a, uint32_
 
 template <typename T, bool kExtend>
 __global__ void __launch_bounds__(kMlaThreads, 1)
-attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant__ CUtensorMap tmR, const MlaParams p) {
+attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant__ CUtensorMap tmR,
+                const __grid_constant__ CUtensorMap tmQ, const MlaParams p) {
   using S = MlaShape<kExtend>;
   constexpr int N = S::N, TQ = S::TQ;
   extern __shared__ uint8_t mla_smem_raw[];
@@ -350,7 +359,7 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
       mbar_init(p_full, 128);
       mbar_init(p_empty, 1);
       mbar_init(o_empty, 4);
-      mbar_init(q_full, 64);
+      mbar_init(q_full, kExtend ? 64 : 1);
       mbar_init(q_empty, 1);
       *dead = 0;
       fence_barrier_init();
@@ -358,7 +367,13 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
     __syncwarp();
     tmem_alloc(tmem_slot, S::kTmem);
     tmem_relinquish();
+  } else if (tid == 128) {
+    tma_prefetch_desc(&tmKV);
+    tma_prefetch_desc(&tmR);
+    if constexpr (!kExtend) tma_prefetch_desc(&tmQ);
   }
+  // the merge's blocks wait for this grid's end beside its CTAs, instead of being launched then
+  if (!p.snap) griddep_launch_dependents();
   griddep_wait();
 
   // ---- this CTA's range of the tile list ----
@@ -366,7 +381,10 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
   const int per_thread = (p.batch + kMlaThreads - 1) / kMlaThreads;
   const int r0 = tid * per_thread, r1 = min(p.batch, r0 + per_thread);
   int sum = 0;
-  for (int r = r0; r < r1; ++r) sum += mla_request_tiles<kExtend>(p, r);
+  for (int r = r0; r < r1; ++r) {
+    prefetch_l2(p.req_pool_indices + r);  // read next, when the range is known
+    sum += mla_request_tiles<kExtend>(p, r);
+  }
   int incl = sum;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -428,7 +446,7 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
     // (it ran at 190 clk per MMA).
     if (elect_one()) {
       constexpr uint32_t idesc_s = umma_idesc<T>(64, N, 0, 0);   // A = K (K-major), B = Q (K-major)
-      constexpr uint32_t idesc_o = umma_idesc<T>(128, N, 1, 0);  // A = V^T (MN-major), B = P^T (K-major)
+      constexpr uint32_t idesc_o = umma_idesc<T>(128, S::kON, 1, 0);  // A = V^T (MN-major), B = P^T (K-major)
       // descriptors in halves: the upper one is a constant, the lower one moves by 16-byte units
       const uint64_t dk = umma_desc_sw128(smem_u32(sK), 16, 1024), dr = umma_desc_sw128(smem_u32(sR), 16, 1024);
       const uint32_t hi = static_cast<uint32_t>(dk >> 32), k_lo = static_cast<uint32_t>(dk), r_lo = static_cast<uint32_t>(dr);
@@ -451,7 +469,7 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
           mbar_wait_bounded(&s_empty[b], ((ts >> 1) & 1) ^ 1, dead);
           const uint32_t d = tmem_S + b * 2 * N;
           mbar_wait_bounded(&t_full[ts & 3], (ts >> 2) & 1, dead);
-          if (cross || s_gath[ts & 3]) fence_proxy_async_smem();  // Q, and gathered tiles, come by cp.async
+          if ((kExtend && cross) || s_gath[ts & 3]) fence_proxy_async_smem();  // extend's Q and gathered tiles come by cp.async
           tc_fence_after_sync();
           // two accumulators in turn; the softmax adds them
           uint32_t qa = q_lo;
@@ -492,12 +510,8 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
             const uint32_t acc = (!first || k > 0) ? 1u : 0u;
-            umma_ss_lo(tmem_O + i * N, v0 + k * 128, p_lo + k * 2, hi, idesc_o, acc);
-            umma_ss_lo(tmem_O + (i + 1) * N, v1 + k * 128, p_lo + k * 2, hi, idesc_o, acc);
-            if constexpr (S::kPParts == 2) {
-              umma_ss_lo(tmem_O + i * N, v0 + k * 128, p_lo + (S::kPPart >> 4) + k * 2, hi, idesc_o, 1u);
-              umma_ss_lo(tmem_O + (i + 1) * N, v1 + k * 128, p_lo + (S::kPPart >> 4) + k * 2, hi, idesc_o, 1u);
-            }
+            umma_ss_lo(tmem_O + i * S::kON, v0 + k * 128, p_lo + k * 2, hi, idesc_o, acc);
+            umma_ss_lo(tmem_O + (i + 1) * S::kON, v1 + k * 128, p_lo + k * 2, hi, idesc_o, acc);
           }
           umma_commit(&k_empty[slot0]);
           umma_commit(&k_empty[slot1]);
@@ -506,14 +520,114 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
         ++tp;
       }
     }
+  } else if (!kExtend && warp >= 4) {
+    // ===================== loaders, decode =====================
+    // Each warp walks the tiles by itself and looks at all 64 rows: warp 4 copies full tiles, warp 5 an item's Q (which may
+    // have to wait for the last S of the item before), both gather.  The five copies of a tile go out by five lanes, each
+    // when its slot is free: one lane after the other took 3650 clk a tile, more than the tile's time in memory.
+    const T* pool = reinterpret_cast<const T*>(p.kv_pool);
+    const int half = warp - 4;
+    // a row is read once unless there are more heads than an item has: first to leave the L2, 64 requests 27.2 -> 26.3 us
+    const uint64_t policy = p.hgs == 1 ? kEvictFirst : kEvictNormal;
+    int t = 0, gather_age = 4;  // gather_age: tiles since one was gathered
+    const int32_t* page = nullptr;
+    int page_r = -1;
+    auto lookup = [&](const MlaCursor<kExtend>& cc, int& base, int& s0, int& s1) {
+      if (cc.it.r != page_r) {
+        page_r = cc.it.r;
+        page = p.req_to_token + p.req_pool_indices[page_r] * p.rtt_stride;
+      }
+      const int pos = cc.tile * kMlaTile, end = cc.it.load_end;
+      base = pos + kMlaTile <= end ? __ldg(page + pos) : -1;  // a full tile: candidate TMA row
+      s0 = pos + lane < end ? __ldg(page + pos + lane) : -1;
+      s1 = pos + 32 + lane < end ? __ldg(page + pos + 32 + lane) : -1;
+    };
+    MlaSlot<S::kPairs> ks;
+    MlaSlot<S::kRopes> rs;
+    int base = -1, s0 = -1, s1 = -1;
+    if (c.valid) lookup(c, base, s0, s1);
+    bool first = true;
+    while (c.valid) {
+      if (half == 1 && first && lane == 0) {
+        mbar_wait_bounded(q_empty, (c.seg & 1) ^ 1, dead);
+        mbar_expect_tx(q_full, S::kQBytes);
+        tma_load_4d(sQ, &tmQ, q_full, 0, c.it.hg * kMlaHeads, p.q_row0 + p.q_dir * c.it.row0, 0, kEvictFirst);
+      }
+      __syncwarp();
+      first = c.ends(p);
+      c.next(p);
+      int nbase = -1, n0 = -1, n1 = -1;
+      if (c.valid) lookup(c, nbase, n0, n1);  // the next tile's page-table entries, off the critical path
+      const bool contig = __all_sync(0xffffffffu, base >= 0 && s0 == base + lane && s1 == base + 32 + lane);
+      gather_age = contig ? gather_age + 1 : 0;
+      uint64_t* full = &t_full[t & 3];
+      if (contig) {
+        if (half == 0) {
+          if (lane == 0) {
+            s_gath[t & 3] = 0;
+            mbar_expect_tx(full, 9 * kMlaBlk);
+          }
+          __syncwarp();
+          if (gather_age < 4) fence_proxy_async_smem();  // the slots may last have been written by the gather path
+          int at = ks.i + lane;  // of lanes 0-3; lane 4: the rope block
+          uint32_t round = ks.round;
+          if (at >= S::kPairs) {
+            at -= S::kPairs;
+            round ^= 1;
+          }
+          uint64_t* empty = lane < 4 ? &k_empty[at] : &r_empty[rs.i];
+          if (lane == 4) round = rs.round;
+          bool todo = lane < 5;
+#pragma unroll 1
+          for (int i = 0; __any_sync(0xffffffffu, todo); ++i) {
+            if (todo && (mbar_test(empty, round ^ 1) || *dead || i == kMbarWaitTries)) {
+              if (i == kMbarWaitTries) *dead = 1;
+              if (lane < 4)
+                tma_load_3d(sK + at * 2 * kMlaBlk, &tmKV, full, 0, base, 2 * lane, policy);
+              else
+                tma_load_2d(sR + rs.i * kMlaBlk, &tmR, full, kMlaDV, base, policy);
+              todo = false;
+            }
+          }
+          if (lane == 0) mbar_arrive_n(full, 64);
+        } else {
+          mbar_wait_bounded(&r_empty[rs.i], rs.round ^ 1, dead);  // so that warp 5 is never a round of a slot ahead
+        }
+#pragma unroll
+        for (int st = 0; st < 4; ++st) ks.next();
+        rs.next();
+      } else {
+        if (half == 0 && lane == 0) s_gath[t & 3] = 1;
+#pragma unroll 1
+        for (int st = 0; st < 5; ++st) {
+          uint8_t* dst = st < 4 ? sK + ks.i * 2 * kMlaBlk : sR + rs.i * kMlaBlk;
+          mbar_wait_bounded(st < 4 ? &k_empty[ks.i] : &r_empty[rs.i], (st < 4 ? ks.round : rs.round) ^ 1, dead);
+          __syncwarp();
+          const int shift = st < 4 ? 4 : 3;  // log2 of the 16-byte chunks of a row in a pair / in the rope block
+#pragma unroll 4
+          for (int i = half * 32 + lane; i < kMlaTile << shift; i += 64) {
+            const int row = i >> shift, ch = i - (row << shift);
+            const int a = __shfl_sync(0xffffffffu, s0, row & 31), b = __shfl_sync(0xffffffffu, s1, row & 31);
+            const int sl = row < 32 ? a : b;
+            cp_async16(smem_u32(dst + (ch >> 3) * kMlaBlk + mla_off(row, ch & 7)),
+                       pool + static_cast<int64_t>(sl < 0 ? 0 : sl) * kMlaDL + st * 128 + ch * 8, sl >= 0);
+          }
+          if (st < 4) ks.next(); else rs.next();
+        }
+        cp_async_mbar_arrive_noinc(full);
+        if (half == 0 && lane == 0) mbar_arrive(full);
+      }
+      ++t;
+      base = nbase;
+      s0 = n0;
+      s1 = n1;
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
   } else if (warp >= 4) {
-    // ===================== loaders =====================
+    // ===================== loaders, extend =====================
     const int lt = tid - 128;  // 0..63: also the row of a tile this thread looks up
     const T* pool = reinterpret_cast<const T*>(p.kv_pool);
-    if (lt == 0) {
-      tma_prefetch_desc(&tmKV);
-      tma_prefetch_desc(&tmR);
-    }
     int t = 0, gather_age = 4;  // gather_age: tiles since one was gathered
     auto lookup = [&](const MlaCursor<kExtend>& cc, int& base) {
       const int32_t* page = p.req_to_token + p.req_pool_indices[cc.it.r] * p.rtt_stride;
@@ -606,14 +720,15 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
     const int col0 = 2 * (lane & 3);
     if (tid == 0 && !p.snap) {
       // what the merge kernel needs of an item that began in an earlier CTA and ends here
-      int* info = p.info + cta * 8;
+      int* info = p.info + (p.by_item ? c.it.hg * p.batch + c.it.r : cta) * 8;
       const bool tail = t_count > 0 && c.tile > 0 && c.it.ntiles - c.tile <= t_count;
-      info[0] = tail;
+      if (tail || !p.by_item) info[0] = tail;
       if (tail) {
         info[1] = (t_begin - c.tile) / per;  // CTA of the item's first tile (tiles are consecutive units)
         info[2] = c.it.row0;
         info[3] = c.it.ntok;
         info[4] = c.it.hg * kMlaHeads;
+        info[5] = cta;
       }
     }
     int t = 0;
@@ -651,11 +766,12 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
         }
         bool exceed = false;
 #pragma unroll
-        for (int i = 0; i < N / 2; ++i) exceed |= s[i] > m_ref[(i >> 2) * 2 + (i & 1)];
+        for (int i = 0; i < N / 2; ++i) exceed |= s[i] > m_ref[(i >> 2) * 2 + (i & 1)] + S::kLag;
         if (mla_bar_or(exceed)) {
-          // The true running max per column, so that a column's largest P is exactly 1: a reference that lags by up to 2^8
-          // saves most of these rescales but rounds that P too (decode: 32.4 instead of 33.8 us and extend 548
-          // instead of 600, but 6 - 14 % more rms error against 64-bit results where P has one part).
+          // The running max per column.  Where P has one part it is the true one, so that a column's largest P is exactly 1: a
+          // reference that lags by up to 2^8 saves most of these rescales (900 of 1500 clk from S to P) but rounds that P
+          // too (extend 548 instead of 600 us, but 6 - 14 % more rms error against 64-bit results).  With two parts
+          // nothing is rounded that counts.
 #pragma unroll
           for (int i = 0; i < C; ++i) {
             float m = fmaxf(s[(i >> 1) * 4 + (i & 1)], s[(i >> 1) * 4 + 2 + (i & 1)]);
@@ -681,7 +797,7 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
             mbar_wait_bounded(p_empty, (t & 1) ^ 1, dead);  // PV of the previous tile has finished: O^T is stable
             tc_fence_after_sync();
 #pragma unroll 1
-            for (int cc = 0; cc < 4 * N; cc += 16) {
+            for (int cc = 0; cc < S::kOCols; cc += 16) {
               uint32_t o[16];
               tmem_ld_32x32b_x16(tmem_O + lane_base + cc, o);
               tmem_ld_wait();
@@ -730,6 +846,7 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
       }
       // ---- epilogue: column sums over the kv rows of all tiles, then O^T / sum (or the partial as it is) ----
       const bool whole = tile0 == 0 && tile_last + 1 == it.ntiles;
+      if (tid == 0 && whole && p.by_item) p.info[(it.hg * p.batch + it.r) * 8] = 0;
       const int h0 = it.hg * kMlaHeads, nh = min(kMlaHeads, p.H - h0), nhm = min(kMlaHeads, p.H);
       const int64_t part0 = static_cast<int64_t>(2 * cta + (tile0 > 0 ? 0 : 1)) * p.cols;
 #pragma unroll
@@ -768,8 +885,16 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
         for (int blk = 0; blk < 4; ++blk, dst += 128) {
           uint32_t o[N];
 #pragma unroll
-          for (int cc = 0; cc < N; cc += 16) tmem_ld_32x32b_x16(tmem_O + lane_base + blk * N + cc, o + cc);
-          tmem_ld_wait();
+          for (int cc = 0; cc < N; cc += 16) tmem_ld_32x32b_x16(tmem_O + lane_base + blk * S::kON + cc, o + cc);
+          if constexpr (S::kPParts == 2) {
+            uint32_t lo[N];
+            tmem_ld_32x32b_x16(tmem_O + lane_base + blk * S::kON + N, lo);
+            tmem_ld_wait();
+#pragma unroll
+            for (int e = 0; e < N; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) + __uint_as_float(lo[e]));
+          } else {
+            tmem_ld_wait();
+          }
 #pragma unroll
           for (int cc = 0; cc < N; cc += 16) {
             if ((cc >> 4) >= it.ntok) break;
@@ -797,8 +922,16 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
         for (int blk = 0; blk < 4; ++blk, dst += 128) {
           uint32_t o[N];
 #pragma unroll
-          for (int cc = 0; cc < N; cc += 16) tmem_ld_32x32b_x16(tmem_O + lane_base + blk * N + cc, o + cc);
-          tmem_ld_wait();
+          for (int cc = 0; cc < N; cc += 16) tmem_ld_32x32b_x16(tmem_O + lane_base + blk * S::kON + cc, o + cc);
+          if constexpr (S::kPParts == 2) {
+            uint32_t lo[N];
+            tmem_ld_32x32b_x16(tmem_O + lane_base + blk * S::kON + N, lo);
+            tmem_ld_wait();
+#pragma unroll
+            for (int e = 0; e < N; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) + __uint_as_float(lo[e]));
+          } else {
+            tmem_ld_wait();
+          }
 #pragma unroll
           for (int cc = 0; cc < N; cc += 16) {
             if ((cc >> 4) >= it.ntok) break;
@@ -887,7 +1020,7 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
     }
   }
 
-  griddep_launch_dependents();
+  if (p.snap) griddep_launch_dependents();
   tc_fence_before_sync();
   __syncthreads();
   if (*dead) {
@@ -899,10 +1032,11 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
 
 // Merges the parts of the items that span several CTAs.  Block (c, 4 columns) serves the item that ends in CTA c after
 // beginning in CTA info[1] < c: that CTA left its part in slot 2 info[1] + 1, the following ones up to c in slot 2 i.
-// info: {any, first CTA, first query row, tokens, first head}.
+// info: {any, first CTA, first query row, tokens, first head, last CTA}.
 template <typename T>
 __global__ void __launch_bounds__(512)
 mla_merge_kernel(const MlaParams p) {
+  griddep_launch_dependents();
   griddep_wait();
   const int c = blockIdx.x, nhm = min(kMlaHeads, p.H);
   const int* info = p.info + c * 8;
@@ -931,6 +1065,53 @@ mla_merge_kernel(const MlaParams p) {
   T* dst = reinterpret_cast<T*>(p.out) + (static_cast<int64_t>(info[2]) + tok) * p.out_stride +
            static_cast<int64_t>(info[4] + h) * kMlaDV + x * 4;
   *reinterpret_cast<uint2*>(dst) = make_uint2(pack2<T>(num.x * inv, num.y * inv), pack2<T>(num.z * inv, num.w * inv));
+}
+
+// The same for few items, which then have many parts each (one request of 8000 keys: 63, read in 20 us by one thread after
+// the other part).  Block (item, column): a warp takes 32 of the column's 512 values, each quarter of it every fourth part
+// with eight on the way; the quarters meet by shuffles, since shared memory would keep the blocks from waiting beside the
+// attention's CTAs.  (Where an item has two or three parts the shuffles cost more than they save: 27.2 -> 28.2 us for 64
+// requests of 1088 keys.)
+template <typename T>
+__global__ void __launch_bounds__(512)
+mla_merge_many_kernel(const MlaParams p) {
+  griddep_launch_dependents();
+  griddep_wait();
+  const int* info = p.info + blockIdx.x * 8;
+  const int col = blockIdx.y;  // a head of the item's one token
+  if (!info[0] || info[4] + col >= p.H) return;
+  const int lane = threadIdx.x & 31, g = lane >> 3, x = (threadIdx.x >> 5) * 8 + (lane & 7);
+  const int c0 = info[1], c = info[5];
+  auto at = [&](int i) { return static_cast<int64_t>(i == c0 ? 2 * i + 1 : 2 * i) * p.cols + col; };
+  const float2* ml = reinterpret_cast<const float2*>(p.ml_part);
+  const float4* o_part = reinterpret_cast<const float4*>(p.o_part) + x;
+  float M = -INFINITY, den = 0.f;
+  float4 num = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+  for (int i = c0 + g; i <= c; i += 4) M = fmaxf(M, ml[at(i)].x);  // (-inf where a part saw no key)
+  M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, 8));
+  M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, 16));
+#pragma unroll 8
+  for (int i = c0 + g; i <= c; i += 4) {
+    const float2 v = ml[at(i)];
+    const float4 o = o_part[at(i) * (kMlaDV / 4)];
+    const float w = v.y > 0.f ? fast_exp2(v.x - M) : 0.f;
+    num.x = fmaf(w, o.x, num.x);
+    num.y = fmaf(w, o.y, num.y);
+    num.z = fmaf(w, o.z, num.z);
+    num.w = fmaf(w, o.w, num.w);
+    den = fmaf(w, v.y, den);
+  }
+  auto all4 = [](float v) {
+    v += __shfl_xor_sync(0xffffffffu, v, 8);
+    return v + __shfl_xor_sync(0xffffffffu, v, 16);
+  };
+  const float d = all4(den), n0 = all4(num.x), n1 = all4(num.y), n2 = all4(num.z), n3 = all4(num.w);
+  const float inv = d > 0.f ? 1.f / d : 0.f;
+  if (g == 0)
+    *reinterpret_cast<uint2*>(reinterpret_cast<T*>(p.out) + static_cast<int64_t>(info[2]) * p.out_stride +
+                              static_cast<int64_t>(info[4] + col) * kMlaDV + x * 4) =
+        make_uint2(pack2<T>(n0 * inv, n1 * inv), pack2<T>(n2 * inv, n3 * inv));
 }
 
 // What stands between the fused q / latent projection and the attention, one CTA per token: the latent row (RMS norm of
@@ -987,19 +1168,35 @@ mla_rotary_store_kernel(T* q_rot, const T* qa, T* __restrict__ pool, const T* __
 }
 
 template <typename T, bool kExtend>
-static int mla_launch(const MlaParams& p, int grid, cudaStream_t st) {
-  CUtensorMap tm, tr;
+static int mla_launch(MlaParams p, int grid, cudaStream_t st) {
+  CUtensorMap tm, tr, tq{};
   // the C-ABI does not carry the pool's slot count: rows are slot ids read from req_to_token, so the maximum is declared
   if (int rc = make_tmap_blocks_sw128(&tm, p.kv_pool, 1ull << 31, 9, kMlaDL, kMlaTile, 2)) return rc;
   if (int rc = get_tmap(&tr, p.kv_pool, 1ull << 31, kMlaDL, kMlaDL, kMlaTile)) return rc;
+  if constexpr (!kExtend) {
+    // [64 columns, heads, tokens, 9 blocks] of Q: an item's 16 heads in one copy, zeros where there is no head.  A row
+    // stride of zero or below is served from the lowest address.
+    const int64_t stride = p.q_stride < 0 ? -p.q_stride : p.q_stride;
+    p.q_dir = p.q_stride > 0 ? 1 : p.q_stride < 0 ? -1 : 0;
+    p.q_row0 = p.q_stride < 0 ? p.batch - 1 : 0;
+    const T* low = reinterpret_cast<const T*>(p.q) + (p.q_stride < 0 ? (p.batch - 1) * p.q_stride : 0);
+    const uint64_t rows = p.q_stride == 0 ? 1 : p.batch;
+    const uint64_t dims[4] = {64, static_cast<uint64_t>(p.H), rows, 9};
+    const uint64_t strides[3] = {kMlaDL, static_cast<uint64_t>(stride > 0 ? stride : kMlaDL), 64};
+    const uint32_t box[4] = {64, kMlaHeads, 1, 9};
+    if (int rc = make_tmap_sw128(&tq, low, 4, dims, strides, box)) return rc;
+  }
   auto kern = attn_mla_kernel<T, kExtend>;
   static bool configured = false;
   if (!configured) {
     SPD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MlaShape<kExtend>::kSmem));
     configured = true;
   }
-  SPD_CUDA(launch(kern, dim3(grid), dim3(kMlaThreads), MlaShape<kExtend>::kSmem, st, pdl_enabled(), tm, tr, p));
-  if (!p.snap) SPD_CUDA(launch(mla_merge_kernel<T>, dim3(grid, (p.cols + 3) / 4), dim3(512), 0, st, pdl_enabled(), p));
+  SPD_CUDA(launch(kern, dim3(grid), dim3(kMlaThreads), MlaShape<kExtend>::kSmem, st, pdl_enabled(), tm, tr, tq, p));
+  if (p.by_item)
+    SPD_CUDA(launch(mla_merge_many_kernel<T>, dim3(p.batch * p.hgs, p.cols), dim3(512), 0, st, pdl_enabled(), p));
+  else if (!p.snap)
+    SPD_CUDA(launch(mla_merge_kernel<T>, dim3(grid, (p.cols + 3) / 4), dim3(512), 0, st, pdl_enabled(), p));
   return 0;
 }
 
@@ -1119,6 +1316,7 @@ static int attn_mla(void* out, const void* q, const void* kv_pool, const int32_t
     p.o_part = reinterpret_cast<float*>(workspace);
     p.ml_part = p.o_part + rows * kMlaDV;
     p.info = reinterpret_cast<int*>(p.ml_part + rows * 2);
+    p.by_item = !extend && 4 * groups <= grid;
   }
   cudaStream_t st = as_stream(stream);
   SPD_DISPATCH_DTYPE(dtype, {
