@@ -175,30 +175,6 @@ __device__ __forceinline__ bool softmax_bar_or(bool pred) {
   return out != 0;
 }
 __device__ __forceinline__ void softmax_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
-// barrier + AND-reduction over the 64 threads of one loader group (named barrier 2: K, 3: V)
-__device__ __forceinline__ bool loader_bar_and(bool pred, int is_v) {
-  uint32_t out;
-  if (is_v) {
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t"
-        "setp.ne.u32 q, %1, 0;\n\t"
-        "barrier.cta.red.and.pred p, 3, 64, q;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}\n"
-        : "=r"(out)
-        : "r"(static_cast<uint32_t>(pred))
-        : "memory");
-  } else {
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t"
-        "setp.ne.u32 q, %1, 0;\n\t"
-        "barrier.cta.red.and.pred p, 2, 64, q;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}\n"
-        : "=r"(out)
-        : "r"(static_cast<uint32_t>(pred))
-        : "memory");
-  }
-  return out != 0;
-}
 
 template <typename T>
 __global__ void __launch_bounds__(kDcThreads, 1)
@@ -255,6 +231,8 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     tmem_alloc(tmem_slot, 64);
     tmem_relinquish();
   }
+  if (threadIdx.x == 128) tma_prefetch_desc(&tmK);
+  if (threadIdx.x == 192) tma_prefetch_desc(&tmV);
   // zero P / Q staging once: rows >= G are never written and only feed ignored output columns
   for (int i = threadIdx.x; i < ((kDcQBufs + 2) * kDcQBytes) / 16; i += kDcThreads)
     reinterpret_cast<uint4*>(sQ)[i] = make_uint4(0, 0, 0, 0);
@@ -274,6 +252,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
   for (int b = b0; b < b1; ++b) {
     const int L = static_cast<int>(p.seq_lens[b]);
     if (b < kDcLenCache) s_len[b] = L;
+    prefetch_l2(p.req_pool_indices + b);  // read when the range is known
     sum += (dc_tiles(L) + kDcItemUnits) * p.Hk;
   }
   const int warp_units = __reduce_add_sync(0xffffffffu, sum);
@@ -334,6 +313,13 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     if (elect_one()) {
       constexpr uint32_t idesc_s = umma_idesc<T>(128, kDcN, 0, 0);  // A = K (K-major), B = Q (K-major)
       constexpr uint32_t idesc_o = umma_idesc<T>(128, kDcN, 1, 0);  // A = V (MN-major), B = P^T (K-major)
+      // descriptors in halves: the upper one is a constant, the lower one moves by 16-byte units (put together for every
+      // MMA, the two streams' 16 a tile made it 51.6 us, so 50.0: the tile waits for them)
+      const uint64_t dk = umma_desc_sw128(smem_u32(sK), 16, 1024);
+      const uint32_t hi = static_cast<uint32_t>(dk >> 32), k_lo = static_cast<uint32_t>(dk);
+      const uint32_t q_lo = static_cast<uint32_t>(umma_desc_sw128(smem_u32(sQ), 16, 1024));
+      const uint32_t v_lo = static_cast<uint32_t>(umma_desc_sw128(smem_u32(sV), 16384, 1024));
+      const uint32_t p_lo = static_cast<uint32_t>(umma_desc_sw128(smem_u32(sP), 16, 1024));
       DcCursor cs = c, cp = c;  // cs runs one tile ahead of cp
       int ts = 0;  // global tile counter of the S stream
       auto issue_s = [&]() {
@@ -342,15 +328,11 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
         fence_proxy_async_smem();  // cp.async (generic proxy) writes -> UMMA operand reads
         mbar_wait(&s_empty[sb], ((ts >> 1) & 1) ^ 1);
         tc_fence_after_sync();
-        const uint32_t k_addr = smem_u32(sK + st * kDcTileBytes);
-        const uint32_t q_addr = smem_u32(sQ + (cs.iter % kDcQBufs) * kDcQBytes);
+        const uint32_t ka = k_lo + st * (kDcTileBytes >> 4), qa = q_lo + (cs.iter % kDcQBufs) * (kDcQBytes >> 4);
 #pragma unroll
-        for (int k = 0; k < kDcD / 16; ++k) {
-          umma_ss(tmem_S + sb * kDcN,
-                  umma_desc_sw128(k_addr + (k >> 2) * 16384 + (k & 3) * 32, 16, 1024),
-                  umma_desc_sw128(q_addr + (k >> 2) * 2048 + (k & 3) * 32, 16, 1024), idesc_s,
-                  k > 0 ? 1u : 0u);
-        }
+        for (int k = 0; k < kDcD / 16; ++k)
+          umma_ss_lo(tmem_S + sb * kDcN, ka + (k >> 2) * (16384 >> 4) + (k & 3) * 2, qa + (k >> 2) * (2048 >> 4) + (k & 3) * 2,
+                     hi, idesc_s, k > 0 ? 1u : 0u);
         umma_commit(&k_empty[st]);  // K_t: consumed once these MMAs have read it
         umma_commit(&s_full[sb]);
         ++ts;
@@ -371,14 +353,11 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
           ++o_uses[ob];
         }
         tc_fence_after_sync();
-        const uint32_t v_addr = smem_u32(sV + st * kDcTileBytes);
-        const uint32_t p_addr = smem_u32(sP + pb * kDcQBytes);
+        const uint32_t va = v_lo + st * (kDcTileBytes >> 4), pa = p_lo + pb * (kDcQBytes >> 4);
 #pragma unroll
-        for (int k = 0; k < kDcTile / 16; ++k) {
-          umma_ss(tmem_O + ob * kDcN, umma_desc_sw128(v_addr + k * 2048, 16384, 1024),
-                  umma_desc_sw128(p_addr + (k >> 2) * 2048 + (k & 3) * 32, 16, 1024), idesc_o,
-                  (!first || k > 0) ? 1u : 0u);
-        }
+        for (int k = 0; k < kDcTile / 16; ++k)
+          umma_ss_lo(tmem_O + ob * kDcN, va + k * (2048 >> 4), pa + (k >> 2) * (2048 >> 4) + (k & 3) * 2, hi, idesc_o,
+                     (!first || k > 0) ? 1u : 0u);
         umma_commit(&v_empty[st]);
         umma_commit(&p_empty[pb]);
         umma_commit(o_done);
@@ -401,37 +380,35 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     uint64_t* empty = is_v ? v_empty : k_empty;
     const int64_t row_elems = static_cast<int64_t>(p.Hk) * kDcD;
     int t = 0;
-    // Page-table lookups run ONE TILE AHEAD of the gather (32 slots per thread), so the dependent
-    // chain req_pool_indices -> req_to_token -> pool row is off the issue path.
+    // Page-table lookups run ONE TILE AHEAD of the gather, so the dependent chain req_pool_indices -> req_to_token -> pool
+    // row is off the issue path.  Each warp looks at the whole tile, four rows a lane: with 32 rows a thread and a vote
+    // between the two warps, 64 requests of 1088 tokens took 53.1 us, so 51.6.
     // `base` = slot of the tile's first row when the tile is FULL (else -1): the candidate TMA row.
     auto lookup = [&](const DcCursor& cc, int* sl, int& base) {
       const int32_t* rtt0 = p.req_to_token + p.req_pool_indices[cc.b] * p.rtt_stride;
       const int tile0 = cc.tile * kDcTile;
-      const int tokb = tile0 + rsub;
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const int tok = tokb + i * 4;
+      for (int i = 0; i < 4; ++i) {
+        const int tok = tile0 + lane + i * 32;
         sl[i] = tok < cc.L ? __ldg(rtt0 + tok) : -1;
       }
       base = (p.use_tma && tile0 + kDcTile <= cc.L) ? __ldg(rtt0 + tile0) : -1;
     };
     const CUtensorMap* tmap = is_v ? &tmV : &tmK;
-    if (lt == 0) tma_prefetch_desc(tmap);
-    int slot[32], base = -1;
+    int slot[4], base = -1;
     if (c.valid) lookup(c, slot, base);
     while (c.valid) {
       const int st = t % kDcStages;
       const int b = c.b, hk = c.hk, citer = c.iter;
       const bool load_q = c.tile == c.tile0;
       c.next(p, s_len);
-      int nslot[32], nbase = -1;
+      int nslot[4], nbase = -1;
       if (c.valid) lookup(c, nslot, nbase);
-      // Are the tile's 128 page-table entries consecutive slots?  Each thread checks its 32 rows
-      // against the first row's slot; the group agrees through one barrier-with-AND.
+      // Are the tile's 128 page-table entries consecutive slots?
       bool contig = base > 0;
 #pragma unroll
-      for (int i = 0; i < 32; ++i) contig &= (slot[i] == base + i * 4 + rsub);
-      if (p.use_tma) contig = loader_bar_and(contig, is_v);
+      for (int i = 0; i < 4; ++i) contig &= (slot[i] == base + i * 32 + lane);
+      contig = __all_sync(0xffffffffu, contig);
       mbar_wait(&empty[st], ((t / kDcStages) & 1) ^ 1);
       if (!is_v && load_q) {
         // stage the G query rows of this (request, kv head) as the K-major B operand, in the same
@@ -459,8 +436,9 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
           const int row = i * 4 + rsub;
-          const bool valid = slot[i] >= 0;
-          const int64_t s64 = valid ? slot[i] : 0;
+          const int sl = __shfl_sync(0xffffffffu, slot[i >> 3], row & 31);
+          const bool valid = sl >= 0;
+          const int64_t s64 = valid ? sl : 0;
           cp_async16(dst + dc_tile_off(row, chunk), pool + s64 * row_elems + col, valid);
         }
       }
@@ -474,7 +452,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
       ++t;
       base = nbase;
 #pragma unroll
-      for (int i = 0; i < 32; ++i) slot[i] = nslot[i];
+      for (int i = 0; i < 4; ++i) slot[i] = nslot[i];
     }
   } else {
     // ===================== softmax / correction / epilogue =====================

@@ -372,8 +372,6 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
     tma_prefetch_desc(&tmR);
     if constexpr (!kExtend) tma_prefetch_desc(&tmQ);
   }
-  // the merge's blocks wait for this grid's end beside its CTAs, instead of being launched then
-  if (!p.snap) griddep_launch_dependents();
   griddep_wait();
 
   // ---- this CTA's range of the tile list ----
@@ -395,6 +393,9 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  // the merge's blocks wait for this grid's end beside its CTAs, instead of being launched then (from here on, since whatever
+  // follows them may want tensor memory and this CTA has its own now)
+  if (!p.snap) griddep_launch_dependents();
   int before = 0, all = 0;
 #pragma unroll
   for (int w = 0; w < kMlaThreads / 32; ++w) {
