@@ -274,6 +274,7 @@ __device__ __forceinline__ bool mla_bar_or(bool pred) {  // barrier + OR over th
   return out != 0;
 }
 __device__ __forceinline__ void mla_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+__device__ __forceinline__ void mla_loader_bar() { asm volatile("bar.sync 2, 64;" ::: "memory"); }  // the loader threads
 __device__ __forceinline__ bool mla_loader_and(bool pred) {  // barrier + AND over the 64 loader threads
   uint32_t out;
   asm volatile(
@@ -523,7 +524,7 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
     }
   } else if (!kExtend && warp >= 4) {
     // ===================== loaders, decode =====================
-    // Each warp walks the tiles by itself and looks at all 64 rows: warp 4 copies full tiles, warp 5 an item's Q (which may
+    // Each warp looks at all 64 rows of a tile: warp 4 copies full tiles, warp 5 an item's Q (which may
     // have to wait for the last S of the item before), both gather.  The five copies of a tile go out by five lanes, each
     // when its slot is free: one lane after the other took 3650 clk a tile, more than the tile's time in memory.
     const T* pool = reinterpret_cast<const T*>(p.kv_pool);
@@ -549,17 +550,21 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
     if (c.valid) lookup(c, base, s0, s1);
     bool first = true;
     while (c.valid) {
-      if (half == 1 && first && lane == 0) {
-        mbar_wait_bounded(q_empty, (c.seg & 1) ^ 1, dead);
-        mbar_expect_tx(q_full, S::kQBytes);
-        tma_load_4d(sQ, &tmQ, q_full, 0, c.it.hg * kMlaHeads, p.q_row0 + p.q_dir * c.it.row0, 0, kEvictFirst);
-      }
-      __syncwarp();
+      const int row0 = c.it.row0, hg = c.it.hg, seg = c.seg;
+      const bool load_q = first;
       first = c.ends(p);
       c.next(p);
       int nbase = -1, n0 = -1, n1 = -1;
       if (c.valid) lookup(c, nbase, n0, n1);  // the next tile's page-table entries, off the critical path
       const bool contig = __all_sync(0xffffffffu, base >= 0 && s0 == base + lane && s1 == base + 32 + lane);
+      // tile by tile together: a warp ahead or behind by two rounds of a slot would take one phase of its barrier for another
+      mla_loader_bar();
+      if (half == 1 && load_q && lane == 0) {
+        mbar_wait_bounded(q_empty, (seg & 1) ^ 1, dead);
+        mbar_expect_tx(q_full, S::kQBytes);
+        tma_load_4d(sQ, &tmQ, q_full, 0, hg * kMlaHeads, p.q_row0 + p.q_dir * row0, 0, kEvictFirst);
+      }
+      __syncwarp();
       gather_age = contig ? gather_age + 1 : 0;
       uint64_t* full = &t_full[t & 3];
       if (contig) {
@@ -591,8 +596,6 @@ attn_mla_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant_
             }
           }
           if (lane == 0) mbar_arrive_n(full, 64);
-        } else {
-          mbar_wait_bounded(&r_empty[rs.i], rs.round ^ 1, dead);  // so that warp 5 is never a round of a slot ahead
         }
 #pragma unroll
         for (int st = 0; st < 4; ++st) ks.next();
