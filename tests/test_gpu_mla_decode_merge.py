@@ -69,3 +69,9 @@ def test_query_row_strides(stride):
                                sl.data_ptr(), None, None, 4, 4, H, R, DR, stride, out.stride(0), rtt_d.stride(0), 0.07,
                                SPD_BF16, ws.data_ptr(), ws.numel(), 0, torch.cuda.current_stream().cuda_stream), "mla")
     assert (out.cpu().double().view(want.shape) - want).abs().max().item() < TOL[torch.bfloat16]
+
+
+@pytest.mark.parametrize("lens", [[100] * 20, [65, 128, 64, 129] * 9, [1] * 30, [64] * 40, [6080], [6081, 6200], [6150, 1, 12300]])
+def test_least_units_per_cta(lens):
+    # items of just three units are not cut, very long ones are cut into ranges of four
+    _run([n - 1 for n in lens], [1] * len(lens), 16, torch.bfloat16, "runs", True)
