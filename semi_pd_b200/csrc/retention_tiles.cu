@@ -846,7 +846,9 @@ retention_tile_kernel(const __grid_constant__ RetTileParams t) {
             rc_load8<__nv_bfloat16>(reinterpret_cast<const __nv_bfloat16*>(state + q * kS + blk * kRtBlock + rc_off(sr, (sc >> 3) + c)), x[q]);
           for (int e = 0; e < 8; ++e) {
             const float sum = (x[0][e] + x[1][e]) + x[2][e];
-            from[8 * c + e] = fabsf(sum) <= 0x1p64f ? sum : st[8 * c + e];  // (no parts: the portion's first state, untouched)
+            // (no parts: the portion's first state, which stands untouched.  Behind an earlier tile a state is finite and has
+            // parts however large it is, and what stands in memory is the portion's last one.)
+            from[8 * c + e] = a4.y > 0 || fabsf(sum) <= 0x1p64f ? sum : st[8 * c + e];
           }
         }
         rc_token_by_token<T, 1>(&p, 0, rest ? b4.y : n, b4.z, b4.w, reinterpret_cast<float*>(sX), from, rest ? st : nullptr, p.decay[h], h,

@@ -79,3 +79,21 @@ def test_values_that_are_not_finite(dtype, what, at):
         assert torch.equal(a.isnan(), b.isnan())
         small = fine & (b.abs() < 1e30)
         assert _rel(a[small], b[small]) < 1e-6
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("what", ["q", "k", "v"])
+@pytest.mark.parametrize("at", [130, 383, 700])
+def test_a_large_state_before_a_tile_that_is_not_finite(dtype, what, at):
+    """The state that one key of the first tile makes is above 2^64, and a later tile goes on from it token by token."""
+    pre, ext, H, dv, scale = [4, 0], [768, 400], 2, 128, 2.0 ** 40
+    q, k, v, state, table, decay = _case(pre, ext, H, dv, 64, dtype, [0.99, 0.9999])
+    assert _tiled(ext, H, dv, 64, dtype)
+    for h in range(H):
+        k[10, h * DK + 100], v[10, h * dv: (h + 1) * dv: 3] = 2.0 ** 15, -2.0 ** 15
+    {"q": q, "k": k, "v": v}[what][at, 70] = float("nan")
+    case = (q, k, v, state, table, decay)
+    for a, b in zip(_run(*case, pre, ext, H, dv, 64, scale), _want(*case, pre, ext, H, dv, 64, scale)):
+        assert torch.equal(a.isnan(), b.isnan())
+        # as above: sums of at most some hundred terms in fp32
+        assert _rel(a[b.isfinite()], b[b.isfinite()]) < 1e-6
