@@ -175,12 +175,18 @@ int spd_bias_act_residual(void* out, const void* x, const void* bias, const void
  * (spd_gemm_workspace_bytes()), zero-initialised ONCE by the caller and then owned by one stream
  * (the kernels re-arm the flags themselves; two streams must not share one workspace).  May be
  * NULL: the call then never splits a tile.
+ * W: up to 256 tokens without an epilogue, W is read before this call waits for the kernels right before it in the stream, each
+ * of which may have let the next one in early: it must not be what one of this library's kernels writes there, unless another
+ * kind of launch (a copy, a kernel of another library) stands in between.  A model's weights never are.  Other calls may
+ * multiply by what the kernel before has just written, unless SPD_EPI_OLDER_W is added to the epilogue, which says the same of
+ * W there.
  * sm_budget: number of SMs the call may occupy (0 = all); a worker running on a green-context
  * partition passes its partition's SM count so that persistent grids and the stream-K split match it.
  * ------------------------------------------------------------------------------------------- */
 #define SPD_EPI_NONE 0
 #define SPD_EPI_SILU_MUL 1
 #define SPD_EPI_GELU 2
+#define SPD_EPI_OLDER_W 256
 int64_t spd_gemm_workspace_bytes(void);
 /* CTAs (pairs of CTAs) over which a decode GEMM that splits along K cuts its tiles x kblocks units, of `slots` that run at
  * once; split: contributors per tile that it aims at (4). */

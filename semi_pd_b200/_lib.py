@@ -23,6 +23,7 @@ SPD_F32 = 2
 SPD_EPI_NONE = 0
 SPD_EPI_SILU_MUL = 1
 SPD_EPI_GELU = 2
+SPD_EPI_OLDER_W = 256
 
 _p = C.c_void_p
 _i64 = C.c_int64

@@ -630,11 +630,11 @@ int gemm_pair_try(void* C, const void* A, const void* W, int64_t M, int64_t N, i
 
 int gemm_swap_tiles(int64_t M, int64_t N, int64_t K, int epilogue, int sms);
 int gemm_pair_swap(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldw, int64_t ldc,
-                   int dtype, int epilogue, int sms, int tok_tiles, int panel_mb, cudaStream_t stream);
+                   int dtype, int epilogue, int sms, int tok_tiles, int panel_mb, bool early, cudaStream_t stream);
 
 int gemm_split_tiles(int64_t M, int64_t N, int64_t K, int epilogue, int out_f32, int sms, int* split);
 int gemm_pair_split(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldw, int64_t ldc,
-                    int dtype, int out_f32, int epilogue, int tok_tiles, int split, cudaStream_t stream);
+                    int dtype, int out_f32, int epilogue, int tok_tiles, int split, bool early, cudaStream_t stream);
 
 int gemm_pair_decode_try(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_t K, int64_t lda,
                          int64_t ldw, int64_t ldc, int dtype, int out_f32, int sms, float* ws, int64_t ws_bytes,
@@ -709,6 +709,8 @@ int spd_gemm(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_
   SPD_REQUIRE(M >= 0 && N > 0 && K > 0, SPD_E_BADARG, "spd_gemm: bad sizes M=%lld N=%lld K=%lld",
               (long long)M, (long long)N, (long long)K);
   SPD_REQUIRE(dtype == SPD_BF16 || dtype == SPD_F16, SPD_E_BADARG, "spd_gemm: bad dtype %d", dtype);
+  const bool older_w = (epilogue & SPD_EPI_OLDER_W) != 0;
+  epilogue &= ~SPD_EPI_OLDER_W;
   SPD_REQUIRE(epilogue == SPD_EPI_NONE || epilogue == SPD_EPI_SILU_MUL || (epilogue == SPD_EPI_GELU && M > 256 && !out_f32),
               SPD_E_BADARG, "spd_gemm: bad epilogue %d (M %lld)", epilogue, (long long)M);
   SPD_REQUIRE(K % 8 == 0 && N % 8 == 0 && lda % 8 == 0 && ldw % 8 == 0 && ldc % (out_f32 ? 4 : 8) == 0,
@@ -766,13 +768,17 @@ int spd_gemm(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_
   // Decode regime, M <= 256: swap-AB.  The token dimension feeds UMMA-N (16, or M rounded up to a
   // multiple of 32), each 128-row weight tile is read once, and no MMA work is spent on padding
   // rows (the un-swapped form would pad 160 tokens to 2 x 128 and read W twice from L2).
+  // In all forms for up to 256 tokens the first weights are on their way before the grid waits for the kernel before it, which
+  // may have let it in early; with an epilogue, whose calls always could take that kernel's output for W, only where the
+  // caller says that W is older (a Llama-3-8B layer of one token 2 us).
+  const bool early = M <= 256 && (epilogue == SPD_EPI_NONE || older_w);
   // few weight tiles: clusters of pairs that cut K, or token tiles beside one another (gemm_split_tiles)
   int split = 0;
   if (const int tiles = gemm_split_tiles(M, N, K, epilogue, out_f32, sms, &split))
-    return split ? gemm_pair_split(C, A, W, M, N, K, lda, ldw, ldc, dtype, out_f32, epilogue, tiles, split, st)
-                 : gemm_pair_swap(C, A, W, M, N, K, lda, ldw, ldc, dtype, epilogue, sms, tiles, env_panel_mb, st);
+    return split ? gemm_pair_split(C, A, W, M, N, K, lda, ldw, ldc, dtype, out_f32, epilogue, tiles, split, early, st)
+                 : gemm_pair_swap(C, A, W, M, N, K, lda, ldw, ldc, dtype, epilogue, sms, tiles, env_panel_mb, early, st);
   if (epilogue == SPD_EPI_SILU_MUL && M <= 256 && !out_f32 && sms >= 2)
-    return gemm_pair_swap(C, A, W, M, N, K, lda, ldw, ldc, dtype, epilogue, sms, 1, env_panel_mb, st);
+    return gemm_pair_swap(C, A, W, M, N, K, lda, ldw, ldc, dtype, epilogue, sms, 1, env_panel_mb, early, st);
   const bool swap = (M <= env_swapmax) && epilogue == SPD_EPI_NONE;
   if (swap) {
     // 32 < M <= 256: CTA pairs share one activation tile between 256 weight rows (gemm_pair_decode.cu)
@@ -814,7 +820,7 @@ int spd_gemm(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_
 
   // prefill regime: token tiles of any width where those take fewer or shorter waves (gemm_pair_swap.cu)
   if (const int tiles = out_f32 ? 0 : gemm_swap_tiles(M, N, K, epilogue, sms))
-    return gemm_pair_swap(C, A, W, M, N, K, lda, ldw, ldc, dtype, epilogue, sms, tiles, env_panel_mb, st);
+    return gemm_pair_swap(C, A, W, M, N, K, lda, ldw, ldc, dtype, epilogue, sms, tiles, env_panel_mb, early, st);
   // else 256 x 256 tiles on CTA pairs (tcgen05.mma.cta_group::2, gemm_pair.cu)
   rc = gemm_pair_try(C, A, W, M, N, K, lda, ldw, ldc, dtype, out_f32, epilogue, sms, env_panel_mb, st);
   if (rc != 1) return rc;

@@ -37,6 +37,7 @@ struct PairSplitParams {
   int tok_tiles, n;    // token tiles, MMA columns of each
   int kblocks, stages, slot;
   int out_f32;
+  int early;  // the first weights are fetched before the grid waits for its predecessor
   unsigned* wait_expired;
 };
 
@@ -104,11 +105,12 @@ gemm_pair_split_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
                            kEvictFirst);
       };
       const int ahead = min(p.stages, kb1 - kb0);
+      if (!p.early) griddep_wait();
       for (int i = 0; i < ahead; ++i) {
         if (rank == 0) mbar_expect_tx(&full[i], bytes);
         load_w(i, kb0 + i);
       }
-      griddep_wait();
+      if (p.early) griddep_wait();
       int stage = 0, phase = 0;
       const int a_row = tt * p.n + static_cast<int>(rank) * half;
       for (int kb = kb0; kb < kb1; ++kb) {
@@ -251,7 +253,7 @@ static int launch_split(const CUtensorMap& tw, const CUtensorMap& ta, const Pair
 int get_gate_up_tmap(CUtensorMap* out, const void* W, uint64_t groups, uint64_t inter, uint64_t cols, uint64_t ldw);
 
 int gemm_pair_split(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldw, int64_t ldc,
-                    int dtype, int out_f32, int epilogue, int tok_tiles, int split, cudaStream_t stream) {
+                    int dtype, int out_f32, int epilogue, int tok_tiles, int split, bool early, cudaStream_t stream) {
   const bool silu = epilogue == SPD_EPI_SILU_MUL;
   PairSplitParams p{};
   p.C = C;
@@ -262,6 +264,7 @@ int gemm_pair_split(void* C, const void* A, const void* W, int64_t M, int64_t N,
   p.n = static_cast<int>(32 * (((M + 31) / 32 + tok_tiles - 1) / tok_tiles));
   p.kblocks = static_cast<int>((K + kPtBK - 1) / kPtBK);
   p.out_f32 = out_f32;
+  p.early = early;
   p.slot = kPtWBytes + p.n * kPtBK;
   const int fit = (kPtMaxSmem - kPtFixedSmem) / p.slot, most = (p.kblocks + split - 1) / split;
   const int sums = (p.n * 512 + p.slot - 1) / p.slot;  // slots that the partial sums need

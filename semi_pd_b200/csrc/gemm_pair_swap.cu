@@ -47,6 +47,7 @@ struct SwapGemmParams {
   int stages, slot;            // ring: slots and bytes of each (128 weight rows, half of the widest token tile)
   int list;                    // token tiles that the list has room for
   int decode;                  // one group: a batch that streams the weights once (see the launch)
+  int early;                   // one group: the first weights are fetched before the grid waits for its predecessor
   int panel;                   // one group: token tiles of a rasterisation panel
   const int2* group_rows;      // (first row, rows) of every group, null: one group
   int num_groups;
@@ -155,8 +156,8 @@ gemm_pair_swap_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
   const uint32_t tmem_base = *tmem_slot;
 
   if (p.decode) griddep_launch_dependents();
-  // (one group: the weights do not depend on the kernel before, so the copies of the first ones precede the wait)
-  if (p.group_rows || warp != 0) griddep_wait();
+  // (early: the weights are older than the kernel before, so the copies of the first ones precede the wait)
+  if (!p.early || warp != 0) griddep_wait();
   // the token tiles of all groups, one behind the other
   if (p.group_rows) {
     const int g = threadIdx.x;
@@ -211,7 +212,7 @@ gemm_pair_swap_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
           tma_load_2d_2cta(smem + slot * p.slot, &tmW, lead_full, static_cast<int>(group * p.w_group_cols) + kb * kPsBK,
                            static_cast<int>(group * p.w_group_rows) + wt * 256 + static_cast<int>(rank) * 128, policy);
       };
-      if (!p.group_rows) {
+      if (p.early) {
         int wt, tt;
         coords(pair, wt, tt);
         const uint32_t bytes = 2 * (kPsHalfBytes + (tiles[tt].y >> 1) * (kPsBK * 2));
@@ -450,7 +451,7 @@ int gemm_swap_tiles(int64_t M, int64_t N, int64_t K, int epilogue, int sms) {
 }
 
 int gemm_pair_swap(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldw, int64_t ldc,
-                   int dtype, int epilogue, int sms, int tok_tiles, int panel_mb, cudaStream_t stream) {
+                   int dtype, int epilogue, int sms, int tok_tiles, int panel_mb, bool early, cudaStream_t stream) {
   SwapGemmParams p{};
   const bool silu = epilogue == SPD_EPI_SILU_MUL;
   p.C = C;
@@ -468,6 +469,7 @@ int gemm_pair_swap(void* C, const void* A, const void* W, int64_t M, int64_t N, 
   p.list = tok_tiles;
   // as the other decode kernels (gemm_pair_decode.cu): the next kernel's weights come under this one's tail
   p.decode = M <= 256;
+  p.early = early;
   return run_swap(p, A, M, K, lda, W, 1, ldw, silu, silu ? 2 * N : N, K, 32 * ((p.units + tok_tiles - 1) / tok_tiles), dtype, pairs, stream);
 }
 

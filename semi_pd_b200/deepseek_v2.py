@@ -119,7 +119,7 @@ class DeepseekV2MLP:
 
     def forward(self, x):
         if ops.silu_fused(x, self.gate_up_proj.weight):
-            h = ops.linear(x, self.gate_up_proj.weight, epilogue=ops.SPD_EPI_SILU_MUL)
+            h = ops.linear(x, self.gate_up_proj.weight, epilogue=ops.SPD_EPI_SILU_MUL, older_weight=True)
         else:
             h = self.act_fn(ops.linear(x, self.gate_up_proj.weight))
         return ops.linear(h, self.down_proj.weight)

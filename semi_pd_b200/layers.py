@@ -170,7 +170,7 @@ class MergedColumnParallelLinear(ColumnParallelLinear):
         super().__init__(input_size, sum(self.output_sizes))
 
     def forward_silu_mul(self, x: torch.Tensor) -> torch.Tensor:
-        return ops.linear(x, self.weight, epilogue=ops.SPD_EPI_SILU_MUL)
+        return ops.linear(x, self.weight, epilogue=ops.SPD_EPI_SILU_MUL, older_weight=True)
 
     @staticmethod
     def shard(full: torch.Tensor, tp_rank, tp_size):

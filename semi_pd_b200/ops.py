@@ -16,7 +16,7 @@ from typing import Optional
 import torch
 
 from . import _lib
-from ._lib import SPD_EPI_GELU, SPD_EPI_NONE, SPD_EPI_SILU_MUL, check, lib
+from ._lib import SPD_EPI_GELU, SPD_EPI_NONE, SPD_EPI_OLDER_W, SPD_EPI_SILU_MUL, check, lib
 
 _DTYPE = {torch.bfloat16: _lib.SPD_BF16, torch.float16: _lib.SPD_F16}
 # the 32-bit capable operators (hybrid model family) additionally take float32
@@ -333,9 +333,12 @@ def _gemm_workspace(device: torch.device) -> torch.Tensor:
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = None,
-           out_f32: bool = False, epilogue: int = SPD_EPI_NONE, exact_f32: bool = False) -> torch.Tensor:
+           out_f32: bool = False, epilogue: int = SPD_EPI_NONE, exact_f32: bool = False,
+           older_weight: bool = False) -> torch.Tensor:
     """F.linear(x, weight) — x [M, K], weight [N, K] (or [2N, K] with SPD_EPI_SILU_MUL).  out_f32:
-    the 16-bit product as fp32 (`.float()` of a 16-bit matmul); with exact_f32 the fp32 accumulator."""
+    the 16-bit product as fp32 (`.float()` of a 16-bit matmul); with exact_f32 the fp32 accumulator.
+    older_weight: the weight is not what this library's kernels right before the call in its stream write (a layer's own weight
+    never is); up to 256 tokens without an epilogue that is taken for granted."""
     _cuda(x, weight)
     if x.dim() != 2 or weight.dim() != 2 or x.stride(1) != 1 or weight.stride(1) != 1:
         raise RuntimeError("linear: x and weight must be 2-D with contiguous last dimension")
@@ -349,8 +352,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = 
         out = torch.empty(M, N, device=x.device, dtype=torch.float32 if out_f32 else x.dtype)
     ws = _gemm_workspace(x.device)
     check(lib.spd_gemm(out.data_ptr(), x.data_ptr(), weight.data_ptr(), M, N, K, x.stride(0),
-                       weight.stride(0), out.stride(0), _dt(x), (2 if exact_f32 else 1) if out_f32 else 0, epilogue,
-                       ws.data_ptr(), ws.numel(), get_sm_budget(), _stream()), "spd_gemm")
+                       weight.stride(0), out.stride(0), _dt(x), (2 if exact_f32 else 1) if out_f32 else 0,
+                       epilogue | SPD_EPI_OLDER_W if older_weight else epilogue, ws.data_ptr(), ws.numel(), get_sm_budget(), _stream()), "spd_gemm")
     return out
 
 
