@@ -395,7 +395,7 @@ def linear_grouped_rows(x_sorted: torch.Tensor, weight: torch.Tensor, tile_group
     M, K = x_sorted.shape
     out = torch.empty(M, n, device=x_sorted.device, dtype=x_sorted.dtype)
     if (group_rows is not None and epilogue in (SPD_EPI_NONE, SPD_EPI_SILU_MUL) and num_groups <= 256
-            and M // 256 + num_groups <= 512):
+            and M // 256 + num_groups <= 512 and get_sm_budget() != 1):  # (pairs of CTAs want two SMs)
         check(lib.spd_gemm_grouped_rows(out.data_ptr(), x_sorted.data_ptr(), weight.data_ptr(), M, n, K, x_sorted.stride(0),
                                         weight.stride(0), out.stride(0), num_groups, group_rows.data_ptr(),
                                         K if k_concat else 0, _dt(x_sorted), epilogue, get_sm_budget(), _stream()),

@@ -90,3 +90,22 @@ def test_align_gives_the_rows():
             assert s % 128 == 0 and (row_token[s: s + c] >= 0).all()
             assert c % 128 == 0 or row_token[s + c] == -1
             assert c == 0 or tile_group[s // 128] == e
+
+
+@pytest.mark.parametrize("sms", [1, 2])
+def test_by_expert_on_few_sms(sms):
+    from semi_pd_b200 import ops
+    E, T, N, K = 5, 150, 136, 64
+    g = torch.Generator(device=DEV).manual_seed(2)
+    ids = torch.randint(0, E, (T, 2), generator=g, device=DEV).int()
+    x = torch.randn(T, K, generator=g, device=DEV).bfloat16()
+    w = (torch.randn(E, N, K, generator=g, device=DEV) * K ** -0.5).bfloat16()
+    row_token, inv_pos, tile_group, rows = ops.moe_align_groups(ids, E)
+    xs = ops.moe_gather(x, row_token)
+    ops.set_sm_budget(sms)
+    try:
+        y = ops.linear_grouped_rows(xs, w.view(E * N, K), tile_group, E, N, group_rows=rows)
+    finally:
+        ops.set_sm_budget(0)
+    got = y[inv_pos.long()].view(T, 2, N).double()
+    _check(got, torch.einsum("tjnk,tk->tjn", w[ids.long()].double(), x.double()), torch.bfloat16)
