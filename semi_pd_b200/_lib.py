@@ -264,7 +264,7 @@ def _load():
     # the per-layer calls without ctypes (csrc/pycalls.cpp): the same functions of the same library
     try:
         from . import _calls
-    except ImportError:  # not built, or for another interpreter: ctypes does all
+    except ImportError:  # not built, or built for another interpreter (its name is the file's): ctypes does all
         return lib
     functions = {name: (C.cast(getattr(lib, name), _p).value, getattr(lib, name)) for name in SIGNATURES}
     for name, fn in _calls.bind(functions).items():
