@@ -279,16 +279,32 @@ int gemm_pair_split(void* C, const void* A, const void* W, int64_t M, int64_t N,
   SPD_DISPATCH_DTYPE(dtype, { return launch_split<T, false>(tw, ta, p, w_tiles * tok_tiles, split, stream); });
 }
 
-// Clusters of 2 `split` CTAs that run at once on the whole device (B200: 74, 33, 22, 15).
-static int split_clusters(int split) {
-  static std::atomic<int> cached[kPtMaxSplit + 1];
-  int n = cached[split].load(std::memory_order_relaxed);
-  if (n > 0) return n;
+// Clusters of 2 `split` CTAs that the choice below reckons with on `sms` SMs when the driver says that `found` run at once
+// (-1: there is no device to ask).  0 is an answer: no cluster of this size fits.
+static int split_room(int split, int found, int sms) {
   static const int b200[kPtMaxSplit + 1] = {0, 74, 33, 22, 15};
+  if (found < 0) {
+    const int whole = device_sm_count_cached();
+    found = sms >= whole ? b200[split] : b200[split] * sms / whole;
+  }
+  const int most = sms / (2 * split);
+  return found < most ? found : most;
+}
+
+// What the driver says of a stream: a partition holds as many clusters as its SMs' places on the chip allow, which its number
+// of SMs does not tell (whole B200: 74, 33, 22, 15 clusters of 2, 4, 6, 8 CTAs; 76 SMs beside 72: 38, 15, 9, 6, the 72: 36, 18, 9, 9;
+// 108 beside 40: 54, 23, 13, 10).  Reckoned by number, 4096 x 14336 got 16 clusters of four on the 76 SMs, two waves: 23 us of
+// one token became 48.  A query takes 1 us of host time, so the whole device is asked once.
+static int split_clusters(int split, int sms, cudaStream_t stream) {
+  static std::atomic<int> cached[kPtMaxSplit + 1];  // the whole device's answer + 2
+  const bool whole = sms >= device_sm_count_cached();
+  int n = whole ? cached[split].load(std::memory_order_relaxed) - 2 : -2;
+  if (n > -2) return n;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(2 * split);
   cfg.blockDim = dim3(kPtThreads);
   cfg.dynamicSmemBytes = kPtMaxSmem;
+  cfg.stream = whole ? nullptr : stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2 * split;
@@ -298,15 +314,16 @@ static int split_clusters(int split) {
   cfg.numAttrs = 1;
   auto kern = gemm_pair_split_kernel<__nv_bfloat16, false>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPtMaxSmem) != cudaSuccess ||
-      cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) {
+      cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
     cudaGetLastError();
-    n = b200[split];  // no device to ask (the choice of kernel can be asked for without one)
+    n = -1;  // no device to ask (the choice of kernel can be asked for without one)
   }
-  cached[split].store(n, std::memory_order_relaxed);
+  if (whole) cached[split].store(n + 2, std::memory_order_relaxed);
   return n;
 }
 
 int gemm_cluster_ctas(int64_t N, int64_t K, int sms);
+int split_room_of(int split, int found, int sms) { return split >= 1 && split <= kPtMaxSplit ? split_room(split, found, sms) : 0; }
 
 // The tiles of a GEMM on few weight tiles, 0: the other kernels.  *split = pairs per tile in a cluster (this kernel), 0: tiles
 // of gemm_pair_swap.cu that one wave holds.
@@ -322,7 +339,7 @@ int gemm_cluster_ctas(int64_t N, int64_t K, int sms);
 // 151.4 here; 4096 x 14336 by itself 21.6 / 21.9).  Beyond 256 tokens the tiles of
 // gemm_pair_swap.cu / gemm_pair.cu serve unless this kernel is estimated a tenth faster, three tenths beyond 512 tokens
 // (4096 x 14336, 448 tokens 51 / 44; 64 x 2048, 1024 9.1 / 7.3; 4096 x 4096, 640 18.5 / 20 and not taken).
-int gemm_split_tiles(int64_t M, int64_t N, int64_t K, int epilogue, int out_f32, int sms, int* split) {
+int gemm_split_tiles(int64_t M, int64_t N, int64_t K, int epilogue, int out_f32, int sms, cudaStream_t on, int* split) {
   *split = 0;
   // Rows beyond 16384 and unrounded fp32 results keep the finer cuts of the other kernels: an accumulator's error grows with
   // the products it adds up.
@@ -334,7 +351,11 @@ int gemm_split_tiles(int64_t M, int64_t N, int64_t K, int epilogue, int out_f32,
   const double bytes = 2.0 * K * (silu ? 2 * N : N), kb = static_cast<double>((K + kPtBK - 1) / kPtBK);
   static const double more[kPtMaxSplit + 1] = {0, 0, 0.36, 0.3, 0.4};
   const int units = static_cast<int>((M + 31) / 32);
-  const int whole = device_sm_count_cached();
+  int room[kPtMaxSplit + 1];
+  for (int s = 1; s <= kPtMaxSplit; ++s) {
+    const bool may = w_tiles * 2 * s <= sms && 8 * (s - 1) <= kb;
+    room[s] = !may ? 0 : split_room(s, s == 1 ? pairs : split_clusters(s, sms, on), sms);
+  }
   double best = 0, swap = 0;
   int tiles = 0, swap_tiles = 0;
   for (int t = (units + 7) / 8; t <= units && t * w_tiles <= pairs; ++t) {
@@ -347,8 +368,7 @@ int gemm_split_tiles(int64_t M, int64_t N, int64_t K, int epilogue, int out_f32,
       swap_tiles = t;
     }
     for (int s = 1; s <= kPtMaxSplit; ++s) {
-      const int64_t room = sms >= whole ? split_clusters(s) : static_cast<int64_t>(split_clusters(s)) * sms / whole;
-      if (t * w_tiles > room || 8 * (s - 1) > kb) continue;
+      if (t * w_tiles > room[s]) continue;
       us = 2.5 + (kb / s) * (0.176 + 0.1 * n / 256) + more[s];
       us = (us > stream ? us > fetch ? us : fetch : stream > fetch ? stream : fetch) + 4.6 * n / 256;
       if (tiles == 0 || us < best) {

@@ -64,3 +64,30 @@ def test_a_row_does_not_hang_on_the_others():
         z = ops.linear(x, w)
         keep = [i for i in range(50) if i not in (7, 49)]
         assert torch.equal(y[keep], z[keep]) and torch.isnan(z[7]).all() and not torch.isfinite(z[49]).any()
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 4096, 14336), (64, 4096, 4096), (256, 1280, 4096), (448, 4096, 2048)])
+def test_on_a_partition(M, N, K):
+    """Clusters are those that fit the stream's SMs, launched and captured."""
+    from semi_pd_b200 import ops
+    part = ops.get_partition(0, 76, 72)
+    g = torch.Generator(device=DEV).manual_seed(M)
+    x = torch.randn(M, K, generator=g, device=DEV).bfloat16()
+    w = (torch.randn(N, K, generator=g, device=DEV) * K ** -0.5).bfloat16()
+    y = x.double() @ w.double().t()
+    torch.cuda.synchronize()
+    for stream, sms in ((part.prefill_stream, part.prefill_sms), (part.decode_stream, part.decode_sms)):
+        ops.set_sm_budget(sms)
+        try:
+            with torch.cuda.stream(stream):
+                got = ops.linear(x, w)
+                stream.synchronize()
+                graph, again = torch.cuda.CUDAGraph(), torch.empty_like(got)
+                with torch.cuda.graph(graph, stream=stream):
+                    ops.linear(x, w, out=again)
+                graph.replay()
+                stream.synchronize()
+        finally:
+            ops.set_sm_budget(0)
+        assert ((got.double() - y).norm() / y.norm()).item() < 2.0 ** -9  # one rounding to 16 bits
+        assert torch.equal(got, again)

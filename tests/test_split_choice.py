@@ -46,3 +46,15 @@ def test_silu_in_the_gemm():
     assert lib.spd_gemm_silu_fused(64, 14336, 4096, 72) == 0  # 112 tiles on 36 pairs: four waves, the last nearly empty
     assert lib.spd_gemm_silu_fused(64, 14336, 4096, 76) == 1 and lib.spd_gemm_silu_fused(64, 2816, 2048, 148) == 1
     assert lib.spd_gemm_silu_fused(64, 2816, 2048, 1) == 0 and lib.spd_gemm_silu_fused(0, 8, 8, 148) < 0
+
+
+def test_room():
+    whole = [lib.spd_gemm_split_room(s, -1, 148) for s in (1, 2, 3, 4)]
+    assert whole == [74, 33, 22, 15]
+    assert [lib.spd_gemm_split_room(s, f, 76) for s, f in ((2, 15), (3, 9), (4, 6))] == [15, 9, 6]  # as the driver says
+    assert lib.spd_gemm_split_room(4, 0, 76) == 0 and lib.spd_gemm_split_room(2, 0, 148) == 0       # none fits: none
+    assert lib.spd_gemm_split_room(2, 33, 40) == 10                                                 # a budget of fewer SMs
+    assert lib.spd_gemm_split_room(0, 5, 148) == 0 and lib.spd_gemm_split_room(5, 5, 148) == 0
+    for sms in range(2, 148, 6):
+        for s in (1, 2, 3, 4):
+            assert 0 <= lib.spd_gemm_split_room(s, -1, sms) <= min(sms // (2 * s), whole[s - 1])
