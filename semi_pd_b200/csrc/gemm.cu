@@ -632,7 +632,8 @@ int gemm_swap_tiles(int64_t M, int64_t N, int64_t K, int epilogue, int sms);
 int gemm_pair_swap(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldw, int64_t ldc,
                    int dtype, int epilogue, int sms, int tok_tiles, int panel_mb, bool early, cudaStream_t stream);
 
-int gemm_split_tiles(int64_t M, int64_t N, int64_t K, int epilogue, int out_f32, int sms, cudaStream_t on, int* split);
+int gemm_split_tiles(int64_t M, int64_t N, int64_t K, int epilogue, int out_f32, int sms, bool scratch, cudaStream_t on,
+                     int* split);
 int split_room_of(int split, int found, int sms);
 int gemm_pair_split(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldw, int64_t ldc,
                     int dtype, int out_f32, int epilogue, int tok_tiles, int split, bool early, cudaStream_t stream);
@@ -692,7 +693,7 @@ int spd_gemm_silu_fused(int64_t M, int64_t N, int64_t K, int sm_budget) {
 
 int spd_gemm_split_tiles(int64_t M, int64_t N, int64_t K, int epilogue, int out_f32, int sm_budget, int* split) {
   SPD_REQUIRE(split && M > 0 && N > 0 && K > 0, SPD_E_BADARG, "spd_gemm_split_tiles: bad arguments");
-  return gemm_split_tiles(M, N, K, epilogue, out_f32, sm_budget > 0 ? sm_budget : device_sm_count_cached(), nullptr, split);
+  return gemm_split_tiles(M, N, K, epilogue, out_f32, sm_budget > 0 ? sm_budget : device_sm_count_cached(), true, nullptr, split);
 }
 
 int spd_gemm_split_room(int split, int found, int sm_budget) {
@@ -779,7 +780,7 @@ int spd_gemm(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_
   const bool early = M <= 256 && (epilogue == SPD_EPI_NONE || older_w);
   // few weight tiles: clusters of pairs that cut K, or token tiles beside one another (gemm_split_tiles)
   int split = 0;
-  if (const int tiles = gemm_split_tiles(M, N, K, epilogue, out_f32, sms, st, &split))
+  if (const int tiles = gemm_split_tiles(M, N, K, epilogue, out_f32, sms, ws_ok, st, &split))
     return split ? gemm_pair_split(C, A, W, M, N, K, lda, ldw, ldc, dtype, out_f32, epilogue, tiles, split, early, st)
                  : gemm_pair_swap(C, A, W, M, N, K, lda, ldw, ldc, dtype, epilogue, sms, tiles, env_panel_mb, early, st);
   if (epilogue == SPD_EPI_SILU_MUL && M <= 256 && !out_f32 && sms >= 2)

@@ -326,7 +326,7 @@ int gemm_cluster_ctas(int64_t N, int64_t K, int sms);
 int split_room_of(int split, int found, int sms) { return split >= 1 && split <= kPtMaxSplit ? split_room(split, found, sms) : 0; }
 
 // The tiles of a GEMM on few weight tiles, 0: the other kernels.  *split = pairs per tile in a cluster (this kernel), 0: tiles
-// of gemm_pair_swap.cu that one wave holds.
+// of gemm_pair_swap.cu that one wave holds.  scratch: the call has the workspace that stream-K wants.
 //
 // Every form's time is estimated in us from what was measured with weights out of L2 (1 - 1024 tokens, weights of 64 x 2048 to
 // 14336 x 1024 and 4096 x 14336; the form chosen took 1.02 times the fastest one's time in the mean): a k-block of a pair 0.175
@@ -338,8 +338,9 @@ int split_room_of(int split, int found, int sms) { return split >= 1 && split <=
 // kernel of a decode step each CTA's ring fills early (a Llama-3-8B layer of one token 151.1 us with 4096 x 4096 there,
 // 151.4 here; 4096 x 14336 by itself 21.6 / 21.9).  Beyond 256 tokens the tiles of
 // gemm_pair_swap.cu / gemm_pair.cu serve unless this kernel is estimated a tenth faster, three tenths beyond 512 tokens
-// (4096 x 14336, 448 tokens 51 / 44; 64 x 2048, 1024 9.1 / 7.3; 4096 x 4096, 640 18.5 / 20 and not taken).
-int gemm_split_tiles(int64_t M, int64_t N, int64_t K, int epilogue, int out_f32, int sms, cudaStream_t on, int* split) {
+// (4096 x 14336, 448 tokens 51 / 44; 64 x 2048, 1024 9.1 / 7.3; 4096 x 4096, 640 18.5 / 20 and not taken), and unless K is not cut
+// (4096 x 14336, 512 tokens on 108 SMs 57 / 77).
+int gemm_split_tiles(int64_t M, int64_t N, int64_t K, int epilogue, int out_f32, int sms, bool scratch, cudaStream_t on, int* split) {
   *split = 0;
   // Rows beyond 16384 and unrounded fp32 results keep the finer cuts of the other kernels: an accumulator's error grows with
   // the products it adds up.
@@ -379,7 +380,7 @@ int gemm_split_tiles(int64_t M, int64_t N, int64_t K, int epilogue, int out_f32,
     }
   }
   if (M > 256) {
-    if (tiles == 0 || swap_tiles == 0 || best > swap * (M <= 512 ? 0.9 : 0.7)) {
+    if (tiles == 0 || swap_tiles == 0 || *split < 2 || best > swap * (M <= 512 ? 0.9 : 0.7)) {
       *split = 0;
       return 0;
     }
@@ -392,6 +393,23 @@ int gemm_split_tiles(int64_t M, int64_t N, int64_t K, int epilogue, int out_f32,
   if (M <= 16 && bytes > 2.5e7 && !silu) {
     const int ctas = static_cast<int>(w_tiles) * tiles * 2 * (*split > 0 ? *split : 1);
     if (gemm_cluster_ctas(N, K, sms) > ctas) {
+      *split = 0;
+      return 0;
+    }
+  }
+  // A partition that has little more SMs than these tiles have CTAs is better used by the kernels that deal k-blocks evenly over
+  // all of them: the cluster of single CTAs and stream-K by single CTAs, or by pairs beyond 32 tokens.  Their time on 40 - 108 SMs,
+  // from the same measurements: weights at 113 MB/ms an SM, at most 7.2 GB/ms, a k-block of a pair 0.15 and 0.1 more for 256
+  // tokens, fix-up.  Stream-K / these, us: 4096 x 14336 on 40 SMs, one token 32.7 / 43, 64 35.5 / 43.7, on 76 SMs 64 26.1 / 43.5, on 72
+  // 1 23.1 / 25.3, 256 46.1 / 42.0; 6144 x 4096 on 72 SMs, one token 13.9 / 15.9; 4096 x 4096 on 40, one token 14.1 / 15.6, 64 16.7 /
+  // 15.9.  Of 859 calls on partitions 13 took up to 9 % more than before this kernel then, the form chosen 0.2 % more than the
+  // faster one in the mean.
+  if (sms < device_sm_count_cached() && scratch && !silu) {
+    const double rate = 113e3 * sms < 7.2e6 ? 113e3 * sms : 7.2e6, even = kb * w_tiles / pairs * (0.15 + 0.1 * (M > 64 ? 32 * units - 64 : 0) / 192);
+    double old = bytes / rate;
+    if (M <= 32) old += M <= 16 ? 6 : 6.6;
+    else old = 7 + 10.0 * 32 * units / 256 + (old > even ? old : even);
+    if ((*split > 0 ? best : swap) > old) {
       *split = 0;
       return 0;
     }

@@ -58,3 +58,11 @@ def test_room():
     for sms in range(2, 148, 6):
         for s in (1, 2, 3, 4):
             assert 0 <= lib.spd_gemm_split_room(s, -1, sms) <= min(sms // (2 * s), whole[s - 1])
+
+
+@pytest.mark.parametrize("M,N,K,sms,taken", [
+    (1, 4096, 14336, 40, False), (64, 4096, 14336, 40, False), (1, 4096, 14336, 72, False), (256, 4096, 14336, 72, True),
+    (1, 6144, 4096, 72, False), (1, 4096, 4096, 40, False), (64, 4096, 4096, 40, True), (64, 2048, 2048, 72, True),
+    (64, 64, 2048, 40, True), (512, 4096, 14336, 108, False), (448, 4096, 14336, 148, True)])
+def test_partitions_that_stream_k_uses_better(M, N, K, sms, taken):
+    assert (_form(M, N, K, sms=sms)[0] > 0) is taken
