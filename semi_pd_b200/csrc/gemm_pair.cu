@@ -305,7 +305,12 @@ int gemm_pair_cols(int64_t M, int64_t N, int64_t K, int epilogue, int sms, int64
     const int64_t cols = (N + n_tile - 1) / n_tile, kblocks = (K + kPgBK - 1) / kPgBK;
     const int64_t waves_single = (rows_single / 128 * cols + sms - 1) / sms;
     if (cost * 9 >= waves_single * (kPgBN + 100) * 10 || waves_single * kblocks < 48) {
-      if (cost_out) *cost_out = waves_single * (kPgBN + 100) * 10 / 9;
+      if (cost_out) {
+        // (few tiles of 256 columns that N does not fill are cut to 128, which the 0.9 does not hold for: see gemm_swap_tiles)
+        const bool narrow = epilogue != SPD_EPI_SILU_MUL && N % kPgBN != 0 && rows_single / 128 * cols < sms;
+        const int64_t waves128 = (rows_single / 128 * ((N + 127) / 128) + sms - 1) / sms;
+        *cost_out = narrow ? waves128 * (128 + 100) : waves_single * (kPgBN + 100) * 10 / 9;
+      }
       return 0;
     }
   }

@@ -426,7 +426,9 @@ int gemm_pair_cols(int64_t M, int64_t N, int64_t K, int epilogue, int sms, int64
 // columns a tile does not get shorter.  Where both count the same (M = 1600: seven tiles of 256 rows, or of 229) the
 // rows saved still pay from three waves on, in power.  On both sides of the line, other tiles / these, us: 1300 tokens,
 // K = 4096, N = 14336 with SiLU 297 / 236, 6144 59 / 53; 800: 201 / 153, 41 / 37; 512: 113 / 111, 22.8 / 23.1; K = 14336,
-// N = 4096: 384 66 / 54, 700 76 / 77, 1100 111 / 121 (single CTAs), 1300 146 / 126, 2500 231 / 268 (not taken).
+// N = 4096: 384 66 / 54, 700 76 / 77, 1100 111 / 121 (single CTAs), 1300 146 / 126, 2500 231 / 268 (not taken).  Single CTAs
+// whose tiles are cut to 128 columns take a wave of those in 228 units: 64 x 2048, 1300 tokens 8.2 / 9.8, 640 on 72 SMs 8.3 / 10.2;
+// 3648 x 2048, 640 11.2 / 12.7, 384 on 108 SMs 10.9 / 11.8; 264 x 1024, 513 6.2 / 7.7; 1000 x 192, 800 4.3 / 5.5 (not taken).
 int gemm_swap_tiles(int64_t M, int64_t N, int64_t K, int epilogue, int sms) {
   if (M <= 256 || sms < 2 || (epilogue != SPD_EPI_NONE && epilogue != SPD_EPI_SILU_MUL) || M >= (1ll << 31) || N >= (1ll << 30))
     return 0;
@@ -437,7 +439,7 @@ int gemm_swap_tiles(int64_t M, int64_t N, int64_t K, int epilogue, int sms) {
   const int64_t pairs = sms / 2;
   int64_t best = 0, cost = 0, waves = 0;
   for (int64_t t = (units + 7) / 8; t <= (units + 3) / 4 && t <= kPsMaxTiles; ++t) {
-    const int64_t w = (t * w_tiles + pairs - 1) / pairs, c = w * (32 * ((units + t - 1) / t) + 100);
+    const int64_t n = 32 * ((units + t - 1) / t), w = (t * w_tiles + pairs - 1) / pairs, c = w * ((n < 128 ? 128 : n) + 100);
     if (best == 0 || c < cost) {
       best = t;
       cost = c;

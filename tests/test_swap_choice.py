@@ -18,3 +18,9 @@ def test_swap_rows(M, N, K, epilogue, sms, rows):
 
 def test_swap_rows_refuses_bad_sizes():
     assert lib.spd_gemm_swap_rows(0, 128, 64, SPD_EPI_NONE, 148) < 0
+
+
+@pytest.mark.parametrize("M,N,K,sms", [(1300, 64, 2048, 148), (640, 64, 2048, 72), (640, 3648, 2048, 148), (384, 3648, 2048, 108),
+                                       (513, 264, 1024, 148), (800, 1000, 192, 148), (257, 6144, 4096, 72)])
+def test_few_tiles_of_128_columns_are_faster(M, N, K, sms):
+    assert lib.spd_gemm_swap_rows(M, N, K, SPD_EPI_NONE, sms) == 0
