@@ -18,6 +18,7 @@ What differs from the reference, all on the kernel side:
 """
 from __future__ import annotations
 
+import functools
 import math
 from typing import Dict, Iterable, Optional, Tuple
 
@@ -29,10 +30,34 @@ from .distributed import get_tensor_model_parallel_world_size
 from .forward_batch_info import ForwardBatch, LogitsProcessorOutput
 from .layers import LinearBase, LogitsProcessor, ParallelLMHead, RMSNorm, SiluAndMul, VocabParallelEmbedding
 
-# Batches in [lo, hi] run all experts densely (see module docstring).  Dense / grouped, us a layer: 16 tokens 206 / 202, 24
-# 216 / 214, 32 219 / 223, 64 224 / 226, 96 232 / 233, 128 242 / 236, 256 317 / 250.
-_MOE_DENSE_MIN_TOKENS = 28
-_MOE_DENSE_MAX_TOKENS = 112
+# The dense form serves batches of these sizes where it is the faster one (moe_dense_pays)
+_MOE_DENSE_MIN_TOKENS = 16
+_MOE_DENSE_MAX_TOKENS = 256
+
+
+@functools.lru_cache(maxsize=1)
+def _device_sms() -> int:
+    return ops.device_sm_count(0)
+
+
+@functools.lru_cache(maxsize=4096)
+def moe_dense_pays(tokens: int, hidden: int, inter: int, num_experts: int, top_k: int, sms: int) -> bool:
+    """Whether a batch is faster through all experts (two plain GEMMs that read every weight once, whatever was chosen) than by
+    expert (which reads the chosen ones, about all of them from 3 num_experts / top_k tokens on, in shorter tiles).  Estimates
+    in us: dense, the weights at 6.76 GB/ms from HBM and, with the tokens, at 8.8 GB/ms into the SMs (0.125 an SM, on a
+    partition), the activations between the GEMMs; by expert, 128 + 6000 / SMs a GB, 14000 / SMs where few SMs bound it.  Over
+    nine layers (8 to 160 experts, 1 to 8 chosen, 0.1 to 7.6 GB) of 16 to 256 tokens on 148, 108, 76, 72 and 40 SMs the form
+    chosen took 0.3 % more than the faster one in the mean.  Dense / by expert: 64 experts, 6 chosen, 2048 x 1408: 16 tokens
+    191 / 182, 24 188 / 199, 112 212 / 211, 160 227 / 214, on 72 SMs 24 198 / 245, 192 286 / 271; 8 experts, 2 chosen,
+    4096 x 7168: 16 230 / 269, 192 289 / 275; 160 experts, 6 chosen, 5120 x 1536: 32 1162 / 923, 96 1206 / 1241."""
+    if not _MOE_DENSE_MIN_TOKENS <= tokens <= _MOE_DENSE_MAX_TOKENS:
+        return False
+    gb = 6e-9 * hidden * inter * num_experts
+    used = 1.0 - (1.0 - top_k / num_experts) ** tokens
+    fetch = max(148.0, (1.0 + tokens / 256) * 1000.0 / min(8.8, 0.125 * sms))
+    dense = 30.0 + gb * fetch + 1.2e-6 * tokens * num_experts * inter + 0.03 * tokens
+    by_expert = 30.0 + gb * used * max(128.0 + 6000.0 / sms, 14000.0 / sms)
+    return dense <= by_expert
 
 
 # The expanded form of MLA prefill keeps K and V of every key while a layer runs: 8 KB per key at 16 heads.
@@ -162,7 +187,7 @@ class DeepseekV2MoE:
         shared = self.shared_experts(x) if self.shared_experts is not None else None
         logits = self.gate(x)
         ids, w = ops.moe_route(logits, self.top_k, scale=self.routed_scaling_factor, renormalize=self.renormalize)
-        if _MOE_DENSE_MIN_TOKENS <= T <= _MOE_DENSE_MAX_TOKENS:
+        if moe_dense_pays(T, x.shape[1], inter, E, self.top_k, ops.get_sm_budget() or _device_sms()):
             gu = ops.linear(x, self.w_gate_up)                        # [T, E * 2I]
             act = ops.moe_dense_act(gu, ids, w, E, inter)             # [T, E * I], routing weight folded in
             y = ops.linear(act, self.w_down_cat)                      # [T, hidden]
