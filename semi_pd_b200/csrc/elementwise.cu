@@ -333,17 +333,15 @@ gather_rows_kernel(T* __restrict__ out, const T* __restrict__ table, const int64
 
 // argmax over fp32 rows; ties resolve to the smallest index (torch.argmax on CUDA/CPU returns the
 // first maximal element for distinct-valued logits; exact ties are measure-zero on this path).
-// A row is cut over the CTAs of a cluster, each thread with four pieces on their way: one CTA of 1024 threads took 13.3 us for a
-// row of 128256 (latency: 31 rounds), eight of 512 take 5.
-constexpr int kArgmaxThreads = 512;
 __device__ __forceinline__ void argmax_take(float a, int id, float& best, int& bi) {
   if (a > best || (a == best && id < bi)) {
     best = a;
     bi = id;
   }
 }
-template <int kCtas>
-__global__ void __launch_bounds__(kArgmaxThreads)
+// kAhead: pieces that a thread has on their way at once
+template <int kCtas, int kThreads, int kAhead>
+__global__ void __launch_bounds__(kThreads)
 argmax_kernel(int32_t* __restrict__ ids, const float* __restrict__ logits, int64_t vocab, int64_t ld,
               int4* __restrict__ pairs, int idx_offset) {
   __shared__ float sv[32];
@@ -360,15 +358,15 @@ argmax_kernel(int32_t* __restrict__ ids, const float* __restrict__ logits, int64
   float best = -INFINITY;
   int bi = 0x7fffffff;
   const int64_t nv4 = ((reinterpret_cast<uintptr_t>(row) & 15u) == 0) ? (vocab >> 2) : 0;
-  constexpr int kStep = kCtas * kArgmaxThreads;
-  for (int64_t i0 = part * kArgmaxThreads + threadIdx.x; i0 < nv4; i0 += 4 * kStep) {
-    float4 f[4];
+  constexpr int kStep = kCtas * kThreads;
+  for (int64_t i0 = part * kThreads + threadIdx.x; i0 < nv4; i0 += kAhead * kStep) {
+    float4 f[kAhead];
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
+    for (int u = 0; u < kAhead; ++u)
       f[u] = i0 + u * kStep < nv4 ? reinterpret_cast<const float4*>(row)[i0 + u * kStep]
                                   : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
+    for (int u = 0; u < kAhead; ++u) {
       if (i0 + u * kStep >= nv4) break;  // (an index past the row would win over no value at all)
       const int id = static_cast<int>((i0 + u * kStep) * 4);
       argmax_take(f[u].x, id, best, bi);
@@ -377,7 +375,7 @@ argmax_kernel(int32_t* __restrict__ ids, const float* __restrict__ logits, int64
       argmax_take(f[u].w, id + 3, best, bi);
     }
   }
-  for (int64_t i = nv4 * 4 + part * kArgmaxThreads + threadIdx.x; i < vocab; i += kStep)
+  for (int64_t i = nv4 * 4 + part * kThreads + threadIdx.x; i < vocab; i += kStep)
     argmax_take(row[i], static_cast<int>(i), best, bi);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -387,7 +385,7 @@ argmax_kernel(int32_t* __restrict__ ids, const float* __restrict__ logits, int64
   }
   if (lane_id() == 0) { sv[threadIdx.x >> 5] = best; si[threadIdx.x >> 5] = bi; }
   __syncthreads();
-  constexpr int kWarps = kArgmaxThreads / 32;
+  constexpr int kWarps = kThreads / 32;
   if constexpr (kCtas > 1) cluster_sync_all();  // every CTA's warps have left their best
   if (threadIdx.x < 32 && part == 0) {
     best = -INFINITY;
@@ -417,15 +415,29 @@ argmax_kernel(int32_t* __restrict__ ids, const float* __restrict__ logits, int64
   if constexpr (kCtas > 1) cluster_sync_all();  // nobody leaves before the first CTA has read it
 }
 
-// Eight CTAs a row as long as the rows leave SMs idle (two of 512 threads an SM).
+// One CTA a row: 512 threads with four pieces each on their way up to 8192 values, 1024 up to 16384, and 1024 that the compiler's
+// order serves better beyond (31 rounds for 128256 values, bound by latency).  A few long rows go to eight CTAs each, a cluster,
+// where that is the faster on 148 SMs and on partitions down to 40, whose SMs more rows soon fill by themselves.  Rows that a GEMM
+// has just left in L2, one CTA / cluster, us on 148, 72 and 40 SMs: 32000 values, 1 row 3.0 / 3.4, 3.0 / 3.3, 3.0 / 3.3 (not taken);
+// 50272, 4 rows 3.8 / 3.6, 3.9 / 3.7, 3.8 / 3.6, 16 rows 4.0 / 4.4 (not taken); 102400, 4 rows 5.5 / 4.2, 8 5.6 / 4.2, 5.6 / 4.8,
+// 5.5 / 5.7 (not taken); 128256, 8 rows 6.6 / 4.4, 6.6 / 5.2, 6.6 / 6.3, 24 6.7 / 6.2, 6.7 / 6.8 (not taken); 256000, 32 rows 11.1 /
+// 8.8, 15.0 / 9.3, 18.4 / 14.1.  (512 threads with four pieces ahead for every row took 23.8 us for 128 rows of 128256, 1024 15.2.)
+template <int kThreads, int kAhead>
+static cudaError_t launch_argmax_rows(int32_t* ids, const float* logits, int64_t batch, int64_t vocab, int64_t ld, int4* pairs,
+                                      int offset, cudaStream_t stream) {
+  return launch(argmax_kernel<1, kThreads, kAhead>, dim3((unsigned)batch), dim3(kThreads), 0, stream, pdl_enabled(), ids, logits,
+                vocab, ld, pairs, offset);
+}
 static cudaError_t launch_argmax(int32_t* ids, const float* logits, int64_t batch, int64_t vocab, int64_t ld, int4* pairs,
                                  int offset, cudaStream_t stream) {
-  if (vocab < 16384 || batch > device_sm_count_cached() / 4)
-    return launch(argmax_kernel<1>, dim3((unsigned)batch), dim3(kArgmaxThreads), 0, stream, pdl_enabled(), ids, logits, vocab, ld,
-                  pairs, offset);
+  const int64_t most = vocab >= 196608 ? 32 : vocab >= 128000 ? 12 : vocab >= 98304 ? 6 : vocab >= 49152 ? 4 : 0;
+  if (batch > most) {
+    auto rows = vocab >= 16384 ? launch_argmax_rows<1024, 1> : vocab > 8192 ? launch_argmax_rows<1024, 4> : launch_argmax_rows<512, 4>;
+    return rows(ids, logits, batch, vocab, ld, pairs, offset, stream);
+  }
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)batch * 8);
-  cfg.blockDim = dim3(kArgmaxThreads);
+  cfg.blockDim = dim3(512);
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -436,7 +448,7 @@ static cudaError_t launch_argmax(int32_t* ids, const float* logits, int64_t batc
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, argmax_kernel<8>, ids, logits, vocab, ld, pairs, offset);
+  return cudaLaunchKernelEx(&cfg, argmax_kernel<8, 512, 4>, ids, logits, vocab, ld, pairs, offset);
 }
 
 // ids[b] = index of the largest of `parts` (max, index) candidates per row; ties resolve to the

@@ -25,3 +25,14 @@ def test_rows(B, V, pad):
     first = (want == best[:, None]).int().argmax(-1)
     assert torch.equal(ops.argmax(x).long(), first)
     assert torch.equal(ops.argmax_merge(ops.argmax_partial(x, 0)[None]).long().view(-1), first)
+
+
+@pytest.mark.parametrize("V", [5, 8192, 8193, 16380, 16384, 49151, 49152, 98303, 98304, 128000, 196608])  # around the lines between the forms
+@pytest.mark.parametrize("B", [1, 4, 5, 6, 7, 12, 13, 32, 33])
+def test_forms(B, V):
+    from semi_pd_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(B + V)
+    x = torch.randint(-50, 50, (B, V), generator=g, device=DEV).float()  # ties everywhere
+    x[0] = float("-inf")
+    best = x.max(-1)[0]
+    assert torch.equal(ops.argmax(x).long(), (x == best[:, None]).int().argmax(-1))
