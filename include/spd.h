@@ -97,6 +97,16 @@ int spd_rope_kvwrite(void* q, void* k, const void* v, void* k_pool, void* v_pool
                      int64_t tokens, int num_q_heads, int num_k_heads, int head_dim, int rot_dim,
                      int64_t q_stride, int64_t k_stride, int64_t v_stride, int interleave,
                      int dtype, spd_stream_t stream);
+/* Both for a caller that has sm_budget SMs (0: all), which decide how many threads a token gets. */
+int spd_rope_inplace_sms(void* q, void* k, const float* cos_sin_cache, const int64_t* pos_ids,
+                         int64_t tokens, int num_q_heads, int num_k_heads, int head_dim, int rot_dim,
+                         int64_t q_stride, int64_t k_stride, int interleave, int dtype, int sm_budget,
+                         spd_stream_t stream);
+int spd_rope_kvwrite_sms(void* q, void* k, const void* v, void* k_pool, void* v_pool,
+                         const float* cos_sin_cache, const int64_t* pos_ids, const int64_t* loc,
+                         int64_t tokens, int num_q_heads, int num_k_heads, int head_dim, int rot_dim,
+                         int64_t q_stride, int64_t k_stride, int64_t v_stride, int interleave,
+                         int dtype, int sm_budget, spd_stream_t stream);
 /* k_pool[loc[t]] = k[t]; v_pool[loc[t]] = v[t] — set_kv_buffer alone (S/mem_cache/memory_pool.py:316-346).
  * v and v_pool may both be NULL: single-buffer pools (MLATokenToKVPool.set_kv_buffer, :426-452). */
 int spd_kv_write(const void* k, const void* v, void* k_pool, void* v_pool, const int64_t* loc,

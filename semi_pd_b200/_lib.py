@@ -51,6 +51,11 @@ SIGNATURES = {
         _i,
         [_p, _p, _p, _p, _p, _p, _p, _p, _i64, _i, _i, _i, _i, _i64, _i64, _i64, _i, _i, _p],
     ),
+    "spd_rope_inplace_sms": (_i, [_p, _p, _p, _p, _i64, _i, _i, _i, _i, _i64, _i64, _i, _i, _i, _p]),
+    "spd_rope_kvwrite_sms": (
+        _i,
+        [_p, _p, _p, _p, _p, _p, _p, _p, _i64, _i, _i, _i, _i, _i64, _i64, _i64, _i, _i, _i, _p],
+    ),
     "spd_kv_write": (_i, [_p, _p, _p, _p, _p, _i64, _i64, _i64, _i64, _i, _p]),
     "spd_gather_rows": (_i, [_p, _p, _p, _i64, _i64, _i64, _i, _p]),
     "spd_argmax_f32": (_i, [_p, _p, _i64, _i64, _i64, _p]),

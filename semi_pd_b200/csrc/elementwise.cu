@@ -723,7 +723,7 @@ int spd_silu_and_mul(void* out, const void* x, int64_t tokens, int64_t d, int dt
 static int rope_common(void* q, void* k, const void* v, void* k_pool, void* v_pool,
                        const float* cos_sin_cache, const int64_t* pos_ids, const int64_t* loc,
                        int64_t tokens, int Hq, int Hk, int D, int rot, int64_t q_stride,
-                       int64_t k_stride, int64_t v_stride, int interleave, int dtype,
+                       int64_t k_stride, int64_t v_stride, int interleave, int dtype, int sm_budget,
                        spd_stream_t stream, bool write_pool) {
   SPD_REQUIRE(q && k && cos_sin_cache && pos_ids, SPD_E_BADARG, "spd_rope: null pointer");
   if (write_pool) SPD_REQUIRE(v && k_pool && v_pool && loc, SPD_E_BADARG, "spd_rope_kvwrite: null pointer");
@@ -736,11 +736,14 @@ static int rope_common(void* q, void* k, const void* v, void* k_pool, void* v_po
                   (!write_pool || (aligned16(v) && aligned16(k_pool) && aligned16(v_pool))),
               SPD_E_ALIGN, "spd_rope: pointers must be 16-B aligned");
   if (tokens == 0) return 0;
-  // Up to three tokens an SM: a thread for each pair of vectors to rotate and each of v to copy, so that a token's rows take
-  // one trip to memory instead of three (32 / 8 heads of 128, 448 threads / 256, us: 1 token 1.7 / 2.1, 160 2.3 / 3.7, 300
-  // 3.1 / 3.9, 450 3.8 / 4.1, 600 4.6 / 4.1, 1300 8.0 / 6.5).
+  // Up to three tokens an SM of the caller's: a thread for each pair of vectors to rotate and each of v to copy, so that a token's
+  // rows take one trip to memory instead of three (32 / 8 heads of 128, 448 threads / 256, us: 1 token 1.7 / 2.1, 160 2.3 / 3.7, 300
+  // 3.1 / 3.9, 450 3.8 / 4.1, 600 4.6 / 4.1, 1300 8.0 / 6.5; on 72 SMs 216 3.6 / 4.4, 340 4.9 / 4.4; on 40 300 6.8 / 6.3).  With more than
+  // 512 pieces it takes two, and pays from two tokens on three SMs on (64 / 8 heads, 512 / 256: 64 tokens 3.7 / 3.4, 120 3.8 / 4.1, 216
+  // 3.9 / 5.3; on 72 SMs 32 3.6 / 3.3, 64 3.6 / 4.5, 300 7.2 / 5.7).
   const int64_t pieces = (Hq + Hk) * static_cast<int64_t>(interleave ? rot >> 3 : rot >> 4) + (write_pool ? Hk * (D >> 3) : 0);
-  const bool wide = tokens <= 3 * device_sm_count_cached();
+  const int sms = sm_budget > 0 ? sm_budget : device_sm_count_cached();
+  const bool wide = tokens <= 3 * sms && (pieces <= 512 || 3 * tokens >= 2 * sms);
   const dim3 threads(static_cast<unsigned>(!wide ? 256 : pieces >= 512 ? 512 : pieces <= 64 ? 64 : (pieces + 31) / 32 * 32));
   SPD_DISPATCH_DTYPE(dtype, {
     auto kern = write_pool ? (wide ? rope_kernel<T, true, true> : rope_kernel<T, true, false>)
@@ -753,23 +756,38 @@ static int rope_common(void* q, void* k, const void* v, void* k_pool, void* v_po
   return 0;
 }
 
+int spd_rope_inplace_sms(void* q, void* k, const float* cos_sin_cache, const int64_t* pos_ids,
+                         int64_t tokens, int num_q_heads, int num_k_heads, int head_dim, int rot_dim,
+                         int64_t q_stride, int64_t k_stride, int interleave, int dtype, int sm_budget,
+                         spd_stream_t stream) {
+  return rope_common(q, k, nullptr, nullptr, nullptr, cos_sin_cache, pos_ids, nullptr, tokens,
+                     num_q_heads, num_k_heads, head_dim, rot_dim, q_stride, k_stride, 0, interleave,
+                     dtype, sm_budget, stream, false);
+}
 int spd_rope_inplace(void* q, void* k, const float* cos_sin_cache, const int64_t* pos_ids,
                      int64_t tokens, int num_q_heads, int num_k_heads, int head_dim, int rot_dim,
                      int64_t q_stride, int64_t k_stride, int interleave, int dtype,
                      spd_stream_t stream) {
-  return rope_common(q, k, nullptr, nullptr, nullptr, cos_sin_cache, pos_ids, nullptr, tokens,
-                     num_q_heads, num_k_heads, head_dim, rot_dim, q_stride, k_stride, 0, interleave,
-                     dtype, stream, false);
+  return spd_rope_inplace_sms(q, k, cos_sin_cache, pos_ids, tokens, num_q_heads, num_k_heads, head_dim, rot_dim, q_stride,
+                              k_stride, interleave, dtype, 0, stream);
 }
 
+int spd_rope_kvwrite_sms(void* q, void* k, const void* v, void* k_pool, void* v_pool,
+                         const float* cos_sin_cache, const int64_t* pos_ids, const int64_t* loc,
+                         int64_t tokens, int num_q_heads, int num_k_heads, int head_dim, int rot_dim,
+                         int64_t q_stride, int64_t k_stride, int64_t v_stride, int interleave,
+                         int dtype, int sm_budget, spd_stream_t stream) {
+  return rope_common(q, k, v, k_pool, v_pool, cos_sin_cache, pos_ids, loc, tokens, num_q_heads,
+                     num_k_heads, head_dim, rot_dim, q_stride, k_stride, v_stride, interleave,
+                     dtype, sm_budget, stream, true);
+}
 int spd_rope_kvwrite(void* q, void* k, const void* v, void* k_pool, void* v_pool,
                      const float* cos_sin_cache, const int64_t* pos_ids, const int64_t* loc,
                      int64_t tokens, int num_q_heads, int num_k_heads, int head_dim, int rot_dim,
                      int64_t q_stride, int64_t k_stride, int64_t v_stride, int interleave,
                      int dtype, spd_stream_t stream) {
-  return rope_common(q, k, v, k_pool, v_pool, cos_sin_cache, pos_ids, loc, tokens, num_q_heads,
-                     num_k_heads, head_dim, rot_dim, q_stride, k_stride, v_stride, interleave,
-                     dtype, stream, true);
+  return spd_rope_kvwrite_sms(q, k, v, k_pool, v_pool, cos_sin_cache, pos_ids, loc, tokens, num_q_heads, num_k_heads, head_dim,
+                              rot_dim, q_stride, k_stride, v_stride, interleave, dtype, 0, stream);
 }
 
 int spd_kv_write(const void* k, const void* v, void* k_pool, void* v_pool, const int64_t* loc,

@@ -72,6 +72,7 @@ struct Call<int(A...)> {
 
 #define SPD_CALLS \
   X(spd_wait_selftest) X(spd_rmsnorm) X(spd_fused_add_rmsnorm) X(spd_silu_and_mul) X(spd_rope_inplace) X(spd_rope_kvwrite) \
+  X(spd_rope_inplace_sms) X(spd_rope_kvwrite_sms) \
   X(spd_kv_write) X(spd_gather_rows) X(spd_argmax_f32) X(spd_argmax_partial_f32) X(spd_argmax_merge) \
   X(spd_compute_positions) X(spd_decode_positions) X(spd_build_kv_indices) X(spd_write_req_to_token) X(spd_layernorm) \
   X(spd_bias_act_residual) X(spd_gemm) X(spd_attn_prefill_ragged) X(spd_attn_decode_paged) X(spd_attn_decode_paged_own) \

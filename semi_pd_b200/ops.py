@@ -152,10 +152,10 @@ def apply_rope_with_cos_sin_cache_inplace(positions: torch.Tensor, query: torch.
         positions = positions.long()
     T = query.shape[0]
     q2, k2 = query.view(T, -1), key.view(T, -1)
-    check(lib.spd_rope_inplace(q2.data_ptr(), k2.data_ptr(), cos_sin_cache.data_ptr(),
-                               positions.data_ptr(), T, q2.shape[1] // head_size,
-                               k2.shape[1] // head_size, head_size, cos_sin_cache.shape[1],
-                               q2.stride(0), k2.stride(0), 0 if is_neox else 1, _dt(query), _stream()),
+    check(lib.spd_rope_inplace_sms(q2.data_ptr(), k2.data_ptr(), cos_sin_cache.data_ptr(),
+                                   positions.data_ptr(), T, q2.shape[1] // head_size,
+                                   k2.shape[1] // head_size, head_size, cos_sin_cache.shape[1],
+                                   q2.stride(0), k2.stride(0), 0 if is_neox else 1, _dt(query), get_sm_budget(), _stream()),
           "spd_rope_inplace")
 
 
@@ -171,12 +171,12 @@ def rope_kvwrite(positions: torch.Tensor, query: torch.Tensor, key: torch.Tensor
         raise RuntimeError("rope_kvwrite: positions and out_cache_loc must be int64")
     T = query.shape[0]
     q2, k2, v2 = query.view(T, -1), key.view(T, -1), value.view(T, -1)
-    check(lib.spd_rope_kvwrite(q2.data_ptr(), k2.data_ptr(), v2.data_ptr(), k_pool.data_ptr(),
-                               v_pool.data_ptr(), cos_sin_cache.data_ptr(), positions.data_ptr(),
-                               out_cache_loc.data_ptr(), T, q2.shape[1] // head_size,
-                               k2.shape[1] // head_size, head_size, cos_sin_cache.shape[1],
-                               q2.stride(0), k2.stride(0), v2.stride(0), 0 if is_neox else 1,
-                               _dt(query), _stream()), "spd_rope_kvwrite")
+    check(lib.spd_rope_kvwrite_sms(q2.data_ptr(), k2.data_ptr(), v2.data_ptr(), k_pool.data_ptr(),
+                                   v_pool.data_ptr(), cos_sin_cache.data_ptr(), positions.data_ptr(),
+                                   out_cache_loc.data_ptr(), T, q2.shape[1] // head_size,
+                                   k2.shape[1] // head_size, head_size, cos_sin_cache.shape[1],
+                                   q2.stride(0), k2.stride(0), v2.stride(0), 0 if is_neox else 1,
+                                   _dt(query), get_sm_budget(), _stream()), "spd_rope_kvwrite")
 
 
 def kv_write(key: torch.Tensor, value: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,

@@ -36,3 +36,14 @@ def test_rope_kvwrite(tokens, heads, neox):
         got = got.double().cpu().reshape(tokens, -1)
         assert ((got - want).abs() <= want.abs() * 2 ** -8 + 1e-5).all()
     assert torch.equal(vp[loc.cuda()].reshape(tokens, -1).cpu(), qkv[:, (Hq + Hk) * D:])
+
+
+@pytest.mark.parametrize("sms,tokens", [(2, 1), (2, 2), (2, 6), (2, 7), (72, 47), (72, 48), (72, 216), (72, 217)])
+@pytest.mark.parametrize("heads", [(32, 8, 128, 128), (64, 8, 128, 128)])
+def test_lines_follow_the_callers_sms(sms, tokens, heads):
+    from semi_pd_b200 import ops
+    ops.set_sm_budget(sms)
+    try:
+        test_rope_kvwrite(tokens, heads, True)
+    finally:
+        ops.set_sm_budget(0)
