@@ -59,7 +59,7 @@ constexpr int kNormThreads = 256;
 // registers) so that the common 4096-wide row costs ~40 registers and 8 CTAs fit per SM — the
 // kernel is a pure HBM stream and needs the bytes in flight.
 
-template <typename T, bool kFusedAdd, int kMaxVec>
+template <typename T, bool kFusedAdd, int kMaxVec, bool kWeightsFirst>
 __global__ void __launch_bounds__(kNormThreads)
 rmsnorm_kernel(T* out, T* x, T* residual,  // out may alias x (fused variant is in place)
                const T* __restrict__ w, int64_t dim, int64_t x_stride, int64_t out_stride,
@@ -78,13 +78,16 @@ rmsnorm_kernel(T* out, T* x, T* residual,  // out may alias x (fused variant is 
   const Vec8* wv = reinterpret_cast<const Vec8*>(w);
   float vals[kMaxVec][8];
   // The weights come beside the row, not behind its sum: one trip to memory instead of two (with the sum of a residual, 4096
-  // wide, behind such a one, 1 token 2.16 -> 1.90 us, 160 3.75 -> 3.15, 1300 6.82 -> 5.54, 4096 16.8 -> 14.5).
-  Vec8 wreg[kMaxVec];
+  // wide, behind such a one, 1 token 2.16 -> 1.90 us, 160 3.75 -> 3.15, 1300 6.82 -> 5.54, 4096 16.8 -> 14.5).  Not in long rows
+  // of many tokens, whose registers for it cost CTAs on an SM (see the launch).
+  Vec8 wreg[kWeightsFirst ? kMaxVec : 1];
   float ss = 0.f;
+  if constexpr (kWeightsFirst) {
 #pragma unroll
-  for (int i = 0; i < kMaxVec; ++i) {
-    const int v = threadIdx.x + i * kNormThreads;
-    if (v < nvec) wreg[i] = wv[v];
+    for (int i = 0; i < kMaxVec; ++i) {
+      const int v = threadIdx.x + i * kNormThreads;
+      if (v < nvec) wreg[i] = wv[v];
+    }
   }
 #pragma unroll
   for (int i = 0; i < kMaxVec; ++i) {
@@ -124,7 +127,7 @@ rmsnorm_kernel(T* out, T* x, T* residual,  // out may alias x (fused variant is 
     const int v = threadIdx.x + i * kNormThreads;
     if (v < nvec) {
       float wf[8], o[8];
-      vec8_to_f32<T>(wreg[i], wf);
+      vec8_to_f32<T>(kWeightsFirst ? wreg[kWeightsFirst ? i : 0] : wv[v], wf);
 #pragma unroll
       for (int j = 0; j < 8; ++j) o[j] = vals[i][j] * inv * wf[j];
       orow[v] = f32_to_vec8<T>(o);
@@ -673,14 +676,25 @@ int spd_rmsnorm(void* out, const void* x, const void* w, int64_t tokens, int64_t
                   aligned16(x) && aligned16(w),
               SPD_E_ALIGN, "spd_rmsnorm: dim/strides must be multiples of 8 and pointers 16-B aligned");
   if (tokens == 0) return 0;
-#define SPD_NORM_LAUNCH(FUSED, VEC, ...)                                                         \
-  SPD_CUDA(launch(rmsnorm_kernel<T, FUSED, VEC>, dim3((unsigned)tokens), dim3(kNormThreads), 0, \
+  // Weights beside the row / behind its sum, us on 148 SMs: 8192 wide with a residual, 160 tokens 3.7 / 4.6, 1000 16.5 / 15.1, 4096
+  // 55 / 51, without one 300 3.9 / 5.1, 4096 30 / 28; 5120 wide without one 1300 7.3 / 7.7, 4096 18.7 / 19.1; 8200 wide 148 2.5 / 3.6, 4096
+  // 36 / 38, with a residual 72 / 76; 16384 wide 64 3.0 / 3.6, 4096 75 / 65 (148 on 72 SMs 6.1 / 5.9), with a residual 120 / 128.
+#define SPD_NORM_LAUNCH(FUSED, VEC, FIRST, ...)                                                         \
+  SPD_CUDA(launch(rmsnorm_kernel<T, FUSED, VEC, FIRST>, dim3((unsigned)tokens), dim3(kNormThreads), 0, \
                   as_stream(stream), pdl_enabled(), __VA_ARGS__))
-#define SPD_NORM_DISPATCH(FUSED, ...)                                         \
-  do {                                                                        \
-    if (dim <= 2 * 8 * kNormThreads) SPD_NORM_LAUNCH(FUSED, 2, __VA_ARGS__);  \
-    else if (dim <= 4 * 8 * kNormThreads) SPD_NORM_LAUNCH(FUSED, 4, __VA_ARGS__); \
-    else SPD_NORM_LAUNCH(FUSED, 8, __VA_ARGS__);                              \
+#define SPD_NORM_DISPATCH(FUSED, ...)                                                                    \
+  do {                                                                                                   \
+    const int64_t sms = device_sm_count_cached();                                                        \
+    if (dim <= 2 * 8 * kNormThreads)                                                                     \
+      SPD_NORM_LAUNCH(FUSED, 2, true, __VA_ARGS__);                                                      \
+    else if (dim <= 4 * 8 * kNormThreads && (tokens <= 3 * sms || (!FUSED && dim <= 3 * 8 * kNormThreads))) \
+      SPD_NORM_LAUNCH(FUSED, 4, true, __VA_ARGS__);                                                      \
+    else if (dim <= 4 * 8 * kNormThreads)                                                                \
+      SPD_NORM_LAUNCH(FUSED, 4, false, __VA_ARGS__);                                                     \
+    else if (FUSED || dim <= 6 * 8 * kNormThreads || 2 * tokens <= sms)                                  \
+      SPD_NORM_LAUNCH(FUSED, 8, true, __VA_ARGS__);                                                      \
+    else                                                                                                 \
+      SPD_NORM_LAUNCH(FUSED, 8, false, __VA_ARGS__);                                                     \
   } while (0)
   SPD_DISPATCH_DTYPE(dtype, {
     SPD_NORM_DISPATCH(false, (T*)out, (T*)x, (T*)nullptr, (const T*)w, dim, x_stride, out_stride,
