@@ -21,8 +21,10 @@ struct __align__(16) MVec8 {
 
 constexpr int kMoeMaxExperts = 256;
 constexpr int kMoeMaxTopK = 8;
-// Every kernel here lets the next one's blocks in at once (they wait for this grid's end themselves): a layer is a chain of
-// seven short launches, 40 tokens through 64 experts 218 -> 214 us.
+// The kernels here but moe_align let the next one's blocks in at once (they wait for this grid's end themselves): a layer is a
+// chain of seven short launches, 40 tokens through 64 experts 218 -> 214 us.  What follows moe_align is better let in at its end:
+// with the gather's blocks and the grouped GEMM's pairs waiting on the SMs behind them, layers by expert of few tokens took longer
+// than without any of it (8 experts of 7168, one token 98.6 -> 105.4 us, 97.9 so; 64 of 1408, 4 tokens 98.9 -> 102.0, 97.8 so).
 constexpr int kMoeTile = 128;  // rows per expert-aligned tile == UMMA M of the grouped GEMM
 
 // One warp per token: softmax over E logits (fp32), then top-k by repeated arg-max (ties -> the
@@ -110,7 +112,6 @@ moe_align_kernel(int32_t* __restrict__ row_token, int32_t* __restrict__ inv_pos,
   __shared__ int cnt[kMoeMaxExperts];  // this CTA's entries per expert
   __shared__ int off[kMoeMaxExperts + 1];
   __shared__ int cur[kMoeMaxExperts];  // the next place
-  griddep_launch_dependents();
   griddep_wait();
   const int tid = threadIdx.x;
   const int rank = kCtas > 1 ? static_cast<int>(cluster_ctarank()) : 0;
