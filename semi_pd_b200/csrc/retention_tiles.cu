@@ -897,14 +897,17 @@ static int rt_launch(const RetTileParams& t, int sms, cudaStream_t stream) {
   return 0;
 }
 
-// Estimated us: 10 and 18.5 a wave of tiles (its sums, its part of the scan, its outputs), 64 value columns at a time 12 and
-// 14 (bf16) or 16 (fp16).  Taken where that is 7 % below the chunks' estimate (retention_chunked_us).  16 heads of 128 x 128,
-// chunks / tiles in us: 1 x 200 tokens 27.6 / 25.8 (not taken), 300 33.2 / 26.3, 1500 67.9 / 43.5, 8000 235 / 148; 4 x 250 34 / 43
-// (not taken), 4 x 500 67 / 51, 8 x 128 43 / 51 (not taken), 8 x 1000 222 / 162.
+// Estimated us: 11 and 18.5 a wave of tiles (its sums, its part of the scan, its outputs), 64 value columns at a time 12 and
+// 15 (bf16) or 16 (fp16).  Taken where that is 7 % below the chunks' estimate (retention_chunked_us) and the portions of a single
+// wave have more than four chunks in the mean.  16 heads of 128 x 128, chunks / tiles in us: 1 x 256 tokens 29.1 / 31.1 (not taken),
+// 300 35.3 / 31.1, 1500 67.9 / 43.5, 8000 235 / 148; 2 x 250 29.8 / 33.2 (not taken), 2 x 450 52 / 35, 4 x 250 31 / 38 (not taken), 4 x
+// 500 67 / 51, 8 x 300 69 / 77 (not taken), 8 x 1000 222 / 162; on 72 SMs 4 x 300 67 / 71 (not taken).  Of 2280 calls (1 - 64 portions of
+// 64 - 8000 tokens, 4 - 32 heads, 64 - 256 value columns, both types, 148, 72 and 40 SMs) 8 take 2 - 6 % more than in chunks.
 static bool rt_pays(int64_t batch, int64_t total_tokens, int H, int dv, bool half, int sms) {
   const int cols = !half && dv % 128 == 0 ? 128 : 64;
   const double items = (static_cast<double>(total_tokens) / kRtTok + 0.5 * static_cast<double>(batch)) * H * (dv / cols);
-  const double waves = ceil(items / sms), us = cols == 128 ? 10 + 18.5 * waves : 12 + (half ? 16.0 : 14.0) * waves;
+  const double waves = ceil(items / sms), us = cols == 128 ? 11 + 18.5 * waves : 12 + (half ? 16.0 : 15.0) * waves;
+  if (waves <= 1 && total_tokens <= 2 * kRtTok * batch) return false;
   return us < 0.93 * retention_chunked_us(batch, total_tokens, H, dv, sms);
 }
 

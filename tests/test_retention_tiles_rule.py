@@ -25,3 +25,16 @@ def test_not_for_other_sizes():
                  (1, 4000, 16, 128, 128, 64, 0, _lib.SPD_F32, 148), (0, 4000, 16, 128, 128, 64, 0, _lib.SPD_BF16, 148),
                  (100, 4000, 16, 128, 128, 64, 0, _lib.SPD_BF16, 148)):
         assert f(*args) == 0
+
+
+@pytest.mark.parametrize("batch,tokens,heads,dv,sms", [(4, 1000, 4, 128, 72), (2, 500, 4, 128, 148), (8, 2000, 4, 128, 148), (2, 500, 16, 128, 148),
+                                                       (8, 2400, 16, 128, 148), (4, 1200, 16, 128, 72), (1, 256, 16, 128, 148)])
+def test_chunks_are_faster(batch, tokens, heads, dv, sms):
+    assert _lib.lib.spd_retention_tiles_workspace_bytes(batch, tokens, heads, 128, dv, 64, 0, _lib.SPD_BF16, sms) == 0
+
+
+@pytest.mark.parametrize("batch,tokens,heads,dv,dtype,sms", [(1, 400, 4, 128, "bf16", 148), (2, 900, 16, 128, "bf16", 148), (4, 2000, 16, 128, "bf16", 148),
+                                                             (2, 1600, 4, 64, "f16", 72), (1, 8000, 8, 256, "bf16", 40)])
+def test_tiles_are_faster(batch, tokens, heads, dv, dtype, sms):
+    dt = _lib.SPD_BF16 if dtype == "bf16" else _lib.SPD_F16
+    assert _lib.lib.spd_retention_tiles_workspace_bytes(batch, tokens, heads, 128, dv, 64, 0, dt, sms) > 0
