@@ -554,7 +554,7 @@ int spd_retention_extend_ws(float* o, const void* q, const void* k, const void* 
                             spd_stream_t stream);
 
 /* The same in tiles of 128 tokens that all run at once, for batches of some hundred tokens and more; workspace of
- * spd_retention_tiles_workspace_bytes (0: not for these sizes), not zeroed, one call at a time.  Everything 16-byte aligned,
+ * spd_retention_tiles_workspace_bytes (512 MB at most; 0: not for these sizes), not zeroed, one call at a time.  Everything 16-byte aligned,
  * strides multiples of 8. */
 int64_t spd_retention_tiles_workspace_bytes(int64_t batch, int64_t total_tokens, int num_heads, int head_dim, int v_dim,
                                             int rot_dims, int in_act, int dtype, int sm_budget);

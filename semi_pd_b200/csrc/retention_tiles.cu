@@ -911,6 +911,10 @@ static bool rt_pays(int64_t batch, int64_t total_tokens, int H, int dv, bool hal
   return us < 0.93 * retention_chunked_us(batch, total_tokens, H, dv, sms);
 }
 
+// A call's scratch at most, beyond which the chunks serve, which want far less or none: it is 10 bytes a state value and 128 tokens
+// (4 x 2048 tokens, 16 heads of 128 x 128: 178 MB), and a server leaves little beside its caches.
+constexpr int64_t kRtMaxScratch = 512ll << 20;
+
 static int64_t rt_tiles(int64_t batch, int64_t total_tokens) { return total_tokens / kRtTok + batch; }
 // fp32 sums, then the states' parts
 static int64_t rt_state_bytes(int64_t tiles, int H, int dv, int bytes) { return tiles * H * static_cast<int64_t>(dv) * kRcDk * bytes; }
@@ -929,7 +933,8 @@ int64_t spd_retention_tiles_workspace_bytes(int64_t batch, int64_t total_tokens,
     return 0;
   if (!rt_pays(batch, total_tokens, num_heads, v_dim, dtype == SPD_F16, sm_budget > 0 ? sm_budget : device_sm_count_cached())) return 0;
   const int64_t tiles = rt_tiles(batch, total_tokens);
-  return rt_state_bytes(tiles, num_heads, v_dim, 10) + tiles * 32 + ((tiles + batch) * (v_dim / kRcDv) + kRtTok + 1) * num_heads * 4;
+  const int64_t room = rt_state_bytes(tiles, num_heads, v_dim, 10) + tiles * 32 + ((tiles + batch) * (v_dim / kRcDv) + kRtTok + 1) * num_heads * 4;
+  return room <= kRtMaxScratch ? room : 0;
 }
 
 int spd_retention_extend_tiles(float* o, const void* q, const void* k, const void* v, float* state,

@@ -38,3 +38,15 @@ def test_chunks_are_faster(batch, tokens, heads, dv, sms):
 def test_tiles_are_faster(batch, tokens, heads, dv, dtype, sms):
     dt = _lib.SPD_BF16 if dtype == "bf16" else _lib.SPD_F16
     assert _lib.lib.spd_retention_tiles_workspace_bytes(batch, tokens, heads, 128, dv, 64, 0, dt, sms) > 0
+
+
+def test_scratch_has_a_limit():
+    """Long batches go to the chunks, which ran in little memory before there were tiles."""
+    room = _lib.lib.spd_retention_tiles_workspace_bytes
+    for batch, tokens, heads, dv in ((1, 131072, 16, 128), (1, 65536, 32, 256), (4, 65536, 64, 256), (8, 32768, 16, 128)):
+        assert room(batch, tokens, heads, 128, dv, 64, 0, _lib.SPD_BF16, 148) == 0
+        chunks = _lib.lib.spd_retention_workspace_bytes(batch, tokens, heads, 128, dv, 64, 0, _lib.SPD_BF16, 148)
+        assert chunks <= 512 << 20
+    assert 0 < room(4, 16384, 16, 128, 128, 64, 0, _lib.SPD_BF16, 148) <= 512 << 20
+    for tokens in range(1000, 200000, 3717):
+        assert room(1, tokens, 16, 128, 128, 64, 0, _lib.SPD_BF16, 148) <= 512 << 20
