@@ -33,7 +33,14 @@ constexpr int kPsHalfBytes = 128 * kPsBK * 2;  // 128 rows of one operand
 constexpr int kPsTokens = 64;                  // tokens staged at a time
 constexpr int kPsMaxTiles = 512;               // token tiles of a call
 constexpr int kPsStageBytes = kPsTokens * (256 + 16);
-constexpr int kPsFixedSmem = kPsStageBytes + 256 + 1024;  // beside the ring and the list of token tiles
+struct PsControl {  // behind the list of token tiles
+  uint64_t full[kPsStages], empty[kPsStages];  // (the leader's full are the live ones)
+  uint64_t tfull[2], tempty[2];                // (the leader's tempty)
+  uint32_t tmem;
+  int dead;
+  int warp_tiles[kPsThreads / 32];
+};
+constexpr int kPsFixedSmem = kPsStageBytes + (sizeof(PsControl) + 15) / 16 * 16 + 1024;  // beside the ring and the list
 constexpr int kPsMaxSmem = 232448;
 static_assert(6 * 2 * kPsHalfBytes + kPsMaxTiles * 16 + kPsFixedSmem <= kPsMaxSmem, "shared memory of a CTA");
 
@@ -113,14 +120,11 @@ gemm_pair_swap_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t* sOut = smem + p.stages * p.slot;
   int4* tiles = reinterpret_cast<int4*>(sOut + kPsStageBytes);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(tiles + p.list);
-  uint64_t* full = bars;                        // [stages]  (leader's are the live ones)
-  uint64_t* empty = bars + kPsStages;           // [stages]
-  uint64_t* tfull = bars + 2 * kPsStages;       // [2]
-  uint64_t* tempty = bars + 2 * kPsStages + 2;  // [2]       (leader's are the live ones)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kPsStages + 4);
-  volatile int* dead = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  int* warp_tiles = reinterpret_cast<int*>(tmem_slot + 2);  // [8]
+  PsControl& control = *reinterpret_cast<PsControl*>(tiles + p.list);
+  uint64_t *full = control.full, *empty = control.empty, *tfull = control.tfull, *tempty = control.tempty;
+  uint32_t* tmem_slot = &control.tmem;
+  volatile int* dead = &control.dead;
+  int* warp_tiles = control.warp_tiles;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
