@@ -21,10 +21,10 @@ struct __align__(16) MVec8 {
 
 constexpr int kMoeMaxExperts = 256;
 constexpr int kMoeMaxTopK = 8;
-// The kernels here but moe_align let the next one's blocks in at once (they wait for this grid's end themselves): a layer is a
-// chain of seven short launches, 40 tokens through 64 experts 218 -> 214 us.  What follows moe_align is better let in at its end:
-// with the gather's blocks and the grouped GEMM's pairs waiting on the SMs behind them, layers by expert of few tokens took longer
-// than without any of it (8 experts of 7168, one token 98.6 -> 105.4 us, 97.9 so; 64 of 1408, 4 tokens 98.9 -> 102.0, 97.8 so).
+// No kernel here lets the next one's blocks in before its end.  Let in at the start of all five (2 % off a layer of 40 tokens
+// through 64 experts, 218 -> 214 us), they now and then brought passes of 4096 tokens to a stand, with route,
+// align (a cluster), gather and the grouped GEMM all on the SMs behind one another.  Why is not known: each waits for the one
+// before it, and none is let in before that one's blocks are all there.
 constexpr int kMoeTile = 128;  // rows per expert-aligned tile == UMMA M of the grouped GEMM
 
 // One warp per token: softmax over E logits (fp32), then top-k by repeated arg-max (ties -> the
@@ -33,7 +33,6 @@ template <typename T>
 __global__ void __launch_bounds__(128)
 moe_route_kernel(int32_t* __restrict__ topk_ids, float* __restrict__ topk_w, const T* __restrict__ logits,
                  int64_t tokens, int E, int k, float scale, int renorm) {
-  griddep_launch_dependents();
   griddep_wait();
   const int lane = threadIdx.x & 31;
   const int64_t t = blockIdx.x * 4ll + (threadIdx.x >> 5);
@@ -209,7 +208,6 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 moe_gather_kernel(T* __restrict__ xs, const T* __restrict__ x, const int32_t* __restrict__ row_token, int64_t rows,
                   int64_t dim, int64_t x_stride) {
-  griddep_launch_dependents();
   griddep_wait();
   const int64_t r = blockIdx.x * 8ll + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
@@ -236,7 +234,6 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 moe_combine_kernel(T* __restrict__ out, const T* __restrict__ y, const T* __restrict__ shared,
                    const int32_t* __restrict__ inv_pos, const float* __restrict__ topk_w, int k, int64_t dim) {
-  griddep_launch_dependents();
   griddep_wait();
   const int64_t t = blockIdx.x;
   const int nv = static_cast<int>(dim >> 3);
@@ -281,7 +278,6 @@ __global__ void __launch_bounds__(256)
 moe_dense_act_kernel(T* __restrict__ act, const T* __restrict__ gate_up, const int32_t* __restrict__ topk_ids,
                      const float* __restrict__ topk_w, int k, int E, int64_t inter) {
   __shared__ float w_e[kMoeMaxExperts];
-  griddep_launch_dependents();
   griddep_wait();
   const int64_t t = blockIdx.x;
   for (int e = threadIdx.x; e < E; e += 256) w_e[e] = 0.f;
