@@ -548,6 +548,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUt
     }
   }
 
+  __syncwarp();  // the warps of the elected lanes come together before the barriers, which count whole warps
   if constexpr (!kSwap) griddep_launch_dependents();
   tc_fence_before_sync();
   __syncthreads();

@@ -206,6 +206,7 @@ gemm_cluster_splitk_kernel(const __grid_constant__ CUtensorMap tmW, const __grid
     }
   }
 
+  __syncwarp();  // the warps of the elected lanes come together before the barriers, which count whole warps
   tc_fence_before_sync();
   __syncthreads();
   cluster_sync_all();  // nobody leaves while a peer may still touch its shared memory / barriers

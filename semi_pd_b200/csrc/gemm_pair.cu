@@ -233,6 +233,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
   }
 
+  __syncwarp();  // the warps of the elected lanes come together before the barriers, which count whole warps
   griddep_launch_dependents();
   tc_fence_before_sync();
   __syncthreads();

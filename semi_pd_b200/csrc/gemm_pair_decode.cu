@@ -468,6 +468,7 @@ gemm_pair_decode_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_co
     PD_STAMP(6);  // epilogue role done
   }
 
+  __syncwarp();  // the warps of the elected lanes come together before the barriers, which count whole warps
   tc_fence_before_sync();
   __syncthreads();
   cluster_sync_all();  // the peer may still read this CTA's shared memory / signal its barriers

@@ -338,6 +338,7 @@ gemm_pair_swap_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_cons
     }
   }
 
+  __syncwarp();  // the warps of the elected lanes come together before the barriers, which count whole warps
   if (!p.decode) griddep_launch_dependents();
   tc_fence_before_sync();
   __syncthreads();
