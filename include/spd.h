@@ -213,6 +213,8 @@ int spd_gemm_split_tiles(int64_t M, int64_t N, int64_t K, int epilogue, int out_
 /* Clusters of `split` pairs that this choice reckons with on sm_budget SMs when the driver says that `found` run at once (-1:
  * there is none to ask).  A call on a partition asks for its own stream, since its SMs' places decide: it may split less. */
 int spd_gemm_split_room(int split, int found, int sm_budget);
+/* After those: CTAs that up to 32 tokens' GEMM without an epilogue takes in clusters of single CTAs that cut K, 0: the others. */
+int spd_gemm_cluster_ctas(int64_t M, int64_t N, int64_t K, int sm_budget);
 /* Whether SPD_EPI_SILU_MUL serves M tokens at least as well as the plain GEMM and spd_silu_and_mul (N: output columns). */
 int spd_gemm_silu_fused(int64_t M, int64_t N, int64_t K, int sm_budget);
 int spd_gemm(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_t K, int64_t lda,

@@ -69,6 +69,7 @@ SIGNATURES = {
     "spd_gemm_swap_rows": (_i, [_i64, _i64, _i64, _i, _i]),
     "spd_gemm_split_tiles": (_i, [_i64, _i64, _i64, _i, _i, _i, _p]),
     "spd_gemm_split_room": (_i, [_i, _i, _i]),
+    "spd_gemm_cluster_ctas": (_i, [_i64, _i64, _i64, _i]),
     "spd_gemm_silu_fused": (_i, [_i64, _i64, _i64, _i]),
     "spd_attn_general_tcgen05": (_i, [_i64, _i64, _i64, _i, _i, _i, _i]),
     "spd_gemm": (

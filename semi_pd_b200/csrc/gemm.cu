@@ -621,6 +621,7 @@ long long streamk_ctas(long long tiles, int kblocks, int split, long long slots)
   return g;
 }
 
+int gemm_cluster_ctas(int64_t M, int64_t N, int64_t K, int sms);
 int gemm_cluster_try(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_t K, int64_t lda,
                      int64_t ldw, int64_t ldc, int dtype, int out_f32, int sms, cudaStream_t stream);
 
@@ -699,6 +700,11 @@ int spd_gemm_split_tiles(int64_t M, int64_t N, int64_t K, int epilogue, int out_
 
 int spd_gemm_split_room(int split, int found, int sm_budget) {
   return split_room_of(split, found, sm_budget > 0 ? sm_budget : device_sm_count_cached());
+}
+
+int spd_gemm_cluster_ctas(int64_t M, int64_t N, int64_t K, int sm_budget) {
+  if (M <= 0 || N <= 0 || K <= 0) return SPD_E_BADARG;
+  return gemm_cluster_ctas(M, N, K, sm_budget > 0 ? sm_budget : device_sm_count_cached());
 }
 
 int spd_gemm_swap_rows(int64_t M, int64_t N, int64_t K, int epilogue, int sm_budget) {

@@ -1,4 +1,4 @@
-// GEMM of up to 16 tokens (gemm_pair_split.cu says which) with split-K across a THREAD-BLOCK CLUSTER, reduced on chip through
+// GEMM of up to 16 tokens, of up to 32 on short rows (those that gemm_pair_split.cu leaves) with split-K across a THREAD-BLOCK CLUSTER, reduced on chip through
 // distributed shared memory — for the layers whose N gives fewer 128-row weight tiles than there
 // are SMs (W_qkv: 48 tiles, W_o and W_down: 32 tiles on Llama-3-8B).  One SM streams ~90-100 GB/s
 // however deep its TMA ring is, so those layers need 3-4 SMs per tile to approach HBM speed; a
@@ -247,8 +247,12 @@ static int cluster_split(int64_t tiles, int64_t kblocks, int sms) {
   return static_cast<int>(S > kblocks / 8 ? kblocks / 8 : S);  // >= 8 k-blocks per rank
 }
 
-// CTAs of a GEMM of up to 16 tokens here, 0: not taken.
-int gemm_cluster_ctas(int64_t N, int64_t K, int sms) {
+// CTAs of a GEMM here, 0: not taken.  17 - 32 tokens come where K is at most 1024 (16 k-blocks: pairs of CTAs): stream-K
+// (gemm.cu), which they take beyond, has an end of its own length.  32 tokens with fp32 results, stream-K / here, us: K = 1024,
+// N = 512 7.2 / 6.8, 2048 8.0 / 7.3, 4096 8.8 / 7.8; K = 2048 1 - 4 % apart either way; K = 4096, N = 4096 0.93 times the time, N =
+// 2048 on 76 SMs 0.52 times.
+int gemm_cluster_ctas(int64_t M, int64_t N, int64_t K, int sms) {
+  if (M > (K <= 16 * kCgBK ? 32 : 16)) return 0;
   const int64_t tiles = (N + kCgBM - 1) / kCgBM;
   const int S = cluster_split(tiles, (K + kCgBK - 1) / kCgBK, sms);
   return S < 2 ? 0 : static_cast<int>(tiles * S);
@@ -259,13 +263,12 @@ int gemm_cluster_ctas(int64_t N, int64_t K, int sms) {
 int gemm_cluster_try(void* C, const void* A, const void* W, int64_t M, int64_t N, int64_t K, int64_t lda,
                      int64_t ldw, int64_t ldc, int dtype, int out_f32, int sms, cudaStream_t stream) {
   static const int enabled = getenv("SPD_GEMM_CLUSTER") ? atoi(getenv("SPD_GEMM_CLUSTER")) : 1;
-  if (!enabled || M > 16) return 1;  // more tokens: gemm_pair_split.cu
+  if (!enabled || gemm_cluster_ctas(M, N, K, sms) == 0) return 1;
   const int tiles = static_cast<int>((N + kCgBM - 1) / kCgBM);
   const int kblocks = static_cast<int>((K + kCgBK - 1) / kCgBK);
-  constexpr int BN = 16;
   const int S = cluster_split(tiles, kblocks, sms);
-  static_assert(3 * cg_part_bytes<BN>() <= cg_stages<BN>() * cg_stage_bytes<BN>(), "the partial sums of a tile fit the ring");
-  if (S < 2) return 1;
+  static_assert(3 * cg_part_bytes<16>() <= cg_stages<16>() * cg_stage_bytes<16>() &&
+                    3 * cg_part_bytes<32>() <= cg_stages<32>() * cg_stage_bytes<32>(), "the partial sums of a tile fit the ring");
   ClusterGemmParams p{};
   p.C = C;
   p.ldc = ldc;
@@ -276,8 +279,9 @@ int gemm_cluster_try(void* C, const void* A, const void* W, int64_t M, int64_t N
   CUtensorMap tw, ta;
   int rc;
   if ((rc = get_tmap(&tw, W, N, K, ldw, kCgBM))) return rc;
-  if ((rc = get_tmap(&ta, A, M, K, lda, BN))) return rc;
-  SPD_DISPATCH_DTYPE(dtype, { return launch_cluster_gemm<T, BN>(tw, ta, p, tiles, S, stream); });
+  if ((rc = get_tmap(&ta, A, M, K, lda, M <= 16 ? 16 : 32))) return rc;
+  if (M <= 16) SPD_DISPATCH_DTYPE(dtype, { return launch_cluster_gemm<T, 16>(tw, ta, p, tiles, S, stream); });
+  SPD_DISPATCH_DTYPE(dtype, { return launch_cluster_gemm<T, 32>(tw, ta, p, tiles, S, stream); });
   return 1;
 }
 

@@ -322,7 +322,7 @@ static int split_clusters(int split, int sms, cudaStream_t stream) {
   return n;
 }
 
-int gemm_cluster_ctas(int64_t N, int64_t K, int sms);
+int gemm_cluster_ctas(int64_t M, int64_t N, int64_t K, int sms);
 int split_room_of(int split, int found, int sms) { return split >= 1 && split <= kPtMaxSplit ? split_room(split, found, sms) : 0; }
 
 // The tiles of a GEMM on few weight tiles, 0: the other kernels.  *split = pairs per tile in a cluster (this kernel), 0: tiles
@@ -392,7 +392,7 @@ int gemm_split_tiles(int64_t M, int64_t N, int64_t K, int epilogue, int out_f32,
   }
   if (M <= 16 && bytes > 2.5e7 && !silu) {
     const int ctas = static_cast<int>(w_tiles) * tiles * 2 * (*split > 0 ? *split : 1);
-    if (gemm_cluster_ctas(N, K, sms) > ctas) {
+    if (gemm_cluster_ctas(M, N, K, sms) > ctas) {
       *split = 0;
       return 0;
     }
