@@ -15,8 +15,8 @@
 // 240 us in chunks, 168 here (sums 46, scan 28, outputs 88); one request of 8000 tokens 242 -> 153.  Against 64 bits the
 // outputs' error is 2.47e-7 -> 2.10e-7, the state's 2.18e-7 -> 1.21e-7 (300 tokens: 2.01e-7 -> 2.04e-7, 1.05e-7 -> 1.07e-7).
 // What bounds it: an output tile's phases (16 k clk: splitting q and k 3.3, Q K^T 2.4, Q S with A's split beside it 3.3, A V
-// 1.7, outputs 1.7) that still follow one another for want of shared memory, issue slots 40 % busy, tensor core 29 %; the
-// sums likewise; the scan HBM (71 MB read, 107 written).
+// 1.7, outputs 1.7) that still follow one another for want of shared memory, issue slots 36 % busy, tensor core 25 %
+// (under ncu, 94 us); the sums likewise (42 %, 12 %); the scan HBM and the L2 (71 MB read, 107 written, of which 49 left it in time).
 #include <math.h>
 
 #include "retention_parts.cuh"
