@@ -30,9 +30,10 @@ from .distributed import get_tensor_model_parallel_world_size
 from .forward_batch_info import ForwardBatch, LogitsProcessorOutput
 from .layers import LinearBase, LogitsProcessor, ParallelLMHead, RMSNorm, SiluAndMul, VocabParallelEmbedding
 
-# The dense form serves batches of these sizes where it is the faster one (moe_dense_pays)
+# The dense form serves batches of these sizes where it is the faster one (moe_dense_pays); beyond 192 tokens its GEMMs' wide
+# token tiles take a step up that the estimate does not see (below: 160 experts on 72 SMs, 160 tokens 1532 / 1584, 200 1955 / 1587)
 _MOE_DENSE_MIN_TOKENS = 16
-_MOE_DENSE_MAX_TOKENS = 256
+_MOE_DENSE_MAX_TOKENS = 192
 
 
 @functools.lru_cache(maxsize=1)
@@ -47,7 +48,7 @@ def moe_dense_pays(tokens: int, hidden: int, inter: int, num_experts: int, top_k
     in us: dense, the weights at 6.76 GB/ms from HBM and, with the tokens, at 8.8 GB/ms into the SMs (0.125 an SM, on a
     partition), the activations between the GEMMs; by expert, 128 + 6000 / SMs a GB, 14000 / SMs where few SMs bound it.  Over
     nine layers (8 to 160 experts, 1 to 8 chosen, 0.1 to 7.6 GB) of 16 to 256 tokens on 148, 108, 76, 72 and 40 SMs the form
-    chosen took 0.3 % more than the faster one in the mean.  Dense / by expert: 64 experts, 6 chosen, 2048 x 1408: 16 tokens
+    chosen took 0.25 % more than the faster one in the mean.  Dense / by expert: 64 experts, 6 chosen, 2048 x 1408: 16 tokens
     191 / 182, 24 188 / 199, 112 212 / 211, 160 227 / 214, on 72 SMs 24 198 / 245, 192 286 / 271; 8 experts, 2 chosen,
     4096 x 7168: 16 230 / 269, 192 289 / 275; 160 experts, 6 chosen, 5120 x 1536: 32 1162 / 923, 96 1206 / 1241."""
     if not _MOE_DENSE_MIN_TOKENS <= tokens <= _MOE_DENSE_MAX_TOKENS:
